@@ -86,6 +86,34 @@ def lib():
     return _lib
 
 
+# The functions that enqueue work are native (csrc/python_calls.cpp): a call here is checked, given torch's current stream
+# and launched in about the time of the launch itself.  `_calls` name -> exported symbol.
+_NATIVE = {n: "bonsai_p40_" + n for n in ("gemv", "quant_activations", "gemm", "repack", "gemv_repack", "fwht", "rmsnorm", "gdn_step", "attn")}
+_NATIVE.update({n: "bonsai_b200_" + n for n in ("fwht_quant", "swiglu", "quant_batch", "linear", "linear_static", "chain_run")})
+_NATIVE.update({n: "bonsai_" + n for n in ("kv_append", "kv_append_batch", "kv_attn_decode")})
+_calls = None
+
+
+def _native():
+    """The module of native calls, bound to the loaded library.  From the first call on, the names of this module that it
+    implements are its functions."""
+    global _calls
+    if _calls is None:
+        import importlib
+        import torch  # noqa: F401  (the module links against it)
+        handle = lib()
+        try:
+            calls = importlib.import_module(__name__ + "._calls")
+        except ImportError as e:
+            raise RuntimeError(f"the native calls are not built ({e}): run `python {os.path.join(_ROOT, 'build.py')}`") from e
+        calls.bind({n: C.cast(getattr(handle, symbol), C.c_void_p).value for n, symbol in _NATIVE.items()})
+        for n in _NATIVE:
+            if n in globals():
+                globals()[n] = getattr(calls, n)
+        _calls = calls
+    return _calls
+
+
 def _stream():
     import torch
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
@@ -119,56 +147,52 @@ def version():
 
 # ---- include/bonsai_p40.h ------------------------------------------------------------------------
 def gemv(W, xq, y, n_out, n_in):
-    return lib().bonsai_p40_gemv(_dev(W, "W"), _dev(xq, "xq"), _dev(y, "y"), n_out, n_in, _stream())
+    return _native().gemv(W, xq, y, n_out, n_in)
 
 
 def quant_activations(x, out, n):
-    return lib().bonsai_p40_quant_activations(_dev(x, "x"), _dev(out, "out"), n, _stream())
+    return _native().quant_activations(x, out, n)
 
 
 def gemm(W, Xq, Y, n_out, n_in, n_tok):
-    return lib().bonsai_p40_gemm(_dev(W, "W"), _dev(Xq, "Xq"), _dev(Y, "Y"), n_out, n_in, n_tok, _stream())
+    return _native().gemm(W, Xq, Y, n_out, n_in, n_tok)
 
 
 def repack(src, dst, n_out, n_in):
-    return lib().bonsai_p40_repack(_dev(src, "src"), _dev(dst, "dst"), n_out, n_in, _stream())
+    return _native().repack(src, dst, n_out, n_in)
 
 
 def gemv_repack(W, x, y, n_out, n_in):
-    return lib().bonsai_p40_gemv_repack(_dev(W, "W"), _dev(x, "x"), _dev(y, "y"), n_out, n_in, _stream())
+    return _native().gemv_repack(W, x, y, n_out, n_in)
 
 
 def rmsnorm(x, w, y, n_rows, n, eps):
-    return lib().bonsai_p40_rmsnorm(_dev(x, "x"), _dev(w, "w"), _dev(y, "y"), n_rows, n, eps, _stream())
+    return _native().rmsnorm(x, w, y, n_rows, n, eps)
 
 
 def gdn_step(state, q, k, v, g, beta, out, n_k_heads, n_v_heads, K, V):
-    return lib().bonsai_p40_gdn_step(_dev(state, "state"), _dev(q, "q"), _dev(k, "k"), _dev(v, "v"), _dev(g, "g"),
-                                     _dev(beta, "beta"), _dev(out, "out"), n_k_heads, n_v_heads, K, V, _stream())
+    return _native().gdn_step(state, q, k, v, g, beta, out, n_k_heads, n_v_heads, K, V)
 
 
 def attn(q, k, v, out, n_tok, n_head, n_head_kv, head_dim, scale):
-    return lib().bonsai_p40_attn(_dev(q, "q"), _dev(k, "k"), _dev(v, "v"), _dev(out, "out"), n_tok, n_head, n_head_kv,
-                                 head_dim, scale, _stream())
+    return _native().attn(q, k, v, out, n_tok, n_head, n_head_kv, head_dim, scale)
 
 
 def fwht(x, signs, n):
-    return lib().bonsai_p40_fwht(_dev(x, "x"), _dev(signs, "signs"), n, _stream())
+    return _native().fwht(x, signs, n)
 
 
 # ---- include/bonsai_b200_ext.h ---------------------------------------------------------------------
 def fwht_quant(x, signs, xq, x_rot, n):
-    return lib().bonsai_b200_fwht_quant(_dev(x, "x"), _dev(signs, "signs"), _dev(xq, "xq"), _dev(x_rot, "x_rot"), n,
-                                        _stream())
+    return _native().fwht_quant(x, signs, xq, x_rot, n)
 
 
 def swiglu(gate, up, y, n):
-    return lib().bonsai_b200_swiglu(_dev(gate, "gate"), _dev(up, "up"), _dev(y, "y"), n, _stream())
+    return _native().swiglu(gate, up, y, n)
 
 
 def quant_batch(X, signs, Xq, n_in, n_tok, rotate):
-    return lib().bonsai_b200_quant_batch(_dev(X, "X"), _dev(signs, "signs"), _dev(Xq, "Xq"), n_in, n_tok,
-                                         int(bool(rotate)), _stream())
+    return _native().quant_batch(X, signs, Xq, n_in, n_tok, rotate)
 
 
 def gemv_chunk_sums(W, xq, out, row0, n_rows, n_in):
@@ -210,14 +234,12 @@ def stream_probe(buf, nbytes, mode, sink):
 
 
 def linear(W, x, signs, y, xq_scratch, n_out, n_in):
-    return lib().bonsai_b200_linear(_dev(W, "W"), _dev(x, "x"), _dev(signs, "signs"), _dev(y, "y"),
-                                    _dev(xq_scratch, "xq_scratch"), n_out, n_in, _stream())
+    return _native().linear(W, x, signs, y, xq_scratch, n_out, n_in)
 
 
 def linear_static(W, x, signs, y, n_out, n_in):
     """The projection whose scratch lives inside the library (no allocation, n_in <= 32768)."""
-    return lib().bonsai_b200_linear_static(_dev(W, "W"), _dev(x, "x"), _dev(signs, "signs"), _dev(y, "y"), n_out,
-                                           n_in, _stream())
+    return _native().linear_static(W, x, signs, y, n_out, n_in)
 
 
 # ---- a list of projections in one launch -------------------------------------------------------------
@@ -263,7 +285,7 @@ class Chain:
         self.n_ops = len(ops)
 
     def run(self):
-        return lib().bonsai_b200_chain_run(self._h, _stream())
+        return _native().chain_run(self._h.value)
 
     def info(self):
         out = (C.c_int64 * 4)()
@@ -297,13 +319,13 @@ class KVCache:
         self.capacity = capacity
 
     def append(self, layer, pos, k, v):
-        return lib().bonsai_kv_append(self._h, layer, pos, _dev(k, "k"), _dev(v, "v"), _stream())
+        return _native().kv_append(self._h, layer, pos, k, v)
 
     def append_batch(self, layer, pos0, n_tok, k, v):
-        return lib().bonsai_kv_append_batch(self._h, layer, pos0, n_tok, _dev(k, "k"), _dev(v, "v"), _stream())
+        return _native().kv_append_batch(self._h, layer, pos0, n_tok, k, v)
 
     def attn_decode(self, layer, pos, q, out):
-        return lib().bonsai_kv_attn_decode(self._h, layer, pos, _dev(q, "q"), _dev(out, "out"), _stream())
+        return _native().kv_attn_decode(self._h, layer, pos, q, out)
 
     def gdn_state(self, layer):
         return lib().bonsai_kv_gdn_state(self._h, layer)

@@ -3,7 +3,8 @@
     python p40-kernel_b200/build.py [--force] [--verbose]
 
 Output: p40-kernel_b200/libbonsai_p40.so (same library name as the reference's build target, so a
-program linked with -lbonsai_p40 picks it up unchanged).  nvcc cross-compiles without a GPU.
+program linked with -lbonsai_p40 picks it up unchanged) and bonsai_b200/_calls.so (the Python package's
+native calls into it).  nvcc cross-compiles without a GPU.
 No fast-math: the quantiser and the rotation must perform IEEE divisions and separate mul / add.
 """
 import argparse
@@ -26,21 +27,42 @@ FLAGS = [
 ]
 
 
+CALLS_SRC = os.path.join(CSRC, "python_calls.cpp")
+CALLS = os.path.join(HERE, "bonsai_b200", "_calls.so")
+
+
 def sources():
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")) +
                   glob.glob(os.path.join(HERE, "..", "include", "*.h")))
 
 
-def stale():
-    if not os.path.exists(LIB):
+def stale(out=LIB, srcs=None):
+    if not os.path.exists(out):
         return True
-    t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(s) > t for s in sources())
+    t = os.path.getmtime(out)
+    return any(os.path.getmtime(s) > t for s in (srcs or sources()))
+
+
+def build_calls(force=False):
+    """The native calls of the Python package (CPython extension, links against torch for tensors and streams)."""
+    if not (force or stale(CALLS, [CALLS_SRC])):
+        return CALLS
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    inc = [*cpp_extension.include_paths("cuda"), sysconfig.get_paths()["include"]]
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
+                           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                           *(f"-I{d}" for d in inc), "-o", CALLS, CALLS_SRC,
+                           f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
+    return CALLS
 
 
 def build(force=False, verbose=False, tuning=True):
     """tuning: compile the geometry knobs of bonsai_b200_set_option in (the parity tests force every tiling through
     them); a production build passes tuning=False (--no-tuning) and keeps only the documented options."""
+    build_calls(force)
     if not (force or stale()):
         return LIB
     cmd = [NVCC, *FLAGS, *(["-DBONSAI_B200_TUNING"] if tuning else []), "-o", LIB, os.path.join(CSRC, "bonsai_b200.cu")]
