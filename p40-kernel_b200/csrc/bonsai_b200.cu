@@ -1406,8 +1406,8 @@ int bonsai_p40_attn(const float *q, const float *k, const float *v, float *out, 
 namespace {
 constexpr int KVM_FULL = 16, KVM_HEADS = 24, KVM_KV_HEADS = 4, KVM_CONTEXT = 262144;
 constexpr int KVM_LINEAR = 48, KVM_V_HEADS = 48, KVM_STATE = 128;
-constexpr int KV_MAX_SPLIT = KV_COMBINE_MAX;
-constexpr size_t KV_SPLIT_SMEM = KV_SPLIT_SMEM_BYTES;
+constexpr int KV_SPLIT_MIN = 2 * KV_TILE;
+constexpr int KVM_GROUP = KVM_HEADS / KVM_KV_HEADS;
 inline int64_t kv_array_bytes(int capacity) { return (int64_t)KVM_FULL * KVM_KV_HEADS * capacity * KV_ROW; }
 inline int64_t kv_gdn_bytes() { return (int64_t)KVM_LINEAR * KVM_V_HEADS * KVM_STATE * KVM_STATE * (int64_t)sizeof(float); }
 }  // namespace
@@ -1416,6 +1416,8 @@ struct bonsai_kv_cache {
     int capacity = 0;
     uint8_t *d_k = nullptr, *d_v = nullptr;
     float *d_gdn = nullptr, *d_ws = nullptr;
+    unsigned int *d_counters = nullptr;         // behind the workspace's records
+    int max_clusters = 1;                       // clusters of the decode kernel per kv head that are resident at once
 };
 
 int64_t bonsai_kv_bytes(int capacity) {
@@ -1431,13 +1433,33 @@ bonsai_kv_cache *bonsai_kv_create(int capacity, bonsai_stream stream) {
     bonsai_kv_cache *kv = new (std::nothrow) bonsai_kv_cache;
     if (!kv) return nullptr;
     kv->capacity = capacity;
-    const size_t ws = (size_t)KVM_HEADS * KV_MAX_SPLIT * KV_WS * sizeof(float);
+    const size_t ws = (size_t)KVM_KV_HEADS * KV_CLUSTER * KV_MAX_CLUSTERS * KV_REC * sizeof(float), ncnt = (size_t)KVM_KV_HEADS * KV_CLUSTER * sizeof(unsigned int);
     if (cudaMalloc(&kv->d_k, (size_t)kv_array_bytes(capacity)) != cudaSuccess || cudaMalloc(&kv->d_v, (size_t)kv_array_bytes(capacity)) != cudaSuccess ||
-        cudaMalloc(&kv->d_gdn, (size_t)kv_gdn_bytes()) != cudaSuccess || cudaMalloc(&kv->d_ws, ws) != cudaSuccess ||
-        cudaFuncSetAttribute(kv_attn_split_kernel<KVM_HEADS / KVM_KV_HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KV_SPLIT_SMEM) != cudaSuccess) {
+        cudaMalloc(&kv->d_gdn, (size_t)kv_gdn_bytes()) != cudaSuccess || cudaMalloc(&kv->d_ws, ws + ncnt) != cudaSuccess ||
+        cudaFuncSetAttribute(kv_attn_kernel<KVM_GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM_BYTES) != cudaSuccess) {
         bonsai_kv_free(kv);
         return nullptr;
     }
+    kv->d_counters = reinterpret_cast<unsigned int *>(reinterpret_cast<char *>(kv->d_ws) + ws);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(KV_CLUSTER * KV_MAX_CLUSTERS, KVM_KV_HEADS);
+    cfg.blockDim = dim3(KV_THREADS);
+    cfg.dynamicSmemBytes = KV_SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = KV_CLUSTER;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int resident = 0;
+    // the counters are zero before the first launch on any stream: the wait is paid once per cache
+    if (cudaOccupancyMaxActiveClusters(&resident, kv_attn_kernel<KVM_GROUP>, &cfg) != cudaSuccess || resident <= 0 ||
+        cudaMemsetAsync(kv->d_counters, 0, ncnt, as_stream(stream)) != cudaSuccess || cudaStreamSynchronize(as_stream(stream)) != cudaSuccess) {
+        bonsai_kv_free(kv);
+        return nullptr;
+    }
+    kv->max_clusters = resident / KVM_KV_HEADS > 0 ? resident / KVM_KV_HEADS : 1;
+    if (kv->max_clusters > KV_MAX_CLUSTERS) kv->max_clusters = KV_MAX_CLUSTERS;
     (void)cudaMemsetAsync(kv->d_gdn, 0, (size_t)kv_gdn_bytes(), as_stream(stream));
     return kv;
 }
@@ -1466,8 +1488,10 @@ int bonsai_kv_append_batch(bonsai_kv_cache *kv, int layer, int pos0, int n_tok, 
     if (layer < 0 || layer >= KVM_FULL) return 1;
     if (n_tok <= 0 || pos0 < 0 || (long long)pos0 + n_tok > kv->capacity) return 1;
     const int nrow = n_tok * KVM_KV_HEADS;
-    kv_append_kernel<<<(nrow + 7) / 8, 256, 0, as_stream(stream)>>>(kv->d_k, kv->d_v, k, v, pos0, n_tok, KVM_KV_HEADS, kv->capacity, layer);
-    return (int)cudaGetLastError();
+    // any float pointer is taken; 16-byte aligned ones get 16-byte loads
+    auto kernel = aligned16(k) && aligned16(v) ? kv_append_kernel<true> : kv_append_kernel<false>;
+    return (int)launch(kernel, dim3((unsigned)((nrow + 7) / 8)), dim3(256), 0, as_stream(stream), true, kv->d_k, kv->d_v, k, v, pos0, n_tok,
+                       KVM_KV_HEADS, kv->capacity, layer);
 }
 
 int bonsai_kv_append(bonsai_kv_cache *kv, int layer, int pos, const float *k, const float *v, bonsai_stream stream) {
@@ -1478,26 +1502,30 @@ int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *
     if (!kv || !q || !out) return 1;
     if (layer < 0 || layer >= KVM_FULL) return 1;
     if (pos < 0 || pos >= kv->capacity) return 1;
-    // splits of at least 4 tiles each, and no more CTAs than are resident at once (one wave): at long context
-    // 2 CTAs per SM x 148 SMs / 4 kv heads = 74 splits
-    const int grp = KVM_HEADS / KVM_KV_HEADS;
-    static int slots = 0;
-    if (slots == 0) {
-        int per_sm = 0, dev = 0, sms = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kv_attn_split_kernel<KVM_HEADS / KVM_KV_HEADS>, grp * 32, KV_SPLIT_SMEM) != cudaSuccess ||
-            cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            return (int)cudaGetLastError();
-        slots = per_sm * sms > 0 ? per_sm * sms : 1;
-    }
-    int n_split = (pos + 1 + 4 * KV_TILE - 1) / (4 * KV_TILE);
-    if (n_split > slots / KVM_KV_HEADS) n_split = slots / KVM_KV_HEADS > 0 ? slots / KVM_KV_HEADS : 1;
-    if (n_split > KV_MAX_SPLIT) n_split = KV_MAX_SPLIT;
-    kv_attn_split_kernel<KVM_HEADS / KVM_KV_HEADS><<<dim3((unsigned)n_split, KVM_KV_HEADS), grp * 32, KV_SPLIT_SMEM, as_stream(stream)>>>(
-        q, kv->d_k, kv->d_v, kv->d_ws, pos, n_split, KVM_KV_HEADS, kv->capacity, layer, 0.0625f);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return (int)e;
-    kv_attn_combine_kernel<<<KVM_HEADS, KV_D, 0, as_stream(stream)>>>(kv->d_ws, out, n_split);
-    return (int)cudaGetLastError();
+    // One cluster (eight splits) per kv head until a split has KV_SPLIT_MIN positions -- two tiles, both in flight at once --
+    // then more, up to what is resident at once (one wave).  Splits are multiples of 16 positions (a warp's share of a
+    // tile), not of whole tiles: at 32 768 positions the longest is 5 % longer than the mean instead of 12 %.
+    const int n_pos = pos + 1;
+    long long n_cl = n_pos / (KV_CLUSTER * KV_SPLIT_MIN);
+    if (n_cl < 1) n_cl = 1;
+    if (n_cl > kv->max_clusters) n_cl = kv->max_clusters;
+    const int n_split = (int)n_cl * KV_CLUSTER;
+    const int chunk = (((n_pos + n_split - 1) / n_split) + 15) / 16 * 16;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n_split, KVM_KV_HEADS);
+    cfg.blockDim = dim3(KV_THREADS);
+    cfg.dynamicSmemBytes = KV_SMEM_BYTES;
+    cfg.stream = as_stream(stream);
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = KV_CLUSTER;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return (int)cudaLaunchKernelEx(&cfg, kv_attn_kernel<KVM_GROUP>, q, (const uint8_t *)kv->d_k, (const uint8_t *)kv->d_v, kv->d_ws, kv->d_counters, out,
+                                   pos, chunk, KVM_KV_HEADS, kv->capacity, layer, 0.0625f);
 }
 
 // Test access to the cache arrays (byte parity of the quantiser): device pointers of K and V.

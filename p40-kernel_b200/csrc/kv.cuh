@@ -9,12 +9,8 @@
 // contiguous, 16-byte aligned span.
 //
 // Decode on B200: one CTA per (kv head, split of the positions) serves the SIX query heads that share the kv head
-// (grouped-query attention), so K and V cross HBM once per group, not once per query head.  Tiles of 32 positions
-// (8.7 KB of K, 8.7 KB of V) arrive by bulk async copy into a four-deep ring; warp w = query head w of the group for
-// the scores (int8 dot products against the query's int8 words in registers, tile-wise online softmax) and = every
-// sixth position for the value sum, where a dequantised V row is added into the accumulators of all six heads.  The
-// query heads are quantised in the kernel's prologue (no separate launch, no buffer).  Partial (m, l, acc) per
-// (head, split) go to a workspace; a second kernel merges the splits (src/kv_cache.h:153-170).
+// (grouped-query attention), so K and V cross HBM once per group, not once per query head; both products run on the
+// tensor cores.  The query heads are quantised in the kernel's prologue (no separate launch, no buffer).
 #pragma once
 
 #include "common.cuh"
@@ -22,8 +18,7 @@
 namespace b200 {
 
 constexpr int KV_D = 256, KV_NBLK = 8, KV_ROW = KV_NBLK * 34;      // 272 bytes per position and head
-constexpr int KV_TILE = 32;                                          // positions per tile
-constexpr int KV_WS = KV_D + 8;                                      // workspace floats per (head, split): acc, m, l, pad (16-byte rows)
+constexpr int KV_TILE = 64;                                          // positions per tile
 constexpr int KV_MAX_GROUP = 8;                                      // query heads per kv head the kernel is built for
 
 // ---- Q8_0 row quantiser: 4 lanes per 32-value block, 8 values per lane ---------------------------------------------
@@ -48,6 +43,7 @@ __device__ __forceinline__ void kv_quantise_8(const float (&x)[8], float &d_out,
 }
 
 // One warp per (token, kv head) row of K and of V: lane = (block lane / 4, eight dims).
+template <bool VEC>
 __global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *__restrict__ K, uint8_t *__restrict__ V,
                                                         const float *__restrict__ ksrc, const float *__restrict__ vsrc,
                                                         int pos0, int n_tok, int n_kv_head, int capacity, int layer) {
@@ -60,8 +56,17 @@ __global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *__restrict__ K,
     const float *kr = ksrc + (size_t)row * KV_D + blk * 32 + sub * 8;
     const float *vr = vsrc + (size_t)row * KV_D + blk * 32 + sub * 8;
     float kx[8], vx[8];
+    pdl_wait_prior_grid();
+    pdl_launch_dependents();
+    if (VEC) {
+        const float4 a = *reinterpret_cast<const float4 *>(kr), b = *reinterpret_cast<const float4 *>(kr + 4);
+        const float4 c = *reinterpret_cast<const float4 *>(vr), e = *reinterpret_cast<const float4 *>(vr + 4);
+        kx[0] = a.x; kx[1] = a.y; kx[2] = a.z; kx[3] = a.w; kx[4] = b.x; kx[5] = b.y; kx[6] = b.z; kx[7] = b.w;
+        vx[0] = c.x; vx[1] = c.y; vx[2] = c.z; vx[3] = c.w; vx[4] = e.x; vx[5] = e.y; vx[6] = e.z; vx[7] = e.w;
+    } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { kx[i] = kr[i]; vx[i] = vr[i]; }
+        for (int i = 0; i < 8; ++i) { kx[i] = kr[i]; vx[i] = vr[i]; }
+    }
     float kd, vd;
     uint32_t kw[2], vw[2];
     kv_quantise_8(kx, kd, kw);
@@ -79,236 +84,395 @@ __global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *__restrict__ K,
     }
 }
 
-__device__ __forceinline__ int dp4a_ss(int a, int b, int c) {
-    int r;
-    asm("dp4a.s32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+// ---- decode attention ----------------------------------------------------------------------------------------------
+// One CTA = four warps, one split of the positions of one kv head, all query heads of its group; tiles of 64 positions.
+//   scores   warp w = positions 16 w .. 16 w + 15 of the tile.  The int8 products of a 32-value block run on mma.sync
+//            (m16n8k32: 16 positions x 8 heads, int32 sums, exact); the two scales are applied per block in fp32.  The
+//            warp's 16 positions form a softmax step of their own: weights relative to the warp's maximum.
+//   values   warp w = output dims 64 w .. 64 w + 63 (two V blocks), all 64 positions and all heads.  V bytes become fp16
+//            exactly (int8 fits), a weight (softmax weight x the chunk's rescale x the V block's scale x a power of two)
+//            is split into two fp16 planes, high and low (22 - 23 bits, the size of expf's own error), which are rows 0 - 7
+//            and 8 - 15 of one m16n8k16: one instruction multiplies both planes, accumulators are fp32.
+// What bounded the kernel before was instruction issue (5860 warp instructions per 32 positions: fp32 multiply-adds of
+// every value for every head on the CUDA cores; 1500 GB/s).  This form issues about 1500.
+//
+// 34-byte blocks: two blocks are 17 words.  Of an even block words 1 .. 7 are eight-aligned code words and word 0's high
+// and word 8's low half make the eighth ("slot 0" = values 0, 1, 30, 31, slot i = values 4 i - 2 .. 4 i + 1); the odd block's
+// eight words start at word 9.  The order of values inside a block does not matter to a sum, so nothing is shifted.
+//
+// Splits: the CTAs of a cluster share one kv head; their (m, l, acc) meet through distributed shared memory, every CTA of
+// the cluster merging one slice of the dims.  With more than one cluster per head the merged slices go to a workspace and
+// the last cluster to arrive at a slice's counter adds them up and writes the output: one launch per call (the merge was
+// a kernel of its own).
+constexpr int KV_THREADS = 128, KV_WARPS = 4, KV_BUFS = 2, KV_CLUSTER = 8;
+constexpr int KV_HALF_BYTES = KV_TILE * KV_ROW;                      // the K (or V) rows of a tile
+constexpr int KV_WT_STRIDE = KV_TILE + 8;                            // weights of a head: 8 g + 2 t are 32 different banks
+constexpr int KV_SLICE = KV_D / KV_CLUSTER;                          // output dims a CTA of the cluster merges
+constexpr int KV_MAX_CLUSTERS = 64;                                  // per kv head
+constexpr int KV_REC = KV_MAX_GROUP * (KV_SLICE + 2);                // floats of a cluster's merged slice: acc, m, l
+constexpr int KV_SMEM_BYTES = 128 + KV_BUFS * 2 * KV_HALF_BYTES + KV_MAX_GROUP * KV_WT_STRIDE * 4 + 3 * KV_MAX_GROUP * 8 * 4 +
+                              KV_MAX_GROUP * 64 * 4;
+static_assert(KV_BUFS * 2 * KV_HALF_BYTES >= (KV_MAX_GROUP * KV_D + KV_MAX_CLUSTERS * KV_MAX_GROUP) * 4, "the merge reuses the tile buffers");
+
+__device__ __forceinline__ void mma_s8_16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+}
+__device__ __forceinline__ void mma_f16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// (a, b) -> high plane and what is left of them, as fp16 pairs
+__device__ __forceinline__ void split_f16x2(float a, float b, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(__fsub_rn(a, f.x), __fsub_rn(b, f.y));
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+__device__ __forceinline__ float half_bits_lo(uint32_t w) { return f16_bits_to_f32(w & 0xFFFFu); }
+__device__ __forceinline__ float half_bits_hi(uint32_t w) { return f16_bits_to_f32(w >> 16); }
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster_f32(const float *p, uint32_t rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
 
-// grid (n_split, n_kv_head), block grp * 32 threads.  Workspace per (head, split): [256 acc][m][l][6 pad].
-// Per tile of 32 positions:
-//   scores   warp w = query head w of the group.  Four lanes share a position and each reads a 68-byte piece of the K
-//            row (17 words: two blocks), eight positions per pass: a warp's loads are one contiguous run (a lane per
-//            position at a row stride of 272 bytes met 4-way bank conflicts on every load).  Tile-wise online softmax;
-//            the head's 32 weights and its rescale factor go to a small table in shared memory.
-//   values   warp w takes the positions p = w, w + grp, ...: it dequantises the V row once (lane = 8 dims, straight from
-//            the raw bytes) and adds it into the accumulators of ALL heads of the group, so the value tile is read from
-//            shared memory once, not once per head, and no fp32 copy of it is made (a thread per (position, block)
-//            writing that copy met a 32-way conflict on every store).  The warps' partial sums meet once, at the end.
-constexpr int KV_BUFS = 4;                                           // raw tiles in flight per CTA
-constexpr int KV_TILE_BYTES = 2 * KV_TILE * KV_ROW;                  // K tile, then V tile
-constexpr int KV_SPLIT_SMEM_BYTES = 128 + KV_BUFS * KV_TILE_BYTES + KV_MAX_GROUP * 64 * 4 + KV_MAX_GROUP * 8 * 4 +
-                                    KV_MAX_GROUP * (KV_TILE + 8) * 4;
-static_assert(KV_BUFS * KV_TILE_BYTES >= KV_MAX_GROUP * KV_MAX_GROUP * KV_D * 4, "the final meeting reuses the raw buffers");
+// grid (n_split, n_kv_head), cluster (KV_CLUSTER, 1, 1), n_split a multiple of KV_CLUSTER; split s covers positions
+// s * chunk .. min((s + 1) * chunk, pos + 1) - 1 (a split may be empty).  counters: one per (kv head, slice), zero before
+// and after every launch.
 template <int GRP>
-__global__ void __launch_bounds__(GRP * 32) kv_attn_split_kernel(const float *__restrict__ q, const uint8_t *__restrict__ K,
-                                                                 const uint8_t *__restrict__ V, float *__restrict__ ws,
-                                                                 int pos, int n_split, int n_kv_head, int capacity,
-                                                                 int layer, float scale) {
+__global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *__restrict__ q, const uint8_t *__restrict__ K,
+                                                                const uint8_t *__restrict__ V, float *__restrict__ ws,
+                                                                unsigned int *__restrict__ counters, float *__restrict__ out,
+                                                                int pos, int chunk, int n_kv_head, int capacity, int layer, float scale) {
+    static_assert(GRP <= KV_MAX_GROUP, "");
     extern __shared__ __align__(128) uint8_t smem[];
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem);                         // [KV_BUFS]
-    uint8_t *raw = smem + 128;                                                   // [KV_BUFS][K tile | V tile]
-    uint32_t *q8 = reinterpret_cast<uint32_t *>(raw + KV_BUFS * KV_TILE_BYTES);  // [grp][8 blocks][8 words]
-    float *qd = reinterpret_cast<float *>(q8 + KV_MAX_GROUP * 64);               // [grp][8] scales x `scale`
-    float *pwt = qd + KV_MAX_GROUP * 8;                                          // [grp][32 weights, rescale factor, 7 pad]
+    uint64_t *kfull = reinterpret_cast<uint64_t *>(smem), *vfull = kfull + KV_BUFS;
+    uint8_t *raw = smem + 128;                                                   // [KV_BUFS][K rows | V rows]
+    float *wt = reinterpret_cast<float *>(raw + KV_BUFS * 2 * KV_HALF_BYTES);    // [8 heads][KV_WT_STRIDE]
+    float *mw = wt + KV_MAX_GROUP * KV_WT_STRIDE;                                // [4 chunks, 4 pad][8 heads] maxima
+    float *lw = mw + KV_MAX_GROUP * 8;                                           // ... and sums of the weights
+    float *qd = lw + KV_MAX_GROUP * 8;                                           // [8 heads][8 blocks] query scales x `scale`
+    uint32_t *q8 = reinterpret_cast<uint32_t *>(qd + KV_MAX_GROUP * 8);          // [8 heads][8 blocks][8 words]
 
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int split = blockIdx.x, kvh = blockIdx.y, head = kvh * GRP + warp;
-    const int n_pos = pos + 1;
-    const int chunk = (((n_pos + n_split - 1) / n_split) + KV_TILE - 1) / KV_TILE * KV_TILE;   // whole tiles per split
-    const int p_begin = split * chunk, p_end = min(p_begin + chunk, n_pos);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int split = blockIdx.x, kvh = blockIdx.y;
+    const int p_begin = split * chunk, p_end = min(p_begin + chunk, pos + 1);
     const int ntiles = p_end > p_begin ? (p_end - p_begin + KV_TILE - 1) / KV_TILE : 0;
     const uint8_t *kbase = K + (((size_t)layer * n_kv_head + kvh) * capacity) * KV_ROW;
     const uint8_t *vbase = V + (((size_t)layer * n_kv_head + kvh) * capacity) * KV_ROW;
-    const uint64_t pol = policy_evict_first();
 
-    auto issue = [&](int t) {           // one thread
-        const int p0 = p_begin + t * KV_TILE, n = min(KV_TILE, p_end - p0);
+    auto issue = [&](int i) {           // one thread
+        const uint64_t pol = policy_evict_first();
+        const int p0 = p_begin + i * KV_TILE, n = min(KV_TILE, p_end - p0), b = i % KV_BUFS;
         const uint32_t bytes = (uint32_t)n * KV_ROW;
-        uint8_t *dst = raw + (size_t)(t % KV_BUFS) * KV_TILE_BYTES;
+        uint8_t *dst = raw + (size_t)b * 2 * KV_HALF_BYTES;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect_tx(&full[t % KV_BUFS], 2 * bytes);
-        bulk_g2s(dst, kbase + (size_t)p0 * KV_ROW, bytes, &full[t % KV_BUFS], pol);
-        bulk_g2s(dst + KV_TILE * KV_ROW, vbase + (size_t)p0 * KV_ROW, bytes, &full[t % KV_BUFS], pol);
+        mbar_expect_tx(&kfull[b], bytes);
+        bulk_g2s(dst, kbase + (size_t)p0 * KV_ROW, bytes, &kfull[b], pol);
+        mbar_expect_tx(&vfull[b], bytes);
+        bulk_g2s(dst + KV_HALF_BYTES, vbase + (size_t)p0 * KV_ROW, bytes, &vfull[b], pol);
     };
-    if (threadIdx.x == 0) {
-        for (int b = 0; b < KV_BUFS; ++b) mbar_init(&full[b], 1);
+    if (tid == 0) {
+        for (int b = 0; b < KV_BUFS; ++b) mbar_init(&kfull[b], 1), mbar_init(&vfull[b], 1);
         mbar_fence_init();
-        for (int t = 0; t < min(ntiles, KV_BUFS - 1); ++t) issue(t);
     }
+    for (int i = tid; i < KV_MAX_GROUP * KV_WT_STRIDE; i += KV_THREADS) wt[i] = 0.0f;      // heads past the group stay 0
+    for (int i = tid; i < KV_MAX_GROUP * 8; i += KV_THREADS) qd[i] = 0.0f, mw[i] = 0.0f, lw[i] = 0.0f;
+    for (int i = tid; i < KV_MAX_GROUP * 64; i += KV_THREADS) q8[i] = 0u;
+    __syncthreads();
+    pdl_wait_prior_grid();              // q and the newest row of the cache come from the kernels before this one
+    pdl_launch_dependents();
+    if (tid == 0)
+        for (int i = 0; i < min(ntiles, KV_BUFS); ++i) issue(i);
     // the group's query heads, quantised as the cache rows are (host rule, src/kv_cache.h:100-117)
-    {
+    for (int h = warp; h < GRP; h += KV_WARPS) {
         const int blk = lane >> 2, sub = lane & 3;
-        const float *qr = q + (size_t)head * KV_D + blk * 32 + sub * 8;
+        const float *qr = q + (size_t)(kvh * GRP + h) * KV_D + blk * 32 + sub * 8;
         float x[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] = qr[i];
         float d;
         uint32_t w[2];
         kv_quantise_8(x, d, w);
-        q8[(warp * 8 + blk) * 8 + 2 * sub] = w[0];
-        q8[(warp * 8 + blk) * 8 + 2 * sub + 1] = w[1];
-        if (sub == 0) qd[warp * 8 + blk] = __fmul_rn(f16_bits_to_f32(f32_to_f16_bits_ties_away(d)), scale);
+        q8[(h * 8 + blk) * 8 + 2 * sub] = w[0];
+        q8[(h * 8 + blk) * 8 + 2 * sub + 1] = w[1];
+        if (sub == 0) qd[h * 8 + blk] = __fmul_rn(f16_bits_to_f32(f32_to_f16_bits_ties_away(d)), scale);
     }
     __syncthreads();
-    // scores: lane = (position of the pass, quarter of the row); the quarter's two query blocks stay in registers
-    const int pp = lane >> 2, sub = lane & 3;
-    uint32_t qw[2][8];
-    float qs[2];
+    // B operand of the scores: head g, words t and t + 4 of every block, in the order the K rows are read in
+    uint32_t qb[8][2];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-#pragma unroll
-        for (int w = 0; w < 8; ++w) qw[j][w] = q8[(warp * 8 + 2 * sub + j) * 8 + w];
-        qs[j] = qd[warp * 8 + 2 * sub + j];
+    for (int b = 0; b < 8; ++b) {
+        const uint32_t *src = q8 + (g * 8 + b) * 8;
+        if (b & 1) {
+            qb[b][0] = src[t];
+            qb[b][1] = src[t + 4];
+        } else {                        // even block: slot 0 = values 0, 1, 30, 31; slot i = values 4 i - 2 .. 4 i + 1
+            qb[b][0] = t == 0 ? __byte_perm(src[0], src[7], 0x7610) : __byte_perm(src[t - 1], src[t], 0x5432);
+            qb[b][1] = __byte_perm(src[t + 3], src[t + 4], 0x5432);
+        }
     }
-    float m = -INFINITY, l = 0.0f;              // of this warp's head
-    float acc[GRP][8];                          // of this warp's positions, every head of the group
+    float m_run = -INFINITY, l_run = 0.0f;                  // of head g
+    uint32_t dv_run[2] = {0u, 0u};                          // largest V scale so far (fp16 bits) of the warp's two blocks
+    float acc[2][4][4];
 #pragma unroll
-    for (int h = 0; h < GRP; ++h)
+    for (int b = 0; b < 2; ++b)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[h][i] = 0.0f;
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[b][j][i] = 0.0f;
+    // the power of two that puts the largest V scale at 2^13 .. 2^14 (weights are at most 1): fp16 planes with room below
+    auto lift = [](uint32_t bits) -> float {
+        const int e = max(1, (int)(bits >> 10) & 31);       // biased fp16 exponent of the scale
+        return __uint_as_float((uint32_t)(127 + 13 + 15 - e) << 23);
+    };
 
-    for (int t = 0; t < ntiles; ++t) {
-        // buffer (t - 1) % KV_BUFS was released by the barrier that ended tile t - 1
-        if (threadIdx.x == 0 && t + KV_BUFS - 1 < ntiles) issue(t + KV_BUFS - 1);
-        // (the outcome of the bounded wait is made uniform: a CTA either goes on as a whole or leaves as a whole)
-        if (!__syncthreads_and(mbar_wait_bounded(&full[t % KV_BUFS], (uint32_t)((t / KV_BUFS) & 1)) ? 1 : 0)) break;
-        const uint8_t *kt = raw + (size_t)(t % KV_BUFS) * KV_TILE_BYTES;
-        const uint8_t *vt = kt + KV_TILE * KV_ROW;
-        const int n = min(KV_TILE, p_end - (p_begin + t * KV_TILE));
-        // scores of the tile's 32 positions in four passes of eight
-        float s[4];
+    for (int i = 0; i < ntiles; ++i) {
+        const int b = i % KV_BUFS;
+        const uint32_t par = (uint32_t)((i / KV_BUFS) & 1);
+        const int n = min(KV_TILE, p_end - (p_begin + i * KV_TILE));
+        uint8_t *kt = raw + (size_t)b * 2 * KV_HALF_BYTES, *vt = kt + KV_HALF_BYTES;
+        bool ok = mbar_wait_hot(&kfull[b], par);
+        {   // ---- scores of positions 16 warp .. + 15
+            const uint32_t *r0 = reinterpret_cast<const uint32_t *>(kt) + (size_t)(16 * warp + g) * (KV_ROW / 4);
+            const uint32_t *r1 = r0 + 8 * (KV_ROW / 4);
+            float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};          // (position g | g + 8, head 2 t | 2 t + 1)
 #pragma unroll
-        for (int ps = 0; ps < 4; ++ps) {
-            const int p = 8 * ps + pp;
-            float part = 0.0f;
-            if (p < n) {
-                // the quarter's 68 bytes = 17 words: block 2 sub (scale in the low half of word 0, its int8 from byte 2)
-                // and block 2 sub + 1 (scale in the high half of word 8, its int8 from word 9)
-                const uint32_t *kw = reinterpret_cast<const uint32_t *>(kt + (size_t)p * KV_ROW + 68 * sub);
-                uint32_t L[17];
-#pragma unroll
-                for (int i = 0; i < 17; ++i) L[i] = kw[i];
-                int s0 = 0, s1 = 0;
-#pragma unroll
-                for (int w = 0; w < 8; ++w) {
-                    s0 = dp4a_ss((int)qw[0][w], (int)__funnelshift_r(L[w], L[w + 1], 16), s0);
-                    s1 = dp4a_ss((int)qw[1][w], (int)L[9 + w], s1);
+            for (int pr = 0; pr < 4; ++pr) {
+                const uint32_t *u0 = r0 + 17 * pr, *u1 = r1 + 17 * pr;
+                const uint32_t d0 = u0[0], d1 = u1[0], e0 = u0[8], e1 = u1[8];
+                uint32_t x0 = u0[t], x1 = u1[t];
+                const uint32_t y0 = u0[t + 4], y1 = u1[t + 4];
+                if (t == 0) {
+                    x0 = __byte_perm(x0, e0, 0x5432);
+                    x1 = __byte_perm(x1, e1, 0x5432);
                 }
-                part = __fmul_rn(__fmul_rn(qs[0], f16_bits_to_f32(L[0] & 0xFFFFu)), (float)s0);
-                part = __fadd_rn(part, __fmul_rn(__fmul_rn(qs[1], f16_bits_to_f32(L[8] >> 16)), (float)s1));
+                int de[4], dq[4];
+                mma_s8_16832(de, x0, x1, y0, y1, qb[2 * pr][0], qb[2 * pr][1]);
+                mma_s8_16832(dq, u0[9 + t], u1[9 + t], u0[13 + t], u1[13 + t], qb[2 * pr + 1][0], qb[2 * pr + 1][1]);
+                const float ke0 = half_bits_lo(d0), ke1 = half_bits_lo(d1), ko0 = half_bits_hi(e0), ko1 = half_bits_hi(e1);
+                const float qe0 = qd[(2 * t) * 8 + 2 * pr], qe1 = qd[(2 * t + 1) * 8 + 2 * pr];
+                const float qo0 = qd[(2 * t) * 8 + 2 * pr + 1], qo1 = qd[(2 * t + 1) * 8 + 2 * pr + 1];
+                s[0] = __fmaf_rn(__fmul_rn(qe0, ke0), (float)de[0], s[0]);
+                s[1] = __fmaf_rn(__fmul_rn(qe1, ke0), (float)de[1], s[1]);
+                s[2] = __fmaf_rn(__fmul_rn(qe0, ke1), (float)de[2], s[2]);
+                s[3] = __fmaf_rn(__fmul_rn(qe1, ke1), (float)de[3], s[3]);
+                s[0] = __fmaf_rn(__fmul_rn(qo0, ko0), (float)dq[0], s[0]);
+                s[1] = __fmaf_rn(__fmul_rn(qo1, ko0), (float)dq[1], s[1]);
+                s[2] = __fmaf_rn(__fmul_rn(qo0, ko1), (float)dq[2], s[2]);
+                s[3] = __fmaf_rn(__fmul_rn(qo1, ko1), (float)dq[3], s[3]);
             }
-            part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, 1));
-            part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, 2));
-            s[ps] = p < n ? part : -INFINITY;
+            const int pa = 16 * warp + g, pb = pa + 8;
+            const bool va = pa < n, vb = pb < n;
+            float mx0 = fmaxf(va ? s[0] : -INFINITY, vb ? s[2] : -INFINITY), mx1 = fmaxf(va ? s[1] : -INFINITY, vb ? s[3] : -INFINITY);
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+            }
+            const float w0 = va ? expf(__fsub_rn(s[0], mx0)) : 0.0f, w1 = va ? expf(__fsub_rn(s[1], mx1)) : 0.0f;
+            const float w2 = vb ? expf(__fsub_rn(s[2], mx0)) : 0.0f, w3 = vb ? expf(__fsub_rn(s[3], mx1)) : 0.0f;
+            float l0 = __fadd_rn(w0, w2), l1 = __fadd_rn(w1, w3);
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                l0 = __fadd_rn(l0, __shfl_xor_sync(0xffffffffu, l0, o));
+                l1 = __fadd_rn(l1, __shfl_xor_sync(0xffffffffu, l1, o));
+            }
+            if (2 * t < GRP) {
+                wt[(2 * t) * KV_WT_STRIDE + pa] = w0;
+                wt[(2 * t) * KV_WT_STRIDE + pb] = w2;
+                if (g == 0) mw[warp * 8 + 2 * t] = mx0, lw[warp * 8 + 2 * t] = l0;
+            }
+            if (2 * t + 1 < GRP) {
+                wt[(2 * t + 1) * KV_WT_STRIDE + pa] = w1;
+                wt[(2 * t + 1) * KV_WT_STRIDE + pb] = w3;
+                if (g == 0) mw[warp * 8 + 2 * t + 1] = mx1, lw[warp * 8 + 2 * t + 1] = l1;
+            }
         }
-        // tile-wise online softmax (every lane of a quad holds the same four scores)
-        float tmax = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+        ok = mbar_wait_hot(&vfull[b], par) && ok;
+        if (n < KV_TILE)                // rows past the end: zeros (their weights are 0, but stale scales need not be finite)
+            for (int z = tid; z < (KV_TILE - n) * (KV_ROW / 4); z += KV_THREADS) reinterpret_cast<uint32_t *>(vt)[n * (KV_ROW / 4) + z] = 0u;
+        // (the outcome of the bounded waits is made uniform: a CTA either goes on as a whole or leaves as a whole)
+        if (!__syncthreads_and(ok ? 1 : 0)) break;
+        {   // ---- values: dims 64 warp .. + 63
+            const uint32_t *v32 = reinterpret_cast<const uint32_t *>(vt) + 17 * warp;
+            uint32_t big[2];
+            {
+                const uint32_t *ra = v32 + (size_t)lane * (KV_ROW / 4), *rb = ra + 32 * (KV_ROW / 4);
+                big[0] = __reduce_max_sync(0xffffffffu, max(ra[0] & 0x7FFFu, rb[0] & 0x7FFFu));
+                big[1] = __reduce_max_sync(0xffffffffu, max((ra[8] >> 16) & 0x7FFFu, (rb[8] >> 16) & 0x7FFFu));
+            }
+            float mc[4], m_new = m_run, f[4], lsum = 0.0f;
 #pragma unroll
-        for (int o = 4; o < 32; o <<= 1) tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-        const float m_new = fmaxf(m, tmax);
-        const float alpha = expf(__fsub_rn(m, m_new));
-        float psum = 0.0f;
+            for (int c = 0; c < 4; ++c) m_new = fmaxf(m_new, mc[c] = mw[c * 8 + g]);
+            const float alpha = expf(__fsub_rn(m_run, m_new));
 #pragma unroll
-        for (int ps = 0; ps < 4; ++ps) {
-            const float w = 8 * ps + pp < n ? expf(__fsub_rn(s[ps], m_new)) : 0.0f;
-            if (sub == 0) pwt[warp * (KV_TILE + 8) + 8 * ps + pp] = w;
-            psum = __fadd_rn(psum, w);
-        }
-        if (lane == 0) pwt[warp * (KV_TILE + 8) + KV_TILE] = alpha;
+            for (int c = 0; c < 4; ++c) {
+                f[c] = expf(__fsub_rn(mc[c], m_new));
+                lsum = __fmaf_rn(lw[c * 8 + g], f[c], lsum);
+            }
+            l_run = __fmaf_rn(l_run, alpha, lsum);
+            m_run = m_new;
+            float up[2];
 #pragma unroll
-        for (int o = 4; o < 32; o <<= 1) psum = __fadd_rn(psum, __shfl_xor_sync(0xffffffffu, psum, o));
-        l = __fadd_rn(__fmul_rn(l, alpha), psum);
-        m = m_new;
-        __syncthreads();                                            // every head's weights of this tile are in the table
+            for (int bb = 0; bb < 2; ++bb) {
+                const float before = lift(dv_run[bb]);
+                dv_run[bb] = max(dv_run[bb], big[bb]);
+                up[bb] = lift(dv_run[bb]);
+                const float keep = i == 0 ? 0.0f : __fmul_rn(alpha, __fdiv_rn(up[bb], before));      // a power of two: exact
+                if (__any_sync(0xffffffffu, keep != 1.0f)) {
 #pragma unroll
-        for (int h = 0; h < GRP; ++h) {
-            const float al = pwt[h * (KV_TILE + 8) + KV_TILE];
+                    for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[h][i] = __fmul_rn(acc[h][i], al);
-        }
-        for (int p = warp; p < n; p += GRP) {
-            const unsigned short *src = reinterpret_cast<const unsigned short *>(vt + (size_t)p * KV_ROW + (lane >> 2) * 34);
-            const float dv = f16_bits_to_f32(src[0]);
-            const unsigned short *b8 = src + 1 + 4 * (lane & 3);
-            // int8 -> fp32 without the conversion unit: the byte, with its sign bit flipped (value + 128), is placed under
-            // the exponent of 2^23 by a byte permute, and 2^23 + 128 is subtracted: exact
-            float v[8];
-#pragma unroll
-            for (int h2 = 0; h2 < 2; ++h2) {
-                const uint32_t four = ((uint32_t)b8[2 * h2] | ((uint32_t)b8[2 * h2 + 1] << 16)) ^ 0x80808080u;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float f = __uint_as_float(__byte_perm(four, 0x4B000000u, 0x7440u + (uint32_t)e));
-                    v[4 * h2 + e] = __fmul_rn(__fsub_rn(f, 8388736.0f), dv);
+                        for (int e = 0; e < 4; ++e) acc[bb][j][e] = __fmul_rn(acc[bb][j][e], keep);
                 }
             }
 #pragma unroll
-            for (int h = 0; h < GRP; ++h) {
-                const float wp = pwt[h * (KV_TILE + 8) + p];
+            for (int c = 0; c < 4; ++c) {
+                if (16 * c >= n) break;                     // CTA-uniform
+                const uint32_t *rows = v32 + (size_t)(16 * c + 2 * t) * (KV_ROW / 4);
+                uint32_t ev[4], od[4];
+                float de[4], dq[4];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) acc[h][i] = __fmaf_rn(wp, v[i], acc[h][i]);
+                for (int r = 0; r < 4; ++r) {
+                    const uint32_t *u = rows + (size_t)((r & 1) + 8 * (r >> 1)) * (KV_ROW / 4);
+                    const uint32_t d0 = u[0], e = u[8];
+                    uint32_t x = u[g];
+                    if (g == 0) x = __byte_perm(x, e, 0x5432);
+                    ev[r] = x ^ 0x80808080u;
+                    od[r] = u[9 + g] ^ 0x80808080u;
+                    de[r] = half_bits_lo(d0);
+                    dq[r] = half_bits_hi(e);
+                }
+                const float2 wa = *reinterpret_cast<const float2 *>(wt + g * KV_WT_STRIDE + 16 * c + 2 * t);
+                const float2 wb = *reinterpret_cast<const float2 *>(wt + g * KV_WT_STRIDE + 16 * c + 2 * t + 8);
+#pragma unroll
+                for (int bb = 0; bb < 2; ++bb) {
+                    const float fu = __fmul_rn(f[c], up[bb]);
+                    const float *dd = bb ? dq : de;
+                    const uint32_t *vv = bb ? od : ev;
+                    uint32_t h01, l01, h23, l23;
+                    split_f16x2(__fmul_rn(__fmul_rn(wa.x, fu), dd[0]), __fmul_rn(__fmul_rn(wa.y, fu), dd[1]), h01, l01);
+                    split_f16x2(__fmul_rn(__fmul_rn(wb.x, fu), dd[2]), __fmul_rn(__fmul_rn(wb.y, fu), dd[3]), h23, l23);
+                    // byte j of four rows -> fp16: under the exponent of 1024 (value + 128, sign bit flipped above), minus 1152
+                    const uint32_t p01 = __byte_perm(vv[0], vv[1], 0x5140), q01 = __byte_perm(vv[0], vv[1], 0x7362);
+                    const uint32_t p23 = __byte_perm(vv[2], vv[3], 0x5140), q23 = __byte_perm(vv[2], vv[3], 0x7362);
+                    const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        uint32_t b0 = __byte_perm(j < 2 ? p01 : q01, 0x64646464u, (j & 1) ? 0x4342 : 0x4140);
+                        uint32_t b1 = __byte_perm(j < 2 ? p23 : q23, 0x64646464u, (j & 1) ? 0x4342 : 0x4140);
+                        const __half2 v0 = __hsub2(*reinterpret_cast<__half2 *>(&b0), bias), v1 = __hsub2(*reinterpret_cast<__half2 *>(&b1), bias);
+                        mma_f16_16816(acc[bb][j], h01, l01, h23, l23, *reinterpret_cast<const uint32_t *>(&v0), *reinterpret_cast<const uint32_t *>(&v1));
+                    }
+                }
             }
         }
-        __syncthreads();                                            // tile t's buffer and the table may be overwritten
+        __syncthreads();                                            // tile i's buffer and the tables may be overwritten
+        if (tid == 0 && i + KV_BUFS < ntiles) issue(i + KV_BUFS);
     }
-    // the warps' partial sums meet: red[warp][head][256] over the raw buffers (nothing is in flight any more)
-    float *red = reinterpret_cast<float *>(raw);
+    // ---- the CTA's (m, l, acc); the tile buffers are free
+    float *so = reinterpret_cast<float *>(raw), *sm = so + KV_MAX_GROUP * KV_D, *sl = sm + KV_MAX_GROUP;
+    if (g < GRP) {
 #pragma unroll
-    for (int h = 0; h < GRP; ++h) {
-        float4 *dst = reinterpret_cast<float4 *>(red + ((size_t)warp * GRP + h) * KV_D + 8 * lane);
-        dst[0] = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
-        dst[1] = make_float4(acc[h][4], acc[h][5], acc[h][6], acc[h][7]);
+        for (int bb = 0; bb < 2; ++bb) {
+            const float down = __fdiv_rn(1.0f, lift(dv_run[bb]));       // a power of two
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int slot = 2 * t + e;
+                    const int in_blk = bb ? 4 * slot + j : (slot == 0 ? (j < 2 ? j : 28 + j) : 4 * slot - 2 + j);
+                    so[g * KV_D + 64 * warp + 32 * bb + in_blk] = __fmul_rn(__fadd_rn(acc[bb][j][e], acc[bb][j][e + 2]), down);
+                }
+        }
+        if (warp == 0 && t == 0) sm[g] = m_run, sl[g] = l_run;
+    }
+    cluster_sync();
+    // ---- one slice of the dims per CTA of the cluster, added over its CTAs in rank order
+    const uint32_t rank = cluster_rank();
+    const int n_cl = gridDim.x / KV_CLUSTER, cl = blockIdx.x / KV_CLUSTER;
+    float *cw = wt, *cm = mw, *cl_sum = lw;                            // [8 heads][8 ranks] weights; maxima; denominators
+    if (warp < 2) {
+        const int h = tid >> 3, rr = tid & 7;
+        const float mm = h < GRP ? ld_cluster_f32(sm + h, (uint32_t)rr) : -INFINITY;
+        const float ll = h < GRP ? ld_cluster_f32(sl + h, (uint32_t)rr) : 0.0f;
+        float mx = mm;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float w = mm == -INFINITY ? 0.0f : expf(__fsub_rn(mm, mx));      // a split without positions: 0
+        float den = __fmul_rn(ll, w);
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) den = __fadd_rn(den, __shfl_xor_sync(0xffffffffu, den, o));
+        cw[h * 8 + rr] = w;
+        if (rr == 0) cm[h] = mx, cl_sum[h] = den;
     }
     __syncthreads();
-    float o[8];
+    float *rec = ws + (((size_t)kvh * KV_CLUSTER + rank) * n_cl + cl) * KV_REC;
+    for (int o = tid; o < GRP * KV_SLICE; o += KV_THREADS) {
+        const int h = o / KV_SLICE, d = o % KV_SLICE;
+        float a = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = 0.0f;
-#pragma unroll
-    for (int w = 0; w < GRP; ++w) {             // this warp's head, the warps in ascending order
-        const float4 *srcp = reinterpret_cast<const float4 *>(red + ((size_t)w * GRP + warp) * KV_D + 8 * lane);
-        const float4 a = srcp[0], b = srcp[1];
-        o[0] = __fadd_rn(o[0], a.x); o[1] = __fadd_rn(o[1], a.y); o[2] = __fadd_rn(o[2], a.z); o[3] = __fadd_rn(o[3], a.w);
-        o[4] = __fadd_rn(o[4], b.x); o[5] = __fadd_rn(o[5], b.y); o[6] = __fadd_rn(o[6], b.z); o[7] = __fadd_rn(o[7], b.w);
+        for (int rr = 0; rr < KV_CLUSTER; ++rr)
+            a = __fmaf_rn(ld_cluster_f32(so + h * KV_D + (int)rank * KV_SLICE + d, (uint32_t)rr), cw[h * 8 + rr], a);
+        if (n_cl == 1) out[((size_t)kvh * GRP + h) * KV_D + (int)rank * KV_SLICE + d] = __fmul_rn(a, __fdiv_rn(1.0f, cl_sum[h]));
+        else rec[o] = a;
     }
-    float *slot = ws + ((size_t)head * n_split + split) * KV_WS;
-    *reinterpret_cast<float4 *>(slot + 8 * lane) = make_float4(o[0], o[1], o[2], o[3]);
-    *reinterpret_cast<float4 *>(slot + 8 * lane + 4) = make_float4(o[4], o[5], o[6], o[7]);
-    if (lane == 0) { slot[KV_D] = m; slot[KV_D + 1] = l; }
-}
-
-// Merge of the splits and normalisation (src/kv_cache.h:153-176): one CTA per query head, thread = output dimension.
-// The weights exp(m_s - max) of the splits are formed once in shared memory; every thread then adds its dimension
-// over the splits with independent, coalesced loads (a single warp walking the splits one dependent load after the
-// other took 65 us at 64 splits).
-constexpr int KV_COMBINE_MAX = 256;
-__global__ void __launch_bounds__(KV_D) kv_attn_combine_kernel(const float *__restrict__ ws, float *__restrict__ out, int n_split) {
-    __shared__ float wgt[KV_COMBINE_MAX];
-    __shared__ float red[2];
-    const int head = blockIdx.x, d = threadIdx.x;
-    const float *base = ws + (size_t)head * n_split * KV_WS;
-    if (d < 32) {                                                   // one warp: maximum, weights, denominator
-        float mx = -INFINITY;
-        for (int s = d; s < n_split; s += 32)
-            if (base[(size_t)s * KV_WS + KV_D + 1] != 0.0f) mx = fmaxf(mx, base[(size_t)s * KV_WS + KV_D]);
+    cluster_sync();                     // nobody leaves while its shared memory is read
+    if (n_cl == 1) return;
+    // ---- several clusters per head: the last one to bring this slice adds them in order (fixed, whichever is last)
+    if (tid < GRP) {
+        rec[KV_MAX_GROUP * KV_SLICE + tid] = cm[tid];
+        rec[KV_MAX_GROUP * KV_SLICE + KV_MAX_GROUP + tid] = cl_sum[tid];
+    }
+    __threadfence();
+    __syncthreads();
+    unsigned int *counter = counters + kvh * KV_CLUSTER + rank;
+    int last = 0;
+    if (tid == 0) last = atomicAdd(counter, 1u) == (unsigned int)n_cl - 1u;
+    if (!__syncthreads_or(last)) return;
+    __threadfence();
+    const float *all = ws + ((size_t)kvh * KV_CLUSTER + rank) * n_cl * KV_REC;
+    for (int h = warp; h < GRP; h += KV_WARPS) {
+        const float *ml = all + KV_MAX_GROUP * KV_SLICE + h;
+        float mx = -INFINITY, den = 0.0f;
+        for (int c = lane; c < n_cl; c += 32) mx = fmaxf(mx, __ldcg(ml + (size_t)c * KV_REC));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        float lsum = 0.0f;
-        for (int s = d; s < n_split; s += 32) {
-            const float sl = base[(size_t)s * KV_WS + KV_D + 1];
-            const float w = sl != 0.0f ? expf(__fsub_rn(base[(size_t)s * KV_WS + KV_D], mx)) : 0.0f;   // a split without positions: 0
-            wgt[s] = w;
-            lsum = __fadd_rn(lsum, __fmul_rn(sl, w));
+        for (int c = lane; c < n_cl; c += 32) {
+            const float mm = __ldcg(ml + (size_t)c * KV_REC);
+            const float w = mm == -INFINITY ? 0.0f : expf(__fsub_rn(mm, mx));
+            wt[c * KV_MAX_GROUP + h] = w;
+            den = __fmaf_rn(__ldcg(ml + (size_t)c * KV_REC + KV_MAX_GROUP), w, den);
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) lsum = __fadd_rn(lsum, __shfl_xor_sync(0xffffffffu, lsum, o));
-        if (d == 0) red[0] = lsum;
+        for (int o = 16; o > 0; o >>= 1) den = __fadd_rn(den, __shfl_xor_sync(0xffffffffu, den, o));
+        if (lane == 0) qd[h] = __fdiv_rn(1.0f, den);
     }
     __syncthreads();
-    float a = 0.0f;
+    for (int o = tid; o < GRP * KV_SLICE; o += KV_THREADS) {
+        const int h = o / KV_SLICE, d = o % KV_SLICE;
+        float a = 0.0f;
 #pragma unroll 8
-    for (int s = 0; s < n_split; ++s) a = __fmaf_rn(base[(size_t)s * KV_WS + d], wgt[s], a);
-    out[(size_t)head * KV_D + d] = __fmul_rn(a, __fdiv_rn(1.0f, red[0]));
+        for (int c = 0; c < n_cl; ++c) a = __fmaf_rn(__ldcg(all + (size_t)c * KV_REC + o), wt[c * KV_MAX_GROUP + h], a);
+        out[((size_t)kvh * GRP + h) * KV_D + (int)rank * KV_SLICE + d] = __fmul_rn(a, qd[h]);
+    }
+    if (tid == 0) *counter = 0u;
 }
 
 }  // namespace b200
