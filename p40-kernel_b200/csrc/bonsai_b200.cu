@@ -1406,7 +1406,7 @@ int bonsai_p40_attn(const float *q, const float *k, const float *v, float *out, 
 namespace {
 constexpr int KVM_FULL = 16, KVM_HEADS = 24, KVM_KV_HEADS = 4, KVM_CONTEXT = 262144;
 constexpr int KVM_LINEAR = 48, KVM_V_HEADS = 48, KVM_STATE = 128;
-constexpr int KV_SPLIT_MIN = 2 * KV_TILE;
+constexpr int KV_SPLIT_MIN = 2 * KV_TILE;      // positions
 constexpr int KVM_GROUP = KVM_HEADS / KVM_KV_HEADS;
 inline int64_t kv_array_bytes(int capacity) { return (int64_t)KVM_FULL * KVM_KV_HEADS * capacity * KV_ROW; }
 inline int64_t kv_gdn_bytes() { return (int64_t)KVM_LINEAR * KVM_V_HEADS * KVM_STATE * KVM_STATE * (int64_t)sizeof(float); }

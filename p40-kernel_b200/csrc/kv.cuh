@@ -112,7 +112,7 @@ constexpr int KV_MAX_CLUSTERS = 64;                                  // per kv h
 constexpr int KV_REC = KV_MAX_GROUP * (KV_SLICE + 2);                // floats of a cluster's merged slice: acc, m, l
 constexpr int KV_SMEM_BYTES = 128 + KV_BUFS * 2 * KV_HALF_BYTES + KV_MAX_GROUP * KV_WT_STRIDE * 4 + 3 * KV_MAX_GROUP * 8 * 4 +
                               KV_MAX_GROUP * 64 * 4;
-static_assert(KV_BUFS * 2 * KV_HALF_BYTES >= (KV_MAX_GROUP * KV_D + KV_MAX_CLUSTERS * KV_MAX_GROUP) * 4, "the merge reuses the tile buffers");
+static_assert(16384 >= KV_MAX_GROUP * (KV_D + 2) * 4 && KV_BUFS * 2 * KV_HALF_BYTES >= 16384 + 3 * KV_MAX_CLUSTERS * KV_MAX_GROUP * 4, "the merge reuses the tile buffers");
 
 __device__ __forceinline__ void mma_s8_16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
@@ -139,8 +139,14 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Adds 1 to a counter in global memory; what the CTA wrote before the barrier in front of this call is visible to whoever
+// reads the sum, and what they wrote to this CTA after the barrier behind it.
+__device__ __forceinline__ unsigned int count_arrival(unsigned int *counter) {
+    unsigned int old;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
+    return old;
 }
 __device__ __forceinline__ float ld_cluster_f32(const float *p, uint32_t rank) {
     uint32_t a;
@@ -200,18 +206,29 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *__r
     if (tid == 0)
         for (int i = 0; i < min(ntiles, KV_BUFS); ++i) issue(i);
     // the group's query heads, quantised as the cache rows are (host rule, src/kv_cache.h:100-117)
-    for (int h = warp; h < GRP; h += KV_WARPS) {
+    {
+        constexpr int ROUNDS = (GRP + KV_WARPS - 1) / KV_WARPS;
         const int blk = lane >> 2, sub = lane & 3;
-        const float *qr = q + (size_t)(kvh * GRP + h) * KV_D + blk * 32 + sub * 8;
-        float x[8];
+        float x[ROUNDS][8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = qr[i];
-        float d;
-        uint32_t w[2];
-        kv_quantise_8(x, d, w);
-        q8[(h * 8 + blk) * 8 + 2 * sub] = w[0];
-        q8[(h * 8 + blk) * 8 + 2 * sub + 1] = w[1];
-        if (sub == 0) qd[h * 8 + blk] = __fmul_rn(f16_bits_to_f32(f32_to_f16_bits_ties_away(d)), scale);
+        for (int r = 0; r < ROUNDS; ++r) {          // every load first: one trip to memory
+            const int h = warp + r * KV_WARPS;
+            const float *qr = q + (size_t)(kvh * GRP + (h < GRP ? h : 0)) * KV_D + blk * 32 + sub * 8;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[r][i] = qr[i];
+        }
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) {
+            const int h = warp + r * KV_WARPS;
+            float d;
+            uint32_t w[2];
+            kv_quantise_8(x[r], d, w);
+            if (h < GRP) {
+                q8[(h * 8 + blk) * 8 + 2 * sub] = w[0];
+                q8[(h * 8 + blk) * 8 + 2 * sub + 1] = w[1];
+                if (sub == 0) qd[h * 8 + blk] = __fmul_rn(f16_bits_to_f32(f32_to_f16_bits_ties_away(d)), scale);
+            }
+        }
     }
     __syncthreads();
     // B operand of the scores: head g, words t and t + 4 of every block, in the order the K rows are read in
@@ -403,11 +420,21 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *__r
         }
         if (warp == 0 && t == 0) sm[g] = m_run, sl[g] = l_run;
     }
-    cluster_sync();
+    cluster_arrive();
+    cluster_wait();
     // ---- one slice of the dims per CTA of the cluster, added over its CTAs in rank order
     const uint32_t rank = cluster_rank();
     const int n_cl = gridDim.x / KV_CLUSTER, cl = blockIdx.x / KV_CLUSTER;
     float *cw = wt, *cm = mw, *cl_sum = lw;                            // [8 heads][8 ranks] weights; maxima; denominators
+    constexpr int OUTS = GRP * KV_SLICE, ROUNDS = (OUTS + KV_THREADS - 1) / KV_THREADS;
+    float part[ROUNDS][KV_CLUSTER];
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+        const int o = tid + r * KV_THREADS;
+#pragma unroll
+        for (int rr = 0; rr < KV_CLUSTER; ++rr)
+            part[r][rr] = o < OUTS ? ld_cluster_f32(so + (o / KV_SLICE) * KV_D + (int)rank * KV_SLICE + o % KV_SLICE, (uint32_t)rr) : 0.0f;
+    }
     if (warp < 2) {
         const int h = tid >> 3, rr = tid & 7;
         const float mm = h < GRP ? ld_cluster_f32(sm + h, (uint32_t)rr) : -INFINITY;
@@ -423,56 +450,80 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *__r
         if (rr == 0) cm[h] = mx, cl_sum[h] = den;
     }
     __syncthreads();
+    cluster_arrive();                   // this CTA has read its share of the others' memory (it leaves when all have: cluster_wait)
     float *rec = ws + (((size_t)kvh * KV_CLUSTER + rank) * n_cl + cl) * KV_REC;
-    for (int o = tid; o < GRP * KV_SLICE; o += KV_THREADS) {
-        const int h = o / KV_SLICE, d = o % KV_SLICE;
-        float a = 0.0f;
+    float *out_slice = out + (size_t)kvh * GRP * KV_D + (int)rank * KV_SLICE;
 #pragma unroll
-        for (int rr = 0; rr < KV_CLUSTER; ++rr)
-            a = __fmaf_rn(ld_cluster_f32(so + h * KV_D + (int)rank * KV_SLICE + d, (uint32_t)rr), cw[h * 8 + rr], a);
-        if (n_cl == 1) out[((size_t)kvh * GRP + h) * KV_D + (int)rank * KV_SLICE + d] = __fmul_rn(a, __fdiv_rn(1.0f, cl_sum[h]));
-        else rec[o] = a;
-    }
-    cluster_sync();                     // nobody leaves while its shared memory is read
-    if (n_cl == 1) return;
-    // ---- several clusters per head: the last one to bring this slice adds them in order (fixed, whichever is last)
-    if (tid < GRP) {
-        rec[KV_MAX_GROUP * KV_SLICE + tid] = cm[tid];
-        rec[KV_MAX_GROUP * KV_SLICE + KV_MAX_GROUP + tid] = cl_sum[tid];
-    }
-    __threadfence();
-    __syncthreads();
-    unsigned int *counter = counters + kvh * KV_CLUSTER + rank;
-    int last = 0;
-    if (tid == 0) last = atomicAdd(counter, 1u) == (unsigned int)n_cl - 1u;
-    if (!__syncthreads_or(last)) return;
-    __threadfence();
-    const float *all = ws + ((size_t)kvh * KV_CLUSTER + rank) * n_cl * KV_REC;
-    for (int h = warp; h < GRP; h += KV_WARPS) {
-        const float *ml = all + KV_MAX_GROUP * KV_SLICE + h;
-        float mx = -INFINITY, den = 0.0f;
-        for (int c = lane; c < n_cl; c += 32) mx = fmaxf(mx, __ldcg(ml + (size_t)c * KV_REC));
+    for (int r = 0; r < ROUNDS; ++r) {
+        const int o = tid + r * KV_THREADS;
+        if (o < OUTS) {
+            const int h = o / KV_SLICE;
+            float a = 0.0f;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        for (int c = lane; c < n_cl; c += 32) {
-            const float mm = __ldcg(ml + (size_t)c * KV_REC);
-            const float w = mm == -INFINITY ? 0.0f : expf(__fsub_rn(mm, mx));
-            wt[c * KV_MAX_GROUP + h] = w;
-            den = __fmaf_rn(__ldcg(ml + (size_t)c * KV_REC + KV_MAX_GROUP), w, den);
+            for (int rr = 0; rr < KV_CLUSTER; ++rr) a = __fmaf_rn(part[r][rr], cw[h * 8 + rr], a);
+            if (n_cl == 1) out_slice[h * KV_D + o % KV_SLICE] = __fmul_rn(a, __fdiv_rn(1.0f, cl_sum[h]));
+            else rec[o] = a;
         }
+    }
+    int last = 0;
+    if (n_cl > 1) {
+        if (tid < GRP) {
+            rec[KV_MAX_GROUP * KV_SLICE + tid] = cm[tid];
+            rec[KV_MAX_GROUP * KV_SLICE + KV_MAX_GROUP + tid] = cl_sum[tid];
+        }
+        __syncthreads();
+        if (tid == 0) last = count_arrival(counters + kvh * KV_CLUSTER + rank) == (unsigned int)n_cl - 1u;
+        last = __syncthreads_or(last);
+    }
+    if (!last) {
+        cluster_wait();
+        return;
+    }
+    // ---- several clusters per head: the last one to bring this slice adds them in order (fixed, whichever is last).  All
+    // loads go out before the weights are formed: one trip to L2 (a dependent trip per step took 5 us).
+    if (tid == 0) counters[kvh * KV_CLUSTER + rank] = 0u;
+    const float *all = ws + ((size_t)kvh * KV_CLUSTER + rank) * n_cl * KV_REC;
+    constexpr int BATCH = 16, PAIRS = OUTS / 2;
+    static_assert(PAIRS <= KV_THREADS, "a thread adds one pair of outputs");
+    const int ho = min(tid, PAIRS - 1) / (KV_SLICE / 2);
+    float2 v[BATCH];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) den = __fadd_rn(den, __shfl_xor_sync(0xffffffffu, den, o));
-        if (lane == 0) qd[h] = __fdiv_rn(1.0f, den);
+    for (int c = 0; c < BATCH; ++c)
+        v[c] = (tid < PAIRS && c < n_cl) ? __ldcg(reinterpret_cast<const float2 *>(all + (size_t)c * KV_REC) + tid) : make_float2(0.0f, 0.0f);
+    float *fm = reinterpret_cast<float *>(raw + 16384), *fl = fm + KV_MAX_CLUSTERS * KV_MAX_GROUP, *fw = fl + KV_MAX_CLUSTERS * KV_MAX_GROUP;
+    for (int i = tid; i < n_cl * KV_MAX_GROUP; i += KV_THREADS) {
+        const float *ml = all + (size_t)(i / KV_MAX_GROUP) * KV_REC + KV_MAX_GROUP * KV_SLICE + i % KV_MAX_GROUP;
+        const bool use = i % KV_MAX_GROUP < GRP;
+        fm[i] = use ? __ldcg(ml) : 0.0f;
+        fl[i] = use ? __ldcg(ml + KV_MAX_GROUP) : 0.0f;
     }
     __syncthreads();
-    for (int o = tid; o < GRP * KV_SLICE; o += KV_THREADS) {
-        const int h = o / KV_SLICE, d = o % KV_SLICE;
-        float a = 0.0f;
-#pragma unroll 8
-        for (int c = 0; c < n_cl; ++c) a = __fmaf_rn(__ldcg(all + (size_t)c * KV_REC + o), wt[c * KV_MAX_GROUP + h], a);
-        out[((size_t)kvh * GRP + h) * KV_D + (int)rank * KV_SLICE + d] = __fmul_rn(a, qd[h]);
+    for (int i = tid; i < n_cl * KV_MAX_GROUP; i += KV_THREADS) {
+        float mx = -INFINITY;
+        for (int c = 0; c < n_cl; ++c) mx = fmaxf(mx, fm[c * KV_MAX_GROUP + i % KV_MAX_GROUP]);
+        fw[i] = fm[i] == -INFINITY ? 0.0f : expf(__fsub_rn(fm[i], mx));
     }
-    if (tid == 0) *counter = 0u;
+    __syncthreads();
+    if (tid < PAIRS) {
+        float den = 0.0f, a = 0.0f, b = 0.0f;
+        for (int c = 0; c < n_cl; ++c) den = __fmaf_rn(fl[c * KV_MAX_GROUP + ho], fw[c * KV_MAX_GROUP + ho], den);
+#pragma unroll
+        for (int c = 0; c < BATCH; ++c) {
+            const float w = c < n_cl ? fw[c * KV_MAX_GROUP + ho] : 0.0f;
+            a = __fmaf_rn(v[c].x, w, a);
+            b = __fmaf_rn(v[c].y, w, b);
+        }
+        for (int c = BATCH; c < n_cl; ++c) {
+            const float2 x = __ldcg(reinterpret_cast<const float2 *>(all + (size_t)c * KV_REC) + tid);
+            a = __fmaf_rn(x.x, fw[c * KV_MAX_GROUP + ho], a);
+            b = __fmaf_rn(x.y, fw[c * KV_MAX_GROUP + ho], b);
+        }
+        const float inv = __fdiv_rn(1.0f, den);
+        float *o2 = out_slice + ho * KV_D + 2 * (tid % (KV_SLICE / 2));
+        o2[0] = __fmul_rn(a, inv);
+        o2[1] = __fmul_rn(b, inv);
+    }
+    cluster_wait();
 }
 
 }  // namespace b200
