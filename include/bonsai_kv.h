@@ -46,6 +46,8 @@ int bonsai_kv_append_batch(bonsai_kv_cache *kv, int layer, int pos0, int n_tok, 
                            bonsai_stream stream);
 
 /* Attention of one query position over positions 0..pos of `layer`: q, out are [24][256] floats; scale 1/sqrt(256).
+ * The workspace is the layer's: calls for different layers of a cache may run at once on different streams, calls for one
+ * layer follow each other.
  * Replaces include/bonsai_kv.h:52-53 / src/kernels/kv_p40.cu:341-367. */
 int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *q, float *out, bonsai_stream stream);
 

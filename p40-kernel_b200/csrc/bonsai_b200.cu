@@ -22,6 +22,7 @@
 #include "repack.cuh"
 #include "synth.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <mutex>
@@ -1410,13 +1411,40 @@ constexpr int KV_SPLIT_MIN = 2 * KV_TILE;      // positions
 constexpr int KVM_GROUP = KVM_HEADS / KVM_KV_HEADS;
 inline int64_t kv_array_bytes(int capacity) { return (int64_t)KVM_FULL * KVM_KV_HEADS * capacity * KV_ROW; }
 inline int64_t kv_gdn_bytes() { return (int64_t)KVM_LINEAR * KVM_V_HEADS * KVM_STATE * KVM_STATE * (int64_t)sizeof(float); }
+constexpr int KV_COUNTERS = KVM_KV_HEADS * KV_CLUSTER;      // per layer
+inline size_t kv_ws_floats(int max_clusters) { return (size_t)KVM_KV_HEADS * KV_CLUSTER * max_clusters * KV_REC; }      // per layer
+
+// Clusters of the decode kernel per kv head that are resident at once on the current device (0: it does not run here).  The
+// query takes milliseconds, so it is made once per device.
+int kv_max_clusters() {
+    static std::atomic<int> known[64];
+    static SmemOptIn opt;
+    int dev = 0, resident = 0;
+    if (opt.ensure(kv_attn_kernel<KVM_GROUP>) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev < 64 && (resident = known[dev].load(std::memory_order_relaxed)) > 0) return resident;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(KV_CLUSTER * KV_MAX_CLUSTERS, KVM_KV_HEADS);
+    cfg.blockDim = dim3(KV_THREADS);
+    cfg.dynamicSmemBytes = KV_SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = KV_CLUSTER;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&resident, kv_attn_kernel<KVM_GROUP>, &cfg) != cudaSuccess || resident <= 0) return 0;
+    resident = std::min(std::max(resident / KVM_KV_HEADS, 1), KV_MAX_CLUSTERS);
+    if (dev < 64) known[dev].store(resident, std::memory_order_relaxed);
+    return resident;
+}
 }  // namespace
 
 struct bonsai_kv_cache {
     int capacity = 0;
     uint8_t *d_k = nullptr, *d_v = nullptr;
     float *d_gdn = nullptr, *d_ws = nullptr;
-    unsigned int *d_counters = nullptr;         // behind the workspace's records
+    unsigned int *d_counters = nullptr;         // behind the workspace's records; records and counters are a layer's own, so
+                                                // that layers may be decoded on different streams at once
     int max_clusters = 1;                       // clusters of the decode kernel per kv head that are resident at once
 };
 
@@ -1433,33 +1461,20 @@ bonsai_kv_cache *bonsai_kv_create(int capacity, bonsai_stream stream) {
     bonsai_kv_cache *kv = new (std::nothrow) bonsai_kv_cache;
     if (!kv) return nullptr;
     kv->capacity = capacity;
-    const size_t ws = (size_t)KVM_KV_HEADS * KV_CLUSTER * KV_MAX_CLUSTERS * KV_REC * sizeof(float), ncnt = (size_t)KVM_KV_HEADS * KV_CLUSTER * sizeof(unsigned int);
-    if (cudaMalloc(&kv->d_k, (size_t)kv_array_bytes(capacity)) != cudaSuccess || cudaMalloc(&kv->d_v, (size_t)kv_array_bytes(capacity)) != cudaSuccess ||
-        cudaMalloc(&kv->d_gdn, (size_t)kv_gdn_bytes()) != cudaSuccess || cudaMalloc(&kv->d_ws, ws + ncnt) != cudaSuccess ||
-        cudaFuncSetAttribute(kv_attn_kernel<KVM_GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM_BYTES) != cudaSuccess) {
+    kv->max_clusters = kv_max_clusters();
+    const size_t ws = (size_t)KVM_FULL * kv_ws_floats(kv->max_clusters) * sizeof(float), ncnt = (size_t)KVM_FULL * KV_COUNTERS * sizeof(unsigned int);
+    if (kv->max_clusters <= 0 || cudaMalloc(&kv->d_k, (size_t)kv_array_bytes(capacity)) != cudaSuccess ||
+        cudaMalloc(&kv->d_v, (size_t)kv_array_bytes(capacity)) != cudaSuccess || cudaMalloc(&kv->d_gdn, (size_t)kv_gdn_bytes()) != cudaSuccess ||
+        cudaMalloc(&kv->d_ws, ws + ncnt) != cudaSuccess) {
         bonsai_kv_free(kv);
         return nullptr;
     }
     kv->d_counters = reinterpret_cast<unsigned int *>(reinterpret_cast<char *>(kv->d_ws) + ws);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(KV_CLUSTER * KV_MAX_CLUSTERS, KVM_KV_HEADS);
-    cfg.blockDim = dim3(KV_THREADS);
-    cfg.dynamicSmemBytes = KV_SMEM_BYTES;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = KV_CLUSTER;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int resident = 0;
     // the counters are zero before the first launch on any stream: the wait is paid once per cache
-    if (cudaOccupancyMaxActiveClusters(&resident, kv_attn_kernel<KVM_GROUP>, &cfg) != cudaSuccess || resident <= 0 ||
-        cudaMemsetAsync(kv->d_counters, 0, ncnt, as_stream(stream)) != cudaSuccess || cudaStreamSynchronize(as_stream(stream)) != cudaSuccess) {
+    if (cudaMemsetAsync(kv->d_counters, 0, ncnt, as_stream(stream)) != cudaSuccess || cudaStreamSynchronize(as_stream(stream)) != cudaSuccess) {
         bonsai_kv_free(kv);
         return nullptr;
     }
-    kv->max_clusters = resident / KVM_KV_HEADS > 0 ? resident / KVM_KV_HEADS : 1;
-    if (kv->max_clusters > KV_MAX_CLUSTERS) kv->max_clusters = KV_MAX_CLUSTERS;
     (void)cudaMemsetAsync(kv->d_gdn, 0, (size_t)kv_gdn_bytes(), as_stream(stream));
     return kv;
 }
@@ -1524,7 +1539,8 @@ int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return (int)cudaLaunchKernelEx(&cfg, kv_attn_kernel<KVM_GROUP>, q, (const uint8_t *)kv->d_k, (const uint8_t *)kv->d_v, kv->d_ws, kv->d_counters, out,
+    return (int)cudaLaunchKernelEx(&cfg, kv_attn_kernel<KVM_GROUP>, q, (const uint8_t *)kv->d_k, (const uint8_t *)kv->d_v,
+                                   kv->d_ws + (size_t)layer * kv_ws_floats(kv->max_clusters), kv->d_counters + layer * KV_COUNTERS, out,
                                    pos, chunk, KVM_KV_HEADS, kv->capacity, layer, 0.0625f);
 }
 

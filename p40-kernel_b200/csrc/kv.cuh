@@ -44,8 +44,8 @@ __device__ __forceinline__ void kv_quantise_8(const float (&x)[8], float &d_out,
 
 // One warp per (token, kv head) row of K and of V: lane = (block lane / 4, eight dims).
 template <bool VEC>
-__global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *__restrict__ K, uint8_t *__restrict__ V,
-                                                        const float *__restrict__ ksrc, const float *__restrict__ vsrc,
+__global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *K, uint8_t *V,
+                                                        const float *ksrc, const float *vsrc,
                                                         int pos0, int n_tok, int n_kv_head, int capacity, int layer) {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);        // token * n_kv_head + head
@@ -160,9 +160,7 @@ __device__ __forceinline__ float ld_cluster_f32(const float *p, uint32_t rank) {
 // s * chunk .. min((s + 1) * chunk, pos + 1) - 1 (a split may be empty).  counters: one per (kv head, slice), zero before
 // and after every launch.
 template <int GRP>
-__global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *__restrict__ q, const uint8_t *__restrict__ K,
-                                                                const uint8_t *__restrict__ V, float *__restrict__ ws,
-                                                                unsigned int *__restrict__ counters, float *__restrict__ out,
+__global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, const uint8_t *K, const uint8_t *V, float *ws, unsigned int *counters, float *out,
                                                                 int pos, int chunk, int n_kv_head, int capacity, int layer, float scale) {
     static_assert(GRP <= KV_MAX_GROUP, "");
     extern __shared__ __align__(128) uint8_t smem[];

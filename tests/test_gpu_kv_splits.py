@@ -1,0 +1,110 @@
+"""Decode attention over the K/V cache at the positions where its splits change: the first and last position of a tile, of a
+warp's share of one, one cluster against several, more clusters than are resident; and what the launches share.
+
+Against float64 on the cache's own bytes (quantised query x cache, softmax, value sum).  Bound: 2e-6 of the largest output:
+scores are exact integers with fp32 scales, weights carry 22 bits, sums are fp32."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+N_LAYERS, N_KV, N_HEADS, D = 16, 4, 24, 256
+REL_TOL = 2e-6
+
+
+def cache_tensors(kv):
+    import torch
+
+    class Raw:
+        def __init__(self, ptr, n):
+            self.__cuda_array_interface__ = {"shape": (n,), "typestr": "|u1", "data": (int(ptr), False), "version": 3}
+    kp, vp, n = kv.arrays()
+    return [torch.as_tensor(Raw(p, n), device="cuda") for p in (kp, vp)]
+
+
+def dequantise(raw, cap, layer, kvh, n):
+    import torch
+    at = (layer * N_KV + kvh) * cap * 272
+    b = raw[at:at + n * 272].view(n, 8, 34)
+    d = b[:, :, :2].contiguous().view(torch.float16).double()
+    return (d * b[:, :, 2:].contiguous().view(torch.int8).double()).view(n, D)
+
+
+def exact(port, kv, cap, layer, n, q):
+    import torch
+    K, V = cache_tensors(kv)
+    qd = np.stack([port.kv_dequantize_row(port.kv_quantize_row(row)) for row in q.cpu().numpy()])
+    qd = torch.from_numpy(qd).cuda().double()
+    out = torch.empty(N_HEADS, D, dtype=torch.float64, device="cuda")
+    for h in range(N_HEADS):
+        s = dequantise(K, cap, layer, h // 6, n) @ qd[h] * 0.0625
+        out[h] = torch.softmax(s, 0) @ dequantise(V, cap, layer, h // 6, n)
+    return out
+
+
+def fill(kv, layer, n, seed, spread):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    k, v = torch.randn(n, N_KV, D, generator=g, device="cuda"), torch.randn(n, N_KV, D, generator=g, device="cuda")
+    if spread:                      # rows of V of very different size
+        v = v * torch.exp(2 * torch.randn(n, N_KV, 1, generator=g, device="cuda"))
+    assert kv.append_batch(layer, 0, n, k, v) == 0
+    return torch.randn(N_HEADS, D, generator=g, device="cuda")
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 63, 64, 65, 127, 128, 129, 1023, 1024, 1025, 2047, 2048, 2049, 4100, 13311, 13312, 14337, 40001])
+@pytest.mark.parametrize("spread", [0, 1])
+def test_against_float64(gpu, port, n, spread):
+    import torch
+    cap, layer = n + 3, 5
+    kv = gpu.KVCache(cap)
+    q = fill(kv, layer, n, n, spread)
+    out = torch.full((N_HEADS, D), float("nan"), device="cuda")
+    for _ in range(2):              # the second call finds the counters as the first one left them
+        assert kv.attn_decode(layer, n - 1, q, out) == 0
+    want = exact(port, kv, cap, layer, n, q)
+    err, top = float((out.double() - want).abs().max()), float(want.abs().max())
+    assert err <= REL_TOL * top, (err, top)
+    assert gpu.device_status() == 0
+    kv.close()
+
+
+def test_layers_on_streams_of_their_own(gpu):
+    """Layers have their own records and counters: decoded at the same time on different streams they give the bits that
+    they give one after the other."""
+    import torch
+    n = 9000
+    kv = gpu.KVCache(n)
+    qs = [fill(kv, layer, n, layer, 0) for layer in range(4)]
+    want = [torch.empty(N_HEADS, D, device="cuda") for _ in range(4)]
+    for layer in range(4):
+        assert kv.attn_decode(layer, n - 1, qs[layer], want[layer]) == 0
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    got = [torch.empty(N_HEADS, D, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for layer, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                assert kv.attn_decode(layer, n - 1, qs[layer], got[layer]) == 0
+    torch.cuda.synchronize()
+    for layer in range(4):
+        assert torch.equal(got[layer], want[layer]), layer
+    kv.close()
+
+
+def test_append_at_odd_offsets(gpu):
+    """Rows at any float address store the bytes of rows at an aligned one."""
+    import torch
+    kv, cap = gpu.KVCache(40), 40
+    g = torch.Generator(device="cuda").manual_seed(1)
+    k, v = torch.randn(37, N_KV, D, generator=g, device="cuda"), torch.randn(37, N_KV, D, generator=g, device="cuda")
+    odd = [torch.empty(t.numel() + 1, device="cuda") for t in (k, v)]
+    for o, t in zip(odd, (k, v)):
+        o[1:].copy_(t.view(-1))
+    assert kv.append_batch(2, 3, 37, k, v) == 0 and kv.append_batch(3, 3, 37, odd[0][1:], odd[1][1:]) == 0
+    for raw in cache_tensors(kv):
+        for h in range(N_KV):
+            a, b = ((layer * N_KV + h) * cap * 272 + 3 * 272 for layer in (2, 3))
+            assert torch.equal(raw[a:a + 37 * 272], raw[b:b + 37 * 272]), h
+    kv.close()
