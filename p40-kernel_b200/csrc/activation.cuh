@@ -68,10 +68,10 @@ __device__ __forceinline__ void store_f4(float *p, float4 v) {
 // One thread per four inputs.  X is [n_tok][n_in]; output block index = chunk * tok_stride + tok
 // (tok_stride = 1 with n_tok = 1 gives the plain vector layout).
 template <bool VEC>
-__global__ void __launch_bounds__(256) quant_q8_1_kernel(const float *__restrict__ X, uint32_t *__restrict__ out,
+__global__ void __launch_bounds__(256) quant_q8_1_kernel(const float *X, uint32_t *__restrict__ out,
                                                          int n_in, int n_tok) {
-    pdl_launch_dependents();
     pdl_wait_prior_grid();
+    pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
     const int per_tok = n_in >> 2;
     const long long total = (long long)per_tok * n_tok;
@@ -191,10 +191,10 @@ __device__ __forceinline__ void fwht_slice_back(const float4 *block, int r, int 
 // blocks = n_tok * (n_in / 1024) warps.  X [n_tok][n_in] read-only; x_rot (nullable, may alias X)
 // receives the rotated values; xq (nullable) the Q8_1 blocks at chunk * n_tok + tok.
 template <bool VEC>
-__global__ void __launch_bounds__(128) fwht_quant_kernel(const float *X, const float *__restrict__ signs, float *x_rot,
+__global__ void __launch_bounds__(128) fwht_quant_kernel(const float *X, const float *signs, float *x_rot,
                                                          uint32_t *__restrict__ xq, int n_in, int n_tok) {
-    pdl_launch_dependents();
     pdl_wait_prior_grid();
+    pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
     const int blocks_per_tok = n_in / FWHT_N;
     const long long nwarps = (long long)blocks_per_tok * n_tok;

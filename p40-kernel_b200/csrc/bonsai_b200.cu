@@ -379,6 +379,13 @@ GemvPlan plan_rows(long long n_out, size_t row_bytes, size_t fixed, int granule,
     return p;
 }
 
+// Any float pointers are taken, as by the reference; 16-byte aligned ones get 16-byte accesses.
+int launch_fwht(bool vec, const float *x, const float *signs, float *x_rot, void *xq, int64_t n_in, int64_t n_tok, bonsai_stream stream) {
+    const long long warps = (n_in / FWHT_N) * n_tok;
+    return (int)launch(vec ? fwht_quant_kernel<true> : fwht_quant_kernel<false>, dim3((unsigned)((warps + 3) / 4)), dim3(128), 0, as_stream(stream), true,
+                       x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
+}
+
 }  // namespace
 
 extern "C" {
@@ -389,34 +396,21 @@ int bonsai_p40_quant_activations(const float *x, void *out, int64_t n, bonsai_st
     const long long threads = n / 4;
     const int blocks = (int)((threads + 255) / 256);
     // any float pointer is taken, as by the reference; 16-byte aligned ones get 16-byte loads
-    if (aligned16(x)) quant_q8_1_kernel<true><<<blocks, 256, 0, as_stream(stream)>>>(x, static_cast<uint32_t *>(out), (int)n, 1);
-    else quant_q8_1_kernel<false><<<blocks, 256, 0, as_stream(stream)>>>(x, static_cast<uint32_t *>(out), (int)n, 1);
-    return (int)cudaGetLastError();
+    return (int)launch(aligned16(x) ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, x,
+                       static_cast<uint32_t *>(out), (int)n, 1);
 }
 
 int bonsai_p40_fwht(float *x, const float *signs, int64_t n, bonsai_stream stream) {
     if (n <= 0 || n % FWHT_N != 0) return 1;
     if (!aligned4(x) || (signs && !aligned4(signs)) || n > INT32_MAX) return 1;
-    const int warps = (int)(n / FWHT_N);
-    if (aligned16(x) && (!signs || aligned16(signs)))
-        fwht_quant_kernel<true><<<(warps + 3) / 4, 128, 0, as_stream(stream)>>>(x, signs, x, nullptr, (int)n, 1);
-    else
-        fwht_quant_kernel<false><<<(warps + 3) / 4, 128, 0, as_stream(stream)>>>(x, signs, x, nullptr, (int)n, 1);
-    return (int)cudaGetLastError();
+    return launch_fwht(aligned16(x) && (!signs || aligned16(signs)), x, signs, x, nullptr, n, 1, stream);
 }
 
 int bonsai_b200_fwht_quant(const float *x, const float *signs, void *xq, float *x_rot, int64_t n,
                            bonsai_stream stream) {
     if (n <= 0 || n % FWHT_N != 0 || n > INT32_MAX) return 1;
     if (!aligned4(x) || (signs && !aligned4(signs)) || (x_rot && !aligned4(x_rot)) || !aligned4(xq)) return 1;
-    const int warps = (int)(n / FWHT_N);
-    if (aligned16(x) && (!signs || aligned16(signs)) && (!x_rot || aligned16(x_rot)))
-        fwht_quant_kernel<true><<<(warps + 3) / 4, 128, 0, as_stream(stream)>>>(x, signs, x_rot, static_cast<uint32_t *>(xq),
-                                                                                (int)n, 1);
-    else
-        fwht_quant_kernel<false><<<(warps + 3) / 4, 128, 0, as_stream(stream)>>>(x, signs, x_rot, static_cast<uint32_t *>(xq),
-                                                                                 (int)n, 1);
-    return (int)cudaGetLastError();
+    return launch_fwht(aligned16(x) && (!signs || aligned16(signs)) && (!x_rot || aligned16(x_rot)), x, signs, x_rot, xq, n, 1, stream);
 }
 
 int bonsai_b200_quant_batch(const float *X, const float *signs, void *Xq, int64_t n_in, int64_t n_tok, int rotate,
@@ -427,21 +421,18 @@ int bonsai_b200_quant_batch(const float *X, const float *signs, void *Xq, int64_
     if (n_in > INT32_MAX || n_tok > INT32_MAX) return 1;
     const bool vec = aligned16(X) && (!signs || aligned16(signs));
     if (rotate) {
-        const long long warps = (n_in / FWHT_N) * n_tok;
-        const unsigned blocks = (unsigned)((warps + 3) / 4);
-        if (vec) fwht_quant_kernel<true><<<blocks, 128, 0, as_stream(stream)>>>(X, signs, nullptr, static_cast<uint32_t *>(Xq), (int)n_in, (int)n_tok);
-        else fwht_quant_kernel<false><<<blocks, 128, 0, as_stream(stream)>>>(X, signs, nullptr, static_cast<uint32_t *>(Xq), (int)n_in, (int)n_tok);
-    } else {
-        const long long threads = n_in / 4 * n_tok;
-        long long blocks = (threads + 255) / 256;
-        if (blocks > 8 * SM_COUNT * 4) blocks = 8 * SM_COUNT * 4;
-        if (vec) quant_q8_1_kernel<true><<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(X, static_cast<uint32_t *>(Xq), (int)n_in, (int)n_tok);
-        else quant_q8_1_kernel<false><<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(X, static_cast<uint32_t *>(Xq), (int)n_in, (int)n_tok);
+        return launch_fwht(vec, X, signs, nullptr, Xq, n_in, n_tok, stream);
     }
-    return (int)cudaGetLastError();
+    const long long threads = n_in / 4 * n_tok;
+    long long blocks = (threads + 255) / 256;
+    if (blocks > 8 * SM_COUNT * 4) blocks = 8 * SM_COUNT * 4;
+    return (int)launch(vec ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, X,
+                       static_cast<uint32_t *>(Xq), (int)n_in, (int)n_tok);
 }
 
-int bonsai_p40_gemv(const void *W, const void *xq, float *y, int64_t n_out, int64_t n_in, bonsai_stream stream) {
+// behind_quantiser: the launch before this one on the stream is this library's quantiser, so nothing that is still running
+// writes the weights and the first tiles are copied before the wait for it.
+static int gemv_launch(const void *W, const void *xq, float *y, int64_t n_out, int64_t n_in, bonsai_stream stream, bool behind_quantiser) {
     if (n_in <= 0 || n_in % 128 != 0) return 1;
     if (n_out <= 0) return 0;
     if (n_out > INT32_MAX || n_in / 128 > INT32_MAX / 64) return 1;
@@ -468,8 +459,9 @@ int bonsai_p40_gemv(const void *W, const void *xq, float *y, int64_t n_out, int6
             static SmemOptIn opt;
             cudaError_t err = opt.ensure(gemv_stream_kernel<false>);
             if (err != cudaSuccess) return (int)err;
+            sp.early = pdl || behind_quantiser;
             return (int)launch(gemv_stream_kernel<false>, dim3((unsigned)((n_out + sp.rows_per_cta - 1) / sp.rows_per_cta)),
-                               dim3(threads), (size_t)smem_bytes, as_stream(stream), pdl,
+                               dim3(threads), (size_t)smem_bytes, as_stream(stream), true,
                                static_cast<const uint8_t *>(W), static_cast<const uint32_t *>(xq), y, sp,
                                static_cast<const float *>(nullptr), static_cast<const float *>(nullptr),
                                static_cast<uint32_t *>(nullptr));
@@ -499,6 +491,10 @@ int bonsai_p40_gemv(const void *W, const void *xq, float *y, int64_t n_out, int6
     return (int)e;
 }
 
+int bonsai_p40_gemv(const void *W, const void *xq, float *y, int64_t n_out, int64_t n_in, bonsai_stream stream) {
+    return gemv_launch(W, xq, y, n_out, n_in, stream, false);
+}
+
 int bonsai_b200_linear(const void *W, const float *x, const float *signs, float *y, void *xq_scratch, int64_t n_out,
                        int64_t n_in, bonsai_stream stream) {
     if (n_out <= 0 || n_in <= 0 || n_in % FWHT_N != 0 || !xq_scratch) return 1;
@@ -512,14 +508,15 @@ int bonsai_b200_linear(const void *W, const float *x, const float *signs, float 
         static SmemOptIn opt;
         cudaError_t err = opt.ensure(gemv_stream_kernel<true>);
         if (err != cudaSuccess) return (int)err;
+        sp.early = g_opt_pdl.load() != 0;
         return (int)launch(gemv_stream_kernel<true>, dim3((unsigned)((n_out + sp.rows_per_cta - 1) / sp.rows_per_cta)),
-                           dim3(threads), (size_t)smem_bytes, as_stream(stream), g_opt_pdl.load() != 0,
+                           dim3(threads), (size_t)smem_bytes, as_stream(stream), true,
                            static_cast<const uint8_t *>(W), static_cast<const uint32_t *>(nullptr), y, sp, x, signs,
                            static_cast<uint32_t *>(xq_scratch));
     }
     const int rc = bonsai_b200_fwht_quant(x, signs, xq_scratch, nullptr, n_in, stream);
     if (rc != 0) return rc;
-    return bonsai_p40_gemv(W, xq_scratch, y, n_out, n_in, stream);
+    return gemv_launch(W, xq_scratch, y, n_out, n_in, stream, true);
 }
 
 // ---- projection without any allocation: the Q8_1 scratch is part of the library image -----------
@@ -546,7 +543,7 @@ int bonsai_b200_linear_static(const void *W, const float *x, const float *signs,
     }
     const int rc = bonsai_b200_fwht_quant(x, signs, scratch, nullptr, n_in, stream);
     if (rc != 0) return rc;
-    return bonsai_p40_gemv(W, scratch, y, n_out, n_in, stream);
+    return gemv_launch(W, scratch, y, n_out, n_in, stream, true);
 }
 
 
@@ -1090,11 +1087,11 @@ static int launch_gemm_small(const void *W, const void *Xq, float *Y, int64_t n_
                                    (uint64_t)nb * W_BLOCK_BYTES, (uint32_t)(mp.stride / 4), 16u, CU_TENSOR_MAP_SWIZZLE_NONE))
         return -1;
     static SmemOptIn opt, opt2, opt_dump;
-    const bool pdl = g_opt_pdl.load() != 0;
+    mp.early = g_opt_pdl.load() != 0;
     if (mp.ntg == 2) {
         cudaError_t err = opt2.ensure(gemm_mma_kernel<false, 2, 1>);
         if (err != cudaSuccess) return (int)err;
-        return (int)launch(gemm_mma_kernel<false, 2, 1>, dim3((unsigned)grid), dim3(MMAB_THREADS), (size_t)smem_bytes, st, pdl,
+        return (int)launch(gemm_mma_kernel<false, 2, 1>, dim3((unsigned)grid), dim3(MMAB_THREADS), (size_t)smem_bytes, st, true,
                            static_cast<const uint8_t *>(W), static_cast<const uint32_t *>(Xq), Y, mp, (int)n_tok, dump, wmap);
     }
     auto go = [&](auto kernel, SmemOptIn &o, bool with_pdl) -> int {
@@ -1105,7 +1102,7 @@ static int launch_gemm_small(const void *W, const void *Xq, float *Y, int64_t n_
     };
     static SmemOptIn opt_r2, opt_dump_r2;
     if (dump) return mp.nrg == 2 ? go(gemm_mma_kernel<true, 1, 2>, opt_dump_r2, false) : go(gemm_mma_kernel<true, 1, 1>, opt_dump, false);
-    return mp.nrg == 2 ? go(gemm_mma_kernel<false, 1, 2>, opt_r2, pdl) : go(gemm_mma_kernel<false, 1, 1>, opt, pdl);
+    return mp.nrg == 2 ? go(gemm_mma_kernel<false, 1, 2>, opt_r2, true) : go(gemm_mma_kernel<false, 1, 1>, opt, true);
 }
 
 int bonsai_p40_gemm(const void *W, const void *Xq, float *Y, int64_t n_out, int64_t n_in, int64_t n_tok,
@@ -1228,8 +1225,9 @@ int bonsai_p40_gemv_repack(const void *W, const float *x, float *y, int64_t n_ou
             static SmemOptIn sopt;
             cudaError_t err = sopt.ensure(gemv_stream_kernel<true, true>);
             if (err != cudaSuccess) return (int)err;
+            sp.early = pdl;
             return (int)launch(gemv_stream_kernel<true, true>, dim3((unsigned)((n_out + sp.rows_per_cta - 1) / sp.rows_per_cta)),
-                               dim3(threads), (size_t)smem_bytes, as_stream(stream), pdl, static_cast<const uint8_t *>(W),
+                               dim3(threads), (size_t)smem_bytes, as_stream(stream), true, static_cast<const uint8_t *>(W),
                                static_cast<const uint32_t *>(nullptr), y, sp, x, static_cast<const float *>(nullptr),
                                static_cast<uint32_t *>(nullptr));
         }
@@ -1365,15 +1363,16 @@ int bonsai_p40_rmsnorm(const float *x, const float *w, float *y, int64_t n_rows,
     // return convention of src/kernels/elementwise_p40.cu:82-88
     if (n <= 0 || n_rows <= 0) return (n <= 0) ? 1 : 0;
     if (n > INT32_MAX || n_rows > INT32_MAX || !aligned4(x) || !aligned4(w) || !aligned4(y)) return 1;
-    if (n % 4 == 0 && aligned16(x)) rmsnorm_kernel<true><<<(unsigned)n_rows, 256, 0, as_stream(stream)>>>(x, w, y, (int)n, eps);
-    else rmsnorm_kernel<false><<<(unsigned)n_rows, 256, 0, as_stream(stream)>>>(x, w, y, (int)n, eps);
-    return (int)cudaGetLastError();
+    return (int)launch(n % 4 == 0 && aligned16(x) && aligned16(w) && aligned16(y) ? rmsnorm_kernel<true> : rmsnorm_kernel<false>, dim3((unsigned)n_rows), dim3(RMS_THREADS), 0, as_stream(stream),
+                       true, x, w, y, (int)n, eps);
 }
 
 int bonsai_b200_swiglu(const float *gate, const float *up, float *y, int64_t n, bonsai_stream stream) {
     if (n <= 0 || n > INT32_MAX || !aligned4(gate) || !aligned4(up) || !aligned4(y)) return 1;
-    swiglu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, as_stream(stream)>>>(gate, up, y, (int)n);
-    return (int)cudaGetLastError();
+    const bool vec = n % 4 == 0 && aligned16(gate) && aligned16(up) && aligned16(y);
+    const int64_t threads = vec ? n / 4 : n;
+    return (int)launch(vec ? swiglu_kernel<true> : swiglu_kernel<false>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, as_stream(stream), true,
+                       gate, up, y, (int)n);
 }
 
 int bonsai_p40_gdn_step(float *state, const float *q, const float *k, const float *v, const float *g, const float *beta,
@@ -1382,8 +1381,8 @@ int bonsai_p40_gdn_step(float *state, const float *q, const float *k, const floa
     if (V <= 0 || V % 32 != 0 || K <= 0 || K > GDN_KMAX) return 1;
     if (n_v_heads <= 0 || n_k_heads <= 0 || n_v_heads % n_k_heads != 0) return 1;
     const int blocks = n_v_heads * (V / 32);
-    gdn_step_kernel<<<blocks, GDN_WARPS * 32, 0, as_stream(stream)>>>(state, q, k, v, g, beta, out, n_k_heads, n_v_heads, K, V);
-    return (int)cudaGetLastError();
+    return (int)launch(gdn_step_kernel, dim3((unsigned)blocks), dim3(GDN_WARPS * 32), 0, as_stream(stream), true, state, q, k, v, g, beta, out, n_k_heads,
+                       n_v_heads, K, V);
 }
 
 int bonsai_p40_attn(const float *q, const float *k, const float *v, float *out, int n_tok, int n_head, int n_head_kv,

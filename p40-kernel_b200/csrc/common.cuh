@@ -180,6 +180,10 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
         ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
         : "memory");
 }
+// Asks L2 for `bytes` (multiple of 16, address 16-byte aligned).
+__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes) {
+    if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ uint64_t policy_evict_first() {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
@@ -196,7 +200,10 @@ __device__ __forceinline__ uint64_t policy_evict_last_or_default() {
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
-// Programmatic dependent launch: both are no-ops unless the launch carries the attribute.
+// Programmatic dependent launch: both are no-ops unless the launches carry the attribute.  Kernels call the wait first:
+// a launch that starts early then has its direct predecessor to wait for and nothing older, which is why a mat-vec behind
+// this library's quantiser may copy weights before its own wait.  What an earlier launch may have written is read through
+// pointers without __restrict__ (a load through one may be moved in front of the wait).
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

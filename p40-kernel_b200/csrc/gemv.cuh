@@ -261,8 +261,8 @@ __global__ void __launch_bounds__(RR == 4 ? 512 : 1024, 1) gemv_ring_kernel(cons
         __syncwarp();
         for (int t = 0; t < min(2, first_fill); ++t) issue_tile(t);
     }
-    pdl_launch_dependents();
     pdl_wait_prior_grid();              // activations (and y) belong to the previous kernel until here
+    pdl_launch_dependents();
     {
         const int nchunks = P.npairs * 8;
         uint32_t v[9];
@@ -348,8 +348,8 @@ __global__ void __launch_bounds__(256) gemv_pq2_generic_kernel(const uint8_t *__
                                                                int n_out, int nblocks) {
     constexpr int SEG = 512;                     // chunks summed per pass
     __shared__ float terms[8][SEG];
-    pdl_launch_dependents();
     pdl_wait_prior_grid();
+    pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int row = blockIdx.x * 8 + warp;
     if (row >= n_out) return;

@@ -216,8 +216,8 @@ __global__ void __launch_bounds__(MMA_THREADS, 1) gemv_mma_kernel(const uint8_t 
     const int first_fill = min(P.nslot, ntiles);
     if (wid == MMA_C)
         for (int T = 0; T < min(2, first_fill); ++T) issue_tile(T);        // weights never depend on the kernel before
-    pdl_launch_dependents();
     pdl_wait_prior_grid();              // activations (and y) belong to the previous kernel until here
+    pdl_launch_dependents();
     {
         const int nchunks = P.nb * 4;
         for (int c0 = 0; c0 < nchunks; c0 += MMA_THREADS) {
@@ -361,6 +361,7 @@ struct MmabGeom {
     int items, ppi;          // items per tile, block pairs per item
     int act_bufs, act_buf_bytes;   // a buffer = the segment's Q8_1 blocks, then {da, 0x4B400000 - s} of every (chunk, token)
     int act_tab_off;               // bytes from a buffer's start to that table
+    int early;                     // 1: two weight tiles may be copied while the previous launch still runs
     int ntg, nrg;                  // token groups of 8, row groups of 16 that share a chunk's operand loads
     uint32_t magic_nslot, magic_bt, magic_items;   // division by nslot, by the tiles of a full batch, by items
 };
@@ -490,17 +491,17 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
         if (P.tiled) asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
     }
     __syncthreads();
-    // The weights do not depend on the launch before this one: two tiles go out at once.  The rest of the first fill
+    // Where the caller says that the launch before this one does not write the weights, two tiles go out at once.  The rest of the first fill
     // goes out after the first step's Q8_1 blocks have been asked for -- copies complete in the order they were issued,
     // and nothing can be multiplied before those blocks are there.
-    const int first_fill = min(P.nslot, ntiles), early = min(2, first_fill);
+    const int first_fill = min(P.nslot, ntiles), early = P.early ? min(2, first_fill) : 0;
     if (wid == MMAB_C) {
         if (lane < early) issue_tile(lane);
         __syncwarp();
         if (lane == 0) issued[0] = early;
     }
-    pdl_launch_dependents();
     pdl_wait_prior_grid();
+    pdl_launch_dependents();
     auto wait_count = [&](volatile int *c, int need) -> bool {
         for (uint32_t n = 0; n < (1u << 22); ++n) {
             if (*c >= need) return true;

@@ -37,6 +37,7 @@ struct StreamParams {
     int nseg;              // segments per row; segment j starts at block j * seg_blocks
     int seg_blocks;        // blocks per segment (<= 8 * STREAM_STEPS), the last one takes the remainder
     int nslot;
+    int early;             // 1: weights may be copied while the previous launch still runs (it does not write them)
     int tpt;               // tasks per tile = (tr / 4) * nseg
     uint32_t magic_tpt, magic_nseg, magic_nslot;   // ceil(2^32 / d), 0 for d == 1
 };
@@ -202,10 +203,10 @@ __device__ __forceinline__ float stream_task_repack(const uint8_t *row, int nb, 
 // REPACK = true (with FUSED) is bonsai_p40_gemv_repack: W is in the repacked layout and x is quantised WITHOUT a
 // rotation (src/kernels/gemv_repack_p40.cu:91-162 fuses exactly that).
 template <bool FUSED, bool REPACK = false>
-__global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__restrict__ W, const uint32_t *__restrict__ xq,
-                                                             float *__restrict__ y, const StreamParams P,
-                                                             const float *__restrict__ x, const float *__restrict__ signs,
-                                                             uint32_t *__restrict__ xq_out) {
+__global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__restrict__ W, const uint32_t *xq,
+                                                             float *y, const StreamParams P,
+                                                             const float *x, const float *signs,
+                                                             uint32_t *xq_out) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
     uint64_t *done = full + RING_MAX_TILES;
@@ -258,12 +259,17 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
         mbar_fence_init();
         __syncwarp();
         if (lane == 0)
-            for (int t = 0; t < min(2, first_fill); ++t) issue_tile(t);
+            for (int t = 0; t < min(2, first_fill); ++t) {
+                // whoever wrote the weights, a request to bring them into L2 is harmless: it holds no copy of them
+                if (P.early) issue_tile(t);
+                else bulk_prefetch_l2(src + (size_t)t * P.tr * row_bytes, (uint32_t)(min(P.tr, rows_here - t * P.tr) * row_bytes) & ~15u);
+            }
     }
     for (int i = threadIdx.x; i < P.rows_per_cta / 4; i += blockDim.x) quad_count[i] = 0;
     if (threadIdx.x == 0) *next_task = 0;
-    pdl_launch_dependents();
     pdl_wait_prior_grid();              // activations (and y) belong to the previous kernel until here
+    pdl_launch_dependents();            // behind the wait: whatever starts now has only this launch to wait for
+    const int first_late = P.early ? min(2, first_fill) : 0;
     if (FUSED) {
         // rotation + quantiser in the prologue: nb / 8 blocks of 1024 activations over the compute warps
         const int nfb = P.nb >> 3;
@@ -283,7 +289,7 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
                 // every warp has issued its first loads: the rest of the ring may queue behind them
                 __syncthreads();
                 if (wid == compute_warps && lane == 0)
-                    for (int t = 2; t < first_fill; ++t) issue_tile(t);
+                    for (int t = first_late; t < first_fill; ++t) issue_tile(t);
                 first = false;
             }
             if (live) {
@@ -319,7 +325,7 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
         const bool mine = (int)threadIdx.x < nchunks;
         if (mine) act_chunk_load(xq, threadIdx.x, v);
         if (wid == compute_warps && lane == 0)
-            for (int t = 2; t < first_fill; ++t) issue_tile(t);
+            for (int t = first_late; t < first_fill; ++t) issue_tile(t);
         for (int chunk = threadIdx.x; chunk < nchunks; chunk += blockDim.x) {
             if (chunk != (int)threadIdx.x) act_chunk_load(xq, chunk, v);
             uint32_t *q = act_q + (chunk >> 2) * STREAM_ACT_WORDS + (chunk & 3) * 8;

@@ -34,36 +34,94 @@ __device__ __forceinline__ float swiglu1(float g, float u) {
     return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), u);
 }
 
-__global__ void __launch_bounds__(256) swiglu_kernel(const float *__restrict__ gate, const float *__restrict__ up,
-                                                     float *__restrict__ y, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = swiglu1(gate[i], up[i]);
+// VEC: four values per thread (n % 4 == 0, 16-byte aligned pointers).
+template <bool VEC>
+__global__ void __launch_bounds__(256) swiglu_kernel(const float *gate, const float *up, float *y, int n) {
+    pdl_wait_prior_grid();
+    pdl_launch_dependents();
+    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (VEC) {
+        if (i < n / 4) {
+            const float4 g = reinterpret_cast<const float4 *>(gate)[i], u = reinterpret_cast<const float4 *>(up)[i];
+            reinterpret_cast<float4 *>(y)[i] = make_float4(swiglu1(g.x, u.x), swiglu1(g.y, u.y), swiglu1(g.z, u.z), swiglu1(g.w, u.w));
+        }
+    } else if (i < n) {
+        y[i] = swiglu1(gate[i], up[i]);
+    }
 }
 
-// One CTA per row, n % 128 == 0 handled by whole slices (VEC: 16-byte loads), any n by the scalar tail path.
+// One CTA per row.  VEC (n % 4 == 0, all pointers 16-byte aligned): 16-byte accesses; otherwise scalar ones, same order of
+// sums.  A row of up to 8 slices per warp (8192 values: the model's width) stays in registers between the sum and the
+// product: bound by latency, it makes one trip to memory instead of two.
+constexpr int RMS_THREADS = 256, RMS_HOLD = 8;
 template <bool VEC>
-__global__ void __launch_bounds__(256) rmsnorm_kernel(const float *__restrict__ x, const float *__restrict__ w,
-                                                      float *__restrict__ y, int n, float eps) {
+__device__ __forceinline__ float4 rms_load(const float *p, int i, int n) {
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (VEC) {
+        if (i + 3 < n) f = *reinterpret_cast<const float4 *>(p + i);
+    } else {
+        if (i < n) f.x = p[i];
+        if (i + 1 < n) f.y = p[i + 1];
+        if (i + 2 < n) f.z = p[i + 2];
+        if (i + 3 < n) f.w = p[i + 3];
+    }
+    return f;
+}
+template <bool VEC>
+__device__ __forceinline__ void rms_store(float *p, int i, int n, float4 f, float sc, float4 w) {
+    f.x = __fmul_rn(__fmul_rn(f.x, sc), w.x);
+    f.y = __fmul_rn(__fmul_rn(f.y, sc), w.y);
+    f.z = __fmul_rn(__fmul_rn(f.z, sc), w.z);
+    f.w = __fmul_rn(__fmul_rn(f.w, sc), w.w);
+    if (VEC) {
+        if (i + 3 < n) *reinterpret_cast<float4 *>(p + i) = f;
+    } else {
+        if (i < n) p[i] = f.x;
+        if (i + 1 < n) p[i + 1] = f.y;
+        if (i + 2 < n) p[i + 2] = f.z;
+        if (i + 3 < n) p[i + 3] = f.w;
+    }
+}
+template <bool VEC>
+__global__ void __launch_bounds__(RMS_THREADS) rmsnorm_kernel(const float *x, const float *w, float *y, int n, float eps) {
+    constexpr int NW = RMS_THREADS / 32;
     __shared__ float part[512];
     __shared__ float scale;
     const float *xr = x + (size_t)blockIdx.x * n;
     float *yr = y + (size_t)blockIdx.x * n;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nslice = (n + 127) >> 7;
-    float acc = 0.0f;                               // rows longer than 512 slices: a warp adds its slices in ascending order
+    pdl_wait_prior_grid();
+    pdl_launch_dependents();
+    if (nslice <= RMS_HOLD * NW) {
+        float4 f[RMS_HOLD], g[RMS_HOLD];
+#pragma unroll
+        for (int r = 0; r < RMS_HOLD; ++r) f[r] = rms_load<VEC>(xr, (wid + NW * r) * 128 + 4 * lane, n);
+#pragma unroll
+        for (int r = 0; r < RMS_HOLD; ++r) g[r] = rms_load<VEC>(w, (wid + NW * r) * 128 + 4 * lane, n);
+#pragma unroll
+        for (int r = 0; r < RMS_HOLD; ++r) {
+            if (wid + NW * r >= nslice) break;              // warp-uniform
+            const float s = slice_sumsq(f[r]);
+            if (lane == 0) part[wid + NW * r] = s;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float acc = 0.0f;
+#pragma unroll 8
+            for (int k = 0; k < nslice; ++k) acc = __fadd_rn(acc, part[k]);
+            scale = rms_scale(acc, n, eps);
+        }
+        __syncthreads();
+        const float sc = scale;
+#pragma unroll
+        for (int r = 0; r < RMS_HOLD; ++r) rms_store<VEC>(yr, (wid + NW * r) * 128 + 4 * lane, n, f[r], sc, g[r]);
+        return;
+    }
+    float acc = 0.0f;                               // rows longer than 512 slices: a part at a time, in ascending order
     for (int s0 = 0; s0 < nslice; s0 += 512) {
-        for (int sl = s0 + wid; sl < min(nslice, s0 + 512); sl += nw) {
-            const int i = sl * 128 + 4 * lane;
-            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (VEC) {
-                if (i + 3 < n) f = *reinterpret_cast<const float4 *>(xr + i);
-            } else {
-                if (i < n) f.x = xr[i];
-                if (i + 1 < n) f.y = xr[i + 1];
-                if (i + 2 < n) f.z = xr[i + 2];
-                if (i + 3 < n) f.w = xr[i + 3];
-            }
-            const float s = slice_sumsq(f);
+        for (int sl = s0 + wid; sl < min(nslice, s0 + 512); sl += NW) {
+            const float s = slice_sumsq(rms_load<VEC>(xr, sl * 128 + 4 * lane, n));
             if (lane == 0) part[sl - s0] = s;
         }
         __syncthreads();
@@ -74,7 +132,16 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float *__restrict__ 
         __syncthreads();
     }
     const float sc = scale;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) yr[i] = __fmul_rn(__fmul_rn(xr[i], sc), w[i]);
+    for (int sl = wid; sl < nslice; sl += 4 * NW) {
+        float4 f[4], g[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            f[r] = rms_load<VEC>(xr, min(sl + NW * r, nslice) * 128 + 4 * lane, n);
+            g[r] = rms_load<VEC>(w, min(sl + NW * r, nslice) * 128 + 4 * lane, n);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) rms_store<VEC>(yr, min(sl + NW * r, nslice) * 128 + 4 * lane, n, f[r], sc, g[r]);
+    }
 }
 
 // ---- gated delta-net step ------------------------------------------------------------------------------------------
@@ -85,10 +152,8 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float *__restrict__ 
 // host's strictly sequential one (src/ops.h:66-92) -- within the 1e-5 this operator is held to.  (A thread per whole
 // column kept 128 values in registers and left 6144 threads for a 3 MB state: 45 us per call against 4 us for this shape.)
 constexpr int GDN_KMAX = 128, GDN_WARPS = 8, GDN_RPW = GDN_KMAX / GDN_WARPS;
-__global__ void __launch_bounds__(GDN_WARPS * 32) gdn_step_kernel(float *__restrict__ state, const float *__restrict__ q,
-                                                                  const float *__restrict__ k, const float *__restrict__ v,
-                                                                  const float *__restrict__ g, const float *__restrict__ beta,
-                                                                  float *__restrict__ out, int n_k_heads, int n_v_heads, int K, int V) {
+__global__ void __launch_bounds__(GDN_WARPS * 32) gdn_step_kernel(float *state, const float *q, const float *k, const float *v,
+                                                                  const float *g, const float *beta, float *out, int n_k_heads, int n_v_heads, int K, int V) {
     __shared__ float ks[GDN_KMAX], qs[GDN_KMAX];
     __shared__ float part[GDN_WARPS][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -96,17 +161,22 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_step_kernel(float *__restr
     const int vh = blockIdx.x / tiles, vt = blockIdx.x - vh * tiles;
     const int j = vt * 32 + lane;
     const int kh = vh / (n_v_heads / n_k_heads);
-    for (int i = threadIdx.x; i < K; i += blockDim.x) {
-        ks[i] = k[(size_t)kh * K + i];
-        qs[i] = q[(size_t)kh * K + i];
-    }
     float *Sg = state + (size_t)vh * K * V + j;
-    const float decay = expf(g[vh]);
+    // the CTA's tile of the state, asked for while the launch before this one still runs: L2 hands out what it finds at the
+    // load below, whoever writes in between
+    if ((int)threadIdx.x < K) asm volatile("prefetch.global.L2 [%0];" ::"l"(state + ((size_t)vh * K + threadIdx.x) * V + vt * 32) : "memory");
+    pdl_wait_prior_grid();
+    pdl_launch_dependents();
     float col[GDN_RPW];
 #pragma unroll
     for (int r = 0; r < GDN_RPW; ++r) {
         const int i = warp + GDN_WARPS * r;
         col[r] = i < K ? Sg[(size_t)i * V] : 0.0f;
+    }
+    const float b = beta[vh], vj = v[(size_t)vh * V + j], decay = expf(g[vh]);
+    for (int i = threadIdx.x; i < K; i += blockDim.x) {
+        ks[i] = k[(size_t)kh * K + i];
+        qs[i] = q[(size_t)kh * K + i];
     }
     __syncthreads();
     float kv = 0.0f;
@@ -124,8 +194,7 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_step_kernel(float *__restr
 #pragma unroll
     for (int w = 0; w < GDN_WARPS; ++w) kv = __fadd_rn(kv, part[w][lane]);
     __syncthreads();                                    // part is reused below
-    const float b = beta[vh];
-    const float d = __fsub_rn(v[(size_t)vh * V + j], kv);
+    const float d = __fsub_rn(vj, kv);
     float o = 0.0f;
 #pragma unroll
     for (int r = 0; r < GDN_RPW; ++r) {

@@ -117,8 +117,8 @@ __global__ void __launch_bounds__(256) gemv_repack_kernel(const uint8_t *__restr
                      W + ((size_t)row0 + r_begin) * row_bytes, bytes, &bars[s], pol);
         }
     }
-    pdl_launch_dependents();
     pdl_wait_prior_grid();
+    pdl_launch_dependents();
 
     // fused quantiser: 8 lanes per 32-chunk, record of chunk 4*b + p stored at unit p*nb + b.
     // Loads run four iterations ahead of the shuffles that consume them.
