@@ -998,13 +998,14 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     P.epoch = g_gemm_epoch.fetch_add(1) + 1u;
     const int n_chunks = (int)(n_in / 32);
     const uint32_t *x32 = static_cast<const uint32_t *>(Xq);
-    unsigned int *maxd = reinterpret_cast<unsigned int *>(scale + n_tok);
-    e = cudaMemsetAsync(maxd, 0, (size_t)n_tok * sizeof(unsigned int), st);
+    // slices: whole passes of a block, as many as bring about two blocks per SM
+    const long long groups = (n_tok + 3) / 4;
+    int passes = (n_chunks + T16_SPLIT_PASS - 1) / T16_SPLIT_PASS;
+    passes = (int)((passes * groups + 2 * sms - 1) / (2 * sms));
+    const int slice = passes * T16_SPLIT_PASS;
+    e = launch(tc16_split_kernel, dim3((unsigned)groups, (unsigned)((n_chunks + slice - 1) / slice)), dim3(T16_SPLIT_THREADS), 0, st, true, x32, n_chunks,
+               (int)n_tok, slice, scale, planes);
     if (e != cudaSuccess) return (int)e;
-    const int slices = n_chunks >= 64 ? 16 : 1;
-    tc16_tokmax_kernel<<<dim3((unsigned)((n_tok + 31) / 32), (unsigned)slices), 256, 0, st>>>(x32, n_chunks, (int)n_tok, maxd);
-    const long long warps = ((n_tok + 3) / 4) * (long long)((n_chunks + 7) / 8);
-    tc16_split_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(x32, n_chunks, (int)n_tok, maxd, scale, planes);
     static SmemOptIn opt;
     e = opt.ensure(gemm_tc16_kernel<TN>);
     if (e != cudaSuccess) return (int)e;

@@ -129,19 +129,6 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 }
 
 // ---- once per call: the activations as two fp16 planes ------------------------------------------------------------
-// maxd[tok] = bits of the largest chunk scale of the token (non-negative floats order like their bit patterns);
-// zeroed by the caller.  Block = 32 tokens x 8 chunk lanes, grid.y slices the chunks.
-__global__ void __launch_bounds__(256) tc16_tokmax_kernel(const uint32_t *__restrict__ Xq, int n_chunks, int n_tok,
-                                                          unsigned int *__restrict__ maxd) {
-    const int tl = threadIdx.x & 31, grp = threadIdx.x >> 5;
-    const int tok = blockIdx.x * 32 + tl;
-    if (tok >= n_tok) return;
-    const int per = (n_chunks + (int)gridDim.y - 1) / (int)gridDim.y;
-    const int c0 = (int)blockIdx.y * per, c1 = min(n_chunks, c0 + per);
-    unsigned int m = 0;
-    for (int c = c0 + grp; c < c1; c += 8) m = max(m, __ldg(Xq + 9 * ((size_t)c * n_tok + tok)) & 0x7FFFu);
-    if (m) atomicMax(maxd + tok, m);
-}
 // 2^S for the token: S = 8 - exponent(max_c da_c), so that every |da * a * 2^S| < 2^15 (da = f * 2^ex, 0.5 <= f < 1,
 // times 128 is below 2^(ex + 7)).
 __device__ __forceinline__ int tc16_shift(unsigned int maxd_bits) {
@@ -150,45 +137,66 @@ __device__ __forceinline__ int tc16_shift(unsigned int maxd_bits) {
     if (m > 0.0f) (void)frexpf(m, &ex);
     return m > 0.0f ? 8 - ex : 0;
 }
-// Thread = (chunk, token): 32 values -> 32 + 32 fp16, in the order the quantiser stored them (the order in which the
-// code producers emit the codes).  planes: H at [tok][n_in], L at [n_tok + tok][n_in]; scale[tok] = 2^-S for the
-// epilogue.  A warp takes 4 tokens x 8 consecutive chunks: its stores are four runs of 512 bytes per plane.
-__global__ void __launch_bounds__(256) tc16_split_kernel(const uint32_t *__restrict__ Xq, int n_chunks, int n_tok,
-                                                         const unsigned int *__restrict__ maxd, float *__restrict__ scale,
-                                                         __half *__restrict__ planes) {
-    const int lane = threadIdx.x & 31;
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int cgroups = (n_chunks + 7) >> 3;
-    const int tg = (int)(warp / cgroups), cgp = (int)(warp - (long long)tg * cgroups);
-    const int tok = 4 * tg + (lane >> 3), c = 8 * cgp + (lane & 7);
-    if (tok >= n_tok || c >= n_chunks) return;
-    const int S = tc16_shift(maxd[tok]);
-    if (c == 0) scale[tok] = ldexpf(1.0f, -S);
-    const uint32_t *src = Xq + 9 * ((size_t)c * n_tok + tok);
-    uint32_t w[9];
+// Block = 4 tokens x one slice of the chunks (grid.y slices).  Every block first finds its tokens' largest chunk scale over
+// ALL chunks -- a slice more reads the headers once more, from L2, and there is no pass, no zeroed array and no launch
+// between the maximum and the split -- then thread = (chunk, token): 32 values -> 32 + 32 fp16, in the order the quantiser
+// stored them (the order in which the code producers emit the codes).  planes: H at [tok][n_in], L at [n_tok + tok][n_in];
+// scale[tok] = 2^-S for the epilogue.  A warp takes 4 tokens x 8 consecutive chunks: its stores are four runs of 512 bytes
+// per plane.  Bound by launch and memory latency.
+constexpr int T16_SPLIT_THREADS = 256, T16_SPLIT_PASS = T16_SPLIT_THREADS / 4;      // chunks of four tokens a block takes at once
+__global__ void __launch_bounds__(T16_SPLIT_THREADS) tc16_split_kernel(const uint32_t *Xq, int n_chunks, int n_tok, int slice, float *scale,
+                                                                       __half *planes) {
+    __shared__ unsigned int top[T16_SPLIT_THREADS / 32][4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tok = 4 * (int)blockIdx.x + (lane >> 3);
+    pdl_wait_prior_grid();
+    pdl_launch_dependents();
+    {   // four tokens are neighbours in memory: four lanes read one chunk's headers
+        const int t = 4 * (int)blockIdx.x + (lane & 3);
+        unsigned int m = 0;
+        if (t < n_tok)
+#pragma unroll 4
+            for (int c = threadIdx.x >> 2; c < n_chunks; c += T16_SPLIT_PASS) m = max(m, Xq[9 * ((size_t)c * n_tok + t)] & 0x7FFFu);
 #pragma unroll
-    for (int k = 0; k < 9; ++k) w[k] = __ldg(src + k);
-    const float ds = __fmul_rn(f16_bits_to_f32(w[0] & 0xFFFFu), ldexpf(1.0f, S));        // da * 2^S: exact (a power of two)
+        for (int o = 4; o < 32; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane < 4) top[warp][lane] = m;
+    }
+    __syncthreads();
+    unsigned int m = 0;
+#pragma unroll
+    for (int w = 0; w < T16_SPLIT_THREADS / 32; ++w) m = max(m, top[w][lane >> 3]);
+    if (tok >= n_tok) return;
+    const int S = tc16_shift(m);
+    const float up = ldexpf(1.0f, S);
     const size_t n_in = (size_t)n_chunks * 32;
-    uint4 *hp = reinterpret_cast<uint4 *>(planes + (size_t)tok * n_in + (size_t)c * 32);
-    uint4 *lp = reinterpret_cast<uint4 *>(planes + ((size_t)n_tok + tok) * n_in + (size_t)c * 32);
-    const int8_t *ab = reinterpret_cast<const int8_t *>(w + 1);      // the chunk's 32 int8 in stored order
+    if (blockIdx.y == 0 && threadIdx.x < 32 && (lane & 7) == 0) scale[tok] = ldexpf(1.0f, -S);
+    const int c1 = min(n_chunks, ((int)blockIdx.y + 1) * slice);
+    for (int c = (int)blockIdx.y * slice + 8 * warp + (lane & 7); c < c1; c += T16_SPLIT_PASS) {
+        const uint32_t *src = Xq + 9 * ((size_t)c * n_tok + tok);
+        uint32_t w[9];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {                       // 8 values per 16-byte store, in the order of tc16_expand
-        uint32_t h[4], l[4];
+        for (int k = 0; k < 9; ++k) w[k] = src[k];
+        const float ds = __fmul_rn(f16_bits_to_f32(w[0] & 0xFFFFu), up);        // da * 2^S: exact (a power of two)
+        uint4 *hp = reinterpret_cast<uint4 *>(planes + (size_t)tok * n_in + (size_t)c * 32);
+        uint4 *lp = reinterpret_cast<uint4 *>(planes + ((size_t)n_tok + tok) * n_in + (size_t)c * 32);
+        const int8_t *ab = reinterpret_cast<const int8_t *>(w + 1);      // the chunk's 32 int8 in stored order
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            constexpr unsigned char PERM[16] = {0, 8, 1, 9, 4, 12, 5, 13, 2, 10, 3, 11, 6, 14, 7, 15};
-            const int j0 = 16 * (q >> 1) + PERM[8 * (q & 1) + 2 * e], j1 = 16 * (q >> 1) + PERM[8 * (q & 1) + 2 * e + 1];
-            const int a0 = (int)ab[j0], a1 = (int)ab[j1];
-            const float v0 = __fmul_rn(ds, (float)a0), v1 = __fmul_rn(ds, (float)a1);      // exact: 11 x 7 bits
-            const __half h0 = __float2half_rn(v0), h1 = __float2half_rn(v1);
-            const __half l0 = __float2half_rn(__fsub_rn(v0, __half2float(h0))), l1 = __float2half_rn(__fsub_rn(v1, __half2float(h1)));
-            h[e] = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
-            l[e] = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
+        for (int q = 0; q < 4; ++q) {                       // 8 values per 16-byte store, in the order of tc16_expand
+            uint32_t h[4], l[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                constexpr unsigned char PERM[16] = {0, 8, 1, 9, 4, 12, 5, 13, 2, 10, 3, 11, 6, 14, 7, 15};
+                const int j0 = 16 * (q >> 1) + PERM[8 * (q & 1) + 2 * e], j1 = 16 * (q >> 1) + PERM[8 * (q & 1) + 2 * e + 1];
+                const int a0 = (int)ab[j0], a1 = (int)ab[j1];
+                const float v0 = __fmul_rn(ds, (float)a0), v1 = __fmul_rn(ds, (float)a1);      // exact: 11 x 7 bits
+                const __half h0 = __float2half_rn(v0), h1 = __float2half_rn(v1);
+                const __half l0 = __float2half_rn(__fsub_rn(v0, __half2float(h0))), l1 = __float2half_rn(__fsub_rn(v1, __half2float(h1)));
+                h[e] = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
+                l[e] = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
+            }
+            hp[q] = make_uint4(h[0], h[1], h[2], h[3]);
+            lp[q] = make_uint4(l[0], l[1], l[2], l[3]);
         }
-        hp[q] = make_uint4(h[0], h[1], h[2], h[3]);
-        lp[q] = make_uint4(l[0], l[1], l[2], l[3]);
     }
 }
 
