@@ -1,0 +1,451 @@
+// attn_tc.cuh -- causal attention of a prompt on the tensor cores (tcgen05.mma.kind::f16), fp32 in and out.
+//
+// attn_kernel (ops.cuh) multiplies on the CUDA cores and is bound by their issue slots and by shared memory.  Here both
+// products run on the tensor cores without giving up fp32: every operand is scaled by a power of two (q and k per row, v per
+// output dim and tile, softmax weights by 2^14) and split into two fp16 planes, high and low, 22 - 24 bits together; what
+// the low plane cannot hold is below 2^-39 of the row's largest value.  The tensor core cuts the last bits of a sum off
+// instead of rounding it, so sums are kept short: a score is six sums over 32 or 48 dims (an accumulator over all 256 was 1.5
+// to 3 times less exact than the CUDA cores), joined by rounded additions, and a tile's weights x v go to a fresh accumulator
+// that the CUDA cores add to the fp32 output.  Error against 64 bits: at
+// ATC_MIN_TOKENS.
+//
+// attn_planes_kernel writes k and v once per call as tile images: the bytes that the attention kernel's shared memory holds
+// for 64 keys of a kv head, planes split, swizzled and (v) transposed, fetched by one bulk copy each.  (Every CTA splitting
+// its own tiles did that 50 times over at 2048 tokens and took twice the time of the products: 370 us.)
+//
+// attn_tc_kernel: CTA = 128 queries of one head, 512 threads, each one row and a quarter of its columns:
+//   q . k, dims 0 .. 63      | outputs of the tile before into registers
+//   q . k, dims 64 .. 255    |
+//   (tensor core idle)       | softmax, weights -> planes in tensor memory
+//   weights x v              |
+// Shared memory: q high, k and v images of one tile, 64 KB each (K-major, 128-byte swizzle).  Tensor memory, all 512
+// columns: 256 output (before that, sums of the scores), 128 scores (then weights), 128 q low.
+// What bounds it: per tile 5900 of 10200 cycles are the tensor core's, most of them the score products (N = 64: it waits for
+// the q rows from shared memory), the rest softmax and the exchanges in front of it.  2048 tokens, 24 heads over 4: 2570 ->
+// 293 us; 1000 tokens 727 -> 94 us, 517 tokens 246 -> 59 us.
+//
+// Infinities, NaN and values past 2^60 do not survive the split; a CTA that meets one does its queries again on the CUDA
+// cores (attn_simt), with that kernel's results.
+#pragma once
+
+#include "gemm_tc16.cuh"
+#include "kv.cuh"
+#include "ops.cuh"
+
+namespace b200 {
+
+// From this token count on.  It is faster from 100 tokens on (301: 40 us against 118 us), but there the CUDA cores' longest sums
+// are short enough to be the more exact ones: relative error against 64 bits (normal values, 24 heads over 4) at 301 tokens
+// 1.8e-7 here and 1.8e-7 there, at 200 1.8e-7 and 1.6e-7; at 517 1.9e-7 and 2.1e-7, at 1000 2.0e-7 and 2.6e-7, at 2048
+// 2.1e-7 and 3.4e-7.
+constexpr int ATC_MIN_TOKENS = 512;
+constexpr int ATC_M = 128, ATC_KEYS = 64, ATC_WARPS = 16, ATC_THREADS = ATC_WARPS * 32;
+constexpr int ATC_CHUNK = 128 * 128;                         // bytes of 128 rows x 64 fp16
+constexpr int ATC_PLANES = 4 * ATC_CHUNK;                    // q high; k high + low; v high + low: 64 KB each
+constexpr int ATC_SMEM_BYTES = 1024 + 3 * ATC_PLANES + (2 * ATC_KEYS + 2 * ATT_D + 4 * ATC_M) * 4 + 64;
+// tile image in global memory: k planes, v planes, 2^-s of the 64 keys, 2^-s of the 256 dims, whether a value is not finite or huge
+constexpr int ATC_IMG_KF = 2 * ATC_PLANES, ATC_IMG_VF = ATC_IMG_KF + ATC_KEYS * 4, ATC_IMG_FLAG = ATC_IMG_VF + ATT_D * 4;   // flag: k, then v
+constexpr int ATC_IMG_BYTES = 2 * ATC_PLANES + 2048;
+constexpr uint32_t ATC_COL_O = 0, ATC_COL_S = 256, ATC_COL_QL = 384;
+constexpr uint32_t ATC_HUGE = (127u + 60u) << 23;            // bits of 2^60
+constexpr int ATC_REDO_QUERIES = ATC_WARPS * ATT_QPW;
+static_assert(ATT_SMEM_BYTES <= 3 * ATC_PLANES, "attn_simt reuses the planes");
+
+__host__ __device__ constexpr uint32_t atc_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(ATC_M >> 4) << 24); }
+
+template <uint32_t IDESC>
+__device__ __forceinline__ void atc_mma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %4};\n\t"
+        "mov.b64 db, {%2, %4};\n\t"
+        "setp.ne.b32 p, 1, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, {%5, %5, %5, %5}, p;\n\t"
+        "}\n"
+        ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(IDESC), "r"(T16_DESC_HI), "r"(0u)
+        : "memory");
+}
+__device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t atc_abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
+// s with 2^14 <= max * 2^s < 2^15, at most `cap` (smaller maxima end lower: their products are that much smaller too)
+__device__ __forceinline__ int atc_shift(uint32_t max_bits, int cap) { return min(cap, 141 - (int)(max_bits >> 23)); }
+__device__ __forceinline__ float atc_pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
+__device__ __forceinline__ void atc_split8(const float *x, float sc, uint4 &hi, uint4 &lo) {
+    split_f16x2(__fmul_rn(x[0], sc), __fmul_rn(x[1], sc), hi.x, lo.x);
+    split_f16x2(__fmul_rn(x[2], sc), __fmul_rn(x[3], sc), hi.y, lo.y);
+    split_f16x2(__fmul_rn(x[4], sc), __fmul_rn(x[5], sc), hi.z, lo.z);
+    split_f16x2(__fmul_rn(x[6], sc), __fmul_rn(x[7], sc), hi.w, lo.w);
+}
+
+constexpr int ATC_PREP_THREADS = 256;
+// grid (tiles, kv heads, 2): z 0 = k (warp = eight keys, lane = eight dims), z 1 = v (thread = one dim, all 64 keys).  Bound
+// by latency: 16 MB in, 17 MB out at 2048 tokens.
+__global__ void __launch_bounds__(ATC_PREP_THREADS) attn_planes_kernel(const float *k, const float *v, uint8_t *images, int n_tok, int n_head_kv) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j0 = (int)blockIdx.x * ATC_KEYS, kvh = blockIdx.y;
+    uint8_t *img = images + ((size_t)kvh * gridDim.x + blockIdx.x) * ATC_IMG_BYTES;
+    uint32_t seen = 0;
+    pdl_wait_prior_grid();
+    pdl_launch_dependents();
+    if (blockIdx.z == 0) {
+        constexpr int ROWS = ATC_KEYS / (ATC_PREP_THREADS / 32);
+        float x[ROWS][8];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            const int key = ROWS * warp + r;
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+            if (j0 + key < n_tok) {
+                const float4 *src = reinterpret_cast<const float4 *>(k + ((size_t)(j0 + key) * n_head_kv + kvh) * ATT_D + 8 * lane);
+                a = src[0];
+                b = src[1];
+            }
+            x[r][0] = a.x; x[r][1] = a.y; x[r][2] = a.z; x[r][3] = a.w; x[r][4] = b.x; x[r][5] = b.y; x[r][6] = b.z; x[r][7] = b.w;
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            const int key = ROWS * warp + r;
+            uint32_t m = 0;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) m = max(m, atc_abs_bits(x[r][e]));
+            m = __reduce_max_sync(0xffffffffu, m);
+            seen = max(seen, m);
+            const int s = atc_shift(m, 63);
+            uint4 hi, lo;
+            atc_split8(x[r], atc_pow2(s), hi, lo);
+            uint8_t *dst = img + (lane >> 3) * ATC_CHUNK + key * 128 + (((lane & 7) ^ (key & 7)) * 16);
+            *reinterpret_cast<uint4 *>(dst) = hi;
+            *reinterpret_cast<uint4 *>(dst + ATC_KEYS * 128) = lo;
+            if (lane == 0) reinterpret_cast<float *>(img + ATC_IMG_KF)[key] = atc_pow2(-s);
+        }
+    } else {
+        const int d = threadIdx.x;
+        float x[ATC_KEYS];
+        const float *src = v + ((size_t)j0 * n_head_kv + kvh) * ATT_D + d;
+#pragma unroll
+        for (int e = 0; e < ATC_KEYS; ++e) x[e] = j0 + e < n_tok ? src[(size_t)e * n_head_kv * ATT_D] : 0.0f;
+#pragma unroll
+        for (int e = 0; e < ATC_KEYS; ++e) seen = max(seen, atc_abs_bits(x[e]));
+        const int s = atc_shift(seen, 112);
+        reinterpret_cast<float *>(img + ATC_IMG_VF)[d] = atc_pow2(-s - 14);          // and the weights' 2^-14
+#pragma unroll
+        for (int g = 0; g < ATC_KEYS / 8; ++g) {
+            uint4 hi, lo;
+            atc_split8(x + 8 * g, atc_pow2(s), hi, lo);
+            uint8_t *dst = img + ATC_PLANES + d * 128 + ((g ^ (d & 7)) * 16);
+            *reinterpret_cast<uint4 *>(dst) = hi;
+            *reinterpret_cast<uint4 *>(dst + 2 * ATC_CHUNK) = lo;
+        }
+    }
+    const int bad = __syncthreads_or(seen >= ATC_HUGE ? 1 : 0);
+    if (threadIdx.x == 0) reinterpret_cast<int *>(img + ATC_IMG_FLAG)[blockIdx.z] = bad;
+}
+
+// Cold path, a call of its own so that it takes no registers from the kernel.
+__device__ __noinline__ void attn_redo(float *smem, const float *q, const float *k, const float *v, float *out, int first, int head, int n_tok,
+                                       int n_head, int n_head_kv, float scale) {
+    for (int q0 = first; q0 < min(n_tok, first + ATC_M); q0 += ATC_REDO_QUERIES) {
+        __syncthreads();
+        attn_simt<ATC_WARPS>(smem, q, k, v, out, q0, head, n_tok, n_head, n_head_kv, scale);
+    }
+}
+
+// grid: query blocks x heads, the longest rows of keys first (block index / n_head counts from the last query block)
+__global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q, const float *k, const float *v, const uint8_t *images, float *out,
+                                                                 int n_tok, int n_head, int n_head_kv, float scale) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint8_t *qhi = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
+    uint8_t *kpl = qhi + ATC_PLANES, *vpl = kpl + ATC_PLANES;
+    float *kf = reinterpret_cast<float *>(vpl + ATC_PLANES);             // [2][64] 2^-s of the tile's keys, tiles alternate
+    float *vf = kf + 2 * ATC_KEYS;                                       // [2][256] 2^-s of the dims (and the weights' 2^-14)
+    float *red = vf + 2 * ATT_D;                                         // [4][128] exchange between the four warps of a row
+    uint64_t *qk1 = reinterpret_cast<uint64_t *>(red + 4 * ATC_M), *qk2 = qk1 + 1, *pv = qk1 + 2, *kfull = qk1 + 3, *vfull = qk1 + 4;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(vfull + 1);
+
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int cg = warp >> 2, row = 32 * (warp & 3) + lane;              // a thread's row, and its quarter of the row's columns
+    const int qblocks = (n_tok + ATC_M - 1) / ATC_M;
+    const int head = (int)blockIdx.x % n_head, first = (qblocks - 1 - (int)blockIdx.x / n_head) * ATC_M;
+    const int kvh = head / (n_head / n_head_kv);
+    const int query = first + row;
+    const int ntiles = (min(n_tok, first + ATC_M) + ATC_KEYS - 1) / ATC_KEYS;
+    const uint8_t *img = images + (size_t)kvh * ((n_tok + ATC_KEYS - 1) / ATC_KEYS) * ATC_IMG_BYTES;
+
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < 5; ++b) mbar_init(qk1 + b, 1);
+        mbar_fence_init();
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // one thread each: the images of tile i
+    auto load_k = [&](int i) {
+        const uint64_t pol = policy_evict_last_or_default();
+        const uint8_t *src = img + (size_t)i * ATC_IMG_BYTES;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the factors were read by ordinary loads
+        mbar_expect_tx(kfull, ATC_PLANES + ATC_KEYS * 4);
+        bulk_g2s(kf + (i & 1) * ATC_KEYS, src + ATC_IMG_KF, ATC_KEYS * 4, kfull, pol);
+        bulk_g2s(kpl, src, ATC_PLANES, kfull, pol);
+    };
+    auto load_v = [&](int i) {
+        const uint64_t pol = policy_evict_last_or_default();
+        const uint8_t *src = img + (size_t)i * ATC_IMG_BYTES;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the factors were read by ordinary loads
+        mbar_expect_tx(vfull, ATC_PLANES + ATT_D * 4);
+        bulk_g2s(vf + (i & 1) * ATT_D, src + ATC_IMG_VF, ATT_D * 4, vfull, pol);
+        bulk_g2s(vpl, src + ATC_PLANES, ATC_PLANES, vfull, pol);
+    };
+
+    // ---- q: row of the thread, 64 dims; high plane to shared memory, low plane to tensor memory.  (The launch this one may
+    // run beside is attn_planes_kernel, which does not write q.)
+    float qf;
+    uint32_t seen = 0;                                                   // largest magnitude bits met
+    {
+        float x[64];
+        uint32_t m = 0;
+        const float *src = q + ((size_t)query * n_head + head) * ATT_D + 64 * cg;
+        if (query < n_tok) {
+            if ((reinterpret_cast<uintptr_t>(q) & 15u) == 0) {
+#pragma unroll
+                for (int e = 0; e < 64; e += 4) {
+                    const float4 a = *reinterpret_cast<const float4 *>(src + e);
+                    x[e] = a.x; x[e + 1] = a.y; x[e + 2] = a.z; x[e + 3] = a.w;
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 64; ++e) x[e] = src[e];
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 64; ++e) x[e] = 0.0f;
+        }
+#pragma unroll
+        for (int e = 0; e < 64; ++e) {
+            x[e] = __fmul_rn(x[e], scale);
+            m = max(m, atc_abs_bits(x[e]));
+        }
+        uint32_t *redu = reinterpret_cast<uint32_t *>(red);
+        redu[cg * ATC_M + row] = m;
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) m = max(m, redu[c * ATC_M + row]);
+        seen = m;
+        const int s = atc_shift(m, 63);
+        qf = atc_pow2(-s);
+        uint32_t lo32[32];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            uint4 hi, lo;
+            atc_split8(x + 8 * j, atc_pow2(s), hi, lo);
+            *reinterpret_cast<uint4 *>(qhi + cg * ATC_CHUNK + row * 128 + ((j ^ (row & 7)) * 16)) = hi;
+            lo32[4 * j] = lo.x; lo32[4 * j + 1] = lo.y; lo32[4 * j + 2] = lo.z; lo32[4 * j + 3] = lo.w;
+        }
+        tc_st32(*tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + ATC_COL_QL + (uint32_t)(32 * cg), lo32);
+    }
+    const uint32_t tmem = *tmem_slot;
+    const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    // The tensor core's instructions, one elected lane of warp 0 (the code stays warp-uniform).  Products with a low plane
+    // come first: the accumulator is small while they are added.
+    // One sum of the scores: 16-dim steps n0 .. n0 + STEPS - 1 into 64 columns at d.
+    auto sum_of = [&](uint32_t d, auto n0c, auto stepsc) {
+        constexpr int N0 = decltype(n0c)::value, STEPS = decltype(stepsc)::value;
+        constexpr uint32_t LOW = (ATC_KEYS * 128) >> 4;
+        const uint32_t a0 = tc16_desc_lo(smem_u32(qhi)), b0 = tc16_desc_lo(smem_u32(kpl)), ql = tmem + ATC_COL_QL;
+        auto at = [](int n) { return (uint32_t)((n >> 2) * (ATC_CHUNK >> 4) + 2 * (n & 3)); };
+        tc_mma_f16_ts<false>(d, ql + (uint32_t)(8 * N0), b0 + at(N0), atc_idesc(ATC_KEYS));
+#pragma unroll
+        for (int n = N0 + 1; n < N0 + STEPS; ++n) tc_mma_f16_ts<true>(d, ql + (uint32_t)(8 * n), b0 + at(n), atc_idesc(ATC_KEYS));
+#pragma unroll
+        for (int n = N0; n < N0 + STEPS; ++n) atc_mma_ss<atc_idesc(ATC_KEYS)>(d, a0 + at(n), b0 + LOW + at(n));
+#pragma unroll
+        for (int n = N0; n < N0 + STEPS; ++n) atc_mma_ss<atc_idesc(ATC_KEYS)>(d, a0 + at(n), b0 + at(n));
+    };
+    auto issue_qk_a = [&] {                                              // dims 0 .. 63, two sums, into the score columns
+        tc_fence_after();
+        if (elect_one()) {
+            sum_of(tmem + ATC_COL_S, std::integral_constant<int, 0>{}, std::integral_constant<int, 2>{});
+            sum_of(tmem + ATC_COL_S + ATC_KEYS, std::integral_constant<int, 2>{}, std::integral_constant<int, 2>{});
+            tc_commit(qk1);
+        }
+        __syncwarp();
+    };
+    auto issue_qk_b = [&] {                                              // dims 64 .. 255, four sums, into the output columns
+        tc_fence_after();
+        if (elect_one()) {
+            sum_of(tmem + ATC_COL_O, std::integral_constant<int, 4>{}, std::integral_constant<int, 3>{});
+            sum_of(tmem + ATC_COL_O + ATC_KEYS, std::integral_constant<int, 7>{}, std::integral_constant<int, 3>{});
+            sum_of(tmem + ATC_COL_O + 2 * ATC_KEYS, std::integral_constant<int, 10>{}, std::integral_constant<int, 3>{});
+            sum_of(tmem + ATC_COL_O + 3 * ATC_KEYS, std::integral_constant<int, 13>{}, std::integral_constant<int, 3>{});
+            tc_commit(qk2);
+        }
+        __syncwarp();
+    };
+    auto issue_pv = [&] {
+        tc_fence_after();
+        const uint32_t b0 = tc16_desc_lo(smem_u32(vpl)), ph = tmem + ATC_COL_S, pl = ph + 32u;
+        if (elect_one()) {
+#pragma unroll
+            for (int n = 0; n < 12; ++n) {
+                const uint32_t a = (n < 4 ? pl : ph) + (uint32_t)(8 * (n & 3));
+                const uint32_t b = b0 + (uint32_t)((n >= 4 && n < 8 ? (2 * ATC_CHUNK) >> 4 : 0) + 2 * (n & 3));
+                if (n == 0) tc_mma_f16_ts<false>(tmem + ATC_COL_O, a, b, atc_idesc(ATT_D));
+                else tc_mma_f16_ts<true>(tmem + ATC_COL_O, a, b, atc_idesc(ATT_D));
+            }
+            tc_commit(pv);
+        }
+        __syncwarp();
+    };
+
+    pdl_wait_prior_grid();                                               // the images
+    if (warp == 4 && lane == 0) {
+        load_k(0);
+        load_v(0);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");        // q high: written here, read by the tensor core
+    tc_st_wait();
+    tc_fence_before();
+    __syncthreads();
+    bool ok = true;
+    if (warp == 0) {
+        ok = mbar_wait_hot(kfull, 0);
+        issue_qk_a();
+        issue_qk_b();
+    }
+
+    float acc[64];                                                       // row, dims 64 cg ..
+#pragma unroll
+    for (int e = 0; e < 64; ++e) acc[e] = 0.0f;
+    float m_run = -INFINITY, l_run = 0.0f, alpha = 0.0f;                 // l_run: of the thread's 16 columns of every tile
+    auto add_tile = [&](int par) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            int o[2][16];
+            tc_ld16(tlane + ATC_COL_O + (uint32_t)(64 * cg + 32 * h), o[0]);
+            tc_ld16(tlane + ATC_COL_O + (uint32_t)(64 * cg + 32 * h + 16), o[1]);
+            tc_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) {
+                const float4 f = *reinterpret_cast<const float4 *>(vf + par * ATT_D + 64 * cg + 32 * h + e);
+                float *a = acc + 32 * h + e;
+                const int *t = o[e >> 4] + (e & 15);
+                a[0] = __fmaf_rn(__int_as_float(t[0]), f.x, __fmul_rn(a[0], alpha));
+                a[1] = __fmaf_rn(__int_as_float(t[1]), f.y, __fmul_rn(a[1], alpha));
+                a[2] = __fmaf_rn(__int_as_float(t[2]), f.z, __fmul_rn(a[2], alpha));
+                a[3] = __fmaf_rn(__int_as_float(t[3]), f.w, __fmul_rn(a[3], alpha));
+            }
+        }
+    };
+    for (int i = 0; i < ntiles; ++i) {
+        const int j0 = i * ATC_KEYS;
+        const uint32_t par = (uint32_t)(i & 1);
+        float s[16], mx = -INFINITY;
+        ok = mbar_wait_hot(kfull, par) && ok;                            // (long complete; makes the copied factors visible)
+        ok = mbar_wait_hot(qk1, par) && ok;
+        ok = mbar_wait_hot(qk2, par) && ok;
+        tc_fence_after();
+        if (warp == 4 && lane == 0 && i + 1 < ntiles) load_k(i + 1);
+        {
+            auto pair = [&](uint32_t col, float (&t)[16]) {
+                int a[16], b[16];
+                tc_ld16(tlane + col + (uint32_t)(16 * cg), a);
+                tc_ld16(tlane + col + (uint32_t)(ATC_KEYS + 16 * cg), b);
+                tc_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 16; ++e) t[e] = __fadd_rn(__int_as_float(a[e]), __int_as_float(b[e]));
+            };
+            float t[16];
+            pair(ATC_COL_S, s);
+            pair(ATC_COL_O, t);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) s[e] = __fadd_rn(s[e], t[e]);
+            pair(ATC_COL_O + 2 * ATC_KEYS, t);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const float f = __fmul_rn(qf, kf[par * ATC_KEYS + 16 * cg + e]);
+                s[e] = j0 + 16 * cg + e <= query ? __fmul_rn(__fadd_rn(s[e], t[e]), f) : -INFINITY;
+                mx = fmaxf(mx, s[e]);
+            }
+        }
+        red[cg * ATC_M + row] = mx;
+        tc_fence_before();
+        if (!__syncthreads_and(ok ? 1 : 0)) break;                       // (a wait ran out: the CTA leaves as a whole)
+        tc_fence_after();                                                // every score has been read: the weights take their place
+        float m_new = m_run;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) m_new = fmaxf(m_new, red[c * ATC_M + row]);
+        alpha = expf(__fsub_rn(m_run, m_new));
+        m_run = m_new;
+        {
+            uint32_t hi[8], lo[8];
+            float sum = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 16; e += 2) {
+                const float p0 = expf(__fsub_rn(s[e], m_new)), p1 = expf(__fsub_rn(s[e + 1], m_new));
+                sum = __fadd_rn(sum, __fadd_rn(p0, p1));
+                split_f16x2(__fmul_rn(p0, 16384.0f), __fmul_rn(p1, 16384.0f), hi[e >> 1], lo[e >> 1]);
+            }
+            l_run = __fadd_rn(__fmul_rn(l_run, alpha), sum);
+            tc_st8(tlane + ATC_COL_S + (uint32_t)(8 * cg), hi);
+            tc_st8(tlane + ATC_COL_S + (uint32_t)(32 + 8 * cg), lo);
+        }
+        tc_st_wait();
+        tc_fence_before();
+        __syncthreads();
+        ok = mbar_wait_hot(vfull, par) && ok;
+        if (warp == 0) issue_pv();
+        ok = mbar_wait_hot(pv, par) && ok;
+        tc_fence_after();
+        if (i + 1 < ntiles) {
+            if (warp == 4 && lane == 0) load_v(i + 1);
+            if (warp == 0) {
+                ok = mbar_wait_hot(kfull, par ^ 1u) && ok;
+                issue_qk_a();
+            }
+        }
+        add_tile((int)par);
+        if (i + 1 < ntiles) {
+            tc_fence_before();
+            __syncthreads();                                             // the output columns have been read: scores may go there
+            if (warp == 0) issue_qk_b();
+        }
+    }
+    __syncthreads();
+    red[cg * ATC_M + row] = l_run;
+    tc_fence_before();
+    for (int t = threadIdx.x; t < ntiles; t += ATC_THREADS) {
+        const int2 f = *reinterpret_cast<const int2 *>(img + (size_t)t * ATC_IMG_BYTES + ATC_IMG_FLAG);
+        if (f.x | f.y) seen = 0x7FFFFFFFu;
+    }
+    const bool redo = __syncthreads_or(seen >= ATC_HUGE ? 1 : 0) != 0;
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+    if (redo) {
+        attn_redo(reinterpret_cast<float *>(qhi), q, k, v, out, first, head, n_tok, n_head, n_head_kv, scale);
+        return;
+    }
+    if (query < n_tok) {
+        const float l = __fadd_rn(__fadd_rn(red[row], red[ATC_M + row]), __fadd_rn(red[2 * ATC_M + row], red[3 * ATC_M + row]));
+        const float inv = __fdiv_rn(1.0f, l);
+        float *dst = out + ((size_t)query * n_head + head) * ATT_D + 64 * cg;
+        if ((reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+#pragma unroll
+            for (int e = 0; e < 64; e += 4)
+                *reinterpret_cast<float4 *>(dst + e) = make_float4(__fmul_rn(acc[e], inv), __fmul_rn(acc[e + 1], inv), __fmul_rn(acc[e + 2], inv), __fmul_rn(acc[e + 3], inv));
+        } else {
+#pragma unroll
+            for (int e = 0; e < 64; ++e) dst[e] = __fmul_rn(acc[e], inv);
+        }
+    }
+}
+
+}  // namespace b200

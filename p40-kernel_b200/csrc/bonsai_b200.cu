@@ -8,6 +8,7 @@
 #include "../../include/bonsai_kv.h"
 
 #include "activation.cuh"
+#include "attn_tc.cuh"
 #include "gemm_simt.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_tc16.cuh"
@@ -947,6 +948,47 @@ static void *gemm_scratch(size_t bytes, cudaStream_t st) {
     return pnew;
 }
 
+// Scratch of the prompt attention (k and v as tile images: 2 KB per position and kv head, what k and v take themselves), kept
+// per stream and bounded: the 17th stream of a device takes the place of the one that called longest ago.  Streams are told
+// apart by their number, which no later stream is given again.  cudaFree waits for the device, so nothing in flight reads
+// what is freed; no graph holds an address (a stream under capture is given none).  The caller holds g_attn_mu until the
+// launches that use the buffer are enqueued.
+struct AttnScratch { int dev; unsigned long long stream, used; void *ptr; size_t bytes; };
+static std::mutex g_attn_mu;
+static std::vector<AttnScratch> g_attn_scratch;
+static void *attn_scratch(size_t bytes, cudaStream_t st) {
+    static unsigned long long calls = 0;
+    int dev = 0, of_dev = 0;
+    unsigned long long id = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaStreamGetId(st, &id) != cudaSuccess) return nullptr;
+    AttnScratch *e = nullptr, *oldest = nullptr;
+    for (auto &g : g_attn_scratch) {
+        if (g.dev != dev) continue;
+        ++of_dev;
+        if (g.stream == id) e = &g;
+        if (!oldest || g.used < oldest->used) oldest = &g;
+    }
+    if (!e && of_dev >= 16) e = oldest;
+    if (!e) {
+        g_attn_scratch.push_back(AttnScratch{dev, id, 0, nullptr, 0});
+        e = &g_attn_scratch.back();
+    }
+    if (e->stream != id || e->bytes < bytes) {
+        // another stream may be under capture: allocating is no part of that
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        (void)cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e->ptr) (void)cudaFree(e->ptr);
+        e->ptr = nullptr;
+        e->bytes = 0;
+        e->stream = id;
+        if (cudaMalloc(&e->ptr, bytes) == cudaSuccess) e->bytes = bytes;
+        else e->ptr = nullptr, (void)cudaGetLastError();
+        (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    e->used = ++calls;
+    return e->ptr;
+}
+
 static std::atomic<unsigned int> g_gemm_epoch{0};       // launch number of the tensor-core mat-muls (tags partial-tile flags)
 
 static void fill_tc_params(TcParams &P, int64_t n_out, int64_t n_in, int64_t n_tok, int tile_m, int tile_n) {
@@ -1143,12 +1185,19 @@ int bonsai_b200_gemm_release(void) {
     std::lock_guard<std::mutex> lock(g_scratch_mu);
     int dev = 0;
     const bool have = cudaGetDevice(&dev) == cudaSuccess;
-    for (auto &g : g_scratch) {
-        if (!g.ptr) continue;
-        if (have) (void)cudaSetDevice(g.dev);
-        (void)cudaFree(g.ptr);
+    auto release = [&](auto &pool) {
+        for (auto &g : pool) {
+            if (!g.ptr) continue;
+            if (have) (void)cudaSetDevice(g.dev);
+            (void)cudaFree(g.ptr);
+        }
+        pool.clear();
+    };
+    release(g_scratch);
+    {
+        std::lock_guard<std::mutex> attn_lock(g_attn_mu);
+        release(g_attn_scratch);
     }
-    g_scratch.clear();
     if (have) (void)cudaSetDevice(dev);
     return 0;
 }
@@ -1386,6 +1435,25 @@ int bonsai_p40_gdn_step(float *state, const float *q, const float *k, const floa
                        n_v_heads, K, V);
 }
 
+// Attention on the tensor cores (attn_tc.cuh).  -1: not taken (a stream that is being captured -- a graph would keep the
+// scratch's address -- or no scratch to be had).
+static int launch_attn_tc(const float *q, const float *k, const float *v, float *out, int n_tok, int n_head, int n_head_kv, float scale, cudaStream_t st) {
+    const int tiles = (n_tok + ATC_KEYS - 1) / ATC_KEYS;
+    const long long ctas = (long long)n_head * ((n_tok + ATC_M - 1) / ATC_M);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (ctas > INT32_MAX || n_head_kv > 65535 || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return -1;
+    std::lock_guard<std::mutex> lock(g_attn_mu);
+    uint8_t *images = static_cast<uint8_t *>(attn_scratch((size_t)tiles * n_head_kv * ATC_IMG_BYTES, st));
+    if (!images) return -1;
+    static SmemOptIn opt;
+    cudaError_t e = opt.ensure(attn_tc_kernel);
+    if (e == cudaSuccess)
+        e = launch(attn_planes_kernel, dim3((unsigned)tiles, (unsigned)n_head_kv, 2), dim3(ATC_PREP_THREADS), 0, st, true, k, v, images, n_tok, n_head_kv);
+    if (e == cudaSuccess)
+        e = launch(attn_tc_kernel, dim3((unsigned)ctas), dim3(ATC_THREADS), (size_t)ATC_SMEM_BYTES, st, true, q, k, v, images, out, n_tok, n_head, n_head_kv, scale);
+    return (int)e;
+}
+
 int bonsai_p40_attn(const float *q, const float *k, const float *v, float *out, int n_tok, int n_head, int n_head_kv,
                     int head_dim, float scale, bonsai_stream stream) {
     // rejections of src/kernels/attn_p40.cu:134-136
@@ -1394,6 +1462,10 @@ int bonsai_p40_attn(const float *q, const float *k, const float *v, float *out, 
     if (!aligned16(k) || !aligned16(v) || !aligned4(q) || !aligned4(out)) return 1;    // rows of 256 floats: 16-byte loads
     const long long blocks = (long long)n_head * ((n_tok + ATT_QPC - 1) / ATT_QPC);
     if (blocks > INT32_MAX) return 1;
+    if (n_tok >= ATC_MIN_TOKENS) {
+        const int rc = launch_attn_tc(q, k, v, out, n_tok, n_head, n_head_kv, scale, as_stream(stream));
+        if (rc >= 0) return rc;
+    }
     static SmemOptIn opt;
     cudaError_t err = opt.ensure(attn_kernel);
     if (err != cudaSuccess) return (int)err;

@@ -243,16 +243,15 @@ __device__ __forceinline__ float transpose_sum32(float (&part)[32], int lane) {
     return part[0];
 }
 
-__global__ void __launch_bounds__(ATT_WARPS * 32) attn_kernel(const float *__restrict__ q, const float *__restrict__ k,
-                                                              const float *__restrict__ v, float *__restrict__ out,
-                                                              int n_tok, int n_head, int n_head_kv, float scale) {
-    extern __shared__ __align__(16) float att_smem[];
+// Queries first .. first + 4 WARPS - 1 of one head, by a CTA of WARPS warps; smem: ATT_SMEM_BYTES, 16-byte aligned.
+template <int WARPS>
+__device__ __forceinline__ void attn_simt(float *att_smem, const float *__restrict__ q, const float *__restrict__ k,
+                                          const float *__restrict__ v, float *__restrict__ out, int first, int head,
+                                          int n_tok, int n_head, int n_head_kv, float scale) {
     float (*kt)[ATT_D] = reinterpret_cast<float (*)[ATT_D]>(att_smem);
     float (*vt)[ATT_D] = reinterpret_cast<float (*)[ATT_D]>(att_smem + ATT_TILE * ATT_D);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int qblocks = (n_tok + ATT_QPC - 1) / ATT_QPC;
-    const int head = blockIdx.x / qblocks, qb = blockIdx.x - head * qblocks;
-    const int q0 = qb * ATT_QPC + ATT_QPW * warp;           // the warp's first query
+    const int q0 = first + ATT_QPW * warp;                  // the warp's first query
     const int kvh = head / (n_head / n_head_kv);
     const int myq = lane >> 3, mykk = lane & 7;             // after the reduction: lane = (query of the warp, key of the group of 8)
     float qreg[ATT_QPW][8], oreg[ATT_QPW][8];
@@ -268,12 +267,12 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attn_kernel(const float *__res
         }
     }
     float m = -INFINITY, l = 0.0f;                          // of query q0 + myq (the same in the 8 lanes of its group)
-    const int last = min(n_tok - 1, qb * ATT_QPC + ATT_QPC - 1);            // keys 0 .. last serve the CTA's queries
+    const int last = min(n_tok - 1, first + WARPS * ATT_QPW - 1);           // keys 0 .. last serve the CTA's queries
     const int wlast = min(n_tok - 1, q0 + ATT_QPW - 1);                     // ... 0 .. wlast this warp's
     for (int j0 = 0; j0 <= last; j0 += ATT_TILE) {
         __syncthreads();
         const int nk = min(ATT_TILE, last + 1 - j0);
-        for (int i = threadIdx.x; i < nk * (ATT_D / 4); i += blockDim.x) {
+        for (int i = threadIdx.x; i < nk * (ATT_D / 4); i += WARPS * 32) {
             const int r = i / (ATT_D / 4), c4 = i - r * (ATT_D / 4);
             const size_t src = ((size_t)(j0 + r) * n_head_kv + kvh) * ATT_D + 4 * c4;
             *reinterpret_cast<float4 *>(&kt[r][4 * c4]) = *reinterpret_cast<const float4 *>(k + src);
@@ -362,6 +361,15 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attn_kernel(const float *__res
             for (int i = 0; i < 8; ++i) op[i] = __fmul_rn(oreg[a][i], inv);
         }
     }
+}
+
+__global__ void __launch_bounds__(ATT_WARPS * 32) attn_kernel(const float *__restrict__ q, const float *__restrict__ k,
+                                                              const float *__restrict__ v, float *__restrict__ out,
+                                                              int n_tok, int n_head, int n_head_kv, float scale) {
+    extern __shared__ __align__(16) float att_smem[];
+    const int qblocks = (n_tok + ATT_QPC - 1) / ATT_QPC;
+    const int head = blockIdx.x / qblocks, qb = blockIdx.x - head * qblocks;
+    attn_simt<ATT_WARPS>(att_smem, q, k, v, out, qb * ATT_QPC, head, n_tok, n_head, n_head_kv, scale);
 }
 
 }  // namespace b200
