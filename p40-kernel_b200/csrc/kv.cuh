@@ -266,7 +266,8 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
         {   // ---- scores of positions 16 warp .. + 15
             const uint32_t *r0 = reinterpret_cast<const uint32_t *>(kt) + (size_t)(16 * warp + g) * (KV_ROW / 4);
             const uint32_t *r1 = r0 + 8 * (KV_ROW / 4);
-            float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};          // (position g | g + 8, head 2 t | 2 t + 1)
+            float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};          // (position g | g + 8, head 2 t | 2 t + 1), even blocks
+            float so[4] = {0.0f, 0.0f, 0.0f, 0.0f};         // odd blocks: two short sums round less than a long one
 #pragma unroll
             for (int pr = 0; pr < 4; ++pr) {
                 const uint32_t *u0 = r0 + 17 * pr, *u1 = r1 + 17 * pr;
@@ -287,11 +288,13 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
                 s[1] = __fmaf_rn(__fmul_rn(qe1, ke0), (float)de[1], s[1]);
                 s[2] = __fmaf_rn(__fmul_rn(qe0, ke1), (float)de[2], s[2]);
                 s[3] = __fmaf_rn(__fmul_rn(qe1, ke1), (float)de[3], s[3]);
-                s[0] = __fmaf_rn(__fmul_rn(qo0, ko0), (float)dq[0], s[0]);
-                s[1] = __fmaf_rn(__fmul_rn(qo1, ko0), (float)dq[1], s[1]);
-                s[2] = __fmaf_rn(__fmul_rn(qo0, ko1), (float)dq[2], s[2]);
-                s[3] = __fmaf_rn(__fmul_rn(qo1, ko1), (float)dq[3], s[3]);
+                so[0] = __fmaf_rn(__fmul_rn(qo0, ko0), (float)dq[0], so[0]);
+                so[1] = __fmaf_rn(__fmul_rn(qo1, ko0), (float)dq[1], so[1]);
+                so[2] = __fmaf_rn(__fmul_rn(qo0, ko1), (float)dq[2], so[2]);
+                so[3] = __fmaf_rn(__fmul_rn(qo1, ko1), (float)dq[3], so[3]);
             }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[e] = __fadd_rn(s[e], so[e]);
             const int pa = 16 * warp + g, pb = pa + 8;
             const bool va = pa < n, vb = pb < n;
             float mx0 = fmaxf(va ? s[0] : -INFINITY, vb ? s[2] : -INFINITY), mx1 = fmaxf(va ? s[1] : -INFINITY, vb ? s[3] : -INFINITY);
@@ -357,9 +360,20 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
                         for (int e = 0; e < 4; ++e) acc[bb][j][e] = __fmul_rn(acc[bb][j][e], keep);
                 }
             }
+            // Two instructions' sums at a time: the tensor core cuts the last bits of a sum off, a rounded addition does not (all of
+            // a split in one accumulator: relative error 3.2e-7 at 32768 positions, 2.6e-7 on the CUDA cores).
+            float sum[2][4][4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 if (16 * c >= n) break;                     // CTA-uniform
+                if ((c & 1) == 0) {
+#pragma unroll
+                    for (int bb = 0; bb < 2; ++bb)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) sum[bb][j][e] = 0.0f;
+                }
                 const uint32_t *rows = v32 + (size_t)(16 * c + 2 * t) * (KV_ROW / 4);
                 uint32_t ev[4], od[4];
                 float de[4], dq[4];
@@ -393,8 +407,16 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
                         uint32_t b0 = __byte_perm(j < 2 ? p01 : q01, 0x64646464u, (j & 1) ? 0x4342 : 0x4140);
                         uint32_t b1 = __byte_perm(j < 2 ? p23 : q23, 0x64646464u, (j & 1) ? 0x4342 : 0x4140);
                         const __half2 v0 = __hsub2(*reinterpret_cast<__half2 *>(&b0), bias), v1 = __hsub2(*reinterpret_cast<__half2 *>(&b1), bias);
-                        mma_f16_16816(acc[bb][j], h01, l01, h23, l23, *reinterpret_cast<const uint32_t *>(&v0), *reinterpret_cast<const uint32_t *>(&v1));
+                        mma_f16_16816(sum[bb][j], h01, l01, h23, l23, *reinterpret_cast<const uint32_t *>(&v0), *reinterpret_cast<const uint32_t *>(&v1));
                     }
+                }
+                if ((c & 1) == 1 || 16 * (c + 1) >= n) {
+#pragma unroll
+                    for (int bb = 0; bb < 2; ++bb)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) acc[bb][j][e] = __fadd_rn(acc[bb][j][e], sum[bb][j][e]);
                 }
             }
         }
