@@ -188,52 +188,38 @@ __device__ __forceinline__ void fwht_slice_back(const float4 *block, int r, int 
     }
 }
 
-// blocks = n_tok * (n_in / 1024) warps.  X [n_tok][n_in] read-only; x_rot (nullable, may alias X)
-// receives the rotated values; xq (nullable) the Q8_1 blocks at chunk * n_tok + tok.
+// One CTA per 1024-block, one warp per slice: n_tok * (n_in / 1024) CTAs.  Bound by latency: a warp that did a whole block
+// alone issued eight times as much in one serial chain (a vector of 5120: 7.2 us against 3.4 us with the launch).  X [n_tok][n_in] read-only;
+// x_rot (nullable, may alias X) receives the rotated values; xq (nullable) the Q8_1 blocks at chunk * n_tok + tok.
+constexpr int FWHT_THREADS = 256;
 template <bool VEC>
-__global__ void __launch_bounds__(128) fwht_quant_kernel(const float *X, const float *signs, float *x_rot,
-                                                         uint32_t *__restrict__ xq, int n_in, int n_tok) {
+__global__ void __launch_bounds__(FWHT_THREADS) fwht_quant_kernel(const float *X, const float *signs, float *x_rot, uint32_t *xq, int n_in, int n_tok) {
+    __shared__ float4 front[FWHT_N / 4];
+    const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
+    const int blocks_per_tok = n_in / FWHT_N;
+    const int tok = (int)blockIdx.x / blocks_per_tok, blk = (int)blockIdx.x - tok * blocks_per_tok;
+    const size_t base = (size_t)tok * n_in + (size_t)blk * FWHT_N + r * 128 + 4 * lane;
     pdl_wait_prior_grid();
     pdl_launch_dependents();
-    const int lane = threadIdx.x & 31;
-    const int blocks_per_tok = n_in / FWHT_N;
-    const long long nwarps = (long long)blocks_per_tok * n_tok;
-    const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (w >= nwarps) return;
-    const int tok = (int)(w / blocks_per_tok);
-    const int blk = (int)(w - (long long)tok * blocks_per_tok);
-    const size_t base = (size_t)tok * n_in + (size_t)blk * FWHT_N;
-
-    float v[8][4];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const float4 f = load_f4<VEC>(X + base + r * 128 + 4 * lane);
-        v[r][0] = f.x; v[r][1] = f.y; v[r][2] = f.z; v[r][3] = f.w;
-    }
+    const float4 f = load_f4<VEC>(X + base);
+    float v[4] = {f.x, f.y, f.z, f.w};
     if (signs) {
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const float4 s = load_f4<VEC>(signs + (size_t)blk * FWHT_N + r * 128 + 4 * lane);
-            v[r][0] = __fmul_rn(v[r][0], s.x); v[r][1] = __fmul_rn(v[r][1], s.y);
-            v[r][2] = __fmul_rn(v[r][2], s.z); v[r][3] = __fmul_rn(v[r][3], s.w);
-        }
+        const float4 s = load_f4<VEC>(signs + (size_t)blk * FWHT_N + r * 128 + 4 * lane);
+        v[0] = __fmul_rn(v[0], s.x); v[1] = __fmul_rn(v[1], s.y);
+        v[2] = __fmul_rn(v[2], s.z); v[3] = __fmul_rn(v[3], s.w);
     }
-    fwht1024_warp(v, lane);
-    if (x_rot) {
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-            store_f4<VEC>(x_rot + base + r * 128 + 4 * lane, make_float4(v[r][0], v[r][1], v[r][2], v[r][3]));
-    }
+    fwht_slice_front(v, lane);
+    front[threadIdx.x] = make_float4(v[0], v[1], v[2], v[3]);
+    __syncthreads();
+    fwht_slice_back(front, r, lane, v);
+    if (x_rot) store_f4<VEC>(x_rot + base, make_float4(v[0], v[1], v[2], v[3]));
     if (xq) {
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            uint32_t word, header;
-            quantise_chunk_8lanes(v[r], lane, word, header);
-            const int chunk = blk * 32 + r * 4 + (lane >> 3);
-            uint32_t *dst = xq + 9 * ((size_t)chunk * n_tok + tok);
-            dst[1 + (lane & 7)] = word;
-            if ((lane & 7) == 0) dst[0] = header;
-        }
+        uint32_t word, header;
+        quantise_chunk_8lanes(v, lane, word, header);
+        const int chunk = blk * 32 + r * 4 + (lane >> 3);
+        uint32_t *dst = xq + 9 * ((size_t)chunk * n_tok + tok);
+        dst[1 + (lane & 7)] = word;
+        if ((lane & 7) == 0) dst[0] = header;
     }
 }
 

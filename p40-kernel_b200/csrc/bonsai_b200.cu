@@ -382,8 +382,9 @@ GemvPlan plan_rows(long long n_out, size_t row_bytes, size_t fixed, int granule,
 
 // Any float pointers are taken, as by the reference; 16-byte aligned ones get 16-byte accesses.
 int launch_fwht(bool vec, const float *x, const float *signs, float *x_rot, void *xq, int64_t n_in, int64_t n_tok, bonsai_stream stream) {
-    const long long warps = (n_in / FWHT_N) * n_tok;
-    return (int)launch(vec ? fwht_quant_kernel<true> : fwht_quant_kernel<false>, dim3((unsigned)((warps + 3) / 4)), dim3(128), 0, as_stream(stream), true,
+    const long long blocks = (n_in / FWHT_N) * n_tok;
+    if (blocks > INT32_MAX) return 1;
+    return (int)launch(vec ? fwht_quant_kernel<true> : fwht_quant_kernel<false>, dim3((unsigned)blocks), dim3(FWHT_THREADS), 0, as_stream(stream), true,
                        x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
 }
 
@@ -1486,8 +1487,8 @@ inline int64_t kv_gdn_bytes() { return (int64_t)KVM_LINEAR * KVM_V_HEADS * KVM_S
 constexpr int KV_COUNTERS = KVM_KV_HEADS * KV_CLUSTER;      // per layer
 inline size_t kv_ws_floats(int max_clusters) { return (size_t)KVM_KV_HEADS * KV_CLUSTER * max_clusters * KV_REC; }      // per layer
 
-// Clusters of the decode kernel per kv head that are resident at once on the current device (0: it does not run here).  The
-// query takes milliseconds, so it is made once per device.
+// Clusters of the decode kernel per kv head that are resident at once on the current device (0: it does not run here).  Asked
+// once per device.
 int kv_max_clusters() {
     static std::atomic<int> known[64];
     static SmemOptIn opt;

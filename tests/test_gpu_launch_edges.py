@@ -1,0 +1,97 @@
+"""Launches that start before their predecessor ends, and work cut into parts: what a call reads must be what the call in
+front of it wrote (weights included), and the parts of a tile must add up wherever the cuts fall."""
+import numpy as np
+import pytest
+
+from bonsai_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+REL_TOL = 1e-5      # the mat-vec's and mat-mul's bound: max |got - want| <= REL_TOL * max |want|
+
+
+def dev(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+@pytest.mark.parametrize("n_out,n_in", [(64, 1024), (1024, 5120), (5120, 17408)])
+def test_calls_read_what_the_call_before_wrote(gpu, n_out, n_in):
+    """Weights, inputs and scratch are written again between the calls, by a copy, by the library's own kernels and by the
+    call in front; every result has the bits of the same call made alone."""
+    import torch
+    Ws = [dev(synth.pq2_0_weights(n_out, n_in, seed=s)) for s in range(2)]
+    xs = [dev(synth.activations(n_in, seed=s)) for s in range(3)]
+    sg = dev(synth.signs(n_in, seed=1))
+    xq = torch.empty(n_in // 32 * 36, dtype=torch.uint8, device="cuda")
+    rot = torch.empty(n_in, device="cuda")
+    W, R, y = torch.empty_like(Ws[0]), torch.empty_like(Ws[0]), torch.empty(n_out, device="cuda")
+
+    def step(i, sync):
+        wait = torch.cuda.synchronize if sync else (lambda: None)
+        out = []
+        W.copy_(Ws[i % 2]); wait()
+        assert gpu.linear(W, xs[i % 3], sg, y, xq, n_out, n_in) == 0; wait()
+        out.append(y.clone()); wait()
+        assert gpu.repack(W, R, n_out, n_in) == 0; wait()
+        assert gpu.gemv_repack(R, rot, y, n_out, n_in) == 0; wait()     # rot: of the step before
+        out.append(y.clone()); wait()
+        assert gpu.fwht_quant(xs[(i + 1) % 3], sg, xq, rot, n_in) == 0; wait()
+        assert gpu.gemv(W, xq, y, n_out, n_in) == 0; wait()
+        out.append(y.clone()); wait()
+        assert gpu.gemv_repack(R, rot, y, n_out, n_in) == 0; wait()
+        out.append(y.clone()); wait()
+        assert gpu.synth_pq2_0(W, 0, n_out * (n_in // 128), 7 + i) == 0; wait()
+        assert gpu.gemv(W, xq, y, n_out, n_in) == 0; wait()
+        out.append(y.clone()); wait()
+        assert gpu.quant_activations(rot, xq, n_in) == 0; wait()
+        assert gpu.gemv(W, xq, y, n_out, n_in) == 0; wait()
+        out.append(y.clone()); wait()
+        return out
+
+    rot.copy_(xs[0])
+    want = [step(i, True) for i in range(6)]
+    rot.copy_(xs[0])
+    got = [step(i, False) for i in range(6)]
+    torch.cuda.synchronize()
+    for i in range(6):
+        for a, b in zip(want[i], got[i]):
+            assert torch.equal(a, b), i
+    assert gpu.device_status() == 0
+
+
+@pytest.mark.parametrize("n_out,n_in,n_tok", [
+    (128, 17408, 17), (129, 17408, 64), (5120, 17408, 37), (1000, 5120, 33), (2000, 17408, 95), (300, 17408, 96), (1030, 9216, 130), (6000, 5120, 257)])
+def test_parts_of_a_tile_add_up(gpu, port, n_out, n_in, n_tok):
+    """Tiles of the many-token mat-mul in one, two, three and four parts, on both tile widths."""
+    import torch
+    W = synth.pq2_0_weights(n_out, n_in, seed=n_tok)
+    Xq = port.quantize_batch_chunk_major(synth.activations(n_in, seed=n_out, batch=n_tok))
+    Wd, Xd = dev(W), dev(Xq)
+    Y = [torch.full((n_out, n_tok), float("nan"), device="cuda") for _ in range(2)]
+    for y in Y:
+        assert gpu.gemm(Wd, Xd, y, n_out, n_in, n_tok) == 0
+    assert torch.equal(Y[0], Y[1])
+    rows = np.unique(np.concatenate([np.arange(min(n_out, 64)), np.arange(max(0, n_out - 64), n_out), np.linspace(0, n_out - 1, 64).astype(np.int64)]))
+    row_bytes = n_in // 128 * 34
+    want = port.gemm(np.concatenate([W[r * row_bytes:(r + 1) * row_bytes] for r in rows]), Xq, len(rows), n_in, n_tok, threads=8)
+    err = np.abs(Y[0].cpu().numpy()[rows] - want).max()
+    assert err <= REL_TOL * np.abs(want).max(), (err, np.abs(want).max())
+    assert gpu.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [124, 128, 8188, 8189, 8192, 8193, 8196, 65537])
+def test_rmsnorm_rows_held_and_not(gpu, port, n):
+    """Rows on both sides of what a CTA keeps in registers (8192), in place and not, with 16-byte accesses and without."""
+    import torch
+    rng = np.random.default_rng(n)
+    x, w = rng.uniform(-2, 2, size=(3, n)).astype(np.float32), rng.uniform(0.5, 1.5, size=n).astype(np.float32)
+    want = port.rmsnorm(x, w, 1e-6)
+    y, xd, wd = torch.empty(3, n, device="cuda"), dev(x), dev(w)
+    assert gpu.rmsnorm(xd, wd, y, 3, n, 1e-6) == 0
+    assert np.abs(y.cpu().numpy() - want).max() <= REL_TOL * np.abs(want).max()
+    odd = torch.empty(3 * n + 1, device="cuda")[1:]
+    assert gpu.rmsnorm(xd, wd, odd, 3, n, 1e-6) == 0
+    assert torch.equal(odd.view(3, n), y)
+    assert gpu.rmsnorm(xd, wd, xd, 3, n, 1e-6) == 0
+    assert torch.equal(xd, y)
