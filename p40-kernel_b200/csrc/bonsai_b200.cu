@@ -1001,6 +1001,12 @@ static void fill_tc_params(TcParams &P, int64_t n_out, int64_t n_in, int64_t n_t
     P.total_it = (long long)P.n_tiles * P.nblocks;
 }
 
+// Scratch of the fp16 mat-mul: a slot per CTA for its part of a tile, the two planes, a scale per token.
+static constexpr size_t T16_PARTS_BYTES = (size_t)TC_MAX_CTAS * T16C<128>::PART_FLOATS * sizeof(float);
+static size_t tc16_scratch_bytes(int64_t n_in, int64_t n_tok) {
+    return T16_PARTS_BYTES + 2 * (size_t)n_tok * (size_t)n_in * sizeof(__half) + (size_t)n_tok * sizeof(float);
+}
+
 // The fp16 tensor-core mat-mul (gemm_tc16.cuh).  -1: not taken (shape, alignment, no scratch, no tensor-map encoder).
 extern "C++" {
 template <int TN>
@@ -1011,11 +1017,11 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     const long long tiles = (long long)((n_out + T16_M - 1) / T16_M) * ((n_tok + T16_N - 1) / T16_N);
     if (tiles > INT32_MAX) return -1;
     const size_t plane_bytes = (size_t)n_tok * (size_t)n_in * sizeof(__half);
-    const size_t bytes = 2 * plane_bytes + 2 * (size_t)n_tok * sizeof(float);
-    uint8_t *ws = static_cast<uint8_t *>(gemm_scratch(bytes, st));
+    uint8_t *ws = static_cast<uint8_t *>(gemm_scratch(tc16_scratch_bytes(n_in, n_tok), st));
     if (!ws) return -1;
-    __half *planes = reinterpret_cast<__half *>(ws);
-    float *scale = reinterpret_cast<float *>(ws + 2 * plane_bytes);
+    float *parts = reinterpret_cast<float *>(ws);
+    __half *planes = reinterpret_cast<__half *>(ws + T16_PARTS_BYTES);
+    float *scale = reinterpret_cast<float *>(ws + T16_PARTS_BYTES + 2 * plane_bytes);
     alignas(64) Tc16Maps maps;
     std::memset(&maps, 0, sizeof(maps));
     if (!encode_w_map(&maps.w, W, n_out, nblocks * W_BLOCK_BYTES)) return -1;
@@ -1028,8 +1034,7 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     if (e != cudaSuccess) return (int)e;
     if (sms > TC_MAX_CTAS - 1) sms = TC_MAX_CTAS - 1;
     // Tiles for at most half of the SMs (a short token batch over few rows): up to four CTAs share a tile's blocks, at least 16
-    // blocks each.  A CTA whose whole range lies inside one tile is both a "late" and an "early" part: it waits for
-    // the part behind it, adds, stores, and raises its own flag -- the sums reach the tile's first CTA along the chain.
+    // blocks each.
     int grid = (int)(tiles < sms ? tiles : sms);
     if (2 * tiles <= sms) {
         long long g = P.total_it / 16;
@@ -1062,7 +1067,7 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN>, Y, P, (const float *)scale, maps);
+    return (int)cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN>, Y, P, (const float *)scale, parts, maps);
 }
 }  // extern "C++"
 // Tiles of 128 tokens from 96 tokens on (the code expansion, the kernel's busiest part, is paid once per tile), of 64 below.
@@ -1205,8 +1210,7 @@ int bonsai_b200_gemm_release(void) {
 
 int bonsai_b200_gemm_reserve(int64_t n_in, int64_t n_tok, bonsai_stream stream) {
     if (n_in <= 0 || n_in % 128 != 0 || n_tok <= 0 || n_tok > (1 << 28)) return 1;
-    const size_t bytes = 2 * (size_t)n_tok * (size_t)n_in * sizeof(__half) + 2 * (size_t)n_tok * sizeof(float);
-    return gemm_scratch(bytes, as_stream(stream)) ? 0 : (int)cudaErrorMemoryAllocation;
+    return gemm_scratch(tc16_scratch_bytes(n_in, n_tok), as_stream(stream)) ? 0 : (int)cudaErrorMemoryAllocation;
 }
 
 int bonsai_b200_gemm_dump(const void *W, const void *Xq, float *Y, int32_t *sums, int64_t n_out, int64_t n_in,
