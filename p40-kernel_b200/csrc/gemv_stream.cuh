@@ -270,7 +270,42 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
     pdl_wait_prior_grid();              // activations (and y) belong to the previous kernel until here
     pdl_launch_dependents();            // behind the wait: whatever starts now has only this launch to wait for
     const int first_late = P.early ? min(2, first_fill) : 0;
-    if (FUSED) {
+    if (REPACK) {
+        // quantiser without rotation: 128-element slices over the compute warps, SLICES at a time so that their loads fly
+        // together (whole 1024-blocks left most warps without work: 1024 x 64 5.1 -> 2.7 us,
+        // 5120 x 5120 6.9 -> 5.2 us, 17408 x 5120 15.0 -> 13.1 us)
+        constexpr int SLICES = 5;
+        bool first = true;
+        for (int s0 = wid; s0 < P.nb || first; s0 += SLICES * compute_warps) {
+            float4 f[SLICES];
+#pragma unroll
+            for (int k = 0; k < SLICES; ++k) {
+                const int sl = s0 + k * compute_warps;
+                f[k] = wid < compute_warps && sl < P.nb ? *reinterpret_cast<const float4 *>(x + (size_t)sl * 128 + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            if (first) {
+                // every warp has issued its first loads: the rest of the ring may queue behind them
+                __syncthreads();
+                if (wid == compute_warps && lane == 0)
+                    for (int t = first_late; t < first_fill; ++t) issue_tile(t);
+                first = false;
+            }
+#pragma unroll
+            for (int k = 0; k < SLICES; ++k) {
+                const int sl = s0 + k * compute_warps;
+                if (wid >= compute_warps || sl >= P.nb) break;          // warp-uniform
+                const float v[4] = {f[k].x, f[k].y, f[k].z, f[k].w};
+                uint32_t word, header;
+                quantise_chunk_8lanes(v, lane, word, header);
+                const int chunk = 4 * sl + (lane >> 3);
+                act_q[sl * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word;
+                if ((lane & 7) == 0) {
+                    act_s[chunk] = f16_bits_to_f32(header & 0xFFFFu);
+                    act_i[chunk] = -64 * (int)(short)(header >> 16);
+                }
+            }
+        }
+    } else if (FUSED) {
         // rotation + quantiser in the prologue: nb / 8 blocks of 1024 activations over the compute warps
         const int nfb = P.nb >> 3;
         bool first = true;
@@ -293,7 +328,7 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
                 first = false;
             }
             if (live) {
-                if (!REPACK && signs) {
+                if (signs) {
 #pragma unroll
                     for (int r = 0; r < 8; ++r) {
                         const float4 sg = *reinterpret_cast<const float4 *>(signs + (size_t)fb * FWHT_N + r * 128 + 4 * lane);
@@ -301,7 +336,7 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
                         v[r][2] = __fmul_rn(v[r][2], sg.z); v[r][3] = __fmul_rn(v[r][3], sg.w);
                     }
                 }
-                if (!REPACK) fwht1024_warp(v, lane);
+                fwht1024_warp(v, lane);
 #pragma unroll
                 for (int r = 0; r < 8; ++r) {
                     uint32_t word, header;
