@@ -22,8 +22,8 @@
 //   warps 8-23  : code producers: thread (row p, K half g), every second block: 64 two-bit codes -> 64 fp16 with byte
 //                 permutes (the fp16 patterns of -1, 0, 1, 2 differ only in their high byte), written to tensor memory
 //   warps 24-25 : issuers (alternate blocks)
-//   warps 26-27 : loaders (tiled TMA copies): weight pieces of 8 blocks x 128 rows; per block two boxes of 64 values x
-//                 64 tokens x {H, L}, landing swizzled as the MMA reads them
+//   warps 26-27 : loaders (tiled TMA copies): weight pieces of 8 blocks x 128 rows; per half block a box of 64 values x
+//                 64 tokens x {H, L}, landing swizzled as the MMA reads it
 // Work split and time-outs as in gemm_tc.cuh (same walk, same flag words); the parts of a tile meet in one step, through slots
 // in the scratch.
 // Every role that feeds the tensor core is a serial chain per block, and each in turn was the kernel's period until it
@@ -62,8 +62,11 @@ struct T16C {
     static constexpr int EPI_THREADS = EPI_WARPS * 32, PROD_THREADS = PROD_WARPS * 32;
     static constexpr int THREADS = EPI_THREADS + PROD_THREADS + 32 * (T16_ISSUERS + 2);      // + two loader warps
     static constexpr int BUNIT = TN * 256;                                  // B bytes of one K half: {H, L} x TN tokens x 128 bytes
-    static constexpr int NB = (128 * 1024) / (2 * BUNIT);                   // B ring: whole blocks, 128 KB in all
-    static constexpr int SMEM_BYTES = 2048 + NB * 2 * BUNIT + T16_DWRING * T16_M * 4 + T16_WBUFS * TC_WRAW_BYTES;
+    // A slot of the B ring (128 KB in all) is a K half of a block at 128 tokens, where a block would be half of the ring (512 tokens
+    // 217 -> 210 us), and a whole block at 64 (halves: 37 tokens 56 -> 58 us).
+    static constexpr int SLOT_HALVES = TN == 128 ? 1 : 2;
+    static constexpr int NB = (128 * 1024) / (SLOT_HALVES * BUNIT);
+    static constexpr int SMEM_BYTES = 2048 + NB * SLOT_HALVES * BUNIT + T16_DWRING * T16_M * 4 + T16_WBUFS * TC_WRAW_BYTES;
     // instruction descriptor: D = fp32, A and B fp16, both K-major, N = TN, M = 128
     static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(T16_M >> 4) << 24);
 };
@@ -234,9 +237,9 @@ __global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *
     using C = T16C<TN>;
     constexpr int T16_N = TN, T16_ACC = C::ACC, T16_NB = C::NB, T16_BUNIT = C::BUNIT, T16_EPI_WARPS = C::EPI_WARPS,
                   T16_PROD_WARPS = C::PROD_WARPS, T16_PROD_SETS = C::PROD_SETS, T16_EPI_THREADS = C::EPI_THREADS,
-                  T16_PROD_THREADS = C::PROD_THREADS, T16_EPI_TOKS = 32, T16_PART_FLOATS = C::PART_FLOATS;
+                  T16_PROD_THREADS = C::PROD_THREADS, T16_EPI_TOKS = 32, T16_PART_FLOATS = C::PART_FLOATS, T16_SLOT = C::SLOT_HALVES;
     extern __shared__ __align__(128) uint8_t smem[];
-    // unit u = 2 * block + K half lives in slot u % NA of the code ring and slot u % NB of the activation ring
+    // unit u = 2 * block + K half lives in slot u % NA of the code ring and slot (u / SLOT_HALVES) % NB of the activation ring
     uint64_t *afull = reinterpret_cast<uint64_t *>(smem);              // [NA] code producers -> issuer
     uint64_t *afree = afull + T16_NA;                                   // [NA] tensor core -> code producers
     uint64_t *bfull = afree + T16_NA;                                   // [NB] loader (bytes landed) -> issuer
@@ -248,7 +251,7 @@ __global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(wfree + T16_WBUFS);
     uint8_t *stages = smem + 1024 + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
     uint8_t *bring = stages;
-    float *dwring = reinterpret_cast<float *>(bring + T16_NB * 2 * T16_BUNIT);
+    float *dwring = reinterpret_cast<float *>(bring + T16_NB * T16_SLOT * T16_BUNIT);
     uint8_t *wraw = reinterpret_cast<uint8_t *>(dwring + T16_DWRING * T16_M);
 
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -447,21 +450,25 @@ __global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *
             }
         }
     } else if (wid == LOADER + 1) {
-        // ---------------- activation loader: a block's boxes (two copies of 64 values x 64 tokens x {H, L}) ----------------
+        // ---------------- activation loader: boxes of 64 values x TN tokens x {H, L}, a slot as soon as it is free ----------------
         int n = 0;
         bool ok = true;
         while (ok && walk.next(P, tile, kb0, kb1)) {
             const int tt = tile % P.tiles_tok;
             for (int kb = kb0; kb < kb1; ++kb, ++n) {
-                const int sb = n % T16_NB;
-                if (!mbar_wait_bounded(&bfree[sb], (uint32_t)(((n / T16_NB) & 1) ^ 1), 20, 80)) { ok = false; break; }
-                if (elect_one()) {
-                    uint8_t *b = bring + (size_t)sb * (2 * T16_BUNIT);
-                    mbar_expect_tx(&bfull[sb], (uint32_t)(2 * T16_BUNIT));
-                    tma_load_3d(b, &maps.x, kb * 128, tt * T16_N, 0, &bfull[sb]);
-                    tma_load_3d(b + T16_BUNIT, &maps.x, kb * 128 + 64, tt * T16_N, 0, &bfull[sb]);
+#pragma unroll
+                for (int g = 0; g < 2; g += T16_SLOT) {
+                    const int w = (2 * n + g) / T16_SLOT, sb = w % T16_NB;
+                    if (!mbar_wait_bounded(&bfree[sb], (uint32_t)(((w / T16_NB) & 1) ^ 1), 20, 80)) { ok = false; break; }
+                    if (elect_one()) {
+                        uint8_t *b = bring + (size_t)sb * (T16_SLOT * T16_BUNIT);
+                        mbar_expect_tx(&bfull[sb], (uint32_t)(T16_SLOT * T16_BUNIT));
+#pragma unroll
+                        for (int h = 0; h < T16_SLOT; ++h) tma_load_3d(b + h * T16_BUNIT, &maps.x, kb * 128 + 64 * (g + h), tt * T16_N, 0, &bfull[sb]);
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
+                if (!ok) break;
             }
         }
     } else {
@@ -483,13 +490,13 @@ __global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *
                 // units are there, and the units are handed back as soon as the MMAs have read them.
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
-                    const int u = 2 * n + g, sa = u % T16_NA, sb = n % T16_NB;
+                    const int u = 2 * n + g, sa = u % T16_NA, w = u / T16_SLOT, sb = w % T16_NB;
                     if (!mbar_wait_hot(&afull[sa], (uint32_t)((u / T16_NA) & 1))) { ok = false; break; }
-                    if (g == 0 && (!mbar_wait_hot(&bfull[sb], (uint32_t)((n / T16_NB) & 1)) ||
-                                   !mbar_wait_hot(&tmem_empty[t], (uint32_t)(((n / T16_ACC) & 1) ^ 1)))) { ok = false; break; }
+                    if (g % T16_SLOT == 0 && !mbar_wait_hot(&bfull[sb], (uint32_t)((w / T16_NB) & 1))) { ok = false; break; }
+                    if (g == 0 && !mbar_wait_hot(&tmem_empty[t], (uint32_t)(((n / T16_ACC) & 1) ^ 1))) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_t = tmem_base + (uint32_t)(T16_A_COL0 + sa * T16_A_UNIT_COLS);
-                    const uint32_t b_lo = tc16_desc_lo(smem_u32(bring + (size_t)(2 * sb + g) * T16_BUNIT));
+                    const uint32_t b_lo = tc16_desc_lo(smem_u32(bring + (size_t)(T16_SLOT * sb + g % T16_SLOT) * T16_BUNIT));
                     if (elect_one()) {
 #pragma unroll
                         for (int m = 0; m < 8; ++m) {
@@ -498,10 +505,8 @@ __global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *
                             else tc_mma_f16_ts<true>(d, a_t + (uint32_t)(8 * i), b_lo + (uint32_t)(pl * ((T16_N * 128) >> 4) + 2 * i), C::IDESC);
                         }
                         tc_commit(&afree[sa]);
-                        if (g == 1) {
-                            tc_commit(&bfree[sb]);
-                            tc_commit(&mma_done[t]);
-                        }
+                        if (g % T16_SLOT == T16_SLOT - 1) tc_commit(&bfree[sb]);
+                        if (g == 1) tc_commit(&mma_done[t]);
                     }
                     __syncwarp();
                 }
