@@ -1471,10 +1471,12 @@ int bonsai_p40_attn(const float *q, const float *k, const float *v, float *out, 
         const int rc = launch_attn_tc(q, k, v, out, n_tok, n_head, n_head_kv, scale, as_stream(stream));
         if (rc >= 0) return rc;
     }
-    static SmemOptIn opt;
-    cudaError_t err = opt.ensure(attn_kernel);
+    static SmemOptIn opt1, opt2;
+    const bool two = blocks > SM_COUNT;
+    auto kernel = two ? attn_kernel<true> : attn_kernel<false>;
+    cudaError_t err = (two ? opt2 : opt1).ensure(kernel);
     if (err != cudaSuccess) return (int)err;
-    attn_kernel<<<(unsigned)blocks, ATT_WARPS * 32, ATT_SMEM_BYTES, as_stream(stream)>>>(q, k, v, out, n_tok, n_head, n_head_kv, scale);
+    kernel<<<(unsigned)blocks, ATT_WARPS * 32, ATT_SMEM_BYTES, as_stream(stream)>>>(q, k, v, out, n_tok, n_head, n_head_kv, scale);
     return (int)cudaGetLastError();
 }
 

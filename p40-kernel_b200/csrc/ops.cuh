@@ -228,6 +228,21 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_step_kernel(float *state, 
 constexpr int ATT_D = 256, ATT_TILE = 32, ATT_WARPS = 8, ATT_QPW = 4, ATT_QPC = ATT_WARPS * ATT_QPW;
 constexpr int ATT_SMEM_BYTES = 2 * ATT_TILE * ATT_D * 4;
 
+// Two fp32 multiply-adds in one instruction (each rounded as __fmaf_rn): half of the kernel's issue slots were multiply-adds.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t"
+        ".reg .b64 a, b, c, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 b, {%4, %5};\n\t"
+        "mov.b64 c, {%6, %7};\n\t"
+        "fma.rn.f32x2 d, a, b, c;\n\t"
+        "mov.b64 {%0, %1}, d;\n\t"
+        "}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
 // part[r] of every lane -> returned value of lane r = sum over the lanes of part[r] (r = 0 .. 31).
 __device__ __forceinline__ float transpose_sum32(float (&part)[32], int lane) {
 #pragma unroll
@@ -254,16 +269,16 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *__restri
     const int q0 = first + ATT_QPW * warp;                  // the warp's first query
     const int kvh = head / (n_head / n_head_kv);
     const int myq = lane >> 3, mykk = lane & 7;             // after the reduction: lane = (query of the warp, key of the group of 8)
-    float qreg[ATT_QPW][8], oreg[ATT_QPW][8];
+    float2 qreg[ATT_QPW][4], oreg[ATT_QPW][4];              // pairs of neighbouring dims
 #pragma unroll
     for (int a = 0; a < ATT_QPW; ++a) {
         const int qi = q0 + a;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { qreg[a][i] = 0.0f; oreg[a][i] = 0.0f; }
+        for (int i = 0; i < 4; ++i) qreg[a][i] = oreg[a][i] = make_float2(0.0f, 0.0f);
         if (qi < n_tok) {
             const float *qp = q + ((size_t)qi * n_head + head) * ATT_D + 8 * lane;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) qreg[a][i] = __fmul_rn(qp[i], scale);
+            for (int i = 0; i < 4; ++i) qreg[a][i] = make_float2(__fmul_rn(qp[2 * i], scale), __fmul_rn(qp[2 * i + 1], scale));
         }
     }
     float m = -INFINITY, l = 0.0f;                          // of query q0 + myq (the same in the 8 lanes of its group)
@@ -294,11 +309,11 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *__restri
                     const float4 kb = *reinterpret_cast<const float4 *>(&kt[r][8 * lane + 4]);
 #pragma unroll
                     for (int a = 0; a < ATT_QPW; ++a) {
-                        float pr = __fmul_rn(qreg[a][0], ka.x);
-                        pr = __fmaf_rn(qreg[a][1], ka.y, pr); pr = __fmaf_rn(qreg[a][2], ka.z, pr); pr = __fmaf_rn(qreg[a][3], ka.w, pr);
-                        pr = __fmaf_rn(qreg[a][4], kb.x, pr); pr = __fmaf_rn(qreg[a][5], kb.y, pr); pr = __fmaf_rn(qreg[a][6], kb.z, pr);
-                        pr = __fmaf_rn(qreg[a][7], kb.w, pr);
-                        part[8 * a + kk] = pr;
+                        float2 pr = make_float2(__fmul_rn(qreg[a][0].x, ka.x), __fmul_rn(qreg[a][0].y, ka.y));
+                        pr = fma2(qreg[a][1], make_float2(ka.z, ka.w), pr);
+                        pr = fma2(qreg[a][2], make_float2(kb.x, kb.y), pr);
+                        pr = fma2(qreg[a][3], make_float2(kb.z, kb.w), pr);
+                        part[8 * a + kk] = __fadd_rn(pr.x, pr.y);
                     }
                 }
                 const float s = transpose_sum32(part, lane);            // lane (myq, mykk): score of key j0 + 8 st + mykk
@@ -326,7 +341,7 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *__restri
         for (int a = 0; a < ATT_QPW; ++a) {
             const float al = __shfl_sync(0xffffffffu, alpha, 8 * a);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) oreg[a][i] = __fmul_rn(oreg[a][i], al);
+            for (int i = 0; i < 4; ++i) oreg[a][i] = make_float2(__fmul_rn(oreg[a][i].x, al), __fmul_rn(oreg[a][i].y, al));
         }
 #pragma unroll
         for (int st = 0; st < 4; ++st) {
@@ -340,10 +355,11 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *__restri
 #pragma unroll
                         for (int a = 0; a < ATT_QPW; ++a) {
                             const float pr = __shfl_sync(0xffffffffu, p[st], 8 * a + kk);
-                            oreg[a][0] = __fmaf_rn(pr, va.x, oreg[a][0]); oreg[a][1] = __fmaf_rn(pr, va.y, oreg[a][1]);
-                            oreg[a][2] = __fmaf_rn(pr, va.z, oreg[a][2]); oreg[a][3] = __fmaf_rn(pr, va.w, oreg[a][3]);
-                            oreg[a][4] = __fmaf_rn(pr, vb.x, oreg[a][4]); oreg[a][5] = __fmaf_rn(pr, vb.y, oreg[a][5]);
-                            oreg[a][6] = __fmaf_rn(pr, vb.z, oreg[a][6]); oreg[a][7] = __fmaf_rn(pr, vb.w, oreg[a][7]);
+                            const float2 pp = make_float2(pr, pr);
+                            oreg[a][0] = fma2(pp, make_float2(va.x, va.y), oreg[a][0]);
+                            oreg[a][1] = fma2(pp, make_float2(va.z, va.w), oreg[a][1]);
+                            oreg[a][2] = fma2(pp, make_float2(vb.x, vb.y), oreg[a][2]);
+                            oreg[a][3] = fma2(pp, make_float2(vb.z, vb.w), oreg[a][3]);
                         }
                     }
                 }
@@ -358,17 +374,25 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *__restri
             const float inv = __fdiv_rn(1.0f, la);
             float *op = out + ((size_t)qi * n_head + head) * ATT_D + 8 * lane;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) op[i] = __fmul_rn(oreg[a][i], inv);
+            for (int i = 0; i < 4; ++i) {
+                op[2 * i] = __fmul_rn(oreg[a][i].x, inv);
+                op[2 * i + 1] = __fmul_rn(oreg[a][i].y, inv);
+            }
         }
     }
 }
 
-__global__ void __launch_bounds__(ATT_WARPS * 32) attn_kernel(const float *__restrict__ q, const float *__restrict__ k,
+// TWO: two CTAs per SM (128 registers, a few spilled); without it one, for calls whose CTAs do not fill the SMs once (128 tokens
+// of 24 heads: 34 us, 37 us with TWO).  Bound by issue: with packed multiply-adds and the longest rows first 511 tokens took
+// 186 us instead of 232 us, 340 tokens 102 instead of 123 us.
+template <bool TWO>
+__global__ void __launch_bounds__(ATT_WARPS * 32, TWO ? 2 : 1) attn_kernel(const float *__restrict__ q, const float *__restrict__ k,
                                                               const float *__restrict__ v, float *__restrict__ out,
                                                               int n_tok, int n_head, int n_head_kv, float scale) {
     extern __shared__ __align__(16) float att_smem[];
+    // the longest rows of keys first: what starts last is short
     const int qblocks = (n_tok + ATT_QPC - 1) / ATT_QPC;
-    const int head = blockIdx.x / qblocks, qb = blockIdx.x - head * qblocks;
+    const int head = (int)blockIdx.x % n_head, qb = qblocks - 1 - (int)blockIdx.x / n_head;
     attn_simt<ATT_WARPS>(att_smem, q, k, v, out, qb * ATT_QPC, head, n_tok, n_head, n_head_kv, scale);
 }
 
