@@ -90,8 +90,10 @@ int bonsai_b200_gemm_dump(const void *W, const void *Xq, float *Y, int32_t *sums
  * 0, 1 for bad arguments, cudaErrorMemoryAllocation (2) when the buffer cannot be had.  No reference counterpart. */
 int bonsai_b200_gemm_reserve(int64_t n_in, int64_t n_tok, bonsai_stream stream);
 
-/* Frees every scratch buffer of bonsai_p40_gemm (all devices, all streams); they are otherwise kept for the life of the
- * process.  No mat-mul of this library may be in flight or captured in a graph that will still be replayed.  Returns 0. */
+/* Frees every scratch buffer of bonsai_p40_gemm and of bonsai_p40_attn (all devices, all streams); they are otherwise kept
+ * for the life of the process.  (Attention of 512 tokens and more keeps 2 KB per position and kv head for each of at most 16
+ * streams of a device; a stream under capture gets none and runs the kernel that needs none.)  No mat-mul of this library may
+ * be in flight or captured in a graph that will still be replayed.  Returns 0. */
 int bonsai_b200_gemm_release(void);
 
 /* PTQ1_0: the denser packing of the same ternary weights, 28 bytes per 128 weights instead of 34 (described, not
@@ -116,9 +118,10 @@ int bonsai_b200_synth_pq2_0(void *W, int64_t first_block, int64_t n_blocks, uint
  * B200 counterpart of the reference's tools/bwtest.cu:37-90. */
 int bonsai_b200_stream_probe(const void *buf, int64_t bytes, int mode, void *sink, bonsai_stream stream);
 
-/* Launch options.  key "pdl": 1 = launch the mat-vec with programmatic stream serialisation,
- * so that its weight stream starts while the previous kernel of the stream drains (weights
- * must not be written by that previous kernel); 0 = plain launches (default).
+/* Launch options.  key "pdl": 1 = the weight stream of every mat-vec starts while the previous
+ * kernel of the stream drains (weights must not be written by that previous kernel); 0 (default) =
+ * only where the previous kernel is this library's own quantiser.  Launches overlap either way, and
+ * wait for the previous kernel before they read what it may have written.
  * key "gemv_order": 0 (default) = the streaming mat-vec, whose fp32 terms equal the host's bit for
  * bit and are added in a fixed tree order (outputs within 1e-5 of the host's, identical from launch
  * to launch); 1 = the mat-vec that also adds them in the host's sequential order (outputs
@@ -131,8 +134,9 @@ int bonsai_b200_stream_probe(const void *buf, int64_t bytes, int mode, void *sin
  * bit-identical to the host loop), 1 = tensor cores (the fp16 form, csrc/gemm_tc16.cuh, where it takes the call,
  * else the integer form), 2 = the small-batch kernel where it takes the shape, 3 = the integer tensor-core kernel
  * (csrc/gemm_tc.cuh: forms the host's int32 chunk sums, needs no scratch).  1, 2 and 3 hold fp32 Y to 1e-5 of
- * max |Y|.  The fp16 form keeps one scratch buffer per (device, stream), 4 bytes per token and input value, allocated
- * with cudaMalloc on first use or growth -- never while the stream is being captured (then the integer form runs).
+ * max |Y|.  The fp16 form keeps one scratch buffer per (device, stream), 4 bytes per token and input value, and 16 MB for
+ * the parts of tiles, allocated with cudaMalloc on first use or growth -- never while the stream is being captured (then the
+ * integer form runs).
  * key "fuse_linear": 0 (default) = bonsai_b200_linear is two launches, 1 = one kernel when it can (saves a
  * launch, but every CTA then waits for its own rotation before its first multiply: measured ~6 % slower
  * on the 401-projection decode chain).
