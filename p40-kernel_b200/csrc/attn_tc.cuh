@@ -3,7 +3,7 @@
 // attn_kernel (ops.cuh) multiplies on the CUDA cores and is bound by their issue slots and by shared memory.  Here both
 // products run on the tensor cores without giving up fp32: every operand is scaled by a power of two (q and k per row, v per
 // output dim and tile, softmax weights by 2^14) and split into two fp16 planes, high and low, 22 - 24 bits together; what
-// the low plane cannot hold is below 2^-39 of the row's largest value.  The tensor core cuts the last bits of a sum off
+// the low plane cannot hold is below 2^-39 of the largest value under the same power of two.  The tensor core cuts the last bits of a sum off
 // instead of rounding it, so sums are kept short: a score is six sums over 32 or 48 dims (an accumulator over all 256 was 1.5
 // to 3 times less exact than the CUDA cores), joined by rounded additions, and a tile's weights x v go to a fresh accumulator
 // that the CUDA cores add to the fp32 output.  Error against 64 bits: at
@@ -24,8 +24,9 @@
 // the q rows from shared memory), the rest softmax and the exchanges in front of it.  2048 tokens, 24 heads over 4: 2570 ->
 // 293 us; 1000 tokens 727 -> 94 us, 517 tokens 246 -> 59 us.
 //
-// Infinities, NaN and values past 2^60 do not survive the split; a CTA that meets one does its queries again on the CUDA
-// cores (attn_simt), with that kernel's results.
+// A plane pair holds 2^-39 of the largest value under its power of two, so what is far smaller loses bits to values that a row may not
+// even see.  A CTA whose queries and keys range too widely (atc_too_wide) does its queries again on the CUDA cores (attn_simt), with
+// that kernel's results; so does one that meets an infinity, NaN or a value past 2^60.
 #pragma once
 
 #include "gemm_tc16.cuh"
@@ -43,11 +44,16 @@ constexpr int ATC_M = 128, ATC_KEYS = 64, ATC_WARPS = 16, ATC_THREADS = ATC_WARP
 constexpr int ATC_CHUNK = 128 * 128;                         // bytes of 128 rows x 64 fp16
 constexpr int ATC_PLANES = 4 * ATC_CHUNK;                    // q high; k high + low; v high + low: 64 KB each
 constexpr int ATC_SMEM_BYTES = 1024 + 3 * ATC_PLANES + (2 * ATC_KEYS + 2 * ATT_D + 4 * ATC_M) * 4 + 64;
-// tile image in global memory: k planes, v planes, 2^-s of the 64 keys, 2^-s of the 256 dims, whether a value is not finite or huge
-constexpr int ATC_IMG_KF = 2 * ATC_PLANES, ATC_IMG_VF = ATC_IMG_KF + ATC_KEYS * 4, ATC_IMG_FLAG = ATC_IMG_VF + ATT_D * 4;   // flag: k, then v
+// tile image in global memory: k planes, v planes, 2^-s of the 64 keys, 2^-s of the 256 dims, the tile's range (magnitude bits: largest k,
+// largest v, smallest of the keys' largest v; a key of zeros has none)
+constexpr int ATC_IMG_KF = 2 * ATC_PLANES, ATC_IMG_VF = ATC_IMG_KF + ATC_KEYS * 4, ATC_IMG_RANGE = ATC_IMG_VF + ATT_D * 4;
 constexpr int ATC_IMG_BYTES = 2 * ATC_PLANES + 2048;
 constexpr uint32_t ATC_COL_O = 0, ATC_COL_S = 256, ATC_COL_QL = 384;
 constexpr uint32_t ATC_HUGE = (127u + 60u) << 23;            // bits of 2^60
+constexpr uint32_t ATC_TINY = (127u - 100u) << 23;           // bits of 2^-100: a dim of v all below it is past the shift's cap
+constexpr uint32_t ATC_NONE = 0x7FFFFFFFu;
+constexpr int ATC_V_RANGE = 12;                              // log2
+constexpr float ATC_QK_RANGE = 4096.0f;
 constexpr int ATC_REDO_QUERIES = ATC_WARPS * ATT_QPW;
 static_assert(ATT_SMEM_BYTES <= 3 * ATC_PLANES, "attn_simt reuses the planes");
 
@@ -83,6 +89,22 @@ __device__ __forceinline__ void atc_split8(const float *x, float sc, uint4 &hi, 
     split_f16x2(__fmul_rn(x[6], sc), __fmul_rn(x[7], sc), hi.w, lo.w);
 }
 
+// Whether a CTA's values range too widely for the planes (magnitude bits: largest scaled q, largest k, largest v, smallest of the
+// keys' largest v, over every key that the CTA's tiles hold).
+//   scores   a plane pair is off by at most 2^-40 of its row's largest value (2^-41 in the mean), times the other row's value: with
+//            max |q| max |k| <= 2^12 the 512 products of a score add up to an error of about 2^-25, less than an fp32 sum's.
+//            (Scores of that size do not occur: one channel alone would reach 4096.)
+//   outputs  a key's weighted v is off by at most 2^-39 of the largest v, whatever its weight; a row's own largest output is no
+//            smaller than the smallest key: within 2^12 of each other 1000 such errors add up to 2^-22 of it.
+// Each range alone to 2^30 cost rows 1e-3 of their size (v) and scores 5e-4 (k); as it is every case of
+// tests/test_gpu_prompt_attention.py is as exact as on the CUDA cores.  The ranges are looked at per CTA and not per row: both
+// sides of the line are right, which of them a row takes does not matter.
+__device__ __forceinline__ bool atc_too_wide(uint32_t q, uint32_t k, uint32_t v, uint32_t v_small) {
+    if (max(q, max(k, v)) >= ATC_HUGE) return true;
+    if (__fmul_rn(__uint_as_float(q), __uint_as_float(k)) > ATC_QK_RANGE) return true;
+    return v_small != ATC_NONE && (int)(v >> 23) - (int)(v_small >> 23) > ATC_V_RANGE;
+}
+
 constexpr int ATC_PREP_THREADS = 256;
 // grid (tiles, kv heads, 2): z 0 = k (warp = eight keys, lane = eight dims), z 1 = v (thread = one dim, all 64 keys).  Bound
 // by latency: 16 MB in, 17 MB out at 2048 tokens.
@@ -90,12 +112,14 @@ __global__ void __launch_bounds__(ATC_PREP_THREADS) attn_planes_kernel(const flo
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j0 = (int)blockIdx.x * ATC_KEYS, kvh = blockIdx.y;
     uint8_t *img = images + ((size_t)kvh * gridDim.x + blockIdx.x) * ATC_IMG_BYTES;
-    uint32_t seen = 0;
+    uint32_t *range = reinterpret_cast<uint32_t *>(img + ATC_IMG_RANGE);
+    __shared__ uint32_t top[ATC_PREP_THREADS / 32][ATC_KEYS];
     pdl_wait_prior_grid();
     pdl_launch_dependents();
     if (blockIdx.z == 0) {
         constexpr int ROWS = ATC_KEYS / (ATC_PREP_THREADS / 32);
         float x[ROWS][8];
+        uint32_t seen = 0;
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             const int key = ROWS * warp + r;
@@ -123,12 +147,19 @@ __global__ void __launch_bounds__(ATC_PREP_THREADS) attn_planes_kernel(const flo
             *reinterpret_cast<uint4 *>(dst + ATC_KEYS * 128) = lo;
             if (lane == 0) reinterpret_cast<float *>(img + ATC_IMG_KF)[key] = atc_pow2(-s);
         }
+        if (lane == 0) top[warp][0] = seen;
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t m = __reduce_max_sync(0xffffffffu, top[lane & (ATC_PREP_THREADS / 32 - 1)][0]);
+            if (lane == 0) range[0] = m;
+        }
     } else {
         const int d = threadIdx.x;
         float x[ATC_KEYS];
         const float *src = v + ((size_t)j0 * n_head_kv + kvh) * ATT_D + d;
 #pragma unroll
         for (int e = 0; e < ATC_KEYS; ++e) x[e] = j0 + e < n_tok ? src[(size_t)e * n_head_kv * ATT_D] : 0.0f;
+        uint32_t seen = 0;
 #pragma unroll
         for (int e = 0; e < ATC_KEYS; ++e) seen = max(seen, atc_abs_bits(x[e]));
         const int s = atc_shift(seen, 112);
@@ -141,9 +172,29 @@ __global__ void __launch_bounds__(ATC_PREP_THREADS) attn_planes_kernel(const flo
             *reinterpret_cast<uint4 *>(dst) = hi;
             *reinterpret_cast<uint4 *>(dst + 2 * ATC_CHUNK) = lo;
         }
+        // the keys' largest values: over the warp's 32 dims (lane e keeps keys e and e + 32), then over the warps
+        uint32_t own[2] = {0u, 0u};
+#pragma unroll
+        for (int e = 0; e < ATC_KEYS; ++e) {
+            const uint32_t m = __reduce_max_sync(0xffffffffu, atc_abs_bits(x[e]));
+            if (lane == (e & 31)) own[e >> 5] = m;
+        }
+        top[warp][lane] = own[0];
+        top[warp][lane + 32] = own[1];
+        const int tiny = __syncthreads_or(seen > 0u && seen < ATC_TINY ? 1 : 0);
+        if (warp == 0) {
+#pragma unroll
+            for (int w = 0; w < ATC_PREP_THREADS / 32; ++w)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) own[h] = max(own[h], top[w][lane + 32 * h]);
+            const uint32_t most = __reduce_max_sync(0xffffffffu, max(own[0], own[1]));
+            const uint32_t least = __reduce_min_sync(0xffffffffu, min(own[0] ? own[0] : ATC_NONE, own[1] ? own[1] : ATC_NONE));
+            if (lane == 0) {
+                range[1] = tiny ? ATC_NONE : most;
+                range[2] = least;
+            }
+        }
     }
-    const int bad = __syncthreads_or(seen >= ATC_HUGE ? 1 : 0);
-    if (threadIdx.x == 0) reinterpret_cast<int *>(img + ATC_IMG_FLAG)[blockIdx.z] = bad;
 }
 
 // Cold path, a call of its own so that it takes no registers from the kernel.
@@ -205,7 +256,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
     // ---- q: row of the thread, 64 dims; high plane to shared memory, low plane to tensor memory.  (The launch this one may
     // run beside is attn_planes_kernel, which does not write q.)
     float qf;
-    uint32_t seen = 0;                                                   // largest magnitude bits met
+    uint32_t seen;                                                       // magnitude bits of the row's largest q
     {
         float x[64];
         uint32_t m = 0;
@@ -420,11 +471,23 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
     __syncthreads();
     red[cg * ATC_M + row] = l_run;
     tc_fence_before();
+    uint32_t k_most = 0, v_most = 0, v_least = ATC_NONE;
     for (int t = threadIdx.x; t < ntiles; t += ATC_THREADS) {
-        const int2 f = *reinterpret_cast<const int2 *>(img + (size_t)t * ATC_IMG_BYTES + ATC_IMG_FLAG);
-        if (f.x | f.y) seen = 0x7FFFFFFFu;
+        const uint32_t *range = reinterpret_cast<const uint32_t *>(img + (size_t)t * ATC_IMG_BYTES + ATC_IMG_RANGE);
+        k_most = max(k_most, range[0]);
+        v_most = max(v_most, range[1]);
+        v_least = min(v_least, range[2]);
     }
-    const bool redo = __syncthreads_or(seen >= ATC_HUGE ? 1 : 0) != 0;
+    uint4 *ranges = reinterpret_cast<uint4 *>(kf);                       // a warp each; every tile's factors have been read
+    seen = __reduce_max_sync(0xffffffffu, seen);
+    k_most = __reduce_max_sync(0xffffffffu, k_most);
+    v_most = __reduce_max_sync(0xffffffffu, v_most);
+    v_least = __reduce_min_sync(0xffffffffu, v_least);
+    if (lane == 0) ranges[warp] = make_uint4(seen, k_most, v_most, v_least);
+    __syncthreads();
+    const uint4 r = ranges[lane & (ATC_WARPS - 1)];
+    const bool redo = atc_too_wide(__reduce_max_sync(0xffffffffu, r.x), __reduce_max_sync(0xffffffffu, r.y), __reduce_max_sync(0xffffffffu, r.z),
+                                   __reduce_min_sync(0xffffffffu, r.w));
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");

@@ -115,3 +115,66 @@ def test_streams_release_and_capture(gpu):
     torch.cuda.synchronize()
     close(out, want[0].double())
     assert gpu.device_status() == 0
+
+
+ROW_TOL = 3e-6      # of the row's OWN largest output: fp32 sums over up to 600 keys; the CUDA cores' worst row of these cases is 1.9e-6
+
+
+def rows_close(got, want):
+    err = (got.double() - want).abs().amax(-1) / want.abs().amax(-1)
+    assert float(err.max()) <= ROW_TOL, (float(err.max()), int(err.max(-1).values.argmax()))
+
+
+@pytest.mark.parametrize("weight", [True, False])
+@pytest.mark.parametrize("at", [320, 351, 383])         # first, middle and last key of a tile
+@pytest.mark.parametrize("x", [1e3, 1e5, 1e6, 1e8, 1e10, 1e12, 1e15])
+def test_rows_do_not_depend_on_keys_they_do_not_see(gpu, x, at, weight):
+    """One key whose v is x, in every dim or in one: the rows in front of it (they do not see it), behind it without a weight for it
+    (its score is -100) and with one."""
+    import torch
+    n, heads, kv_heads = 600, 6, 2
+    for dims in (slice(None), slice(200, 201)):
+        q, k, v = inputs(n, heads, kv_heads, 9)
+        v[at, :, dims] *= x
+        if not weight:
+            q[:, :, 0], k[:, :, 0] = 16.0, 0.0
+            k[at, :, 0] = -100.0
+        out = torch.empty(n, heads, D, device="cuda")
+        assert gpu.attn(q, k, v, out, n, heads, kv_heads, D, SCALE) == 0
+        rows_close(out, exact(q, k, v))
+    assert gpu.device_status() == 0
+
+
+@pytest.mark.parametrize("x", [1e3, 1e4, 1e5, 1e6, 1e9, 1e12])
+@pytest.mark.parametrize("large", ["q", "k"])
+def test_channels_that_the_other_side_does_not_use(gpu, x, large):
+    import torch
+    n, heads, kv_heads = 600, 6, 2
+    q, k, v = inputs(n, heads, kv_heads, 10)
+    a, b = (q, k) if large == "q" else (k, q)
+    a[:, :, 7], b[:, :, 7] = x, 0.0
+    out = torch.empty(n, heads, D, device="cuda")
+    assert gpu.attn(q, k, v, out, n, heads, kv_heads, D, SCALE) == 0
+    rows_close(out, exact(q, k, v))
+
+
+@pytest.mark.parametrize("size", [1e-38, 1e-33, 1e-28, 1e17])
+def test_values_of_any_size(gpu, size):
+    """All of v very small or large, one dim of it, and tiles of large v whose small weights make them count as much as the rest."""
+    import torch
+    n, heads, kv_heads = 600, 6, 2
+    for dims in (slice(None), slice(9, 10)):
+        q, k, v = inputs(n, heads, kv_heads, 11)
+        v[:, :, dims] *= size
+        out = torch.empty(n, heads, D, device="cuda")
+        assert gpu.attn(q, k, v, out, n, heads, kv_heads, D, SCALE) == 0
+        want = exact(q, k, v)
+        err = (out.double() - want)[:, :, dims].abs().amax(-1) / want[:, :, dims].abs().amax(-1).clamp_min(float(v[:, :, dims].abs().max()) * 0.02)
+        assert float(err.max()) <= max(ROW_TOL, 2 ** -149 / size * 600), float(err.max())
+    q, k, v = inputs(n, heads, kv_heads, 12)
+    q[:, :, 0], k[:, :, 0] = 16.0, 0.0
+    k[300:, :, 0] = -28.0
+    v[300:] *= 1e12
+    out = torch.empty(n, heads, D, device="cuda")
+    assert gpu.attn(q, k, v, out, n, heads, kv_heads, D, SCALE) == 0
+    rows_close(out, exact(q, k, v))
