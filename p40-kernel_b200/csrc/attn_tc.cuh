@@ -402,7 +402,6 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
         ok = mbar_wait_hot(qk1, par) && ok;
         ok = mbar_wait_hot(qk2, par) && ok;
         tc_fence_after();
-        if (warp == 4 && lane == 0 && i + 1 < ntiles) load_k(i + 1);
         {
             auto pair = [&](uint32_t col, float (&t)[16]) {
                 int a[16], b[16];
@@ -429,6 +428,9 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
         tc_fence_before();
         if (!__syncthreads_and(ok ? 1 : 0)) break;                       // (a wait ran out: the CTA leaves as a whole)
         tc_fence_after();                                                // every score has been read: the weights take their place
+        // (a barrier's next phase is begun only when the whole CTA has waited for this one: a thread that came later than a
+        // phase's successor would wait for a parity that has passed)
+        if (warp == 4 && lane == 0 && i + 1 < ntiles) load_k(i + 1);
         float m_new = m_run;
 #pragma unroll
         for (int c = 0; c < 4; ++c) m_new = fmaxf(m_new, red[c * ATC_M + row]);
@@ -448,9 +450,9 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
             tc_st8(tlane + ATC_COL_S + (uint32_t)(32 + 8 * cg), lo);
         }
         tc_st_wait();
+        ok = mbar_wait_hot(vfull, par) && ok;                            // in front of the CTA's barrier: load_v below begins the next phase
         tc_fence_before();
         __syncthreads();
-        ok = mbar_wait_hot(vfull, par) && ok;
         if (warp == 0) issue_pv();
         ok = mbar_wait_hot(pv, par) && ok;
         tc_fence_after();
