@@ -203,13 +203,15 @@ __device__ __forceinline__ uint64_t policy_evict_last_or_default() {
 // Programmatic dependent launch: both are no-ops unless the launches carry the attribute.  Kernels call the wait first:
 // a launch that starts early then has its direct predecessor to wait for and nothing older, which is why a mat-vec behind
 // this library's quantiser may copy weights before its own wait.  What an earlier launch may have written is read through
-// pointers without __restrict__ (a load through one may be moved in front of the wait).
+// pointers without __restrict__ and with plain loads: a non-coherent one (ld.global.nc, __ldg) is for memory that nothing writes
+// while the kernel is there, and may be moved in front of the wait.  (Weights of a mat-vec: plain loads too, unless only an
+// option of the caller, who promises that nobody writes them, makes the kernel start early.)
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-__device__ __forceinline__ uint32_t ldg_nc_u32(const void *p) {
+__device__ __forceinline__ uint32_t ldg_u32(const void *p) {
     uint32_t v;
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ uint32_t ldg_nc_u16(const void *p) {

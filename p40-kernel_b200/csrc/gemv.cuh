@@ -72,9 +72,9 @@ struct RingParams {
 // Re-lay the Q8_1 vector (global, 9 words per chunk) into padded per-pair records: one thread per
 // chunk, nine loads in flight, two 16-byte stores plus the scale and the pre-scaled sum.  Split in a
 // load half and a store half so that a caller can issue other memory traffic behind the loads.
-__device__ __forceinline__ void act_chunk_load(const uint32_t *__restrict__ xq, int chunk, uint32_t (&v)[9]) {
+__device__ __forceinline__ void act_chunk_load(const uint32_t *xq, int chunk, uint32_t (&v)[9]) {
 #pragma unroll
-    for (int j = 0; j < 9; ++j) v[j] = __ldg(xq + 9 * chunk + j);
+    for (int j = 0; j < 9; ++j) v[j] = xq[9 * chunk + j];
 }
 __device__ __forceinline__ void act_chunk_store(uint32_t *rec, int chunk, const uint32_t (&v)[9]) {
     uint32_t *r = rec + (chunk >> 3) * ACT_REC_WORDS;
@@ -188,8 +188,7 @@ __device__ __forceinline__ void gemv_item(const uint32_t *pair_words, int row_wo
 // Roles: warps [0, NC) compute, warps [NC, NC + chain_warps) add, the last warp issues copies.
 template <int RR>
 __global__ void __launch_bounds__(RR == 4 ? 512 : 1024, 1) gemv_ring_kernel(const uint8_t *__restrict__ W,
-                                                                            const uint32_t *__restrict__ xq,
-                                                                            float *__restrict__ y, const RingParams P) {
+                                                                            const uint32_t *xq, float *y, const RingParams P) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
     uint64_t *done = full + RING_MAX_TILES;
@@ -230,7 +229,7 @@ __global__ void __launch_bounds__(RR == 4 ? 512 : 1024, 1) gemv_ring_kernel(cons
                 const uint32_t bytes = (uint32_t)(r_cnt * row_bytes);
                 const uint32_t bulk = bytes & ~15u;
                 const uint8_t *s = src + (size_t)r_begin * row_bytes;
-                for (uint32_t o = bulk; o < bytes; o += 4) *reinterpret_cast<uint32_t *>(dst + o) = ldg_nc_u32(s + o);
+                for (uint32_t o = bulk; o < bytes; o += 4) *reinterpret_cast<uint32_t *>(dst + o) = ldg_u32(s + o);
                 mbar_expect_tx(&full[t], bulk);
                 if (bulk) bulk_g2s(dst, s, bulk, &full[t], pol);
             }
@@ -344,8 +343,7 @@ __global__ void __launch_bounds__(RR == 4 ? 512 : 1024, 1) gemv_ring_kernel(cons
 // ---- fallback for shapes the staged kernel does not take (odd block count, unaligned W) ---------
 // One warp per row, 2-byte loads straight from global, same term order.
 __global__ void __launch_bounds__(256) gemv_pq2_generic_kernel(const uint8_t *__restrict__ W,
-                                                               const uint8_t *__restrict__ xq, float *__restrict__ y,
-                                                               int n_out, int nblocks) {
+                                                               const uint8_t *xq, float *y, int n_out, int nblocks) {
     constexpr int SEG = 512;                     // chunks summed per pass
     __shared__ float terms[8][SEG];
     pdl_wait_prior_grid();
@@ -365,10 +363,10 @@ __global__ void __launch_bounds__(256) gemv_pq2_generic_kernel(const uint8_t *__
             const uint32_t c0w = ldg_nc_u16(cp) | (ldg_nc_u16(cp + 2) << 16);
             const uint32_t c1w = ldg_nc_u16(cp + 4) | (ldg_nc_u16(cp + 6) << 16);
             const uint32_t *ab = reinterpret_cast<const uint32_t *>(xq + (size_t)c * A_BLOCK_BYTES);
-            const uint32_t hdr = __ldg(ab);
+            const uint32_t hdr = ab[0];
             int a[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) a[k] = (int)__ldg(ab + 1 + k);
+            for (int k = 0; k < 8; ++k) a[k] = (int)ab[1 + k];
             const int sumi = chunk_sumi_scaled(c0w, c1w, a, -64 * (int)(short)(hdr >> 16));
             const float d = __fmul_rn(f16_bits_to_f32(ldg_nc_u16(wb)), f16_bits_to_f32(hdr & 0xFFFFu));
             terms[warp][i] = __fmul_rn(d, (float)sumi);

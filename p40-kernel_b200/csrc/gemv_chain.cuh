@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                 const uint32_t bytes = (uint32_t)(r_cnt * row_bytes);
                 const uint32_t bulk = bytes & ~15u;
                 const uint8_t *s = src + (size_t)t * tr * row_bytes;
-                for (uint32_t o = bulk; o < bytes; o += 4) *reinterpret_cast<uint32_t *>(dst + o) = ldg_nc_u32(s + o);
+                for (uint32_t o = bulk; o < bytes; o += 4) *reinterpret_cast<uint32_t *>(dst + o) = ldg_u32(s + o);
                 mbar_expect_tx(&full[slot], bulk);
                 if (bulk) bulk_g2s(dst, s, bulk, &full[slot], pol);
                 __threadfence_block();

@@ -153,8 +153,8 @@ __device__ __forceinline__ void mma_pair_rows(const uint8_t *rows, int stride, i
 
 // DUMP: also writes the int32 chunk sums (sum code * a - sum a) of every row to dump[row][n_in / 32] (parity probe).
 template <bool DUMP>
-__global__ void __launch_bounds__(MMA_THREADS, 1) gemv_mma_kernel(const uint8_t *__restrict__ W, const uint32_t *__restrict__ xq,
-                                                                 float *__restrict__ y, const MmaGeom P,
+__global__ void __launch_bounds__(MMA_THREADS, 1) gemv_mma_kernel(const uint8_t *__restrict__ W, const uint32_t *xq,
+                                                                 float *y, const MmaGeom P,
                                                                  int32_t *__restrict__ dump) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);       // [12] tile landed in slot
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(MMA_THREADS, 1) gemv_mma_kernel(const uint8_t 
                 // a ragged last group of rows whose length is no multiple of 16 bytes (n_in / 128 not a multiple of
                 // 8): the last few bytes by plain loads, stored before the arrive that releases them to the waiters
                 const uint32_t bytes = (uint32_t)(r_cnt * row_bytes), bulk = bytes & ~15u;
-                for (uint32_t o = bulk; o < bytes; o += 4) *reinterpret_cast<uint32_t *>(dst + o) = ldg_nc_u32(src + o);
+                for (uint32_t o = bulk; o < bytes; o += 4) *reinterpret_cast<uint32_t *>(dst + o) = ldg_u32(src + o);
                 mbar_expect_tx(&full[slot], bulk);
                 if (bulk) bulk_g2s(dst, src, bulk, &full[slot], pol);
             } else {
@@ -384,8 +384,8 @@ __device__ __forceinline__ void mmab_tile_copy(void *dst, const CUtensorMap *map
 }
 
 template <bool DUMP, int NTG, int NRG>
-__global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t *__restrict__ W, const uint32_t *__restrict__ Xq,
-                                                                  float *__restrict__ Y, const MmabGeom P, const int n_tok,
+__global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t *__restrict__ W, const uint32_t *Xq,
+                                                                  float *Y, const MmabGeom P, const int n_tok,
                                                                   int32_t *__restrict__ dump,
                                                                   const __grid_constant__ CUtensorMap wmap) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
                 const uint8_t *src = W + (size_t)16 * gi * row_bytes;
                 uint8_t *d = dst + (size_t)h * group_bytes;
                 const uint32_t bytes = (uint32_t)(r_cnt * row_bytes), bulk = bytes & ~15u;
-                for (uint32_t o = bulk; o < bytes; o += 4) *reinterpret_cast<uint32_t *>(d + o) = ldg_nc_u32(src + o);
+                for (uint32_t o = bulk; o < bytes; o += 4) *reinterpret_cast<uint32_t *>(d + o) = ldg_u32(src + o);
                 total += bulk;
             }
             mbar_expect_tx(&full[slot], total);
@@ -743,8 +743,17 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
                 for (uint32_t o = lane * PIECE; o < bytes; o += 32 * PIECE)
                     bulk_g2s(dst + o, src + o, min(PIECE, bytes - o), &actfull[ab], keep);
             } else {                                            // a vector that is only word-aligned: plain loads
-                for (uint32_t i = lane; i < bytes / 4; i += 32)
-                    reinterpret_cast<uint32_t *>(dst)[i] = __ldg(reinterpret_cast<const uint32_t *>(src) + i);
+                constexpr uint32_t AHEAD = 8;                   // loads in flight per lane
+                const uint32_t *from = reinterpret_cast<const uint32_t *>(src);
+                uint32_t *to = reinterpret_cast<uint32_t *>(dst);
+                for (uint32_t i = lane; i < bytes / 4; i += 32 * AHEAD) {
+                    uint32_t w[AHEAD];
+#pragma unroll
+                    for (uint32_t u = 0; u < AHEAD; ++u) w[u] = i + 32 * u < bytes / 4 ? from[i + 32 * u] : 0u;
+#pragma unroll
+                    for (uint32_t u = 0; u < AHEAD; ++u)
+                        if (i + 32 * u < bytes / 4) to[i + 32 * u] = w[u];
+                }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&actfull[ab]);
             }

@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
         const uint32_t bytes = (uint32_t)(r_cnt * row_bytes);
         const uint32_t bulk = bytes & ~15u;
         const uint8_t *s = src + (size_t)r_begin * row_bytes;
-        for (uint32_t o = bulk; o < bytes; o += 4) *reinterpret_cast<uint32_t *>(dst + o) = ldg_nc_u32(s + o);
+        for (uint32_t o = bulk; o < bytes; o += 4) *reinterpret_cast<uint32_t *>(dst + o) = ldg_u32(s + o);
         mbar_expect_tx(&full[t], bulk);
         if (bulk) bulk_g2s(dst, s, bulk, &full[t], pol);
     };

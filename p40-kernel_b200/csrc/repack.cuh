@@ -90,8 +90,8 @@ __global__ void __launch_bounds__(256) repack_staged_kernel(const uint8_t *__res
 // butterfly) -- a fixed order like that of the default mat-vec, within 1e-5 of repack_row_dot; !TREE: by one lane in
 // unit order, bit-identical to repack_row_dot (bonsai_b200_set_option("gemv_order", 1)), several times slower.
 template <int RR, bool VEC, bool TREE>
-__global__ void __launch_bounds__(256) gemv_repack_kernel(const uint8_t *__restrict__ W, const float *__restrict__ x,
-                                                          float *__restrict__ y, int n_out, int nb, int rows_per_cta,
+__global__ void __launch_bounds__(256) gemv_repack_kernel(const uint8_t *__restrict__ W, const float *x,
+                                                          float *y, int n_out, int nb, int rows_per_cta,
                                                           int rows_per_stage) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);

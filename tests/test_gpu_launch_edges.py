@@ -60,6 +60,36 @@ def test_calls_read_what_the_call_before_wrote(gpu, n_out, n_in):
     assert gpu.device_status() == 0
 
 
+@pytest.mark.parametrize("n_tok", [2, 5, 8, 9, 16])
+@pytest.mark.parametrize("offset", [0, 4])      # of Xq in bytes: bulk copies or plain loads
+def test_token_batches_read_what_the_call_before_wrote(gpu, n_tok, offset):
+    """Weights, inputs and quantised blocks change between the mat-muls of 2 - 16 tokens: bits of the same calls made one by one."""
+    import torch
+    n_out, n_in = 1030, 5120
+    Ws = [dev(synth.pq2_0_weights(n_out, n_in, seed=s)) for s in range(2)]
+    Xs = [dev(synth.activations(n_in, seed=s, batch=n_tok)) for s in range(3)]
+    sg, W = dev(synth.signs(n_in, seed=1)), torch.empty_like(Ws[0])
+    Xq = torch.empty(n_in // 32 * 36 * n_tok + 16, dtype=torch.uint8, device="cuda")[offset:offset + n_in // 32 * 36 * n_tok]
+    Y = torch.empty(n_out, n_tok, device="cuda")
+
+    def step(i, sync):
+        wait = torch.cuda.synchronize if sync else (lambda: None)
+        out = []
+        for rotate in (True, False):
+            W.copy_(Ws[(i + rotate) % 2]); wait()
+            assert gpu.quant_batch(Xs[i % 3], sg, Xq, n_in, n_tok, rotate) == 0; wait()
+            assert gpu.gemm(W, Xq, Y, n_out, n_in, n_tok) == 0; wait()
+            out.append(Y.clone()); wait()
+        return out
+
+    want = [step(i, True) for i in range(6)]
+    got = [step(i, False) for i in range(6)]
+    for i in range(6):
+        for a, b in zip(want[i], got[i]):
+            assert torch.equal(a, b), i
+    assert gpu.device_status() == 0
+
+
 @pytest.mark.parametrize("n_out,n_in,n_tok", [
     (128, 17408, 17), (129, 17408, 64), (5120, 17408, 37), (1000, 5120, 33), (2000, 17408, 95), (300, 17408, 96), (1030, 9216, 130), (6000, 5120, 257)])
 def test_parts_of_a_tile_add_up(gpu, port, n_out, n_in, n_tok):
