@@ -15,6 +15,8 @@
 
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace b200 {
 
 constexpr int KV_D = 256, KV_NBLK = 8, KV_ROW = KV_NBLK * 34;      // 272 bytes per position and head
@@ -92,7 +94,9 @@ __global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *K, uint8_t *V,
 //   values   warp w = output dims 64 w .. 64 w + 63 (two V blocks), all 64 positions and all heads.  V bytes become fp16
 //            exactly (int8 fits), a weight (softmax weight x the chunk's rescale x the V block's scale x a power of two)
 //            is split into two fp16 planes, high and low (22 - 23 bits, the size of expf's own error), which are rows 0 - 7
-//            and 8 - 15 of one m16n8k16: one instruction multiplies both planes, accumulators are fp32.
+//            and 8 - 15 of one m16n8k16: one instruction multiplies both planes, accumulators are fp32.  The planes hold
+//            2^-39 of the largest V scale of the split and of the warp's two blocks; where scales lie further apart than
+//            KV_V_RANGE, a second pass over the tile multiplies what they left.
 // What bounded the kernel before was instruction issue (5860 warp instructions per 32 positions: fp32 multiply-adds of
 // every value for every head on the CUDA cores; 1500 GB/s).  This form issues about 1500.
 //
@@ -109,6 +113,10 @@ constexpr int KV_HALF_BYTES = KV_TILE * KV_ROW;                      // the K (o
 constexpr int KV_WT_STRIDE = KV_TILE + 8;                            // weights of a head: 8 g + 2 t are 32 different banks
 constexpr int KV_SLICE = KV_D / KV_CLUSTER;                          // output dims a CTA of the cluster merges
 constexpr int KV_MAX_CLUSTERS = 64;                                  // per kv head
+// Exponents between the largest V scale so far and the smallest (not zero) of a tile up to which two planes of a weight do: a position
+// of full weight keeps 2^-26 of itself.  Past it a large scale without weight took bits from the others (1e6 among values of
+// 0.06: 3e-6 of the output).  A scale below fp16's normal range counts as the smallest there is.
+constexpr int KV_V_RANGE = 12;
 constexpr int KV_REC = KV_MAX_GROUP * (KV_SLICE + 2);                // floats of a cluster's merged slice: acc, m, l
 constexpr int KV_SMEM_BYTES = 128 + KV_BUFS * 2 * KV_HALF_BYTES + KV_MAX_GROUP * KV_WT_STRIDE * 4 + 3 * KV_MAX_GROUP * 8 * 4 +
                               KV_MAX_GROUP * 64 * 4;
@@ -131,6 +139,13 @@ __device__ __forceinline__ void split_f16x2(float a, float b, uint32_t &hi, uint
     const __half2 l = __floats2half2_rn(__fsub_rn(a, f.x), __fsub_rn(b, f.y));
     hi = *reinterpret_cast<const uint32_t *>(&h);
     lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+// What the planes left of (a, b), times 2^24 (at most 2^-10 of a value below 2^14): together they hold 2^-63 of the largest.  Of an
+// infinity nothing is left.
+__device__ __forceinline__ void split_rest_f16x2(float a, float b, uint32_t &hi, uint32_t &lo) {
+    const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&hi)), l = __half22float2(*reinterpret_cast<const __half2 *>(&lo));
+    const float ra = __fsub_rn(__fsub_rn(a, h.x), l.x), rb = __fsub_rn(__fsub_rn(b, h.y), l.y);
+    split_f16x2(fabsf(ra) < 1.0f ? __fmul_rn(ra, 0x1p24f) : 0.0f, fabsf(rb) < 1.0f ? __fmul_rn(rb, 0x1p24f) : 0.0f, hi, lo);
 }
 __device__ __forceinline__ float half_bits_lo(uint32_t w) { return f16_bits_to_f32(w & 0xFFFFu); }
 __device__ __forceinline__ float half_bits_hi(uint32_t w) { return f16_bits_to_f32(w >> 16); }
@@ -243,7 +258,7 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
         }
     }
     float m_run = -INFINITY, l_run = 0.0f;                  // of head g
-    uint32_t dv_run[2] = {0u, 0u};                          // largest V scale so far (fp16 bits) of the warp's two blocks
+    int top_run = 1;                                        // fp16 exponent of the largest V scale so far in the warp's two blocks
     float acc[2][4][4];
 #pragma unroll
     for (int b = 0; b < 2; ++b)
@@ -251,11 +266,9 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[b][j][i] = 0.0f;
-    // the power of two that puts the largest V scale at 2^13 .. 2^14 (weights are at most 1): fp16 planes with room below
-    auto lift = [](uint32_t bits) -> float {
-        const int e = max(1, (int)(bits >> 10) & 31);       // biased fp16 exponent of the scale
-        return __uint_as_float((uint32_t)(127 + 13 + 15 - e) << 23);
-    };
+    // The planes are of weight x scale x 2^(13 + 15 - top_run): the largest scale ends at 2^13 .. 2^14 (weights are at most 1), room for an
+    // fp16 pair below.
+    constexpr int LIFT = 127 + 13 + 15;
 
     for (int i = 0; i < ntiles; ++i) {
         const int b = i % KV_BUFS;
@@ -329,11 +342,12 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
         if (!__syncthreads_and(ok ? 1 : 0)) break;
         {   // ---- values: dims 64 warp .. + 63
             const uint32_t *v32 = reinterpret_cast<const uint32_t *>(vt) + 17 * warp;
-            uint32_t big[2];
+            uint32_t exps;                                  // which fp16 exponents the tile's scales have (0: none but zeros)
             {
                 const uint32_t *ra = v32 + (size_t)lane * (KV_ROW / 4), *rb = ra + 32 * (KV_ROW / 4);
-                big[0] = __reduce_max_sync(0xffffffffu, max(ra[0] & 0x7FFFu, rb[0] & 0x7FFFu));
-                big[1] = __reduce_max_sync(0xffffffffu, max((ra[8] >> 16) & 0x7FFFu, (rb[8] >> 16) & 0x7FFFu));
+                auto exponent = [](uint32_t scale) { return min(scale, 1u) << (scale >> 10); };
+                exps = __reduce_or_sync(0xffffffffu, exponent(ra[0] & 0x7FFFu) | exponent(rb[0] & 0x7FFFu) | exponent((ra[8] >> 16) & 0x7FFFu) |
+                                                         exponent((rb[8] >> 16) & 0x7FFFu));
             }
             float mc[4], m_new = m_run, f[4], lsum = 0.0f;
 #pragma unroll
@@ -346,79 +360,89 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
             }
             l_run = __fmaf_rn(l_run, alpha, lsum);
             m_run = m_new;
-            float up[2];
+            const int top = max(top_run, 31 - __clz((int)(exps | 1u)));
+            const bool wide = exps != 0u && top - ((exps & 1u) ? -9 : __ffs((int)exps) - 1) > KV_V_RANGE;      // warp-uniform
+            const float up = __uint_as_float((uint32_t)(LIFT - top) << 23);
+            const float keep = i == 0 ? 0.0f : __fmul_rn(alpha, __uint_as_float((uint32_t)(127 + top_run - top) << 23));      // a power of two: exact
+            top_run = top;
+            if (__any_sync(0xffffffffu, keep != 1.0f)) {
 #pragma unroll
-            for (int bb = 0; bb < 2; ++bb) {
-                const float before = lift(dv_run[bb]);
-                dv_run[bb] = max(dv_run[bb], big[bb]);
-                up[bb] = lift(dv_run[bb]);
-                const float keep = i == 0 ? 0.0f : __fmul_rn(alpha, __fdiv_rn(up[bb], before));      // a power of two: exact
-                if (__any_sync(0xffffffffu, keep != 1.0f)) {
+                for (int bb = 0; bb < 2; ++bb)
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
 #pragma unroll
                         for (int e = 0; e < 4; ++e) acc[bb][j][e] = __fmul_rn(acc[bb][j][e], keep);
-                }
             }
             // Two instructions' sums at a time: the tensor core cuts the last bits of a sum off, a rounded addition does not (all of
             // a split in one accumulator: relative error 3.2e-7 at 32768 positions, 2.6e-7 on the CUDA cores).
-            float sum[2][4][4];
+            auto weigh = [&](auto rest) {                   // rest: the second pass, over what the planes of the first left
+                constexpr bool REST = decltype(rest)::value;
+                float sum[2][4][4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                if (16 * c >= n) break;                     // CTA-uniform
-                if ((c & 1) == 0) {
+                for (int c = 0; c < 4; ++c) {
+                    if (16 * c >= n) break;                     // CTA-uniform
+                    if ((c & 1) == 0) {
 #pragma unroll
-                    for (int bb = 0; bb < 2; ++bb)
+                        for (int bb = 0; bb < 2; ++bb)
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
+                            for (int j = 0; j < 4; ++j)
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) sum[bb][j][e] = 0.0f;
-                }
-                const uint32_t *rows = v32 + (size_t)(16 * c + 2 * t) * (KV_ROW / 4);
-                uint32_t ev[4], od[4];
-                float de[4], dq[4];
+                                for (int e = 0; e < 4; ++e) sum[bb][j][e] = 0.0f;
+                    }
+                    const uint32_t *rows = v32 + (size_t)(16 * c + 2 * t) * (KV_ROW / 4);
+                    uint32_t ev[4], od[4];
+                    float de[4], dq[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const uint32_t *u = rows + (size_t)((r & 1) + 8 * (r >> 1)) * (KV_ROW / 4);
-                    const uint32_t d0 = u[0], e = u[8];
-                    uint32_t x = u[g];
-                    if (g == 0) x = __byte_perm(x, e, 0x5432);
-                    ev[r] = x ^ 0x80808080u;
-                    od[r] = u[9 + g] ^ 0x80808080u;
-                    de[r] = half_bits_lo(d0);
-                    dq[r] = half_bits_hi(e);
-                }
-                const float2 wa = *reinterpret_cast<const float2 *>(wt + g * KV_WT_STRIDE + 16 * c + 2 * t);
-                const float2 wb = *reinterpret_cast<const float2 *>(wt + g * KV_WT_STRIDE + 16 * c + 2 * t + 8);
+                    for (int r = 0; r < 4; ++r) {
+                        const uint32_t *u = rows + (size_t)((r & 1) + 8 * (r >> 1)) * (KV_ROW / 4);
+                        const uint32_t d0 = u[0], e = u[8];
+                        uint32_t x = u[g];
+                        if (g == 0) x = __byte_perm(x, e, 0x5432);
+                        ev[r] = x ^ 0x80808080u;
+                        od[r] = u[9 + g] ^ 0x80808080u;
+                        de[r] = half_bits_lo(d0);
+                        dq[r] = half_bits_hi(e);
+                    }
+                    const float2 wa = *reinterpret_cast<const float2 *>(wt + g * KV_WT_STRIDE + 16 * c + 2 * t);
+                    const float2 wb = *reinterpret_cast<const float2 *>(wt + g * KV_WT_STRIDE + 16 * c + 2 * t + 8);
+                    const float fu = __fmul_rn(f[c], up);
 #pragma unroll
-                for (int bb = 0; bb < 2; ++bb) {
-                    const float fu = __fmul_rn(f[c], up[bb]);
-                    const float *dd = bb ? dq : de;
-                    const uint32_t *vv = bb ? od : ev;
-                    uint32_t h01, l01, h23, l23;
-                    split_f16x2(__fmul_rn(__fmul_rn(wa.x, fu), dd[0]), __fmul_rn(__fmul_rn(wa.y, fu), dd[1]), h01, l01);
-                    split_f16x2(__fmul_rn(__fmul_rn(wb.x, fu), dd[2]), __fmul_rn(__fmul_rn(wb.y, fu), dd[3]), h23, l23);
-                    // byte j of four rows -> fp16: under the exponent of 1024 (value + 128, sign bit flipped above), minus 1152
-                    const uint32_t p01 = __byte_perm(vv[0], vv[1], 0x5140), q01 = __byte_perm(vv[0], vv[1], 0x7362);
-                    const uint32_t p23 = __byte_perm(vv[2], vv[3], 0x5140), q23 = __byte_perm(vv[2], vv[3], 0x7362);
-                    const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);
+                    for (int bb = 0; bb < 2; ++bb) {
+                        const float *dd = bb ? dq : de;
+                        const uint32_t *vv = bb ? od : ev;
+                        uint32_t h01, l01, h23, l23;
+                        const float p0 = __fmul_rn(__fmul_rn(wa.x, fu), dd[0]), p1 = __fmul_rn(__fmul_rn(wa.y, fu), dd[1]);
+                        const float p2 = __fmul_rn(__fmul_rn(wb.x, fu), dd[2]), p3 = __fmul_rn(__fmul_rn(wb.y, fu), dd[3]);
+                        split_f16x2(p0, p1, h01, l01);
+                        split_f16x2(p2, p3, h23, l23);
+                        if (REST) {
+                            split_rest_f16x2(p0, p1, h01, l01);
+                            split_rest_f16x2(p2, p3, h23, l23);
+                        }
+                        // byte j of four rows -> fp16: under the exponent of 1024 (value + 128, sign bit flipped above), minus 1152
+                        const uint32_t p01 = __byte_perm(vv[0], vv[1], 0x5140), q01 = __byte_perm(vv[0], vv[1], 0x7362);
+                        const uint32_t p23 = __byte_perm(vv[2], vv[3], 0x5140), q23 = __byte_perm(vv[2], vv[3], 0x7362);
+                        const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint32_t b0 = __byte_perm(j < 2 ? p01 : q01, 0x64646464u, (j & 1) ? 0x4342 : 0x4140);
-                        uint32_t b1 = __byte_perm(j < 2 ? p23 : q23, 0x64646464u, (j & 1) ? 0x4342 : 0x4140);
-                        const __half2 v0 = __hsub2(*reinterpret_cast<__half2 *>(&b0), bias), v1 = __hsub2(*reinterpret_cast<__half2 *>(&b1), bias);
-                        mma_f16_16816(sum[bb][j], h01, l01, h23, l23, *reinterpret_cast<const uint32_t *>(&v0), *reinterpret_cast<const uint32_t *>(&v1));
+                        for (int j = 0; j < 4; ++j) {
+                            uint32_t b0 = __byte_perm(j < 2 ? p01 : q01, 0x64646464u, (j & 1) ? 0x4342 : 0x4140);
+                            uint32_t b1 = __byte_perm(j < 2 ? p23 : q23, 0x64646464u, (j & 1) ? 0x4342 : 0x4140);
+                            const __half2 v0 = __hsub2(*reinterpret_cast<__half2 *>(&b0), bias), v1 = __hsub2(*reinterpret_cast<__half2 *>(&b1), bias);
+                            mma_f16_16816(sum[bb][j], h01, l01, h23, l23, *reinterpret_cast<const uint32_t *>(&v0), *reinterpret_cast<const uint32_t *>(&v1));
+                        }
+                    }
+                    if ((c & 1) == 1 || 16 * (c + 1) >= n) {
+#pragma unroll
+                        for (int bb = 0; bb < 2; ++bb)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) acc[bb][j][e] = REST ? __fmaf_rn(sum[bb][j][e], 0x1p-24f, acc[bb][j][e]) : __fadd_rn(acc[bb][j][e], sum[bb][j][e]);
                     }
                 }
-                if ((c & 1) == 1 || 16 * (c + 1) >= n) {
-#pragma unroll
-                    for (int bb = 0; bb < 2; ++bb)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) acc[bb][j][e] = __fadd_rn(acc[bb][j][e], sum[bb][j][e]);
-                }
-            }
+            };
+            weigh(std::false_type{});
+            if (__builtin_expect(wide, 0)) weigh(std::true_type{});
         }
         __syncthreads();                                            // tile i's buffer and the tables may be overwritten
         if (tid == 0 && i + KV_BUFS < ntiles) issue(i + KV_BUFS);
@@ -428,14 +452,16 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
     if (g < GRP) {
 #pragma unroll
         for (int bb = 0; bb < 2; ++bb) {
-            const float down = __fdiv_rn(1.0f, lift(dv_run[bb]));       // a power of two
+            const float down = __uint_as_float((uint32_t)(254 - LIFT + top_run) << 23);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int slot = 2 * t + e;
                     const int in_blk = bb ? 4 * slot + j : (slot == 0 ? (j < 2 ? j : 28 + j) : 4 * slot - 2 + j);
-                    so[g * KV_D + 64 * warp + 32 * bb + in_blk] = __fmul_rn(__fadd_rn(acc[bb][j][e], acc[bb][j][e + 2]), down);
+                    // (of an infinity the low plane is NaN: the high plane alone is the sum then)
+                    const float high = acc[bb][j][e], both = isinf(high) ? high : __fadd_rn(high, acc[bb][j][e + 2]);
+                    so[g * KV_D + 64 * warp + 32 * bb + in_blk] = __fmul_rn(both, down);
                 }
         }
         if (warp == 0 && t == 0) sm[g] = m_run, sl[g] = l_run;

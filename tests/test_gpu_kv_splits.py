@@ -69,6 +69,54 @@ def test_against_float64(gpu, port, n, spread):
     kv.close()
 
 
+@pytest.mark.parametrize("n", [70, 1000, 5000])
+@pytest.mark.parametrize("size", [1e-4, 1e1, 1e2, 1e3, 1e5, 1e6])
+def test_scales_far_apart(gpu, port, n, size):
+    """One position with a very large (or small) V: in one dim or all, without weight (its score is -225) or with.  Each head to 2e-6
+    of its own largest output in the blocks that the large values leave alone, and in all of them."""
+    import torch
+    layer, at = 5, n // 3
+    for dims in (slice(None), slice(40, 41)):
+        for weight in (False, True):
+            kv = gpu.KVCache(n)
+            g = torch.Generator(device="cuda").manual_seed(n)
+            k, v = torch.randn(n, N_KV, D, generator=g, device="cuda"), torch.randn(n, N_KV, D, generator=g, device="cuda") * 0.06
+            q = torch.randn(N_HEADS, D, generator=g, device="cuda")
+            v[at, :, dims] = size
+            if not weight:
+                q[:, 0], k[:, :, 0], k[at, :, 0] = 60.0, 0.0, -60.0
+            assert kv.append_batch(layer, 0, n, k, v) == 0
+            out = torch.full((N_HEADS, D), float("nan"), device="cuda")
+            assert kv.attn_decode(layer, n - 1, q, out) == 0
+            err, want = out.double(), exact(port, kv, n, layer, n, q)
+            err = (err - want).abs()
+            for block in (slice(None), slice(64, None)):
+                assert float((err[:, block].amax(1) / want[:, block].abs().amax(1)).max()) <= REL_TOL
+            kv.close()
+    assert gpu.device_status() == 0
+
+
+def test_infinite_scale(gpu, port):
+    """A V block past fp16's range: infinities with their signs where its values are not 0, NaN where they are, nothing else touched."""
+    import torch
+    n, layer = 1500, 2
+    kv = gpu.KVCache(n)
+    q = fill(kv, layer, n, 3, 0)
+    row = torch.randn(2, 1, N_KV, D, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda")
+    row[1, 0, 1, 3], row[1, 0, 1, 4], row[1, 0, 1, 40] = 1e7, -1e7, 1e6
+    assert kv.append(layer, 700, row[0], row[1]) == 0
+    out = torch.full((N_HEADS, D), float("nan"), device="cuda")
+    assert kv.attn_decode(layer, n - 1, q, out) == 0
+    want = exact(port, kv, n, layer, n, q)
+    hit = out[6:12]
+    assert bool((hit[:, 3] == float("inf")).all()) and bool((hit[:, 4] == -float("inf")).all())
+    assert bool(torch.isnan(hit[:, [d for d in range(32) if d not in (3, 4)]]).all())
+    assert float((hit[:, 32:].double() - want[6:12, 32:]).abs().max()) <= REL_TOL * float(want[6:12, 32:].abs().max())
+    rest = [h for h in range(N_HEADS) if not 6 <= h < 12]
+    assert float((out[rest].double() - want[rest]).abs().max()) <= REL_TOL * float(want[rest].abs().max())
+    kv.close()
+
+
 def test_layers_on_streams_of_their_own(gpu):
     """Layers have their own records and counters: decoded at the same time on different streams they give the bits that
     they give one after the other."""
