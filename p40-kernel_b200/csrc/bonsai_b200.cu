@@ -21,6 +21,7 @@
 #include "probe.cuh"
 #include "ptq.cuh"
 #include "repack.cuh"
+#include "scratch.cuh"
 #include "synth.cuh"
 
 #include <algorithm>
@@ -918,36 +919,10 @@ static bool encode_w_map(CUtensorMap *map, const void *W, int64_t n_out, int64_t
                          68u, (uint32_t)TC_M, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
-// Scratch of the fp16 tensor-core mat-mul (the activations as two fp16 planes + the per-token scales): one buffer per
-// (device, stream), grown with cudaMalloc when a call needs more -- never while the stream is being captured (then,
-// and when 16 buffers exist already, the caller takes the integer kernel, which needs no scratch).
-struct GemmScratch { int dev; cudaStream_t st; void *ptr; size_t bytes; };
-static std::mutex g_scratch_mu;
-static std::vector<GemmScratch> g_scratch;
-static void *gemm_scratch(size_t bytes, cudaStream_t st) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-    std::lock_guard<std::mutex> lock(g_scratch_mu);
-    GemmScratch *e = nullptr;
-    for (auto &g : g_scratch)
-        if (g.dev == dev && g.st == st) e = &g;
-    if (e && e->bytes >= bytes) return e->ptr;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return nullptr;
-    if (!e) {
-        if (g_scratch.size() >= 16) return nullptr;
-        g_scratch.push_back(GemmScratch{dev, st, nullptr, 0});
-        e = &g_scratch.back();
-    }
-    if (e->ptr) cudaFree(e->ptr);               // synchronises the device: nothing in flight reads the old buffer
-    e->ptr = nullptr;
-    e->bytes = 0;
-    void *pnew = nullptr;
-    if (cudaMalloc(&pnew, bytes) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
-    e->ptr = pnew;
-    e->bytes = bytes;
-    return pnew;
-}
+// Scratch of the fp16 tensor-core mat-mul: a flag and a slot per CTA for its part of a tile, the activations as two fp16 planes, a
+// scale per token.  A call that gets none takes the integer kernel, which needs no scratch.
+static constexpr size_t T16_FLAGS_BYTES = (size_t)TC_MAX_CTAS * sizeof(unsigned int);
+static StreamScratch g_gemm_scratch(T16_FLAGS_BYTES);
 
 // Scratch of the prompt attention (k and v as tile images: 2 KB per position and kv head, what k and v take themselves), kept
 // per stream and bounded: the 17th stream of a device takes the place of the one that called longest ago.  Streams are told
@@ -1001,10 +976,9 @@ static void fill_tc_params(TcParams &P, int64_t n_out, int64_t n_in, int64_t n_t
     P.total_it = (long long)P.n_tiles * P.nblocks;
 }
 
-// Scratch of the fp16 mat-mul: a slot per CTA for its part of a tile, the two planes, a scale per token.
 static constexpr size_t T16_PARTS_BYTES = (size_t)TC_MAX_CTAS * T16C<128>::PART_FLOATS * sizeof(float);
 static size_t tc16_scratch_bytes(int64_t n_in, int64_t n_tok) {
-    return T16_PARTS_BYTES + 2 * (size_t)n_tok * (size_t)n_in * sizeof(__half) + (size_t)n_tok * sizeof(float);
+    return T16_FLAGS_BYTES + T16_PARTS_BYTES + 2 * (size_t)n_tok * (size_t)n_in * sizeof(__half) + (size_t)n_tok * sizeof(float);
 }
 
 // The fp16 tensor-core mat-mul (gemm_tc16.cuh).  -1: not taken (shape, alignment, no scratch, no tensor-map encoder).
@@ -1017,11 +991,13 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     const long long tiles = (long long)((n_out + T16_M - 1) / T16_M) * ((n_tok + T16_N - 1) / T16_N);
     if (tiles > INT32_MAX) return -1;
     const size_t plane_bytes = (size_t)n_tok * (size_t)n_in * sizeof(__half);
-    uint8_t *ws = static_cast<uint8_t *>(gemm_scratch(tc16_scratch_bytes(n_in, n_tok), st));
+    const StreamScratch::Lease lease = g_gemm_scratch.get(tc16_scratch_bytes(n_in, n_tok), st);      // held until both launches are enqueued
+    uint8_t *ws = static_cast<uint8_t *>(lease.ptr);
     if (!ws) return -1;
-    float *parts = reinterpret_cast<float *>(ws);
-    __half *planes = reinterpret_cast<__half *>(ws + T16_PARTS_BYTES);
-    float *scale = reinterpret_cast<float *>(ws + T16_PARTS_BYTES + 2 * plane_bytes);
+    unsigned int *flags = reinterpret_cast<unsigned int *>(ws);
+    float *parts = reinterpret_cast<float *>(ws + T16_FLAGS_BYTES);
+    __half *planes = reinterpret_cast<__half *>(ws + T16_FLAGS_BYTES + T16_PARTS_BYTES);
+    float *scale = reinterpret_cast<float *>(ws + T16_FLAGS_BYTES + T16_PARTS_BYTES + 2 * plane_bytes);
     alignas(64) Tc16Maps maps;
     std::memset(&maps, 0, sizeof(maps));
     if (!encode_w_map(&maps.w, W, n_out, nblocks * W_BLOCK_BYTES)) return -1;
@@ -1043,7 +1019,6 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
         if (g > grid) grid = (int)g;
     }
     P.stream_k = (tiles % grid != 0 && (grid > tiles || P.total_it / grid >= P.nblocks)) ? 1 : 0;
-    P.epoch = g_gemm_epoch.fetch_add(1) + 1u;
     const int n_chunks = (int)(n_in / 32);
     const uint32_t *x32 = static_cast<const uint32_t *>(Xq);
     // slices: whole passes of a block, as many as bring about two blocks per SM
@@ -1067,7 +1042,7 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN>, Y, P, (const float *)scale, parts, maps);
+    return (int)cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN>, Y, P, (const float *)scale, parts, flags, maps);
 }
 }  // extern "C++"
 // Tiles of 128 tokens from 96 tokens on (the code expansion, the kernel's busiest part, is paid once per tile), of 64 below.
@@ -1188,7 +1163,7 @@ int bonsai_p40_gemm(const void *W, const void *Xq, float *Y, int64_t n_out, int6
 }
 
 int bonsai_b200_gemm_release(void) {
-    std::lock_guard<std::mutex> lock(g_scratch_mu);
+    g_gemm_scratch.release();
     int dev = 0;
     const bool have = cudaGetDevice(&dev) == cudaSuccess;
     auto release = [&](auto &pool) {
@@ -1199,7 +1174,6 @@ int bonsai_b200_gemm_release(void) {
         }
         pool.clear();
     };
-    release(g_scratch);
     {
         std::lock_guard<std::mutex> attn_lock(g_attn_mu);
         release(g_attn_scratch);
@@ -1210,7 +1184,7 @@ int bonsai_b200_gemm_release(void) {
 
 int bonsai_b200_gemm_reserve(int64_t n_in, int64_t n_tok, bonsai_stream stream) {
     if (n_in <= 0 || n_in % 128 != 0 || n_tok <= 0 || n_tok > (1 << 28)) return 1;
-    return gemm_scratch(tc16_scratch_bytes(n_in, n_tok), as_stream(stream)) ? 0 : (int)cudaErrorMemoryAllocation;
+    return g_gemm_scratch.get(tc16_scratch_bytes(n_in, n_tok), as_stream(stream), true).ptr ? 0 : (int)cudaErrorMemoryAllocation;
 }
 
 int bonsai_b200_gemm_dump(const void *W, const void *Xq, float *Y, int32_t *sums, int64_t n_out, int64_t n_in,

@@ -24,8 +24,9 @@
 //   warps 24-25 : issuers (alternate blocks)
 //   warps 26-27 : loaders (tiled TMA copies): weight pieces of 8 blocks x 128 rows; per half block a box of 64 values x
 //                 64 tokens x {H, L}, landing swizzled as the MMA reads it
-// Work split and time-outs as in gemm_tc.cuh (same walk, same flag words); the parts of a tile meet in one step, through slots
-// in the scratch.
+// Work split and time-outs as in gemm_tc.cuh (same walk); the parts of a tile meet in one step, through slots and flags (one per CTA) in the
+// scratch, which is the stream's own.  (Flags in eight sets that launches took in turn were shared by the ninth launch on another
+// stream, or by a replayed one.)
 // Every role that feeds the tensor core is a serial chain per block, and each in turn was the kernel's period until it
 // was split or shortened (measured with per-role cycle stamps): descriptors built per MMA in a one-lane branch (70
 // cycles per MMA; now two adds in warp-uniform code), one loader polling two rings (1000 cycles per unit; now two
@@ -233,7 +234,7 @@ struct Tc16Maps {
 
 template <int TN>
 __global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *Y, const TcParams P, const float *__restrict__ tokscale, float *parts,
-                                                                         const __grid_constant__ Tc16Maps maps) {
+                                                                         unsigned int *flags, const __grid_constant__ Tc16Maps maps) {
     using C = T16C<TN>;
     constexpr int T16_N = TN, T16_ACC = C::ACC, T16_NB = C::NB, T16_BUNIT = C::BUNIT, T16_EPI_WARPS = C::EPI_WARPS,
                   T16_PROD_WARPS = C::PROD_WARPS, T16_PROD_SETS = C::PROD_SETS, T16_EPI_THREADS = C::EPI_THREADS,
@@ -286,7 +287,6 @@ __global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *
         // ---------------- epilogue: one weight row per thread, 32 tokens ----------------
         const int q = wid & 3, cg = wid >> 2;
         const int row_l = 32 * q + lane;
-        unsigned int *flags = g_gemm_flags[P.epoch & (TC_FLAG_SETS - 1)];
         bool ok = true;
         int n = 0;
         while (ok && walk.next(P, tile, kb0, kb1)) {
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *
                 for (int j = 0; j < T16_EPI_TOKS; ++j) slot[j * T16_M] = acc[j];
                 __threadfence();
                 asm volatile("bar.sync 1, %0;" ::"n"(T16_EPI_THREADS) : "memory");
-                if (threadIdx.x == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + blockIdx.x), "r"(P.epoch) : "memory");
+                if (threadIdx.x == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + blockIdx.x), "r"(1u) : "memory");
                 continue;
             }
             float *yrow = Y + (size_t)row * n_tok + tokb;
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *
                             ns = min(ns * 2, 256u);
                         }
                         if (!there) atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);
-                        *const_cast<volatile unsigned int *>(f) = 0u;     // lowered by its only reader (graph replays reuse the number)
+                        *const_cast<volatile unsigned int *>(f) = 0u;     // lowered by its only reader: the next launch on this scratch finds zeros
                     }
                 }
                 asm volatile("bar.sync 1, %0;" ::"n"(T16_EPI_THREADS) : "memory");

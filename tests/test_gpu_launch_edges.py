@@ -125,3 +125,44 @@ def test_rmsnorm_rows_held_and_not(gpu, port, n):
     assert torch.equal(odd.view(3, n), y)
     assert gpu.rmsnorm(xd, wd, xd, 3, n, 1e-6) == 0
     assert torch.equal(xd, y)
+
+
+def test_threads_on_their_per_thread_streams(gpu):
+    """Mat-muls cut into parts, from three host threads at once on cudaStreamPerThread (one handle, a stream per thread), with sizes that
+    make the scratch grow in between: every result has the bits of the same call made alone."""
+    import ctypes
+    import threading
+    import torch
+    per_thread = ctypes.c_void_p(2)
+    n_in, cases = 17408, [(128, 17), (640, 37), (300, 64)]
+    data = []
+    for i, (n_out, n_tok) in enumerate(cases):
+        W, Xq = dev(synth.pq2_0_weights(n_out, n_in, seed=i)), torch.empty(n_in // 32 * 36 * 130, dtype=torch.uint8, device="cuda")
+        assert gpu.quant_batch(dev(synth.activations(n_in, seed=i, batch=130)), None, Xq, n_in, 130, True) == 0
+        toks = [n_tok, n_tok + 3, 2 * n_tok]
+        data.append((W, Xq, n_out, toks, [[torch.zeros(n_out, t, device="cuda") for t in toks] for _ in range(21)]))
+    torch.cuda.synchronize()
+    fn = gpu.lib().bonsai_p40_gemm
+
+    def calls(i, rounds):
+        W, Xq, n_out, toks, Y = data[i]
+        for r in rounds:
+            for t, y in zip(toks, Y[r]):
+                failed.append(fn(W.data_ptr(), Xq.data_ptr(), y.data_ptr(), n_out, n_in, t, per_thread))
+
+    failed = []
+    for i in range(len(cases)):          # alone
+        calls(i, [0])
+        torch.cuda.synchronize()
+    threads = [threading.Thread(target=calls, args=(i, range(1, 21))) for i in range(len(cases))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not any(failed)
+    for _, _, _, toks, Y in data:
+        for r in range(1, 21):
+            for a, b in zip(Y[0], Y[r]):
+                assert torch.equal(a, b), r
+    assert gpu.device_status() == 0
