@@ -90,10 +90,16 @@ int bonsai_b200_gemm_dump(const void *W, const void *Xq, float *Y, int32_t *sums
  * 0, 1 for bad arguments, cudaErrorMemoryAllocation (2) when the buffer cannot be had.  No reference counterpart. */
 int bonsai_b200_gemm_reserve(int64_t n_in, int64_t n_tok, bonsai_stream stream);
 
-/* Frees every scratch buffer of bonsai_p40_gemm and of bonsai_p40_attn (all devices, all streams); they are otherwise kept
- * for the life of the process.  (Attention of 512 tokens and more keeps 2 KB per position and kv head for each of at most 16
- * streams of a device; a stream under capture gets none and runs the kernel that needs none.)  No mat-mul of this library may
- * be in flight or captured in a graph that will still be replayed.  Returns 0. */
+/* The same for bonsai_p40_attn, which keeps 2 KB per position and kv head per (device, stream) for prompts of 512 tokens and more: a
+ * captured call whose buffer is large enough gives the bits of a plain one, otherwise it runs the CUDA-core kernel, several times
+ * slower.  Returns 0 (also where no buffer is needed), 1 for bad arguments, 2 when the buffer cannot be had.  No reference counterpart. */
+int bonsai_b200_attn_reserve(int n_tok, int n_head_kv, bonsai_stream stream);
+
+/* Frees every scratch buffer of bonsai_p40_gemm and of bonsai_p40_attn (all devices, all streams).  They are otherwise kept for the
+ * life of the process, for at most 16 streams of a device each: a 17th takes the place of one that has not called for a while -- never of
+ * one that reserved its buffer or was captured with it -- or runs the kernel that needs none.  Graphs that were captured on one
+ * stream share its buffer with each other and with plain calls on that stream: let one follow the other.  No mat-mul or attention of this
+ * library may be in flight, or captured in a graph that will still be replayed, when this is called.  Returns 0. */
 int bonsai_b200_gemm_release(void);
 
 /* PTQ1_0: the denser packing of the same ternary weights, 28 bytes per 128 weights instead of 34 (described, not

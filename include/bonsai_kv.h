@@ -31,8 +31,8 @@ typedef struct bonsai_kv_cache bonsai_kv_cache;
 int64_t bonsai_kv_bytes(int capacity);
 int64_t bonsai_kv_gdn_bytes(void);
 
-/* Allocates cache, state and the decode workspace on the current device (the only calls of this library family that
- * allocate: as in the reference, src/kernels/kv_p40.cu:257-291); the state is zeroed on `stream`.  NULL on failure or
+/* Allocates cache, state and the decode workspace on the current device (as in the reference,
+ * src/kernels/kv_p40.cu:257-291); the state is zeroed on `stream`.  NULL on failure or
  * capacity <= 0.  bonsai_kv_reset zeroes the state again (position counters belong to the caller). */
 bonsai_kv_cache *bonsai_kv_create(int capacity, bonsai_stream stream);
 void bonsai_kv_free(bonsai_kv_cache *kv);

@@ -9,7 +9,8 @@
  * Common contract (reference: src/kernels/gemv_p40.cu:200-219, gemm_p40.cu:143-154,
  * gemv_repack_p40.cu:196-220, elementwise_p40.cu:75-80):
  *   - every pointer is a DEVICE pointer owned by the caller; the library allocates nothing,
- *     frees nothing and never synchronises; each call enqueues work on `stream` and returns;
+ *     frees nothing and never synchronises -- but for the scratch that bonsai_p40_gemm and bonsai_p40_attn keep, see
+ *     there; each call enqueues work on `stream` and returns;
  *   - return 0 on success, 1 on a rejected shape, otherwise the CUDA error code of the launch;
  *   - a call with nothing to do (n_out <= 0 where noted) returns 0 without launching.
  *
@@ -90,8 +91,10 @@ int bonsai_p40_gdn_step(float *state, const float *q, const float *k, const floa
 
 /* Causal attention, head_dim 256, grouped-query heads: q, out [n_tok][n_head][256]; k, v [n_tok][n_head_kv][256]
  * (16-byte aligned).  Returns 1 if head_dim != 256 or n_head % n_head_kv != 0; 0 without a launch if n_tok <= 0.
- * Online softmax, one key at a time (src/kernels/attn_p40.cu:92-118).  Replaces include/bonsai_p40.h:54 /
- * src/kernels/attn_p40.cu:131. */
+ * Online softmax, a tile of keys at a time; the reference's kernel takes one key at a time (src/kernels/attn_p40.cu:92-118).  From
+ * 512 tokens on the call keeps a scratch buffer per (device, stream), 2 KB per position and kv head: cudaMalloc, and when a longer
+ * prompt comes cudaFree, which waits for the device -- outside graph capture only (bonsai_b200_attn_reserve, bonsai_b200_gemm_release in
+ * bonsai_b200_ext.h).  Replaces include/bonsai_p40.h:54 / src/kernels/attn_p40.cu:131. */
 int bonsai_p40_attn(const float *q, const float *k, const float *v, float *out, int n_tok, int n_head,
                     int n_head_kv, int head_dim, float scale, bonsai_stream stream);
 

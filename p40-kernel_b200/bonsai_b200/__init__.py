@@ -43,6 +43,7 @@ SIGNATURES = {
     "bonsai_b200_gemv_dump": (_INT, [_VP, _VP, _VP, _VP, _I64, _I64, _VP]),
     "bonsai_b200_gemm_dump": (_INT, [_VP, _VP, _VP, _VP, _I64, _I64, _I64, _VP]),
     "bonsai_b200_gemm_reserve": (_INT, [_I64, _I64, _VP]),
+    "bonsai_b200_attn_reserve": (_INT, [_INT, _INT, _VP]),
     "bonsai_b200_gemm_release": (_INT, []),
     "bonsai_b200_ptq1_pack": (_INT, [_VP, _VP, _I64, _VP, _VP]),
     "bonsai_b200_ptq1_unpack": (_INT, [_VP, _VP, _I64, _VP]),
@@ -211,6 +212,11 @@ def gemm_dump(W, Xq, Y, sums, n_out, n_in, n_tok):
 
 def gemm_reserve(n_in, n_tok):
     return lib().bonsai_b200_gemm_reserve(n_in, n_tok, _stream())
+
+
+def attn_reserve(n_tok, n_head_kv):
+    """Allocates the prompt attention's scratch of the current stream for n_tok tokens (before capturing a graph on it)."""
+    return lib().bonsai_b200_attn_reserve(n_tok, n_head_kv, _stream())
 
 
 def gemm_release():

@@ -922,48 +922,11 @@ static bool encode_w_map(CUtensorMap *map, const void *W, int64_t n_out, int64_t
 // Scratch of the fp16 tensor-core mat-mul: a flag and a slot per CTA for its part of a tile, the activations as two fp16 planes, a
 // scale per token.  A call that gets none takes the integer kernel, which needs no scratch.
 static constexpr size_t T16_FLAGS_BYTES = (size_t)TC_MAX_CTAS * sizeof(unsigned int);
-static StreamScratch g_gemm_scratch(T16_FLAGS_BYTES);
+static StreamScratch g_gemm_scratch(T16_FLAGS_BYTES, false);
 
-// Scratch of the prompt attention (k and v as tile images: 2 KB per position and kv head, what k and v take themselves), kept
-// per stream and bounded: the 17th stream of a device takes the place of the one that called longest ago.  Streams are told
-// apart by their number, which no later stream is given again.  cudaFree waits for the device, so nothing in flight reads
-// what is freed; no graph holds an address (a stream under capture is given none).  The caller holds g_attn_mu until the
-// launches that use the buffer are enqueued.
-struct AttnScratch { int dev; unsigned long long stream, used; void *ptr; size_t bytes; };
-static std::mutex g_attn_mu;
-static std::vector<AttnScratch> g_attn_scratch;
-static void *attn_scratch(size_t bytes, cudaStream_t st) {
-    static unsigned long long calls = 0;
-    int dev = 0, of_dev = 0;
-    unsigned long long id = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaStreamGetId(st, &id) != cudaSuccess) return nullptr;
-    AttnScratch *e = nullptr, *oldest = nullptr;
-    for (auto &g : g_attn_scratch) {
-        if (g.dev != dev) continue;
-        ++of_dev;
-        if (g.stream == id) e = &g;
-        if (!oldest || g.used < oldest->used) oldest = &g;
-    }
-    if (!e && of_dev >= 16) e = oldest;
-    if (!e) {
-        g_attn_scratch.push_back(AttnScratch{dev, id, 0, nullptr, 0});
-        e = &g_attn_scratch.back();
-    }
-    if (e->stream != id || e->bytes < bytes) {
-        // another stream may be under capture: allocating is no part of that
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        (void)cudaThreadExchangeStreamCaptureMode(&mode);
-        if (e->ptr) (void)cudaFree(e->ptr);
-        e->ptr = nullptr;
-        e->bytes = 0;
-        e->stream = id;
-        if (cudaMalloc(&e->ptr, bytes) == cudaSuccess) e->bytes = bytes;
-        else e->ptr = nullptr, (void)cudaGetLastError();
-        (void)cudaThreadExchangeStreamCaptureMode(&mode);
-    }
-    e->used = ++calls;
-    return e->ptr;
-}
+// Scratch of the prompt attention: k and v as tile images, 2 KB per position and kv head, what k and v take themselves.  Prompts of one
+// conversation grow a little each time.  A call that gets none takes the CUDA-core kernel.
+static StreamScratch g_attn_scratch(0, true);
 
 static std::atomic<unsigned int> g_gemm_epoch{0};       // launch number of the tensor-core mat-muls (tags partial-tile flags)
 
@@ -1164,21 +1127,7 @@ int bonsai_p40_gemm(const void *W, const void *Xq, float *Y, int64_t n_out, int6
 
 int bonsai_b200_gemm_release(void) {
     g_gemm_scratch.release();
-    int dev = 0;
-    const bool have = cudaGetDevice(&dev) == cudaSuccess;
-    auto release = [&](auto &pool) {
-        for (auto &g : pool) {
-            if (!g.ptr) continue;
-            if (have) (void)cudaSetDevice(g.dev);
-            (void)cudaFree(g.ptr);
-        }
-        pool.clear();
-    };
-    {
-        std::lock_guard<std::mutex> attn_lock(g_attn_mu);
-        release(g_attn_scratch);
-    }
-    if (have) (void)cudaSetDevice(dev);
+    g_attn_scratch.release();
     return 0;
 }
 
@@ -1414,15 +1363,15 @@ int bonsai_p40_gdn_step(float *state, const float *q, const float *k, const floa
                        n_v_heads, K, V);
 }
 
-// Attention on the tensor cores (attn_tc.cuh).  -1: not taken (a stream that is being captured -- a graph would keep the
-// scratch's address -- or no scratch to be had).
+static size_t attn_scratch_bytes(int n_tok, int n_head_kv) { return (size_t)((n_tok + ATC_KEYS - 1) / ATC_KEYS) * n_head_kv * ATC_IMG_BYTES; }
+
+// Attention on the tensor cores (attn_tc.cuh).  -1: not taken (no scratch to be had).
 static int launch_attn_tc(const float *q, const float *k, const float *v, float *out, int n_tok, int n_head, int n_head_kv, float scale, cudaStream_t st) {
     const int tiles = (n_tok + ATC_KEYS - 1) / ATC_KEYS;
     const long long ctas = (long long)n_head * ((n_tok + ATC_M - 1) / ATC_M);
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (ctas > INT32_MAX || n_head_kv > 65535 || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return -1;
-    std::lock_guard<std::mutex> lock(g_attn_mu);
-    uint8_t *images = static_cast<uint8_t *>(attn_scratch((size_t)tiles * n_head_kv * ATC_IMG_BYTES, st));
+    if (ctas > INT32_MAX || n_head_kv > 65535) return -1;
+    const StreamScratch::Lease lease = g_attn_scratch.get(attn_scratch_bytes(n_tok, n_head_kv), st);      // held until both launches are enqueued
+    uint8_t *images = static_cast<uint8_t *>(lease.ptr);
     if (!images) return -1;
     static SmemOptIn opt;
     cudaError_t e = opt.ensure(attn_tc_kernel);
@@ -1431,6 +1380,12 @@ static int launch_attn_tc(const float *q, const float *k, const float *v, float 
     if (e == cudaSuccess)
         e = launch(attn_tc_kernel, dim3((unsigned)ctas), dim3(ATC_THREADS), (size_t)ATC_SMEM_BYTES, st, true, q, k, v, images, out, n_tok, n_head, n_head_kv, scale);
     return (int)e;
+}
+
+int bonsai_b200_attn_reserve(int n_tok, int n_head_kv, bonsai_stream stream) {
+    if (n_tok <= 0 || n_head_kv <= 0) return 1;
+    if (n_tok < ATC_MIN_TOKENS || n_head_kv > 65535) return 0;          // served without scratch
+    return g_attn_scratch.get(attn_scratch_bytes(n_tok, n_head_kv), as_stream(stream), true).ptr ? 0 : (int)cudaErrorMemoryAllocation;
 }
 
 int bonsai_p40_attn(const float *q, const float *k, const float *v, float *out, int n_tok, int n_head, int n_head_kv,

@@ -34,8 +34,9 @@ inline bool zero_new_memory(void *p, size_t bytes) {
 
 class StreamScratch {
 public:
-    // zeroed: the first bytes of a new buffer that the kernels expect to be zero (and leave zero behind)
-    explicit StreamScratch(size_t zeroed) : zeroed_(zeroed) {}
+    // zeroed: the first bytes of a new buffer that the kernels expect to be zero (and leave zero behind).  steps: a buffer that
+    // has become too small grows by half at least -- for calls whose need rises a little from one to the next.
+    StreamScratch(size_t zeroed, bool steps) : zeroed_(zeroed), steps_(steps) {}
 
     struct Lease {
         void *ptr = nullptr;                        // nullptr: none to be had
@@ -130,11 +131,13 @@ private:
         (void)cudaThreadExchangeStreamCaptureMode(&mode);
         if (b.in_graph) retire(d, b.ptr);
         else (void)cudaFree(b.ptr);
-        const bool reserved = b.stream == id && b.reserved;
+        const bool same = b.stream == id, reserved = same && b.reserved;
+        const size_t exact = bytes;
+        if (steps_ && same && bytes < b.bytes + b.bytes / 2) bytes = b.bytes + b.bytes / 2;
         b = Buffer();
         b.stream = id;
         b.reserved = reserved;
-        if (cudaMalloc(&b.ptr, bytes) != cudaSuccess) b.ptr = nullptr;
+        if (cudaMalloc(&b.ptr, bytes) != cudaSuccess && (bytes == exact || cudaMalloc(&b.ptr, bytes = exact) != cudaSuccess)) b.ptr = nullptr;
         if (b.ptr && zeroed_ && !zero_new_memory(b.ptr, zeroed_)) (void)cudaFree(b.ptr), b.ptr = nullptr;
         if (b.ptr) b.bytes = bytes;
         else (void)cudaGetLastError();
@@ -149,6 +152,7 @@ private:
     }
 
     const size_t zeroed_;
+    const bool steps_;
     Device devices_[DEVICES];
 };
 

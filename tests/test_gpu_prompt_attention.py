@@ -178,3 +178,64 @@ def test_values_of_any_size(gpu, size):
     out = torch.empty(n, heads, D, device="cuda")
     assert gpu.attn(q, k, v, out, n, heads, kv_heads, D, SCALE) == 0
     rows_close(out, exact(q, k, v))
+
+
+@pytest.mark.parametrize("how", ["reserve", "plain call"])
+def test_captured_with_a_buffer(gpu, how):
+    """A captured call on a stream that has a buffer gives the bits of a plain one, also when the stream's buffer has grown since: the
+    graph keeps its own."""
+    import torch
+    n, heads, kv_heads = 800, 6, 1
+    q, k, v = inputs(n, heads, kv_heads, 50)
+    big = inputs(1700, heads, kv_heads, 51)
+    want, out, out_big = (torch.empty(m, heads, D, device="cuda") for m in (n, n, 1700))
+    assert gpu.attn(q, k, v, want, n, heads, kv_heads, D, SCALE) == 0
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        if how == "reserve":
+            assert gpu.attn_reserve(n, kv_heads) == 0
+        else:
+            assert gpu.attn(q, k, v, out, n, heads, kv_heads, D, SCALE) == 0
+        with torch.cuda.graph(graph, stream=side):
+            assert gpu.attn(q, k, v, out, n, heads, kv_heads, D, SCALE) == 0
+        assert gpu.attn(*big, out_big, 1700, heads, kv_heads, D, SCALE) == 0
+    torch.cuda.current_stream().wait_stream(side)
+    for _ in range(3):
+        out.fill_(7.0)
+        graph.replay()
+        assert torch.equal(out, want)
+    close(out_big, exact(*big))
+    assert gpu.attn_reserve(0, 1) == 1 and gpu.attn_reserve(600, 0) == 1 and gpu.attn_reserve(100, 4) == 0
+    del graph
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    assert gpu.gemm_release() == 0
+    assert torch.cuda.mem_get_info()[0] > free0
+    assert gpu.device_status() == 0
+
+
+def test_buffers_are_bounded(gpu):
+    """200 streams one after the other, destroyed each: never more than 16 buffers, and new streams get one again.  (Buffers of 25 MB,
+    seen as device memory.)"""
+    import ctypes
+    import torch
+    n, heads, kv_heads = 1536, 8, 8
+    q, k, v = inputs(n, heads, kv_heads, 60)
+    want = exact(q, k, v)
+    rt = ctypes.CDLL("libcudart.so.12")
+    out = torch.empty(n, heads, D, device="cuda")
+    torch.cuda.synchronize()
+    assert gpu.gemm_release() == 0
+    free0, got = torch.cuda.mem_get_info()[0], set()
+    for i in range(200):
+        st = ctypes.c_void_p()
+        assert rt.cudaStreamCreate(ctypes.byref(st)) == 0
+        rc = gpu.lib().bonsai_p40_attn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), n, heads, kv_heads, D, SCALE, st)
+        torch.cuda.synchronize()
+        assert rc == 0 and rt.cudaStreamDestroy(st) == 0
+        if i % 20 == 0:
+            close(out, want)
+        got.add(free0 - torch.cuda.mem_get_info()[0])
+    assert max(got) <= 16 * 32 << 20 and max(got) >= 16 * 24 << 20
+    assert gpu.gemm_release() == 0
