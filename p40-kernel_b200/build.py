@@ -3,15 +3,17 @@
     python p40-kernel_b200/build.py [--force] [--verbose]
 
 Output: p40-kernel_b200/libbonsai_p40.so (same library name as the reference's build target, so a
-program linked with -lbonsai_p40 picks it up unchanged) and bonsai_b200/_calls.so (the Python package's
-native calls into it).  nvcc cross-compiles without a GPU.
+program linked with -lbonsai_p40 picks it up unchanged), then bonsai_b200/_calls*.so (the Python package's native
+calls into it; left out where there is no torch, which C and C++ programs do not need).  nvcc cross-compiles without a GPU.
 No fast-math: the quantiser and the rotation must perform IEEE divisions and separate mul / add.
 """
 import argparse
 import glob
+import importlib.metadata
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -28,7 +30,8 @@ FLAGS = [
 
 
 CALLS_SRC = os.path.join(CSRC, "python_calls.cpp")
-CALLS = os.path.join(HERE, "bonsai_b200", "_calls.so")
+CALLS = os.path.join(HERE, "bonsai_b200", "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+CALLS_STAMP = os.path.join(HERE, "build", "calls.stamp")      # what the present _calls file was built for
 
 
 def sources():
@@ -43,32 +46,52 @@ def stale(out=LIB, srcs=None):
     return any(os.path.getmtime(s) > t for s in (srcs or sources()))
 
 
+def compile_to(out, cmd):
+    """Runs cmd with a temporary output that takes out's place when it is complete."""
+    tmp = f"{out}.{os.getpid()}.tmp"
+    try:
+        subprocess.check_call([*cmd, "-o", tmp])
+        os.replace(tmp, out)
+    finally:
+        if os.path.exists(tmp):
+            os.remove(tmp)
+
+
 def build_calls(force=False):
-    """The native calls of the Python package (CPython extension, links against torch for tensors and streams)."""
-    if not (force or stale(CALLS, [CALLS_SRC])):
+    """The native calls of the Python package (CPython extension, links against torch for tensors and streams): built again
+    when the source, Python or torch has changed.  None where torch is not installed."""
+    try:
+        made_for = f"python {sys.version} torch {importlib.metadata.version('torch')}\n"
+    except importlib.metadata.PackageNotFoundError:
+        return None
+    stamp = open(CALLS_STAMP).read() if os.path.exists(CALLS_STAMP) else ""
+    if not (force or stamp != made_for or stale(CALLS, [CALLS_SRC])):
         return CALLS
-    import sysconfig
-    import torch
-    from torch.utils import cpp_extension
+    try:
+        import torch
+        from torch.utils import cpp_extension
+    except ImportError as e:
+        print(f"bonsai_b200: the Python calls are left out ({e})", file=sys.stderr)
+        return None
     inc = [*cpp_extension.include_paths("cuda"), sysconfig.get_paths()["include"]]
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
-                           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-                           *(f"-I{d}" for d in inc), "-o", CALLS, CALLS_SRC,
-                           f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
+    compile_to(CALLS, [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
+                       f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                       *(f"-I{d}" for d in inc), CALLS_SRC,
+                       f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
+    os.makedirs(os.path.dirname(CALLS_STAMP), exist_ok=True)
+    with open(CALLS_STAMP, "w") as f:
+        f.write(made_for)
     return CALLS
 
 
 def build(force=False, verbose=False, tuning=True):
     """tuning: compile the geometry knobs of bonsai_b200_set_option in (the parity tests force every tiling through
     them); a production build passes tuning=False (--no-tuning) and keeps only the documented options."""
+    if force or stale():
+        compile_to(LIB, [NVCC, *(["-Xptxas", "-v"] if verbose else []), *FLAGS, *(["-DBONSAI_B200_TUNING"] if tuning else []),
+                         os.path.join(CSRC, "bonsai_b200.cu")])
     build_calls(force)
-    if not (force or stale()):
-        return LIB
-    cmd = [NVCC, *FLAGS, *(["-DBONSAI_B200_TUNING"] if tuning else []), "-o", LIB, os.path.join(CSRC, "bonsai_b200.cu")]
-    if verbose:
-        cmd[1:1] = ["-Xptxas", "-v"]
-    subprocess.check_call(cmd)
     return LIB
 
 

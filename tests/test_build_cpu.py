@@ -1,0 +1,56 @@
+"""The build script: the C library needs no torch, and the Python calls follow torch and Python.  Compilers are replaced by a script
+that writes down its call and its output file."""
+import importlib.metadata
+import importlib.util
+import os
+import stat
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture
+def script(tmp_path, monkeypatch):
+    spec = importlib.util.spec_from_file_location("bonsai_b200_build_test", os.path.join(ROOT, "p40-kernel_b200", "build.py"))
+    b = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(b)
+    for tool in ("nvcc", "cxx"):
+        path = tmp_path / tool
+        path.write_text('#!/bin/sh\necho %s >> %s/log\nwhile [ "$1" != -o ]; do shift; done\necho made > "$2"\n' % (tool, tmp_path))
+        path.chmod(path.stat().st_mode | stat.S_IXUSR)
+    monkeypatch.setattr(b, "LIB", str(tmp_path / "lib.so"))
+    monkeypatch.setattr(b, "CALLS", str(tmp_path / "calls.so"))
+    if hasattr(b, "CALLS_STAMP"):
+        monkeypatch.setattr(b, "CALLS_STAMP", str(tmp_path / "stamps" / "calls.stamp"))
+    monkeypatch.setattr(b, "NVCC", str(tmp_path / "nvcc"))
+    monkeypatch.setenv("CXX", str(tmp_path / "cxx"))
+    b.stale.__defaults__ = (b.LIB, None)
+    b.log = lambda: (tmp_path / "log").read_text().split()
+    return b
+
+
+def test_library_without_torch(script, monkeypatch):
+    monkeypatch.setitem(sys.modules, "torch", None)
+    script.build()
+    assert script.log() == ["nvcc"] and os.path.exists(script.LIB)
+
+
+def test_calls_are_built_again_for_another_torch(script, monkeypatch):
+    script.build()
+    assert script.log() == ["nvcc", "cxx"]
+    script.build()
+    assert script.log() == ["nvcc", "cxx"]
+    real = importlib.metadata.version
+    monkeypatch.setattr(importlib.metadata, "version", lambda name: "99.0" if name == "torch" else real(name))
+    script.build()
+    assert script.log() == ["nvcc", "cxx", "cxx"]
+
+
+def test_a_failed_compiler_leaves_the_old_file(script, tmp_path):
+    script.build()
+    (tmp_path / "nvcc").write_text('#!/bin/sh\nwhile [ "$1" != -o ]; do shift; done\necho half > "$2"\nexit 1\n')
+    with pytest.raises(Exception):
+        script.build(force=True)
+    assert open(script.LIB).read() == "made\n"
