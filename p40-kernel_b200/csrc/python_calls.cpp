@@ -24,15 +24,38 @@ struct Mem { void *p; };
 struct Handle { void *p; };
 struct Truth { int v; };
 
+// An object that is no torch tensor but has a tensor's is_cuda, is_contiguous() and data_ptr().
+bool get_like_tensor(PyObject *o, const char *name, Mem &out) {
+    auto truth = [](PyObject *v) {
+        const int t = v ? PyObject_IsTrue(v) : -1;
+        Py_XDECREF(v);
+        return t;
+    };
+    const int cuda = truth(PyObject_GetAttrString(o, "is_cuda"));
+    if (cuda < 0) return false;
+    if (!cuda) {
+        PyErr_Format(PyExc_RuntimeError, "%s must be a CUDA tensor: this library has no CPU path", name);
+        return false;
+    }
+    const int contiguous = truth(PyObject_CallMethod(o, "is_contiguous", nullptr));
+    if (contiguous < 0) return false;
+    if (!contiguous) {
+        PyErr_Format(PyExc_RuntimeError, "%s must be contiguous", name);
+        return false;
+    }
+    PyObject *p = PyObject_CallMethod(o, "data_ptr", nullptr);
+    if (!p) return false;
+    out.p = PyLong_AsVoidPtr(p);
+    Py_DECREF(p);
+    return !PyErr_Occurred();
+}
+
 bool get(PyObject *o, const char *name, Mem &out) {
     if (o == Py_None) {
         out.p = nullptr;
         return true;
     }
-    if (!THPVariable_Check(o)) {
-        PyErr_Format(PyExc_TypeError, "%s must be a CUDA tensor, not %s", name, Py_TYPE(o)->tp_name);
-        return false;
-    }
+    if (!THPVariable_Check(o)) return get_like_tensor(o, name, out);
     const at::Tensor &t = THPVariable_Unpack(o);
     if (!t.is_cuda()) {
         PyErr_Format(PyExc_RuntimeError, "%s must be a CUDA tensor: this library has no CPU path", name);
@@ -42,7 +65,7 @@ bool get(PyObject *o, const char *name, Mem &out) {
         PyErr_Format(PyExc_RuntimeError, "%s must be contiguous", name);
         return false;
     }
-    out.p = const_cast<void *>(t.const_data_ptr());
+    out.p = t.mutable_data_ptr();           // outputs are written: a tensor that shares its memory until then gets its own, as by data_ptr()
     return true;
 }
 bool get(PyObject *o, const char *, Handle &out) {
