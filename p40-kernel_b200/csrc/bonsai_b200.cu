@@ -1478,8 +1478,8 @@ bonsai_kv_cache *bonsai_kv_create(int capacity, bonsai_stream stream) {
         return nullptr;
     }
     kv->d_counters = reinterpret_cast<unsigned int *>(reinterpret_cast<char *>(kv->d_ws) + ws);
-    // the counters are zero before the first launch on any stream: the wait is paid once per cache
-    if (cudaMemsetAsync(kv->d_counters, 0, ncnt, as_stream(stream)) != cudaSuccess || cudaStreamSynchronize(as_stream(stream)) != cudaSuccess) {
+    // the counters are zero before the first launch on any stream, and the caller's stream is not waited for
+    if (!zero_new_memory(kv->d_counters, ncnt)) {
         bonsai_kv_free(kv);
         return nullptr;
     }

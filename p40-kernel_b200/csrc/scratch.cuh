@@ -23,13 +23,19 @@
 
 namespace b200 {
 
-// Zeroes new device memory, complete on return, without a wait for any stream of the caller.
+// Zeroes new memory of the current device, complete on return, without a wait for any stream of the caller: on a stream of the library's own,
+// one per device, made when first needed (making one per call took milliseconds).
 inline bool zero_new_memory(void *p, size_t bytes) {
-    cudaStream_t own;
-    if (cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) != cudaSuccess) return false;
-    const bool ok = cudaMemsetAsync(p, 0, bytes, own) == cudaSuccess && cudaStreamSynchronize(own) == cudaSuccess;
-    (void)cudaStreamDestroy(own);
-    return ok;
+    static std::mutex mu;
+    static cudaStream_t own[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!own[dev] && cudaStreamCreateWithFlags(&own[dev], cudaStreamNonBlocking) != cudaSuccess) {
+        own[dev] = nullptr;
+        return false;
+    }
+    return cudaMemsetAsync(p, 0, bytes, own[dev]) == cudaSuccess && cudaStreamSynchronize(own[dev]) == cudaSuccess;
 }
 
 class StreamScratch {

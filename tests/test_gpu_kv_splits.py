@@ -156,3 +156,24 @@ def test_append_at_odd_offsets(gpu):
             a, b = ((layer * N_KV + h) * cap * 272 + 3 * 272 for layer in (2, 3))
             assert torch.equal(raw[a:a + 37 * 272], raw[b:b + 37 * 272]), h
     kv.close()
+
+
+def test_create_does_not_wait_for_the_stream(gpu):
+    """A cache is made while the caller's stream is busy (a kernel of a tenth of a second); decoding on another stream at once finds its
+    counters zero."""
+    import torch
+    gpu.KVCache(16).close()
+    busy, other, done = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Event()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(200_000_000)
+        done.record()
+        kv = gpu.KVCache(3000)
+        waited = done.query()
+    with torch.cuda.stream(other):
+        q, out = fill(kv, 1, 3000, 7, 0), torch.full((2, N_HEADS, D), float("nan"), device="cuda")
+        assert kv.attn_decode(1, 2999, q, out[0]) == 0 and kv.attn_decode(1, 2999, q, out[1]) == 0
+    torch.cuda.synchronize()
+    assert not waited
+    assert bool(torch.isfinite(out).all()) and torch.equal(out[0], out[1])
+    kv.close()
