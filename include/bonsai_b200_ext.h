@@ -126,8 +126,9 @@ int bonsai_b200_stream_probe(const void *buf, int64_t bytes, int mode, void *sin
 
 /* Launch options.  key "pdl": 1 = the weight stream of every mat-vec starts while the previous
  * kernel of the stream drains (weights must not be written by that previous kernel); 0 (default) =
- * only where the previous kernel is this library's own quantiser.  Launches overlap either way, and
- * wait for the previous kernel before they read what it may have written.
+ * only where the previous kernel is this library's own quantiser.
+ * key "overlap": 1 (default) = kernels are launched while the previous kernel of the stream drains and
+ * wait for it before they read what it may have written; 0 = plain launches, whatever "pdl" is.
  * key "gemv_order": 0 (default) = the streaming mat-vec, whose fp32 terms equal the host's bit for
  * bit and are added in a fixed tree order (outputs within 1e-5 of the host's, identical from launch
  * to launch); 1 = the mat-vec that also adds them in the host's sequential order (outputs

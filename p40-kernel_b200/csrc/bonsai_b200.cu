@@ -40,6 +40,7 @@ constexpr int SM_COUNT = 148;                 // B200
 constexpr int SMEM_LIMIT = 227 * 1024;        // dynamic shared memory a CTA may opt into
 
 std::atomic<int> g_opt_pdl{0};
+std::atomic<int> g_opt_overlap{1};             // 0: plain launches, each begins when its predecessor has ended
 std::atomic<int> g_opt_gemv_variant{-1};
 std::atomic<int> g_opt_gemv_order{0};
 std::atomic<int> g_opt_fuse_linear{0};         // 1: bonsai_b200_linear runs as one kernel when it can (measured slower)
@@ -80,7 +81,7 @@ cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
-    if (pdl) {
+    if (pdl && g_opt_overlap.load()) {
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
@@ -1276,6 +1277,7 @@ int bonsai_b200_stream_probe(const void *buf, int64_t bytes, int mode, void *sin
 int bonsai_b200_set_option(const char *key, int64_t value) {
     if (!key) return 1;
     if (!std::strcmp(key, "pdl")) { g_opt_pdl.store(value != 0); return 0; }
+    if (!std::strcmp(key, "overlap")) { g_opt_overlap.store(value != 0); return 0; }
     if (!std::strcmp(key, "gemv_order")) {
         if (value < 0 || value > 2) return 1;
         g_opt_gemv_order.store((int)value);
@@ -1546,7 +1548,7 @@ int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = g_opt_overlap.load() ? 2 : 1;
     return (int)cudaLaunchKernelEx(&cfg, kv_attn_kernel<KVM_GROUP>, q, (const uint8_t *)kv->d_k, (const uint8_t *)kv->d_v,
                                    kv->d_ws + (size_t)layer * kv_ws_floats(kv->max_clusters), kv->d_counters + layer * KV_COUNTERS, out,
                                    pos, chunk, KVM_KV_HEADS, kv->capacity, layer, 0.0625f);

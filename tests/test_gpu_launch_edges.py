@@ -166,3 +166,27 @@ def test_threads_on_their_per_thread_streams(gpu):
             for a, b in zip(Y[0], Y[r]):
                 assert torch.equal(a, b), r
     assert gpu.device_status() == 0
+
+
+def test_plain_launches(gpu):
+    """Option "overlap" = 0: the bits of the default, also with "pdl" = 1 beside it."""
+    import torch
+    n_out, n_in, n = 640, 5120, 300
+    W, x, sg = dev(synth.pq2_0_weights(n_out, n_in, seed=3)), dev(synth.activations(n_in, seed=3)), dev(synth.signs(n_in, seed=3))
+    kv = gpu.KVCache(n)
+    k, q = torch.randn(n, 4, 256, device="cuda"), torch.randn(24, 256, device="cuda")
+
+    def step():
+        xq, y, out = torch.empty(n_in // 32 * 36, dtype=torch.uint8, device="cuda"), torch.empty(n_out, device="cuda"), torch.empty(24, 256, device="cuda")
+        assert gpu.linear(W, x, sg, y, xq, n_out, n_in) == 0
+        assert kv.append_batch(3, 0, n, k, k) == 0 and kv.attn_decode(3, n - 1, q, out) == 0
+        return y, out
+
+    want = step()
+    try:
+        for pdl in (0, 1):
+            assert gpu.set_option("overlap", 0) == 0 and gpu.set_option("pdl", pdl) == 0
+            assert all(torch.equal(a, b) for a, b in zip(want, step()))
+    finally:
+        gpu.set_option("overlap", 1), gpu.set_option("pdl", 0)
+    kv.close()
