@@ -928,7 +928,7 @@ def prefill_leg(args, torch, bb, dist):
     except Exception:
         pass
     return {"metric": "pq2_0_prefill_gemm", "value": tops, "unit": "TOPS", "n_tok": n_tok, "ms_per_step": ms_step,
-            "steps": steps, "passes_per_step": reps, "gpu_launches": 4 * steps * reps, "per_matrix": per,
+            "steps": steps, "passes_per_step": reps, "gpu_launches": (6 if fp16_form else 4) * steps * reps, "per_matrix": per,
             "frac": tops / peak, "peak": peak,
             "peak_kind": (f"{kind} dense bf16; the kernel issues two fp16 MMAs per useful product, its ceiling is half"
                           if fp16_form else f"2 x {kind} dense bf16 (int8)"),
@@ -1052,7 +1052,7 @@ def beside_leg(args, torch, bb, dist):
             assert bb.gdn_step(s_, q, k, v, gg, be, o, nk, nv, K, V) == 0
     out["gdn_step_48_layers"] = rate(gdn, 2 * layers * nv * K * V * 4, layers)
     del st
-    # causal attention, prefill of 2048 tokens: 24 heads over 4 kv heads, head dimension 256, fp32 on the CUDA cores
+    # causal attention, prefill of 2048 tokens: 24 heads over 4 kv heads, head dimension 256, fp32 operands as two fp16 planes
     T, H, HKV, D = 2048, 24, 4, 256
     qa = torch.randn(T, H, D, generator=g).cuda()
     ka = torch.randn(T, HKV, D, generator=g).cuda()
@@ -1061,8 +1061,8 @@ def beside_leg(args, torch, bb, dist):
     ms, reps, _ = timed(torch, lambda: bb.attn(qa, ka, va, oa, T, H, HKV, D, 1.0 / 16.0), 3, 1, None, None, True)
     us = ms * 1e3 / (3 * reps)
     flops = 4.0 * H * D * (T * (T + 1) / 2)
-    out["attn_prefill_2048"] = {"TFLOP/s": flops / us / 1e6, "us": us, "bound": "fp32 FMA on the CUDA cores (no tensor cores: "
-                                "the reference's kernel and its test are fp32)", "gpu_launches": 1}
+    out["attn_prefill_2048"] = {"TFLOP/s": flops / us / 1e6, "us": us, "bound": "tensor cores (three fp16 plane products stand for one "
+                                "fp32 product) and their operand reads", "gpu_launches": 2}
     del qa, ka, va, oa
     # K/V cache: 32 768 positions in every one of the 16 cached layers (1.14 GB of Q8_0 blocks)
     P = 32768
@@ -1084,7 +1084,7 @@ def beside_leg(args, torch, bb, dist):
         def decode():
             for layer in range(16):
                 assert kv.attn_decode(layer, P - 1, qd, od) == 0
-        out["kv_attn_decode_16_layers_at_32768"] = rate(decode, 16 * P * 2 * 4 * 272, 32)
+        out["kv_attn_decode_16_layers_at_32768"] = rate(decode, 16 * P * 2 * 4 * 272, 16)
     finally:
         kv.close()
     # load-time steps on 5120 x 17408 x 8 copies (190 MB of PQ2_0): repack (read + write), PTQ1_0 pack and unpack
@@ -1158,7 +1158,7 @@ def batch_leg(args, torch, bb, dist, n_tok=8):
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         bad, worst = int(t[0].item()), float(t[1].item())
     peak, _, kind = measured_peaks()
-    kernels_per_call = 1 if n_tok <= 16 else 3      # streaming kernel; tensor cores: two launches prepare the fp16 planes
+    kernels_per_call = 1 if n_tok <= 16 else 2      # streaming kernel; tensor cores: a launch prepares the fp16 planes
     return {"metric": f"pq2_0_gemm_batch{n_tok}_weight_stream", "value": gbs, "unit": UNIT, "n_tok": n_tok, "us_per_sweep": us,
             "token_weight_gbs": gbs * n_tok, "gpu_launches": len(mats) * steps * reps * kernels_per_call,
             "frac": gbs / world / peak, "peak_kind": kind, "resident_weight_bytes": total_w,
@@ -1214,8 +1214,8 @@ def main():
                          "every rank's buffer (CUDA IPC mapping, no collective); auto = both are timed at start-up on the "
                          "box the benchmark runs on and the faster one is used for `value` and `e2e`")
     ap.add_argument("--seed", type=int, default=0)
-    ap.add_argument("--pdl", type=int, default=1, help="0 plain launches, 1 programmatic launches (weights of the next "
-                    "mat-vec stream while the previous kernel drains)")
+    ap.add_argument("--pdl", type=int, default=1, help="1: weights of the next mat-vec stream while the previous kernel "
+                    "drains, whatever that kernel is; 0: only behind the library's own quantiser")
     ap.add_argument("--cpu-seconds", type=float, default=8.0)
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--no-secondary", action="store_true", help="skip the decode-step / prefill / repack legs of the default line")
