@@ -382,11 +382,27 @@ GemvPlan plan_rows(long long n_out, size_t row_bytes, size_t fixed, int granule,
     return p;
 }
 
+// Whether a grid of small CTAs gains from being launched while its predecessor drains.  One that leaves much of the chip free does; one that
+// fills more than half of it, but not all of it, is spread unevenly when its first CTAs take what the predecessor leaves free (eight CTAs
+// per SM are resident: 2500 blocks through the rotation and the quantiser, 625 CTAs, 9.2 us and 11.9 with overlap; 629 CTAs of the
+// quantiser alone 2.9 and 3.3); a larger one does not care.
+bool worth_overlap(long long ctas, int upto_per_sm) { return ctas <= 4 * SM_COUNT || ctas > (long long)upto_per_sm * SM_COUNT; }
+
 // Any float pointers are taken, as by the reference; 16-byte aligned ones get 16-byte accesses.
 int launch_fwht(bool vec, const float *x, const float *signs, float *x_rot, void *xq, int64_t n_in, int64_t n_tok, bonsai_stream stream) {
     const long long blocks = (n_in / FWHT_N) * n_tok;
     if (blocks > INT32_MAX) return 1;
-    return (int)launch(vec ? fwht_quant_kernel<true> : fwht_quant_kernel<false>, dim3((unsigned)blocks), dim3(FWHT_THREADS), 0, as_stream(stream), true,
+    // A CTA per block for few blocks (a short chain, eight warps on it), a block per warp for many (a third of the instructions).  The line,
+    // in blocks per SM, with the times on both sides: 10 with the quantiser (1480 blocks: 6.5 us and 6.4, 1000: 5.0 and 5.5, 34816:
+    // 116 and 78); 18 where the rotated vector is stored as well or accesses are scalar (2500: 9.7 and 9.9, 3000: 11.3 and 11.0); 2 for
+    // the rotation alone (256: 2.3 and 2.2, 148: 2.0 and 2.4).
+    const bool warps = blocks > (long long)SM_COUNT * (!xq ? 2 : (x_rot || !vec ? 18 : 10));
+    const long long ctas = warps ? (blocks + FWHT_WARP_BLOCKS - 1) / FWHT_WARP_BLOCKS : blocks;
+    const bool overlap = worth_overlap(ctas, warps ? 8 : 6);
+    if (warps)
+        return (int)launch(vec ? fwht_quant_warp_kernel<true> : fwht_quant_warp_kernel<false>, dim3((unsigned)ctas), dim3(32 * FWHT_WARP_BLOCKS), 0,
+                           as_stream(stream), overlap, x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
+    return (int)launch(vec ? fwht_quant_kernel<true> : fwht_quant_kernel<false>, dim3((unsigned)ctas), dim3(FWHT_THREADS), 0, as_stream(stream), overlap,
                        x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
 }
 
@@ -400,7 +416,7 @@ int bonsai_p40_quant_activations(const float *x, void *out, int64_t n, bonsai_st
     const long long threads = n / 4;
     const int blocks = (int)((threads + 255) / 256);
     // any float pointer is taken, as by the reference; 16-byte aligned ones get 16-byte loads
-    return (int)launch(aligned16(x) ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, x,
+    return (int)launch(aligned16(x) ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), worth_overlap(blocks, 6), x,
                        static_cast<uint32_t *>(out), (int)n, 1);
 }
 
@@ -430,7 +446,7 @@ int bonsai_b200_quant_batch(const float *X, const float *signs, void *Xq, int64_
     const long long threads = n_in / 4 * n_tok;
     long long blocks = (threads + 255) / 256;
     if (blocks > 8 * SM_COUNT * 4) blocks = 8 * SM_COUNT * 4;
-    return (int)launch(vec ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, X,
+    return (int)launch(vec ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), worth_overlap(blocks, 6), X,
                        static_cast<uint32_t *>(Xq), (int)n_in, (int)n_tok);
 }
 

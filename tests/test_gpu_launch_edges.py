@@ -190,3 +190,32 @@ def test_plain_launches(gpu):
     finally:
         gpu.set_option("overlap", 1), gpu.set_option("pdl", 0)
     kv.close()
+
+
+@pytest.mark.parametrize("odd", [0, 1])
+@pytest.mark.parametrize("blocks", [1, 5, 296, 297, 298, 592, 593, 888, 889, 1480, 1481, 2664, 2665, 4737, 9473])
+def test_rotation_and_quantiser_forms(gpu, blocks, odd):
+    """Block counts on both sides of the forms' lines and of the overlap's: every block's bytes and rotated values are those of the block
+    alone, in one vector and in a batch of tokens."""
+    import torch
+    N, Q = 1024, 1152
+    g = torch.Generator(device="cuda").manual_seed(blocks)
+    x = torch.empty(blocks * N + 1, device="cuda")[odd:blocks * N + odd]
+    x.copy_(torch.randn(blocks * N, generator=g, device="cuda"))
+    sg = torch.randn(blocks * N, generator=g, device="cuda").sign()
+    ones = torch.randn(N, generator=g, device="cuda").sign()
+    new = lambda n, t=torch.float32: torch.zeros(n, dtype=t, device="cuda")
+    xq, both, xb, xn, rot, inplace = new(blocks * Q, torch.uint8), new(blocks * Q, torch.uint8), new(blocks * Q, torch.uint8), new(blocks * Q, torch.uint8), new(blocks * N), x.clone()
+    assert gpu.fwht_quant(x, sg, xq, None, blocks * N) == 0 and gpu.fwht_quant(x, sg, both, rot, blocks * N) == 0
+    assert gpu.fwht(inplace, sg, blocks * N) == 0
+    assert gpu.quant_batch(x, ones, xb, N, blocks, True) == 0 and gpu.quant_batch(x, None, xn, N, blocks, False) == 0
+    assert torch.equal(both, xq) and torch.equal(inplace, rot)
+    xb, xn = xb.view(32, blocks, 36), xn.view(32, blocks, 36)
+    for b in {0, 1 % blocks, blocks // 2, blocks - 1}:
+        one, q1, r1, part = x[b * N:(b + 1) * N].clone(), new(Q, torch.uint8), new(N), sg[b * N:(b + 1) * N].clone()
+        assert gpu.fwht_quant(one, part, q1, r1, N) == 0
+        assert torch.equal(xq[b * Q:(b + 1) * Q], q1) and torch.equal(rot[b * N:(b + 1) * N], r1), b
+        assert gpu.fwht_quant(one, ones, q1, None, N) == 0
+        assert torch.equal(xb[:, b].reshape(-1), q1), b
+        assert gpu.quant_activations(one, q1, N) == 0
+        assert torch.equal(xn[:, b].reshape(-1), q1), b
