@@ -51,9 +51,10 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const float *gate, const fl
 }
 
 // One CTA per row.  VEC (n % 4 == 0, all pointers 16-byte aligned): 16-byte accesses; otherwise scalar ones, same order of
-// sums.  A row of up to 8 slices per warp (8192 values: the model's width) stays in registers between the sum and the
-// product: bound by latency, it makes one trip to memory instead of two.
-constexpr int RMS_THREADS = 256, RMS_HOLD = 8;
+// sums.  HOLD > 0: rows of up to HOLD slices per warp stay in registers between the sum and the product, one trip to memory
+// instead of two; HOLD <= 0 takes rows of any length; HOLD < 0 with few registers, for many CTAs per SM.  A row of less than
+// eight slices has a warp per slice.
+constexpr int RMS_THREADS = 256, RMS_WARPS = RMS_THREADS / 32;
 template <bool VEC>
 __device__ __forceinline__ float4 rms_load(const float *p, int i, int n) {
     float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -82,9 +83,9 @@ __device__ __forceinline__ void rms_store(float *p, int i, int n, float4 f, floa
         if (i + 3 < n) p[i + 3] = f.w;
     }
 }
-template <bool VEC>
-__global__ void __launch_bounds__(RMS_THREADS) rmsnorm_kernel(const float *x, const float *w, float *y, int n, float eps) {
-    constexpr int NW = RMS_THREADS / 32;
+template <bool VEC, int HOLD>
+__global__ void __launch_bounds__(RMS_THREADS, HOLD < 0 ? 8 : (HOLD == 8 && !VEC ? 3 : 0)) rmsnorm_kernel(const float *x, const float *w, float *y, int n, float eps) {
+    constexpr int NW = RMS_WARPS;
     __shared__ float part[512];
     __shared__ float scale;
     const float *xr = x + (size_t)blockIdx.x * n;
@@ -93,14 +94,14 @@ __global__ void __launch_bounds__(RMS_THREADS) rmsnorm_kernel(const float *x, co
     const int nslice = (n + 127) >> 7;
     pdl_wait_prior_grid();
     pdl_launch_dependents();
-    if (nslice <= RMS_HOLD * NW) {
-        float4 f[RMS_HOLD], g[RMS_HOLD];
+    if constexpr (HOLD > 0) {
+        float4 f[HOLD], g[HOLD];
 #pragma unroll
-        for (int r = 0; r < RMS_HOLD; ++r) f[r] = rms_load<VEC>(xr, (wid + NW * r) * 128 + 4 * lane, n);
+        for (int r = 0; r < HOLD; ++r) f[r] = rms_load<VEC>(xr, (wid + NW * r) * 128 + 4 * lane, n);
 #pragma unroll
-        for (int r = 0; r < RMS_HOLD; ++r) g[r] = rms_load<VEC>(w, (wid + NW * r) * 128 + 4 * lane, n);
+        for (int r = 0; r < HOLD; ++r) g[r] = rms_load<VEC>(w, (wid + NW * r) * 128 + 4 * lane, n);
 #pragma unroll
-        for (int r = 0; r < RMS_HOLD; ++r) {
+        for (int r = 0; r < HOLD; ++r) {
             if (wid + NW * r >= nslice) break;              // warp-uniform
             const float s = slice_sumsq(f[r]);
             if (lane == 0) part[wid + NW * r] = s;
@@ -115,32 +116,44 @@ __global__ void __launch_bounds__(RMS_THREADS) rmsnorm_kernel(const float *x, co
         __syncthreads();
         const float sc = scale;
 #pragma unroll
-        for (int r = 0; r < RMS_HOLD; ++r) rms_store<VEC>(yr, (wid + NW * r) * 128 + 4 * lane, n, f[r], sc, g[r]);
-        return;
-    }
-    float acc = 0.0f;                               // rows longer than 512 slices: a part at a time, in ascending order
-    for (int s0 = 0; s0 < nslice; s0 += 512) {
-        for (int sl = s0 + wid; sl < min(nslice, s0 + 512); sl += NW) {
-            const float s = slice_sumsq(rms_load<VEC>(xr, sl * 128 + 4 * lane, n));
-            if (lane == 0) part[sl - s0] = s;
+        for (int r = 0; r < HOLD; ++r) rms_store<VEC>(yr, (wid + NW * r) * 128 + 4 * lane, n, f[r], sc, g[r]);
+    } else {
+        float acc = 0.0f;                           // rows longer than 512 slices: a part at a time, in ascending order
+        for (int s0 = 0; s0 < nslice; s0 += 512) {
+            for (int sl = s0 + wid; sl < min(nslice, s0 + 512); sl += NW) {
+                const float s = slice_sumsq(rms_load<VEC>(xr, sl * 128 + 4 * lane, n));
+                if (lane == 0) part[sl - s0] = s;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                for (int k = 0; k < min(512, nslice - s0); ++k) acc = __fadd_rn(acc, part[k]);
+                scale = rms_scale(acc, n, eps);
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int k = 0; k < min(512, nslice - s0); ++k) acc = __fadd_rn(acc, part[k]);
-            scale = rms_scale(acc, n, eps);
-        }
-        __syncthreads();
-    }
-    const float sc = scale;
-    for (int sl = wid; sl < nslice; sl += 4 * NW) {
-        float4 f[4], g[4];
+        const float sc = scale;
+        if (HOLD == 0) {
+            for (int sl = wid; sl < nslice; sl += 4 * NW) {
+                float4 f[4], g[4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            f[r] = rms_load<VEC>(xr, min(sl + NW * r, nslice) * 128 + 4 * lane, n);
-            g[r] = rms_load<VEC>(w, min(sl + NW * r, nslice) * 128 + 4 * lane, n);
-        }
+                for (int r = 0; r < 4; ++r) {
+                    f[r] = rms_load<VEC>(xr, min(sl + NW * r, nslice) * 128 + 4 * lane, n);
+                    g[r] = rms_load<VEC>(w, min(sl + NW * r, nslice) * 128 + 4 * lane, n);
+                }
 #pragma unroll
-        for (int r = 0; r < 4; ++r) rms_store<VEC>(yr, min(sl + NW * r, nslice) * 128 + 4 * lane, n, f[r], sc, g[r]);
+                for (int r = 0; r < 4; ++r) rms_store<VEC>(yr, min(sl + NW * r, nslice) * 128 + 4 * lane, n, f[r], sc, g[r]);
+            }
+        } else {
+            const int nt = (int)blockDim.x;
+            for (int i = threadIdx.x; i < n; i += 4 * nt) {          // (y may be x: the loads of a round first)
+                float f[4], g[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) f[r] = i + nt * r < n ? xr[i + nt * r] : 0.0f, g[r] = i + nt * r < n ? w[i + nt * r] : 0.0f;
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    if (i + nt * r < n) yr[i + nt * r] = __fmul_rn(__fmul_rn(f[r], sc), g[r]);
+            }
+        }
     }
 }
 

@@ -193,6 +193,29 @@ def test_plain_launches(gpu):
 
 
 @pytest.mark.parametrize("odd", [0, 1])
+@pytest.mark.parametrize("n", [60, 128, 1000, 1024, 1028, 2048, 3072, 3076, 5120, 5124, 8192, 8196])
+def test_rmsnorm_rows_and_forms(gpu, port, n, odd):
+    """Row counts on both sides of the forms' lines (two, three, four and eight rows per SM), in place too: every row has the bits of the
+    same row alone, and the first is the host's within the bound."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    w = torch.randn(n, generator=g, device="cuda")
+    for rows in (1, 296, 297, 444, 445, 592, 593, 1185):
+        x = torch.empty(rows * n + 1, device="cuda")[odd:rows * n + odd]
+        x.copy_(torch.randn(rows * n, generator=g, device="cuda"))
+        y = torch.full((rows, n), float("nan"), device="cuda")
+        assert gpu.rmsnorm(x, w, y, rows, n, 1e-6) == 0
+        for r in (0, rows // 2, rows - 1):
+            one = torch.empty(n, device="cuda")
+            assert gpu.rmsnorm(x[r * n:(r + 1) * n].clone(), w, one, 1, n, 1e-6) == 0
+            assert torch.equal(y[r], one), (rows, r)
+        want = port.rmsnorm(x[:n].cpu().numpy().reshape(1, n), w.cpu().numpy(), 1e-6)
+        assert np.abs(y[0].cpu().numpy() - want).max() <= REL_TOL * np.abs(want).max()
+        assert gpu.rmsnorm(x, w, x, rows, n, 1e-6) == 0
+        assert torch.equal(x.view(rows, n), y), rows
+
+
+@pytest.mark.parametrize("odd", [0, 1])
 @pytest.mark.parametrize("blocks", [1, 5, 296, 297, 298, 592, 593, 888, 889, 1480, 1481, 2664, 2665, 4737, 9473])
 def test_rotation_and_quantiser_forms(gpu, blocks, odd):
     """Block counts on both sides of the forms' lines and of the overlap's: every block's bytes and rotated values are those of the block
