@@ -5,11 +5,10 @@
 // HOST functions: fwht_blocks (src/fwht.h:20-42) and quantize_row_q8_1(..., permute = true)
 // (src/pq2_0.h:99-126).
 //
-// Both kernels are a handful of warps of latency-bound work (<= 70 KB in, <= 20 KB out per
-// decode vector), so the design goal is one launch and no shared-memory round trips:
-//   * rotation: one warp per 1024-block, 32 values per lane in registers; the ten butterfly
-//     stages run in the host's order (h = 1, 2, ..., 512), each output produced by exactly one
-//     a + b or a - b with a the lower-index operand, so the fp32 bits equal the host's;
+// A decode vector is a handful of latency-bound warps (<= 70 KB in, <= 20 KB out), a prompt's batch is bound by issue:
+//   * rotation: a CTA per 1024-block with a warp per slice of 128 for few blocks, a warp per block (32 values per lane in
+//     registers) for many; the ten butterfly stages run in the host's order (h = 1, 2, ..., 512), each output produced by
+//     exactly one a + b or a - b with a the lower-index operand, so the fp32 bits equal the host's in either form;
 //   * quantiser: eight lanes per 32-chunk, four values per lane (the same register layout the
 //     rotation leaves behind, which is what lets the two fuse without a shuffle stage between).
 #pragma once
@@ -96,7 +95,7 @@ __global__ void __launch_bounds__(256) quant_q8_1_kernel(const float *X, uint32_
     }
 }
 
-// ---- rotation: one warp per 1024-block ---------------------------------------------------------
+// ---- rotation of a 1024-block by one warp -------------------------------------------------------
 // Lane l holds v[r][e] = element r*128 + 4*l + e (r = 0..7, e = 0..3): index bits 0-1 are e,
 // bits 2-6 the lane, bits 7-9 r.
 __device__ __forceinline__ void fwht1024_warp(float (&v)[8][4], int lane) {

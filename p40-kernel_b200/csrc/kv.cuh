@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *K, uint8_t *V,
 //            2^-39 of the largest V scale of the split and of the warp's two blocks; where scales lie further apart than
 //            KV_V_RANGE, a second pass over the tile multiplies what they left.
 // What bounded the kernel before was instruction issue (5860 warp instructions per 32 positions: fp32 multiply-adds of
-// every value for every head on the CUDA cores; 1500 GB/s).  This form issues about 1500.
+// every value for every head on the CUDA cores; 1500 GB/s).  This form issues 2700, start and merge included.
 //
 // 34-byte blocks: two blocks are 17 words.  Of an even block words 1 .. 7 are eight-aligned code words and word 0's high
 // and word 8's low half make the eighth ("slot 0" = values 0, 1, 30, 31, slot i = values 4 i - 2 .. 4 i + 1); the odd block's
