@@ -209,9 +209,10 @@ __device__ __forceinline__ uint64_t policy_evict_last_or_default() {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// A coherent load that stays behind the wait (both are volatile), and that the compiler may take in front of stores to shared memory.
 __device__ __forceinline__ uint32_t ldg_u32(const void *p) {
     uint32_t v;
-    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ uint32_t ldg_nc_u16(const void *p) {
