@@ -20,9 +20,9 @@
 //   weights x v              |
 // Shared memory: q high, k and v images of one tile, 64 KB each (K-major, 128-byte swizzle).  Tensor memory, all 512
 // columns: 256 output (before that, sums of the scores), 128 scores (then weights), 128 q low.
-// What bounds it: per tile 5900 of 10200 cycles are the tensor core's, most of them the score products (N = 64: it waits for
-// the q rows from shared memory), the rest softmax and the exchanges in front of it.  2048 tokens, 24 heads over 4: 2570 ->
-// 293 us; 1000 tokens 727 -> 94 us, 517 tokens 246 -> 59 us.
+// What bounds it (counted while a score was four sums): per tile 5900 of 10200 cycles were the tensor core's, most of them the score
+// products (N = 64: it waits for the q rows from shared memory), the rest softmax and the exchanges in front of it.  2048 tokens, 24 heads over 4: 2570 ->
+// 292 us; 1000 tokens 727 -> 94 us, 517 tokens 246 -> 59 us.
 //
 // A plane pair holds 2^-39 of the largest value under its power of two, so what is far smaller loses bits to values that a row may not
 // even see.  A CTA whose queries and keys range too widely (atc_too_wide) does its queries again on the CUDA cores (attn_simt), with
