@@ -58,6 +58,12 @@ __global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *K, uint8_t *V,
     const float *kr = ksrc + (size_t)row * KV_D + blk * 32 + sub * 8;
     const float *vr = vsrc + (size_t)row * KV_D + blk * 32 + sub * 8;
     float kx[8], vx[8];
+    // The rows, asked for while the launch before this one still runs (L2 hands out what it finds at the load, whoever writes in
+    // between): 512 tokens in 16 layers 61.8 -> 53.5 us.  (The first tiles of the attention below, asked for likewise: no gain.)
+    if (sub == 0) {
+        prefetch_l2(kr);
+        prefetch_l2(vr);
+    }
     pdl_wait_prior_grid();
     pdl_launch_dependents();
     if (VEC) {
