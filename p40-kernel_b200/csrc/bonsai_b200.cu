@@ -1459,27 +1459,36 @@ inline int64_t kv_gdn_bytes() { return (int64_t)KVM_LINEAR * KVM_V_HEADS * KVM_S
 constexpr int KV_COUNTERS = KVM_KV_HEADS * KV_CLUSTER;      // per layer
 inline size_t kv_ws_floats(int max_clusters) { return (size_t)KVM_KV_HEADS * KV_CLUSTER * max_clusters * KV_REC; }      // per layer
 
-// Clusters of the decode kernel per kv head that are resident at once on the current device (0: it does not run here).  Asked
-// once per device.
-int kv_max_clusters() {
-    static std::atomic<int> known[64];
-    static SmemOptIn opt;
+// Clusters (of 8 or of 16 CTAs) of the decode kernel per kv head that are resident at once on the current device (0: they do not run
+// here).  Asked once per device.
+int kv_max_clusters(bool wide) {
+    static std::atomic<int> known[2][64];
+    static SmemOptIn opt[2];
     int dev = 0, resident = 0;
-    if (opt.ensure(kv_attn_kernel<KVM_GROUP>) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (dev < 64 && (resident = known[dev].load(std::memory_order_relaxed)) > 0) return resident;
+    auto *kernel = wide ? kv_attn_kernel<KVM_GROUP, KV_WIDE_CLUSTER> : kv_attn_kernel<KVM_GROUP, KV_CLUSTER>;
+    if (opt[wide].ensure(kernel) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev < 64 && (resident = known[wide][dev].load(std::memory_order_relaxed)) > 0) return resident;
+    if (wide && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    const unsigned cluster = wide ? KV_WIDE_CLUSTER : KV_CLUSTER;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(KV_CLUSTER * KV_MAX_CLUSTERS, KVM_KV_HEADS);
+    cfg.gridDim = dim3(cluster * KV_MAX_CLUSTERS, KVM_KV_HEADS);
     cfg.blockDim = dim3(KV_THREADS);
     cfg.dynamicSmemBytes = KV_SMEM_BYTES;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = KV_CLUSTER;
+    attr[0].val.clusterDim.x = cluster;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&resident, kv_attn_kernel<KVM_GROUP>, &cfg) != cudaSuccess || resident <= 0) return 0;
+    if (cudaOccupancyMaxActiveClusters(&resident, kernel, &cfg) != cudaSuccess || resident <= 0) {
+        (void)cudaGetLastError();
+        return 0;
+    }
     resident = std::min(std::max(resident / KVM_KV_HEADS, 1), KV_MAX_CLUSTERS);
-    if (dev < 64) known[dev].store(resident, std::memory_order_relaxed);
+    if (dev < 64) known[wide][dev].store(resident, std::memory_order_relaxed);
     return resident;
 }
 }  // namespace
@@ -1491,6 +1500,7 @@ struct bonsai_kv_cache {
     unsigned int *d_counters = nullptr;         // behind the workspace's records; records and counters are a layer's own, so
                                                 // that layers may be decoded on different streams at once
     int max_clusters = 1;                       // clusters of the decode kernel per kv head that are resident at once
+    bool wide_clusters = false;                 // clusters of 16 run here
 };
 
 int64_t bonsai_kv_bytes(int capacity) {
@@ -1506,7 +1516,8 @@ bonsai_kv_cache *bonsai_kv_create(int capacity, bonsai_stream stream) {
     bonsai_kv_cache *kv = new (std::nothrow) bonsai_kv_cache;
     if (!kv) return nullptr;
     kv->capacity = capacity;
-    kv->max_clusters = kv_max_clusters();
+    kv->max_clusters = kv_max_clusters(false);
+    kv->wide_clusters = kv_max_clusters(true) > 0;
     const size_t ws = (size_t)KVM_FULL * kv_ws_floats(kv->max_clusters) * sizeof(float), ncnt = (size_t)KVM_FULL * KV_COUNTERS * sizeof(unsigned int);
     if (kv->max_clusters <= 0 || cudaMalloc(&kv->d_k, (size_t)kv_array_bytes(capacity)) != cudaSuccess ||
         cudaMalloc(&kv->d_v, (size_t)kv_array_bytes(capacity)) != cudaSuccess || cudaMalloc(&kv->d_gdn, (size_t)kv_gdn_bytes()) != cudaSuccess ||
@@ -1569,7 +1580,13 @@ int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *
     long long n_cl = n_pos / (KV_CLUSTER * KV_SPLIT_MIN);
     if (n_cl < 1) n_cl = 1;
     if (n_cl > kv->max_clusters) n_cl = kv->max_clusters;
-    const int n_split = (int)n_cl * KV_CLUSTER;
+    // One cluster of 16 where one or two of eight would do and each of their splits would have more than a tile: 701 positions are a
+    // tile a split, not two one after the other, and 2048 need no merge through memory.  16 layers with their appends, in us, with
+    // clusters of 8 and of 16: 701 positions 150 / 127, 1501 184 / 150, 2048 191 / 159, 3001 215 / 185.  Up to 512 a split of eight
+    // is one tile already; from 3072 on three clusters of eight have more splits.
+    const bool wide = kv->wide_clusters && n_cl <= 2 && n_pos > KV_CLUSTER * KV_TILE;
+    const int cluster = wide ? KV_WIDE_CLUSTER : KV_CLUSTER;
+    const int n_split = wide ? KV_WIDE_CLUSTER : (int)n_cl * KV_CLUSTER;
     const int chunk = (((n_pos + n_split - 1) / n_split) + 15) / 16 * 16;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_split, KVM_KV_HEADS);
@@ -1578,13 +1595,13 @@ int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *
     cfg.stream = as_stream(stream);
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = KV_CLUSTER;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_opt_overlap.load() ? 2 : 1;
-    return (int)cudaLaunchKernelEx(&cfg, kv_attn_kernel<KVM_GROUP>, q, (const uint8_t *)kv->d_k, (const uint8_t *)kv->d_v,
+    return (int)cudaLaunchKernelEx(&cfg, wide ? kv_attn_kernel<KVM_GROUP, KV_WIDE_CLUSTER> : kv_attn_kernel<KVM_GROUP, KV_CLUSTER>, q, (const uint8_t *)kv->d_k, (const uint8_t *)kv->d_v,
                                    kv->d_ws + (size_t)layer * kv_ws_floats(kv->max_clusters), kv->d_counters + layer * KV_COUNTERS, out,
                                    pos, chunk, KVM_KV_HEADS, kv->capacity, layer, 0.0625f);
 }

@@ -113,8 +113,9 @@ __global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *K, uint8_t *V,
 // Splits: the CTAs of a cluster share one kv head; their (m, l, acc) meet through distributed shared memory, every CTA of
 // the cluster merging one slice of the dims.  With more than one cluster per head the merged slices go to a workspace and
 // the last cluster to arrive at a slice's counter adds them up and writes the output: one launch per call (the merge was
-// a kernel of its own).
-constexpr int KV_THREADS = 128, KV_WARPS = 4, KV_BUFS = 2, KV_CLUSTER = 8;
+// a kernel of its own).  Clusters of 16 serve the lengths where they halve the tiles of a split (513 positions on) and where two
+// clusters of eight would need the second merge (up to 3071).
+constexpr int KV_THREADS = 128, KV_WARPS = 4, KV_BUFS = 2, KV_CLUSTER = 8, KV_WIDE_CLUSTER = 16;
 constexpr int KV_HALF_BYTES = KV_TILE * KV_ROW;                      // the K (or V) rows of a tile
 constexpr int KV_WT_STRIDE = KV_TILE + 8;                            // weights of a head: 8 g + 2 t are 32 different banks
 constexpr int KV_SLICE = KV_D / KV_CLUSTER;                          // output dims a CTA of the cluster merges
@@ -177,10 +178,10 @@ __device__ __forceinline__ float ld_cluster_f32(const float *p, uint32_t rank) {
     return v;
 }
 
-// grid (n_split, n_kv_head), cluster (KV_CLUSTER, 1, 1), n_split a multiple of KV_CLUSTER; split s covers positions
+// grid (n_split, n_kv_head), cluster (CL, 1, 1), n_split a multiple of CL (KV_WIDE_CLUSTER: one cluster per head); split s covers positions
 // s * chunk .. min((s + 1) * chunk, pos + 1) - 1 (a split may be empty).  counters: one per (kv head, slice), zero before
 // and after every launch.
-template <int GRP>
+template <int GRP, int CL = KV_CLUSTER>
 __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, const uint8_t *K, const uint8_t *V, float *ws, unsigned int *counters, float *out,
                                                                 int pos, int chunk, int n_kv_head, int capacity, int layer, float scale) {
     static_assert(GRP <= KV_MAX_GROUP, "");
@@ -476,55 +477,63 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
     cluster_wait();
     // ---- one slice of the dims per CTA of the cluster, added over its CTAs in rank order
     const uint32_t rank = cluster_rank();
-    const int n_cl = gridDim.x / KV_CLUSTER, cl = blockIdx.x / KV_CLUSTER;
-    float *cw = wt, *cm = mw, *cl_sum = lw;                            // [8 heads][8 ranks] weights; maxima; denominators
-    constexpr int OUTS = GRP * KV_SLICE, ROUNDS = (OUTS + KV_THREADS - 1) / KV_THREADS;
-    float part[ROUNDS][KV_CLUSTER];
+    const int n_cl = gridDim.x / CL, cl = blockIdx.x / CL;
+    constexpr int SLICE = KV_D / CL;
+    float *cw = wt, *cm = mw, *cl_sum = lw;                            // [8 heads][CL ranks] weights; maxima; denominators
+    constexpr int OUTS = GRP * SLICE, ROUNDS = (OUTS + KV_THREADS - 1) / KV_THREADS;
+    float part[ROUNDS][CL];
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
         const int o = tid + r * KV_THREADS;
 #pragma unroll
-        for (int rr = 0; rr < KV_CLUSTER; ++rr)
-            part[r][rr] = o < OUTS ? ld_cluster_f32(so + (o / KV_SLICE) * KV_D + (int)rank * KV_SLICE + o % KV_SLICE, (uint32_t)rr) : 0.0f;
+        for (int rr = 0; rr < CL; ++rr)
+            part[r][rr] = o < OUTS ? ld_cluster_f32(so + (o / SLICE) * KV_D + (int)rank * SLICE + o % SLICE, (uint32_t)rr) : 0.0f;
     }
-    if (warp < 2) {
-        const int h = tid >> 3, rr = tid & 7;
+    static_assert(KV_MAX_GROUP * CL <= KV_THREADS, "a thread weighs one head of one rank");
+    if (tid < KV_MAX_GROUP * CL) {
+        const int h = tid / CL, rr = tid % CL;
         const float mm = h < GRP ? ld_cluster_f32(sm + h, (uint32_t)rr) : -INFINITY;
         const float ll = h < GRP ? ld_cluster_f32(sl + h, (uint32_t)rr) : 0.0f;
         float mx = mm;
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (int o = 1; o < CL; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float w = mm == -INFINITY ? 0.0f : expf(__fsub_rn(mm, mx));      // a split without positions: 0
         float den = __fmul_rn(ll, w);
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) den = __fadd_rn(den, __shfl_xor_sync(0xffffffffu, den, o));
-        cw[h * 8 + rr] = w;
+        for (int o = 1; o < CL; o <<= 1) den = __fadd_rn(den, __shfl_xor_sync(0xffffffffu, den, o));
+        cw[h * CL + rr] = w;
         if (rr == 0) cm[h] = mx, cl_sum[h] = den;
     }
     __syncthreads();
     cluster_arrive();                   // this CTA has read its share of the others' memory (it leaves when all have: cluster_wait)
-    float *rec = ws + (((size_t)kvh * KV_CLUSTER + rank) * n_cl + cl) * KV_REC;
-    float *out_slice = out + (size_t)kvh * GRP * KV_D + (int)rank * KV_SLICE;
+    float *rec = ws + (((size_t)kvh * CL + rank) * n_cl + cl) * KV_REC;
+    float *out_slice = out + (size_t)kvh * GRP * KV_D + (int)rank * SLICE;
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
         const int o = tid + r * KV_THREADS;
         if (o < OUTS) {
-            const int h = o / KV_SLICE;
-            float a = 0.0f;
+            const int h = o / SLICE;
+            float chain[CL / 4];                // of four ranks: sixteen in one sum round more than eight did
 #pragma unroll
-            for (int rr = 0; rr < KV_CLUSTER; ++rr) a = __fmaf_rn(part[r][rr], cw[h * 8 + rr], a);
-            if (n_cl == 1) out_slice[h * KV_D + o % KV_SLICE] = __fmul_rn(a, __fdiv_rn(1.0f, cl_sum[h]));
+            for (int c = 0; c < CL / 4; ++c) {
+                chain[c] = 0.0f;
+#pragma unroll
+                for (int rr = 4 * c; rr < 4 * c + 4; ++rr) chain[c] = __fmaf_rn(part[r][rr], cw[h * CL + rr], chain[c]);
+            }
+            float a = __fadd_rn(chain[0], chain[1]);
+            if (CL == 16) a = __fadd_rn(a, __fadd_rn(chain[2], chain[CL / 4 - 1]));
+            if (n_cl == 1) out_slice[h * KV_D + o % SLICE] = __fmul_rn(a, __fdiv_rn(1.0f, cl_sum[h]));
             else rec[o] = a;
         }
     }
     int last = 0;
     if (n_cl > 1) {
         if (tid < GRP) {
-            rec[KV_MAX_GROUP * KV_SLICE + tid] = cm[tid];
-            rec[KV_MAX_GROUP * KV_SLICE + KV_MAX_GROUP + tid] = cl_sum[tid];
+            rec[KV_MAX_GROUP * SLICE + tid] = cm[tid];
+            rec[KV_MAX_GROUP * SLICE + KV_MAX_GROUP + tid] = cl_sum[tid];
         }
         __syncthreads();
-        if (tid == 0) last = count_arrival(counters + kvh * KV_CLUSTER + rank) == (unsigned int)n_cl - 1u;
+        if (tid == 0) last = count_arrival(counters + kvh * CL + rank) == (unsigned int)n_cl - 1u;
         last = __syncthreads_or(last);
     }
     if (!last) {
@@ -533,18 +542,18 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
     }
     // ---- several clusters per head: the last one to bring this slice adds them in order (fixed, whichever is last).  All
     // loads go out before the weights are formed: one trip to L2 (a dependent trip per step took 5 us).
-    if (tid == 0) counters[kvh * KV_CLUSTER + rank] = 0u;
-    const float *all = ws + ((size_t)kvh * KV_CLUSTER + rank) * n_cl * KV_REC;
+    if (tid == 0) counters[kvh * CL + rank] = 0u;
+    const float *all = ws + ((size_t)kvh * CL + rank) * n_cl * KV_REC;
     constexpr int BATCH = 16, PAIRS = OUTS / 2;
     static_assert(PAIRS <= KV_THREADS, "a thread adds one pair of outputs");
-    const int ho = min(tid, PAIRS - 1) / (KV_SLICE / 2);
+    const int ho = min(tid, PAIRS - 1) / (SLICE / 2);
     float2 v[BATCH];
 #pragma unroll
     for (int c = 0; c < BATCH; ++c)
         v[c] = (tid < PAIRS && c < n_cl) ? __ldcg(reinterpret_cast<const float2 *>(all + (size_t)c * KV_REC) + tid) : make_float2(0.0f, 0.0f);
     float *fm = reinterpret_cast<float *>(raw + 16384), *fl = fm + KV_MAX_CLUSTERS * KV_MAX_GROUP, *fw = fl + KV_MAX_CLUSTERS * KV_MAX_GROUP;
     for (int i = tid; i < n_cl * KV_MAX_GROUP; i += KV_THREADS) {
-        const float *ml = all + (size_t)(i / KV_MAX_GROUP) * KV_REC + KV_MAX_GROUP * KV_SLICE + i % KV_MAX_GROUP;
+        const float *ml = all + (size_t)(i / KV_MAX_GROUP) * KV_REC + KV_MAX_GROUP * SLICE + i % KV_MAX_GROUP;
         const bool use = i % KV_MAX_GROUP < GRP;
         fm[i] = use ? __ldcg(ml) : 0.0f;
         fl[i] = use ? __ldcg(ml + KV_MAX_GROUP) : 0.0f;
@@ -571,7 +580,7 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
             b = __fmaf_rn(x.y, fw[c * KV_MAX_GROUP + ho], b);
         }
         const float inv = __fdiv_rn(1.0f, den);
-        float *o2 = out_slice + ho * KV_D + 2 * (tid % (KV_SLICE / 2));
+        float *o2 = out_slice + ho * KV_D + 2 * (tid % (SLICE / 2));
         o2[0] = __fmul_rn(a, inv);
         o2[1] = __fmul_rn(b, inv);
     }
