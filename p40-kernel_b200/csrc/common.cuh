@@ -158,6 +158,30 @@ __device__ __forceinline__ bool mbar_wait_hot(uint64_t *bar, uint32_t parity) {
     if (ok) return true;
     return mbar_wait_bounded(bar, parity, 32, 128);
 }
+// The same wait in the hardware's blocking form: a dozen warps that wait for the same thing need no sleeps between their polls.
+__device__ __forceinline__ bool mbar_wait_suspended(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .u32 n;\n\t"
+        "mov.u32 n, %3;\n\t"
+        "mov.u32 %0, 1;\n\t"
+        "TRY_LOOP:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra TRY_DONE;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "setp.ne.u32 p, n, 0;\n\t"
+        "@p bra TRY_LOOP;\n\t"
+        "mov.u32 %0, 0;\n\t"
+        "TRY_DONE:\n\t"
+        "}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(1u << 24)
+        : "memory");
+    if (!ok) atomicExch(&g_device_status, STATUS_MBARRIER_TIMEOUT);
+    return ok != 0;
+}
 // One non-blocking poll: has the phase with this parity completed?
 __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
     uint32_t ok;

@@ -57,6 +57,7 @@ constexpr int CHAIN_MAX_SLOTS = 16;
 constexpr int CHAIN_OP_RING = 8;
 constexpr int CHAIN_TABLES = 3;          // activation-table buffers: the sequencer prepares this many inputs ahead
 constexpr uint32_t CHAIN_NS0 = 32, CHAIN_NSMAX = 256;             // first and longest sleep between two polls of a wait
+constexpr uint32_t CHAIN_MEET_NSMAX = 64;                         // ... of the waits that hold up the whole grid
 constexpr uint32_t CHAIN_GATE_NS0 = 32, CHAIN_GATE_NSMAX = 256;   // ... of the waits that usually last microseconds
 constexpr int CHAIN_GATES = 3;           // a warp may run this many ops ahead of the slowest one
 
@@ -134,7 +135,7 @@ __device__ __forceinline__ bool grid_counter_wait(const unsigned int *counter, u
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
         if ((int)(v - target) >= 0) return true;
         __nanosleep(ns);
-        ns = min(ns * 2, CHAIN_NSMAX);
+        ns = min(ns * 2, CHAIN_MEET_NSMAX);
     }
     atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);
     return false;
@@ -193,6 +194,43 @@ struct ChainPeers {
     unsigned int *counter[CHAIN_MAX_RANKS];     // rank p's counter block
 };
 
+// Back butterflies and quantiser of a warp's units (u0, u0 + step, ... of `units` slices of the scratch area) into the tables, up to
+// three side by side: one after the other they took 1600 clocks each, a chain of shuffles and divisions.  Not inlined: beside the multiply's
+// registers it would spill, and a spilled value of the multiply costs more than this saves.
+template <int N>
+__device__ __forceinline__ void chain_back_units(const float4 *scratch, int u0, int step, int units, int chunk0, int lane, uint32_t *act_q, float *act_s, int *act_i) {
+    float v[N][4];
+    uint32_t word[N], header[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int u = min(u0 + k * step, units - 1);                // (a warp with one less does the last again, stores nothing)
+        fwht_slice_back(scratch + (u >> 3) * 256, u & 7, lane, v[k]);
+    }
+    quantise_chunks_8lanes<N>(v, lane, word, header);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int u = u0 + k * step;
+        if (u < units) {
+            const int chunk = chunk0 + u * 4 + (lane >> 3);
+            act_q[(chunk >> 2) * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word[k];
+            if ((lane & 7) == 0) {
+                act_s[chunk] = f16_bits_to_f32(header[k] & 0xFFFFu);
+                act_i[chunk] = -64 * (int)(short)(header[k] >> 16);
+            }
+        }
+    }
+}
+__device__ __noinline__ void chain_back(const float4 *scratch, int u0, int step, int units, int chunk0, int lane, uint32_t *act_q, float *act_s, int *act_i) {
+    for (int rounds = (units + step - 1) / step; u0 < units;) {
+        const int n = rounds == 4 ? 2 : min(rounds, 3);
+        if (n == 1) chain_back_units<1>(scratch, u0, step, units, chunk0, lane, act_q, act_s, act_i);
+        else if (n == 2) chain_back_units<2>(scratch, u0, step, units, chunk0, lane, act_q, act_s, act_i);
+        else chain_back_units<3>(scratch, u0, step, units, chunk0, lane, act_q, act_s, act_i);
+        rounds -= n;
+        u0 += n * step;
+    }
+}
+
 template <int THREADS, int MAXSTEPS, bool TP>
 __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *__restrict__ ops, const int n_ops,
                                                                 const ChainGeom G, unsigned int *grid_counter,
@@ -204,6 +242,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
     uint64_t *xs = ready + CHAIN_TABLES;                                  // [1]  rotate: every warp has written its blocks
     uint64_t *dep = xs + 1;                                   // [1]  rotate: the producers of x have arrived
     uint64_t *stage_full = dep + 1;                           // [1]  Q8_1 staging copy landed
+    uint64_t *image = stage_full + 1;                         // [1]  a spread op's tables have been copied from the image
     int *done_cnt = reinterpret_cast<int *>(smem + 192);      // [16] tasks of the slot's tile that have copied out
     int *expect_cnt = done_cnt + CHAIN_MAX_SLOTS;             // [16] ... of how many
     volatile int *ctrl = expect_cnt + CHAIN_MAX_SLOTS;        // [16] 0 issued, 1 ops_loaded, 2 next_task, 3 copy_op, 4-7 warps that
@@ -236,6 +275,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
         mbar_init(xs, C);
         mbar_init(dep, 1);
         mbar_init(stage_full, 1);
+        mbar_init(image, 1);
         mbar_fence_init();
     }
     for (int i = threadIdx.x; i < 3 * CHAIN_MAX_SLOTS; i += THREADS) done_cnt[i] = 0;     // done, expect, ctrl
@@ -276,7 +316,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
         const int rr = lane & 3, bl = lane >> 2;
         int op = -1, flags = 0;
         int issued_seen = 0;
-        uint32_t xs_phase = 0, dep_phase = 0;     // every compute warp takes part in every meeting, so it counts them itself
+        uint32_t xs_phase = 0, dep_phase = 0, image_phase = 0;     // every compute warp takes part in every meeting, so it counts them itself
         int task_base = 0, ntasks = 0, g_base = 0, ntiles = 0, row0 = 0, rows_here = 0;
         for (;;) {
             int task = 0;
@@ -286,9 +326,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
             while (task >= task_base + ntasks) {
                 // ---- leave op `op`
                 if (op >= 0) {
-                    // this warp's y rows are in memory (device scope) before it is counted out below: other CTAs read them
-                    // once everybody has arrived (several ranks: the peer warp reads its copy in shared memory)
-                    if (flags & CHAIN_SIGNAL) __threadfence();
+                    // several ranks: this warp's y rows are in memory (device scope) before it is counted out below (one rank: the last
+                    // warp out has the fence, which covers what the others had written when they were counted)
+                    if (TP && (flags & CHAIN_SIGNAL)) __threadfence();
                     if (!TP && (flags & CHAIN_MAXSRC)) {                // the warp's largest |y|, then the CTA's (float bits order as ints)
 #pragma unroll
                         for (int o = 16; o > 0; o >>= 1) ymax = fmaxf(ymax, __shfl_xor_sync(0xffffffffu, ymax, o));
@@ -327,9 +367,32 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                 ymax = 0.0f;
                 if (!(flags & CHAIN_SAME_INPUT)) {
                     if (flags & CHAIN_ROTATE) {
+                        // Wide inputs of dependent ops are rotated ONCE for the whole grid instead of once per CTA
+                        // (every CTA repeating 17 blocks costs ~10 us): block fb is rotated by CTA fb, which writes
+                        // its part of the tables to an image in global memory; a second arrival counter tells
+                        // everybody when all blocks are there, and every CTA copies the image into its tables.  A CTA without
+                        // a block has nothing else to wait for.
+                        const bool spread = flags & CHAIN_SPREAD;
+                        const int nfb = R.nb >> 3;
+                        const int fb_lo = spread ? min((int)blockIdx.x, nfb) : 0;
+                        const int fb_hi = spread ? min((int)blockIdx.x + 1, nfb) : nfb;
+                        // What the vector is multiplied by waits for nobody: norm weights (from memory, once a run) go to this thread's
+                        // places in the scratch area while the producers of x finish, signs are asked into L2.
+                        const float *x = static_cast<const float *>(R.x);
+                        const float *signs = R.signs;
+                        const float *aux = R.aux;
+                        constexpr int UPW = (7 * 8 + C - 1) / C;               // units per warp and round trip
+#pragma unroll
+                        for (int k = 0; k < UPW; ++k) {
+                            const int u = wid + k * C;
+                            if (u < min(G.rot_blocks, fb_hi - fb_lo) * 8) {
+                                if (signs) prefetch_l2(signs + (size_t)fb_lo * FWHT_N + (size_t)u * 128 + 4 * lane);
+                                if (flags & CHAIN_RMSNORM) scratch[u * 32 + lane] = __ldg(reinterpret_cast<const float4 *>(aux + (size_t)u * 128 + 4 * lane));
+                            }
+                        }
                         // every compute warp has left op - 1: both table buffers' readers are gone
-                        if (op >= 1 && !spin_until_gt(&ctrl[8], op - 1)) { alive = false; break; }
-                        if (flags & CHAIN_DEPENDS) {
+                        if (op >= 1 && !spin_until_gt(&ctrl[8], op - 1, CHAIN_NS0, CHAIN_MEET_NSMAX)) { alive = false; break; }
+                        if ((flags & CHAIN_DEPENDS) && (TP || fb_lo < fb_hi)) {
                             if (wid == 0) {
                                 bool ok = true;
                                 if (TP) ok = rank_flags_wait(grid_counter + 8, PE.world, arrive_base + R.arrivals_needed,
@@ -338,24 +401,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                 __syncwarp();
                                 if (lane == 0 && ok) mbar_arrive(dep);
                             }
-                            if (!mbar_wait_bounded(dep, dep_phase & 1u, CHAIN_NS0, CHAIN_NSMAX)) { alive = false; break; }
+                            if (!(TP ? mbar_wait_bounded(dep, dep_phase & 1u, CHAIN_NS0, CHAIN_NSMAX) : mbar_wait_suspended(dep, dep_phase & 1u))) { alive = false; break; }
                             ++dep_phase;
                         }
-                        // Wide inputs of dependent ops are rotated ONCE for the whole grid instead of once per CTA
-                        // (every CTA repeating 17 blocks costs ~10 us): block fb is rotated by CTA fb, which writes
-                        // its part of the tables to an image in global memory; a second arrival counter tells
-                        // everybody when all blocks are there, and every CTA copies the image into its tables.
-                        const bool spread = flags & CHAIN_SPREAD;
                         uint8_t *own = tables + (size_t)R.buf * table_bytes;
                         uint32_t *act_q = reinterpret_cast<uint32_t *>(spread ? table_image : own);
                         float *act_s = reinterpret_cast<float *>(act_q + (size_t)G.nb_max * STREAM_ACT_WORDS);
                         int *act_i = reinterpret_cast<int *>(act_s + (size_t)G.nb_max * 4);
-                        const float *x = static_cast<const float *>(R.x);
-                        const float *signs = R.signs;
-                        const float *aux = R.aux;
-                        const int nfb = R.nb >> 3;
-                        const int fb_lo = spread ? min((int)blockIdx.x, nfb) : 0;
-                        const int fb_hi = spread ? min((int)blockIdx.x + 1, nfb) : nfb;
                         // the exact power-of-two rescale of the synthetic decode step: the producer recorded max |x|
                         float rescale = 1.0f;
                         const int src_len = R.src_len;
@@ -371,7 +423,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                             const int units = min(G.rot_blocks, fb_hi - fb0) * 8;
                             // all of this warp's loads first (they come from L2: written by other SMs
                             // during this launch), then the butterflies
-                            constexpr int UPW = (7 * 8 + C - 1) / C;           // units per warp and round trip
                             float4 f[UPW];
 #pragma unroll
                             for (int k = 0; k < UPW; ++k) {
@@ -409,17 +460,22 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                 }
                                 __syncwarp();
                                 if (lane == 0) mbar_arrive(xs);
-                                ok = mbar_wait_bounded(xs, xs_phase & 1u, CHAIN_NS0, CHAIN_NSMAX);
+                                ok = mbar_wait_suspended(xs, xs_phase & 1u);
                                 ++xs_phase;
                                 if (!ok) break;
                                 float ss = 0.0f;
-                                for (int u = 0; u < units; ++u) ss = __fadd_rn(ss, ssum[u]);
+#pragma unroll 2
+                                for (int u = 0; u < units; u += 8) {
+                                    const float4 a = *reinterpret_cast<const float4 *>(ssum + u), b = *reinterpret_cast<const float4 *>(ssum + u + 4);
+                                    ss = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(ss, a.x), a.y), a.z), a.w);
+                                    ss = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(ss, b.x), b.y), b.z), b.w);
+                                }
                                 const float sc = rms_scale(ss, R.nb * 128, R.eps);
 #pragma unroll
                                 for (int k = 0; k < UPW; ++k) {
                                     const int u = wid + k * C;
                                     if (u < units) {
-                                        const float4 wv = __ldg(reinterpret_cast<const float4 *>(aux + (size_t)u * 128 + 4 * lane));
+                                        const float4 wv = scratch[u * 32 + lane];
                                         f[k] = make_float4(__fmul_rn(__fmul_rn(f[k].x, sc), wv.x), __fmul_rn(__fmul_rn(f[k].y, sc), wv.y),
                                                            __fmul_rn(__fmul_rn(f[k].z, sc), wv.z), __fmul_rn(__fmul_rn(f[k].w, sc), wv.w));
                                     }
@@ -441,52 +497,36 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                             }
                             __syncwarp();
                             if (lane == 0) mbar_arrive(xs);
-                            ok = mbar_wait_bounded(xs, xs_phase & 1u, CHAIN_NS0, CHAIN_NSMAX);
+                            ok = mbar_wait_suspended(xs, xs_phase & 1u);
                             ++xs_phase;
                             if (!ok) break;
-                            for (int u = wid; u < units; u += C) {
-                                float v[4];
-                                fwht_slice_back(scratch + (u >> 3) * 256, u & 7, lane, v);
-                                uint32_t word, header;
-                                quantise_chunk_8lanes(v, lane, word, header);
-                                const int chunk = fb0 * 32 + u * 4 + (lane >> 3);
-                                act_q[(chunk >> 2) * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word;
-                                if ((lane & 7) == 0) {
-                                    act_s[chunk] = f16_bits_to_f32(header & 0xFFFFu);
-                                    act_i[chunk] = -64 * (int)(short)(header >> 16);
-                                }
-                            }
-                            if (spread) __threadfence();                // the image rows written above, before the arrival below
+                            chain_back(scratch, wid, C, units, fb0 * 32, lane, act_q, act_s, act_i);
                             __syncwarp();
                             if (lane == 0) mbar_arrive(xs);
-                            ok = mbar_wait_bounded(xs, xs_phase & 1u, CHAIN_NS0, CHAIN_NSMAX);
+                            ok = mbar_wait_suspended(xs, xs_phase & 1u);
                             ++xs_phase;
                         }
                         if (!ok) { alive = false; break; }
                         if (spread) {
-                            if (wid == 0) {
-                                bool there = true;
-                                if (lane == 0) {
-                                    if (fb_lo < fb_hi) {                // this CTA's block is in the image (every warp has fenced)
-                                        __threadfence();
-                                        atomicAdd(grid_counter + 1, (unsigned)(fb_hi - fb_lo));
-                                    }
-                                    there = grid_counter_wait(grid_counter + 1, spread_base + R.spread_blocks);
+                            if (wid == 0 && lane == 0) {
+                                if (fb_lo < fb_hi) {                    // this CTA's block is in the image (behind the meeting: every warp's part)
+                                    __threadfence();
+                                    atomicAdd(grid_counter + 1, (unsigned)(fb_hi - fb_lo));
                                 }
-                                __syncwarp();
-                                if (lane == 0 && there) mbar_arrive(dep);
+                                if (grid_counter_wait(grid_counter + 1, spread_base + R.spread_blocks)) {
+                                    // image -> this CTA's tables, by the copy unit: written by other SMs during this launch
+                                    asm volatile("fence.proxy.async;" ::: "memory");
+                                    const uint64_t pol = policy_evict_normal();
+                                    const size_t q_at = (size_t)G.nb_max * STREAM_ACT_WORDS * 4, i_at = q_at + (size_t)G.nb_max * 16;
+                                    mbar_expect_tx(image, (uint32_t)R.nb * 176);
+                                    bulk_g2s(own, table_image, (uint32_t)R.nb * STREAM_ACT_WORDS * 4, image, pol);
+                                    bulk_g2s(own + q_at, table_image + q_at, (uint32_t)R.nb * 16, image, pol);
+                                    bulk_g2s(own + i_at, table_image + i_at, (uint32_t)R.nb * 16, image, pol);
+                                }
                             }
-                            if (!mbar_wait_bounded(dep, dep_phase & 1u, CHAIN_NS0, CHAIN_NSMAX)) { alive = false; break; }
-                            ++dep_phase;
-                            // image -> this CTA's tables (written by other SMs during this launch: read at L2)
-                            const uint4 *src16 = reinterpret_cast<const uint4 *>(table_image);
-                            uint4 *dst16 = reinterpret_cast<uint4 *>(own);
-                            const int n16 = (int)(table_bytes >> 4);
-                            for (int i = wid * 32 + lane; i < n16; i += C * 32) dst16[i] = __ldcg(src16 + i);
                             __syncwarp();
-                            if (lane == 0) mbar_arrive(xs);
-                            if (!mbar_wait_bounded(xs, xs_phase & 1u, CHAIN_NS0, CHAIN_NSMAX)) { alive = false; break; }
-                            ++xs_phase;
+                            if (!mbar_wait_suspended(image, image_phase & 1u)) { alive = false; break; }
+                            ++image_phase;
                         }
                     } else {
                         if (!mbar_wait_bounded(&ready[R.buf], (uint32_t)R.ready_parity, CHAIN_GATE_NS0, CHAIN_GATE_NSMAX)) { alive = false; break; }
