@@ -22,7 +22,7 @@
 // columns: 256 output (before that, sums of the scores), 128 scores (then weights), 128 q low.
 // What bounds it (counted while a score was four sums): per tile 5900 of 10200 cycles were the tensor core's, most of them the score
 // products (N = 64: it waits for the q rows from shared memory), the rest softmax and the exchanges in front of it.  2048 tokens, 24 heads over 4: 2570 ->
-// 292 us; 1000 tokens 727 -> 94 us, 517 tokens 246 -> 59 us.
+// 287 us; 1000 tokens 727 -> 91 us, 600 tokens 60 us.
 //
 // A plane pair holds 2^-39 of the largest value under its power of two, so what is far smaller loses bits to values that a row may not
 // even see.  A CTA whose queries and keys range too widely (atc_too_wide) does its queries again on the CUDA cores (attn_simt), with
@@ -403,25 +403,28 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
         ok = mbar_wait_hot(qk2, par) && ok;
         tc_fence_after();
         {
-            auto pair = [&](uint32_t col, float (&t)[16]) {
-                int a[16], b[16];
-                tc_ld16(tlane + col + (uint32_t)(16 * cg), a);
-                tc_ld16(tlane + col + (uint32_t)(ATC_KEYS + 16 * cg), b);
+            // (eight columns at a time: sixteen of two sums beside the outputs and the scores were more registers than a thread has, and what is
+            // spilled beside 200 KB of shared memory comes from L2: 2048 tokens 293 -> 287 us)
+#pragma unroll
+            for (uint32_t h = 0; h < 16; h += 8) {
+                int a[8], b[8], c[8], d[8];
+                tc_ld8(tlane + ATC_COL_S + h + (uint32_t)(16 * cg), a);
+                tc_ld8(tlane + ATC_COL_S + ATC_KEYS + h + (uint32_t)(16 * cg), b);
+                tc_ld8(tlane + ATC_COL_O + h + (uint32_t)(16 * cg), c);
+                tc_ld8(tlane + ATC_COL_O + ATC_KEYS + h + (uint32_t)(16 * cg), d);
+                tc_ld_wait();
+                float t[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) t[e] = __fadd_rn(__fadd_rn(__int_as_float(a[e]), __int_as_float(b[e])), __fadd_rn(__int_as_float(c[e]), __int_as_float(d[e])));
+                tc_ld8(tlane + ATC_COL_O + 2 * ATC_KEYS + h + (uint32_t)(16 * cg), a);
+                tc_ld8(tlane + ATC_COL_O + 3 * ATC_KEYS + h + (uint32_t)(16 * cg), b);
                 tc_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 16; ++e) t[e] = __fadd_rn(__int_as_float(a[e]), __int_as_float(b[e]));
-            };
-            float t[16];
-            pair(ATC_COL_S, s);
-            pair(ATC_COL_O, t);
-#pragma unroll
-            for (int e = 0; e < 16; ++e) s[e] = __fadd_rn(s[e], t[e]);
-            pair(ATC_COL_O + 2 * ATC_KEYS, t);
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                const float f = __fmul_rn(qf, kf[par * ATC_KEYS + 16 * cg + e]);
-                s[e] = j0 + 16 * cg + e <= query ? __fmul_rn(__fadd_rn(s[e], t[e]), f) : -INFINITY;
-                mx = fmaxf(mx, s[e]);
+                for (int e = 0; e < 8; ++e) {
+                    const float f = __fmul_rn(qf, kf[par * ATC_KEYS + 16 * cg + (int)h + e]);
+                    s[h + e] = j0 + 16 * cg + (int)h + e <= query ? __fmul_rn(__fadd_rn(t[e], __fadd_rn(__int_as_float(a[e]), __int_as_float(b[e]))), f) : -INFINITY;
+                    mx = fmaxf(mx, s[h + e]);
+                }
             }
         }
         red[cg * ATC_M + row] = mx;
