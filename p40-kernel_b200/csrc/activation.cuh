@@ -311,13 +311,21 @@ __global__ void __launch_bounds__(32 * FWHT_WARP_BLOCKS, 8) fwht_quant_warp_kern
     }
     if (xq) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            uint32_t word, header;
-            quantise_chunk_8lanes(v[r], lane, word, header);
-            const int chunk = blk * 32 + r * 4 + (lane >> 3);
-            uint32_t *dst = xq + 9 * ((size_t)chunk * n_tok + tok);
-            dst[1 + (lane & 7)] = word;
-            if ((lane & 7) == 0) dst[0] = header;
+        for (int r0 = 0; r0 < 8; r0 += 4) {             // four slices side by side
+            float s[4][4];
+            uint32_t word[4], header[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[r][e] = v[r0 + r][e];
+            quantise_chunks_8lanes<4>(s, lane, word, header);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int chunk = blk * 32 + (r0 + r) * 4 + (lane >> 3);
+                uint32_t *dst = xq + 9 * ((size_t)chunk * n_tok + tok);
+                dst[1 + (lane & 7)] = word[r];
+                if ((lane & 7) == 0) dst[0] = header[r];
+            }
         }
     }
 }

@@ -21,6 +21,8 @@
 // broadcast): no term buffers, no ordered adder, about 30 instructions per 32 weights.
 #pragma once
 
+#include <type_traits>
+
 #include "activation.cuh"
 #include "common.cuh"
 #include "gemv.cuh"
@@ -290,19 +292,33 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
                     for (int t = first_late; t < first_fill; ++t) issue_tile(t);
                 first = false;
             }
+            // a warp's slices side by side, their divisions shared (one per lane of a chunk): one after the other each was a chain
+            // of shuffles and two divisions, before the first product (17408 -> 5120 16.05 -> 15.2 us, 5 slices and then 4 or 5)
+            auto quantise = [&](auto count) {
+                constexpr int N = decltype(count)::value;
+                float v[N][4];
+                uint32_t word[N], header[N];
 #pragma unroll
-            for (int k = 0; k < SLICES; ++k) {
-                const int sl = s0 + k * compute_warps;
-                if (wid >= compute_warps || sl >= P.nb) break;          // warp-uniform
-                const float v[4] = {f[k].x, f[k].y, f[k].z, f[k].w};
-                uint32_t word, header;
-                quantise_chunk_8lanes(v, lane, word, header);
-                const int chunk = 4 * sl + (lane >> 3);
-                act_q[sl * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word;
-                if ((lane & 7) == 0) {
-                    act_s[chunk] = f16_bits_to_f32(header & 0xFFFFu);
-                    act_i[chunk] = -64 * (int)(short)(header >> 16);
+                for (int k = 0; k < N; ++k) v[k][0] = f[k].x, v[k][1] = f[k].y, v[k][2] = f[k].z, v[k][3] = f[k].w;
+                quantise_chunks_8lanes<N>(v, lane, word, header);
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const int sl = s0 + k * compute_warps;
+                    if (sl < P.nb) {
+                        const int chunk = 4 * sl + (lane >> 3);
+                        act_q[sl * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word[k];
+                        if ((lane & 7) == 0) {
+                            act_s[chunk] = f16_bits_to_f32(header[k] & 0xFFFFu);
+                            act_i[chunk] = -64 * (int)(short)(header[k] >> 16);
+                        }
+                    }
                 }
+            };
+            if (wid < compute_warps && s0 < P.nb) {                     // warp-uniform
+                const int n = (P.nb - s0 + compute_warps - 1) / compute_warps;
+                if (n == 1) quantise(std::integral_constant<int, 1>());
+                else if (n <= 3) quantise(std::integral_constant<int, 3>());
+                else quantise(std::integral_constant<int, SLICES>());
             }
         }
     } else if (FUSED) {
