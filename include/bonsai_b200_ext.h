@@ -191,6 +191,8 @@ int bonsai_b200_clear_status(void);
  * (reference: src/ops.h:13-31; its device code runs them as kernels of their own, src/kernels/elementwise_p40.cu:48-88).
  *   BONSAI_B200_OP_RMSNORM     input = x * (1 / sqrt(mean(x^2) + eps)) * aux[0 .. n_in); n_in <= 7168.  Same bits as
  *                              bonsai_p40_rmsnorm followed by the op without the flag.
+ *                              aux (and signs) may be outputs of the list like x: of an op that says OP_DEPENDS they
+ *                              are then read behind its wait, otherwise they may be read before it.
  *   BONSAI_B200_OP_SWIGLU      input = silu(x) * aux  (x = gate, aux = up, both n_in floats).  Same bits as
  *                              bonsai_b200_swiglu followed by the op without the flag.
  *   BONSAI_B200_OP_RESCALE     x is the whole output (src_len floats) of an earlier op of the list;

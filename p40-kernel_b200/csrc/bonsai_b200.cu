@@ -27,9 +27,11 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <iterator>
 #include <mutex>
 #include <new>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 using namespace b200;
@@ -627,6 +629,23 @@ static int chain_create_impl(const bonsai_b200_op *ops, int64_t n_ops, int tp_ra
                              !(ops[i - 1].flags & BONSAI_B200_OP_ROTATE));
         if (!shared) ++q8_fills;
     }
+    // What the list writes, in order of address, each with the furthest end so far: norm weights or signs in there are read late.
+    std::vector<std::pair<uintptr_t, uintptr_t>> written;
+    for (int64_t i = 0; i < n_ops; ++i) {
+        const uintptr_t y = reinterpret_cast<uintptr_t>(ops[i].y);
+        if (ops[i].n_out > 0) written.emplace_back(y, y + 4 * (uintptr_t)ops[i].n_out);
+    }
+    if (tp) {                                                   // the other ranks write their rows here too
+        const uintptr_t b = reinterpret_cast<uintptr_t>(peer_base[tp_rank]);
+        written.emplace_back(b, b + (uintptr_t)counter_offset);
+    }
+    std::sort(written.begin(), written.end());
+    for (size_t i = 1; i < written.size(); ++i) written[i].second = std::max(written[i].second, written[i - 1].second);
+    auto list_writes = [&](const float *p, int64_t n) {
+        const uintptr_t lo = reinterpret_cast<uintptr_t>(p), hi = lo + 4 * (uintptr_t)n;
+        const auto behind = std::lower_bound(written.begin(), written.end(), std::make_pair(hi, (uintptr_t)0));   // the first that starts behind them
+        return behind != written.begin() && std::prev(behind)->second > lo;
+    };
     const int ntables = q8_ops == 0 ? 1 : (2 * q8_fills > q8_ops ? CHAIN_TABLES : 2);
     int shift = 0, buf = ntables - 1, last_user[CHAIN_TABLES], ready_uses[CHAIN_TABLES];
     for (int b = 0; b < CHAIN_TABLES; ++b) last_user[b] = -1, ready_uses[b] = 0;
@@ -704,6 +723,7 @@ static int chain_create_impl(const bonsai_b200_op *ops, int64_t n_ops, int tp_ra
         r.flags = (rotate ? CHAIN_ROTATE : 0) | (depends ? CHAIN_DEPENDS : 0) | (same ? CHAIN_SAME_INPUT : 0) |
                   ((producer & BONSAI_B200_OP_RMSNORM) ? CHAIN_RMSNORM : 0) | ((producer & BONSAI_B200_OP_SWIGLU) ? CHAIN_SWIGLU : 0) |
                   ((producer & BONSAI_B200_OP_RESCALE) ? CHAIN_RESCALE : 0);
+        if (((producer & BONSAI_B200_OP_RMSNORM) && list_writes(o.aux, o.n_in)) || (o.signs && list_writes(o.signs, o.n_in))) r.flags |= CHAIN_LATE;
         r.aux = o.aux;
         r.eps = o.eps;
         r.src_len = (int)o.src_len;

@@ -50,7 +50,8 @@ enum : int {
     CHAIN_SWIGLU = 16,        // input = silu(x) * aux                     (src/ops.h:27-31)
     CHAIN_RESCALE = 32,       // input[j] = x[j mod src_len] * 2^-e, e = floor(log2(max |x|)): the exact glue of the synthetic decode step
     CHAIN_SIGNAL = 64, CHAIN_SPREAD = 128,
-    CHAIN_MAXSRC = 256        // a later CHAIN_RESCALE op reads this op's output: its largest magnitude is recorded
+    CHAIN_MAXSRC = 256,       // a later CHAIN_RESCALE op reads this op's output: its largest magnitude is recorded
+    CHAIN_LATE = 512          // norm weights or signs are (part of) an output of the list: read behind the wait, not before it
 };
 
 constexpr int CHAIN_MAX_SLOTS = 16;
@@ -376,18 +377,20 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                         const int nfb = R.nb >> 3;
                         const int fb_lo = spread ? min((int)blockIdx.x, nfb) : 0;
                         const int fb_hi = spread ? min((int)blockIdx.x + 1, nfb) : nfb;
-                        // What the vector is multiplied by waits for nobody: norm weights (from memory, once a run) go to this thread's
-                        // places in the scratch area while the producers of x finish, signs are asked into L2.
+                        // What the vector is multiplied by waits for nobody, unless the list itself writes it (CHAIN_LATE): norm weights
+                        // (from memory, once a run) go to this thread's places in the scratch area while the producers of x finish,
+                        // signs are asked into L2.
                         const float *x = static_cast<const float *>(R.x);
                         const float *signs = R.signs;
                         const float *aux = R.aux;
+                        const bool late = flags & CHAIN_LATE;
                         constexpr int UPW = (7 * 8 + C - 1) / C;               // units per warp and round trip
 #pragma unroll
                         for (int k = 0; k < UPW; ++k) {
                             const int u = wid + k * C;
                             if (u < min(G.rot_blocks, fb_hi - fb_lo) * 8) {
                                 if (signs) prefetch_l2(signs + (size_t)fb_lo * FWHT_N + (size_t)u * 128 + 4 * lane);
-                                if (flags & CHAIN_RMSNORM) scratch[u * 32 + lane] = __ldg(reinterpret_cast<const float4 *>(aux + (size_t)u * 128 + 4 * lane));
+                                if ((flags & CHAIN_RMSNORM) && !late) scratch[u * 32 + lane] = __ldg(reinterpret_cast<const float4 *>(aux + (size_t)u * 128 + 4 * lane));
                             }
                         }
                         // every compute warp has left op - 1: both table buffers' readers are gone
@@ -475,7 +478,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                 for (int k = 0; k < UPW; ++k) {
                                     const int u = wid + k * C;
                                     if (u < units) {
-                                        const float4 wv = scratch[u * 32 + lane];
+                                        const float4 wv = late ? __ldcg(reinterpret_cast<const float4 *>(aux + (size_t)u * 128 + 4 * lane)) : scratch[u * 32 + lane];
                                         f[k] = make_float4(__fmul_rn(__fmul_rn(f[k].x, sc), wv.x), __fmul_rn(__fmul_rn(f[k].y, sc), wv.y),
                                                            __fmul_rn(__fmul_rn(f[k].z, sc), wv.z), __fmul_rn(__fmul_rn(f[k].w, sc), wv.w));
                                     }
@@ -487,7 +490,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                 if (u < units) {
                                     float v[4] = {f[k].x, f[k].y, f[k].z, f[k].w};
                                     if (signs) {
-                                        const float4 sg = __ldg(reinterpret_cast<const float4 *>(signs + (size_t)fb0 * FWHT_N + (size_t)u * 128 + 4 * lane));
+                                        const float4 *sp = reinterpret_cast<const float4 *>(signs + (size_t)fb0 * FWHT_N + (size_t)u * 128 + 4 * lane);
+                                        const float4 sg = late ? __ldcg(sp) : __ldg(sp);
                                         v[0] = __fmul_rn(v[0], sg.x); v[1] = __fmul_rn(v[1], sg.y);
                                         v[2] = __fmul_rn(v[2], sg.z); v[3] = __fmul_rn(v[3], sg.w);
                                     }
