@@ -158,29 +158,42 @@ __device__ __forceinline__ bool mbar_wait_hot(uint64_t *bar, uint32_t parity) {
     if (ok) return true;
     return mbar_wait_bounded(bar, parity, 32, 128);
 }
-// The same wait in the hardware's blocking form: a dozen warps that wait for the same thing need no sleeps between their polls.
-__device__ __forceinline__ bool mbar_wait_suspended(uint64_t *bar, uint32_t parity) {
+__device__ __forceinline__ unsigned long long global_timer_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ uint32_t global_timer_ms() { return (uint32_t)(global_timer_ns() >> 20); }       // steps of 1.05 ms
+// The blocking form of the test: the unit gives the thread back when the phase has completed, after suspend_ns at the latest.
+__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity, uint32_t suspend_ns) {
     uint32_t ok;
     asm volatile(
         "{\n\t"
         ".reg .pred p;\n\t"
-        ".reg .u32 n;\n\t"
-        "mov.u32 n, %3;\n\t"
-        "mov.u32 %0, 1;\n\t"
-        "TRY_LOOP:\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra TRY_DONE;\n\t"
-        "sub.u32 n, n, 1;\n\t"
-        "setp.ne.u32 p, n, 0;\n\t"
-        "@p bra TRY_LOOP;\n\t"
-        "mov.u32 %0, 0;\n\t"
-        "TRY_DONE:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
         "}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(1u << 24)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(suspend_ns)
         : "memory");
-    if (!ok) atomicExch(&g_device_status, STATUS_MBARRIER_TIMEOUT);
     return ok != 0;
+}
+// The bounded wait in the blocking form: a dozen warps that wait for the same thing need no sleeps between their polls.  Between two
+// suspensions a thread looks at *stop and at the clock.  False when *stop was set -- by a thread of the CTA that has given up, and said
+// so, on something that this one waits for in the end -- or when limit_ms milliseconds have passed (status word; *stop is set).
+constexpr uint32_t MBAR_SUSPEND_NS = 10000;
+__device__ __forceinline__ bool mbar_wait_suspended(uint64_t *bar, uint32_t parity, volatile int *stop, uint32_t limit_ms) {
+    if (mbar_try_wait(bar, parity, MBAR_SUSPEND_NS)) return true;
+    const uint32_t t0 = global_timer_ms();
+    while (!mbar_try_wait(bar, parity, MBAR_SUSPEND_NS)) {
+        if (*stop) return false;
+        if (global_timer_ms() - t0 > limit_ms) {
+            *stop = 1;
+            atomicExch(&g_device_status, STATUS_MBARRIER_TIMEOUT);
+            return false;
+        }
+    }
+    return true;
 }
 // One non-blocking poll: has the phase with this parity completed?
 __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {

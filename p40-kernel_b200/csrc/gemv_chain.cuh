@@ -24,15 +24,18 @@
 //
 // Barrier discipline.  Shared-memory barriers are reused, so a waiter identifies a phase by parity;
 // that is only sound when the barrier cannot complete a second phase before the waiter has seen the
-// first.  Only three kinds of barrier are waited on by parity, and each has that property by
+// first.  Only these kinds of barrier are waited on by parity, and each has that property by
 // construction: ready[buf] (its next phase needs every compute warp to have left an op that comes
 // after the one being waited for), xs and dep (every waiter must arrive, or pass xs, before the next
-// phase can complete), full[slot] (a task first sees `issued > g`, published after the barrier was
+// phase can complete), image (it is armed for a later op only when every compute warp has left the one
+// before that op, and a warp leaves an op that waits for the image behind that wait), full[slot] (a task first sees `issued > g`, published after the barrier was
 // armed for tile g, and the slot cannot be re-armed before that task has copied out).  Everything
 // that a warp may fall arbitrarily far behind on is a monotonic counter instead: ops_done (every
 // compute warp has left ops [0, ops_done)), ops_loaded, issued, copy_op.  Slot release is a plain
 // counter too, because the number of tasks per tile changes from op to op.
-// Every wait is bounded; a time-out sets the status word and the warp leaves.
+// Every wait is bounded: a second or so by counted polls with sleeps (the copy, sequencer and peer warps, the ring), some three seconds
+// for other CTAs (grid_counter_wait), the caller's limit for other ranks, and for warps that wait for each other's part of these until
+// one of them has given up.  A time-out sets the status word and the warp leaves.
 #pragma once
 
 #include "activation.cuh"
@@ -60,6 +63,9 @@ constexpr int CHAIN_TABLES = 3;          // activation-table buffers: the sequen
 constexpr uint32_t CHAIN_NS0 = 32, CHAIN_NSMAX = 256;             // first and longest sleep between two polls of a wait
 constexpr uint32_t CHAIN_MEET_NSMAX = 64;                         // ... of the waits that hold up the whole grid
 constexpr uint32_t CHAIN_GATE_NS0 = 32, CHAIN_GATE_NSMAX = 256;   // ... of the waits that usually last microseconds
+// The warps of a CTA that wait for each other, or for what one lane of them waits for, leave when that lane has given up (ctrl[14]); should it
+// say nothing either, after this time (several ranks: and their own limit).
+constexpr uint32_t CHAIN_WAIT_MS = 8000;
 constexpr int CHAIN_GATES = 3;           // a warp may run this many ops ahead of the slowest one
 
 struct __align__(16) ChainOp {                 // 128 bytes, one per projection, device table
@@ -109,7 +115,7 @@ __host__ __device__ inline size_t chain_fixed_bytes(const ChainGeom &G) {
 __device__ __forceinline__ bool spin_until_gt(volatile int *p, int v, uint32_t first_ns = CHAIN_NS0,
                                               uint32_t max_ns = CHAIN_NSMAX) {
     uint32_t ns = first_ns;
-    for (uint32_t n = 0; n < (1u << 22); ++n) {
+    for (uint32_t n = 0; n < (1u << 30) / max_ns; ++n) {                // about a second of sleep
         if (*p > v) return true;
         __nanosleep(ns);
         ns = min(ns * 2, max_ns);
@@ -127,8 +133,8 @@ __device__ __forceinline__ bool spin_until_eq(volatile int *p, int v) {
     atomicExch(&g_device_status, STATUS_MBARRIER_TIMEOUT);
     return false;
 }
-// Arrival counter of this GPU's own CTAs, polled by one lane, bounded by an iteration count.  Counters only grow,
-// so "reached" is a wrap-safe signed difference.
+// Arrival counter of this GPU's own CTAs, polled by one lane, bounded by an iteration count: four million trips to L2 with sleeps of up
+// to 64 ns between them, some three seconds.  Counters only grow, so "reached" is a wrap-safe signed difference.
 __device__ __forceinline__ bool grid_counter_wait(const unsigned int *counter, unsigned int target) {
     uint32_t ns = CHAIN_NS0;
     for (uint32_t n = 0; n < (1u << 22); ++n) {
@@ -140,11 +146,6 @@ __device__ __forceinline__ bool grid_counter_wait(const unsigned int *counter, u
     }
     atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);
     return false;
-}
-__device__ __forceinline__ unsigned long long global_timer_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
 }
 // Several ranks: flag word q of this rank's counter block is written by rank q (one store over NVLink per signal).
 // Lane q < world polls flag q (acquire at system scope) until it has reached `target`; the wait ends for the whole
@@ -249,7 +250,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
     volatile int *ctrl = expect_cnt + CHAIN_MAX_SLOTS;        // [16] 0 issued, 1 ops_loaded, 2 next_task, 3 copy_op, 4-7 warps that
                                                               //      left op (index & 3), 8 ops_done: every compute warp has left ops [0, ops_done),
                                                               //      9 (several ranks) ops whose rows the peer warp has sent,
-                                                              //      10-13 largest |y| of op (index & 3) so far, as float bits
+                                                              //      10-13 largest |y| of op (index & 3) so far, as float bits,
+                                                              //      14 a compute warp has given up on a wait: the others leave too
     float *ssum = reinterpret_cast<float *>(smem + 384);     // [56] sums of squares of the slices of an RMSNorm input
     ChainOp *opring = reinterpret_cast<ChainOp *>(smem + 640);
     uint8_t *p = smem + 640 + CHAIN_OP_RING * sizeof(ChainOp);
@@ -317,6 +319,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
         const int rr = lane & 3, bl = lane >> 2;
         int op = -1, flags = 0;
         int issued_seen = 0;
+        volatile int *stop = &ctrl[14];
+        const uint32_t wait_ms = CHAIN_WAIT_MS + (TP ? (uint32_t)(PE.wait_limit_ns >> 20) : 0u);
         uint32_t xs_phase = 0, dep_phase = 0, image_phase = 0;     // every compute warp takes part in every meeting, so it counts them itself
         int task_base = 0, ntasks = 0, g_base = 0, ntiles = 0, row0 = 0, rows_here = 0;
         for (;;) {
@@ -402,9 +406,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                                              PE.wait_limit_ns, lane);
                                 else if (lane == 0) ok = grid_counter_wait(grid_counter, R.arrivals_needed * (unsigned)ncta);
                                 __syncwarp();
-                                if (lane == 0 && ok) mbar_arrive(dep);
+                                if (lane == 0) {
+                                    if (ok) mbar_arrive(dep);
+                                    else *stop = 1;
+                                }
                             }
-                            if (!(TP ? mbar_wait_bounded(dep, dep_phase & 1u, CHAIN_NS0, CHAIN_NSMAX) : mbar_wait_suspended(dep, dep_phase & 1u))) { alive = false; break; }
+                            if (!mbar_wait_suspended(dep, dep_phase & 1u, stop, wait_ms)) { alive = false; break; }
                             ++dep_phase;
                         }
                         uint8_t *own = tables + (size_t)R.buf * table_bytes;
@@ -463,7 +470,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                 }
                                 __syncwarp();
                                 if (lane == 0) mbar_arrive(xs);
-                                ok = mbar_wait_suspended(xs, xs_phase & 1u);
+                                ok = mbar_wait_suspended(xs, xs_phase & 1u, stop, wait_ms);
                                 ++xs_phase;
                                 if (!ok) break;
                                 float ss = 0.0f;
@@ -501,17 +508,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                             }
                             __syncwarp();
                             if (lane == 0) mbar_arrive(xs);
-                            ok = mbar_wait_suspended(xs, xs_phase & 1u);
+                            ok = mbar_wait_suspended(xs, xs_phase & 1u, stop, wait_ms);
                             ++xs_phase;
                             if (!ok) break;
                             chain_back(scratch, wid, C, units, fb0 * 32, lane, act_q, act_s, act_i);
                             __syncwarp();
                             if (lane == 0) mbar_arrive(xs);
-                            ok = mbar_wait_suspended(xs, xs_phase & 1u);
+                            ok = mbar_wait_suspended(xs, xs_phase & 1u, stop, wait_ms);
                             ++xs_phase;
                         }
                         if (!ok) { alive = false; break; }
                         if (spread) {
+                            bool armed = false;
                             if (wid == 0 && lane == 0) {
                                 if (fb_lo < fb_hi) {                    // this CTA's block is in the image (behind the meeting: every warp's part)
                                     __threadfence();
@@ -526,10 +534,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                     bulk_g2s(own, table_image, (uint32_t)R.nb * STREAM_ACT_WORDS * 4, image, pol);
                                     bulk_g2s(own + q_at, table_image + q_at, (uint32_t)R.nb * 16, image, pol);
                                     bulk_g2s(own + i_at, table_image + i_at, (uint32_t)R.nb * 16, image, pol);
+                                    armed = true;
+                                } else {
+                                    *stop = 1;
                                 }
                             }
                             __syncwarp();
-                            if (!mbar_wait_suspended(image, image_phase & 1u)) { alive = false; break; }
+                            if (!mbar_wait_suspended(image, image_phase & 1u, stop, wait_ms)) {
+                                if (armed) mbar_wait_bounded(image, image_phase & 1u);      // nobody leaves with copies of its own in flight
+                                alive = false;
+                                break;
+                            }
                             ++image_phase;
                         }
                     } else {
@@ -537,7 +552,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                     }
                 }
             }
-            if (!alive) break;
+            if (!alive) {
+                if (op < n_ops) *stop = 1;
+                break;
+            }
 
             // ---- one task of op `op`: same lanes, terms and sums as gemv_stream_kernel
             const ChainOp &R = opring[op & (CHAIN_OP_RING - 1)];
@@ -554,10 +572,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
             const int lap = (int)fast_div((uint32_t)g, G.magic_nslot);
             const int slot = g - lap * G.nslot;
             if (g >= issued_seen) {                                 // tile g must be armed: then the parity below is unambiguous
-                if (!spin_until_gt(&ctrl[0], g)) break;
+                if (!spin_until_gt(&ctrl[0], g)) { *stop = 1; break; }
                 issued_seen = ctrl[0];
             }
-            if (!mbar_wait_bounded(&full[slot], (uint32_t)(lap & 1), CHAIN_NS0, CHAIN_NSMAX)) break;
+            if (!mbar_wait_bounded(&full[slot], (uint32_t)(lap & 1), CHAIN_NS0, CHAIN_NSMAX)) { *stop = 1; break; }
             const int b0 = j * R.seg_blocks;
             const int blocks = min(R.seg_blocks, nb - b0);
             const uint8_t *rowp = ring + (size_t)slot * G.slot_bytes + (size_t)(quad * 4 + rr) * row_bytes +

@@ -387,3 +387,47 @@ def test_a_rank_that_never_comes_makes_the_wait_run_out(gpu, port):
     assert float(np.abs(host(y2).astype(np.float64) - want).max()) <= REL_TOL * float(np.abs(want).max())
     chain.close()
     assert gpu.device_status() == 0
+
+
+@pytest.mark.parametrize("missing", ["rank", "blocks"])
+def test_a_dependent_op_whose_input_never_comes(gpu, missing):
+    """A two-rank list, one rank of it launched, whose second op waits for something that nobody brings: the other rank's rows (3 ms), or --
+    with both ranks' signals set beforehand and a run number that does not fit -- the rotated blocks of the other CTAs (the limit of the grid
+    counter, some seconds).  The lane that waits gives up and reports it, the warps that wait for that lane leave with it."""
+    import time
+    import torch
+    n_in, n_mid, n_out = 1024, 5120, 64
+    W0, W1 = dev(synth.pq2_0_weights(n_mid, n_in, seed=5)), dev(synth.pq2_0_weights(n_out, n_mid, seed=6))
+    xd = dev(synth.activations(n_in, seed=5))
+    payload = 32768
+
+    class TwoBuffers:
+        rank, world, counter_offset, total_bytes = 0, 2, payload, payload + 64
+
+    mine, other = (torch.zeros(payload + 64, dtype=torch.uint8, device="cuda") for _ in range(2))
+    TwoBuffers.ptrs = [mine.data_ptr(), other.data_ptr()]
+    words = mine[payload:].view(torch.int32)
+    if missing == "blocks":
+        words[2], words[8], words[9] = 1, 1 << 20, 1 << 20
+    y0, y1 = mine[:n_mid * 4].view(torch.float32), mine[n_mid * 4:(n_mid + n_out) * 4].view(torch.float32)
+    chain = gpu.Chain([(W0, xd, None, y0, n_mid, n_in, gpu.OP_ROTATE), (W1, y0, None, y1, n_out, n_mid, gpu.OP_ROTATE | gpu.OP_DEPENDS)],
+                      peers=TwoBuffers, wait_limit_us=3000)
+    assert gpu.device_status() == 0
+    t0 = time.perf_counter()
+    assert chain.run() == 0
+    torch.cuda.synchronize()
+    assert time.perf_counter() - t0 < 7.0                # below the limit of the warps that are told
+    assert gpu.device_status() != 0
+    chain.close()
+    assert gpu.clear_status() == 0
+    # the context is intact: the same list of one rank
+    got0, got1, ref0, ref1 = torch.zeros(n_mid, device="cuda"), torch.zeros(n_out, device="cuda"), torch.zeros(n_mid, device="cuda"), torch.zeros(n_out, device="cuda")
+    scratch = torch.zeros(n_mid // 32 * 36, dtype=torch.uint8, device="cuda")
+    assert gpu.linear(W0, xd, None, ref0, scratch, n_mid, n_in) == 0
+    assert gpu.linear(W1, ref0, None, ref1, scratch, n_out, n_mid) == 0
+    chain = gpu.Chain([(W0, xd, None, got0, n_mid, n_in, gpu.OP_ROTATE), (W1, got0, None, got1, n_out, n_mid, gpu.OP_ROTATE | gpu.OP_DEPENDS)])
+    assert chain.run() == 0
+    torch.cuda.synchronize()
+    assert torch.equal(got0, ref0) and torch.equal(got1, ref1)
+    chain.close()
+    assert gpu.device_status() == 0
