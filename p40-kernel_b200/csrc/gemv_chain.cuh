@@ -196,41 +196,33 @@ struct ChainPeers {
     unsigned int *counter[CHAIN_MAX_RANKS];     // rank p's counter block
 };
 
-// Back butterflies and quantiser of a warp's units (u0, u0 + step, ... of `units` slices of the scratch area) into the tables, up to
-// three side by side: one after the other they took 1600 clocks each, a chain of shuffles and divisions.  Not inlined: beside the multiply's
-// registers it would spill, and a spilled value of the multiply costs more than this saves.
+// Back butterflies and quantiser of N units (u0, u0 + step, ... slices of the scratch area) side by side into the tables.
 template <int N>
-__device__ __forceinline__ void chain_back_units(const float4 *scratch, int u0, int step, int units, int chunk0, int lane, uint32_t *act_q, float *act_s, int *act_i) {
+__device__ __forceinline__ void chain_back_units(const float4 *scratch, int u0, int step, int chunk0, int lane, uint32_t *act_q, float *act_s, int *act_i) {
     float v[N][4];
     uint32_t word[N], header[N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-        const int u = min(u0 + k * step, units - 1);                // (a warp with one less does the last again, stores nothing)
+        const int u = u0 + k * step;
         fwht_slice_back(scratch + (u >> 3) * 256, u & 7, lane, v[k]);
     }
     quantise_chunks_8lanes<N>(v, lane, word, header);
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-        const int u = u0 + k * step;
-        if (u < units) {
-            const int chunk = chunk0 + u * 4 + (lane >> 3);
-            act_q[(chunk >> 2) * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word[k];
-            if ((lane & 7) == 0) {
-                act_s[chunk] = f16_bits_to_f32(header[k] & 0xFFFFu);
-                act_i[chunk] = -64 * (int)(short)(header[k] >> 16);
-            }
+        const int chunk = chunk0 + (u0 + k * step) * 4 + (lane >> 3);
+        act_q[(chunk >> 2) * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word[k];
+        if ((lane & 7) == 0) {
+            act_s[chunk] = f16_bits_to_f32(header[k] & 0xFFFFu);
+            act_i[chunk] = -64 * (int)(short)(header[k] >> 16);
         }
     }
 }
-__device__ __noinline__ void chain_back(const float4 *scratch, int u0, int step, int units, int chunk0, int lane, uint32_t *act_q, float *act_s, int *act_i) {
-    for (int rounds = (units + step - 1) / step; u0 < units;) {
-        const int n = rounds == 4 ? 2 : min(rounds, 3);
-        if (n == 1) chain_back_units<1>(scratch, u0, step, units, chunk0, lane, act_q, act_s, act_i);
-        else if (n == 2) chain_back_units<2>(scratch, u0, step, units, chunk0, lane, act_q, act_s, act_i);
-        else chain_back_units<3>(scratch, u0, step, units, chunk0, lane, act_q, act_s, act_i);
-        rounds -= n;
-        u0 += n * step;
-    }
+// A warp's units, PAIRS: two at a time (one after the other each is a chain of shuffles and divisions of 1600 clocks).
+template <bool PAIRS>
+__device__ __forceinline__ void chain_back(const float4 *scratch, int u0, int step, int units, int chunk0, int lane, uint32_t *act_q, float *act_s, int *act_i) {
+    if (PAIRS)
+        for (; u0 + step < units; u0 += 2 * step) chain_back_units<2>(scratch, u0, step, chunk0, lane, act_q, act_s, act_i);
+    for (; u0 < units; u0 += step) chain_back_units<1>(scratch, u0, step, chunk0, lane, act_q, act_s, act_i);
 }
 
 template <int THREADS, int MAXSTEPS, bool TP>
@@ -316,13 +308,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
 
     if (wid < C) {
         // ================================ compute warps ================================
+        // The multiply fills the registers of a thread, so a warp carries little through it: the rows of the op come from its record and
+        // the armed tiles from their counter each time, and nothing is called (what a caller keeps beyond the registers that a callee
+        // preserves goes to memory, of which 227 KB of shared memory leave L1 little).  With these in registers and the back butterflies in a
+        // function, 8 bytes of spills at 512 threads, 116 at 640, 152 at 768, 44 with several ranks; now 0, 0, 16 and 4.  Sweep of 8 layers
+        // and 12 layers of a decode step, us: 512 threads 118.9, 717 -> 118.2, 708; 640 158, 894 -> 145, 797; 768 154, 952 -> 139, 803; one
+        // rank of two alone 157, 1698 -> 144, 1626.
         const int rr = lane & 3, bl = lane >> 2;
         int op = -1, flags = 0;
-        int issued_seen = 0;
         volatile int *stop = &ctrl[14];
         const uint32_t wait_ms = CHAIN_WAIT_MS + (TP ? (uint32_t)(PE.wait_limit_ns >> 20) : 0u);
         uint32_t xs_phase = 0, dep_phase = 0, image_phase = 0;     // every compute warp takes part in every meeting, so it counts them itself
-        int task_base = 0, ntasks = 0, g_base = 0, ntiles = 0, row0 = 0, rows_here = 0;
+        int task_base = 0, ntasks = 0, g_base = 0, ntiles = 0;
         for (;;) {
             int task = 0;
             if (lane == 0) task = atomicAdd(const_cast<int *>(&ctrl[2]), 1);
@@ -366,6 +363,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                 if (TP && op >= CHAIN_GATES && !spin_until_gt(&ctrl[9], op - CHAIN_GATES)) { alive = false; break; }
                 const ChainOp &R = opring[op & (CHAIN_OP_RING - 1)];
                 flags = R.flags;
+                int row0, rows_here;
                 cta_rows(R, row0, rows_here);
                 ntiles = (rows_here + R.tr - 1) / R.tr;
                 ntasks = ntiles * R.tpt;
@@ -511,7 +509,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                             ok = mbar_wait_suspended(xs, xs_phase & 1u, stop, wait_ms);
                             ++xs_phase;
                             if (!ok) break;
-                            chain_back(scratch, wid, C, units, fb0 * 32, lane, act_q, act_s, act_i);
+                            chain_back<THREADS == 512>(scratch, wid, C, units, fb0 * 32, lane, act_q, act_s, act_i);
                             __syncwarp();
                             if (lane == 0) mbar_arrive(xs);
                             ok = mbar_wait_suspended(xs, xs_phase & 1u, stop, wait_ms);
@@ -559,6 +557,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
 
             // ---- one task of op `op`: same lanes, terms and sums as gemv_stream_kernel
             const ChainOp &R = opring[op & (CHAIN_OP_RING - 1)];
+            int row0, rows_here;
+            cta_rows(R, row0, rows_here);
             const int nb = R.nb, nseg = R.nseg;
             const int row_bytes = nb * W_BLOCK_BYTES;
             const int local_task = task - task_base;
@@ -571,10 +571,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
             const int g = g_base + t;
             const int lap = (int)fast_div((uint32_t)g, G.magic_nslot);
             const int slot = g - lap * G.nslot;
-            if (g >= issued_seen) {                                 // tile g must be armed: then the parity below is unambiguous
-                if (!spin_until_gt(&ctrl[0], g)) { *stop = 1; break; }
-                issued_seen = ctrl[0];
-            }
+            if (!spin_until_gt(&ctrl[0], g)) { *stop = 1; break; }      // tile g must be armed: then the parity below is unambiguous
             if (!mbar_wait_bounded(&full[slot], (uint32_t)(lap & 1), CHAIN_NS0, CHAIN_NSMAX)) { *stop = 1; break; }
             const int b0 = j * R.seg_blocks;
             const int blocks = min(R.seg_blocks, nb - b0);

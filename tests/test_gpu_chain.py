@@ -431,3 +431,55 @@ def test_a_dependent_op_whose_input_never_comes(gpu, missing):
     assert torch.equal(got0, ref0) and torch.equal(got1, ref1)
     chain.close()
     assert gpu.device_status() == 0
+
+
+def test_one_rank_of_two_alone(gpu):
+    """The several-rank form on one device: rank 0 of two, with the other rank's rows and its signals there beforehand.  Its own rows -- plain,
+    rotated for itself and once for the grid, behind a norm, with shared inputs -- are the per-matrix bits in its buffer and in the other's."""
+    import torch
+    widths = [1024, 5120, 6144, 5120, 2048, 17408, 1024]
+    eps = 1e-6
+    x0 = dev(synth.activations(widths[0], seed=3))
+    scratch = torch.zeros(17408 // 32 * 36, dtype=torch.uint8, device="cuda")
+    at = np.concatenate([[0], np.cumsum([*widths[1:], 700])]).astype(int)
+    payload = (int(at[-1]) * 4 + 63) // 64 * 64
+    mine, other = (torch.zeros(payload + 64, dtype=torch.uint8, device="cuda") for _ in range(2))
+    mine[payload:].view(torch.int32)[9] = 1 << 30
+
+    class TwoBuffers:
+        rank, world, counter_offset, total_bytes, ptrs = 0, 2, payload, payload + 64, [mine.data_ptr(), other.data_ptr()]
+
+    got, sent = mine[:payload].view(torch.float32), other[:payload].view(torch.float32)
+    ops, refs, x, x_ref = [], [], x0, x0
+
+    def add(place, n_out, n_in, sg, norm, more):
+        W, half, ref, t = synth.pq2_0_weights(n_out, n_in, seed=70 + len(ops)), n_out // 2, torch.zeros(n_out, device="cuda"), torch.empty(n_in, device="cuda")
+        if norm is not None:
+            assert gpu.rmsnorm(x_ref, norm, t, 1, n_in, eps) == 0
+        assert gpu.linear(dev(W), x_ref if norm is None else t, sg, ref, scratch, n_out, n_in) == 0
+        ops.append((dev(W[:half * (n_in // 128) * 34]), x, sg, got[at[place]:at[place] + half], half, n_in, gpu.OP_ROTATE | more,
+                    *((norm, eps) if norm is not None else ())))
+        refs.append((place, half, ref))
+
+    for i, (n_in, n_out) in enumerate(zip(widths, widths[1:])):
+        sg = dev(synth.signs(n_in, seed=i)) if i % 2 else None
+        norm = 1 + 0.1 * dev(synth.activations(n_in, seed=i)) if n_in == 5120 else None
+        kind = gpu.OP_RMSNORM if norm is not None else 0
+        add(i, n_out, n_in, sg, norm, kind | (gpu.OP_DEPENDS if i else 0))
+        ref = refs[-1][2]
+        if i == 2:
+            add(len(widths) - 1, 700, n_in, sg, norm, kind | gpu.OP_SAME_INPUT)
+        x, x_ref = got[at[i]:at[i] + n_out], ref
+    for place, half, ref in refs:
+        got[at[place] + half:at[place] + ref.numel()] = ref[half:]
+    chain = gpu.Chain(ops, peers=TwoBuffers)
+    for run in range(3):
+        for place, half, ref in refs:
+            got[at[place]:at[place] + half] = -3.0
+        assert chain.run() == 0
+        torch.cuda.synchronize()
+        assert gpu.device_status() == 0
+        for place, half, ref in refs:
+            assert torch.equal(got[at[place]:at[place] + ref.numel()], ref), (run, place)
+            assert torch.equal(sent[at[place]:at[place] + half], ref[:half]), (run, place)
+    chain.close()
