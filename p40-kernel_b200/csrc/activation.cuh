@@ -55,7 +55,7 @@ __device__ __forceinline__ void quantise_chunk_8lanes(const float (&v)[4], int l
 // g alone.
 template <int N>
 __device__ __forceinline__ void quantise_chunks_8lanes(const float (&v)[N][4], int lane, uint32_t (&word)[N], uint32_t (&header)[N]) {
-    static_assert(N <= 8, "a lane of the eight per chunk");
+    static_assert(N > 1 && N <= 8, "a lane of the eight per chunk; nothing to share in one");
     float amax[N], mine;
 #pragma unroll
     for (int k = 0; k < N; ++k) amax[k] = fmaxf(fmaxf(fabsf(v[k][0]), fabsf(v[k][1])), fmaxf(fabsf(v[k][2]), fabsf(v[k][3])));
@@ -101,6 +101,11 @@ __device__ __forceinline__ void quantise_chunks_8lanes(const float (&v)[N][4], i
         }
         header[k] = d16[k] | (((uint32_t)sum[k] & 0xFFFFu) << 16);
     }
+}
+
+template <>
+__device__ __forceinline__ void quantise_chunks_8lanes<1>(const float (&v)[1][4], int lane, uint32_t (&word)[1], uint32_t (&header)[1]) {
+    quantise_chunk_8lanes(v[0], lane, word[0], header[0]);
 }
 
 // Four consecutive floats: one 16-byte access when the caller's pointer allows it (VEC), else four 4-byte

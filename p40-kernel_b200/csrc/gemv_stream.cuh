@@ -280,6 +280,7 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
         bool first = true;
         for (int s0 = wid; s0 < P.nb || first; s0 += SLICES * compute_warps) {
             float4 f[SLICES];
+            const int left = P.nb - s0, n = 1 + (left > compute_warps) + (left > 2 * compute_warps) + (left > 3 * compute_warps);
 #pragma unroll
             for (int k = 0; k < SLICES; ++k) {
                 const int sl = s0 + k * compute_warps;
@@ -293,7 +294,9 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
                 first = false;
             }
             // a warp's slices side by side, their divisions shared (one per lane of a chunk): one after the other each was a chain
-            // of shuffles and two divisions, before the first product (17408 -> 5120 16.05 -> 15.2 us, 5 slices and then 4 or 5)
+            // of shuffles and two divisions, before the first product.  As many as there are: a slice that is not there costs what one does
+            // (n by comparisons: a division is 40 clocks).  us one after the other / three or five always / now, to 5120 rows: 1024 2.81 / 2.91 /
+            // 2.84, 3072 3.92 / 4.16 / 3.75, 5120 4.97 / 4.86 / 4.69, 17408 12.61 / 11.82 / 11.49.  (Four of their own: 1024 2.91, 17408 11.45.)
             auto quantise = [&](auto count) {
                 constexpr int N = decltype(count)::value;
                 float v[N][4];
@@ -315,9 +318,9 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
                 }
             };
             if (wid < compute_warps && s0 < P.nb) {                     // warp-uniform
-                const int n = (P.nb - s0 + compute_warps - 1) / compute_warps;
                 if (n == 1) quantise(std::integral_constant<int, 1>());
-                else if (n <= 3) quantise(std::integral_constant<int, 3>());
+                else if (n == 2) quantise(std::integral_constant<int, 2>());
+                else if (n == 3) quantise(std::integral_constant<int, 3>());
                 else quantise(std::integral_constant<int, SLICES>());
             }
         }

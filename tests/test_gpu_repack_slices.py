@@ -1,5 +1,5 @@
-"""The repacked mat-vec's own quantiser at every number of 128-element slices a warp takes side by side (one, up to three, up to five, a
-second round of one, two and five): the bits of quantiser and plain mat-vec in two steps."""
+"""The repacked mat-vec's own quantiser at every number of 128-element slices a warp takes side by side (one, two, three, four or five, a
+second round of one to five): the bits of quantiser and plain mat-vec in two steps."""
 import numpy as np
 import pytest
 
@@ -8,7 +8,7 @@ from bonsai_b200 import synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n_in", [1024 * k for k in (1, 2, 4, 5, 6, 9, 10, 12, 17, 19)])
+@pytest.mark.parametrize("n_in", [1024 * k for k in (1, 2, 3, 4, 5, 6, 7, 9, 10, 12, 14, 17, 19)])
 def test_slices(gpu, n_in):
     import torch
     n_out = 37
