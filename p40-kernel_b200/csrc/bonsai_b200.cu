@@ -1580,8 +1580,12 @@ int bonsai_kv_append_batch(bonsai_kv_cache *kv, int layer, int pos0, int n_tok, 
     if (n_tok <= 0 || pos0 < 0 || (long long)pos0 + n_tok > kv->capacity) return 1;
     const int nrow = n_tok * KVM_KV_HEADS;
     // any float pointer is taken; 16-byte aligned ones get 16-byte loads
-    auto kernel = aligned16(k) && aligned16(v) ? kv_append_kernel<true> : kv_append_kernel<false>;
-    return (int)launch(kernel, dim3((unsigned)((nrow + 7) / 8)), dim3(256), 0, as_stream(stream), true, kv->d_k, kv->d_v, k, v, pos0, n_tok,
+    const bool vec = aligned16(k) && aligned16(v);
+    const int blocks = (nrow + 7) / 8;
+    const bool early = blocks <= 8 * SM_COUNT;              // 2368 tokens: one wave of eight blocks of 256 threads per SM
+    auto kernel = early ? (vec ? kv_append_kernel<true, true> : kv_append_kernel<false, true>)
+                        : (vec ? kv_append_kernel<true, false> : kv_append_kernel<false, false>);
+    return (int)launch(kernel, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, kv->d_k, kv->d_v, k, v, pos0, n_tok,
                        KVM_KV_HEADS, kv->capacity, layer);
 }
 

@@ -70,6 +70,32 @@ def test_append_bytes_and_layout(gpu, port):
     kv.close()
 
 
+@pytest.mark.parametrize("n_tok", [1, 2, 3, 2368, 2369])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_append_of_many_tokens(gpu, port, n_tok, offset):
+    """The last number of tokens whose blocks are resident at once and the next one, rows that start on 16 bytes and rows that do not: the
+    host quantiser's bytes of the first, last and sampled rows, behind a kernel that writes the rows just before."""
+    import torch
+    cap, layer = n_tok + 2, 11
+    kv = gpu.KVCache(cap)
+    rng = np.random.default_rng(n_tok)
+    src = [dev(rng.standard_normal(n_tok * N_KV * D).astype(np.float32)) for _ in range(2)]
+    room = [torch.full((n_tok * N_KV * D + 4,), 9.0, device="cuda") for _ in range(2)]
+    rows = [r[offset:offset + n_tok * N_KV * D] for r in room]
+    torch.cuda.synchronize()
+    for r, s in zip(rows, src):
+        r.copy_(s)
+    assert kv.append_batch(layer, 1, n_tok, *rows) == 0
+    torch.cuda.synchronize()
+    for raw, s in zip(cache_bytes(gpu, kv), src):
+        want = host(s).reshape(n_tok, N_KV, D)
+        for t in np.unique(np.linspace(0, n_tok - 1, 40).astype(int)):
+            for h in range(N_KV):
+                at = ((layer * N_KV + h) * cap + 1 + t) * 272
+                assert np.array_equal(raw[at:at + 272], port.kv_quantize_row(want[t, h])), (t, h)
+    kv.close()
+
+
 @pytest.mark.parametrize("pos", [0, 1, 31, 32, 255, 256, 300, 2100])
 def test_attn_decode(gpu, port, pos):
     import torch
