@@ -150,7 +150,8 @@ int bonsai_b200_stream_probe(const void *buf, int64_t bytes, int mode, void *sin
  * Options are process-wide: set them once at start-up, not from threads that call the library concurrently.
  * A library compiled with -DBONSAI_B200_TUNING (the test build) also takes geometry keys ("gemv_variant",
  * "chain_threads", "chain_seg", "chain_tile_kb", "chain_spread_nb", "gemm_tile") that force a tiling; they change no result bits
- * beyond what the documented options say and are not part of the interface.
+ * beyond what the documented options say and are not part of the interface; nor is "kv_wide" (0 = decode attention over the cache keeps
+ * clusters of eight CTAs at every length: the same bound, another order of sums).
  * Returns 0, or 1 for an unknown key. */
 int bonsai_b200_set_option(const char *key, int64_t value);
 
@@ -249,6 +250,11 @@ int bonsai_b200_chain_info(const bonsai_b200_chain *chain, int64_t out[4]);
  * each: lets a test read the Q8_0 bytes back.  No counterpart in the reference, whose cache object is opaque. */
 struct bonsai_kv_cache;
 int bonsai_b200_kv_arrays(struct bonsai_kv_cache *kv, void **k, void **v, int64_t *bytes_each);
+
+/* How bonsai_kv_attn_decode divides n_pos positions of a kv head on a device where resident8 clusters of 8 CTAs and resident16 of 16 run
+ * at once (negative: as many as on the current device; 0: none): out = CTAs per cluster, clusters, positions per CTA.  Launches nothing;
+ * with both numbers given it needs no GPU.  For tests.  Returns 1 for bad arguments or where clusters of 8 do not run. */
+int bonsai_b200_kv_splits(int n_pos, int resident8, int resident16, int64_t out[3]);
 
 /* Version of this build as major * 100 + minor. */
 int bonsai_b200_version(void);

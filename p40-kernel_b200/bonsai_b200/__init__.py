@@ -55,6 +55,7 @@ SIGNATURES = {
     "bonsai_b200_chain_destroy": (_INT, [_VP]),
     "bonsai_b200_chain_info": (_INT, [_VP, _VP]),
     "bonsai_b200_kv_arrays": (_INT, [_VP, _VP, _VP, _VP]),
+    "bonsai_b200_kv_splits": (_INT, [_INT, _INT, _INT, _VP]),
     "bonsai_kv_bytes": (_I64, [_INT]),
     "bonsai_kv_gdn_bytes": (_I64, []),
     "bonsai_kv_create": (_VP, [_INT, _VP]),

@@ -50,6 +50,7 @@ std::atomic<int> g_opt_chain_threads{512};       // threads per CTA of the chain
 std::atomic<int> g_opt_chain_spread_nb{40};      // dependent ops with at least this many blocks per row rotate their input
                                                  // once for the grid instead of once per CTA; 0 = never
 std::atomic<int> g_opt_chain_tile_kb{16};
+std::atomic<int> g_opt_kv_wide{1};                // decode attention: 0 = clusters of eight CTAs at every length
 std::atomic<int> g_opt_gemm_tile{0};              // fp16 tensor-core mat-mul: 0 by token count, 64 or 128 tokens per tile
 std::atomic<int> g_opt_chain_seg{40};            // longest row segment of one task, in blocks: 8, 16, 24, 32 or 40        // target bytes of one ring slot
 std::atomic<int> g_opt_gemm_path{-1};          // -1: by token count, 0: integer SIMT kernel, 1: tensor cores, 2: small-batch kernel, 3: integer tensor-core kernel          // 0: streaming kernel (fixed tree order), 1: the host's sequential order
@@ -1345,6 +1346,7 @@ int bonsai_b200_set_option(const char *key, int64_t value) {
         g_opt_gemm_tile.store((int)value);
         return 0;
     }
+    if (!std::strcmp(key, "kv_wide")) { g_opt_kv_wide.store(value != 0); return 0; }
     if (!std::strcmp(key, "chain_tile_kb")) {
         if (value < 4 || value > 48) return 1;
         g_opt_chain_tile_kb.store((int)value);
@@ -1479,9 +1481,9 @@ inline int64_t kv_gdn_bytes() { return (int64_t)KVM_LINEAR * KVM_V_HEADS * KVM_S
 constexpr int KV_COUNTERS = KVM_KV_HEADS * KV_CLUSTER;      // per layer
 inline size_t kv_ws_floats(int max_clusters) { return (size_t)KVM_KV_HEADS * KV_CLUSTER * max_clusters * KV_REC; }      // per layer
 
-// Clusters (of 8 or of 16 CTAs) of the decode kernel per kv head that are resident at once on the current device (0: they do not run
-// here).  Asked once per device.
-int kv_max_clusters(bool wide) {
+// Clusters of 8 (or, wide, of 16) CTAs of the decode kernel that are resident at once on the current device (0: they do not run here).
+// Asked once per device.
+int kv_resident(bool wide) {
     static std::atomic<int> known[2][64];
     static SmemOptIn opt[2];
     int dev = 0, resident = 0;
@@ -1507,10 +1509,32 @@ int kv_max_clusters(bool wide) {
         (void)cudaGetLastError();
         return 0;
     }
-    resident = std::min(std::max(resident / KVM_KV_HEADS, 1), KV_MAX_CLUSTERS);
     if (dev < 64) known[wide][dev].store(resident, std::memory_order_relaxed);
     return resident;
 }
+// Clusters of eight per kv head that a device with so many of them resident gets at most: one wave.
+inline int kv_max_clusters(int resident) { return resident <= 0 ? 0 : std::min(std::max(resident / KVM_KV_HEADS, 1), KV_MAX_CLUSTERS); }
+
+// How n_pos positions of a kv head are divided: clusters of `cluster` CTAs, a split per CTA, `chunk` positions per split.
+struct KvSplits {
+    int cluster, clusters, chunk;
+};
+KvSplits kv_splits(int n_pos, int max_clusters, bool wide_runs) {
+    // One cluster (eight splits) per kv head until a split has KV_SPLIT_MIN positions -- two tiles, both in flight at once --
+    // then more, up to what is resident at once (one wave).  Splits are multiples of 16 positions (a warp's share of a
+    // tile), not of whole tiles: at 32 768 positions the longest is 5 % longer than the mean instead of 12 %.
+    KvSplits s{KV_CLUSTER, std::max(1, std::min(n_pos / (KV_CLUSTER * KV_SPLIT_MIN), max_clusters)), 0};
+    // One cluster of 16 where one or two of eight would do and each of their splits would have more than a tile, 513 to 3071 positions: 701
+    // are a tile a split, not two one after the other, and 2048 need no merge through memory.  16 layers with their appends, in us,
+    // with clusters of 8 and of 16: 513 positions 145 / 126, 701 148 / 128, 1501 180 / 150, 2048 187 / 158, 3001 213 / 186.  Up to 512 a split
+    // of eight is one tile already; from 3072 on three clusters of eight have more splits than the one of 16 that the kernel is laid out for.
+    if (wide_runs && n_pos > KV_CLUSTER * KV_TILE && n_pos < 3 * KV_CLUSTER * KV_SPLIT_MIN) s.cluster = KV_WIDE_CLUSTER, s.clusters = 1;
+    const int n_split = s.cluster * s.clusters;
+    s.chunk = (((n_pos + n_split - 1) / n_split) + 15) / 16 * 16;
+    return s;
+}
+// Clusters of 16 serve where those of all kv heads run at once; in waves they would be slower than clusters of eight.
+inline bool kv_wide_runs(int resident_wide) { return g_opt_kv_wide.load() && resident_wide >= KVM_KV_HEADS; }
 }  // namespace
 
 struct bonsai_kv_cache {
@@ -1519,8 +1543,8 @@ struct bonsai_kv_cache {
     float *d_gdn = nullptr, *d_ws = nullptr;
     unsigned int *d_counters = nullptr;         // behind the workspace's records; records and counters are a layer's own, so
                                                 // that layers may be decoded on different streams at once
-    int max_clusters = 1;                       // clusters of the decode kernel per kv head that are resident at once
-    bool wide_clusters = false;                 // clusters of 16 run here
+    int max_clusters = 1;                       // clusters of eight of the decode kernel per kv head, at most
+    int resident_wide = 0;                      // clusters of 16 that are resident at once
 };
 
 int64_t bonsai_kv_bytes(int capacity) {
@@ -1536,8 +1560,8 @@ bonsai_kv_cache *bonsai_kv_create(int capacity, bonsai_stream stream) {
     bonsai_kv_cache *kv = new (std::nothrow) bonsai_kv_cache;
     if (!kv) return nullptr;
     kv->capacity = capacity;
-    kv->max_clusters = kv_max_clusters(false);
-    kv->wide_clusters = kv_max_clusters(true) > 0;
+    kv->max_clusters = kv_max_clusters(kv_resident(false));
+    kv->resident_wide = kv_resident(true);
     const size_t ws = (size_t)KVM_FULL * kv_ws_floats(kv->max_clusters) * sizeof(float), ncnt = (size_t)KVM_FULL * KV_COUNTERS * sizeof(unsigned int);
     if (kv->max_clusters <= 0 || cudaMalloc(&kv->d_k, (size_t)kv_array_bytes(capacity)) != cudaSuccess ||
         cudaMalloc(&kv->d_v, (size_t)kv_array_bytes(capacity)) != cudaSuccess || cudaMalloc(&kv->d_gdn, (size_t)kv_gdn_bytes()) != cudaSuccess ||
@@ -1597,29 +1621,16 @@ int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *
     if (!kv || !q || !out) return 1;
     if (layer < 0 || layer >= KVM_FULL) return 1;
     if (pos < 0 || pos >= kv->capacity) return 1;
-    // One cluster (eight splits) per kv head until a split has KV_SPLIT_MIN positions -- two tiles, both in flight at once --
-    // then more, up to what is resident at once (one wave).  Splits are multiples of 16 positions (a warp's share of a
-    // tile), not of whole tiles: at 32 768 positions the longest is 5 % longer than the mean instead of 12 %.
-    const int n_pos = pos + 1;
-    long long n_cl = n_pos / (KV_CLUSTER * KV_SPLIT_MIN);
-    if (n_cl < 1) n_cl = 1;
-    if (n_cl > kv->max_clusters) n_cl = kv->max_clusters;
-    // One cluster of 16 where one or two of eight would do and each of their splits would have more than a tile: 701 positions are a
-    // tile a split, not two one after the other, and 2048 need no merge through memory.  16 layers with their appends, in us, with
-    // clusters of 8 and of 16: 701 positions 150 / 127, 1501 184 / 150, 2048 191 / 159, 3001 215 / 185.  Up to 512 a split of eight
-    // is one tile already; from 3072 on three clusters of eight have more splits.
-    const bool wide = kv->wide_clusters && n_cl <= 2 && n_pos > KV_CLUSTER * KV_TILE;
-    const int cluster = wide ? KV_WIDE_CLUSTER : KV_CLUSTER;
-    const int n_split = wide ? KV_WIDE_CLUSTER : (int)n_cl * KV_CLUSTER;
-    const int chunk = (((n_pos + n_split - 1) / n_split) + 15) / 16 * 16;
+    const KvSplits s = kv_splits(pos + 1, kv->max_clusters, kv_wide_runs(kv->resident_wide));
+    const bool wide = s.cluster == KV_WIDE_CLUSTER;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)n_split, KVM_KV_HEADS);
+    cfg.gridDim = dim3((unsigned)(s.cluster * s.clusters), KVM_KV_HEADS);
     cfg.blockDim = dim3(KV_THREADS);
     cfg.dynamicSmemBytes = KV_SMEM_BYTES;
     cfg.stream = as_stream(stream);
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.x = (unsigned)s.cluster;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
@@ -1627,7 +1638,18 @@ int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *
     cfg.numAttrs = g_opt_overlap.load() ? 2 : 1;
     return (int)cudaLaunchKernelEx(&cfg, wide ? kv_attn_kernel<KVM_GROUP, KV_WIDE_CLUSTER> : kv_attn_kernel<KVM_GROUP, KV_CLUSTER>, q, (const uint8_t *)kv->d_k, (const uint8_t *)kv->d_v,
                                    kv->d_ws + (size_t)layer * kv_ws_floats(kv->max_clusters), kv->d_counters + layer * KV_COUNTERS, out,
-                                   pos, chunk, KVM_KV_HEADS, kv->capacity, layer, 0.0625f);
+                                   pos, s.chunk, KVM_KV_HEADS, kv->capacity, layer, 0.0625f);
+}
+
+int bonsai_b200_kv_splits(int n_pos, int resident8, int resident16, int64_t out[3]) {
+    if (n_pos <= 0 || n_pos > KVM_CONTEXT || !out) return 1;
+    const int max_clusters = kv_max_clusters(resident8 < 0 ? kv_resident(false) : resident8);
+    if (max_clusters <= 0) return 1;
+    const KvSplits s = kv_splits(n_pos, max_clusters, kv_wide_runs(resident16 < 0 ? kv_resident(true) : resident16));
+    out[0] = s.cluster;
+    out[1] = s.clusters;
+    out[2] = s.chunk;
+    return 0;
 }
 
 // Test access to the cache arrays (byte parity of the quantiser): device pointers of K and V.

@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
     cluster_wait();
     // ---- one slice of the dims per CTA of the cluster, added over its CTAs in rank order
     const uint32_t rank = cluster_rank();
-    const int n_cl = gridDim.x / CL, cl = blockIdx.x / CL;
+    const int n_cl = CL == KV_CLUSTER ? gridDim.x / CL : 1, cl = CL == KV_CLUSTER ? blockIdx.x / CL : 0;      // (records and counters are laid out for clusters of eight)
     constexpr int SLICE = KV_D / CL;
     float *cw = wt, *cm = mw, *cl_sum = lw;                            // [8 heads][CL ranks] weights; maxima; denominators
     constexpr int OUTS = GRP * SLICE, ROUNDS = (OUTS + KV_THREADS - 1) / KV_THREADS;

@@ -1,5 +1,8 @@
 """Decode attention at the lengths between which one cluster of sixteen CTAs serves a kv head: the first and last of them, the first
-with a second tile in a split, splits that are empty.  Oracle and bound as in test_gpu_kv_splits."""
+with a second tile in a split, splits that are empty; and with the clusters of eight that serve there where sixteen cannot be placed.
+Oracle and bound as in test_gpu_kv_splits."""
+import ctypes as C
+
 import pytest
 
 from test_gpu_kv_splits import D, N_HEADS, REL_TOL, exact, fill
@@ -7,15 +10,22 @@ from test_gpu_kv_splits import D, N_HEADS, REL_TOL, exact, fill
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [512, 513, 528, 529, 769, 1040, 1041, 3071, 3072])
+@pytest.mark.parametrize("n", [512, 513, 528, 529, 769, 1025, 1040, 1041, 2047, 2048, 3071, 3072])
 @pytest.mark.parametrize("spread", [0, 1])
-def test_against_float64(gpu, port, n, spread):
+@pytest.mark.parametrize("wide", [1, 0])
+def test_against_float64(gpu, port, n, spread, wide):
     import torch
-    kv, layer = gpu.KVCache(n), 9
+    kv, layer, splits = gpu.KVCache(n), 9, (C.c_int64 * 3)()
     q = fill(kv, layer, n, n, spread)
     out = torch.full((N_HEADS, D), float("nan"), device="cuda")
-    for _ in range(2):
-        assert kv.attn_decode(layer, n - 1, q, out) == 0
+    try:
+        assert gpu.set_option("kv_wide", wide) == 0
+        assert gpu.lib().bonsai_b200_kv_splits(n, -1, -1, splits) == 0
+        assert splits[0] == (16 if wide and 513 <= n <= 3071 else 8)
+        for _ in range(2):
+            assert kv.attn_decode(layer, n - 1, q, out) == 0
+    finally:
+        gpu.set_option("kv_wide", 1)
     want = exact(port, kv, n, layer, n, q)
     err, top = float((out.double() - want).abs().max()), float(want.abs().max())
     assert err <= REL_TOL * top, (err, top)
