@@ -316,7 +316,9 @@ __global__ void __launch_bounds__(32 * FWHT_WARP_BLOCKS, 8) fwht_quant_warp_kern
     }
     if (xq) {
 #pragma unroll
-        for (int r0 = 0; r0 < 8; r0 += 4) {             // four slices side by side
+        // four slices side by side, their divisions shared: one after the other each was a chain of shuffles and two divisions (us per call:
+        // 5120 wide, 512 tokens 9.10 -> 8.03, 2048 tokens 24.7 -> 21.7; 17408 wide, 128 tokens 7.53 -> 6.61, 2048 tokens 78.0 -> 67.5; same bits)
+        for (int r0 = 0; r0 < 8; r0 += 4) {
             float s[4][4];
             uint32_t word[4], header[4];
 #pragma unroll

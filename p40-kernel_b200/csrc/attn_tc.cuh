@@ -22,7 +22,7 @@
 // columns: 256 output (before that, sums of the scores), 128 scores (then weights), 128 q low.
 // What bounds it (counted while a score was four sums): per tile 5900 of 10200 cycles were the tensor core's, most of them the score
 // products (N = 64: it waits for the q rows from shared memory), the rest softmax and the exchanges in front of it.  2048 tokens, 24 heads over 4: 2570 ->
-// 287 us; 1000 tokens 727 -> 91 us, 600 tokens 60 us.
+// 286 us; 1000 tokens 727 -> 92 us, 600 tokens 62 us.
 //
 // A plane pair holds 2^-39 of the largest value under its power of two, so what is far smaller loses bits to values that a row may not
 // even see.  A CTA whose queries and keys range too widely (atc_too_wide) does its queries again on the CUDA cores (attn_simt), with
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
         tc_fence_after();
         {
             // (eight columns at a time: sixteen of two sums beside the outputs and the scores were more registers than a thread has, and what is
-            // spilled beside 200 KB of shared memory comes from L2: 2048 tokens 293 -> 287 us)
+            // spilled beside 200 KB of shared memory comes from L2: 2048 tokens 292 -> 286 us, 600 tokens 63.2 -> 61.6 us)
 #pragma unroll
             for (uint32_t h = 0; h < 16; h += 8) {
                 int a[8], b[8], c[8], d[8];

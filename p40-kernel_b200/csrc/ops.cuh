@@ -177,7 +177,8 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_step_kernel(float *state, 
     float *Sg = state + (size_t)vh * K * V + j;
     // the CTA's tile of the state, asked for while the launch before this one still runs: L2 hands out what it finds at the
     // load below, whoever writes in between
-    // (and so are its row of v, its q and k, decay and step: behind the wait each was a trip to memory, 2.9 -> 2.6 us a step of 48)
+    // (and so are its row of v, its q and k, decay and step: behind the wait each was a trip to memory, 2.9 -> 2.6 us a step of 48, 3.0 -> 2.75 where a graph
+    // replays them or their inputs are in memory)
     if ((int)threadIdx.x < K) {
         prefetch_l2(state + ((size_t)vh * K + threadIdx.x) * V + vt * 32);
     } else {

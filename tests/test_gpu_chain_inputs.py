@@ -1,4 +1,4 @@
-"""fp32 inputs of a list's ops at every number of units a warp rotates side by side (widths 1024 to 9216 and the longest of the model), by
+"""fp32 inputs of a list's ops at every number of units that a warp rotates, two at a time or one by one (widths 1024 to 9216 and the longest of the model), by
 every CTA for itself and once for the grid: the bits of the per-matrix calls."""
 import numpy as np
 import pytest
