@@ -977,19 +977,53 @@ static void fill_tc_params(TcParams &P, int64_t n_out, int64_t n_in, int64_t n_t
     P.total_it = (long long)P.n_tiles * P.nblocks;
 }
 
-static constexpr size_t T16_PARTS_BYTES = (size_t)TC_MAX_CTAS * T16C<128>::PART_FLOATS * sizeof(float);
+static constexpr size_t T16_PARTS_BYTES = (size_t)TC_MAX_CTAS * T16C<128, 2>::PART_FLOATS * sizeof(float);
 static size_t tc16_scratch_bytes(int64_t n_in, int64_t n_tok) {
     return T16_FLAGS_BYTES + T16_PARTS_BYTES + 2 * (size_t)n_tok * (size_t)n_in * sizeof(__half) + (size_t)n_tok * sizeof(float);
 }
 
-// The fp16 tensor-core mat-mul (gemm_tc16.cuh).  -1: not taken (shape, alignment, no scratch, no tensor-map encoder).
+// The fp16 tensor-core mat-mul (gemm_tc16.cuh).  -1: not taken (shape, alignment, no scratch, no tensor-map encoder, no SMs in pairs).
 extern "C++" {
-template <int TN>
+// Pairs of CTAs that are resident at once on the current device (0: they do not run here).  Asked once per device.
+static int tc16_pairs() {
+    static std::atomic<int> known[64];
+    auto *kernel = gemm_tc16_kernel<128, 2>;
+    static SmemOptIn opt;
+    int dev = 0, resident = 0;
+    if (opt.ensure(kernel) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev < 64 && (resident = known[dev].load(std::memory_order_relaxed)) != 0) return std::max(resident, 0);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(TC_MAX_CTAS);
+    cfg.blockDim = dim3(T16C<128, 2>::THREADS);
+    cfg.dynamicSmemBytes = T16C<128, 2>::SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&resident, kernel, &cfg) != cudaSuccess || resident <= 0) {
+        (void)cudaGetLastError();
+        resident = -1;
+    }
+    if (dev < 64) known[dev].store(resident, std::memory_order_relaxed);
+    return std::max(resident, 0);
+}
+
+template <int TN, int CTAS>
 static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n_out, int64_t n_in, int64_t n_tok, cudaStream_t st) {
-    constexpr int T16_N = TN;
     const int64_t nblocks = n_in / 128;
     if (nblocks % 8 != 0 || !aligned16(W) || !aligned4(Xq) || n_tok > (1 << 28)) return -1;
-    const long long tiles = (long long)((n_out + T16_M - 1) / T16_M) * ((n_tok + T16_N - 1) / T16_N);
+    int dev = 0, sms = 0, workers = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return (int)e;
+    workers = std::min(CTAS == 1 ? sms : tc16_pairs(), (TC_MAX_CTAS - 1) / CTAS);
+    if (workers <= 0) return -1;
+    // As many token tiles as TN asks for, all of about the same width: the MMAs' time is the tokens' (37 tokens take 48 columns, not 64).
+    const long long tiles_tok = (n_tok + TN - 1) / TN, step = 16 * CTAS;
+    const int tile_n = (int)(((n_tok + tiles_tok - 1) / tiles_tok + step - 1) / step * step);
+    const long long tiles = (n_out + T16_M * CTAS - 1) / (T16_M * CTAS) * tiles_tok;
     if (tiles > INT32_MAX) return -1;
     const size_t plane_bytes = (size_t)n_tok * (size_t)n_in * sizeof(__half);
     const StreamScratch::Lease lease = g_gemm_scratch.get(tc16_scratch_bytes(n_in, n_tok), st);      // held until both launches are enqueued
@@ -1002,24 +1036,23 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     alignas(64) Tc16Maps maps;
     std::memset(&maps, 0, sizeof(maps));
     if (!encode_w_map(&maps.w, W, n_out, nblocks * W_BLOCK_BYTES)) return -1;
-    if (!tensor_map_planes(&maps.x, planes, (uint64_t)n_in, (uint64_t)n_tok, (uint32_t)TN)) return -1;
-    TcParams P{};
-    fill_tc_params(P, n_out, n_in, n_tok, T16_M, T16_N);
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return (int)e;
-    if (sms > TC_MAX_CTAS - 1) sms = TC_MAX_CTAS - 1;
-    // Tiles for at most half of the SMs (a short token batch over few rows): up to four CTAs share a tile's blocks, at least 16
+    if (!tensor_map_planes(&maps.x, planes, (uint64_t)n_in, (uint64_t)n_tok, (uint32_t)(tile_n / CTAS))) return -1;
+    T16Params P{};
+    P.n_out = (int)n_out;
+    P.nblocks = (int)nblocks;
+    P.n_tok = (int)n_tok;
+    P.tile_n = tile_n;
+    P.tiles_tok = (int)tiles_tok;
+    P.n_tiles = (int)tiles;
+    P.idesc = t16_idesc(tile_n, CTAS);
+    // Tiles for at most half of the workers (a short token batch over few rows): up to four share a tile's blocks, at least 16
     // blocks each.
-    int grid = (int)(tiles < sms ? tiles : sms);
-    if (2 * tiles <= sms) {
-        long long g = P.total_it / 16;
-        if (g > 4 * tiles) g = 4 * tiles;
-        if (g > sms) g = sms;
-        if (g > grid) grid = (int)g;
-    }
-    P.stream_k = (tiles % grid != 0 && (grid > tiles || P.total_it / grid >= P.nblocks)) ? 1 : 0;
+    const long long total = tiles * nblocks;
+    int grid = (int)std::min<long long>(tiles, workers);
+    if (2 * tiles <= workers) grid = (int)std::max<long long>(grid, std::min<long long>({total / 16, 4 * tiles, workers}));
+    P.stream_k = (tiles % grid != 0 && (grid > tiles || total / grid >= nblocks)) ? 1 : 0;
+    P.per_worker = total / grid;
+    P.rest = (int)(total % grid);
     const int n_chunks = (int)(n_in / 32);
     const uint32_t *x32 = static_cast<const uint32_t *>(Xq);
     // slices: whole passes of a block, as many as bring about two blocks per SM
@@ -1027,30 +1060,37 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     int passes = (n_chunks + T16_SPLIT_PASS - 1) / T16_SPLIT_PASS;
     passes = (int)((passes * groups + 2 * sms - 1) / (2 * sms));
     const int slice = passes * T16_SPLIT_PASS;
+    static SmemOptIn opt;
+    e = opt.ensure(gemm_tc16_kernel<TN, CTAS>);
+    if (e != cudaSuccess) return (int)e;
     e = launch(tc16_split_kernel, dim3((unsigned)groups, (unsigned)((n_chunks + slice - 1) / slice)), dim3(T16_SPLIT_THREADS), 0, st, true, x32, n_chunks,
                (int)n_tok, slice, scale, planes);
     if (e != cudaSuccess) return (int)e;
-    static SmemOptIn opt;
-    e = opt.ensure(gemm_tc16_kernel<TN>);
-    if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(T16C<TN>::THREADS);
-    cfg.dynamicSmemBytes = T16C<TN>::SMEM_BYTES;
+    cfg.gridDim = dim3((unsigned)(grid * CTAS));
+    cfg.blockDim = dim3(T16C<TN, CTAS>::THREADS);
+    cfg.dynamicSmemBytes = T16C<TN, CTAS>::SMEM_BYTES;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeCooperative;        // a CTA may wait for another's part of a tile: all must be resident
     attr[0].val.cooperative = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = CTAS;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN>, Y, P, (const float *)scale, parts, flags, maps);
+    cfg.numAttrs = CTAS == 1 ? 1 : 2;
+    return (int)cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN, CTAS>, Y, P, (const float *)scale, parts, flags, maps);
 }
 }  // extern "C++"
-// Tiles of 128 tokens from 96 tokens on (the code expansion, the kernel's busiest part, is paid once per tile), of 64 below.
+// Pairs of CTAs and tiles of 128 tokens from 96 tokens on (the code expansion is paid once per tile, and each CTA fetches half of the
+// activations), tiles of 64 below.
 static int launch_gemm_tc16(const void *W, const void *Xq, float *Y, int64_t n_out, int64_t n_in, int64_t n_tok, cudaStream_t st) {
     const int tile = g_opt_gemm_tile.load();
-    if (tile == 64 || (tile != 128 && n_tok < 96)) return launch_gemm_tc16_n<64>(W, Xq, Y, n_out, n_in, n_tok, st);
-    return launch_gemm_tc16_n<128>(W, Xq, Y, n_out, n_in, n_tok, st);
+    if (tile == 128 || (tile != 64 && n_tok >= 96)) {
+        const int rc = launch_gemm_tc16_n<128, 2>(W, Xq, Y, n_out, n_in, n_tok, st);
+        if (rc >= 0) return rc;
+    }
+    return launch_gemm_tc16_n<64, 1>(W, Xq, Y, n_out, n_in, n_tok, st);
 }
 
 // The tensor-core mat-mul: one CTA per SM walks its share of the (tile, weight block) iterations.

@@ -1,77 +1,115 @@
 // gemm_tc16.cuh -- prefill mat-mul with the WHOLE contraction on the tensor cores (tcgen05.mma.kind::f16).
 //
 // gemm_tc.cuh keeps the integers of the host loop (one int8 MMA per 32-weight chunk, the per-chunk scales folded in
-// by the CUDA cores) and is bound by exactly that fold: ~5400 warp instructions per 128 x 64 x 128 unit, 70 % of the
-// issue slots, the tensor pipe 6.5 % busy.  This kernel moves the per-chunk activation scale to the OTHER side of the
+// by the CUDA cores) and is bound by exactly that fold.  This kernel moves the per-chunk activation scale to the OTHER side of the
 // tensor core.  The dequantised activation  xh = da * a  (fp16 scale x int8, 18 significant bits) is split once per
 // call into two fp16 numbers H + L = xh * 2^S exactly (S per token, a power of two that puts the token's largest
 // value just under 2^15; L is the exact remainder, and where it underflows the loss is below 2^-38 of the token's
 // largest value), the codes go to the tensor core as fp16 -1, 0, 1, 2, and one accumulator in tensor memory
 // collects  sum_k (code_k - 1) * (H_k + L_k)  over a whole 128-weight block: products are exact, sums are the tensor
 // core's fp32.  The CUDA cores are left with one fused multiply-add per output and BLOCK (the fp16 weight scale) and
-// the expansion of the codes: 2900 warp instructions per unit against 5400, and the tensor pipe 44 % busy.
+// the expansion of the codes.
 // Accuracy: the only roundings are the tensor core's fp32 additions inside a block (256 terms) and one fp32 FMA per
 // block, against the host's one rounding per chunk term: Y is held to 1e-5 of max |Y| like the integer kernel's
 // (measured ~1e-6); the INTEGERS of the host loop are not formed here: bonsai_b200_gemm_dump and
 // bonsai_b200_set_option("gemm_path", 3) keep the integer kernel.
 // Oracle: tests/test_p40.cpp:438-467 + src/pq2_0.h:149-169 (the host loop); kernel replaced: src/kernels/gemm_p40.cu:44-139.
 //
-// CTA tile 128 rows x 64 tokens, one CTA per SM, K stepped one weight block at a time = 16 MMAs (M 128, N 64, K 16):
-// two K halves of 64 values x {H, L} x four K = 16 steps, all into one 64-column accumulator (4 in flight).
-//   warps 0-7   : epilogue: per block two tcgen05.ld of 16 columns, acc += dw * D (one row x 32 tokens per thread)
-//   warps 8-23  : code producers: thread (row p, K half g), every second block: 64 two-bit codes -> 64 fp16 with byte
-//                 permutes (the fp16 patterns of -1, 0, 1, 2 differ only in their high byte), written to tensor memory
-//   warps 24-25 : issuers (alternate blocks)
-//   warps 26-27 : loaders (tiled TMA copies): weight pieces of 8 blocks x 128 rows; per half block a box of 64 values x
-//                 64 tokens x {H, L}, landing swizzled as the MMA reads it
-// Work split and time-outs as in gemm_tc.cuh (same walk); the parts of a tile meet in one step, through slots and flags (one per CTA) in the
-// scratch, which is the stream's own.  (Flags in eight sets that launches took in turn were shared by the ninth launch on another
-// stream, or by a replayed one.)
-// Every role that feeds the tensor core is a serial chain per block, and each in turn was the kernel's period until it
-// was split or shortened (measured with per-role cycle stamps): descriptors built per MMA in a one-lane branch (70
-// cycles per MMA; now two adds in warp-uniform code), one loader polling two rings (1000 cycles per unit; now two
-// loader warps with blocking waits and one barrier round per block), both operands in shared memory (the tensor
-// core's operand reads; now A in tensor memory), every producer warp on every block (1300 cycles; now alternate blocks).
+// CTA tile 128 rows x 64 tokens, one CTA per SM, or 256 rows x 128 tokens by a pair of CTAs (cta_group::2: each has 128 rows of the
+// codes in its tensor memory and 64 tokens' activations in its shared memory, and every MMA reads both CTAs' activations).  K is
+// stepped one weight block at a time = 16 MMAs (M 128 per CTA, N the tile's tokens, K 16): two K halves of 64 values x {H, L} x four
+// K = 16 steps, all into one accumulator (4 in flight at 64 tokens, 2 at 128).
+//   epilogue   TN / 8 warps: per block two tcgen05.ld of 16 columns, acc += dw * D (one row x 32 tokens per thread)
+//   producers  thread (row p, K half g): 64 two-bit codes -> 64 fp16, written to tensor memory; two sets of eight warps on alternate
+//              blocks at 64 tokens, one set at 128
+//   issuer     one warp, of a pair: the first CTA's
+//   loaders    one warp each (tiled TMA copies): weight pieces of 8 blocks x 128 rows; a block's activations, two boxes of 64 values x
+//              tokens x {H, L}, landing swizzled as the MMA reads them
+// Block n of a CTA's walk lives in slot n % 4 of both rings.  One barrier per slot says that codes and activations are there (an arrival per
+// producer warp, the loader's and its bytes), one that the block is multiplied: codes, activations and accumulator are handed
+// on by the same commit.
 #pragma once
 
 #include "gemm_tc.cuh"
 
 namespace b200 {
 
-constexpr int T16_M = 128;
-// Operands move in units of one K half of a weight block (64 values).  The codes (A) never touch shared memory: the
-// producers write the fp16 values straight into TENSOR memory (tcgen05.st, lane = weight row, 32 columns per unit) and
-// the MMA takes A from there -- with both operands in shared memory the tensor core's operand reads alone (6 KB per
-// 128 x 64 x 16 MMA, 96 KB per block) ate 3/4 of the shared-memory bandwidth of the block's whole time budget.  The
-// activations (B: the H and L planes of the tile's tokens) land in a shared-memory ring by TMA, asked for as far ahead
-// as the ring allows: the boxes come from L2 and take ~1000-1500 cycles.
-constexpr int T16_NA = 8;                                  // A ring: half-block units in tensor memory
-constexpr int T16_A_COL0 = 256, T16_A_UNIT_COLS = 32;      // tensor memory: accumulators in columns 0..255, then 8 A units x 32
+constexpr int T16_M = 128;                                 // weight rows of a CTA's tile
+// The codes (A) never touch shared memory: the producers write the fp16 values straight into TENSOR memory (tcgen05.st, lane =
+// weight row, 64 columns per block) and the MMA takes A from there -- with both operands in shared memory the tensor core's
+// operand reads alone (6 KB per 128 x 64 x 16 MMA, 96 KB per block) ate 3/4 of the shared-memory bandwidth of the block's whole
+// time budget.  The activations (B: the H and L planes of the tile's tokens) land in a shared-memory ring by TMA, asked for as far
+// ahead as the ring allows: the boxes come from L2 and take ~1000-1500 cycles.
+constexpr int T16_RING = 4;                                // blocks in flight: slots of the code ring and of the activation ring
+constexpr int T16_A_COL0 = 256, T16_A_COLS = 64;           // tensor memory: accumulators in columns 0..255, then 4 blocks of codes x 64
+constexpr int T16_SLOT_BYTES = 64 * 512;                   // activations of a block: 2 K halves x {H, L} x 64 tokens x 128 bytes
 constexpr int T16_WBUFS = 2;
-constexpr int T16_DWRING = 8;                              // weight scales of the last 8 blocks (epilogue lags the producers)
+constexpr int T16_DWRING = 8;                              // weight scales of the last 8 blocks (the epilogue lags the producers)
 constexpr int T16_ISSUERS = 2;                             // issuing warps: warp k takes the blocks n with n % 2 == k
-// The token width of a tile is a template parameter: 128 tokens per tile halve the code expansion per output (the
-// kernel's busiest part) and are used for large batches; 64 keep small batches from padding.
-template <int TN>
+// TN: the most tokens of a tile; CTAS: CTAs that multiply one tile together.
+template <int TN, int CTAS>
 struct T16C {
-    static constexpr int N = TN;
     static constexpr int ACC = 256 / TN;                                    // accumulators in flight (TN columns each)
     static constexpr int PART_FLOATS = T16_M * TN;                          // a CTA's slot for its part of a tile
     static constexpr int EPI_WARPS = TN / 8;                                // 4 lane quarters x (TN / 32) column groups of 32 tokens
     static constexpr int PROD_SETS = TN == 64 ? 2 : 1;                      // sets of producer warps on alternate blocks
     static constexpr int PROD_WARPS = 8 * PROD_SETS;                        // 4 row quarters x 2 K halves per set
-    static constexpr int EPI_THREADS = EPI_WARPS * 32, PROD_THREADS = PROD_WARPS * 32;
-    static constexpr int THREADS = EPI_THREADS + PROD_THREADS + 32 * (T16_ISSUERS + 2);      // + two loader warps
-    static constexpr int BUNIT = TN * 256;                                  // B bytes of one K half: {H, L} x TN tokens x 128 bytes
-    // A slot of the B ring (128 KB in all) is a K half of a block at 128 tokens, where a block would be half of the ring (512 tokens
-    // 217 -> 210 us), and a whole block at 64 (halves: 37 tokens 56 -> 58 us).
-    static constexpr int SLOT_HALVES = TN == 128 ? 1 : 2;
-    static constexpr int NB = (128 * 1024) / (SLOT_HALVES * BUNIT);
-    static constexpr int SMEM_BYTES = 2048 + NB * SLOT_HALVES * BUNIT + T16_DWRING * T16_M * 4 + T16_WBUFS * TC_WRAW_BYTES;
-    // instruction descriptor: D = fp32, A and B fp16, both K-major, N = TN, M = 128
-    static constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(T16_M >> 4) << 24);
+    static constexpr int THREADS = 32 * (EPI_WARPS + PROD_WARPS + T16_ISSUERS + 2);      // + weight loader, activation loader
+    static constexpr int CHUNK = TN == 64 ? 16 : 8;                         // tokens that an epilogue warp turns round at once
+    static constexpr int TURN_FLOATS = 32 * (CHUNK + 1);
+    static constexpr int SMEM_BYTES = 2048 + T16_RING * T16_SLOT_BYTES + T16_DWRING * T16_M * 4 + T16_WBUFS * TC_WRAW_BYTES + EPI_WARPS * TURN_FLOATS * 4;
+    static_assert(TN / CTAS == 64, "a CTA's slot holds 64 tokens");
+};
+// Instruction descriptor: D = fp32, A and B fp16, both K-major; n tokens, 128 rows per CTA.
+constexpr uint32_t t16_idesc(int n, int ctas) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(T16_M * ctas >> 4) << 24); }
+
+struct T16Params {
+    int n_out, nblocks, n_tok;
+    int tile_n;                      // tokens of a tile: a multiple of 16 per CTA, at most TN
+    int tiles_tok, n_tiles;          // token tiles per row tile, tiles in all (token tile runs fastest)
+    int stream_k;                    // 1: contiguous ranges of (tile, block) iterations; 0: whole tiles, round-robin
+    uint32_t idesc;
+    long long per_worker;            // n_tiles * nblocks = per_worker * workers + rest
+    int rest;
 };
 
+// The worker's (a CTA's or a pair's) next piece of work: blocks [kb0, kb1) of `tile`.  Every role walks the same sequence.
+__device__ __forceinline__ long long t16_first(const T16Params &P, int worker, int workers) {
+    return worker * P.per_worker + (long long)((uint32_t)(worker * P.rest) / (uint32_t)workers);
+}
+struct T16Walk {
+    long long left;
+    int tile, kb, step;
+    __device__ __forceinline__ void start(const T16Params &P, int worker, int workers) {
+        step = workers;
+        if (P.stream_k) {
+            const long long it = t16_first(P, worker, workers);
+            left = t16_first(P, worker + 1, workers) - it;
+            tile = it >> 32 ? (int)(it / P.nblocks) : (int)((uint32_t)it / (uint32_t)P.nblocks);
+            kb = (int)(it - (long long)tile * P.nblocks);
+        } else {
+            tile = worker - workers;
+            kb = 0;
+        }
+    }
+    __device__ __forceinline__ bool next(const T16Params &P, int &t, int &kb0, int &kb1) {
+        if (P.stream_k) {
+            if (left <= 0) return false;
+            t = tile++;
+            kb0 = kb;
+            kb1 = (int)min((long long)P.nblocks, kb + left);
+            left -= kb1 - kb;
+            kb = 0;
+            return true;
+        }
+        tile += step;
+        if (tile >= P.n_tiles) return false;
+        t = tile;
+        kb0 = 0;
+        kb1 = P.nblocks;
+        return true;
+    }
+};
 
 // The descriptors' upper words are the same for every operand of this kernel (128-byte swizzle, 1024 bytes between
 // 8-row groups); only the 14-bit address field of the lower word moves.  The issuing thread runs alone, one dependent
@@ -79,18 +117,97 @@ struct T16C {
 // 64-bit descriptors from an address cost ~75 cycles per MMA, 16 times per block).
 constexpr uint32_t T16_DESC_HI = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t tc16_desc_lo(uint32_t smem_addr) { return ((smem_addr >> 4) & 0x3FFFu) | (1u << 16); }
-template <bool ACC>
+template <bool ACC, int CTAS = 1>
 __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc) {
+    if (CTAS == 1)
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            ".reg .b64 db;\n\t"
+            "mov.b64 db, {%2, %4};\n\t"
+            "setp.ne.b32 p, %5, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t"
+            "}\n"
+            ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(T16_DESC_HI), "n"(ACC ? 1 : 0)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            ".reg .b64 db;\n\t"
+            "mov.b64 db, {%2, %4};\n\t"
+            "setp.ne.b32 p, %5, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], db, %3, p;\n\t"
+            "}\n"
+            ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(T16_DESC_HI), "n"(ACC ? 1 : 0)
+            : "memory");
+}
+// All of this thread's MMAs so far arrive on `bar`, of a pair: on both CTAs' barrier at this place.
+template <int CTAS>
+__device__ __forceinline__ void tc16_commit(uint32_t bar) {
+    if (CTAS == 1)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
+                     : "memory");
+}
+// The first CTA of the cluster's shared-memory address for this CTA's `addr`.
+__device__ __forceinline__ uint32_t cluster_first(uint32_t addr) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+// An arrival at a barrier of the pair's first CTA.  What it announces to the tensor core is ordered by the tcgen05 fence in front of it, so
+// it needs no release at cluster scope (which costs 1200 cycles here: 2400 per block of 128 tokens instead of 1250).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Bounded wait in the unit's own blocking form (no time-out operand: with one the compiler makes a loop of a few dozen instructions
+// of it), then as mbar_wait_bounded.  A barrier that has completed costs the waiting warp a third of mbar_wait_hot's instructions.
+__device__ __forceinline__ bool mbar_wait_try(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
     asm volatile(
         "{\n\t"
         ".reg .pred p;\n\t"
-        ".reg .b64 db;\n\t"
-        "mov.b64 db, {%2, %4};\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, {%6, %6, %6, %6}, p;\n\t"
-        "}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(T16_DESC_HI), "n"(ACC ? 1 : 0), "r"(0u)
+        ".reg .u32 n;\n\t"
+        "mov.u32 n, 4096;\n\t"
+        "TRY_LOOP:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra TRY_DONE;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "setp.ne.u32 p, n, 0;\n\t"
+        "@p bra TRY_LOOP;\n\t"
+        "TRY_DONE:\n\t"
+        "mov.u32 %0, n;\n\t"
+        "}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
+    return ok != 0 || mbar_wait_bounded(bar, parity, 32, 128);
+}
+// Both of two barriers: their latencies lie beside each other.
+__device__ __forceinline__ bool mbar_wait_both(uint64_t *bar0, uint32_t parity0, uint64_t *bar1, uint32_t parity1) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .u32 n;\n\t"
+        "mov.u32 n, 4096;\n\t"
+        "BOTH_LOOP:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+        "and.pred p, p, q;\n\t"
+        "@p bra BOTH_DONE;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "setp.ne.u32 p, n, 0;\n\t"
+        "@p bra BOTH_LOOP;\n\t"
+        "BOTH_DONE:\n\t"
+        "mov.u32 %0, n;\n\t"
+        "}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar0)), "r"(parity0), "r"(smem_u32(bar1)), "r"(parity1)
+        : "memory");
+    return ok != 0 || (mbar_wait_bounded(bar0, parity0, 32, 128) && mbar_wait_bounded(bar1, parity1, 32, 128));
 }
 __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&v)[16]) {
     asm volatile(
@@ -115,6 +232,12 @@ __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sy
 __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+                 : "memory");
+}
+// The same for a CTA of a pair: the bytes are counted on `bar`, an address in the cluster's window.
+__device__ __forceinline__ void tma_load_3d_pair(void *dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
                  : "memory");
 }
 __device__ __forceinline__ bool elect_one() {
@@ -191,7 +314,7 @@ __global__ void __launch_bounds__(T16_SPLIT_THREADS) tc16_split_kernel(const uin
             uint32_t h[4], l[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                constexpr unsigned char PERM[16] = {0, 8, 1, 9, 4, 12, 5, 13, 2, 10, 3, 11, 6, 14, 7, 15};
+                constexpr unsigned char PERM[16] = {0, 2, 4, 6, 8, 10, 12, 14, 1, 3, 5, 7, 9, 11, 13, 15};
                 const int j0 = 16 * (q >> 1) + PERM[8 * (q & 1) + 2 * e], j1 = 16 * (q >> 1) + PERM[8 * (q & 1) + 2 * e + 1];
                 const int a0 = (int)ab[j0], a1 = (int)ab[j1];
                 const float v0 = __fmul_rn(ds, (float)a0), v1 = __fmul_rn(ds, (float)a1);      // exact: 11 x 7 bits
@@ -206,205 +329,261 @@ __global__ void __launch_bounds__(T16_SPLIT_THREADS) tc16_split_kernel(const uin
     }
 }
 
-// 16 two-bit codes of one word -> 16 fp16 (-1, 0, 1, 2) in eight words.  The four fp16 patterns 0xBC00, 0x0000, 0x3C00,
-// 0x4000 have a zero low byte, so the high bytes are looked up four at a time by a byte permute whose selector nibbles
-// ARE the codes (w & 0x3333 leaves a code in every nibble), and a second permute spreads them over two words.  19
-// integer instructions per word: the expansion runs on the half-rate integer pipe, which this kernel keeps busiest.
+// 16 two-bit codes of one word -> 16 fp16 (-1, 0, 1, 2) in eight words.  A code in bits p, p + 1 (p = 0, 2 .. 8) of a halfword that
+// carries the exponent of 1024 is the fp16 number 1024 + 2^p code, so one three-input logic instruction makes two values and one
+// packed multiply-add takes them to code - 1, exactly: 1024 2^-p + 1 has 11 bits.  9 instructions per word on the half-rate integer
+// pipe, which this kernel kept busiest, and 8 on the multiply-add pipe (byte permutes whose selectors are the codes: 19 on the integer pipe).
 // Order of the 16 values (the split kernel writes the activations in the same order): code (byte b, field k)
 // of the word pairs with activation byte 4 k + b of the word's 16 (src/pq2_0.h:120-125, 158-166);
-//   o[0..1] = (b0k0 b0k2 b1k0 b1k2)   o[2..3] = (b0k1 b0k3 b1k1 b1k3)   o[4..5], o[6..7]: the same for bytes 2, 3.
+//   o[0..3] = (b0k0 b2k0) (b0k1 b2k1) (b0k2 b2k2) (b0k3 b2k3)   o[4..7]: the same for bytes 1 and 3.
+template <int P>
+__device__ __forceinline__ uint32_t tc16_pair(uint32_t w) {
+    const uint32_t v = (w & (0x00030003u << P)) | 0x64006400u;
+    const __half2 mul = __half2half2(__ushort_as_half((unsigned short)((15 - P) << 10)));               // 2^-P
+    const __half2 sub = __half2half2(__float2half_rn(-(1024.0f / (float)(1 << P) + 1.0f)));
+    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&v), mul, sub);
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
 __device__ __forceinline__ void tc16_expand(uint32_t w, uint32_t *o) {
-    constexpr uint32_t TB = 0x403C00BCu;
-    const uint32_t wh = w >> 16;
-    const uint32_t s0 = w & 0x3333u, s1 = (w >> 2) & 0x3333u, s2 = wh & 0x3333u, s3 = (wh >> 2) & 0x3333u;
-    const uint32_t h0 = __byte_perm(TB, 0u, s0), h1 = __byte_perm(TB, 0u, s1), h2 = __byte_perm(TB, 0u, s2), h3 = __byte_perm(TB, 0u, s3);
-    o[0] = __byte_perm(h0, 0u, 0x1404u);
-    o[1] = __byte_perm(h0, 0u, 0x3424u);
-    o[2] = __byte_perm(h1, 0u, 0x1404u);
-    o[3] = __byte_perm(h1, 0u, 0x3424u);
-    o[4] = __byte_perm(h2, 0u, 0x1404u);
-    o[5] = __byte_perm(h2, 0u, 0x3424u);
-    o[6] = __byte_perm(h3, 0u, 0x1404u);
-    o[7] = __byte_perm(h3, 0u, 0x3424u);
+    const uint32_t w8 = w >> 8;
+    o[0] = tc16_pair<0>(w);
+    o[1] = tc16_pair<2>(w);
+    o[2] = tc16_pair<4>(w);
+    o[3] = tc16_pair<6>(w);
+    o[4] = tc16_pair<8>(w);
+    o[5] = tc16_pair<2>(w8);
+    o[6] = tc16_pair<4>(w8);
+    o[7] = tc16_pair<6>(w8);
+}
+// acc += dw * v, each rounded once: two multiply-adds per instruction.
+__device__ __forceinline__ void tc16_fold(float *acc, const int (&v)[16], float dw) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 2)
+        asm("{\n\t"
+            ".reg .b64 x, y, z;\n\t"
+            "mov.b64 x, {%2, %3};\n\t"
+            "mov.b64 y, {%4, %4};\n\t"
+            "mov.b64 z, {%0, %1};\n\t"
+            "fma.rn.f32x2 z, x, y, z;\n\t"
+            "mov.b64 {%0, %1}, z;\n\t"
+            "}"
+            : "+f"(acc[i]), "+f"(acc[i + 1]) : "r"(v[i]), "r"(v[i + 1]), "f"(dw));
 }
 struct Tc16Maps {
     CUtensorMap w;        // PQ2_0 matrix as [n_out][row words], box 68 x 128
-    CUtensorMap x;        // fp16 planes as [2][n_tok][n_in], box 64 values x TN tokens x 2 planes, 128-byte swizzle
+    CUtensorMap x;        // fp16 planes as [2][n_tok][n_in], box 64 values x a CTA's tokens of a tile x 2 planes, 128-byte swizzle
 };
 
-template <int TN>
-__global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *Y, const TcParams P, const float *__restrict__ tokscale, float *parts,
-                                                                         unsigned int *flags, const __grid_constant__ Tc16Maps maps) {
-    using C = T16C<TN>;
-    constexpr int T16_N = TN, T16_ACC = C::ACC, T16_NB = C::NB, T16_BUNIT = C::BUNIT, T16_EPI_WARPS = C::EPI_WARPS,
-                  T16_PROD_WARPS = C::PROD_WARPS, T16_PROD_SETS = C::PROD_SETS, T16_EPI_THREADS = C::EPI_THREADS,
-                  T16_PROD_THREADS = C::PROD_THREADS, T16_EPI_TOKS = 32, T16_PART_FLOATS = C::PART_FLOATS, T16_SLOT = C::SLOT_HALVES;
+template <int TN, int CTAS>
+__global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(float *Y, const T16Params P, const float *__restrict__ tokscale,
+                                                                               float *parts, unsigned int *flags, const __grid_constant__ Tc16Maps maps) {
+    using C = T16C<TN, CTAS>;
+    constexpr int EPI_WARPS = C::EPI_WARPS, PROD_WARPS = C::PROD_WARPS, SETS = C::PROD_SETS, ACC = C::ACC, COLS = 32;
     extern __shared__ __align__(128) uint8_t smem[];
-    // unit u = 2 * block + K half lives in slot u % NA of the code ring and slot (u / SLOT_HALVES) % NB of the activation ring
-    uint64_t *afull = reinterpret_cast<uint64_t *>(smem);              // [NA] code producers -> issuer
-    uint64_t *afree = afull + T16_NA;                                   // [NA] tensor core -> code producers
-    uint64_t *bfull = afree + T16_NA;                                   // [NB] loader (bytes landed) -> issuer
-    uint64_t *bfree = bfull + T16_NB;                                   // [NB] tensor core -> loader
-    uint64_t *mma_done = bfree + T16_NB;                                // [4] tensor core -> epilogue
-    uint64_t *tmem_empty = mma_done + T16_ACC;                          // [4] epilogue -> issuer
-    uint64_t *wfull = tmem_empty + T16_ACC;                             // [2] loader -> producers
-    uint64_t *wfree = wfull + T16_WBUFS;                                // [2] producers -> loader
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(wfree + T16_WBUFS);
-    uint8_t *stages = smem + 1024 + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
-    uint8_t *bring = stages;
-    float *dwring = reinterpret_cast<float *>(bring + T16_NB * T16_SLOT * T16_BUNIT);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem);               // [4] producers and activation loader -> issuer (of a pair: the first CTA's is used)
+    uint64_t *done = full + T16_RING;                                   // [4] tensor core -> producers, activation loader, epilogue
+    uint64_t *acc_free = done + T16_RING;                               // [ACC] epilogue -> issuer (the first CTA's)
+    uint64_t *wfull = acc_free + ACC;                                   // [2] weight loader -> producers
+    uint64_t *wfree = wfull + T16_WBUFS;                                // [2] producers -> weight loader
+    uint64_t *dwfull = wfree + T16_WBUFS;                               // [8] of a pair: producers -> epilogue, a block's scales are in the ring
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(dwfull + T16_DWRING);
+    uint8_t *bring = smem + 1024 + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
+    float *dwring = reinterpret_cast<float *>(bring + T16_RING * T16_SLOT_BYTES);
     uint8_t *wraw = reinterpret_cast<uint8_t *>(dwring + T16_DWRING * T16_M);
+    float *turn = reinterpret_cast<float *>(wraw + T16_WBUFS * TC_WRAW_BYTES);
 
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nblocks = P.nblocks, n_tok = P.n_tok, n_out = P.n_out;
+    const int rank = CTAS == 1 ? 0 : (int)(blockIdx.x & 1), worker = (int)blockIdx.x / CTAS, workers = (int)gridDim.x / CTAS;
+    const int epi_warps = min(EPI_WARPS, 4 * ((P.tile_n + COLS - 1) / COLS));        // those that have tokens
+    constexpr int ISSUER = EPI_WARPS + PROD_WARPS, LOADER = ISSUER + T16_ISSUERS;
+    T16Walk walk;
+    walk.start(P, worker, workers);
+    int tile, kb0, kb1;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < T16_NA; ++s) { mbar_init(&afull[s], T16_PROD_THREADS / (2 * T16_PROD_SETS)); mbar_init(&afree[s], 1); }
-        for (int s = 0; s < T16_NB; ++s) { mbar_init(&bfull[s], 1); mbar_init(&bfree[s], 1); }
-        for (int s = 0; s < T16_ACC; ++s) { mbar_init(&mma_done[s], 1); mbar_init(&tmem_empty[s], T16_EPI_WARPS); }
-        for (int s = 0; s < T16_WBUFS; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wfree[s], T16_PROD_THREADS); }
+        for (int s = 0; s < T16_RING; ++s) { mbar_init(&full[s], 8 * CTAS + 1); mbar_init(&done[s], 1); }
+        for (int s = 0; s < ACC; ++s) mbar_init(&acc_free[s], CTAS * epi_warps);
+        for (int s = 0; s < T16_DWRING; ++s) mbar_init(&dwfull[s], 4);
         mbar_fence_init();
     }
-    constexpr int ISSUER = T16_EPI_WARPS + T16_PROD_WARPS, LOADER = ISSUER + T16_ISSUERS;
     if (threadIdx.x == LOADER * 32) {
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.w) : "memory");
+        // the first piece of weights, which comes from memory, is asked for before anything else is set up
+        for (int s = 0; s < T16_WBUFS; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wfree[s], PROD_WARPS); }
+        mbar_fence_init();
+        T16Walk first = walk;
+        if (first.next(P, tile, kb0, kb1)) {
+            mbar_expect_tx(&wfull[0], (uint32_t)TC_WRAW_BYTES);
+            tma_load_2d(wraw, &maps.w, (kb0 >> 3) * 68, (tile / P.tiles_tok) * (T16_M * CTAS) + T16_M * rank, &wfull[0]);
+        }
         asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x) : "memory");
     }
     if (wid == ISSUER) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (CTAS == 1) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
-    __syncthreads();
+    if (CTAS == 1) __syncthreads();
+    else asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    TcWalk walk;
-    walk.start(P);
-    int tile, kb0, kb1;
 
-    if (wid < T16_EPI_WARPS) {
+    if (wid < EPI_WARPS) {
         // ---------------- epilogue: one weight row per thread, 32 tokens ----------------
         const int q = wid & 3, cg = wid >> 2;
         const int row_l = 32 * q + lane;
-        bool ok = true;
+        const bool second = COLS * cg + 16 < P.tile_n;
+        const uint32_t tlane = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(COLS * cg);
+        const uint32_t acc_free0 = CTAS == 1 ? 0u : cluster_first(smem_u32(acc_free));
+        bool ok = wid < epi_warps;
         int n = 0;
         while (ok && walk.next(P, tile, kb0, kb1)) {
             const int rt = tile / P.tiles_tok, tt = tile - rt * P.tiles_tok;
-            const int row = rt * T16_M + row_l, tokb = tt * T16_N + T16_EPI_TOKS * cg;
-            float acc[T16_EPI_TOKS];
+            const int row0 = rt * (T16_M * CTAS) + T16_M * rank + 32 * q, col0 = COLS * cg, tokb = tt * P.tile_n + col0;
+            float acc[COLS];
 #pragma unroll
-            for (int j = 0; j < T16_EPI_TOKS; ++j) acc[j] = 0.0f;
-            const uint32_t tlane = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(T16_EPI_TOKS * cg);
-            for (int kb = kb0; kb < kb1; ++kb, ++n) {
-                const int t = n & (T16_ACC - 1);
-                if (!mbar_wait_bounded(&mma_done[t], (uint32_t)((n / T16_ACC) & 1), 20, 80)) { ok = false; break; }
+            for (int j = 0; j < COLS; ++j) acc[j] = 0.0f;
+            // At 64 tokens two blocks at a time (four accumulators): the waits of both lie beside each other.
+            constexpr int STEP = ACC == 4 ? 2 : 1;
+            for (int kb = kb0; kb < kb1; kb += STEP, n += STEP) {
+                const bool pair = STEP == 2 && kb + 1 < kb1;
+                const int n1 = pair ? n + 1 : n;
+                if (CTAS != 1 && !mbar_wait_try(&dwfull[n & (T16_DWRING - 1)], (uint32_t)((n / T16_DWRING) & 1))) { ok = false; break; }
+                if (STEP == 2 ? !mbar_wait_both(&done[n & (T16_RING - 1)], (uint32_t)((n / T16_RING) & 1), &done[n1 & (T16_RING - 1)], (uint32_t)((n1 / T16_RING) & 1))
+                              : !mbar_wait_try(&done[n & (T16_RING - 1)], (uint32_t)((n / T16_RING) & 1))) { ok = false; break; }
                 tc_fence_after();
-                int v[16];
-                tc_ld16(tlane + (uint32_t)(t * T16_N), v);
-                const float dw = dwring[(n & (T16_DWRING - 1)) * T16_M + row_l];
-                tc_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 16; ++j) acc[j] = __fmaf_rn(dw, __int_as_float(v[j]), acc[j]);
-                tc_ld16(tlane + (uint32_t)(t * T16_N + 16), v);
-                tc_ld_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&tmem_empty[t]);          // the block's sums are in registers
-#pragma unroll
-                for (int j = 0; j < 16; ++j) acc[16 + j] = __fmaf_rn(dw, __int_as_float(v[j]), acc[16 + j]);
+                for (int i = 0; i < STEP; ++i) {
+                    if (i && !pair) break;
+                    const int t = (n + i) & (ACC - 1);
+                    // Of a pair, whose two accumulators are what the tensor core waits for, all 32 columns are read before anything is done with
+                    // them (256 tokens of 6144 -> 5120: 57.4 -> 56.4 us); with tiles of 64 tokens that is slower.
+                    int v[16], v2[16];
+                    tc_ld16(tlane + (uint32_t)(t * TN), v);
+                    if (CTAS != 1) tc_ld16(tlane + (uint32_t)(t * TN + 16), v2);
+                    const float dw = dwring[((n + i) & (T16_DWRING - 1)) * T16_M + row_l];
+                    tc_ld_wait();
+                    if (CTAS == 1) {
+                        tc16_fold(acc, v, dw);
+                        if (second) {
+                            tc_ld16(tlane + (uint32_t)(t * TN + 16), v);
+                            tc_ld_wait();
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {                                     // the block's sums are in registers
+                        if (CTAS == 1) mbar_arrive(&acc_free[t]);
+                        else mbar_arrive_cluster(acc_free0 + 8u * (uint32_t)t);
+                    }
+                    if (CTAS != 1) {
+                        tc16_fold(acc, v, dw);
+                        tc16_fold(acc + 16, v2, dw);
+                    } else if (second) {
+                        tc16_fold(acc + 16, v, dw);
+                    }
+                }
             }
+            if (STEP == 2) n -= (kb1 - kb0) & 1;
             if (!ok) break;
-            // ---- the tile (or this CTA's part of it) is done: undo the token's power-of-two scale
+            // ---- the tile (or this CTA's part of it) is done
+            const int toks = min(min(COLS, P.tile_n - col0), n_tok - tokb);         // may be none
+            constexpr int CH = C::CHUNK;
+            const int rt0 = lane / CH, tk = lane % CH;
+            float scale[COLS / CH];
 #pragma unroll
-            for (int j = 0; j < T16_EPI_TOKS; ++j) acc[j] = __fmul_rn(acc[j], tokb + j < n_tok ? __ldg(tokscale + tokb + j) : 0.0f);
+            for (int c = 0; c < COLS / CH; ++c) scale[c] = c * CH + tk < toks ? __ldg(tokscale + tokb + c * CH + tk) : 0.0f;
             if (kb0 > 0) {
                 // A later part of a tile: left in this CTA's slot, one row per lane.  The CTA that has the tile's first blocks
                 // adds the parts.  (They were handed from CTA to CTA, each waiting for the one behind it: 37 tokens of
                 // 17408 -> 5120, four parts per tile, 69 us against 43 us.)
-                float *slot = parts + (size_t)blockIdx.x * T16_PART_FLOATS + (size_t)(T16_EPI_TOKS * cg) * T16_M + row_l;
+                float *slot = parts + (size_t)blockIdx.x * C::PART_FLOATS + (size_t)col0 * T16_M + row_l;
 #pragma unroll
-                for (int j = 0; j < T16_EPI_TOKS; ++j) slot[j * T16_M] = acc[j];
+                for (int j = 0; j < COLS; ++j)
+                    if (j < toks) slot[j * T16_M] = acc[j];
                 __threadfence();
-                asm volatile("bar.sync 1, %0;" ::"n"(T16_EPI_THREADS) : "memory");
+                asm volatile("bar.sync 1, %0;" ::"r"(32 * epi_warps) : "memory");
                 if (threadIdx.x == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + blockIdx.x), "r"(1u) : "memory");
                 continue;
             }
-            float *yrow = Y + (size_t)row * n_tok + tokb;
-            const bool vec = (n_tok & 3) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15u) == 0;
             if (kb1 < nblocks) {
-                // the CTAs behind this one have the tile's other parts: added from the last to the first, then to this one
+                // the workers behind this one have the tile's other parts: added in their order
                 const long long tile_end = (long long)(tile + 1) * nblocks;
-                int last = (int)blockIdx.x + 1;
-                while (last + 1 < (int)gridDim.x && P.total_it * (long long)(last + 1) / (long long)gridDim.x < tile_end) ++last;
-                if (threadIdx.x == 0) {
-                    for (int c = (int)blockIdx.x + 1; c <= last; ++c) {
-                        const unsigned int *f = flags + c;
-                        uint32_t ns = 32;
+                int last = worker + 1;
+                while (last + 1 < workers && t16_first(P, last + 1, workers) < tile_end) ++last;
+                if (wid == 0) {
+                    for (int c = worker + 1 + lane; c <= last; c += 32) {
+                        unsigned int *f = flags + CTAS * c + rank;
                         bool there = false;
-                        for (uint32_t k = 0; k < (1u << 22); ++k) {
+                        for (uint32_t k = 0; k < (1u << 23); ++k) {
                             unsigned int fv;
                             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(fv) : "l"(f) : "memory");
                             if (fv != 0u) { there = true; break; }
-                            __nanosleep(ns);
-                            ns = min(ns * 2, 256u);
+                            __nanosleep(32);
                         }
                         if (!there) atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);
                         *const_cast<volatile unsigned int *>(f) = 0u;     // lowered by its only reader: the next launch on this scratch finds zeros
                     }
                 }
-                asm volatile("bar.sync 1, %0;" ::"n"(T16_EPI_THREADS) : "memory");
-                const float *slots = parts + (size_t)(T16_EPI_TOKS * cg) * T16_M + row_l;
+                asm volatile("bar.sync 1, %0;" ::"r"(32 * epi_warps) : "memory");
+                const float *slots = parts + (size_t)rank * C::PART_FLOATS + (size_t)col0 * T16_M + row_l;
+                for (int c = worker + 1; c <= last; ++c) {
+                    const float *slot = slots + (size_t)(CTAS * c) * C::PART_FLOATS;
 #pragma unroll
-                for (int j0 = 0; j0 < T16_EPI_TOKS; j0 += 8) {
-                    float t[8];
+                    for (int j0 = 0; j0 < COLS; j0 += 8) {
+                        float t[8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) t[j] = __ldcg(slots + (size_t)last * T16_PART_FLOATS + (j0 + j) * T16_M);
-                    for (int c = last - 1; c > (int)blockIdx.x; --c)
+                        for (int j = 0; j < 8; ++j) t[j] = j0 + j < toks ? __ldcg(slot + (j0 + j) * T16_M) : 0.0f;
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) t[j] = __fadd_rn(__ldcg(slots + (size_t)c * T16_PART_FLOATS + (j0 + j) * T16_M), t[j]);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[j0 + j] = __fadd_rn(acc[j0 + j], t[j]);
+                        for (int j = 0; j < 8; ++j) acc[j0 + j] = __fadd_rn(acc[j0 + j], t[j]);
+                    }
                 }
             }
-            if (row < n_out) {
-                if (vec) {
+            // A row's tokens lie side by side in Y: turned round through shared memory, a store writes 32 (or 64) bytes of each of four (two)
+            // rows.  (A row per lane, 16 bytes of 32 rows per store: 7000 cycles per tile of 128 tokens, in which both accumulators waited; turned
+            // round by shuffles: 3400, most of it code that had to be fetched.)  The token's power-of-two scale is undone here.
+            float *box = turn + wid * C::TURN_FLOATS;
 #pragma unroll
-                    for (int j = 0; j < T16_EPI_TOKS; j += 4)
-                        if (tokb + j < n_tok) *reinterpret_cast<float4 *>(yrow + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-                } else {
+            for (int c = 0; c < COLS; c += CH) {
+                if (c >= toks) break;
+                const bool have = c + tk < toks;
+                __syncwarp();
 #pragma unroll
-                    for (int j = 0; j < T16_EPI_TOKS; ++j)
-                        if (tokb + j < n_tok) yrow[j] = acc[j];
-                }
+                for (int j = 0; j < CH; ++j) box[lane * (CH + 1) + j] = acc[c + j];
+                __syncwarp();
+                float *y = Y + (size_t)(row0 + rt0) * n_tok + tokb + c + tk;
+                const float *b = box + rt0 * (CH + 1) + tk;
+#pragma unroll 4
+                for (int r = 0; r < CH; ++r)
+                    if (have && row0 + rt0 + r * (32 / CH) < n_out) y[(size_t)(r * (32 / CH)) * n_tok] = __fmul_rn(b[r * (32 / CH) * (CH + 1)], scale[c / CH]);
             }
         }
     } else if (wid < ISSUER) {
-        // ---------------- code producers: thread (row p, K half g) of every second block: 64 codes -> 64 fp16 ----------------
-        const int pi = threadIdx.x - T16_EPI_THREADS;
+        // ---------------- code producers: thread (row p, K half g), with two sets every second block ----------------
         // A warp reaches only the 32 tensor-memory lanes of its own quarter (warp index mod 4): producer warp pw takes
-        // rows 32 (pw % 4) + lane, K half (pw / 4) % 2, and the blocks n with n % 2 == pw / 8.  Two sets on alternate
-        // blocks because a warp's own chain per block -- raw loads, expansion, tcgen05.st, wait::st, fence, arrive -- is
-        // ~1300 cycles long and was the kernel's period when every warp took every block.  The store of one block is
-        // completed (wait::st, fence, arrive) only after the NEXT own block has been loaded and expanded.
-        const int pw = pi >> 5, p = 32 * (pw & 3) + lane, g = (pw >> 2) & 1, set = pw >> 3;    // set: 0 when there is one set
-        const uint32_t a_lane = tmem_base + ((uint32_t)(32 * (pw & 3)) << 16) + (uint32_t)T16_A_COL0;
+        // rows 32 (pw % 4) + lane, K half (pw / 4) % 2, and with two sets the blocks n with n % 2 == pw / 8.
+        const int pw = wid - EPI_WARPS, p = 32 * (pw & 3) + lane, g = (pw >> 2) & 1, set = pw >> 3;
+        const uint32_t a_lane = tmem_base + ((uint32_t)(32 * (pw & 3)) << 16) + (uint32_t)(T16_A_COL0 + 32 * g);
+        const uint32_t full0 = CTAS == 1 ? 0u : cluster_first(smem_u32(full));
         bool ok = true;
-        int n = 0, oct = 0, pending = -1;           // pending: slot whose store is in flight
+        int n = 0, oct = 0;
         while (ok && walk.next(P, tile, kb0, kb1)) {
-            for (int kb = kb0; kb < kb1; ++kb, ++n) {
-                if (kb == kb0 || (kb & 7) == 0) {
-                    if (!mbar_wait_bounded(&wfull[oct % T16_WBUFS], (uint32_t)((oct / T16_WBUFS) & 1))) { ok = false; break; }
-                    ++oct;
-                }
-                const int wbuf = (oct - 1) % T16_WBUFS;
-                if ((n & (T16_PROD_SETS - 1)) == set) {
-                    const int u = 2 * n + g, sa = u % T16_NA;
+            for (int kb = kb0; ok && kb < kb1; ++oct) {
+                const int wbuf = oct % T16_WBUFS, end = min(kb1, (kb | 7) + 1);
+                if (!mbar_wait_try(&wfull[wbuf], (uint32_t)((oct / T16_WBUFS) & 1))) { ok = false; break; }
+                const uint8_t *rowp = wraw + (size_t)wbuf * TC_WRAW_BYTES + (size_t)p * 272;
+                for (; kb < end; ++kb, ++n) {
+                    if (SETS > 1 && (n & (SETS - 1)) != set) continue;
+                    const int s = n & (T16_RING - 1);
                     // The half's four code words sit at byte 34 j + 2 + 16 g of the row's 272-byte piece, 2-byte aligned:
                     // five aligned words and funnel shifts by 0 or 16 bits.  (Rows are 68 words apart: a warp's loads
                     // spread over eight banks, four passes each.)
                     const uint32_t off = (uint32_t)(kb & 7) * 34u + 2u + 16u * (uint32_t)g;
-                    const uint8_t *rowp = wraw + (size_t)wbuf * TC_WRAW_BYTES + (size_t)p * 272;
                     const uint32_t *wa = reinterpret_cast<const uint32_t *>(rowp + (off & ~3u));
                     const uint32_t x0 = wa[0], x1 = wa[1], x2 = wa[2], x3 = wa[3], x4 = wa[4], sh = (off & 2u) * 8u;
                     const uint32_t dbits = g == 0 ? (uint32_t)*reinterpret_cast<const unsigned short *>(rowp + (kb & 7) * 34) : 0u;
@@ -413,112 +592,108 @@ __global__ void __launch_bounds__(T16C<TN>::THREADS, 1) gemm_tc16_kernel(float *
                     tc16_expand(__funnelshift_r(x1, x2, sh), pc + 8);
                     tc16_expand(__funnelshift_r(x2, x3, sh), pc + 16);
                     tc16_expand(__funnelshift_r(x3, x4, sh), pc + 24);
-                    if (pending >= 0) {
-                        tc_st_wait();
-                        tc_fence_before();
-                        mbar_arrive(&afull[pending]);
-                    }
-                    if (!mbar_wait_bounded(&afree[sa], (uint32_t)(((u / T16_NA) & 1) ^ 1), 20, 80)) { ok = false; pending = -1; break; }
+                    if (!mbar_wait_try(&done[s], (uint32_t)(((n / T16_RING) & 1) ^ 1))) { ok = false; break; }
                     tc_fence_after();
                     if (g == 0) dwring[(n & (T16_DWRING - 1)) * T16_M + p] = f16_bits_to_f32(dbits);
-                    tc_st32(a_lane + (uint32_t)(sa * T16_A_UNIT_COLS), pc);     // 64 fp16 = 32 columns of this thread's lane
-                    pending = sa;
+                    tc_st32(a_lane + (uint32_t)(s * T16_A_COLS), pc);     // 64 fp16 = 32 columns of this thread's lane
+                    tc_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (CTAS == 1) mbar_arrive(&full[s]);
+                        else mbar_arrive_cluster(full0 + 8u * (uint32_t)s);
+                        if (CTAS != 1 && g == 0) mbar_arrive(&dwfull[n & (T16_DWRING - 1)]);
+                    }
                 }
-                // every producer passes every block: at a piece's last block it has read all it needs of the piece
-                if ((kb & 7) == 7 || kb == kb1 - 1) mbar_arrive(&wfree[wbuf]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&wfree[wbuf]);
             }
-        }
-        if (pending >= 0) {
-            tc_st_wait();
-            tc_fence_before();
-            mbar_arrive(&afull[pending]);
         }
     } else if (wid == LOADER) {
         // ---------------- weight loader: a piece (8 blocks x 128 rows, one tiled copy) as soon as its buffer is free ----------------
         int oct = 0;
         bool ok = true;
         while (ok && walk.next(P, tile, kb0, kb1)) {
+            const int row = (tile / P.tiles_tok) * (T16_M * CTAS) + T16_M * rank;
             for (int kb = kb0; kb < kb1 && ok; kb = min(kb1, (kb | 7) + 1), ++oct) {
                 const int wb = oct % T16_WBUFS;
-                if (!mbar_wait_bounded(&wfree[wb], (uint32_t)(((oct / T16_WBUFS) & 1) ^ 1))) { ok = false; break; }
+                if (oct == 0) continue;                              // asked for at the start
+                if (!mbar_wait_try(&wfree[wb], (uint32_t)(((oct / T16_WBUFS) & 1) ^ 1))) { ok = false; break; }
                 if (elect_one()) {
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     mbar_expect_tx(&wfull[wb], (uint32_t)TC_WRAW_BYTES);
-                    tma_load_2d(wraw + (size_t)wb * TC_WRAW_BYTES, &maps.w, (kb >> 3) * 68, (tile / P.tiles_tok) * T16_M, &wfull[wb]);
+                    tma_load_2d(wraw + (size_t)wb * TC_WRAW_BYTES, &maps.w, (kb >> 3) * 68, row, &wfull[wb]);
                 }
                 __syncwarp();
             }
         }
     } else if (wid == LOADER + 1) {
-        // ---------------- activation loader: boxes of 64 values x TN tokens x {H, L}, a slot as soon as it is free ----------------
+        // ---------------- activation loader: a block's two boxes as soon as its slot is free ----------------
+        const int bn = P.tile_n / CTAS;
+        const uint32_t full0 = CTAS == 1 ? 0u : cluster_first(smem_u32(full));
         int n = 0;
         bool ok = true;
         while (ok && walk.next(P, tile, kb0, kb1)) {
-            const int tt = tile % P.tiles_tok;
+            const int tok = (tile % P.tiles_tok) * P.tile_n + bn * rank;
             for (int kb = kb0; kb < kb1; ++kb, ++n) {
+                const int s = n & (T16_RING - 1);
+                if (!mbar_wait_try(&done[s], (uint32_t)(((n / T16_RING) & 1) ^ 1))) { ok = false; break; }
+                if (elect_one()) {
+                    uint8_t *b = bring + (size_t)s * T16_SLOT_BYTES;
+                    if (rank == 0) mbar_expect_tx(&full[s], (uint32_t)(CTAS * bn * 512));          // both CTAs' bytes are counted on the first's barrier
 #pragma unroll
-                for (int g = 0; g < 2; g += T16_SLOT) {
-                    const int w = (2 * n + g) / T16_SLOT, sb = w % T16_NB;
-                    if (!mbar_wait_bounded(&bfree[sb], (uint32_t)(((w / T16_NB) & 1) ^ 1), 20, 80)) { ok = false; break; }
-                    if (elect_one()) {
-                        uint8_t *b = bring + (size_t)sb * (T16_SLOT * T16_BUNIT);
-                        mbar_expect_tx(&bfull[sb], (uint32_t)(T16_SLOT * T16_BUNIT));
-#pragma unroll
-                        for (int h = 0; h < T16_SLOT; ++h) tma_load_3d(b + h * T16_BUNIT, &maps.x, kb * 128 + 64 * (g + h), tt * T16_N, 0, &bfull[sb]);
+                    for (int h = 0; h < 2; ++h) {
+                        if (CTAS == 1) tma_load_3d(b + h * bn * 256, &maps.x, kb * 128 + 64 * h, tok, 0, &full[s]);
+                        else tma_load_3d_pair(b + h * bn * 256, &maps.x, kb * 128 + 64 * h, tok, 0, full0 + 8u * (uint32_t)s);
                     }
-                    __syncwarp();
                 }
-                if (!ok) break;
+                __syncwarp();
             }
         }
-    } else {
-        // ---------------- issuer: sixteen K = 16 MMAs per weight block, one accumulator ----------------
+    } else if (rank == 0) {
+        // ---------------- issuers: sixteen K = 16 MMAs per weight block, one accumulator ----------------
         // The whole warp walks the loop and waits; one elected lane issues.  Kept warp-uniform on purpose: the MMA takes
         // its operands from uniform registers, and inside a one-lane branch every operand had to be moved there first
-        // (~70 cycles per MMA, measured).  Two such warps take alternate blocks: one warp's waits, fences and commits
-        // are a serial chain of ~2000 cycles per block, more than the block's MMAs take; blocks use different
+        // (~70 cycles per MMA, measured).  A wait costs the warp 190 cycles even where its barrier has completed, and the queue behind it
+        // holds a few MMAs only, so two warps take alternate blocks: one's waits lie beside the other's MMAs (alone with its waits and
+        // commits, 16 MMAs of 64 tokens per block: 57 cycles each from one warp, 33 from two).  Blocks use different
         // accumulators, so their MMAs may interleave, and a commit covers the issuing thread's own MMAs.
+        const uint32_t b_lo0 = tc16_desc_lo(smem_u32(bring)), half = (uint32_t)(P.tile_n / CTAS * 256) >> 4, plane = half >> 1;
+        const uint32_t done0 = smem_u32(done), idesc = P.idesc;
         const int me = wid - ISSUER;
         bool ok = true;
         int n = 0;
         while (ok && walk.next(P, tile, kb0, kb1)) {
-            for (int kb = kb0; kb < kb1; ++kb, ++n) {
-                if ((n & (T16_ISSUERS - 1)) != me) continue;
-                const int t = n & (T16_ACC - 1);
-                const uint32_t d = tmem_base + (uint32_t)(t * T16_N);
-                // K half 0, then K half 1: each half's 8 MMAs (H and L planes x four K steps) go out as soon as its two
-                // units are there, and the units are handed back as soon as the MMAs have read them.
+            const int skip = (n ^ me) & (T16_ISSUERS - 1);
+            int m0 = n + skip;
+            n += kb1 - kb0;
+            for (int kb = kb0 + skip; kb < kb1; kb += T16_ISSUERS, m0 += T16_ISSUERS) {
+                const int s = m0 & (T16_RING - 1), t = m0 & (ACC - 1);
+                if (!mbar_wait_both(&full[s], (uint32_t)((m0 / T16_RING) & 1), &acc_free[t], (uint32_t)(((m0 / ACC) & 1) ^ 1))) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t d = tmem_base + (uint32_t)(t * TN), a = tmem_base + (uint32_t)(T16_A_COL0 + s * T16_A_COLS);
+                const uint32_t b = b_lo0 + (uint32_t)(s * (T16_SLOT_BYTES >> 4));
+                if (elect_one()) {
 #pragma unroll
-                for (int g = 0; g < 2; ++g) {
-                    const int u = 2 * n + g, sa = u % T16_NA, w = u / T16_SLOT, sb = w % T16_NB;
-                    if (!mbar_wait_hot(&afull[sa], (uint32_t)((u / T16_NA) & 1))) { ok = false; break; }
-                    if (g % T16_SLOT == 0 && !mbar_wait_hot(&bfull[sb], (uint32_t)((w / T16_NB) & 1))) { ok = false; break; }
-                    if (g == 0 && !mbar_wait_hot(&tmem_empty[t], (uint32_t)(((n / T16_ACC) & 1) ^ 1))) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t a_t = tmem_base + (uint32_t)(T16_A_COL0 + sa * T16_A_UNIT_COLS);
-                    const uint32_t b_lo = tc16_desc_lo(smem_u32(bring + (size_t)(T16_SLOT * sb + g % T16_SLOT) * T16_BUNIT));
-                    if (elect_one()) {
-#pragma unroll
-                        for (int m = 0; m < 8; ++m) {
-                            const int pl = m >> 2, i = m & 3;
-                            if (g == 0 && m == 0) tc_mma_f16_ts<false>(d, a_t, b_lo, C::IDESC);        // K step i: 16 fp16 = 8 columns of A
-                            else tc_mma_f16_ts<true>(d, a_t + (uint32_t)(8 * i), b_lo + (uint32_t)(pl * ((T16_N * 128) >> 4) + 2 * i), C::IDESC);
-                        }
-                        tc_commit(&afree[sa]);
-                        if (g % T16_SLOT == T16_SLOT - 1) tc_commit(&bfree[sb]);
-                        if (g == 1) tc_commit(&mma_done[t]);
+                    for (int m = 0; m < 16; ++m) {
+                        const uint32_t g = m >> 3, pl = (m >> 2) & 1, i = m & 3;              // K half, plane, K step: 16 fp16 = 8 columns of A
+                        if (m == 0) tc_mma_f16_ts<false, CTAS>(d, a, b, idesc);
+                        else tc_mma_f16_ts<true, CTAS>(d, a + 32u * g + 8u * i, b + g * half + pl * plane + 2u * i, idesc);
                     }
-                    __syncwarp();
+                    tc16_commit<CTAS>(done0 + 8u * (uint32_t)s);
                 }
-                if (!ok) break;
+                __syncwarp();
             }
         }
     }
     tc_fence_before();
-    __syncthreads();
+    // of a pair: neither CTA leaves while the other's MMAs or arrivals may still reach it
+    if (CTAS == 1) __syncthreads();
+    else asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
     if (wid == ISSUER) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+        if (CTAS == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
 }
 
