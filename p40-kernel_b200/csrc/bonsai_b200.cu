@@ -959,7 +959,7 @@ static bool encode_w_map(CUtensorMap *map, const void *W, int64_t n_out, int64_t
 
 // Scratch of the fp16 tensor-core mat-mul: a flag and a slot per CTA for its part of a tile, the activations as two fp16 planes, a
 // scale per token.  A call that gets none takes the integer kernel, which needs no scratch.
-static constexpr size_t T16_FLAGS_BYTES = (size_t)TC_MAX_CTAS * sizeof(unsigned int);
+static constexpr size_t T16_FLAGS_BYTES = (size_t)TC_MAX_CTAS * T16_PART_FLAGS * sizeof(unsigned int);
 static StreamScratch g_gemm_scratch(T16_FLAGS_BYTES, false);
 
 // Scratch of the prompt attention: k and v as tile images, 2 KB per position and kv head, what k and v take themselves.  Prompts of one

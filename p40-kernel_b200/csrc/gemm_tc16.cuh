@@ -20,9 +20,9 @@
 // stepped one weight block at a time = 16 MMAs (M 128 per CTA, N the tile's tokens, K 16): two K halves of 64 values x {H, L} x four
 // K = 16 steps, all into one accumulator (4 in flight at 64 tokens, 2 at 128).
 //   epilogue   TN / 8 warps: per block two tcgen05.ld of 16 columns, acc += dw * D (one row x 32 tokens per thread)
-//   producers  thread (row p, K half g): 64 two-bit codes -> 64 fp16, written to tensor memory; two sets of eight warps on alternate
-//              blocks at 64 tokens, one set at 128
-//   issuer     one warp, of a pair: the first CTA's
+//   producers  sets of four warps, thread = row: 128 two-bit codes -> 128 fp16, written to tensor memory; four sets in turn at 64 tokens,
+//              each on a slot of its own, two at 128
+//   issuers    two warps on alternate blocks, of a pair: the first CTA's
 //   loaders    one warp each (tiled TMA copies): weight pieces of 8 blocks x 128 rows; a block's activations, two boxes of 64 values x
 //              tokens x {H, L}, landing swizzled as the MMA reads them
 // Block n of a CTA's walk lives in slot n % 4 of both rings.  One barrier per slot says that codes and activations are there (an arrival per
@@ -46,18 +46,18 @@ constexpr int T16_SLOT_BYTES = 64 * 512;                   // activations of a b
 constexpr int T16_WBUFS = 2;
 constexpr int T16_DWRING = 8;                              // weight scales of the last 8 blocks (the epilogue lags the producers)
 constexpr int T16_ISSUERS = 2;                             // issuing warps: warp k takes the blocks n with n % 2 == k
+constexpr int T16_TURN_STRIDE = 36, T16_TURN_FLOATS = 8 * T16_TURN_STRIDE;      // an epilogue warp turns 8 rows x 32 tokens round at once
+constexpr int T16_PART_FLAGS = 16;                         // flags of a CTA: one per epilogue warp
 // TN: the most tokens of a tile; CTAS: CTAs that multiply one tile together.
 template <int TN, int CTAS>
 struct T16C {
     static constexpr int ACC = 256 / TN;                                    // accumulators in flight (TN columns each)
     static constexpr int PART_FLOATS = T16_M * TN;                          // a CTA's slot for its part of a tile
     static constexpr int EPI_WARPS = TN / 8;                                // 4 lane quarters x (TN / 32) column groups of 32 tokens
-    static constexpr int PROD_SETS = TN == 64 ? 2 : 1;                      // sets of producer warps on alternate blocks
-    static constexpr int PROD_WARPS = 8 * PROD_SETS;                        // 4 row quarters x 2 K halves per set
+    static constexpr int PROD_SETS = TN == 64 ? 4 : 2;                      // sets of producer warps, each on every fourth (second) block
+    static constexpr int PROD_WARPS = 4 * PROD_SETS;                        // 4 row quarters per set
     static constexpr int THREADS = 32 * (EPI_WARPS + PROD_WARPS + T16_ISSUERS + 2);      // + weight loader, activation loader
-    static constexpr int CHUNK = TN == 64 ? 16 : 8;                         // tokens that an epilogue warp turns round at once
-    static constexpr int TURN_FLOATS = 32 * (CHUNK + 1);
-    static constexpr int SMEM_BYTES = 2048 + T16_RING * T16_SLOT_BYTES + T16_DWRING * T16_M * 4 + T16_WBUFS * TC_WRAW_BYTES + EPI_WARPS * TURN_FLOATS * 4;
+    static constexpr int SMEM_BYTES = 2048 + T16_RING * T16_SLOT_BYTES + T16_DWRING * T16_M * 4 + T16_WBUFS * TC_WRAW_BYTES + EPI_WARPS * T16_TURN_FLOATS * 4;
     static_assert(TN / CTAS == 64, "a CTA's slot holds 64 tokens");
 };
 // Instruction descriptor: D = fp32, A and B fp16, both K-major; n tokens, 128 rows per CTA.
@@ -369,6 +369,25 @@ __device__ __forceinline__ void tc16_fold(float *acc, const int (&v)[16], float 
             "}"
             : "+f"(acc[i]), "+f"(acc[i + 1]) : "r"(v[i]), "r"(v[i + 1]), "f"(dw));
 }
+// acc += dw0 * v0 + dw1 * v1, two of them per instruction: the two products are added first, so that a sum over n blocks is a chain of n / 2
+// additions to a large number.
+__device__ __forceinline__ void tc16_fold2(float *acc, const int (&v0)[8], float dw0, const int (&v1)[8], float dw1) {
+#pragma unroll
+    for (int i = 0; i < 8; i += 2)
+        asm("{\n\t"
+            ".reg .b64 x, y, z, t;\n\t"
+            "mov.b64 x, {%2, %3};\n\t"
+            "mov.b64 y, {%6, %6};\n\t"
+            "mul.rn.f32x2 t, x, y;\n\t"
+            "mov.b64 x, {%4, %5};\n\t"
+            "mov.b64 y, {%7, %7};\n\t"
+            "fma.rn.f32x2 t, x, y, t;\n\t"
+            "mov.b64 z, {%0, %1};\n\t"
+            "add.rn.f32x2 z, z, t;\n\t"
+            "mov.b64 {%0, %1}, z;\n\t"
+            "}"
+            : "+f"(acc[i]), "+f"(acc[i + 1]) : "r"(v0[i]), "r"(v0[i + 1]), "r"(v1[i]), "r"(v1[i + 1]), "f"(dw0), "f"(dw1));
+}
 struct Tc16Maps {
     CUtensorMap w;        // PQ2_0 matrix as [n_out][row words], box 68 x 128
     CUtensorMap x;        // fp16 planes as [2][n_tok][n_in], box 64 values x a CTA's tokens of a tile x 2 planes, 128-byte swizzle
@@ -402,7 +421,7 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
     int tile, kb0, kb1;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < T16_RING; ++s) { mbar_init(&full[s], 8 * CTAS + 1); mbar_init(&done[s], 1); }
+        for (int s = 0; s < T16_RING; ++s) { mbar_init(&full[s], 4 * CTAS + 1); mbar_init(&done[s], 1); }
         for (int s = 0; s < ACC; ++s) mbar_init(&acc_free[s], CTAS * epi_warps);
         for (int s = 0; s < T16_DWRING; ++s) mbar_init(&dwfull[s], 4);
         mbar_fence_init();
@@ -448,67 +467,83 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
             float acc[COLS];
 #pragma unroll
             for (int j = 0; j < COLS; ++j) acc[j] = 0.0f;
-            // At 64 tokens two blocks at a time (four accumulators): the waits of both lie beside each other.
-            constexpr int STEP = ACC == 4 ? 2 : 1;
-            for (int kb = kb0; kb < kb1; kb += STEP, n += STEP) {
-                const bool pair = STEP == 2 && kb + 1 < kb1;
-                const int n1 = pair ? n + 1 : n;
+            // At 64 tokens two blocks at a time (four accumulators): the waits of both lie beside each other, and the chain of rounded additions is
+            // half as long (error against 64 bits 1.14e-7 -> 9.0e-8 at 5120, 1.44e-7 -> 1.13e-7 at 17408).
+            for (int kb = kb0; kb < kb1; ++kb, ++n) {
+                const int t = n & (ACC - 1);
                 if (CTAS != 1 && !mbar_wait_try(&dwfull[n & (T16_DWRING - 1)], (uint32_t)((n / T16_DWRING) & 1))) { ok = false; break; }
-                if (STEP == 2 ? !mbar_wait_both(&done[n & (T16_RING - 1)], (uint32_t)((n / T16_RING) & 1), &done[n1 & (T16_RING - 1)], (uint32_t)((n1 / T16_RING) & 1))
-                              : !mbar_wait_try(&done[n & (T16_RING - 1)], (uint32_t)((n / T16_RING) & 1))) { ok = false; break; }
-                tc_fence_after();
+                if (ACC == 4 && kb + 1 < kb1) {
+                    const int n1 = n + 1, t1 = n1 & (ACC - 1);
+                    if (!mbar_wait_both(&done[n & (T16_RING - 1)], (uint32_t)((n / T16_RING) & 1), &done[n1 & (T16_RING - 1)], (uint32_t)((n1 / T16_RING) & 1))) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const float dw = dwring[(n & (T16_DWRING - 1)) * T16_M + row_l], dw1 = dwring[(n1 & (T16_DWRING - 1)) * T16_M + row_l];
 #pragma unroll
-                for (int i = 0; i < STEP; ++i) {
-                    if (i && !pair) break;
-                    const int t = (n + i) & (ACC - 1);
-                    // Of a pair, whose two accumulators are what the tensor core waits for, all 32 columns are read before anything is done with
-                    // them (256 tokens of 6144 -> 5120: 57.4 -> 56.4 us); with tiles of 64 tokens that is slower.
-                    int v[16], v2[16];
-                    tc_ld16(tlane + (uint32_t)(t * TN), v);
-                    if (CTAS != 1) tc_ld16(tlane + (uint32_t)(t * TN + 16), v2);
-                    const float dw = dwring[((n + i) & (T16_DWRING - 1)) * T16_M + row_l];
-                    tc_ld_wait();
-                    if (CTAS == 1) {
-                        tc16_fold(acc, v, dw);
-                        if (second) {
-                            tc_ld16(tlane + (uint32_t)(t * TN + 16), v);
-                            tc_ld_wait();
-                        }
+                    for (int h = 0; h < COLS; h += 8) {
+                        if (h == 16 && !second) break;
+                        int v[8], v1[8];
+                        tc_ld8(tlane + (uint32_t)(t * TN + h), v);
+                        tc_ld8(tlane + (uint32_t)(t1 * TN + h), v1);
+                        tc_ld_wait();
+                        tc16_fold2(acc + h, v, dw, v1, dw1);
                     }
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) {                                     // the block's sums are in registers
-                        if (CTAS == 1) mbar_arrive(&acc_free[t]);
-                        else mbar_arrive_cluster(acc_free0 + 8u * (uint32_t)t);
+                    if (lane == 0) {                                     // the blocks' sums are in registers
+                        mbar_arrive(&acc_free[t]);
+                        mbar_arrive(&acc_free[t1]);
                     }
-                    if (CTAS != 1) {
-                        tc16_fold(acc, v, dw);
-                        tc16_fold(acc + 16, v2, dw);
-                    } else if (second) {
-                        tc16_fold(acc + 16, v, dw);
+                    ++kb, ++n;
+                    continue;
+                }
+                if (!mbar_wait_try(&done[n & (T16_RING - 1)], (uint32_t)((n / T16_RING) & 1))) { ok = false; break; }
+                tc_fence_after();
+                const float dw = dwring[(n & (T16_DWRING - 1)) * T16_M + row_l];
+                if (CTAS == 1) {
+#pragma unroll
+                    for (int h = 0; h < COLS; h += 16) {
+                        if (h == 16 && !second) break;
+                        int v[16];
+                        tc_ld16(tlane + (uint32_t)(t * TN + h), v);
+                        tc_ld_wait();
+                        tc16_fold(acc + h, v, dw);
                     }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_free[t]);
+                } else {
+                    // Of a pair, whose two accumulators are what the tensor core waits for, all 32 columns are read before anything is done
+                    // with them (256 tokens of 6144 -> 5120: 57.4 -> 56.4 us).
+                    int v[16], v2[16];
+                    tc_ld16(tlane + (uint32_t)(t * TN), v);
+                    tc_ld16(tlane + (uint32_t)(t * TN + 16), v2);
+                    tc_ld_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(acc_free0 + 8u * (uint32_t)t);
+                    tc16_fold(acc, v, dw);
+                    tc16_fold(acc + 16, v2, dw);
                 }
             }
-            if (STEP == 2) n -= (kb1 - kb0) & 1;
             if (!ok) break;
             // ---- the tile (or this CTA's part of it) is done
             const int toks = min(min(COLS, P.tile_n - col0), n_tok - tokb);         // may be none
-            constexpr int CH = C::CHUNK;
-            const int rt0 = lane / CH, tk = lane % CH;
-            float scale[COLS / CH];
-#pragma unroll
-            for (int c = 0; c < COLS / CH; ++c) scale[c] = c * CH + tk < toks ? __ldg(tokscale + tokb + c * CH + tk) : 0.0f;
+            const float scale = lane < toks ? __ldg(tokscale + tokb + lane) : 0.0f;
             if (kb0 > 0) {
-                // A later part of a tile: left in this CTA's slot, one row per lane.  The CTA that has the tile's first blocks
-                // adds the parts.  (They were handed from CTA to CTA, each waiting for the one behind it: 37 tokens of
-                // 17408 -> 5120, four parts per tile, 69 us against 43 us.)
+                // A later part of a tile: left in this CTA's slot, four tokens of a row per lane and store.  The CTA that has the tile's
+                // first blocks adds the parts, each of its warps those of its counterparts as soon as they are there.  (They were handed from CTA
+                // to CTA, each waiting for the one behind it: 37 tokens of 17408 -> 5120, four parts per tile, 69 us against 43 us.)
                 float *slot = parts + (size_t)blockIdx.x * C::PART_FLOATS + (size_t)col0 * T16_M + row_l;
 #pragma unroll
-                for (int j = 0; j < COLS; ++j)
-                    if (j < toks) slot[j * T16_M] = acc[j];
-                __threadfence();
-                asm volatile("bar.sync 1, %0;" ::"r"(32 * epi_warps) : "memory");
-                if (threadIdx.x == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + blockIdx.x), "r"(1u) : "memory");
+                for (int j0 = 0; j0 < COLS; j0 += 8) {
+                    if (j0 >= toks) break;
+#pragma unroll
+                    for (int j = j0; j < j0 + 8; ++j) slot[j * T16_M] = acc[j];
+                }
+                __syncwarp();
+                if (lane == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + blockIdx.x * T16_PART_FLAGS + wid), "r"(1u) : "memory");
                 continue;
             }
             if (kb1 < nblocks) {
@@ -516,59 +551,70 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
                 const long long tile_end = (long long)(tile + 1) * nblocks;
                 int last = worker + 1;
                 while (last + 1 < workers && t16_first(P, last + 1, workers) < tile_end) ++last;
-                if (wid == 0) {
-                    for (int c = worker + 1 + lane; c <= last; c += 32) {
-                        unsigned int *f = flags + CTAS * c + rank;
-                        bool there = false;
-                        for (uint32_t k = 0; k < (1u << 23); ++k) {
-                            unsigned int fv;
-                            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(fv) : "l"(f) : "memory");
-                            if (fv != 0u) { there = true; break; }
-                            __nanosleep(32);
-                        }
-                        if (!there) atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);
-                        *const_cast<volatile unsigned int *>(f) = 0u;     // lowered by its only reader: the next launch on this scratch finds zeros
+                for (int c = worker + 1 + lane; c <= last; c += 32) {
+                    unsigned int *f = flags + (CTAS * c + rank) * T16_PART_FLAGS + wid;
+                    bool there = false;
+                    for (uint32_t k = 0; k < (1u << 23); ++k) {
+                        unsigned int fv;
+                        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(fv) : "l"(f) : "memory");
+                        if (fv != 0u) { there = true; break; }
+                        __nanosleep(32);
                     }
+                    if (!there) atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);
+                    *const_cast<volatile unsigned int *>(f) = 0u;     // lowered by its only reader: the next launch on this scratch finds zeros
                 }
-                asm volatile("bar.sync 1, %0;" ::"r"(32 * epi_warps) : "memory");
+                __syncwarp();
                 const float *slots = parts + (size_t)rank * C::PART_FLOATS + (size_t)col0 * T16_M + row_l;
                 for (int c = worker + 1; c <= last; ++c) {
                     const float *slot = slots + (size_t)(CTAS * c) * C::PART_FLOATS;
 #pragma unroll
-                    for (int j0 = 0; j0 < COLS; j0 += 8) {
-                        float t[8];
+                    for (int j0 = 0; j0 < COLS; j0 += 32) {
+                        if (j0 >= toks) break;
+                        float t[32];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) t[j] = j0 + j < toks ? __ldcg(slot + (j0 + j) * T16_M) : 0.0f;
+                        for (int j = 0; j < 32; ++j) t[j] = __ldcg(slot + (j0 + j) * T16_M);
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) acc[j0 + j] = __fadd_rn(acc[j0 + j], t[j]);
+                        for (int j = 0; j < 32; ++j) acc[j0 + j] = __fadd_rn(acc[j0 + j], t[j]);
                     }
                 }
             }
-            // A row's tokens lie side by side in Y: turned round through shared memory, a store writes 32 (or 64) bytes of each of four (two)
-            // rows.  (A row per lane, 16 bytes of 32 rows per store: 7000 cycles per tile of 128 tokens, in which both accumulators waited; turned
-            // round by shuffles: 3400, most of it code that had to be fetched.)  The token's power-of-two scale is undone here.
-            float *box = turn + wid * C::TURN_FLOATS;
-#pragma unroll
-            for (int c = 0; c < COLS; c += CH) {
-                if (c >= toks) break;
-                const bool have = c + tk < toks;
+            // A row's tokens lie side by side in Y: turned round through shared memory eight rows at a time, a store writes 128 bytes of one
+            // row.  (A row per lane, 16 bytes of 32 rows per store: 7000 cycles per tile of 128 tokens, in which both accumulators waited.)  The token's power-of-two scale is undone here.
+            float *box = turn + wid * T16_TURN_FLOATS;
+            float *y = Y + (size_t)row0 * n_tok + tokb + lane;
+#pragma unroll 1
+            for (int r0 = 0; r0 < 32; r0 += 8) {
                 __syncwarp();
+                if ((lane & 24) == r0) {
+                    float4 *b = reinterpret_cast<float4 *>(box + (lane & 7) * T16_TURN_STRIDE);
 #pragma unroll
-                for (int j = 0; j < CH; ++j) box[lane * (CH + 1) + j] = acc[c + j];
+                    for (int j = 0; j < COLS; j += 4) b[j / 4] = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+                }
                 __syncwarp();
-                float *y = Y + (size_t)(row0 + rt0) * n_tok + tokb + c + tk;
-                const float *b = box + rt0 * (CH + 1) + tk;
-#pragma unroll 4
-                for (int r = 0; r < CH; ++r)
-                    if (have && row0 + rt0 + r * (32 / CH) < n_out) y[(size_t)(r * (32 / CH)) * n_tok] = __fmul_rn(b[r * (32 / CH) * (CH + 1)], scale[c / CH]);
+                float v[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) v[r] = box[r * T16_TURN_STRIDE + lane];
+                if (lane < toks) {
+                    // (a condition for all eight: one per row cost a hundred cycles each)
+                    if (row0 + r0 + 8 <= n_out) {
+#pragma unroll
+                        for (int r = 0; r < 8; ++r) y[(size_t)r * n_tok] = __fmul_rn(v[r], scale);
+                    } else {
+#pragma unroll
+                        for (int r = 0; r < 8; ++r)
+                            if (row0 + r0 + r < n_out) y[(size_t)r * n_tok] = __fmul_rn(v[r], scale);
+                    }
+                }
+                y += (size_t)8 * n_tok;
             }
         }
     } else if (wid < ISSUER) {
-        // ---------------- code producers: thread (row p, K half g), with two sets every second block ----------------
-        // A warp reaches only the 32 tensor-memory lanes of its own quarter (warp index mod 4): producer warp pw takes
-        // rows 32 (pw % 4) + lane, K half (pw / 4) % 2, and with two sets the blocks n with n % 2 == pw / 8.
-        const int pw = wid - EPI_WARPS, p = 32 * (pw & 3) + lane, g = (pw >> 2) & 1, set = pw >> 3;
-        const uint32_t a_lane = tmem_base + ((uint32_t)(32 * (pw & 3)) << 16) + (uint32_t)(T16_A_COL0 + 32 * g);
+        // ---------------- code producers: thread = row, a set's every fourth (second) block ----------------
+        // A warp reaches only the 32 tensor-memory lanes of its own quarter (warp index mod 4).  A warp takes both K halves of a block, one
+        // after the other: its waits, addresses and arrivals are spent once per block (two sets of eight warps, a K half each: 5120 -> 17408
+        // at 64 tokens 36.4 -> 35.0 us).
+        const int pw = wid - EPI_WARPS, p = 32 * (pw & 3) + lane, set = pw >> 2;
+        const uint32_t a_lane = tmem_base + ((uint32_t)(32 * (pw & 3)) << 16) + (uint32_t)T16_A_COL0;
         const uint32_t full0 = CTAS == 1 ? 0u : cluster_first(smem_u32(full));
         bool ok = true;
         int n = 0, oct = 0;
@@ -580,29 +626,35 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
                 for (; kb < end; ++kb, ++n) {
                     if (SETS > 1 && (n & (SETS - 1)) != set) continue;
                     const int s = n & (T16_RING - 1);
-                    // The half's four code words sit at byte 34 j + 2 + 16 g of the row's 272-byte piece, 2-byte aligned:
-                    // five aligned words and funnel shifts by 0 or 16 bits.  (Rows are 68 words apart: a warp's loads
-                    // spread over eight banks, four passes each.)
-                    const uint32_t off = (uint32_t)(kb & 7) * 34u + 2u + 16u * (uint32_t)g;
+                    // The block's eight code words sit at byte 34 j + 2 of the row's 272-byte piece, 2-byte aligned: nine aligned words and
+                    // funnel shifts by 0 or 16 bits.  (Rows are 68 words apart: a warp's loads spread over eight banks, four passes each.)
+                    const uint32_t off = (uint32_t)(kb & 7) * 34u + 2u;
                     const uint32_t *wa = reinterpret_cast<const uint32_t *>(rowp + (off & ~3u));
-                    const uint32_t x0 = wa[0], x1 = wa[1], x2 = wa[2], x3 = wa[3], x4 = wa[4], sh = (off & 2u) * 8u;
-                    const uint32_t dbits = g == 0 ? (uint32_t)*reinterpret_cast<const unsigned short *>(rowp + (kb & 7) * 34) : 0u;
-                    uint32_t pc[32];
-                    tc16_expand(__funnelshift_r(x0, x1, sh), pc);
-                    tc16_expand(__funnelshift_r(x1, x2, sh), pc + 8);
-                    tc16_expand(__funnelshift_r(x2, x3, sh), pc + 16);
-                    tc16_expand(__funnelshift_r(x3, x4, sh), pc + 24);
-                    if (!mbar_wait_try(&done[s], (uint32_t)(((n / T16_RING) & 1) ^ 1))) { ok = false; break; }
-                    tc_fence_after();
-                    if (g == 0) dwring[(n & (T16_DWRING - 1)) * T16_M + p] = f16_bits_to_f32(dbits);
-                    tc_st32(a_lane + (uint32_t)(s * T16_A_COLS), pc);     // 64 fp16 = 32 columns of this thread's lane
+                    const uint32_t sh = (off & 2u) * 8u;
+                    const uint32_t dbits = (uint32_t)*reinterpret_cast<const unsigned short *>(rowp + (kb & 7) * 34);
+                    uint32_t x[9];
+#pragma unroll
+                    for (int i = 0; i < 9; ++i) x[i] = wa[i];
+#pragma unroll
+                    for (int g = 0; g < 2; ++g) {
+                        uint32_t pc[32];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) tc16_expand(__funnelshift_r(x[4 * g + i], x[4 * g + i + 1], sh), pc + 8 * i);
+                        if (g == 0) {
+                            if (!mbar_wait_try(&done[s], (uint32_t)(((n / T16_RING) & 1) ^ 1))) { ok = false; break; }
+                            tc_fence_after();
+                        }
+                        tc_st32(a_lane + (uint32_t)(s * T16_A_COLS + 32 * g), pc);     // 64 fp16 = 32 columns of this thread's lane
+                    }
+                    if (!ok) break;
+                    dwring[(n & (T16_DWRING - 1)) * T16_M + p] = f16_bits_to_f32(dbits);
                     tc_st_wait();
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
                         if (CTAS == 1) mbar_arrive(&full[s]);
                         else mbar_arrive_cluster(full0 + 8u * (uint32_t)s);
-                        if (CTAS != 1 && g == 0) mbar_arrive(&dwfull[n & (T16_DWRING - 1)]);
+                        if (CTAS != 1) mbar_arrive(&dwfull[n & (T16_DWRING - 1)]);
                     }
                 }
                 __syncwarp();
