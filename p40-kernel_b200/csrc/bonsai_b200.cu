@@ -1010,21 +1010,51 @@ static int tc16_pairs() {
     return std::max(resident, 0);
 }
 
+// How a mat-mul is divided over `workers` CTAs (or pairs of them), and about how long that takes.
+struct Tc16Plan {
+    int tile_n = 0, grid = 0, stream_k = 0;
+    long long tiles_tok = 0, tiles = 0;
+    double ns = 0;
+};
+template <int TN, int CTAS>
+static Tc16Plan plan_tc16(int64_t n_out, int64_t nblocks, int64_t n_tok, int workers) {
+    Tc16Plan p;
+    // As many token tiles as TN asks for, all of about the same width: the MMAs' time is the tokens' (37 tokens take 48 columns, not 64).
+    const long long step = 16 * CTAS;
+    p.tiles_tok = (n_tok + TN - 1) / TN;
+    p.tile_n = (int)(((n_tok + p.tiles_tok - 1) / p.tiles_tok + step - 1) / step * step);
+    p.tiles = (n_out + T16_M * CTAS - 1) / (T16_M * CTAS) * p.tiles_tok;
+    if (p.tiles > INT32_MAX) return p;
+    // Whole tiles in turn, or the blocks of all tiles in equal shares: at most four workers to a tile, at least 16 blocks each.  Measured at
+    // 33 - 192 tokens of 1024 -> 12288, 5120 -> 5120, 5120 -> 17408 and 17408 -> 5120: 5.5 us and 0.53 per block for a CTA, 8 us and 0.39 + 0.003 per token
+    // and block for a pair, 7 us for leaving, fetching and adding the parts of tiles that are shared.
+    const double start = CTAS == 1 ? 5500 : 8000, block = CTAS == 1 ? 530 : 390 + 3 * p.tile_n;
+    const long long total = p.tiles * nblocks;
+    p.grid = (int)std::min<long long>(p.tiles, workers);
+    p.ns = start + block * (double)((p.tiles + workers - 1) / workers * nblocks);
+    const long long sharing = p.tiles >= workers ? workers : std::min<long long>({total / 16, 4 * p.tiles, workers});
+    if (p.tiles % workers != 0 && sharing >= p.grid && sharing > 1) {
+        const double ns = start + block * (double)((total + sharing - 1) / sharing) + 7000;
+        if (ns < p.ns) p.grid = (int)sharing, p.stream_k = 1, p.ns = ns;
+    }
+    return p;
+}
+static int tc16_workers(int ctas) {
+    int dev = 0, sms = 0;
+    if (ctas != 1) return std::min(tc16_pairs(), (TC_MAX_CTAS - 1) / ctas);
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return std::min(sms, TC_MAX_CTAS - 1);
+}
+
 template <int TN, int CTAS>
 static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n_out, int64_t n_in, int64_t n_tok, cudaStream_t st) {
     const int64_t nblocks = n_in / 128;
     if (nblocks % 8 != 0 || !aligned16(W) || !aligned4(Xq) || n_tok > (1 << 28)) return -1;
-    int dev = 0, sms = 0, workers = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return (int)e;
-    workers = std::min(CTAS == 1 ? sms : tc16_pairs(), (TC_MAX_CTAS - 1) / CTAS);
+    const int workers = tc16_workers(CTAS), sms = tc16_workers(1);
     if (workers <= 0) return -1;
-    // As many token tiles as TN asks for, all of about the same width: the MMAs' time is the tokens' (37 tokens take 48 columns, not 64).
-    const long long tiles_tok = (n_tok + TN - 1) / TN, step = 16 * CTAS;
-    const int tile_n = (int)(((n_tok + tiles_tok - 1) / tiles_tok + step - 1) / step * step);
-    const long long tiles = (n_out + T16_M * CTAS - 1) / (T16_M * CTAS) * tiles_tok;
-    if (tiles > INT32_MAX) return -1;
+    const Tc16Plan plan = plan_tc16<TN, CTAS>(n_out, nblocks, n_tok, workers);
+    if (plan.tiles > INT32_MAX) return -1;
+    cudaError_t e;
     const size_t plane_bytes = (size_t)n_tok * (size_t)n_in * sizeof(__half);
     const StreamScratch::Lease lease = g_gemm_scratch.get(tc16_scratch_bytes(n_in, n_tok), st);      // held until both launches are enqueued
     uint8_t *ws = static_cast<uint8_t *>(lease.ptr);
@@ -1036,23 +1066,19 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     alignas(64) Tc16Maps maps;
     std::memset(&maps, 0, sizeof(maps));
     if (!encode_w_map(&maps.w, W, n_out, nblocks * W_BLOCK_BYTES)) return -1;
-    if (!tensor_map_planes(&maps.x, planes, (uint64_t)n_in, (uint64_t)n_tok, (uint32_t)(tile_n / CTAS))) return -1;
+    if (!tensor_map_planes(&maps.x, planes, (uint64_t)n_in, (uint64_t)n_tok, (uint32_t)(plan.tile_n / CTAS))) return -1;
     T16Params P{};
     P.n_out = (int)n_out;
     P.nblocks = (int)nblocks;
     P.n_tok = (int)n_tok;
-    P.tile_n = tile_n;
-    P.tiles_tok = (int)tiles_tok;
-    P.n_tiles = (int)tiles;
-    P.idesc = t16_idesc(tile_n, CTAS);
-    // Tiles for at most half of the workers (a short token batch over few rows): up to four share a tile's blocks, at least 16
-    // blocks each.
-    const long long total = tiles * nblocks;
-    int grid = (int)std::min<long long>(tiles, workers);
-    if (2 * tiles <= workers) grid = (int)std::max<long long>(grid, std::min<long long>({total / 16, 4 * tiles, workers}));
-    P.stream_k = (tiles % grid != 0 && (grid > tiles || total / grid >= nblocks)) ? 1 : 0;
-    P.per_worker = total / grid;
-    P.rest = (int)(total % grid);
+    P.tile_n = plan.tile_n;
+    P.tiles_tok = (int)plan.tiles_tok;
+    P.n_tiles = (int)plan.tiles;
+    P.idesc = t16_idesc(plan.tile_n, CTAS);
+    P.stream_k = plan.stream_k;
+    const int grid = plan.grid;
+    P.per_worker = plan.tiles * nblocks / grid;
+    P.rest = (int)(plan.tiles * nblocks % grid);
     const int n_chunks = (int)(n_in / 32);
     const uint32_t *x32 = static_cast<const uint32_t *>(Xq);
     // slices: whole passes of a block, as many as bring about two blocks per SM
@@ -1082,11 +1108,14 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     return (int)cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN, CTAS>, Y, P, (const float *)scale, parts, flags, maps);
 }
 }  // extern "C++"
-// Pairs of CTAs and tiles of 128 tokens from 96 tokens on (the code expansion is paid once per tile, and each CTA fetches half of the
-// activations), tiles of 64 below.
+// Tiles of up to 64 tokens by a CTA, or of up to 128 by a pair of CTAs (the code expansion is paid once per tile, and each CTA fetches half
+// of the activations): what the plans say takes less time.  (us, a CTA / a pair: 64 tokens of 5120 -> 17408 26.8 / 30.8, 65 44.5 / 33.7, 129
+// 61.7 / 59.6; of 5120 -> 5120, where pairs have too few tiles, 64 22.5 / 24.7, 128 25.3 / 29.0; 129 of 1024 -> 12288 20.6 / 22.9.)
 static int launch_gemm_tc16(const void *W, const void *Xq, float *Y, int64_t n_out, int64_t n_in, int64_t n_tok, cudaStream_t st) {
-    const int tile = g_opt_gemm_tile.load();
-    if (tile == 128 || (tile != 64 && n_tok >= 96)) {
+    const int tile = g_opt_gemm_tile.load(), ones = tc16_workers(1), pairs = n_tok > 64 || tile == 128 ? tc16_workers(2) : 0;
+    if (ones <= 0) return -1;
+    if (tile != 64 && pairs > 0 &&
+        (tile == 128 || plan_tc16<128, 2>(n_out, n_in / 128, n_tok, pairs).ns < plan_tc16<64, 1>(n_out, n_in / 128, n_tok, ones).ns)) {
         const int rc = launch_gemm_tc16_n<128, 2>(W, Xq, Y, n_out, n_in, n_tok, st);
         if (rc >= 0) return rc;
     }
