@@ -47,8 +47,9 @@ std::atomic<int> g_opt_gemv_variant{-1};
 std::atomic<int> g_opt_gemv_order{0};
 std::atomic<int> g_opt_fuse_linear{0};         // 1: bonsai_b200_linear runs as one kernel when it can (measured slower)
 std::atomic<int> g_opt_chain_threads{512};       // threads per CTA of the chain kernel: 512 (5 blocks per lane and task), 640 (4), 768 (3)
-std::atomic<int> g_opt_chain_spread_nb{40};      // dependent ops with at least this many blocks per row rotate their input
-                                                 // once for the grid instead of once per CTA; 0 = never
+// Dependent ops with at least this many blocks per row rotate their input once for the grid instead of once per CTA; 0 = never.  us per op of a list
+// n -> n, once per CTA / once for the grid: 1024 behind a norm 5.3 / 5.7, 2048 6.5 / 6.2 (plain 5.6 / 5.3), 3072 7.5 / 6.9, 5120 9.8 / 8.1.
+std::atomic<int> g_opt_chain_spread_nb{16};
 std::atomic<int> g_opt_chain_tile_kb{16};
 std::atomic<int> g_opt_kv_wide{1};                // decode attention: 0 = clusters of eight CTAs at every length
 std::atomic<int> g_opt_gemm_tile{0};              // fp16 tensor-core mat-mul: 0 by token count, 64 or 128 tokens per tile
@@ -573,8 +574,8 @@ int bonsai_b200_linear_static(const void *W, const float *x, const float *signs,
 // ---- a list of projections in one persistent launch ------------------------------------------------
 struct bonsai_b200_chain {
     ChainOp *d_ops = nullptr;
-    unsigned int *d_counter = nullptr;      // [0] arrivals of ops that others wait for, [1] rotated blocks in the image
-    uint8_t *d_image = nullptr;             // activation tables of a spread op, shared through L2
+    unsigned int *d_counter = nullptr;      // [0] arrivals of ops that others wait for
+    unsigned long long *d_image = nullptr;  // activation tables of a spread op, shared through L2 (one rank: behind the counters)
     bool tp = false;                        // several ranks: counters live in the caller's peer-mapped buffer, never reset
     ChainPeers peers{};
     int n_ops = 0, threads = 0, grid = 0, device = 0;
@@ -741,8 +742,7 @@ static int chain_create_impl(const bonsai_b200_op *ops, int64_t n_ops, int tp_ra
         last_user[buf] = (int)i;
         if (!same && !rotate) r.ready_parity = ready_uses[buf]++ & 1;
         if (rotate) any_rotate = true; else any_q8 = true;
-        // (an RMSNorm producer needs the whole vector in every CTA for its sum of squares: such an op rotates for itself)
-        if (rotate && depends && !same && !(r.flags & CHAIN_RMSNORM) && spread_nb > 0 && r.nb >= spread_nb && r.nb / 8 <= sms) {
+        if (rotate && depends && !same && spread_nb > 0 && r.nb >= spread_nb && r.nb / 8 <= sms) {
             r.flags |= CHAIN_SPREAD;
             spread_total += (unsigned)(r.nb / 8);
             r.spread_blocks = spread_total;
@@ -814,8 +814,15 @@ static int chain_create_impl(const bonsai_b200_op *ops, int64_t n_ops, int tp_ra
     if (e == cudaSuccess) e = cudaMalloc(&c->d_ops, sizeof(ChainOp) * (size_t)n_ops);
     if (e == cudaSuccess && tp) c->d_counter = c->peers.counter[tp_rank];
     c->counter_bytes = 256 + (any_rescale ? 4 * (size_t)n_ops : 0);        // counters, then the largest |y| of every op
-    if (e == cudaSuccess && !tp) e = cudaMalloc(&c->d_counter, c->counter_bytes);
-    if (e == cudaSuccess && any_spread) e = cudaMalloc(&c->d_image, (size_t)G.nb_max * 176);
+    c->counter_bytes = (size_t)round_up((int64_t)c->counter_bytes, 256);
+    const size_t image_bytes = any_spread ? (size_t)G.nb_max * CHAIN_IMAGE_WORDS * 8 : 0;
+    if (e == cudaSuccess && !tp) e = cudaMalloc(&c->d_counter, c->counter_bytes + image_bytes);
+    if (e == cudaSuccess && any_spread && tp) e = cudaMalloc(&c->d_image, image_bytes);
+    if (e == cudaSuccess && any_spread && tp && !zero_new_memory(c->d_image, image_bytes)) e = cudaErrorUnknown;      // no tag of any run
+    if (e == cudaSuccess && any_spread && !tp) {
+        c->d_image = reinterpret_cast<unsigned long long *>(reinterpret_cast<uint8_t *>(c->d_counter) + c->counter_bytes);
+        c->counter_bytes += image_bytes;
+    }
     if (e == cudaSuccess) e = cudaMemcpy(c->d_ops, rec.data(), sizeof(ChainOp) * (size_t)n_ops, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         bonsai_b200_chain_destroy(c);
@@ -840,7 +847,7 @@ int bonsai_b200_chain_run(bonsai_b200_chain *c, bonsai_stream stream) {
     if (!c || !c->d_ops) return 1;
     cudaStream_t st = as_stream(stream);
     cudaError_t e = cudaSuccess;
-    if (!c->tp) e = cudaMemsetAsync(c->d_counter, 0, c->counter_bytes > 256 ? c->counter_bytes : 2 * sizeof(unsigned int), st);
+    if (!c->tp) e = cudaMemsetAsync(c->d_counter, 0, c->counter_bytes > 256 ? c->counter_bytes : 2 * sizeof(unsigned int), st);      // and the image's tags
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)c->grid);
@@ -867,7 +874,7 @@ int bonsai_b200_chain_destroy(bonsai_b200_chain *c) {
     if (!c) return 0;
     cudaError_t e1 = c->d_ops ? cudaFree(c->d_ops) : cudaSuccess;
     cudaError_t e2 = (c->d_counter && !c->tp) ? cudaFree(c->d_counter) : cudaSuccess;
-    if (c->d_image) cudaFree(c->d_image);
+    if (c->d_image && c->tp) cudaFree(c->d_image);
     delete c;
     return (int)(e1 != cudaSuccess ? e1 : e2);
 }

@@ -27,8 +27,7 @@
 // first.  Only these kinds of barrier are waited on by parity, and each has that property by
 // construction: ready[buf] (its next phase needs every compute warp to have left an op that comes
 // after the one being waited for), xs and dep (every waiter must arrive, or pass xs, before the next
-// phase can complete), image (it is armed for a later op only when every compute warp has left the one
-// before that op, and a warp leaves an op that waits for the image behind that wait), full[slot] (a task first sees `issued > g`, published after the barrier was
+// phase can complete), full[slot] (a task first sees `issued > g`, published after the barrier was
 // armed for tile g, and the slot cannot be re-armed before that task has copied out).  Everything
 // that a warp may fall arbitrarily far behind on is a monotonic counter instead: ops_done (every
 // compute warp has left ops [0, ops_done)), ops_loaded, issued, copy_op.  Slot release is a plain
@@ -66,6 +65,7 @@ constexpr uint32_t CHAIN_GATE_NS0 = 32, CHAIN_GATE_NSMAX = 256;   // ... of the 
 // The warps of a CTA that wait for each other, or for what one lane of them waits for, leave when that lane has given up (ctrl[14]); should it
 // say nothing either, after this time (several ranks: and their own limit).
 constexpr uint32_t CHAIN_WAIT_MS = 8000;
+constexpr uint32_t CHAIN_IMAGE_POLLS = 1u << 21;                  // trips to L2 with sleeps of 32 ns, some two seconds, that a warp waits for a spread op's image
 constexpr int CHAIN_GATES = 3;           // a warp may run this many ops ahead of the slowest one
 
 struct __align__(16) ChainOp {                 // 128 bytes, one per projection, device table
@@ -184,7 +184,8 @@ __device__ __forceinline__ bool rank_flags_wait(const unsigned int *flags, int w
 // words of its own block.  Sequence numbers are never reset: a launch reads its run number from counter word 2 and
 // the last CTA to leave adds 1 to it; every launch ends with one more signal + wait, so that no rank starts its
 // next run (and writes into its peers' outputs) before every rank has finished this one.
-// Counter block (16 words): [0] arrivals of dependent-op producers (one-rank form) [1] spread blocks [2] run
+// Counter block (16 words): [0] arrivals of dependent-op producers (one-rank form) [1] blocks rotated by spread ops in all runs before: who
+// writes an image counts its tags from here, who reads it from the run number [2] run
 // [3] CTAs out [4] CTAs of this GPU that have sent their rows, all signals so far [8 + q] last signal of rank q.
 constexpr int CHAIN_MAX_RANKS = 8;
 struct ChainPeers {
@@ -196,9 +197,20 @@ struct ChainPeers {
     unsigned int *counter[CHAIN_MAX_RANKS];     // rank p's counter block
 };
 
-// Back butterflies and quantiser of N units (u0, u0 + step, ... slices of the scratch area) side by side into the tables.
+// The image of a spread op's tables in global memory: per block 32 words of values and four chunk headers, each beside the op's tag in one
+// 64-bit word.  A reader that finds the tag has the value, so nobody fences, counts or waits for a count between the two.
+constexpr int CHAIN_IMAGE_WORDS = 36;
+__device__ __forceinline__ void image_store(unsigned long long *at, uint32_t value, uint32_t tag) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(at), "l"((unsigned long long)tag << 32 | value) : "memory");
+}
+__device__ __forceinline__ void image_load2(const unsigned long long *at, unsigned long long &a, unsigned long long &b) {
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(at) : "memory");
+}
+
+// Back butterflies and quantiser of N units (u0, u0 + step, ... slices of the scratch area) side by side into the tables, or into the image.
 template <int N>
-__device__ __forceinline__ void chain_back_units(const float4 *scratch, int u0, int step, int chunk0, int lane, uint32_t *act_q, float *act_s, int *act_i) {
+__device__ __forceinline__ void chain_back_units(const float4 *scratch, int u0, int step, int chunk0, int lane, uint32_t *act_q, float *act_s, int *act_i,
+                                                 unsigned long long *image, uint32_t tag) {
     float v[N][4];
     uint32_t word[N], header[N];
 #pragma unroll
@@ -210,6 +222,12 @@ __device__ __forceinline__ void chain_back_units(const float4 *scratch, int u0, 
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         const int chunk = chunk0 + (u0 + k * step) * 4 + (lane >> 3);
+        if (image) {
+            unsigned long long *at = image + (size_t)(chunk >> 2) * CHAIN_IMAGE_WORDS;
+            image_store(at + (chunk & 3) * 8 + (lane & 7), word[k], tag);
+            if ((lane & 7) == 0) image_store(at + 32 + (chunk & 3), header[k], tag);
+            continue;
+        }
         act_q[(chunk >> 2) * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word[k];
         if ((lane & 7) == 0) {
             act_s[chunk] = f16_bits_to_f32(header[k] & 0xFFFFu);
@@ -219,16 +237,17 @@ __device__ __forceinline__ void chain_back_units(const float4 *scratch, int u0, 
 }
 // A warp's units, PAIRS: two at a time (one after the other each is a chain of shuffles and divisions of 1600 clocks).
 template <bool PAIRS>
-__device__ __forceinline__ void chain_back(const float4 *scratch, int u0, int step, int units, int chunk0, int lane, uint32_t *act_q, float *act_s, int *act_i) {
+__device__ __forceinline__ void chain_back(const float4 *scratch, int u0, int step, int units, int chunk0, int lane, uint32_t *act_q, float *act_s, int *act_i,
+                                           unsigned long long *image, uint32_t tag) {
     if (PAIRS)
-        for (; u0 + step < units; u0 += 2 * step) chain_back_units<2>(scratch, u0, step, chunk0, lane, act_q, act_s, act_i);
-    for (; u0 < units; u0 += step) chain_back_units<1>(scratch, u0, step, chunk0, lane, act_q, act_s, act_i);
+        for (; u0 + step < units; u0 += 2 * step) chain_back_units<2>(scratch, u0, step, chunk0, lane, act_q, act_s, act_i, image, tag);
+    for (; u0 < units; u0 += step) chain_back_units<1>(scratch, u0, step, chunk0, lane, act_q, act_s, act_i, image, tag);
 }
 
 template <int THREADS, int MAXSTEPS, bool TP>
 __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *__restrict__ ops, const int n_ops,
                                                                 const ChainGeom G, unsigned int *grid_counter,
-                                                                uint8_t *table_image, const ChainPeers PE) {
+                                                                unsigned long long *table_image, const ChainPeers PE) {
     constexpr int C = THREADS / 32 - 2 - (TP ? 1 : 0);      // compute warps (several ranks: one warp talks to the peers)
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);      // [16] tile landed in slot
@@ -236,14 +255,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
     uint64_t *xs = ready + CHAIN_TABLES;                                  // [1]  rotate: every warp has written its blocks
     uint64_t *dep = xs + 1;                                   // [1]  rotate: the producers of x have arrived
     uint64_t *stage_full = dep + 1;                           // [1]  Q8_1 staging copy landed
-    uint64_t *image = stage_full + 1;                         // [1]  a spread op's tables have been copied from the image
     int *done_cnt = reinterpret_cast<int *>(smem + 192);      // [16] tasks of the slot's tile that have copied out
     int *expect_cnt = done_cnt + CHAIN_MAX_SLOTS;             // [16] ... of how many
     volatile int *ctrl = expect_cnt + CHAIN_MAX_SLOTS;        // [16] 0 issued, 1 ops_loaded, 2 next_task, 3 copy_op, 4-7 warps that
                                                               //      left op (index & 3), 8 ops_done: every compute warp has left ops [0, ops_done),
                                                               //      9 (several ranks) ops whose rows the peer warp has sent,
                                                               //      10-13 largest |y| of op (index & 3) so far, as float bits,
-                                                              //      14 a compute warp has given up on a wait: the others leave too
+                                                              //      14 a compute warp has given up on a wait: the others leave too,
+                                                              //      15 (several ranks) blocks rotated for the grid in all runs before
     float *ssum = reinterpret_cast<float *>(smem + 384);     // [56] sums of squares of the slices of an RMSNorm input
     ChainOp *opring = reinterpret_cast<ChainOp *>(smem + 640);
     uint8_t *p = smem + 640 + CHAIN_OP_RING * sizeof(ChainOp);
@@ -270,10 +289,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
         mbar_init(xs, C);
         mbar_init(dep, 1);
         mbar_init(stage_full, 1);
-        mbar_init(image, 1);
         mbar_fence_init();
     }
-    for (int i = threadIdx.x; i < 3 * CHAIN_MAX_SLOTS; i += THREADS) done_cnt[i] = 0;     // done, expect, ctrl
+    for (int i = threadIdx.x; i < 3 * CHAIN_MAX_SLOTS; i += THREADS) done_cnt[i] = TP && i == 2 * CHAIN_MAX_SLOTS + 15 ? (int)__ldcg(grid_counter + 1) : 0;     // done, expect, ctrl
     for (int i = threadIdx.x; i < CHAIN_GATES * G.quad_ints; i += THREADS) quad_base[i] = 0;
     __syncthreads();
 
@@ -318,7 +336,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
         int op = -1, flags = 0;
         volatile int *stop = &ctrl[14];
         const uint32_t wait_ms = CHAIN_WAIT_MS + (TP ? (uint32_t)(PE.wait_limit_ns >> 20) : 0u);
-        uint32_t xs_phase = 0, dep_phase = 0, image_phase = 0;     // every compute warp takes part in every meeting, so it counts them itself
+        uint32_t xs_phase = 0, dep_phase = 0;     // every compute warp takes part in every meeting, so it counts them itself
         int task_base = 0, ntasks = 0, g_base = 0, ntiles = 0;
         for (;;) {
             int task = 0;
@@ -372,13 +390,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                     if (flags & CHAIN_ROTATE) {
                         // Wide inputs of dependent ops are rotated ONCE for the whole grid instead of once per CTA
                         // (every CTA repeating 17 blocks costs ~10 us): block fb is rotated by CTA fb, which writes
-                        // its part of the tables to an image in global memory; a second arrival counter tells
-                        // everybody when all blocks are there, and every CTA copies the image into its tables.  A CTA without
-                        // a block has nothing else to wait for.
+                        // its part of the tables to an image in global memory, tagged, and every CTA reads the image into its tables.  A CTA
+                        // without a block has nothing else to wait for.  (With a counter of the blocks that are there and a copy of the whole image
+                        // behind it: 2.1 us from the quantiser to the tables, 0.9 now.)  Of an RMSNorm input, whose sum of squares
+                        // needs all of it, such a CTA sums all and rotates its block (every CTA rotating 5120 values for itself: 4.8 us from the
+                        // arrival of x to the tables, 3.6 now).
                         const bool spread = flags & CHAIN_SPREAD;
                         const int nfb = R.nb >> 3;
                         const int fb_lo = spread ? min((int)blockIdx.x, nfb) : 0;
                         const int fb_hi = spread ? min((int)blockIdx.x + 1, nfb) : nfb;
+                        const bool whole = spread && (flags & CHAIN_RMSNORM);      // read all, rotate units [own, own + 8)
+                        const int own = whole ? fb_lo * 8 : 0;
+                        const int fb_first = whole ? 0 : fb_lo;
                         // What the vector is multiplied by waits for nobody, unless the list itself writes it (CHAIN_LATE): norm weights
                         // (from memory, once a run) go to this thread's places in the scratch area while the producers of x finish,
                         // signs are asked into L2.
@@ -389,10 +412,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                         constexpr int UPW = (7 * 8 + C - 1) / C;               // units per warp and round trip
 #pragma unroll
                         for (int k = 0; k < UPW; ++k) {
-                            const int u = wid + k * C;
-                            if (u < min(G.rot_blocks, fb_hi - fb_lo) * 8) {
-                                if (signs) prefetch_l2(signs + (size_t)fb_lo * FWHT_N + (size_t)u * 128 + 4 * lane);
-                                if ((flags & CHAIN_RMSNORM) && !late) scratch[u * 32 + lane] = __ldg(reinterpret_cast<const float4 *>(aux + (size_t)u * 128 + 4 * lane));
+                            const int v = wid + k * C - own;                   // (own: at most 7 x 8, and a warp has at most one unit of a block)
+                            if ((unsigned)v < (unsigned)(min(G.rot_blocks, fb_hi - fb_lo) * 8)) {
+                                const size_t at = (size_t)fb_lo * FWHT_N + (size_t)v * 128 + 4 * lane;
+                                if (signs) prefetch_l2(signs + at);
+                                if ((flags & CHAIN_RMSNORM) && !late) scratch[v * 32 + lane] = __ldg(reinterpret_cast<const float4 *>(aux + at));
                             }
                         }
                         // every compute warp has left op - 1: both table buffers' readers are gone
@@ -412,10 +436,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                             if (!mbar_wait_suspended(dep, dep_phase & 1u, stop, wait_ms)) { alive = false; break; }
                             ++dep_phase;
                         }
-                        uint8_t *own = tables + (size_t)R.buf * table_bytes;
-                        uint32_t *act_q = reinterpret_cast<uint32_t *>(spread ? table_image : own);
+                        uint32_t *act_q = reinterpret_cast<uint32_t *>(tables + (size_t)R.buf * table_bytes);
                         float *act_s = reinterpret_cast<float *>(act_q + (size_t)G.nb_max * STREAM_ACT_WORDS);
                         int *act_i = reinterpret_cast<int *>(act_s + (size_t)G.nb_max * 4);
+                        // a spread op's tag counts up over a list, and over the runs of several ranks (whose kernel has no register for it here)
+                        const uint32_t tag1 = !TP && spread ? R.spread_blocks : 0u;
                         // the exact power-of-two rescale of the synthetic decode step: the producer recorded max |x|
                         float rescale = 1.0f;
                         const int src_len = R.src_len;
@@ -427,8 +452,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                         // One warp per 128-element slice, G.rot_blocks 1024-blocks per round trip through
                         // the scratch area: front butterflies, meet, back butterflies + quantiser, meet.
                         bool ok = true;
-                        for (int fb0 = fb_lo; fb0 < fb_hi && ok; fb0 += G.rot_blocks) {
-                            const int units = min(G.rot_blocks, fb_hi - fb0) * 8;
+                        for (int fb0 = fb_first; fb_lo < fb_hi && fb0 < fb_hi && ok; fb0 += whole ? nfb : G.rot_blocks) {
+                            const int units = (whole ? nfb : min(G.rot_blocks, fb_hi - fb0)) * 8;
                             // all of this warp's loads first (they come from L2: written by other SMs
                             // during this launch), then the butterflies
                             float4 f[UPW];
@@ -472,7 +497,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                 ++xs_phase;
                                 if (!ok) break;
                                 float ss = 0.0f;
-#pragma unroll 2
+#pragma unroll 4
                                 for (int u = 0; u < units; u += 8) {
                                     const float4 a = *reinterpret_cast<const float4 *>(ssum + u), b = *reinterpret_cast<const float4 *>(ssum + u + 4);
                                     ss = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(ss, a.x), a.y), a.z), a.w);
@@ -482,8 +507,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
 #pragma unroll
                                 for (int k = 0; k < UPW; ++k) {
                                     const int u = wid + k * C;
-                                    if (u < units) {
-                                        const float4 wv = late ? __ldcg(reinterpret_cast<const float4 *>(aux + (size_t)u * 128 + 4 * lane)) : scratch[u * 32 + lane];
+                                    if (whole ? (unsigned)(u - own) < 8u : u < units) {
+                                        const float4 wv = late ? __ldcg(reinterpret_cast<const float4 *>(aux + (size_t)u * 128 + 4 * lane)) : scratch[(u - own) * 32 + lane];
                                         f[k] = make_float4(__fmul_rn(__fmul_rn(f[k].x, sc), wv.x), __fmul_rn(__fmul_rn(f[k].y, sc), wv.y),
                                                            __fmul_rn(__fmul_rn(f[k].z, sc), wv.z), __fmul_rn(__fmul_rn(f[k].w, sc), wv.w));
                                     }
@@ -492,7 +517,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
 #pragma unroll
                             for (int k = 0; k < UPW; ++k) {
                                 const int u = wid + k * C;
-                                if (u < units) {
+                                if (whole ? (unsigned)(u - own) < 8u : u < units) {
                                     float v[4] = {f[k].x, f[k].y, f[k].z, f[k].w};
                                     if (signs) {
                                         const float4 *sp = reinterpret_cast<const float4 *>(signs + (size_t)fb0 * FWHT_N + (size_t)u * 128 + 4 * lane);
@@ -501,7 +526,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                         v[2] = __fmul_rn(v[2], sg.z); v[3] = __fmul_rn(v[3], sg.w);
                                     }
                                     fwht_slice_front(v, lane);
-                                    scratch[u * 32 + lane] = make_float4(v[0], v[1], v[2], v[3]);
+                                    scratch[(u - own) * 32 + lane] = make_float4(v[0], v[1], v[2], v[3]);
                                 }
                             }
                             __syncwarp();
@@ -509,7 +534,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                             ok = mbar_wait_suspended(xs, xs_phase & 1u, stop, wait_ms);
                             ++xs_phase;
                             if (!ok) break;
-                            chain_back<THREADS == 512>(scratch, wid, C, units, fb0 * 32, lane, act_q, act_s, act_i);
+                            chain_back<THREADS == 512>(scratch, wid, C, whole ? 8 : units, fb0 * 32 + own * 4, lane, act_q, act_s, act_i, spread ? table_image : nullptr,
+                                                       TP ? (uint32_t)ctrl[15] + R.spread_blocks : tag1);
+                            if (spread) break;                          // one block: the scratch area is not written again before the meeting below
                             __syncwarp();
                             if (lane == 0) mbar_arrive(xs);
                             ok = mbar_wait_suspended(xs, xs_phase & 1u, stop, wait_ms);
@@ -517,33 +544,51 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                         }
                         if (!ok) { alive = false; break; }
                         if (spread) {
-                            bool armed = false;
-                            if (wid == 0 && lane == 0) {
-                                if (fb_lo < fb_hi) {                    // this CTA's block is in the image (behind the meeting: every warp's part)
-                                    __threadfence();
-                                    atomicAdd(grid_counter + 1, (unsigned)(fb_hi - fb_lo));
+                            // image -> this CTA's tables, 16 bytes (two words and their tags) per lane and load
+                            const uint32_t tag = TP ? spread_base + R.spread_blocks : tag1;
+                            constexpr int BATCH = THREADS == 512 ? 4 : 2;
+                            const int n = R.nb * (CHAIN_IMAGE_WORDS / 2);
+                            for (int i0 = wid * 32 + lane; i0 - lane < n && ok; i0 += BATCH * C * 32) {
+                                unsigned long long w[BATCH][2];
+                                for (uint32_t polls = 0;; ++polls) {
+                                    bool there = true;
+#pragma unroll
+                                    for (int k = 0; k < BATCH; ++k) {
+                                        const int i = i0 + k * C * 32;
+                                        w[k][0] = w[k][1] = (unsigned long long)tag << 32;
+                                        if (i < n) image_load2(table_image + 2 * (size_t)i, w[k][0], w[k][1]);
+                                    }
+#pragma unroll
+                                    for (int k = 0; k < BATCH; ++k) there = there && (uint32_t)(w[k][0] >> 32) == tag && (uint32_t)(w[k][1] >> 32) == tag;
+                                    if (__all_sync(0xffffffffu, there)) break;
+                                    if (polls >= CHAIN_IMAGE_POLLS || *stop) { ok = false; break; }
+                                    __nanosleep(CHAIN_NS0);
                                 }
-                                if (grid_counter_wait(grid_counter + 1, spread_base + R.spread_blocks)) {
-                                    // image -> this CTA's tables, by the copy unit: written by other SMs during this launch
-                                    asm volatile("fence.proxy.async;" ::: "memory");
-                                    const uint64_t pol = policy_evict_normal();
-                                    const size_t q_at = (size_t)G.nb_max * STREAM_ACT_WORDS * 4, i_at = q_at + (size_t)G.nb_max * 16;
-                                    mbar_expect_tx(image, (uint32_t)R.nb * 176);
-                                    bulk_g2s(own, table_image, (uint32_t)R.nb * STREAM_ACT_WORDS * 4, image, pol);
-                                    bulk_g2s(own + q_at, table_image + q_at, (uint32_t)R.nb * 16, image, pol);
-                                    bulk_g2s(own + i_at, table_image + i_at, (uint32_t)R.nb * 16, image, pol);
-                                    armed = true;
-                                } else {
-                                    *stop = 1;
+                                if (!ok) break;
+#pragma unroll
+                                for (int k = 0; k < BATCH; ++k) {
+                                    const int i = i0 + k * C * 32;
+                                    if (i >= n) continue;
+                                    const int b = i / (CHAIN_IMAGE_WORDS / 2), q = i - b * (CHAIN_IMAGE_WORDS / 2);
+                                    const uint32_t a0 = (uint32_t)w[k][0], a1 = (uint32_t)w[k][1];
+                                    if (q < 16) {
+                                        *reinterpret_cast<uint2 *>(act_q + b * STREAM_ACT_WORDS + 2 * q) = make_uint2(a0, a1);
+                                    } else {
+                                        const int c = b * 4 + 2 * (q - 16);
+                                        *reinterpret_cast<float2 *>(act_s + c) = make_float2(f16_bits_to_f32(a0 & 0xFFFFu), f16_bits_to_f32(a1 & 0xFFFFu));
+                                        *reinterpret_cast<int2 *>(act_i + c) = make_int2(-64 * (int)(short)(a0 >> 16), -64 * (int)(short)(a1 >> 16));
+                                    }
                                 }
                             }
-                            __syncwarp();
-                            if (!mbar_wait_suspended(image, image_phase & 1u, stop, wait_ms)) {
-                                if (armed) mbar_wait_bounded(image, image_phase & 1u);      // nobody leaves with copies of its own in flight
+                            if (!ok) {
+                                if (lane == 0) atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);
                                 alive = false;
                                 break;
                             }
-                            ++image_phase;
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(xs);
+                            if (!mbar_wait_suspended(xs, xs_phase & 1u, stop, wait_ms)) { alive = false; break; }
+                            ++xs_phase;
                         }
                     } else {
                         if (!mbar_wait_bounded(&ready[R.buf], (uint32_t)R.ready_parity, CHAIN_GATE_NS0, CHAIN_GATE_NSMAX)) { alive = false; break; }
@@ -706,6 +751,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
         if (good && lane == 0) {
             if (atomicAdd(grid_counter + 3, 1u) == (unsigned)ncta - 1u) {        // last CTA out: the next launch is run + 1
                 grid_counter[3] = 0u;
+                grid_counter[1] = spread_base + PE.spread_per_run;
                 __threadfence();
                 atomicAdd(grid_counter + 2, 1u);
             }
