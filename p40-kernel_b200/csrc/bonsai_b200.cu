@@ -1314,14 +1314,34 @@ int bonsai_p40_gemv_repack(const void *W, const float *x, float *y, int64_t n_ou
         StreamParams sp;
         int threads = 0, smem_bytes = 0;
         if (tree && vec && n_in % FWHT_N == 0 && plan_stream(n_out, nb, g_opt_gemv_variant.load(), sp, threads, smem_bytes)) {
-            static SmemOptIn sopt;
-            cudaError_t err = sopt.ensure(gemv_stream_kernel<true, true>);
-            if (err != cudaSuccess) return (int)err;
+            // Long rows: the CTAs of a cluster share the quantiser.  In fours while they are few enough to leave no SM to two of them (clusters do
+            // not cross a group of SMs; 147 CTAs in fours ran two to an SM in places and took twice as long), else in pairs, whose
+            // barrier is worth it from 96 blocks on.  us, alone / in pairs / in fours: 17408 -> 64 6.96 / 5.62 / 4.82, -> 1000 7.66 / 6.66 / 6.00, -> 5120
+            // 11.7 / 10.7 / 18.7; 12288 -> 5120 9.06 / 9.00 / 16.0; 9216 -> 5120 7.43 / 8.10; 5120 -> 64 3.57 / 3.57 / 3.20, -> 1000 3.96 / 4.16 / 3.83.
+            const unsigned ctas = (unsigned)((n_out + sp.rows_per_cta - 1) / sp.rows_per_cta);
+            const unsigned cl = ctas <= 128 && nb >= 40 ? 4 : nb >= 96 ? 2 : 1;
             sp.early = pdl;
-            return (int)launch(gemv_stream_kernel<true, true>, dim3((unsigned)((n_out + sp.rows_per_cta - 1) / sp.rows_per_cta)),
-                               dim3(threads), (size_t)smem_bytes, as_stream(stream), true, static_cast<const uint8_t *>(W),
-                               static_cast<const uint32_t *>(nullptr), y, sp, x, static_cast<const float *>(nullptr),
-                               static_cast<uint32_t *>(nullptr));
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((ctas + cl - 1) / cl * cl);
+            cfg.blockDim = dim3(threads);
+            cfg.dynamicSmemBytes = (size_t)smem_bytes;
+            cfg.stream = as_stream(stream);
+            cudaLaunchAttribute attr[2];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = cl;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[1].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = cl == 1 ? attr + 1 : attr;
+            cfg.numAttrs = (cl > 1) + (g_opt_overlap.load() != 0);
+            static SmemOptIn sopt[3];
+            auto go = [&](auto kernel, SmemOptIn &o) -> int {
+                cudaError_t err = o.ensure(kernel);
+                if (err != cudaSuccess) return (int)err;
+                return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<const uint8_t *>(W), static_cast<const uint32_t *>(nullptr), y, sp, x,
+                                               static_cast<const float *>(nullptr), static_cast<uint32_t *>(nullptr));
+            };
+            return cl == 4 ? go(gemv_stream_kernel<true, true, 4>, sopt[2]) : cl == 2 ? go(gemv_stream_kernel<true, true, 2>, sopt[1]) : go(gemv_stream_kernel<true, true>, sopt[0]);
         }
     }
     auto pick = [&](auto t, auto v, int base) -> cudaError_t {

@@ -87,6 +87,18 @@ __device__ __forceinline__ int chunk_sumi_scaled(uint32_t w0, uint32_t w1, const
 // ---- shared-memory barriers and bulk copies (sm_90+ PTX, every copy is local to its CTA) -------
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// ---- clusters of CTAs ----
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Into CTA `rank`'s shared memory, at the place that `addr` is in this one's.
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t rank, uint32_t v) {
+    asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.u32 [a], %2;\n\t}" ::"r"(addr), "r"(rank), "r"(v) : "memory");
+}
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }

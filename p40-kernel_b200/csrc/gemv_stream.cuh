@@ -204,7 +204,8 @@ __device__ __forceinline__ float stream_task_repack(const uint8_t *row, int nb, 
 // to `xq_out` so that the caller's scratch holds what the two-launch form would have left there.
 // REPACK = true (with FUSED) is bonsai_p40_gemv_repack: W is in the repacked layout and x is quantised WITHOUT a
 // rotation (src/kernels/gemv_repack_p40.cu:91-162 fuses exactly that).
-template <bool FUSED, bool REPACK = false>
+// CL > 1 (with REPACK): the CTAs of a cluster quantise a share of x each and store it into the tables of all of them.
+template <bool FUSED, bool REPACK = false, int CL = 1>
 __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__restrict__ W, const uint32_t *xq,
                                                              float *y, const StreamParams P,
                                                              const float *x, const float *signs,
@@ -223,8 +224,9 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
     const int slot_bytes = P.tr * (int)row_bytes + 16;
 
     const int row0 = blockIdx.x * P.rows_per_cta;
-    const int rows_here = min(P.rows_per_cta, P.n_out - row0);
-    if (rows_here <= 0) return;
+    const int rows_here = max(0, min(P.rows_per_cta, P.n_out - row0));
+    if (CL == 1 && rows_here == 0) return;
+    if (CL > 1) cluster_arrive();                       // this CTA runs: the others may store into its tables
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nwarps = blockDim.x >> 5;
     const int compute_warps = nwarps - 1;
@@ -278,13 +280,14 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
         // 5120 x 5120 6.9 -> 5.2 us, 17408 x 5120 15.0 -> 13.1 us)
         constexpr int SLICES = 5;
         bool first = true;
-        for (int s0 = wid; s0 < P.nb || first; s0 += SLICES * compute_warps) {
+        const int mine = CL == 1 ? 0 : (int)cluster_rank(), nb = CL == 1 ? P.nb : (P.nb - mine + CL - 1) / CL;     // this CTA's slices: CL * s + mine
+        for (int s0 = wid; s0 < nb || first; s0 += SLICES * compute_warps) {
             float4 f[SLICES];
-            const int left = P.nb - s0, n = 1 + (left > compute_warps) + (left > 2 * compute_warps) + (left > 3 * compute_warps);
+            const int left = nb - s0, n = 1 + (left > compute_warps) + (left > 2 * compute_warps) + (left > 3 * compute_warps);
 #pragma unroll
             for (int k = 0; k < SLICES; ++k) {
                 const int sl = s0 + k * compute_warps;
-                f[k] = wid < compute_warps && sl < P.nb ? *reinterpret_cast<const float4 *>(x + (size_t)sl * 128 + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+                f[k] = wid < compute_warps && sl < nb ? *reinterpret_cast<const float4 *>(x + (size_t)(CL * sl + mine) * 128 + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             if (first) {
                 // every warp has issued its first loads: the rest of the ring may queue behind them
@@ -292,6 +295,10 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
                 if (wid == compute_warps && lane == 0)
                     for (int t = first_late; t < first_fill; ++t) issue_tile(t);
                 first = false;
+                if (CL > 1) {
+                    __syncwarp();
+                    cluster_wait();
+                }
             }
             // a warp's slices side by side, their divisions shared (one per lane of a chunk): one after the other each was a chain
             // of shuffles and two divisions, before the first product.  As many as there are: a slice that is not there costs what one does
@@ -306,8 +313,21 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
                 quantise_chunks_8lanes<N>(v, lane, word, header);
 #pragma unroll
                 for (int k = 0; k < N; ++k) {
+                    if (CL > 1 && s0 + k * compute_warps < nb) {
+                        const int sl = CL * (s0 + k * compute_warps) + mine, chunk = 4 * sl + (lane >> 3);
+                        const uint32_t at_q = smem_u32(act_q + sl * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7));
+                        const uint32_t at_s = smem_u32(act_s + chunk), at_i = smem_u32(act_i + chunk);
+#pragma unroll
+                        for (uint32_t c = 0; c < CL; ++c) {
+                            st_cluster_u32(at_q, c, word[k]);
+                            if ((lane & 7) == 0) {
+                                st_cluster_u32(at_s, c, __float_as_uint(f16_bits_to_f32(header[k] & 0xFFFFu)));
+                                st_cluster_u32(at_i, c, (uint32_t)(-64 * (int)(short)(header[k] >> 16)));
+                            }
+                        }
+                    }
                     const int sl = s0 + k * compute_warps;
-                    if (sl < P.nb) {
+                    if (CL == 1 && sl < P.nb) {
                         const int chunk = 4 * sl + (lane >> 3);
                         act_q[sl * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word[k];
                         if ((lane & 7) == 0) {
@@ -317,7 +337,7 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
                     }
                 }
             };
-            if (wid < compute_warps && s0 < P.nb) {                     // warp-uniform
+            if (wid < compute_warps && s0 < nb) {                       // warp-uniform
                 if (n == 1) quantise(std::integral_constant<int, 1>());
                 else if (n == 2) quantise(std::integral_constant<int, 2>());
                 else if (n == 3) quantise(std::integral_constant<int, 3>());
@@ -389,7 +409,13 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
             act_i[chunk] = -64 * (int)(short)(v[0] >> 16);
         }
     }
-    __syncthreads();                    // activation arrays, counters and barrier inits visible to all
+    if (CL > 1) {                       // activation arrays, counters and barrier inits visible to all, of every CTA of the cluster
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    } else {
+        __syncthreads();
+    }
 
     if (wid < compute_warps) {
         const int rr = lane & 3, bl = lane >> 2;

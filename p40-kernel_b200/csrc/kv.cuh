@@ -164,13 +164,6 @@ __device__ __forceinline__ void split_rest_f16x2(float a, float b, uint32_t &hi,
 }
 __device__ __forceinline__ float half_bits_lo(uint32_t w) { return f16_bits_to_f32(w & 0xFFFFu); }
 __device__ __forceinline__ float half_bits_hi(uint32_t w) { return f16_bits_to_f32(w >> 16); }
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Adds 1 to a counter in global memory; what the CTA wrote before the barrier in front of this call is visible to whoever
 // reads the sum, and what they wrote to this CTA after the barrier behind it.
 __device__ __forceinline__ unsigned int count_arrival(unsigned int *counter) {
