@@ -1096,8 +1096,8 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     static SmemOptIn opt;
     e = opt.ensure(gemm_tc16_kernel<TN, CTAS>);
     if (e != cudaSuccess) return (int)e;
-    e = launch(tc16_split_kernel, dim3((unsigned)groups, (unsigned)((n_chunks + slice - 1) / slice)), dim3(T16_SPLIT_THREADS), 0, st, true, x32, n_chunks,
-               (int)n_tok, slice, scale, planes);
+    e = launch(groups <= 2 * sms ? tc16_split_kernel<true> : tc16_split_kernel<false>, dim3((unsigned)groups, (unsigned)((n_chunks + slice - 1) / slice)),
+               dim3(T16_SPLIT_THREADS), 0, st, true, x32, n_chunks, (int)n_tok, slice, scale, planes);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(grid * CTAS));
