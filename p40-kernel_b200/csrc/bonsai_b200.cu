@@ -989,7 +989,7 @@ static size_t tc16_scratch_bytes(int64_t n_in, int64_t n_tok) {
     return T16_FLAGS_BYTES + T16_PARTS_BYTES + 2 * (size_t)n_tok * (size_t)n_in * sizeof(__half) + (size_t)n_tok * sizeof(float);
 }
 
-// The fp16 tensor-core mat-mul (gemm_tc16.cuh).  -1: not taken (shape, alignment, no scratch, no tensor-map encoder, no SMs in pairs).
+// The fp16 tensor-core mat-mul (gemm_tc16.cuh).  -1: not taken (shape, alignment, no scratch, no tensor-map encoder, no SMs in pairs or no launch of them).
 extern "C++" {
 // Pairs of CTAs that are resident at once on the current device (0: they do not run here).  Asked once per device.
 static int tc16_pairs() {
@@ -1112,7 +1112,12 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = CTAS == 1 ? 1 : 2;
-    return (int)cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN, CTAS>, Y, P, (const float *)scale, parts, flags, maps);
+    e = cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN, CTAS>, Y, P, (const float *)scale, parts, flags, maps);
+    if (CTAS != 1 && (e == cudaErrorInvalidConfiguration || e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
+        (void)cudaGetLastError();                        // a cooperative launch in clusters is refused, by a profiler that replays it for instance
+        return -1;
+    }
+    return (int)e;
 }
 }  // extern "C++"
 // Tiles of up to 64 tokens by a CTA, or of up to 128 by a pair of CTAs (the code expansion is paid once per tile, and each CTA fetches half
