@@ -575,7 +575,7 @@ int bonsai_b200_linear_static(const void *W, const float *x, const float *signs,
 struct bonsai_b200_chain {
     ChainOp *d_ops = nullptr;
     unsigned int *d_counter = nullptr;      // [0] arrivals of ops that others wait for
-    unsigned long long *d_image = nullptr;  // activation tables of a spread op, shared through L2 (one rank: behind the counters)
+    uint8_t *d_image = nullptr;             // activation tables of a spread op, shared through L2 (one rank: behind the counters)
     bool tp = false;                        // several ranks: counters live in the caller's peer-mapped buffer, never reset
     ChainPeers peers{};
     int n_ops = 0, threads = 0, grid = 0, device = 0;
@@ -820,7 +820,7 @@ static int chain_create_impl(const bonsai_b200_op *ops, int64_t n_ops, int tp_ra
     if (e == cudaSuccess && any_spread && tp) e = cudaMalloc(&c->d_image, image_bytes);
     if (e == cudaSuccess && any_spread && tp && !zero_new_memory(c->d_image, image_bytes)) e = cudaErrorUnknown;      // no tag of any run
     if (e == cudaSuccess && any_spread && !tp) {
-        c->d_image = reinterpret_cast<unsigned long long *>(reinterpret_cast<uint8_t *>(c->d_counter) + c->counter_bytes);
+        c->d_image = reinterpret_cast<uint8_t *>(c->d_counter) + c->counter_bytes;
         c->counter_bytes += image_bytes;
     }
     if (e == cudaSuccess) e = cudaMemcpy(c->d_ops, rec.data(), sizeof(ChainOp) * (size_t)n_ops, cudaMemcpyHostToDevice);

@@ -33,7 +33,7 @@
 // compute warp has left ops [0, ops_done)), ops_loaded, issued, copy_op.  Slot release is a plain
 // counter too, because the number of tasks per tile changes from op to op.
 // Every wait is bounded: a second or so by counted polls with sleeps (the copy, sequencer and peer warps, the ring), some three seconds
-// for other CTAs (grid_counter_wait), the caller's limit for other ranks, and for warps that wait for each other's part of these until
+// for other CTAs (grid_counter_wait; two for the words of an image), the caller's limit for other ranks, and for warps that wait for each other's part of these until
 // one of them has given up.  A time-out sets the status word and the warp leaves.
 #pragma once
 
@@ -247,8 +247,9 @@ __device__ __forceinline__ void chain_back(const float4 *scratch, int u0, int st
 template <int THREADS, int MAXSTEPS, bool TP>
 __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *__restrict__ ops, const int n_ops,
                                                                 const ChainGeom G, unsigned int *grid_counter,
-                                                                unsigned long long *table_image, const ChainPeers PE) {
+                                                                uint8_t *image_bytes, const ChainPeers PE) {
     constexpr int C = THREADS / 32 - 2 - (TP ? 1 : 0);      // compute warps (several ranks: one warp talks to the peers)
+    unsigned long long *table_image = reinterpret_cast<unsigned long long *>(image_bytes);
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);      // [16] tile landed in slot
     uint64_t *ready = full + CHAIN_MAX_SLOTS;                 // [2]  tables of a Q8_1 op are filled
