@@ -22,7 +22,7 @@
 // columns: 256 output (before that, sums of the scores), 128 scores (then weights), 128 q low.
 // What bounds it (counted while a score was four sums): per tile 5900 of 10200 cycles were the tensor core's, most of them the score
 // products (N = 64: it waits for the q rows from shared memory), the rest softmax and the exchanges in front of it.  2048 tokens, 24 heads over 4: 2570 ->
-// 286 us; 1000 tokens 727 -> 92 us, 600 tokens 62 us.
+// 279 us; 1000 tokens 727 -> 90 us, 600 tokens 59 us.
 //
 // A plane pair holds 2^-39 of the largest value under its power of two, so what is far smaller loses bits to values that a row may not
 // even see.  A CTA whose queries and keys range too widely (atc_too_wide) does its queries again on the CUDA cores (attn_simt), with
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
     float *kf = reinterpret_cast<float *>(vpl + ATC_PLANES);             // [2][64] 2^-s of the tile's keys, tiles alternate
     float *vf = kf + 2 * ATC_KEYS;                                       // [2][256] 2^-s of the dims (and the weights' 2^-14)
     float *red = vf + 2 * ATT_D;                                         // [4][128] exchange between the four warps of a row
-    uint64_t *qk1 = reinterpret_cast<uint64_t *>(red + 4 * ATC_M), *qk2 = qk1 + 1, *pv = qk1 + 2, *kfull = qk1 + 3, *vfull = qk1 + 4;
+    uint64_t *qk = reinterpret_cast<uint64_t *>(red + 4 * ATC_M), *pv = qk + 1, *kfull = qk + 2, *vfull = qk + 3;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(vfull + 1);
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -228,7 +228,8 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
     const uint8_t *img = images + (size_t)kvh * ((n_tok + ATC_KEYS - 1) / ATC_KEYS) * ATC_IMG_BYTES;
 
     if (threadIdx.x == 0) {
-        for (int b = 0; b < 5; ++b) mbar_init(qk1 + b, 1);
+        mbar_init(qk, 2);                                                // an arrival of each issuing warp
+        for (int b = 1; b < 4; ++b) mbar_init(qk + b, 1);
         mbar_fence_init();
     }
     if (warp == 0) {
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
     }
     const uint32_t tmem = *tmem_slot;
     const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-    // The tensor core's instructions, one elected lane of warp 0 (the code stays warp-uniform).  Products with a low plane
+    // The tensor core's instructions, one elected lane of warp 0 or 1 (the code stays warp-uniform).  Products with a low plane
     // come first: the accumulator is small while they are added.
     // One sum of the scores: 16-dim steps n0 .. n0 + STEPS - 1 into 64 columns at d.
     auto sum_of = [&](uint32_t d, auto n0c, auto stepsc) {
@@ -319,23 +320,32 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
 #pragma unroll
         for (int n = N0; n < N0 + STEPS; ++n) atc_mma_ss<atc_idesc(ATC_KEYS)>(d, a0 + at(n), b0 + at(n));
     };
+    // Two warps issue the scores' products, half of the sums each: from one warp 16 dims take 39 (q low) or 55 cycles, and its chain of waits and
+    // issues is not overlapped.  (One warp, a barrier for each half of the dims, waits polled back to back: 2048 tokens 287 us, 600 tokens 60.6;
+    // now 279 and 58.9.)
     auto issue_qk_a = [&] {                                              // dims 0 .. 63, two sums, into the score columns
         tc_fence_after();
-        if (elect_one()) {
-            sum_of(tmem + ATC_COL_S, std::integral_constant<int, 0>{}, std::integral_constant<int, 2>{});
-            sum_of(tmem + ATC_COL_S + ATC_KEYS, std::integral_constant<int, 2>{}, std::integral_constant<int, 2>{});
-            tc_commit(qk1);
+        if (warp == 0) {
+            if (elect_one()) sum_of(tmem + ATC_COL_S, std::integral_constant<int, 0>{}, std::integral_constant<int, 2>{});
+        } else {
+            if (elect_one()) sum_of(tmem + ATC_COL_S + ATC_KEYS, std::integral_constant<int, 2>{}, std::integral_constant<int, 2>{});
         }
         __syncwarp();
     };
-    auto issue_qk_b = [&] {                                              // dims 64 .. 255, four sums, into the output columns
+    auto issue_qk_b = [&] {                                              // dims 64 .. 255, four sums, into the output columns; the commit covers the others too
         tc_fence_after();
-        if (elect_one()) {
-            sum_of(tmem + ATC_COL_O, std::integral_constant<int, 4>{}, std::integral_constant<int, 3>{});
-            sum_of(tmem + ATC_COL_O + ATC_KEYS, std::integral_constant<int, 7>{}, std::integral_constant<int, 3>{});
-            sum_of(tmem + ATC_COL_O + 2 * ATC_KEYS, std::integral_constant<int, 10>{}, std::integral_constant<int, 3>{});
-            sum_of(tmem + ATC_COL_O + 3 * ATC_KEYS, std::integral_constant<int, 13>{}, std::integral_constant<int, 3>{});
-            tc_commit(qk2);
+        if (warp == 0) {
+            if (elect_one()) {
+                sum_of(tmem + ATC_COL_O, std::integral_constant<int, 4>{}, std::integral_constant<int, 3>{});
+                sum_of(tmem + ATC_COL_O + ATC_KEYS, std::integral_constant<int, 7>{}, std::integral_constant<int, 3>{});
+                tc_commit(qk);
+            }
+        } else {
+            if (elect_one()) {
+                sum_of(tmem + ATC_COL_O + 2 * ATC_KEYS, std::integral_constant<int, 10>{}, std::integral_constant<int, 3>{});
+                sum_of(tmem + ATC_COL_O + 3 * ATC_KEYS, std::integral_constant<int, 13>{}, std::integral_constant<int, 3>{});
+                tc_commit(qk);
+            }
         }
         __syncwarp();
     };
@@ -365,8 +375,8 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
     tc_fence_before();
     __syncthreads();
     bool ok = true;
-    if (warp == 0) {
-        ok = mbar_wait_hot(kfull, 0);
+    if (warp < 2) {
+        ok = mbar_wait_try(kfull, 0);
         issue_qk_a();
         issue_qk_b();
     }
@@ -398,9 +408,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
         const int j0 = i * ATC_KEYS;
         const uint32_t par = (uint32_t)(i & 1);
         float s[16], mx = -INFINITY;
-        ok = mbar_wait_hot(kfull, par) && ok;                            // (long complete; makes the copied factors visible)
-        ok = mbar_wait_hot(qk1, par) && ok;
-        ok = mbar_wait_hot(qk2, par) && ok;
+        ok = mbar_wait_both(kfull, par, qk, par) && ok;                  // (the first is long complete; it makes the copied factors visible)
         tc_fence_after();
         {
             // (eight columns at a time: sixteen of two sums beside the outputs and the scores were more registers than a thread has, and what is
@@ -453,16 +461,16 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
             tc_st8(tlane + ATC_COL_S + (uint32_t)(32 + 8 * cg), lo);
         }
         tc_st_wait();
-        ok = mbar_wait_hot(vfull, par) && ok;                            // in front of the CTA's barrier: load_v below begins the next phase
+        ok = mbar_wait_try(vfull, par) && ok;                            // in front of the CTA's barrier: load_v below begins the next phase
         tc_fence_before();
         __syncthreads();
         if (warp == 0) issue_pv();
-        ok = mbar_wait_hot(pv, par) && ok;
+        ok = mbar_wait_try(pv, par) && ok;
         tc_fence_after();
         if (i + 1 < ntiles) {
             if (warp == 4 && lane == 0) load_v(i + 1);
-            if (warp == 0) {
-                ok = mbar_wait_hot(kfull, par ^ 1u) && ok;
+            if (warp < 2) {
+                ok = mbar_wait_try(kfull, par ^ 1u) && ok;
                 issue_qk_a();
             }
         }
@@ -470,7 +478,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
         if (i + 1 < ntiles) {
             tc_fence_before();
             __syncthreads();                                             // the output columns have been read: scores may go there
-            if (warp == 0) issue_qk_b();
+            if (warp < 2) issue_qk_b();
         }
     }
     __syncthreads();
