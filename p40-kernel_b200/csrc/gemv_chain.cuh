@@ -33,7 +33,7 @@
 // compute warp has left ops [0, ops_done)), ops_loaded, issued, copy_op.  Slot release is a plain
 // counter too, because the number of tasks per tile changes from op to op.
 // Every wait is bounded: a second or so by counted polls with sleeps (the copy, sequencer and peer warps, the ring), some three seconds
-// for other CTAs (grid_counter_wait; two for the words of an image), the caller's limit for other ranks, and for warps that wait for each other's part of these until
+// for other CTAs (grid_counter_wait; five for the words of an image), the caller's limit for other ranks, and for warps that wait for each other's part of these until
 // one of them has given up.  A time-out sets the status word and the warp leaves.
 #pragma once
 
@@ -65,7 +65,11 @@ constexpr uint32_t CHAIN_GATE_NS0 = 32, CHAIN_GATE_NSMAX = 256;   // ... of the 
 // The warps of a CTA that wait for each other, or for what one lane of them waits for, leave when that lane has given up (ctrl[14]); should it
 // say nothing either, after this time (several ranks: and their own limit).
 constexpr uint32_t CHAIN_WAIT_MS = 8000;
-constexpr uint32_t CHAIN_IMAGE_POLLS = 1u << 21;                  // trips to L2 with sleeps of 32 ns, some two seconds, that a warp waits for a spread op's image
+// Trips to L2 and back with sleeps between them: 32 to 64 ns for the rows of other CTAs, some three seconds in all; 32 ns for the words of a
+// spread op's image, some five.  The CTA that writes a part of an image waits for other CTAs' rows first, so its readers wait longer, and the
+// warps of a reader's CTA longer still.
+constexpr uint32_t CHAIN_GRID_POLLS = 8u << 19, CHAIN_IMAGE_POLLS = 11u << 19;
+static_assert(4 * (uint64_t)CHAIN_IMAGE_POLLS >= 5 * (uint64_t)CHAIN_GRID_POLLS, "who waits for a waiter waits longer");
 constexpr int CHAIN_GATES = 3;           // a warp may run this many ops ahead of the slowest one
 
 struct __align__(16) ChainOp {                 // 128 bytes, one per projection, device table
@@ -137,7 +141,7 @@ __device__ __forceinline__ bool spin_until_eq(volatile int *p, int v) {
 // to 64 ns between them, some three seconds.  Counters only grow, so "reached" is a wrap-safe signed difference.
 __device__ __forceinline__ bool grid_counter_wait(const unsigned int *counter, unsigned int target) {
     uint32_t ns = CHAIN_NS0;
-    for (uint32_t n = 0; n < (1u << 22); ++n) {
+    for (uint32_t n = 0; n < CHAIN_GRID_POLLS; ++n) {
         unsigned int v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
         if ((int)(v - target) >= 0) return true;
