@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
 #pragma unroll
                                     for (int k = 0; k < BATCH; ++k) there = there && (uint32_t)(w[k][0] >> 32) == tag && (uint32_t)(w[k][1] >> 32) == tag;
                                     if (__all_sync(0xffffffffu, there)) break;
-                                    if (polls >= CHAIN_IMAGE_POLLS || *stop) { ok = false; break; }
+                                    if (polls >= CHAIN_IMAGE_POLLS || __any_sync(0xffffffffu, *stop)) { ok = false; break; }      // (each lane reads *stop for itself)
                                     __nanosleep(CHAIN_NS0);
                                 }
                                 if (!ok) break;

@@ -19,3 +19,17 @@ def test_an_image_is_waited_for_longer_than_its_writer_waits():
     polls = {name: value(v) for name, v in re.findall(r"\b(CHAIN_\w+_POLLS) = ([^,;]+)", SOURCE)}
     writer = re.search(r"n < \(?([^;)]+)\)?;", function("bool grid_counter_wait("))[1]
     assert 4 * polls["CHAIN_IMAGE_POLLS"] >= 5 * (polls[writer] if writer in polls else value(writer))
+
+
+def image_poll():
+    loop = SOURCE[SOURCE.index("image_load2(table_image"):]
+    return loop[:loop.index("__nanosleep(")]
+
+
+def test_a_warp_leaves_the_poll_of_an_image_as_a_whole():
+    """The poll votes with all 32 lanes, and what one lane reads of another warp's word may not be what its neighbour reads."""
+    exits = [line for line in image_poll().splitlines() if "break;" in line]
+    assert len(exits) >= 2
+    for line in exits:
+        alone = re.sub(r"__(all|any)_sync\(0xffffffffu, [^()]*\)", "", line.split("//")[0])
+        assert "there" not in alone and "stop" not in alone, line
