@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                 }
                             }
                             if (!ok) {
-                                if (lane == 0) atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);
+                                if (lane == 0 && !*stop) atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);      // (else: whoever set it has said why)
                                 alive = false;
                                 break;
                             }

@@ -33,3 +33,10 @@ def test_a_warp_leaves_the_poll_of_an_image_as_a_whole():
     for line in exits:
         alone = re.sub(r"__(all|any)_sync\(0xffffffffu, [^()]*\)", "", line.split("//")[0])
         assert "there" not in alone and "stop" not in alone, line
+
+
+def test_a_poll_that_ends_for_another_warp_reports_nothing():
+    """A warp that was told to leave (*stop) does not write over what the one that gave up has put into the status word."""
+    after = SOURCE[SOURCE.index("image_load2(table_image"):]
+    report = next(line for line in after.splitlines() if "STATUS_GRID_TIMEOUT" in line)
+    assert re.search(r"if \(lane == 0 && !\*stop\)", report), report
