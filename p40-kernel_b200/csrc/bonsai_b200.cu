@@ -94,6 +94,54 @@ cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Launches in clusters of CTAs, which a device, a limit on its SMs or a tool may refuse (a profiler that replays kernels: cooperative ones).
+std::atomic<int> g_opt_refuse_clusters{0};        // test build: so many of them are refused without being tried
+template <typename... KArgs, typename... Args>
+cudaError_t launch_clusters(const cudaLaunchConfig_t &cfg, void (*kernel)(KArgs...), Args... args) {
+    if (g_opt_refuse_clusters.load() > 0 && g_opt_refuse_clusters.fetch_sub(1) > 0) return cudaErrorInvalidConfiguration;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+// Clusters of a kernel that are resident at once with an SM for each CTA, per device: asked once; none from the first launch on that was refused.
+class ClusterRoom {
+public:
+    template <typename K>
+    int ask(K kernel, SmemOptIn &opt, unsigned cluster, unsigned threads) {
+        int dev = 0, resident = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
+        if ((resident = known_[dev].load(std::memory_order_relaxed)) != 0) return std::max(resident, 0);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(SM_COUNT / cluster * cluster);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = SMEM_LIMIT;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = cluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (opt.ensure(kernel) != cudaSuccess || cudaOccupancyMaxActiveClusters(&resident, kernel, &cfg) != cudaSuccess || resident <= 0) {
+            (void)cudaGetLastError();
+            resident = -1;
+        }
+        known_[dev].store(resident, std::memory_order_relaxed);
+        return std::max(resident, 0);
+    }
+    // Whether e says that clusters are not launched here; no later call tries them then.
+    bool refused(cudaError_t e) {
+        if (e != cudaErrorInvalidConfiguration && e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return false;
+        (void)cudaGetLastError();
+        int dev = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess && dev < 64) known_[dev].store(-1, std::memory_order_relaxed);
+        return true;
+    }
+    void forget() {
+        for (auto &k : known_) k.store(0, std::memory_order_relaxed);
+    }
+
+private:
+    std::atomic<int> known_[64] = {};
+};
+
 // ceil(2^32 / d): __umulhi(n, magic) == n / d for every n with n * d < 2^32; 0 stands for d == 1.
 inline uint32_t magic_u32(uint32_t d) {
     if (d <= 1) return 0u;
@@ -989,33 +1037,10 @@ static size_t tc16_scratch_bytes(int64_t n_in, int64_t n_tok) {
     return T16_FLAGS_BYTES + T16_PARTS_BYTES + 2 * (size_t)n_tok * (size_t)n_in * sizeof(__half) + (size_t)n_tok * sizeof(float);
 }
 
-// The fp16 tensor-core mat-mul (gemm_tc16.cuh).  -1: not taken (shape, alignment, no scratch, no tensor-map encoder, no SMs in pairs or no launch of them).
+// The fp16 tensor-core mat-mul (gemm_tc16.cuh).  -1: not taken (shape, alignment, no scratch, no tensor-map encoder).
 extern "C++" {
-// Pairs of CTAs that are resident at once on the current device (0: they do not run here).  Asked once per device.
-static int tc16_pairs() {
-    static std::atomic<int> known[64];
-    auto *kernel = gemm_tc16_kernel<128, 2>;
-    static SmemOptIn opt;
-    int dev = 0, resident = 0;
-    if (opt.ensure(kernel) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (dev < 64 && (resident = known[dev].load(std::memory_order_relaxed)) != 0) return std::max(resident, 0);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(TC_MAX_CTAS);
-    cfg.blockDim = dim3(T16C<128, 2>::THREADS);
-    cfg.dynamicSmemBytes = T16C<128, 2>::SMEM_BYTES;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&resident, kernel, &cfg) != cudaSuccess || resident <= 0) {
-        (void)cudaGetLastError();
-        resident = -1;
-    }
-    if (dev < 64) known[dev].store(resident, std::memory_order_relaxed);
-    return std::max(resident, 0);
-}
+static ClusterRoom g_tc16_pairs;
+static SmemOptIn g_tc16_pairs_smem;
 
 // How a mat-mul is divided over `workers` CTAs (or pairs of them), and about how long that takes.
 struct Tc16Plan {
@@ -1048,59 +1073,37 @@ static Tc16Plan plan_tc16(int64_t n_out, int64_t nblocks, int64_t n_tok, int wor
 }
 static int tc16_workers(int ctas) {
     int dev = 0, sms = 0;
-    if (ctas != 1) return std::min(tc16_pairs(), (TC_MAX_CTAS - 1) / ctas);
+    if (ctas != 1) return std::min(g_tc16_pairs.ask(gemm_tc16_kernel<128, 2>, g_tc16_pairs_smem, 2, T16C<128, 2>::THREADS), (TC_MAX_CTAS - 1) / ctas);
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
     return std::min(sms, TC_MAX_CTAS - 1);
 }
 
+// One launch over activations that lie in `planes`.
+struct Tc16Args {
+    float *Y;
+    int64_t n_out, nblocks, n_tok;
+    const float *scale;
+    float *parts;
+    unsigned int *flags;
+    Tc16Maps maps;
+};
 template <int TN, int CTAS>
-static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n_out, int64_t n_in, int64_t n_tok, cudaStream_t st) {
-    const int64_t nblocks = n_in / 128;
-    if (nblocks % 8 != 0 || !aligned16(W) || !aligned4(Xq) || n_tok > (1 << 28)) return -1;
-    const int workers = tc16_workers(CTAS), sms = tc16_workers(1);
-    if (workers <= 0) return -1;
-    const Tc16Plan plan = plan_tc16<TN, CTAS>(n_out, nblocks, n_tok, workers);
-    if (plan.tiles > INT32_MAX) return -1;
-    cudaError_t e;
-    const size_t plane_bytes = (size_t)n_tok * (size_t)n_in * sizeof(__half);
-    const StreamScratch::Lease lease = g_gemm_scratch.get(tc16_scratch_bytes(n_in, n_tok), st);      // held until both launches are enqueued
-    uint8_t *ws = static_cast<uint8_t *>(lease.ptr);
-    if (!ws) return -1;
-    unsigned int *flags = reinterpret_cast<unsigned int *>(ws);
-    float *parts = reinterpret_cast<float *>(ws + T16_FLAGS_BYTES);
-    __half *planes = reinterpret_cast<__half *>(ws + T16_FLAGS_BYTES + T16_PARTS_BYTES);
-    float *scale = reinterpret_cast<float *>(ws + T16_FLAGS_BYTES + T16_PARTS_BYTES + 2 * plane_bytes);
-    alignas(64) Tc16Maps maps;
-    std::memset(&maps, 0, sizeof(maps));
-    if (!encode_w_map(&maps.w, W, n_out, nblocks * W_BLOCK_BYTES)) return -1;
-    if (!tensor_map_planes(&maps.x, planes, (uint64_t)n_in, (uint64_t)n_tok, (uint32_t)(plan.tile_n / CTAS))) return -1;
+static cudaError_t launch_gemm_tc16_n(const Tc16Args &a, const Tc16Plan &plan, SmemOptIn &opt, cudaStream_t st) {
     T16Params P{};
-    P.n_out = (int)n_out;
-    P.nblocks = (int)nblocks;
-    P.n_tok = (int)n_tok;
+    P.n_out = (int)a.n_out;
+    P.nblocks = (int)a.nblocks;
+    P.n_tok = (int)a.n_tok;
     P.tile_n = plan.tile_n;
     P.tiles_tok = (int)plan.tiles_tok;
     P.n_tiles = (int)plan.tiles;
     P.idesc = t16_idesc(plan.tile_n, CTAS);
     P.stream_k = plan.stream_k;
-    const int grid = plan.grid;
-    P.per_worker = plan.tiles * nblocks / grid;
-    P.rest = (int)(plan.tiles * nblocks % grid);
-    const int n_chunks = (int)(n_in / 32);
-    const uint32_t *x32 = static_cast<const uint32_t *>(Xq);
-    // slices: whole passes of a block, as many as bring about two blocks per SM
-    const long long groups = (n_tok + 3) / 4;
-    int passes = (n_chunks + T16_SPLIT_PASS - 1) / T16_SPLIT_PASS;
-    passes = (int)((passes * groups + 2 * sms - 1) / (2 * sms));
-    const int slice = passes * T16_SPLIT_PASS;
-    static SmemOptIn opt;
-    e = opt.ensure(gemm_tc16_kernel<TN, CTAS>);
-    if (e != cudaSuccess) return (int)e;
-    e = launch(groups <= 2 * sms ? tc16_split_kernel<true> : tc16_split_kernel<false>, dim3((unsigned)groups, (unsigned)((n_chunks + slice - 1) / slice)),
-               dim3(T16_SPLIT_THREADS), 0, st, true, x32, n_chunks, (int)n_tok, slice, scale, planes);
-    if (e != cudaSuccess) return (int)e;
+    P.per_worker = plan.tiles * a.nblocks / plan.grid;
+    P.rest = (int)(plan.tiles * a.nblocks % plan.grid);
+    cudaError_t e = opt.ensure(gemm_tc16_kernel<TN, CTAS>);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(grid * CTAS));
+    cfg.gridDim = dim3((unsigned)(plan.grid * CTAS));
     cfg.blockDim = dim3(T16C<TN, CTAS>::THREADS);
     cfg.dynamicSmemBytes = T16C<TN, CTAS>::SMEM_BYTES;
     cfg.stream = st;
@@ -1112,26 +1115,50 @@ static int launch_gemm_tc16_n(const void *W, const void *Xq, float *Y, int64_t n
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = CTAS == 1 ? 1 : 2;
-    e = cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN, CTAS>, Y, P, (const float *)scale, parts, flags, maps);
-    if (CTAS != 1 && (e == cudaErrorInvalidConfiguration || e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
-        (void)cudaGetLastError();                        // a cooperative launch in clusters is refused, by a profiler that replays it for instance
-        return -1;
-    }
-    return (int)e;
+    if (CTAS != 1) return launch_clusters(cfg, gemm_tc16_kernel<TN, CTAS>, a.Y, P, a.scale, a.parts, a.flags, a.maps);
+    return cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN, CTAS>, a.Y, P, a.scale, a.parts, a.flags, a.maps);
 }
 }  // extern "C++"
 // Tiles of up to 64 tokens by a CTA, or of up to 128 by a pair of CTAs (the code expansion is paid once per tile, and each CTA fetches half
 // of the activations): what the plans say takes less time.  (us, a CTA / a pair: 64 tokens of 5120 -> 17408 26.8 / 30.8, 65 44.5 / 33.7, 129
 // 61.7 / 59.6; of 5120 -> 5120, where pairs have too few tiles, 64 22.5 / 24.7, 128 25.3 / 29.0; 129 of 1024 -> 12288 20.6 / 22.9.)
 static int launch_gemm_tc16(const void *W, const void *Xq, float *Y, int64_t n_out, int64_t n_in, int64_t n_tok, cudaStream_t st) {
-    const int tile = g_opt_gemm_tile.load(), ones = tc16_workers(1), pairs = n_tok > 64 || tile == 128 ? tc16_workers(2) : 0;
-    if (ones <= 0) return -1;
-    if (tile != 64 && pairs > 0 &&
-        (tile == 128 || plan_tc16<128, 2>(n_out, n_in / 128, n_tok, pairs).ns < plan_tc16<64, 1>(n_out, n_in / 128, n_tok, ones).ns)) {
-        const int rc = launch_gemm_tc16_n<128, 2>(W, Xq, Y, n_out, n_in, n_tok, st);
-        if (rc >= 0) return rc;
+    const int64_t nblocks = n_in / 128;
+    if (nblocks % 8 != 0 || !aligned16(W) || !aligned4(Xq) || n_tok > (1 << 28)) return -1;
+    const int tile = g_opt_gemm_tile.load(), sms = tc16_workers(1), pairs = tile != 64 && (n_tok > 64 || tile == 128) ? tc16_workers(2) : 0;
+    if (sms <= 0) return -1;
+    const Tc16Plan one = plan_tc16<64, 1>(n_out, nblocks, n_tok, sms);
+    Tc16Plan two;
+    if (pairs > 0) two = plan_tc16<128, 2>(n_out, nblocks, n_tok, pairs);
+    const bool paired = pairs > 0 && two.tiles <= INT32_MAX && (tile == 128 || two.ns < one.ns);
+    if (one.tiles > INT32_MAX) return -1;
+    const size_t plane_bytes = (size_t)n_tok * (size_t)n_in * sizeof(__half);
+    const StreamScratch::Lease lease = g_gemm_scratch.get(tc16_scratch_bytes(n_in, n_tok), st);      // held until the launches are enqueued
+    uint8_t *ws = static_cast<uint8_t *>(lease.ptr);
+    if (!ws) return -1;
+    __half *planes = reinterpret_cast<__half *>(ws + T16_FLAGS_BYTES + T16_PARTS_BYTES);
+    float *scale = reinterpret_cast<float *>(ws + T16_FLAGS_BYTES + T16_PARTS_BYTES + 2 * plane_bytes);
+    alignas(64) Tc16Args a{Y, n_out, nblocks, n_tok, scale, reinterpret_cast<float *>(ws + T16_FLAGS_BYTES), reinterpret_cast<unsigned int *>(ws), {}};
+    auto map_activations = [&](int tokens) { return tensor_map_planes(&a.maps.x, planes, (uint64_t)n_in, (uint64_t)n_tok, (uint32_t)tokens); };
+    if (!encode_w_map(&a.maps.w, W, n_out, nblocks * W_BLOCK_BYTES) || !map_activations(paired ? two.tile_n / 2 : one.tile_n)) return -1;
+    const int n_chunks = (int)(n_in / 32);
+    const uint32_t *x32 = static_cast<const uint32_t *>(Xq);
+    // slices: whole passes of a block, as many as bring about two blocks per SM
+    const int groups = (int)((n_tok + 3) / 4);
+    int passes = (n_chunks + T16_SPLIT_PASS - 1) / T16_SPLIT_PASS;
+    passes = (int)((passes * groups + 2 * sms - 1) / (2 * sms));
+    const int slice = passes * T16_SPLIT_PASS;
+    cudaError_t e = launch(groups <= 2 * sms ? tc16_split_kernel<true> : tc16_split_kernel<false>,
+                           dim3((unsigned)groups, (unsigned)((n_chunks + slice - 1) / slice)), dim3(T16_SPLIT_THREADS), 0, st, true, x32, n_chunks, (int)n_tok, slice,
+                           scale, planes);
+    if (e != cudaSuccess) return (int)e;
+    if (paired) {
+        e = launch_gemm_tc16_n<128, 2>(a, two, g_tc16_pairs_smem, st);
+        if (!g_tc16_pairs.refused(e)) return (int)e;
+        if (!map_activations(one.tile_n)) return -1;      // the same planes, by single CTAs: here, and in later calls from the start
     }
-    return launch_gemm_tc16_n<64, 1>(W, Xq, Y, n_out, n_in, n_tok, st);
+    static SmemOptIn opt;
+    return (int)launch_gemm_tc16_n<64, 1>(a, one, opt, st);
 }
 
 // The tensor-core mat-mul: one CTA per SM walks its share of the (tile, weight block) iterations.
@@ -1445,6 +1472,12 @@ int bonsai_b200_set_option(const char *key, int64_t value) {
     if (!std::strcmp(key, "gemm_tile")) {
         if (value != 0 && value != 64 && value != 128) return 1;
         g_opt_gemm_tile.store((int)value);
+        return 0;
+    }
+    if (!std::strcmp(key, "refuse_clusters")) {         // 0 forgets the refusals too
+        if (value < 0) return 1;
+        g_opt_refuse_clusters.store((int)value);
+        if (value == 0) g_tc16_pairs.forget();
         return 0;
     }
     if (!std::strcmp(key, "kv_wide")) { g_opt_kv_wide.store(value != 0); return 0; }

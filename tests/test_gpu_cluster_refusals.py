@@ -1,0 +1,45 @@
+"""Calls that launch clusters of CTAs where a device lets them, when a launch of clusters is refused: the call runs in the form that needs none
+with what it has enqueued so far, and later calls do not try again.  The kernels of a call are read from a capture of it."""
+import numpy as np
+import pytest
+
+from bonsai_b200 import synth
+from captured import launches
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def refuse(gpu):
+    assert gpu.set_option("refuse_clusters", 0) == 0
+    yield lambda n: gpu.set_option("refuse_clusters", n)
+    gpu.set_option("refuse_clusters", 0)
+
+
+def test_matmul(gpu, port, refuse):
+    """Two launches, the activations split once: refused in the capture, refused in the call in front of it and remembered, and not refused."""
+    import torch
+    n_out, n_in, n_tok = 300, 2048, 200
+    W, X = synth.pq2_0_weights(n_out, n_in, seed=1), synth.activations(n_in, seed=2, batch=n_tok)
+    Xq = port.quantize_batch_chunk_major(X)
+    Wd, Xqd, Y = torch.from_numpy(W).cuda(), torch.from_numpy(Xq).cuda(), torch.zeros(n_out, n_tok, device="cuda")
+    want = port.gemm(W, Xq, n_out, n_in, n_tok, threads=8)
+    call = lambda: gpu.gemm(Wd, Xqd, Y, n_out, n_in, n_tok)
+
+    def right():
+        ok = np.abs(Y.cpu().numpy() - want).max() <= 1e-5 * np.abs(want).max()
+        Y.fill_(float("nan"))
+        return ok
+
+    try:
+        assert gpu.set_option("gemm_tile", 128) == 0
+        assert launches(call) == [1, 2] and right()
+        assert launches(call, lambda: refuse(1)) == [1, 1] and right()
+        assert refuse(0) == 0
+        assert launches(call) == [1, 2] and right()
+        assert refuse(1) == 0
+        assert launches(call) == [1, 1] and right()
+        assert call() == 0 and right()
+    finally:
+        gpu.set_option("gemm_tile", 0)
+    assert gpu.device_status() == 0
