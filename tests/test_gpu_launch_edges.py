@@ -92,15 +92,20 @@ def test_token_batches_read_what_the_call_before_wrote(gpu, n_tok, offset):
 
 @pytest.mark.parametrize("n_out,n_in,n_tok", [
     (128, 17408, 17), (129, 17408, 64), (5120, 17408, 37), (1000, 5120, 33), (2000, 17408, 95), (300, 17408, 96), (1030, 9216, 130), (6000, 5120, 257)])
-def test_parts_of_a_tile_add_up(gpu, port, n_out, n_in, n_tok):
-    """Tiles of the many-token mat-mul in one, two, three and four parts, on both tile widths."""
+@pytest.mark.parametrize("tile", [0, 64, 128])
+def test_parts_of_a_tile_add_up(gpu, port, tile, n_out, n_in, n_tok):
+    """Tiles of the many-token mat-mul in one to five parts: as the call divides them, and on each tile width."""
     import torch
     W = synth.pq2_0_weights(n_out, n_in, seed=n_tok)
     Xq = port.quantize_batch_chunk_major(synth.activations(n_in, seed=n_out, batch=n_tok))
     Wd, Xd = dev(W), dev(Xq)
     Y = [torch.full((n_out, n_tok), float("nan"), device="cuda") for _ in range(2)]
-    for y in Y:
-        assert gpu.gemm(Wd, Xd, y, n_out, n_in, n_tok) == 0
+    try:
+        assert gpu.set_option("gemm_tile", tile) == 0
+        for y in Y:
+            assert gpu.gemm(Wd, Xd, y, n_out, n_in, n_tok) == 0
+    finally:
+        gpu.set_option("gemm_tile", 0)
     assert torch.equal(Y[0], Y[1])
     rows = np.unique(np.concatenate([np.arange(min(n_out, 64)), np.arange(max(0, n_out - 64), n_out), np.linspace(0, n_out - 1, 64).astype(np.int64)]))
     row_bytes = n_in // 128 * 34
