@@ -142,6 +142,8 @@ private:
     std::atomic<int> known_[64] = {};
 };
 
+ClusterRoom g_tc16_pairs, g_repack_pairs, g_repack_fours;
+
 // ceil(2^32 / d): __umulhi(n, magic) == n / d for every n with n * d < 2^32; 0 stands for d == 1.
 inline uint32_t magic_u32(uint32_t d) {
     if (d <= 1) return 0u;
@@ -1039,7 +1041,6 @@ static size_t tc16_scratch_bytes(int64_t n_in, int64_t n_tok) {
 
 // The fp16 tensor-core mat-mul (gemm_tc16.cuh).  -1: not taken (shape, alignment, no scratch, no tensor-map encoder).
 extern "C++" {
-static ClusterRoom g_tc16_pairs;
 static SmemOptIn g_tc16_pairs_smem;
 
 // How a mat-mul is divided over `workers` CTAs (or pairs of them), and about how long that takes.
@@ -1346,34 +1347,48 @@ int bonsai_p40_gemv_repack(const void *W, const float *x, float *y, int64_t n_ou
         StreamParams sp;
         int threads = 0, smem_bytes = 0;
         if (tree && vec && n_in % FWHT_N == 0 && plan_stream(n_out, nb, g_opt_gemv_variant.load(), sp, threads, smem_bytes)) {
-            // Long rows: the CTAs of a cluster share the quantiser.  In fours while they are few enough to leave no SM to two of them (clusters do
-            // not cross a group of SMs; 147 CTAs in fours ran two to an SM in places and took twice as long), else in pairs, whose
-            // barrier is worth it from 96 blocks on.  us, alone / in pairs / in fours: 17408 -> 64 6.96 / 5.62 / 4.82, -> 1000 7.66 / 6.66 / 6.00, -> 5120
-            // 11.7 / 10.7 / 18.7; 12288 -> 5120 9.06 / 9.00 / 16.0; 9216 -> 5120 7.43 / 8.10; 5120 -> 64 3.57 / 3.57 / 3.20, -> 1000 3.96 / 4.16 / 3.83.
+            // Long rows: the CTAs of a cluster share the quantiser.  In fours where each of their CTAs finds an SM (clusters do not cross a group of
+            // SMs: 147 CTAs in fours ran two to an SM in places and took twice as long), else in pairs, whose barrier is worth it from 96
+            // blocks on.  us, alone / in pairs / in fours: 17408 -> 64 6.94 / 5.60 / 4.80, -> 1000 7.65 / 6.63 / 5.99, -> 5120 11.75 / 10.69 / 18.7;
+            // 12288 -> 1056 6.14 / 6.05 / 5.19, -> 4096 8.49 / 8.37 / 14.8, -> 5120 9.04 / 8.97, -> 17408 17.97 / 17.77; 11264 -> 5120 8.42 / 8.45;
+            // 5120 -> 64 3.55 / 3.55 / 3.18, -> 1056 3.96 / 4.16 / 3.81.  Fours with more than 28 rows per CTA are worth it from 80 blocks on: -> 4160,
+            // alone / in fours and the same behind the rotation, 5120 4.54 / 5.13, 6.53 / 6.75; 9216 6.78 / 7.28, 8.79 / 8.80; 10240 7.38 / 7.37, 9.41 / 8.90.
+            // (At 16 to 28 rows and 40 to 72 blocks fours are up to 7 % behind alone and up to 6 % ahead behind the rotation.)
+            static SmemOptIn sopt[3];
             const unsigned ctas = (unsigned)((n_out + sp.rows_per_cta - 1) / sp.rows_per_cta);
-            const unsigned cl = ctas <= 128 && nb >= 40 ? 4 : nb >= 96 ? 2 : 1;
+            auto room = [&](ClusterRoom &r, auto kernel, SmemOptIn &o, unsigned cluster) { return ctas <= cluster * (unsigned)r.ask(kernel, o, cluster, 512); };
+            unsigned cl = 1;
+            if (nb >= (sp.rows_per_cta <= 28 ? 40 : 80) && room(g_repack_fours, gemv_stream_kernel<true, true, 4>, sopt[2], 4)) cl = 4;
+            else if (nb >= 96 && room(g_repack_pairs, gemv_stream_kernel<true, true, 2>, sopt[1], 2)) cl = 2;
             sp.early = pdl;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((ctas + cl - 1) / cl * cl);
-            cfg.blockDim = dim3(threads);
-            cfg.dynamicSmemBytes = (size_t)smem_bytes;
-            cfg.stream = as_stream(stream);
             cudaLaunchAttribute attr[2];
             attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = cl;
             attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
             attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr[1].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = cl == 1 ? attr + 1 : attr;
-            cfg.numAttrs = (cl > 1) + (g_opt_overlap.load() != 0);
-            static SmemOptIn sopt[3];
-            auto go = [&](auto kernel, SmemOptIn &o) -> int {
+            cudaLaunchConfig_t cfg = {};
+            cfg.blockDim = dim3(threads);
+            cfg.dynamicSmemBytes = (size_t)smem_bytes;
+            cfg.stream = as_stream(stream);
+            auto go = [&](auto kernel, SmemOptIn &o) -> cudaError_t {
                 cudaError_t err = o.ensure(kernel);
-                if (err != cudaSuccess) return (int)err;
-                return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<const uint8_t *>(W), static_cast<const uint32_t *>(nullptr), y, sp, x,
-                                               static_cast<const float *>(nullptr), static_cast<uint32_t *>(nullptr));
+                if (err != cudaSuccess) return err;
+                attr[0].val.clusterDim.x = cl;
+                cfg.gridDim = dim3((ctas + cl - 1) / cl * cl);
+                cfg.attrs = cl == 1 ? attr + 1 : attr;
+                cfg.numAttrs = (cl > 1) + (g_opt_overlap.load() != 0);
+                const uint8_t *w8 = static_cast<const uint8_t *>(W);
+                const uint32_t *no_xq = nullptr;
+                const float *no_signs = nullptr;
+                uint32_t *no_out = nullptr;
+                return cl > 1 ? launch_clusters(cfg, kernel, w8, no_xq, y, sp, x, no_signs, no_out) : cudaLaunchKernelEx(&cfg, kernel, w8, no_xq, y, sp, x, no_signs, no_out);
             };
-            return cl == 4 ? go(gemv_stream_kernel<true, true, 4>, sopt[2]) : cl == 2 ? go(gemv_stream_kernel<true, true, 2>, sopt[1]) : go(gemv_stream_kernel<true, true>, sopt[0]);
+            if (cl > 1) {
+                const cudaError_t err = cl == 4 ? go(gemv_stream_kernel<true, true, 4>, sopt[2]) : go(gemv_stream_kernel<true, true, 2>, sopt[1]);
+                if (!g_repack_fours.refused(err) || !g_repack_pairs.refused(err)) return (int)err;
+                cl = 1;
+            }
+            return (int)go(gemv_stream_kernel<true, true>, sopt[0]);
         }
     }
     auto pick = [&](auto t, auto v, int base) -> cudaError_t {
@@ -1477,7 +1492,7 @@ int bonsai_b200_set_option(const char *key, int64_t value) {
     if (!std::strcmp(key, "refuse_clusters")) {         // 0 forgets the refusals too
         if (value < 0) return 1;
         g_opt_refuse_clusters.store((int)value);
-        if (value == 0) g_tc16_pairs.forget();
+        if (value == 0) g_tc16_pairs.forget(), g_repack_pairs.forget(), g_repack_fours.forget();
         return 0;
     }
     if (!std::strcmp(key, "kv_wide")) { g_opt_kv_wide.store(value != 0); return 0; }

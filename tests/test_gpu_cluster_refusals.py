@@ -43,3 +43,30 @@ def test_matmul(gpu, port, refuse):
     finally:
         gpu.set_option("gemm_tile", 0)
     assert gpu.device_status() == 0
+
+
+# (how many fours find an SM for each CTA is the device's: 33 on the one that was looked at)
+@pytest.mark.parametrize("n_out,n_in,forms", [(400, 17408, [4]), (400, 5120, [4]), (1024, 5120, [4, 1]), (1060, 5120, [4, 1]), (5120, 17408, [2]), (4160, 9216, [1]),
+                                              (4160, 10240, [4, 1]), (4150, 12288, [4, 2]), (5120, 11264, [1]), (700, 4096, [1])])
+def test_repacked_matvec(gpu, refuse, n_out, n_in, forms):
+    """Fours as far as they find an SM for each CTA, pairs, single CTAs; one launch, and the same bits, refused or not."""
+    import torch
+    W = torch.from_numpy(synth.pq2_0_weights(n_out, n_in, seed=3)).cuda()
+    Wr, xq, x = torch.zeros_like(W), torch.zeros(n_in // 32 * 36, dtype=torch.uint8, device="cuda"), torch.from_numpy(synth.activations(n_in, seed=4)).cuda()
+    y, want = torch.zeros(n_out, device="cuda"), torch.zeros(n_out, device="cuda")
+    assert gpu.repack(W, Wr, n_out, n_in) == 0 and gpu.quant_activations(x, xq, n_in) == 0 and gpu.gemv(W, xq, want, n_out, n_in) == 0
+    call = lambda: gpu.gemv_repack(Wr, x, y, n_out, n_in)
+
+    def right():
+        ok = torch.equal(y, want)
+        y.fill_(float("nan"))
+        return ok
+
+    (ctas,) = launches(call)
+    assert ctas in forms and right()
+    if ctas > 1:
+        assert launches(call, lambda: refuse(1)) == [1] and right()
+        assert launches(call) == [1] and right()
+        assert refuse(0) == 0
+        assert launches(call) == [ctas] and right()
+    assert gpu.device_status() == 0
