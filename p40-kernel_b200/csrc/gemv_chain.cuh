@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
         // The multiply fills the registers of a thread, so a warp carries little through it: the rows of the op come from its record and
         // the armed tiles from their counter each time, and nothing is called (what a caller keeps beyond the registers that a callee
         // preserves goes to memory, of which 227 KB of shared memory leave L1 little).  With these in registers and the back butterflies in a
-        // function, 8 bytes of spills at 512 threads, 116 at 640, 152 at 768, 44 with several ranks; now 0, 0, 16 and 4.  Sweep of 8 layers
+        // function, 8 bytes of spills at 512 threads, 116 at 640, 152 at 768, 44 with several ranks; now 0, 0, 16 and 8.  Sweep of 8 layers
         // and 12 layers of a decode step, us: 512 threads 118.9, 717 -> 118.2, 708; 640 158, 894 -> 145, 797; 768 154, 952 -> 139, 803; one
         // rank of two alone 157, 1698 -> 144, 1626.
         const int rr = lane & 3, bl = lane >> 2;
@@ -458,7 +458,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                         // the scratch area: front butterflies, meet, back butterflies + quantiser, meet.
                         bool ok = true;
                         for (int fb0 = fb_first; fb_lo < fb_hi && fb0 < fb_hi && ok; fb0 += whole ? nfb : G.rot_blocks) {
-                            const int units = (whole ? nfb : min(G.rot_blocks, fb_hi - fb0)) * 8;
+                            // Units read and units rotated.  (With a condition of its own for an image at each use an op that has none was slower than
+                            // before there were images, us per op: 1024 wide behind a norm 5.00 -> 5.32, now 5.18; plain 4.36 -> 4.50, now 4.48.)
+                            const int units = (whole ? nfb : min(G.rot_blocks, fb_hi - fb0)) * 8, mine = whole ? 8 : units;
                             // all of this warp's loads first (they come from L2: written by other SMs
                             // during this launch), then the butterflies
                             float4 f[UPW];
@@ -502,7 +504,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                                 ++xs_phase;
                                 if (!ok) break;
                                 float ss = 0.0f;
-#pragma unroll 4
+#pragma unroll 2
                                 for (int u = 0; u < units; u += 8) {
                                     const float4 a = *reinterpret_cast<const float4 *>(ssum + u), b = *reinterpret_cast<const float4 *>(ssum + u + 4);
                                     ss = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(ss, a.x), a.y), a.z), a.w);
@@ -512,7 +514,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
 #pragma unroll
                                 for (int k = 0; k < UPW; ++k) {
                                     const int u = wid + k * C;
-                                    if (whole ? (unsigned)(u - own) < 8u : u < units) {
+                                    if ((unsigned)(u - own) < (unsigned)mine) {
                                         const float4 wv = late ? __ldcg(reinterpret_cast<const float4 *>(aux + (size_t)u * 128 + 4 * lane)) : scratch[(u - own) * 32 + lane];
                                         f[k] = make_float4(__fmul_rn(__fmul_rn(f[k].x, sc), wv.x), __fmul_rn(__fmul_rn(f[k].y, sc), wv.y),
                                                            __fmul_rn(__fmul_rn(f[k].z, sc), wv.z), __fmul_rn(__fmul_rn(f[k].w, sc), wv.w));
@@ -522,7 +524,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
 #pragma unroll
                             for (int k = 0; k < UPW; ++k) {
                                 const int u = wid + k * C;
-                                if (whole ? (unsigned)(u - own) < 8u : u < units) {
+                                if ((unsigned)(u - own) < (unsigned)mine) {
                                     float v[4] = {f[k].x, f[k].y, f[k].z, f[k].w};
                                     if (signs) {
                                         const float4 *sp = reinterpret_cast<const float4 *>(signs + (size_t)fb0 * FWHT_N + (size_t)u * 128 + 4 * lane);
@@ -539,7 +541,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_chain_kernel(const ChainOp *_
                             ok = mbar_wait_suspended(xs, xs_phase & 1u, stop, wait_ms);
                             ++xs_phase;
                             if (!ok) break;
-                            chain_back<THREADS == 512>(scratch, wid, C, whole ? 8 : units, fb0 * 32 + own * 4, lane, act_q, act_s, act_i, spread ? table_image : nullptr,
+                            chain_back<THREADS == 512>(scratch, wid, C, mine, fb0 * 32 + own * 4, lane, act_q, act_s, act_i, spread ? table_image : nullptr,
                                                        TP ? (uint32_t)ctrl[15] + R.spread_blocks : tag1);
                             if (spread) break;                          // one block: the scratch area is not written again before the meeting below
                             __syncwarp();
