@@ -80,3 +80,23 @@ def test_list_kernel_keeps_its_registers(tmp_path):
         spilt[f"{threads}, {steps}, {'true' if ranks == '1' else 'false'}"] = int(stores)
     assert set(spilt) == set(forms), run.stderr[-2000:]
     assert all(spilt[f] <= most for f, most in forms.items()), spilt
+
+
+def test_mat_mul_kernel_keeps_its_registers(tmp_path):
+    """The same of the many-token mat-mul, whose warps have 72 registers a thread: pairs of CTAs spill nothing, single CTAs three words."""
+    spec = importlib.util.spec_from_file_location("bonsai_b200_build_spills16", os.path.join(ROOT, "p40-kernel_b200", "build.py"))
+    b = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(b)
+    if not shutil.which(b.NVCC):
+        pytest.skip("no nvcc")
+    forms = {"64, 1": 12, "128, 2": 0}
+    src = tmp_path / "forms16.cu"
+    src.write_text('#include "gemm_tc16.cuh"\nusing namespace b200;\n' + "".join(
+        f"template __global__ void b200::gemm_tc16_kernel<{f}>(float *, const T16Params, const float *__restrict__, float *, unsigned int *, "
+        "const __grid_constant__ Tc16Maps);\n" for f in forms))
+    run = subprocess.run([b.NVCC, *[f for f in b.FLAGS if f != "-shared"], "-Xptxas", "-v", f"-I{b.CSRC}", "-c", str(src), "-o", str(tmp_path / "forms16.o")],
+                         capture_output=True, text=True)
+    assert run.returncode == 0, run.stderr[-2000:]
+    spilt = {f"{n}, {ctas}": int(stores) for n, ctas, stores in
+             re.findall(r"properties for \S*gemm_tc16_kernelILi(\d+)ELi(\d)E\S*\n.*?(\d+) bytes spill stores", run.stderr)}
+    assert set(spilt) == set(forms) and all(spilt[f] <= most for f, most in forms.items()), spilt or run.stderr[-2000:]
