@@ -141,7 +141,8 @@ int bonsai_b200_stream_probe(const void *buf, int64_t bytes, int mode, void *sin
  * bit-identical to the host loop), 1 = tensor cores (the fp16 form, csrc/gemm_tc16.cuh, where it takes the call,
  * else the integer form), 2 = the small-batch kernel where it takes the shape, 3 = the integer tensor-core kernel
  * (csrc/gemm_tc.cuh: forms the host's int32 chunk sums, needs no scratch).  1, 2 and 3 hold fp32 Y to 1e-5 of
- * max |Y|.  The fp16 form keeps one scratch buffer per (device, stream), 4 bytes per token and input value, and 16 MB for
+ * max |Y|.  How the fp16 form divides a call, and with it the order of a row's sum, follows from n_out, n_in and n_tok: the same call gives the same
+ * bits every time, a row or a token of it in a call of another shape those of another order, within the bound.  The fp16 form keeps one scratch buffer per (device, stream), 4 bytes per token and input value, and 16 MB for
  * the parts of tiles, allocated with cudaMalloc on first use or growth -- never while the stream is being captured (then the
  * integer form runs).
  * key "fuse_linear": 0 (default) = bonsai_b200_linear is two launches, 1 = one kernel when it can (saves a
@@ -150,7 +151,7 @@ int bonsai_b200_stream_probe(const void *buf, int64_t bytes, int mode, void *sin
  * Options are process-wide: set them once at start-up, not from threads that call the library concurrently.
  * A library compiled with -DBONSAI_B200_TUNING (the test build) also takes geometry keys ("gemv_variant",
  * "chain_threads", "chain_seg", "chain_tile_kb", "chain_spread_nb", "gemm_tile") that force a tiling; they change no result bits
- * beyond what the documented options say and are not part of the interface; nor are "kv_wide" (0 = decode attention over the cache keeps
+ * beyond what the documented options say ("gemm_tile": as another shape of the call would, the bound holds) and are not part of the interface; nor are "kv_wide" (0 = decode attention over the cache keeps
  * clusters of eight CTAs at every length: the same bound, another order of sums) and "refuse_clusters" (the next n launches in clusters
  * of CTAs that have a form without them are refused; 0 forgets that any was).
  * Returns 0, or 1 for an unknown key. */
@@ -185,8 +186,9 @@ int bonsai_b200_clear_status(void);
  *                              OP_DEPENDS is treated this way without the flag.
  * Shapes: n_in a multiple of 256 (of 1024 with OP_ROTATE), W and x 16-byte aligned.
  * create() allocates a small device table (cudaMalloc) and copies the list; run() allocates nothing,
- * launches one cooperative kernel of one CTA per SM on `stream` (plus a 4-byte memset) and can be
- * captured in a CUDA graph; a chain object must not run on two streams at once.  Errors: 1 for a bad
+ * launches one cooperative kernel of one CTA per SM on `stream`, behind a memset of what its CTAs tell each other through (8 bytes; more
+ * where an op rescales, 4 per op, or waits with an input of 2048 values and more, 288 per 128 values of the list's longest input: 39 KB at 17408),
+ * and can be captured in a CUDA graph; a chain object must not run on two streams at once.  Errors: 1 for a bad
  * argument, otherwise the CUDA error code. */
 /* Producers (with OP_ROTATE, at most one per op): what turns the fp32 vector at x into the vector that is rotated and
  * quantised, fused into the op's prologue -- the step that precedes every projection of a decode step
@@ -231,8 +233,8 @@ int bonsai_b200_chain_destroy(bonsai_b200_chain *chain);
  * this process (peer_base[rank] is the local one).  The kernel stores every y element it produces into all `world`
  * buffers, so each rank ends up with the whole vector without a collective, and OP_DEPENDS waits for every row of
  * every rank.  The buffer is buffer_bytes long on every rank; BONSAI_B200_TP_COUNTER_BYTES bytes at counter_offset
- * (a multiple of 64, behind every output) are the kernel's counters and flags: zero them once after allocation and
- * never touch them again.  Refused (1): an output that does not lie inside [buffer, buffer + counter_offset), a
+ * (a multiple of 64, behind every output) are the kernel's counters and flags, of one list and its runs: zero them once after allocation
+ * and never touch them again.  Refused (1): an output that does not lie inside [buffer, buffer + counter_offset), a
  * counter block that does not fit in buffer_bytes, a mapping that is not 16-byte aligned.  Every rank must run on a
  * GPU with the same number of SMs.  All ranks must call run() the same number of times; the launches of different
  * ranks wait for each other, so each rank needs its own GPU.  The waits are bounded by wait_limit_us microseconds

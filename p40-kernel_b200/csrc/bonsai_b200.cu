@@ -48,7 +48,7 @@ std::atomic<int> g_opt_gemv_order{0};
 std::atomic<int> g_opt_fuse_linear{0};         // 1: bonsai_b200_linear runs as one kernel when it can (measured slower)
 std::atomic<int> g_opt_chain_threads{512};       // threads per CTA of the chain kernel: 512 (5 blocks per lane and task), 640 (4), 768 (3)
 // Dependent ops with at least this many blocks per row rotate their input once for the grid instead of once per CTA; 0 = never.  us per op of a list
-// n -> n, once per CTA / once for the grid: 1024 behind a norm 5.3 / 5.7, 2048 6.5 / 6.2 (plain 5.6 / 5.3), 3072 7.5 / 6.9, 5120 9.8 / 8.1.
+// n -> n, once per CTA / once for the grid: 1024 behind a norm 5.2 / 5.7, 2048 6.4 / 6.2 (plain 5.5 / 5.35), 3072 7.3 / 6.8, 5120 9.6 / 8.1.
 std::atomic<int> g_opt_chain_spread_nb{16};
 std::atomic<int> g_opt_chain_tile_kb{16};
 std::atomic<int> g_opt_kv_wide{1};                // decode attention: 0 = clusters of eight CTAs at every length
@@ -1058,7 +1058,8 @@ static Tc16Plan plan_tc16(int64_t n_out, int64_t nblocks, int64_t n_tok, int wor
     p.tile_n = (int)(((n_tok + p.tiles_tok - 1) / p.tiles_tok + step - 1) / step * step);
     p.tiles = (n_out + T16_M * CTAS - 1) / (T16_M * CTAS) * p.tiles_tok;
     if (p.tiles > INT32_MAX) return p;
-    // Whole tiles in turn, or the blocks of all tiles in equal shares: at most four workers to a tile, at least 16 blocks each.  Measured at
+    // Whole tiles in turn, or the blocks of all tiles in equal shares: at most four workers per tile on average (a tile that begins inside a share can
+    // be cut into five parts), at least 16 blocks each.  Measured at
     // 33 - 192 tokens of 1024 -> 12288, 5120 -> 5120, 5120 -> 17408 and 17408 -> 5120: 5.5 us and 0.53 per block for a CTA, 8 us and 0.39 + 0.003 per token
     // and block for a pair, 7 us for leaving, fetching and adding the parts of tiles that are shared.
     const double start = CTAS == 1 ? 5500 : 8000, block = CTAS == 1 ? 530 : 390 + 3 * p.tile_n;
