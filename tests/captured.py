@@ -1,8 +1,9 @@
 """What a call launches, read from a capture of it."""
+import pytest
 
 
 def launches(call, between=lambda: None):
-    """The CTAs per cluster of each kernel that call() launches, the second time on a stream of its own."""
+    """The CTAs per cluster of each kernel that call() launches, the second time on a stream of its own; the captured launches have run once."""
     import torch
     from cuda.bindings import runtime as rt
     st, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
@@ -12,8 +13,7 @@ def launches(call, between=lambda: None):
         between()
         with torch.cuda.graph(graph, stream=st):
             assert call() == 0
-    raw = rt.cudaGraph_t(init_value=graph.raw_cuda_graph())
-    nodes = rt.cudaGraphGetNodes(raw, 16)[1]
+    nodes = rt.cudaGraphGetNodes(rt.cudaGraph_t(init_value=graph.raw_cuda_graph()), 16)[1]
     out = []
     for node in nodes:
         if int(node) and rt.cudaGraphNodeGetType(node)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel:
@@ -23,3 +23,12 @@ def launches(call, between=lambda: None):
     graph.replay()
     torch.cuda.synchronize()
     return out
+
+
+@pytest.fixture
+def scratch_given_back(gpu):
+    """For tests that capture mat-muls: the graphs hold the scratch of their streams, of which a device has sixteen, until it is released."""
+    import torch
+    yield
+    torch.cuda.synchronize()
+    assert gpu.gemm_release() == 0

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from bonsai_b200 import synth
-from captured import launches
+from captured import launches, scratch_given_back  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -16,7 +16,7 @@ def refuse(gpu):
     gpu.set_option("refuse_clusters", 0)
 
 
-def test_matmul(gpu, port, refuse):
+def test_matmul(gpu, port, scratch_given_back, refuse):
     """Two launches, the activations split once: refused in the capture, refused in the call in front of it and remembered, and not refused."""
     import torch
     n_out, n_in, n_tok = 300, 2048, 200

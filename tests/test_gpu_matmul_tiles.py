@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from bonsai_b200 import synth
-from captured import launches
+from captured import launches, scratch_given_back  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -54,7 +54,7 @@ def test_edges_of_each_tile(gpu, port, n_out, n_in, n_tok, tile):
 
 # (4000 x 17408 at 65 tokens: four parts per tile; 5120 x 17408 at 128: five; 2048 x 5120 at 577: three; the others whole tiles in turn)
 @pytest.mark.parametrize("n_out,n_in,n_tok", [(4000, 17408, 65), (5120, 17408, 128), (2048, 5120, 577), (6000, 5120, 257), (12288, 1024, 300)])
-def test_calls_that_take_pairs_by_themselves(gpu, port, n_out, n_in, n_tok):
+def test_calls_that_take_pairs_by_themselves(gpu, port, scratch_given_back, n_out, n_in, n_tok):
     import torch
     W, Xq = torch.zeros(n_out * n_in // 128 * 34, dtype=torch.uint8, device="cuda"), torch.zeros(n_in // 32 * 36 * n_tok, dtype=torch.uint8, device="cuda")
     Y = torch.empty(n_out, n_tok, device="cuda")
