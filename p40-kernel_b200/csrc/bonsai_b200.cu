@@ -1017,11 +1017,11 @@ static bool encode_w_map(CUtensorMap *map, const void *W, int64_t n_out, int64_t
 // Scratch of the fp16 tensor-core mat-mul: a flag and a slot per CTA for its part of a tile, the activations as two fp16 planes, a
 // scale per token.  A call that gets none takes the integer kernel, which needs no scratch.
 static constexpr size_t T16_FLAGS_BYTES = (size_t)TC_MAX_CTAS * T16_PART_FLAGS * sizeof(unsigned int);
-static StreamScratch g_gemm_scratch(T16_FLAGS_BYTES, false);
+static StreamScratch g_gemm_scratch(false);
 
 // Scratch of the prompt attention: k and v as tile images, 2 KB per position and kv head, what k and v take themselves.  Prompts of one
 // conversation grow a little each time.  A call that gets none takes the CUDA-core kernel.
-static StreamScratch g_attn_scratch(0, true);
+static StreamScratch g_attn_scratch(true);
 
 static std::atomic<unsigned int> g_gemm_epoch{0};       // launch number of the tensor-core mat-muls (tags partial-tile flags)
 
@@ -1150,9 +1150,10 @@ static int launch_gemm_tc16(const void *W, const void *Xq, float *Y, int64_t n_o
     int passes = (n_chunks + T16_SPLIT_PASS - 1) / T16_SPLIT_PASS;
     passes = (int)((passes * groups + 2 * sms - 1) / (2 * sms));
     const int slice = passes * T16_SPLIT_PASS;
+    const int flagged = std::max(one.stream_k ? one.grid : 0, paired && two.stream_k ? 2 * two.grid : 0);      // CTAs that may raise flags
     cudaError_t e = launch(groups <= 2 * sms ? tc16_split_kernel<true> : tc16_split_kernel<false>,
                            dim3((unsigned)groups, (unsigned)((n_chunks + slice - 1) / slice)), dim3(T16_SPLIT_THREADS), 0, st, true, x32, n_chunks, (int)n_tok, slice,
-                           scale, planes);
+                           scale, planes, reinterpret_cast<uint4 *>(ws), flagged * T16_PART_FLAGS / 4);
     if (e != cudaSuccess) return (int)e;
     if (paired) {
         e = launch_gemm_tc16_n<128, 2>(a, two, g_tc16_pairs_smem, st);

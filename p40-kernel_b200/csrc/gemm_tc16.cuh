@@ -271,11 +271,12 @@ __device__ __forceinline__ int tc16_shift(unsigned int maxd_bits) {
 // between the maximum and the split -- then thread = (chunk, token): 32 values -> 32 + 32 fp16, in the order the quantiser
 // stored them (the order in which the code producers emit the codes).  planes: H at [tok][n_in], L at [n_tok + tok][n_in];
 // scale[tok] = 2^-S for the epilogue.  A warp takes 4 tokens x 8 consecutive chunks: its stores are four runs of 512 bytes
-// per plane.  Bound by launch and memory latency.
+// per plane.  Bound by launch and memory latency.  The first threads also lower the flags that the mat-mul's CTAs raise where they share
+// tiles, four at a time: a launch whose wait ran out leaves those raised that came later, and the next must not take them for its own.
 constexpr int T16_SPLIT_THREADS = 256, T16_SPLIT_PASS = T16_SPLIT_THREADS / 4;      // chunks of four tokens a block takes at once
 template <bool FEW>
 __global__ void __launch_bounds__(T16_SPLIT_THREADS) tc16_split_kernel(const uint32_t *Xq, int n_chunks, int n_tok, int slice, float *scale,
-                                                                       __half *planes) {
+                                                                       __half *planes, uint4 *flags, int n_flags4) {
     __shared__ unsigned int top[T16_SPLIT_THREADS / 32][4];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tok = 4 * (int)blockIdx.x + (lane >> 3), c_first = (int)blockIdx.y * slice + 8 * warp + (lane & 7);
@@ -291,6 +292,9 @@ __global__ void __launch_bounds__(T16_SPLIT_THREADS) tc16_split_kernel(const uin
         for (int k = 0; k < 9; ++k) w[k] = src[k];
     };
     if (FEW) fetch(c_first);
+    for (int i = ((int)blockIdx.y * (int)gridDim.x + (int)blockIdx.x) * T16_SPLIT_THREADS + (int)threadIdx.x; i < n_flags4;
+         i += (int)(gridDim.x * gridDim.y) * T16_SPLIT_THREADS)
+        flags[i] = make_uint4(0u, 0u, 0u, 0u);
     {   // four tokens are neighbours in memory: four lanes read one chunk's headers
         const int t = min(4 * (int)blockIdx.x + (lane & 3), n_tok - 1);
         unsigned int m = 0;
@@ -574,7 +578,7 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
                 int last = worker + 1;
                 while (last + 1 < workers && t16_first(P, last + 1, workers) < tile_end) ++last;
                 for (int c = worker + 1 + lane; c <= last; c += 32) {
-                    unsigned int *f = flags + (CTAS * c + rank) * T16_PART_FLAGS + wid;
+                    const unsigned int *f = flags + (CTAS * c + rank) * T16_PART_FLAGS + wid;
                     bool there = false;
                     for (uint32_t k = 0; k < (1u << 23); ++k) {
                         unsigned int fv;
@@ -583,7 +587,6 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
                         __nanosleep(32);
                     }
                     if (!there) atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);
-                    *const_cast<volatile unsigned int *>(f) = 0u;     // lowered by its only reader: the next launch on this scratch finds zeros
                 }
                 __syncwarp();
                 const float *slots = parts + (size_t)rank * C::PART_FLOATS + (size_t)col0 * T16_M + row_l;

@@ -40,9 +40,9 @@ inline bool zero_new_memory(void *p, size_t bytes) {
 
 class StreamScratch {
 public:
-    // zeroed: the first bytes of a new buffer that the kernels expect to be zero (and leave zero behind).  steps: a buffer that
-    // has become too small grows by half at least -- for calls whose need rises a little from one to the next.
-    StreamScratch(size_t zeroed, bool steps) : zeroed_(zeroed), steps_(steps) {}
+    // steps: a buffer that has become too small grows by half at least -- for calls whose need rises a little from one to the next.  (What is in
+    // a buffer is whatever was there: the kernels write before they read.)
+    explicit StreamScratch(bool steps) : steps_(steps) {}
 
     struct Lease {
         void *ptr = nullptr;                        // nullptr: none to be had
@@ -144,7 +144,6 @@ private:
         b.stream = id;
         b.reserved = reserved;
         if (cudaMalloc(&b.ptr, bytes) != cudaSuccess && (bytes == exact || cudaMalloc(&b.ptr, bytes = exact) != cudaSuccess)) b.ptr = nullptr;
-        if (b.ptr && zeroed_ && !zero_new_memory(b.ptr, zeroed_)) (void)cudaFree(b.ptr), b.ptr = nullptr;
         if (b.ptr) b.bytes = bytes;
         else (void)cudaGetLastError();
         (void)cudaThreadExchangeStreamCaptureMode(&mode);
@@ -157,7 +156,6 @@ private:
         }
     }
 
-    const size_t zeroed_;
     const bool steps_;
     Device devices_[DEVICES];
 };

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from bonsai_b200 import synth
-from captured import launches, scratch_given_back  # noqa: F401
+from captured import capture, launches, pointer_argument, scratch_given_back  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -60,3 +60,34 @@ def test_calls_that_take_pairs_by_themselves(gpu, port, scratch_given_back, n_ou
     Y = torch.empty(n_out, n_tok, device="cuda")
     assert launches(lambda: gpu.gemm(W, Xq, Y, n_out, n_in, n_tok)) == [1, 2]
     check(gpu, port, n_out, n_in, n_tok, 0)
+
+@pytest.mark.parametrize("n_out,n_in,n_tok,tile", [(300, 17408, 40, 64), (300, 17408, 96, 128), (5120, 17408, 37, 0)])
+def test_flags_that_an_earlier_launch_left_raised(gpu, port, scratch_given_back, n_out, n_in, n_tok, tile):
+    """A launch whose wait for a part ran out may leave that part's flag raised (all of them here, by a memset): the next calls on the same
+    scratch, and replays of a captured one, wait for parts of their own."""
+    import torch
+    from cuda.bindings import runtime as rt
+    X = [torch.from_numpy(port.quantize_batch_chunk_major(synth.activations(n_in, seed=s, batch=n_tok))).cuda() for s in range(2)]
+    W, Xq = torch.from_numpy(synth.pq2_0_weights(n_out, n_in, seed=n_tok)).cuda(), X[0].clone()
+    Y, want = torch.zeros(n_out, n_tok, device="cuda"), []
+    call = lambda: gpu.gemm(W, Xq, Y, n_out, n_in, n_tok)
+    try:
+        assert gpu.set_option("gemm_path", 1) == 0 and gpu.set_option("gemm_tile", tile) == 0
+        graph, kernels, st = capture(call)
+        flags = pointer_argument(kernels[1], 4)
+        with torch.cuda.stream(st):
+            for x in X:
+                Xq.copy_(x)
+                assert call() == 0
+                want.append(Y.clone())
+            for again in (call, lambda: graph.replay() or 0):
+                for i in range(4):
+                    assert int(rt.cudaMemsetAsync(flags, 1, 148 * 16 * 4, st.cuda_stream)[0]) == 0
+                    Xq.copy_(X[i % 2])
+                    assert again() == 0
+                    assert torch.equal(Y, want[i % 2]), i
+        torch.cuda.synchronize()
+    finally:
+        gpu.set_option("gemm_path", -1)
+        gpu.set_option("gemm_tile", 0)
+    assert gpu.device_status() == 0
