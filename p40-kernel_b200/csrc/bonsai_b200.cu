@@ -52,7 +52,7 @@ std::atomic<int> g_opt_chain_threads{512};       // threads per CTA of the chain
 std::atomic<int> g_opt_chain_spread_nb{16};
 std::atomic<int> g_opt_chain_tile_kb{16};
 std::atomic<int> g_opt_kv_wide{1};                // decode attention: 0 = clusters of eight CTAs at every length
-std::atomic<int> g_opt_gemm_tile{0};              // fp16 tensor-core mat-mul: 0 by token count, 64 or 128 tokens per tile
+std::atomic<int> g_opt_gemm_tile{0};              // fp16 tensor-core mat-mul: 0 by estimated time, else tiles of up to 64 tokens (a CTA) or 128 (a pair)
 std::atomic<int> g_opt_chain_seg{40};            // longest row segment of one task, in blocks: 8, 16, 24, 32 or 40        // target bytes of one ring slot
 std::atomic<int> g_opt_gemm_path{-1};          // -1: by token count, 0: integer SIMT kernel, 1: tensor cores, 2: small-batch kernel, 3: integer tensor-core kernel          // 0: streaming kernel (fixed tree order), 1: the host's sequential order
 

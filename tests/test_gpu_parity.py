@@ -820,7 +820,7 @@ def test_gemm_in_a_captured_graph_after_reserve(gpu, port):
 
 @pytest.mark.parametrize("tile", [64, 128])
 def test_gemm_fp16_both_tile_widths(gpu, port, tile):
-    """The fp16 tensor-core mat-mul is built for token tiles of 64 and of 128 (picked by token count); each forced on a
+    """The fp16 tensor-core mat-mul is built for token tiles of 64 and of 128 (picked by estimated time); each forced on a
     batch the other would normally take: ragged rows and tokens, bound against the host loop."""
     import torch
     for n_out, n_in, n_tok in ((300, 2048, 100), (129, 1024, 513)):
