@@ -134,9 +134,11 @@ public:
         if (cudaGetDevice(&dev) == cudaSuccess && dev < 64) known_[dev].store(-1, std::memory_order_relaxed);
         return true;
     }
+#ifdef BONSAI_B200_TUNING
     void forget() {
         for (auto &k : known_) k.store(0, std::memory_order_relaxed);
     }
+#endif
 
 private:
     std::atomic<int> known_[64] = {};
