@@ -1634,15 +1634,23 @@ inline int64_t kv_gdn_bytes() { return (int64_t)KVM_LINEAR * KVM_V_HEADS * KVM_S
 constexpr int KV_COUNTERS = KVM_KV_HEADS * KV_CLUSTER;      // per layer
 inline size_t kv_ws_floats(int max_clusters) { return (size_t)KVM_KV_HEADS * KV_CLUSTER * max_clusters * KV_REC; }      // per layer
 
-// Clusters of 8 (or, wide, of 16) CTAs of the decode kernel that are resident at once on the current device (0: they do not run here).
-// Asked once per device.
-int kv_resident(bool wide) {
-    static std::atomic<int> known[2][64];
-    static SmemOptIn opt[2];
+// The decode kernel in clusters of 8 (or, wide, of 16) CTAs.  push: tile buffers of the form for one cluster per kv head, 0 the form for several.
+using KvKernel = decltype(&kv_attn_kernel<KVM_GROUP>);
+inline KvKernel kv_kernel(bool wide, int push) {
+    static const KvKernel kernels[2][3] = {{kv_attn_kernel<KVM_GROUP, KV_CLUSTER, 0>, kv_attn_kernel<KVM_GROUP, KV_CLUSTER, 1>, kv_attn_kernel<KVM_GROUP, KV_CLUSTER, 2>},
+                                           {nullptr, kv_attn_kernel<KVM_GROUP, KV_WIDE_CLUSTER, 1>, kv_attn_kernel<KVM_GROUP, KV_WIDE_CLUSTER, 2>}};
+    return kernels[wide][push];
+}
+inline unsigned kv_threads(int push) { return push ? 32 * KV_PUSH_WARPS : KV_THREADS; }
+inline unsigned kv_smem(int push) { return push ? KV_PUSH_SMEM_BYTES + push * 2 * KV_HALF_BYTES : KV_SMEM_BYTES; }
+// Its clusters that are resident at once on the current device (0: they do not run here).  Asked once per device.
+int kv_resident(bool wide, int push) {
+    static std::atomic<int> known[2][3][64];
+    static SmemOptIn opt[2][3];
     int dev = 0, resident = 0;
-    auto *kernel = wide ? kv_attn_kernel<KVM_GROUP, KV_WIDE_CLUSTER> : kv_attn_kernel<KVM_GROUP, KV_CLUSTER>;
-    if (opt[wide].ensure(kernel) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (dev < 64 && (resident = known[wide][dev].load(std::memory_order_relaxed)) > 0) return resident;
+    const KvKernel kernel = kv_kernel(wide, push);
+    if (opt[wide][push].ensure(kernel) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev < 64 && (resident = known[wide][push][dev].load(std::memory_order_relaxed)) > 0) return resident;
     if (wide && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
@@ -1650,8 +1658,8 @@ int kv_resident(bool wide) {
     const unsigned cluster = wide ? KV_WIDE_CLUSTER : KV_CLUSTER;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cluster * KV_MAX_CLUSTERS, KVM_KV_HEADS);
-    cfg.blockDim = dim3(KV_THREADS);
-    cfg.dynamicSmemBytes = KV_SMEM_BYTES;
+    cfg.blockDim = dim3(kv_threads(push));
+    cfg.dynamicSmemBytes = kv_smem(push);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = cluster;
@@ -1662,7 +1670,7 @@ int kv_resident(bool wide) {
         (void)cudaGetLastError();
         return 0;
     }
-    if (dev < 64) known[wide][dev].store(resident, std::memory_order_relaxed);
+    if (dev < 64) known[wide][push][dev].store(resident, std::memory_order_relaxed);
     return resident;
 }
 // Clusters of eight per kv head that a device with so many of them resident gets at most: one wave.
@@ -1679,8 +1687,8 @@ KvSplits kv_splits(int n_pos, int max_clusters, bool wide_runs) {
     KvSplits s{KV_CLUSTER, std::max(1, std::min(n_pos / (KV_CLUSTER * KV_SPLIT_MIN), max_clusters)), 0};
     // One cluster of 16 where one or two of eight would do and each of their splits would have more than a tile, 513 to 3071 positions: 701
     // are a tile a split, not two one after the other, and 2048 need no merge through memory.  16 layers with their appends, in us,
-    // with clusters of 8 and of 16: 513 positions 145 / 126, 701 148 / 128, 1501 180 / 150, 2048 187 / 158, 3001 213 / 186.  Up to 512 a split
-    // of eight is one tile already; from 3072 on three clusters of eight have more splits than the one of 16 that the kernel is laid out for.
+    // with clusters of 8 and of 16 (both merged by reading): 513 positions 145 / 126, 701 148 / 128, 1501 180 / 150, 2048 187 / 158, 3001 213 / 186.  Up to 512 a split
+    // of eight is one tile already (401 positions 102 by eight, 103 by 16; 271 102 and 101); from 3072 on three clusters of eight have more splits than the one of 16 that the kernel is laid out for.
     if (wide_runs && n_pos > KV_CLUSTER * KV_TILE && n_pos < 3 * KV_CLUSTER * KV_SPLIT_MIN) s.cluster = KV_WIDE_CLUSTER, s.clusters = 1;
     const int n_split = s.cluster * s.clusters;
     s.chunk = (((n_pos + n_split - 1) / n_split) + 15) / 16 * 16;
@@ -1698,6 +1706,7 @@ struct bonsai_kv_cache {
                                                 // that layers may be decoded on different streams at once
     int max_clusters = 1;                       // clusters of eight of the decode kernel per kv head, at most
     int resident_wide = 0;                      // clusters of 16 that are resident at once
+    bool push_runs = false;                     // whether the form for one cluster of eight per kv head runs here
 };
 
 int64_t bonsai_kv_bytes(int capacity) {
@@ -1713,8 +1722,9 @@ bonsai_kv_cache *bonsai_kv_create(int capacity, bonsai_stream stream) {
     bonsai_kv_cache *kv = new (std::nothrow) bonsai_kv_cache;
     if (!kv) return nullptr;
     kv->capacity = capacity;
-    kv->max_clusters = kv_max_clusters(kv_resident(false));
-    kv->resident_wide = kv_resident(true);
+    kv->max_clusters = kv_max_clusters(kv_resident(false, 0));
+    kv->resident_wide = std::min(kv_resident(true, 1), kv_resident(true, 2));
+    kv->push_runs = std::min(kv_resident(false, 1), kv_resident(false, 2)) > 0;
     const size_t ws = (size_t)KVM_FULL * kv_ws_floats(kv->max_clusters) * sizeof(float), ncnt = (size_t)KVM_FULL * KV_COUNTERS * sizeof(unsigned int);
     if (kv->max_clusters <= 0 || cudaMalloc(&kv->d_k, (size_t)kv_array_bytes(capacity)) != cudaSuccess ||
         cudaMalloc(&kv->d_v, (size_t)kv_array_bytes(capacity)) != cudaSuccess || cudaMalloc(&kv->d_gdn, (size_t)kv_gdn_bytes()) != cudaSuccess ||
@@ -1776,10 +1786,11 @@ int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *
     if (pos < 0 || pos >= kv->capacity) return 1;
     const KvSplits s = kv_splits(pos + 1, kv->max_clusters, kv_wide_runs(kv->resident_wide));
     const bool wide = s.cluster == KV_WIDE_CLUSTER;
+    const int push = s.clusters == 1 && (wide || kv->push_runs) ? (s.chunk <= KV_TILE ? 1 : 2) : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(s.cluster * s.clusters), KVM_KV_HEADS);
-    cfg.blockDim = dim3(KV_THREADS);
-    cfg.dynamicSmemBytes = KV_SMEM_BYTES;
+    cfg.blockDim = dim3(kv_threads(push));
+    cfg.dynamicSmemBytes = kv_smem(push);
     cfg.stream = as_stream(stream);
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1789,16 +1800,16 @@ int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_opt_overlap.load() ? 2 : 1;
-    return (int)cudaLaunchKernelEx(&cfg, wide ? kv_attn_kernel<KVM_GROUP, KV_WIDE_CLUSTER> : kv_attn_kernel<KVM_GROUP, KV_CLUSTER>, q, (const uint8_t *)kv->d_k, (const uint8_t *)kv->d_v,
+    return (int)cudaLaunchKernelEx(&cfg, kv_kernel(wide, push), q, (const uint8_t *)kv->d_k, (const uint8_t *)kv->d_v,
                                    kv->d_ws + (size_t)layer * kv_ws_floats(kv->max_clusters), kv->d_counters + layer * KV_COUNTERS, out,
                                    pos, s.chunk, KVM_KV_HEADS, kv->capacity, layer, 0.0625f);
 }
 
 int bonsai_b200_kv_splits(int n_pos, int resident8, int resident16, int64_t out[3]) {
     if (n_pos <= 0 || n_pos > KVM_CONTEXT || !out) return 1;
-    const int max_clusters = kv_max_clusters(resident8 < 0 ? kv_resident(false) : resident8);
+    const int max_clusters = kv_max_clusters(resident8 < 0 ? kv_resident(false, 0) : resident8);
     if (max_clusters <= 0) return 1;
-    const KvSplits s = kv_splits(n_pos, max_clusters, kv_wide_runs(resident16 < 0 ? kv_resident(true) : resident16));
+    const KvSplits s = kv_splits(n_pos, max_clusters, kv_wide_runs(resident16 < 0 ? std::min(kv_resident(true, 1), kv_resident(true, 2)) : resident16));
     out[0] = s.cluster;
     out[1] = s.clusters;
     out[2] = s.chunk;

@@ -5,7 +5,7 @@
 //
 // Layout (unchanged, it is the format, src/kv_cache.h:35-46): head-major, K and V separate,
 // block[((layer * n_kv_head + kv_head) * capacity + pos) * 8 + blk], 34-byte blocks -- the 8 blocks of a position are
-// 272 contiguous bytes, consecutive positions follow each other, so a run of positions of one (layer, kv head) is ONE
+// 272 contiguous bytes, consecutive positions follow each other, so a run of positions of one (layer, kv head) is PUSH
 // contiguous, 16-byte aligned span.
 //
 // Decode on B200: one CTA per (kv head, split of the positions) serves the SIX query heads that share the kv head
@@ -26,14 +26,14 @@ constexpr int KV_MAX_GROUP = 8;                                      // query he
 // ---- Q8_0 row quantiser: 4 lanes per 32-value block, 8 values per lane ---------------------------------------------
 // Bytes equal kv_quantize_row_q8_0 (src/kv_cache.h:100-117).  (The reference's device kernels give a lane 4 values,
 // which covers only half of every block, src/kernels/kv_p40.cu:47-51,72; the host function is the one followed.)
-__device__ __forceinline__ void kv_quantise_8(const float (&x)[8], float &d_out, uint32_t (&word)[2]) {
+__device__ __forceinline__ float kv_amax_8(const float (&x)[8]) {
     float amax = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(x[i]));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    const float d = __fdiv_rn(amax, 127.0f);
-    const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+    return fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+}
+__device__ __forceinline__ void kv_words_8(const float (&x)[8], float id, uint32_t (&word)[2]) {
     word[0] = word[1] = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -41,6 +41,10 @@ __device__ __forceinline__ void kv_quantise_8(const float (&x)[8], float &d_out,
         v = max(-127, min(127, v));
         word[i >> 2] |= ((uint32_t)v & 0xFFu) << (8 * (i & 3));
     }
+}
+__device__ __forceinline__ void kv_quantise_8(const float (&x)[8], float &d_out, uint32_t (&word)[2]) {
+    const float d = __fdiv_rn(kv_amax_8(x), 127.0f);
+    kv_words_8(x, d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f, word);
     d_out = d;
 }
 
@@ -123,6 +127,13 @@ __global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *K, uint8_t *V,
 // the last cluster to arrive at a slice's counter adds them up and writes the output: one launch per call (the merge was
 // a kernel of its own).  Clusters of 16 serve the lengths where they halve the tiles of a split (513 positions on) and where two
 // clusters of eight would need the second merge (up to 3071).
+//
+// Up to 3071 positions, one cluster per kv head (PUSH), the kernel is a chain of latencies: 9400 cycles from the end of the launch in front to
+// the output of 9 positions, 10500 of 701.  What that form does about them: eight warps (a warp has half of the dims of 16 scores, the halves meet
+// through shared memory, and one V block), and every CTA sends its slices and its (m, l) to whom they concern, who counts the bytes on a barrier
+// (behind ordinary stores, at the cluster's barrier, and read from there: 3500 cycles; now 1500).  PUSH = 1: splits of at most one tile, without the second buffer and
+// what a loop carries.  16 layers with their appends, us, before -> now (four warps, merged by reading): 9 positions 116 -> 96, 131 121 -> 100, 701 131 ->
+// 105, 1024 133 -> 106, 1101 147 -> 133, 3001 185 -> 171.  (PUSH = 2 at 701: 111.)
 constexpr int KV_THREADS = 128, KV_WARPS = 4, KV_BUFS = 2, KV_CLUSTER = 8, KV_WIDE_CLUSTER = 16;
 constexpr int KV_HALF_BYTES = KV_TILE * KV_ROW;                      // the K (or V) rows of a tile
 constexpr int KV_WT_STRIDE = KV_TILE + 8;                            // weights of a head: 8 g + 2 t are 32 different banks
@@ -133,8 +144,11 @@ constexpr int KV_MAX_CLUSTERS = 64;                                  // per kv h
 // 0.06: 3e-6 of the output).  A scale below fp16's normal range counts as the smallest there is.
 constexpr int KV_V_RANGE = 12;
 constexpr int KV_REC = KV_MAX_GROUP * (KV_SLICE + 2);                // floats of a cluster's merged slice: acc, m, l
-constexpr int KV_SMEM_BYTES = 128 + KV_BUFS * 2 * KV_HALF_BYTES + KV_MAX_GROUP * KV_WT_STRIDE * 4 + 3 * KV_MAX_GROUP * 8 * 4 +
-                              KV_MAX_GROUP * 64 * 4;
+constexpr int KV_Q_STRIDE = 64 + 4;                                  // words of a quantised query head: 4 g + t are 32 different banks
+constexpr int KV_TABLE_BYTES = 128 + KV_MAX_GROUP * KV_WT_STRIDE * 4 + 3 * KV_MAX_GROUP * 8 * 4 + KV_MAX_GROUP * KV_Q_STRIDE * 4;
+constexpr int KV_SMEM_BYTES = KV_TABLE_BYTES + KV_BUFS * 2 * KV_HALF_BYTES;
+constexpr int KV_PUSH_WARPS = 8;
+constexpr int KV_PUSH_SMEM_BYTES = KV_TABLE_BYTES + KV_MAX_GROUP * KV_D * 4 + KV_WIDE_CLUSTER * KV_MAX_GROUP * 8 + KV_PUSH_WARPS * 32 * 16;
 static_assert(16384 >= KV_MAX_GROUP * (KV_D + 2) * 4 && KV_BUFS * 2 * KV_HALF_BYTES >= 16384 + 3 * KV_MAX_CLUSTERS * KV_MAX_GROUP * 4, "the merge reuses the tile buffers");
 
 __device__ __forceinline__ void mma_s8_16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -179,21 +193,38 @@ __device__ __forceinline__ float ld_cluster_f32(const float *p, uint32_t rank) {
     return v;
 }
 
-// grid (n_split, n_kv_head), cluster (CL, 1, 1), n_split a multiple of CL (KV_WIDE_CLUSTER: one cluster per head); split s covers positions
+// Into CTA `rank`'s shared memory, at the place that p is in this one's (8- and 16-byte aligned), counted on its barrier at `bar`.
+__device__ __forceinline__ void st_async_f32x2(const float *p, uint64_t *bar, uint32_t rank, float a, float b) {
+    asm volatile("{\n\t.reg .u32 x, y;\n\tmapa.shared::cluster.u32 x, %0, %2;\n\tmapa.shared::cluster.u32 y, %1, %2;\n\t"
+                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [x], {%3, %4}, [y];\n\t}"
+                 ::"r"(smem_u32(p)), "r"(smem_u32(bar)), "r"(rank), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void st_async_f32x4(const float *p, uint64_t *bar, uint32_t rank, float a, float b, float c, float d) {
+    asm volatile("{\n\t.reg .u32 x, y;\n\tmapa.shared::cluster.u32 x, %0, %2;\n\tmapa.shared::cluster.u32 y, %1, %2;\n\t"
+                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [x], {%3, %4, %5, %6}, [y];\n\t}"
+                 ::"r"(smem_u32(p)), "r"(smem_u32(bar)), "r"(rank), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+// grid (n_split, n_kv_head), cluster (CL, 1, 1), n_split a multiple of CL (PUSH: CL, else CL is KV_CLUSTER); split s covers positions
 // s * chunk .. min((s + 1) * chunk, pos + 1) - 1 (a split may be empty).  counters: one per (kv head, slice), zero before
 // and after every launch.
-template <int GRP, int CL = KV_CLUSTER>
-__global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, const uint8_t *K, const uint8_t *V, float *ws, unsigned int *counters, float *out,
+template <int GRP, int CL = KV_CLUSTER, int PUSH = 0>
+__global__ void __launch_bounds__(PUSH ? 32 * KV_PUSH_WARPS : KV_THREADS, PUSH ? 2 : 3) kv_attn_kernel(const float *q, const uint8_t *K, const uint8_t *V, float *ws, unsigned int *counters, float *out,
                                                                 int pos, int chunk, int n_kv_head, int capacity, int layer, float scale) {
     static_assert(GRP <= KV_MAX_GROUP, "");
+    constexpr int WARPS = PUSH ? KV_PUSH_WARPS : KV_WARPS, THREADS = 32 * WARPS;
+    constexpr int NB = KV_NBLK / WARPS;                                          // V blocks of a warp
     extern __shared__ __align__(128) uint8_t smem[];
-    uint64_t *kfull = reinterpret_cast<uint64_t *>(smem), *vfull = kfull + KV_BUFS;
+    uint64_t *kfull = reinterpret_cast<uint64_t *>(smem), *vfull = kfull + KV_BUFS, *met = vfull + KV_BUFS;
     uint8_t *raw = smem + 128;                                                   // [KV_BUFS][K rows | V rows]
-    float *wt = reinterpret_cast<float *>(raw + KV_BUFS * 2 * KV_HALF_BYTES);    // [8 heads][KV_WT_STRIDE]
+    constexpr int BUFS = PUSH == 1 ? 1 : KV_BUFS;
+    float *wt = reinterpret_cast<float *>(raw + BUFS * 2 * KV_HALF_BYTES);       // [8 heads][KV_WT_STRIDE]
     float *mw = wt + KV_MAX_GROUP * KV_WT_STRIDE;                                // [4 chunks, 4 pad][8 heads] maxima
     float *lw = mw + KV_MAX_GROUP * 8;                                           // ... and sums of the weights
     float *qd = lw + KV_MAX_GROUP * 8;                                           // [8 heads][8 blocks] query scales x `scale`
-    uint32_t *q8 = reinterpret_cast<uint32_t *>(qd + KV_MAX_GROUP * 8);          // [8 heads][8 blocks][8 words]
+    uint32_t *q8 = reinterpret_cast<uint32_t *>(qd + KV_MAX_GROUP * 8);          // [8 heads][KV_Q_STRIDE]: 8 blocks x 8 words
+    float *inbox = reinterpret_cast<float *>(q8 + KV_MAX_GROUP * KV_Q_STRIDE);   // PUSH: [CL ranks][GRP heads][dims of a slice], from every CTA of the cluster
+    float2 *inbox_ml = reinterpret_cast<float2 *>(inbox + KV_MAX_GROUP * KV_D);  // PUSH: [CL ranks][8 heads] (m, l)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -205,7 +236,7 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
 
     auto issue = [&](int i) {           // one thread
         const uint64_t pol = policy_evict_first();
-        const int p0 = p_begin + i * KV_TILE, n = min(KV_TILE, p_end - p0), b = i % KV_BUFS;
+        const int p0 = p_begin + i * KV_TILE, n = min(KV_TILE, p_end - p0), b = i % BUFS;
         const uint32_t bytes = (uint32_t)n * KV_ROW;
         uint8_t *dst = raw + (size_t)b * 2 * KV_HALF_BYTES;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -214,49 +245,64 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
         mbar_expect_tx(&vfull[b], bytes);
         bulk_g2s(dst + KV_HALF_BYTES, vbase + (size_t)p0 * KV_ROW, bytes, &vfull[b], pol);
     };
+    float4 *halves = reinterpret_cast<float4 *>(inbox_ml + KV_WIDE_CLUSTER * KV_MAX_GROUP);      // PUSH: [8 warps][32] scores over half of the dims
     if (tid == 0) {
-        for (int b = 0; b < KV_BUFS; ++b) mbar_init(&kfull[b], 1), mbar_init(&vfull[b], 1);
+        for (int b = 0; b < BUFS; ++b) mbar_init(&kfull[b], 1), mbar_init(&vfull[b], 1);
+        mbar_init(met, 1);
         mbar_fence_init();
+        if (PUSH) mbar_expect_tx(met, CL * GRP * (KV_D / CL * 4 + 8));
     }
-    for (int i = tid; i < KV_MAX_GROUP * KV_WT_STRIDE; i += KV_THREADS) wt[i] = 0.0f;      // heads past the group stay 0
-    for (int i = tid; i < KV_MAX_GROUP * 8; i += KV_THREADS) qd[i] = 0.0f, mw[i] = 0.0f, lw[i] = 0.0f;
-    for (int i = tid; i < KV_MAX_GROUP * 64; i += KV_THREADS) q8[i] = 0u;
+    for (int i = tid; i < KV_MAX_GROUP * KV_WT_STRIDE; i += THREADS) wt[i] = 0.0f;      // heads past the group stay 0
+    for (int i = tid; i < KV_MAX_GROUP * 8; i += THREADS) qd[i] = 0.0f, mw[i] = 0.0f, lw[i] = 0.0f;
+    for (int i = tid; i < KV_MAX_GROUP * KV_Q_STRIDE; i += THREADS) q8[i] = 0u;
     __syncthreads();
+    if (PUSH) cluster_arrive();          // the others may write into this CTA's shared memory
     pdl_wait_prior_grid();              // q and the newest row of the cache come from the kernels before this one
     pdl_launch_dependents();
     if (tid == 0)
-        for (int i = 0; i < min(ntiles, KV_BUFS); ++i) issue(i);
+        for (int i = 0; i < min(ntiles, BUFS); ++i) issue(i);
     // the group's query heads, quantised as the cache rows are (host rule, src/kv_cache.h:100-117)
     {
-        constexpr int ROUNDS = (GRP + KV_WARPS - 1) / KV_WARPS;
+        constexpr int ROUNDS = (GRP + WARPS - 1) / WARPS;
         const int blk = lane >> 2, sub = lane & 3;
-        float x[ROUNDS][8];
+        float x[ROUNDS][8], amax[ROUNDS];
 #pragma unroll
         for (int r = 0; r < ROUNDS; ++r) {          // every load first: one trip to memory
-            const int h = warp + r * KV_WARPS;
+            const int h = warp + r * WARPS;
             const float *qr = q + (size_t)(kvh * GRP + (h < GRP ? h : 0)) * KV_D + blk * 32 + sub * 8;
+            if ((reinterpret_cast<uintptr_t>(q) & 15u) == 0) {
+                const float4 a = *reinterpret_cast<const float4 *>(qr), c = *reinterpret_cast<const float4 *>(qr + 4);
+                x[r][0] = a.x; x[r][1] = a.y; x[r][2] = a.z; x[r][3] = a.w; x[r][4] = c.x; x[r][5] = c.y; x[r][6] = c.z; x[r][7] = c.w;
+            } else {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) x[r][i] = qr[i];
+                for (int i = 0; i < 8; ++i) x[r][i] = qr[i];
+            }
         }
 #pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) amax[r] = kv_amax_8(x[r]);
+        // the divisions of round r by lane r of the four
+        static_assert(ROUNDS <= 4, "a lane of the four per round");
+        float mine = amax[0];
+#pragma unroll
+        for (int r = 1; r < ROUNDS; ++r) mine = sub == r ? amax[r] : mine;
+        const float d = __fdiv_rn(mine, 127.0f), my_id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+        if (warp + sub * WARPS < GRP && sub < ROUNDS) qd[(warp + sub * WARPS) * 8 + blk] = __fmul_rn(f16_bits_to_f32(f32_to_f16_bits_ties_away(d)), scale);
+#pragma unroll
         for (int r = 0; r < ROUNDS; ++r) {
-            const int h = warp + r * KV_WARPS;
-            float d;
+            const int h = warp + r * WARPS;
+            const float id = __shfl_sync(0xffffffffu, my_id, (lane & ~3) + r);
             uint32_t w[2];
-            kv_quantise_8(x[r], d, w);
-            if (h < GRP) {
-                q8[(h * 8 + blk) * 8 + 2 * sub] = w[0];
-                q8[(h * 8 + blk) * 8 + 2 * sub + 1] = w[1];
-                if (sub == 0) qd[h * 8 + blk] = __fmul_rn(f16_bits_to_f32(f32_to_f16_bits_ties_away(d)), scale);
-            }
+            kv_words_8(x[r], id, w);
+            if (h < GRP) *reinterpret_cast<uint2 *>(q8 + h * KV_Q_STRIDE + blk * 8 + 2 * sub) = make_uint2(w[0], w[1]);
         }
     }
     __syncthreads();
     // B operand of the scores: head g, words t and t + 4 of every block, in the order the K rows are read in
-    uint32_t qb[8][2];
+    constexpr int QB = PUSH ? 4 : 8;                         // blocks of a warp
+    uint32_t qb[QB][2];
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        const uint32_t *src = q8 + (g * 8 + b) * 8;
+    for (int b = 0; b < QB; ++b) {
+        const uint32_t *src = q8 + g * KV_Q_STRIDE + (PUSH ? QB * (warp >> 2) + b : b) * 8;
         if (b & 1) {
             qb[b][0] = src[t];
             qb[b][1] = src[t + 4];
@@ -265,11 +311,12 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
             qb[b][1] = __byte_perm(src[t + 3], src[t + 4], 0x5432);
         }
     }
+    const bool odd = NB == 1 && (warp & 1);                 // a warp of one block: whether it is the pair's second
     float m_run = -INFINITY, l_run = 0.0f;                  // of head g
     int top_run = 1;                                        // fp16 exponent of the largest V scale so far in the warp's two blocks
-    float acc[2][4][4];
+    float acc[NB][4][4];
 #pragma unroll
-    for (int b = 0; b < 2; ++b)
+    for (int b = 0; b < NB; ++b)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -278,19 +325,21 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
     // fp16 pair below.
     constexpr int LIFT = 127 + 13 + 15;
 
-    for (int i = 0; i < ntiles; ++i) {
-        const int b = i % KV_BUFS;
-        const uint32_t par = (uint32_t)((i / KV_BUFS) & 1);
+    for (int i = 0; i < (PUSH == 1 ? min(ntiles, 1) : ntiles); ++i) {
+        const int b = i % BUFS;
+        const uint32_t par = (uint32_t)((i / BUFS) & 1);
         const int n = min(KV_TILE, p_end - (p_begin + i * KV_TILE));
         uint8_t *kt = raw + (size_t)b * 2 * KV_HALF_BYTES, *vt = kt + KV_HALF_BYTES;
         bool ok = mbar_wait_hot(&kfull[b], par);
-        {   // ---- scores of positions 16 warp .. + 15
-            const uint32_t *r0 = reinterpret_cast<const uint32_t *>(kt) + (size_t)(16 * warp + g) * (KV_ROW / 4);
+        {   // ---- scores of positions 16 (warp % 4) .. + 15; of eight warps over half of the dims each
+            const int pw = warp & 3;
+            const uint32_t *r0 = reinterpret_cast<const uint32_t *>(kt) + (size_t)(16 * pw + g) * (KV_ROW / 4);
             const uint32_t *r1 = r0 + 8 * (KV_ROW / 4);
             float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};          // (position g | g + 8, head 2 t | 2 t + 1), even blocks
             float so[4] = {0.0f, 0.0f, 0.0f, 0.0f};         // odd blocks: two short sums round less than a long one
 #pragma unroll
-            for (int pr = 0; pr < 4; ++pr) {
+            for (int i4 = 0; i4 < (PUSH ? 2 : 4); ++i4) {
+                const int pr = PUSH ? 2 * (warp >> 2) + i4 : i4;
                 const uint32_t *u0 = r0 + 17 * pr, *u1 = r1 + 17 * pr;
                 const uint32_t d0 = u0[0], d1 = u1[0], e0 = u0[8], e1 = u1[8];
                 uint32_t x0 = u0[t], x1 = u1[t];
@@ -300,8 +349,8 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
                     x1 = __byte_perm(x1, e1, 0x5432);
                 }
                 int de[4], dq[4];
-                mma_s8_16832(de, x0, x1, y0, y1, qb[2 * pr][0], qb[2 * pr][1]);
-                mma_s8_16832(dq, u0[9 + t], u1[9 + t], u0[13 + t], u1[13 + t], qb[2 * pr + 1][0], qb[2 * pr + 1][1]);
+                mma_s8_16832(de, x0, x1, y0, y1, qb[2 * i4][0], qb[2 * i4][1]);
+                mma_s8_16832(dq, u0[9 + t], u1[9 + t], u0[13 + t], u1[13 + t], qb[2 * i4 + 1][0], qb[2 * i4 + 1][1]);
                 const float ke0 = half_bits_lo(d0), ke1 = half_bits_lo(d1), ko0 = half_bits_hi(e0), ko1 = half_bits_hi(e1);
                 const float qe0 = qd[(2 * t) * 8 + 2 * pr], qe1 = qd[(2 * t + 1) * 8 + 2 * pr];
                 const float qo0 = qd[(2 * t) * 8 + 2 * pr + 1], qo1 = qd[(2 * t + 1) * 8 + 2 * pr + 1];
@@ -316,7 +365,13 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) s[e] = __fadd_rn(s[e], so[e]);
-            const int pa = 16 * warp + g, pb = pa + 8;
+            if (PUSH) {                              // the two warps of a group add their halves, both in the same order
+                halves[warp * 32 + lane] = make_float4(s[0], s[1], s[2], s[3]);
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + pw) : "memory");
+                const float4 a = halves[pw * 32 + lane], c = halves[(pw + 4) * 32 + lane];
+                s[0] = __fadd_rn(a.x, c.x); s[1] = __fadd_rn(a.y, c.y); s[2] = __fadd_rn(a.z, c.z); s[3] = __fadd_rn(a.w, c.w);
+            }
+            const int pa = 16 * pw + g, pb = pa + 8;
             const bool va = pa < n, vb = pb < n;
             float mx0 = fmaxf(va ? s[0] : -INFINITY, vb ? s[2] : -INFINITY), mx1 = fmaxf(va ? s[1] : -INFINITY, vb ? s[3] : -INFINITY);
 #pragma unroll
@@ -332,30 +387,33 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
                 l0 = __fadd_rn(l0, __shfl_xor_sync(0xffffffffu, l0, o));
                 l1 = __fadd_rn(l1, __shfl_xor_sync(0xffffffffu, l1, o));
             }
-            if (2 * t < GRP) {
+            if (2 * t < GRP && warp < 4) {
                 wt[(2 * t) * KV_WT_STRIDE + pa] = w0;
                 wt[(2 * t) * KV_WT_STRIDE + pb] = w2;
                 if (g == 0) mw[warp * 8 + 2 * t] = mx0, lw[warp * 8 + 2 * t] = l0;
             }
-            if (2 * t + 1 < GRP) {
+            if (2 * t + 1 < GRP && warp < 4) {
                 wt[(2 * t + 1) * KV_WT_STRIDE + pa] = w1;
                 wt[(2 * t + 1) * KV_WT_STRIDE + pb] = w3;
                 if (g == 0) mw[warp * 8 + 2 * t + 1] = mx1, lw[warp * 8 + 2 * t + 1] = l1;
             }
         }
         ok = mbar_wait_hot(&vfull[b], par) && ok;
-        if (n < KV_TILE)                // rows past the end: zeros (their weights are 0, but stale scales need not be finite)
-            for (int z = tid; z < (KV_TILE - n) * (KV_ROW / 4); z += KV_THREADS) reinterpret_cast<uint32_t *>(vt)[n * (KV_ROW / 4) + z] = 0u;
+        if (n < KV_TILE)                // rows past the end: scales of zero (their weights are 0, but stale scales need not be finite)
+            for (int z = tid; z < (KV_TILE - n) * 8; z += THREADS)
+                reinterpret_cast<uint32_t *>(vt)[(n + (z >> 3)) * (KV_ROW / 4) + 17 * ((z >> 1) & 3) + 8 * (z & 1)] = 0u;
         // (the outcome of the bounded waits is made uniform: a CTA either goes on as a whole or leaves as a whole)
         if (!__syncthreads_and(ok ? 1 : 0)) break;
-        {   // ---- values: dims 64 warp .. + 63
-            const uint32_t *v32 = reinterpret_cast<const uint32_t *>(vt) + 17 * warp;
+        {   // ---- values: dims 64 warp .. + 63, of eight warps 32 warp .. + 31
+            const uint32_t *v32 = reinterpret_cast<const uint32_t *>(vt) + 17 * (NB == 2 ? warp : warp >> 1);
             uint32_t exps;                                  // which fp16 exponents the tile's scales have (0: none but zeros)
             {
                 const uint32_t *ra = v32 + (size_t)lane * (KV_ROW / 4), *rb = ra + 32 * (KV_ROW / 4);
                 auto exponent = [](uint32_t scale) { return min(scale, 1u) << (scale >> 10); };
-                exps = __reduce_or_sync(0xffffffffu, exponent(ra[0] & 0x7FFFu) | exponent(rb[0] & 0x7FFFu) | exponent((ra[8] >> 16) & 0x7FFFu) |
-                                                         exponent((rb[8] >> 16) & 0x7FFFu));
+                uint32_t mine = 0;
+                if (NB == 2 || !odd) mine |= exponent(ra[0] & 0x7FFFu) | exponent(rb[0] & 0x7FFFu);
+                if (NB == 2 || odd) mine |= exponent((ra[8] >> 16) & 0x7FFFu) | exponent((rb[8] >> 16) & 0x7FFFu);
+                exps = __reduce_or_sync(0xffffffffu, mine);
             }
             float mc[4], m_new = m_run, f[4], lsum = 0.0f;
 #pragma unroll
@@ -375,7 +433,7 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
             top_run = top;
             if (__any_sync(0xffffffffu, keep != 1.0f)) {
 #pragma unroll
-                for (int bb = 0; bb < 2; ++bb)
+                for (int bb = 0; bb < NB; ++bb)
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -385,39 +443,41 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
             // a split in one accumulator: relative error 3.2e-7 at 32768 positions, 2.6e-7 on the CUDA cores).
             auto weigh = [&](auto rest) {                   // rest: the second pass, over what the planes of the first left
                 constexpr bool REST = decltype(rest)::value;
-                float sum[2][4][4];
+                float sum[NB][4][4];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     if (16 * c >= n) break;                     // CTA-uniform
                     if ((c & 1) == 0) {
 #pragma unroll
-                        for (int bb = 0; bb < 2; ++bb)
+                        for (int bb = 0; bb < NB; ++bb)
 #pragma unroll
                             for (int j = 0; j < 4; ++j)
 #pragma unroll
                                 for (int e = 0; e < 4; ++e) sum[bb][j][e] = 0.0f;
                     }
                     const uint32_t *rows = v32 + (size_t)(16 * c + 2 * t) * (KV_ROW / 4);
-                    uint32_t ev[4], od[4];
-                    float de[4], dq[4];
+                    uint32_t vals[NB][4];                       // four rows' bytes of a block, and their scales
+                    float vd[NB][4];
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
                         const uint32_t *u = rows + (size_t)((r & 1) + 8 * (r >> 1)) * (KV_ROW / 4);
                         const uint32_t d0 = u[0], e = u[8];
-                        uint32_t x = u[g];
-                        if (g == 0) x = __byte_perm(x, e, 0x5432);
-                        ev[r] = x ^ 0x80808080u;
-                        od[r] = u[9 + g] ^ 0x80808080u;
-                        de[r] = half_bits_lo(d0);
-                        dq[r] = half_bits_hi(e);
+                        uint32_t x = NB == 1 && odd ? u[9 + g] : u[g];
+                        if (g == 0 && !odd) x = __byte_perm(x, e, 0x5432);
+                        vals[0][r] = x ^ 0x80808080u;
+                        vd[0][r] = NB == 1 && odd ? half_bits_hi(e) : half_bits_lo(d0);
+                        if constexpr (NB == 2) {
+                            vals[1][r] = u[9 + g] ^ 0x80808080u;
+                            vd[1][r] = half_bits_hi(e);
+                        }
                     }
                     const float2 wa = *reinterpret_cast<const float2 *>(wt + g * KV_WT_STRIDE + 16 * c + 2 * t);
                     const float2 wb = *reinterpret_cast<const float2 *>(wt + g * KV_WT_STRIDE + 16 * c + 2 * t + 8);
                     const float fu = __fmul_rn(f[c], up);
 #pragma unroll
-                    for (int bb = 0; bb < 2; ++bb) {
-                        const float *dd = bb ? dq : de;
-                        const uint32_t *vv = bb ? od : ev;
+                    for (int bb = 0; bb < NB; ++bb) {
+                        const float *dd = vd[bb];
+                        const uint32_t *vv = vals[bb];
                         uint32_t h01, l01, h23, l23;
                         const float p0 = __fmul_rn(__fmul_rn(wa.x, fu), dd[0]), p1 = __fmul_rn(__fmul_rn(wa.y, fu), dd[1]);
                         const float p2 = __fmul_rn(__fmul_rn(wb.x, fu), dd[2]), p3 = __fmul_rn(__fmul_rn(wb.y, fu), dd[3]);
@@ -441,7 +501,7 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
                     }
                     if ((c & 1) == 1 || 16 * (c + 1) >= n) {
 #pragma unroll
-                        for (int bb = 0; bb < 2; ++bb)
+                        for (int bb = 0; bb < NB; ++bb)
 #pragma unroll
                             for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -452,36 +512,89 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
             weigh(std::false_type{});
             if (__builtin_expect(wide, 0)) weigh(std::true_type{});
         }
-        __syncthreads();                                            // tile i's buffer and the tables may be overwritten
-        if (tid == 0 && i + KV_BUFS < ntiles) issue(i + KV_BUFS);
+        if (PUSH != 1) __syncthreads();                             // tile i's buffer and the tables may be overwritten
+        if (PUSH != 1 && tid == 0 && i + BUFS < ntiles) issue(i + BUFS);
+    }
+    constexpr int SLICE = KV_D / CL;
+    constexpr int OUTS = GRP * SLICE, ROUNDS = (OUTS + THREADS - 1) / THREADS;
+    const float down = __uint_as_float((uint32_t)(254 - LIFT + top_run) << 23);
+    auto part_of = [&](int bb, int j, int e) {                  // (of an infinity the low plane is NaN: the high plane alone is the sum then)
+        const float high = acc[bb][j][e], both = isinf(high) ? high : __fadd_rn(high, acc[bb][j][e + 2]);
+        return __fmul_rn(both, down);
+    };
+    if constexpr (PUSH) {
+        // ---- every CTA's (m, l) goes to all of the cluster, its slices to the CTA that merges them, which counts the bytes: one trip, and nobody
+        // reads another's memory
+        cluster_wait();                                         // all have started
+        const uint32_t me = cluster_rank();
+        if (g < GRP) {
+            float *box = inbox + ((int)me * GRP + g) * SLICE;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int slot = 2 * t + e, dim = 32 * warp;
+                if (odd) {
+                    const int at = dim + 4 * slot;
+                    st_async_f32x4(box + at % SLICE, met, (uint32_t)(at / SLICE), part_of(0, 0, e), part_of(0, 1, e), part_of(0, 2, e), part_of(0, 3, e));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; j += 2) {            // the even block's values go in pairs: slot 0 has 0, 1 and 30, 31
+                        const int at = dim + (slot == 0 ? (j == 0 ? 0 : 30) : 4 * slot - 2 + j);
+                        st_async_f32x2(box + at % SLICE, met, (uint32_t)(at / SLICE), part_of(0, j, e), part_of(0, j + 1, e));
+                    }
+                }
+            }
+            if (warp < CL / 4) st_async_f32x2(reinterpret_cast<float *>(inbox_ml + me * KV_MAX_GROUP + g), met, (uint32_t)(4 * warp + t), m_run, l_run);
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait_hot(met, 0))) {  // (nobody's bytes may find this CTA gone)
+            cluster_arrive();
+            cluster_wait();
+            return;
+        }
+        if (tid / 32 * 32 >= OUTS) return;
+        const int o = min(tid, OUTS - 1), h = o / SLICE, rr = lane & (CL - 1);
+        static_assert(OUTS <= THREADS && (CL == SLICE || 32 % SLICE == 0) && CL <= SLICE, "lane rr of a head's CL weighs rank rr");
+        float part[CL];
+#pragma unroll
+        for (int r = 0; r < CL; ++r) part[r] = inbox[r * OUTS + o];
+        const float2 ml = inbox_ml[rr * KV_MAX_GROUP + h];
+        float mx = ml.x;
+#pragma unroll
+        for (int i = 1; i < CL; i <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, i));
+        const float w = ml.x == -INFINITY ? 0.0f : expf(__fsub_rn(ml.x, mx));          // a split without positions: 0
+        float den = __fmul_rn(ml.y, w);
+#pragma unroll
+        for (int i = 1; i < CL; i <<= 1) den = __fadd_rn(den, __shfl_xor_sync(0xffffffffu, den, i));
+        const float inv = __fdiv_rn(1.0f, den);
+        float chain[CL / 4];                                    // of four ranks: sixteen in one sum round more than eight did
+#pragma unroll
+        for (int r = 0; r < CL; ++r) chain[r / 4] = __fmaf_rn(part[r], __shfl_sync(0xffffffffu, w, (lane & ~(CL - 1)) + r), r % 4 ? chain[r / 4] : 0.0f);
+        float a = __fadd_rn(chain[0], chain[1]);
+        if (CL == 16) a = __fadd_rn(a, __fadd_rn(chain[2], chain[CL / 4 - 1]));
+        if (tid < OUTS) out[(size_t)kvh * GRP * KV_D + h * KV_D + (int)me * SLICE + o % SLICE] = __fmul_rn(a, inv);
+        return;
     }
     // ---- the CTA's (m, l, acc); the tile buffers are free
     float *so = reinterpret_cast<float *>(raw), *sm = so + KV_MAX_GROUP * KV_D, *sl = sm + KV_MAX_GROUP;
     if (g < GRP) {
 #pragma unroll
-        for (int bb = 0; bb < 2; ++bb) {
-            const float down = __uint_as_float((uint32_t)(254 - LIFT + top_run) << 23);
+        for (int bb = 0; bb < NB; ++bb)
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int slot = 2 * t + e;
                     const int in_blk = bb ? 4 * slot + j : (slot == 0 ? (j < 2 ? j : 28 + j) : 4 * slot - 2 + j);
-                    // (of an infinity the low plane is NaN: the high plane alone is the sum then)
-                    const float high = acc[bb][j][e], both = isinf(high) ? high : __fadd_rn(high, acc[bb][j][e + 2]);
-                    so[g * KV_D + 64 * warp + 32 * bb + in_blk] = __fmul_rn(both, down);
+                    so[g * KV_D + 64 * warp + 32 * bb + in_blk] = part_of(bb, j, e);
                 }
-        }
         if (warp == 0 && t == 0) sm[g] = m_run, sl[g] = l_run;
     }
     cluster_arrive();
     cluster_wait();
     // ---- one slice of the dims per CTA of the cluster, added over its CTAs in rank order
     const uint32_t rank = cluster_rank();
-    const int n_cl = CL == KV_CLUSTER ? gridDim.x / CL : 1, cl = CL == KV_CLUSTER ? blockIdx.x / CL : 0;      // (records and counters are laid out for clusters of eight)
-    constexpr int SLICE = KV_D / CL;
+    const int n_cl = gridDim.x / CL, cl = blockIdx.x / CL;
+    static_assert(PUSH || CL == KV_CLUSTER, "records and counters are laid out for clusters of eight");
     float *cw = wt, *cm = mw, *cl_sum = lw;                            // [8 heads][CL ranks] weights; maxima; denominators
-    constexpr int OUTS = GRP * SLICE, ROUNDS = (OUTS + KV_THREADS - 1) / KV_THREADS;
     float part[ROUNDS][CL];
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
@@ -514,15 +627,10 @@ __global__ void __launch_bounds__(KV_THREADS, 3) kv_attn_kernel(const float *q, 
         const int o = tid + r * KV_THREADS;
         if (o < OUTS) {
             const int h = o / SLICE;
-            float chain[CL / 4];                // of four ranks: sixteen in one sum round more than eight did
+            float chain[2] = {0.0f, 0.0f};      // of four ranks
 #pragma unroll
-            for (int c = 0; c < CL / 4; ++c) {
-                chain[c] = 0.0f;
-#pragma unroll
-                for (int rr = 4 * c; rr < 4 * c + 4; ++rr) chain[c] = __fmaf_rn(part[r][rr], cw[h * CL + rr], chain[c]);
-            }
-            float a = __fadd_rn(chain[0], chain[1]);
-            if (CL == 16) a = __fadd_rn(a, __fadd_rn(chain[2], chain[CL / 4 - 1]));
+            for (int rr = 0; rr < CL; ++rr) chain[rr / 4 % 2] = __fmaf_rn(part[r][rr], cw[h * CL + rr], chain[rr / 4 % 2]);
+            const float a = __fadd_rn(chain[0], chain[1]);
             if (n_cl == 1) out_slice[h * KV_D + o % SLICE] = __fmul_rn(a, __fdiv_rn(1.0f, cl_sum[h]));
             else rec[o] = a;
         }

@@ -158,6 +158,20 @@ def test_append_at_odd_offsets(gpu):
     kv.close()
 
 
+@pytest.mark.parametrize("n", [16, 65, 512, 513, 1024, 1025, 3071, 3072])
+def test_query_and_output_at_odd_offsets(gpu, n):
+    """A query that is not 16-byte aligned is read by words, outputs are stored by words: the bits of aligned ones."""
+    import torch
+    kv = gpu.KVCache(n)
+    q = fill(kv, 3, n, n, 1)
+    odd = torch.empty(q.numel() + 1, device="cuda")
+    odd[1:].copy_(q.view(-1))
+    out, at = torch.full((N_HEADS * D,), float("nan"), device="cuda"), torch.full((N_HEADS * D + 2,), float("nan"), device="cuda")
+    assert kv.attn_decode(3, n - 1, q, out) == 0 and kv.attn_decode(3, n - 1, odd[1:], at[1:-1]) == 0
+    assert torch.equal(out, at[1:-1]) and bool(torch.isnan(at[[0, -1]]).all())
+    kv.close()
+
+
 def test_create_does_not_wait_for_the_stream(gpu):
     """A cache is made while the caller's stream is busy (a kernel of a tenth of a second); decoding on another stream at once finds its
     counters zero."""
