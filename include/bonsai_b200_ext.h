@@ -22,9 +22,9 @@ int bonsai_b200_fwht_quant(const float *x, const float *signs, void *xq, float *
 
 /* One decode projection in one call: xq_scratch = Q8_1(FWHT1024(signs * x)), then y = W . xq_scratch.
  * xq_scratch is caller-provided device memory of n_in / 32 * 36 bytes (4-byte aligned) that the call
- * overwrites; x is left untouched.  Two launches by default; with the option "fuse_linear" = 1 and a shape
- * the streaming mat-vec takes, ONE launch (rotation and quantiser run in the mat-vec's prologue, once per
- * CTA).  Either way y and the scratch equal bonsai_b200_fwht_quant followed by bonsai_p40_gemv.  No counterpart in the reference, whose callers issue the steps themselves
+ * overwrites; x is left untouched.  One launch where that is faster (up to 1920 rows of 5120, 1024 values
+ * whatever the rows) and y and the scratch lie apart from x and signs, else two (option "fuse_linear"); either
+ * way y and the scratch equal bonsai_b200_fwht_quant followed by bonsai_p40_gemv.  No counterpart in the reference, whose callers issue the steps themselves
  * (docs/INTEGRATION.md:260-263).  Returns 1 if n_in % 1024 != 0 or n_out <= 0. */
 int bonsai_b200_linear(const void *W, const float *x, const float *signs, float *y, void *xq_scratch,
                        int64_t n_out, int64_t n_in, bonsai_stream stream);
@@ -145,9 +145,9 @@ int bonsai_b200_stream_probe(const void *buf, int64_t bytes, int mode, void *sin
  * bits every time, a row or a token of it in a call of another shape those of another order, within the bound.  The fp16 form keeps one scratch buffer per (device, stream), 4 bytes per token and input value, and 16 MB for
  * the parts of tiles, allocated with cudaMalloc on first use or growth -- never while the stream is being captured (then the
  * integer form runs).
- * key "fuse_linear": 0 (default) = bonsai_b200_linear is two launches, 1 = one kernel when it can (saves a
- * launch, but every CTA then waits for its own rotation before its first multiply: measured ~6 % slower
- * on the 401-projection decode chain).
+ * key "fuse_linear": bonsai_b200_linear and _linear_static are -1 (default) = one launch where that is faster, else
+ * two; 0 = two launches; 1 = one launch when it can (from several thousand rows on slower than two: every CTA
+ * rotates the vector for itself).
  * Options are process-wide: set them once at start-up, not from threads that call the library concurrently.
  * A library compiled with -DBONSAI_B200_TUNING (the test build) also takes geometry keys ("gemv_variant",
  * "chain_threads", "chain_seg", "chain_tile_kb", "chain_spread_nb", "gemm_tile") that force a tiling; they change no result bits

@@ -15,6 +15,7 @@
 #include "gemv.cuh"
 #include "gemv_stream.cuh"
 #include "gemv_chain.cuh"
+#include "gemv_few.cuh"
 #include "gemv_mma.cuh"
 #include "kv.cuh"
 #include "ops.cuh"
@@ -45,7 +46,7 @@ std::atomic<int> g_opt_pdl{0};
 std::atomic<int> g_opt_overlap{1};             // 0: plain launches, each begins when its predecessor has ended
 std::atomic<int> g_opt_gemv_variant{-1};
 std::atomic<int> g_opt_gemv_order{0};
-std::atomic<int> g_opt_fuse_linear{0};         // 1: bonsai_b200_linear runs as one kernel when it can (measured slower)
+std::atomic<int> g_opt_fuse_linear{-1};        // bonsai_b200_linear: -1 one kernel or two by shape, 0 two, 1 one when it can
 std::atomic<int> g_opt_chain_threads{512};       // threads per CTA of the chain kernel: 512 (5 blocks per lane and task), 640 (4), 768 (3)
 // Dependent ops with at least this many blocks per row rotate their input once for the grid instead of once per CTA; 0 = never.  us per op of a list
 // n -> n, once per CTA / once for the grid: 1024 behind a norm 5.2 / 5.7, 2048 6.4 / 6.2 (plain 5.5 / 5.35), 3072 7.3 / 6.8, 5120 9.6 / 8.1.
@@ -144,7 +145,8 @@ private:
     std::atomic<int> known_[64] = {};
 };
 
-ClusterRoom g_tc16_pairs, g_repack_pairs, g_repack_fours;
+ClusterRoom g_tc16_pairs, g_repack_pairs, g_repack_fours, g_few_clusters[FEW_MAX_CLUSTER + 1];
+SmemOptIn g_few_opt[FEW_HELD];
 
 // ceil(2^32 / d): __umulhi(n, magic) == n / d for every n with n * d < 2^32; 0 stands for d == 1.
 inline uint32_t magic_u32(uint32_t d) {
@@ -154,7 +156,8 @@ inline uint32_t magic_u32(uint32_t d) {
 
 // Geometry of the streaming mat-vec (gemv_stream.cuh).
 // variant = thr_code * 1000 + seg_code * 100 + tile_code * 10 + cap_code, -1 = default.
-bool plan_stream(long long n_out, int nb, int variant, StreamParams &p, int &threads, int &smem_bytes) {
+// `behind`: bytes of shared memory kept free behind the ring, taken from it.
+bool plan_stream(long long n_out, int nb, int variant, StreamParams &p, int &threads, int &smem_bytes, int behind = 0) {
     if (nb % 2 != 0) return false;                  // rows must start on a word boundary
     int seg = 8 * STREAM_STEPS, tile_kb = 16, cap_kb = 108;
     threads = 512;
@@ -183,7 +186,7 @@ bool plan_stream(long long n_out, int nb, int variant, StreamParams &p, int &thr
     p.nseg = (nb + p.seg_blocks - 1) / p.seg_blocks;
     for (int attempt = 0;; ++attempt) {
         const size_t fixed = 2 * RING_MAX_TILES * 8 + (size_t)nb * (STREAM_ACT_WORDS * 4 + 32) +
-                             (size_t)rows * p.nseg * 4 + (size_t)((rows / 4 + 3) & ~3) * 4 + 16;
+                             (size_t)rows * p.nseg * 4 + (size_t)((rows / 4 + 3) & ~3) * 4 + 16 + (size_t)behind;
         if ((size_t)cap_kb * 1024 < fixed + 64) return false;
         const size_t room = (size_t)cap_kb * 1024 - fixed - 64;
         long long tr = ((long long)tile_kb * 1024 / (long long)row_bytes) & ~3ll;
@@ -571,28 +574,83 @@ int bonsai_p40_gemv(const void *W, const void *xq, float *y, int64_t n_out, int6
     return gemv_launch(W, xq, y, n_out, n_in, stream, false);
 }
 
+// One projection in one launch, rotation and quantiser in the prologue of the streaming mat-vec.  -1: two launches serve.
+static int linear_one_launch(const void *W, const float *x, const float *signs, float *y, void *xq, int64_t n_out, int64_t n_in, bonsai_stream stream) {
+    const int fuse = g_opt_fuse_linear.load();
+    if (g_opt_gemv_order.load() != 0 || fuse == 0 || !aligned16(W) || !aligned16(x) || (signs && !aligned16(signs)) || n_out > INT32_MAX || n_in > INT32_MAX) return -1;
+    // (of two launches the second may overwrite what the first has read: here CTAs still read it)
+    auto apart = [&](const float *p) {
+        const auto lo = reinterpret_cast<uintptr_t>(p), hi = lo + 4 * (uintptr_t)n_in, y0 = reinterpret_cast<uintptr_t>(y), q0 = reinterpret_cast<uintptr_t>(xq);
+        return !p || ((hi <= y0 || y0 + 4 * (uintptr_t)n_out <= lo) && (hi <= q0 || q0 + (uintptr_t)n_in / 32 * A_BLOCK_BYTES <= lo));
+    };
+    if (!apart(x) || !apart(signs)) return -1;
+    const int nb = (int)(n_in / 128), nfb = nb / 8;
+    StreamParams sp;
+    int threads = 0, smem_bytes = 0;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = as_stream(stream);
+    const uint8_t *w8 = static_cast<const uint8_t *>(W);
+    uint32_t *blocks = static_cast<uint32_t *>(xq);
+    // The kernel for few rows: as few row quads per CTA as let every CTA find an SM of its own, at most two pieces per warp.  Clusters of nfb CTAs
+    // of which two fit an SM are packed two to an SM from FEW_ALONE[nfb] of them on (us for that many and for one more: 3072 wide 3.35 and 4.00, 4096
+    // 3.31 and 3.68, 5120 3.52 and 3.85, 6144 4.04 and 4.60, 7168 4.18 and 5.24).  us, two launches / one (calls; with a graph's replay): 1024 -> 64 3.96 / 2.70 (3.26 /
+    // 2.45), -> 4096 4.36 / 3.03; 3072 -> 1500 4.80 / 3.45; 5120 -> 64 4.54 / 3.24 (3.78 / 3.04), -> 1024 4.92 / 3.91 (3.88 / 3.68), -> 1850 5.38 / 4.10;
+    // 6144 -> 1000 5.15 / 4.22; 8192 -> 600 5.48 / 4.44.  With more pieces per warp, two blocks per CTA or CTAs two to an SM a graph's replay of two launches
+    // is ahead: 5120 -> 3000 5.70 / 5.61 (4.84 / 5.28), 9216 -> 600 5.54 / 5.00 (4.40 / 4.80), 4096 -> 1500 in 32 clusters 5.07 / 4.41 (3.90 / 4.18).
+    if (nfb <= FEW_MAX_CLUSTER && plan_stream(n_out, nb, -1, sp, threads, smem_bytes)) {
+        static const int FEW_ALONE[FEW_MAX_CLUSTER + 1] = {0, SM_COUNT, 74, 44, 24, 24, 15, 15, 15};
+        const int room = nfb == 1 ? SM_COUNT : g_few_clusters[nfb].ask(gemv_few_kernel<FEW_HELD>, g_few_opt[FEW_HELD - 1], (unsigned)nfb, 32 * FEW_WARPS);
+        const long long most = std::min(room, FEW_ALONE[nfb]), quads_in_all = (n_out + 3) / 4;
+        const long long need = most > 0 ? (quads_in_all + most * nfb - 1) / (most * nfb) : FEW_HELD * FEW_WARPS + 1;
+        if (need * nfb <= (nfb == 1 ? 1 : FEW_HELD) * FEW_WARPS) {
+            const int quads = (int)need;
+            const unsigned clusters = (unsigned)((quads_in_all + (long long)quads * nfb - 1) / ((long long)quads * nfb));
+            attr[0].val.clusterDim.x = (unsigned)nfb;
+            cfg.gridDim = dim3(clusters * (unsigned)nfb);
+            cfg.blockDim = dim3(32 * FEW_WARPS);
+            cfg.dynamicSmemBytes = (size_t)few_smem_bytes(nb, quads);
+            cfg.attrs = nfb == 1 ? attr + 1 : attr;
+            cfg.numAttrs = (nfb > 1) + (g_opt_overlap.load() != 0);
+            auto go = [&](auto kernel, SmemOptIn &o) -> cudaError_t {
+                const cudaError_t err = o.ensure(kernel);
+                if (err != cudaSuccess) return err;
+                const int rows = (int)n_out, seg_steps = sp.seg_blocks / 8;
+                return nfb > 1 ? launch_clusters(cfg, kernel, w8, x, signs, y, blocks, rows, nb, seg_steps, quads) : cudaLaunchKernelEx(&cfg, kernel, w8, x, signs, y, blocks, rows, nb, seg_steps, quads);
+            };
+            const cudaError_t err = quads * nfb <= FEW_WARPS ? go(gemv_few_kernel<1>, g_few_opt[0]) : go(gemv_few_kernel<2>, g_few_opt[1]);
+            if (nfb == 1 || !g_few_clusters[nfb].refused(err)) return (int)err;
+        }
+    }
+    // One block of 1024, whatever the rows: every CTA rotates it for itself (us, two launches / one: -> 10240 5.27 / 4.40, -> 40000 8.51 / 7.54; 2048 wide a graph's
+    // replay of two launches is ahead: -> 17408 6.97 / 6.50 (5.84 / 6.05), 5120 wide calls are too: -> 17408 10.91 / 12.17).
+    if (fuse < 0 && nfb > 1) return -1;
+    if (!plan_stream(n_out, nb, g_opt_gemv_variant.load(), sp, threads, smem_bytes, std::min(nfb, LIN_BLOCKS) * FWHT_N * 4) || threads != 512) return -1;
+    sp.early = g_opt_pdl.load() != 0;
+    static SmemOptIn opt;
+    const cudaError_t err = opt.ensure(gemv_stream_kernel<true>);
+    if (err != cudaSuccess) return (int)err;
+    return (int)launch(gemv_stream_kernel<true>, dim3((unsigned)((n_out + sp.rows_per_cta - 1) / sp.rows_per_cta)), dim3(threads), (size_t)smem_bytes, as_stream(stream),
+                       true, w8, static_cast<const uint32_t *>(nullptr), y, sp, x, signs, blocks);
+}
+
+static int linear_launch(const void *W, const float *x, const float *signs, float *y, void *xq, int64_t n_out, int64_t n_in, bonsai_stream stream) {
+    const int one = linear_one_launch(W, x, signs, y, xq, n_out, n_in, stream);
+    if (one >= 0) return one;
+    const int rc = bonsai_b200_fwht_quant(x, signs, xq, nullptr, n_in, stream);
+    if (rc != 0) return rc;
+    return gemv_launch(W, xq, y, n_out, n_in, stream, true);
+}
+
 int bonsai_b200_linear(const void *W, const float *x, const float *signs, float *y, void *xq_scratch, int64_t n_out,
                        int64_t n_in, bonsai_stream stream) {
     if (n_out <= 0 || n_in <= 0 || n_in % FWHT_N != 0 || !xq_scratch) return 1;
     if (n_out > INT32_MAX || !aligned4(x) || (signs && !aligned4(signs)) || !aligned4(xq_scratch)) return 1;
-    // one launch when the streaming mat-vec takes the shape: rotation and quantiser run in its prologue
-    StreamParams sp;
-    int threads = 0, smem_bytes = 0;
-    if (g_opt_gemv_order.load() == 0 && g_opt_fuse_linear.load() != 0 && aligned16(W) && aligned16(x) &&
-        (!signs || aligned16(signs)) &&
-        plan_stream(n_out, (int)(n_in / 128), g_opt_gemv_variant.load(), sp, threads, smem_bytes)) {
-        static SmemOptIn opt;
-        cudaError_t err = opt.ensure(gemv_stream_kernel<true>);
-        if (err != cudaSuccess) return (int)err;
-        sp.early = g_opt_pdl.load() != 0;
-        return (int)launch(gemv_stream_kernel<true>, dim3((unsigned)((n_out + sp.rows_per_cta - 1) / sp.rows_per_cta)),
-                           dim3(threads), (size_t)smem_bytes, as_stream(stream), true,
-                           static_cast<const uint8_t *>(W), static_cast<const uint32_t *>(nullptr), y, sp, x, signs,
-                           static_cast<uint32_t *>(xq_scratch));
-    }
-    const int rc = bonsai_b200_fwht_quant(x, signs, xq_scratch, nullptr, n_in, stream);
-    if (rc != 0) return rc;
-    return gemv_launch(W, xq_scratch, y, n_out, n_in, stream, true);
+    return linear_launch(W, x, signs, y, xq_scratch, n_out, n_in, stream);
 }
 
 // ---- projection without any allocation: the Q8_1 scratch is part of the library image -----------
@@ -617,9 +675,7 @@ int bonsai_b200_linear_static(const void *W, const float *x, const float *signs,
         if (!scratch) return (int)cudaErrorInvalidSymbol;
         scratch_of_device[dev].store(scratch, std::memory_order_release);
     }
-    const int rc = bonsai_b200_fwht_quant(x, signs, scratch, nullptr, n_in, stream);
-    if (rc != 0) return rc;
-    return gemv_launch(W, scratch, y, n_out, n_in, stream, true);
+    return linear_launch(W, x, signs, y, scratch, n_out, n_in, stream);
 }
 
 
@@ -1468,7 +1524,7 @@ int bonsai_b200_set_option(const char *key, int64_t value) {
         return 0;
     }
     if (!std::strcmp(key, "gemm_path")) { g_opt_gemm_path.store((int)value); return 0; }
-    if (!std::strcmp(key, "fuse_linear")) { g_opt_fuse_linear.store(value != 0); return 0; }
+    if (!std::strcmp(key, "fuse_linear")) { g_opt_fuse_linear.store(value < 0 ? -1 : value != 0); return 0; }
 #ifdef BONSAI_B200_TUNING
     // Geometry knobs of the test build (build.py --tuning, the default of this repository's build script): they let the
     // parity tests force every tiling.  A build without the macro has no such keys and always uses the tuned defaults.
@@ -1496,7 +1552,10 @@ int bonsai_b200_set_option(const char *key, int64_t value) {
     if (!std::strcmp(key, "refuse_clusters")) {         // 0 forgets the refusals too
         if (value < 0) return 1;
         g_opt_refuse_clusters.store((int)value);
-        if (value == 0) g_tc16_pairs.forget(), g_repack_pairs.forget(), g_repack_fours.forget();
+        if (value == 0) {
+            g_tc16_pairs.forget(), g_repack_pairs.forget(), g_repack_fours.forget();
+            for (auto &few : g_few_clusters) few.forget();
+        }
         return 0;
     }
     if (!std::strcmp(key, "kv_wide")) { g_opt_kv_wide.store(value != 0); return 0; }

@@ -95,10 +95,6 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// Into CTA `rank`'s shared memory, at the place that `addr` is in this one's.
-__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t rank, uint32_t v) {
-    asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.u32 [a], %2;\n\t}" ::"r"(addr), "r"(rank), "r"(v) : "memory");
-}
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
@@ -111,6 +107,22 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// Into CTA `rank`'s shared memory, at the place that p is in this one's (aligned to what is stored), counted on its barrier at the place of `bar`.
+__device__ __forceinline__ void st_async_u32(const void *p, uint64_t *bar, uint32_t rank, uint32_t a) {
+    asm volatile("{\n\t.reg .u32 x, y;\n\tmapa.shared::cluster.u32 x, %0, %2;\n\tmapa.shared::cluster.u32 y, %1, %2;\n\t"
+                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [x], %3, [y];\n\t}"
+                 ::"r"(smem_u32(p)), "r"(smem_u32(bar)), "r"(rank), "r"(a) : "memory");
+}
+__device__ __forceinline__ void st_async_f32x2(const float *p, uint64_t *bar, uint32_t rank, float a, float b) {
+    asm volatile("{\n\t.reg .u32 x, y;\n\tmapa.shared::cluster.u32 x, %0, %2;\n\tmapa.shared::cluster.u32 y, %1, %2;\n\t"
+                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [x], {%3, %4}, [y];\n\t}"
+                 ::"r"(smem_u32(p)), "r"(smem_u32(bar)), "r"(rank), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void st_async_f32x4(const float *p, uint64_t *bar, uint32_t rank, float a, float b, float c, float d) {
+    asm volatile("{\n\t.reg .u32 x, y;\n\tmapa.shared::cluster.u32 x, %0, %2;\n\tmapa.shared::cluster.u32 y, %1, %2;\n\t"
+                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [x], {%3, %4, %5, %6}, [y];\n\t}"
+                 ::"r"(smem_u32(p)), "r"(smem_u32(bar)), "r"(rank), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 // Bounded wait: returns false (and records the status word) instead of spinning forever.  The
 // barrier is polled with the non-blocking test; between polls the thread sleeps first_ns, 2 first_ns, ... max_ns,

@@ -30,6 +30,7 @@
 namespace b200 {
 
 constexpr int STREAM_STEPS = 5;         // blocks per lane and task: segments hold at most 8 * 5 = 40 blocks
+constexpr int LIN_SLICES = 3, LIN_BLOCKS = 6;       // fused rotation: slices of 128 a warp holds, blocks of 1024 that 16 warps rotate at a time
 constexpr int STREAM_ACT_WORDS = 36;    // per block: 4 chunks x 8 words int8, 4 pad (stride 144 B: 8 blocks, 8 bank groups)
 
 struct StreamParams {
@@ -191,6 +192,29 @@ __device__ __forceinline__ float stream_task_repack(const uint8_t *row, int nb, 
     return acc;
 }
 
+// A lane's word of chunk `chunk` (word lane & 7) and, from a chunk's first lane, its scale and -64 sum into the tables, of every CTA of the cluster: each
+// counts the bytes that it gets on `bar` (CL = 0: of cl CTAs).  (Ordinary stores and the cluster's barrier behind them: 17408 -> 64 repacked 6.72 us with its rotation, 6.58
+// now, -> 5120 13.99 and 13.83.)
+template <int CL>
+__device__ __forceinline__ void put_activation(uint32_t *act_q, float *act_s, int *act_i, uint64_t *bar, int chunk, int lane, uint32_t word, uint32_t header, int cl = CL) {
+    uint32_t *at_q = act_q + (chunk >> 2) * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7);
+    const float s = f16_bits_to_f32(header & 0xFFFFu);
+    const int i = -64 * (int)(short)(header >> 16);
+    if (CL != 1) {
+#pragma unroll
+        for (uint32_t c = 0; c < (uint32_t)cl; ++c) {
+            st_async_u32(at_q, bar, c, word);
+            if ((lane & 7) == 0) {
+                st_async_u32(act_s + chunk, bar, c, __float_as_uint(s));
+                st_async_u32(act_i + chunk, bar, c, (uint32_t)i);
+            }
+        }
+    } else {
+        *at_q = word;
+        if ((lane & 7) == 0) act_s[chunk] = s, act_i[chunk] = i;
+    }
+}
+
 // Shared memory: [full[256] | done[256]] [act int8: nb * 36 words] [act scale: nb * 4 floats]
 // [act -64*sum: nb * 4 ints] [partials: rows_per_cta * nseg floats] [quad counters: rows_per_cta / 4]
 // [task counter] [ring: nslot * (tr * 34 * nb + 16)].
@@ -199,9 +223,9 @@ __device__ __forceinline__ float stream_task_repack(const uint8_t *row, int nb, 
 // Both are single-use (parity 0), so a warp that skipped tiles can never read a stale phase.
 //
 // FUSED = true is the one-launch projection: the CTA takes the fp32 activation vector instead of Q8_1
-// blocks, rotates it (FWHT-1024, one warp per 1024-block) and quantises it straight into its own
+// blocks, rotates it (FWHT-1024, a warp per slice of 128) and quantises it straight into its own
 // shared-memory tables while its first weight tiles are in flight; CTA 0 also writes the Q8_1 blocks
-// to `xq_out` so that the caller's scratch holds what the two-launch form would have left there.
+// to `xq_out` so that the caller's scratch holds what the two-launch form would have left there.  `front` lies behind the ring.
 // REPACK = true (with FUSED) is bonsai_p40_gemv_repack: W is in the repacked layout and x is quantised WITHOUT a
 // rotation (src/kernels/gemv_repack_p40.cu:91-162 fuses exactly that).
 // CL > 1 (with REPACK): the CTAs of a cluster quantise a share of x each and store it into the tables of all of them.
@@ -226,7 +250,16 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
     const int row0 = blockIdx.x * P.rows_per_cta;
     const int rows_here = max(0, min(P.rows_per_cta, P.n_out - row0));
     if (CL == 1 && rows_here == 0) return;
-    if (CL > 1) cluster_arrive();                       // this CTA runs: the others may store into its tables
+    uint64_t *tables = reinterpret_cast<uint64_t *>(next_task + 2);     // CL > 1: every CTA's share of the tables is here
+    if (CL > 1) {
+        if (threadIdx.x == 0) {
+            mbar_init(tables, 1);
+            mbar_fence_init();
+            mbar_expect_tx(tables, (uint32_t)P.nb * 4 * (32 + 4 + 4));
+        }
+        __syncwarp();
+        cluster_arrive();                               // this CTA runs: the others may store into its tables
+    }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nwarps = blockDim.x >> 5;
     const int compute_warps = nwarps - 1;
@@ -274,6 +307,7 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
     pdl_wait_prior_grid();              // activations (and y) belong to the previous kernel until here
     pdl_launch_dependents();            // behind the wait: whatever starts now has only this launch to wait for
     const int first_late = P.early ? min(2, first_fill) : 0;
+    auto put = [&](int chunk, uint32_t word, uint32_t header) { put_activation<CL>(act_q, act_s, act_i, tables, chunk, lane, word, header); };
     if (REPACK) {
         // quantiser without rotation: 128-element slices over the compute warps, SLICES at a time so that their loads fly
         // together (whole 1024-blocks left most warps without work: 1024 x 64 5.1 -> 2.7 us,
@@ -312,30 +346,8 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
                 for (int k = 0; k < N; ++k) v[k][0] = f[k].x, v[k][1] = f[k].y, v[k][2] = f[k].z, v[k][3] = f[k].w;
                 quantise_chunks_8lanes<N>(v, lane, word, header);
 #pragma unroll
-                for (int k = 0; k < N; ++k) {
-                    if (CL > 1 && s0 + k * compute_warps < nb) {
-                        const int sl = CL * (s0 + k * compute_warps) + mine, chunk = 4 * sl + (lane >> 3);
-                        const uint32_t at_q = smem_u32(act_q + sl * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7));
-                        const uint32_t at_s = smem_u32(act_s + chunk), at_i = smem_u32(act_i + chunk);
-#pragma unroll
-                        for (uint32_t c = 0; c < CL; ++c) {
-                            st_cluster_u32(at_q, c, word[k]);
-                            if ((lane & 7) == 0) {
-                                st_cluster_u32(at_s, c, __float_as_uint(f16_bits_to_f32(header[k] & 0xFFFFu)));
-                                st_cluster_u32(at_i, c, (uint32_t)(-64 * (int)(short)(header[k] >> 16)));
-                            }
-                        }
-                    }
-                    const int sl = s0 + k * compute_warps;
-                    if (CL == 1 && sl < P.nb) {
-                        const int chunk = 4 * sl + (lane >> 3);
-                        act_q[sl * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word[k];
-                        if ((lane & 7) == 0) {
-                            act_s[chunk] = f16_bits_to_f32(header[k] & 0xFFFFu);
-                            act_i[chunk] = -64 * (int)(short)(header[k] >> 16);
-                        }
-                    }
-                }
+                for (int k = 0; k < N; ++k)
+                    if (s0 + k * compute_warps < nb) put(4 * (CL * (s0 + k * compute_warps) + mine) + (lane >> 3), word[k], header[k]);
             };
             if (wid < compute_warps && s0 < nb) {                       // warp-uniform
                 if (n == 1) quantise(std::integral_constant<int, 1>());
@@ -345,53 +357,67 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
             }
         }
     } else if (FUSED) {
-        // rotation + quantiser in the prologue: nb / 8 blocks of 1024 activations over the compute warps
+        // Rotation + quantiser in the prologue: a warp per slice of 128, LIN_SLICES slices of a warp side by side; the slices of a block of 1024 meet
+        // in `front`, LIN_BLOCKS blocks at a time.
+        static_assert(REPACK || CL == 1, "projections that share their rotation: gemv_few.cuh");
+        float4 *front = reinterpret_cast<float4 *>(ring + (size_t)P.nslot * slot_bytes);
         const int nfb = P.nb >> 3;
-        bool first = true;
-        for (int fb0 = 0; fb0 < nfb || first; fb0 += compute_warps) {
-            const int fb = fb0 + wid;
-            const bool live = wid < compute_warps && fb < nfb;
-            float v[8][4];
-            if (live) {
+        for (int i0 = 0; i0 < nfb; i0 += LIN_BLOCKS) {
+            const int ns = 8 * min(LIN_BLOCKS, nfb - i0);
+            float v[LIN_SLICES][4];
+            float4 f[LIN_SLICES], sg[LIN_SLICES];
+            auto at = [&](int k) {                      // the warp's slice k, in floats from the start of x
+                return (size_t)i0 * FWHT_N + (wid + nwarps * k) * 128 + 4 * lane;
+            };
 #pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    const float4 f = *reinterpret_cast<const float4 *>(x + (size_t)fb * FWHT_N + r * 128 + 4 * lane);
-                    v[r][0] = f.x; v[r][1] = f.y; v[r][2] = f.z; v[r][3] = f.w;
+            for (int k = 0; k < LIN_SLICES; ++k) {
+                f[k] = sg[k] = make_float4(1.f, 1.f, 1.f, 1.f);
+                if (wid + nwarps * k < ns) {
+                    f[k] = *reinterpret_cast<const float4 *>(x + at(k));
+                    if (signs) sg[k] = *reinterpret_cast<const float4 *>(signs + at(k));
                 }
             }
-            if (first) {
-                // every warp has issued its first loads: the rest of the ring may queue behind them
-                __syncthreads();
-                if (wid == compute_warps && lane == 0)
-                    for (int t = first_late; t < first_fill; ++t) issue_tile(t);
-                first = false;
-            }
-            if (live) {
+            // every warp has issued its loads (and has read what the blocks before left in `front`): the rest of the ring may queue behind them
+            __syncthreads();
+            if (i0 == 0 && wid == compute_warps && lane == 0)
+                for (int t = first_late; t < first_fill; ++t) issue_tile(t);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < LIN_SLICES; ++k) {
+                if (wid + nwarps * k >= ns) break;                      // warp-uniform
+                v[k][0] = f[k].x; v[k][1] = f[k].y; v[k][2] = f[k].z; v[k][3] = f[k].w;
                 if (signs) {
-#pragma unroll
-                    for (int r = 0; r < 8; ++r) {
-                        const float4 sg = *reinterpret_cast<const float4 *>(signs + (size_t)fb * FWHT_N + r * 128 + 4 * lane);
-                        v[r][0] = __fmul_rn(v[r][0], sg.x); v[r][1] = __fmul_rn(v[r][1], sg.y);
-                        v[r][2] = __fmul_rn(v[r][2], sg.z); v[r][3] = __fmul_rn(v[r][3], sg.w);
-                    }
+                    v[k][0] = __fmul_rn(v[k][0], sg[k].x); v[k][1] = __fmul_rn(v[k][1], sg[k].y);
+                    v[k][2] = __fmul_rn(v[k][2], sg[k].z); v[k][3] = __fmul_rn(v[k][3], sg[k].w);
                 }
-                fwht1024_warp(v, lane);
-#pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    uint32_t word, header;
-                    quantise_chunk_8lanes(v[r], lane, word, header);
-                    const int chunk = fb * 32 + r * 4 + (lane >> 3);
-                    act_q[(chunk >> 2) * STREAM_ACT_WORDS + (chunk & 3) * 8 + (lane & 7)] = word;
-                    if ((lane & 7) == 0) {
-                        act_s[chunk] = f16_bits_to_f32(header & 0xFFFFu);
-                        act_i[chunk] = -64 * (int)(short)(header >> 16);
-                    }
-                    if (blockIdx.x == 0 && xq_out) {
-                        xq_out[9 * chunk + 1 + (lane & 7)] = word;
-                        if ((lane & 7) == 0) xq_out[9 * chunk] = header;
-                    }
-                }
+                fwht_slice_front(v[k], lane);
+                front[(wid + nwarps * k) * 32 + lane] = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
             }
+            __syncthreads();
+            auto finish = [&](auto count) {
+                constexpr int N = decltype(count)::value;
+                float u[N][4];
+                uint32_t word[N], header[N];
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const int s = wid + nwarps * k;
+                    fwht_slice_back(front + (s >> 3) * (FWHT_N / 4), s & 7, lane, u[k]);
+                }
+                quantise_chunks_8lanes<N>(u, lane, word, header);
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    const int chunk = i0 * 32 + (wid + nwarps * k) * 4 + (lane >> 3);
+                    put(chunk, word[k], header[k]);
+                    if (blockIdx.x == 0) {              // the first CTA leaves the blocks where the two launches would have
+                        xq_out[9 * chunk + 1 + (lane & 7)] = word[k];
+                        if ((lane & 7) == 0) xq_out[9 * chunk] = header[k];
+                    }
+                }
+            };
+            const int n = (ns - wid + nwarps - 1) / nwarps;             // warp-uniform
+            if (n == 1) finish(std::integral_constant<int, 1>());
+            else if (n == 2) finish(std::integral_constant<int, 2>());
+            else if (n >= 3) finish(std::integral_constant<int, 3>());
         }
     } else {
         const int nchunks = P.nb * 4;
@@ -409,12 +435,11 @@ __global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__re
             act_i[chunk] = -64 * (int)(short)(v[0] >> 16);
         }
     }
-    if (CL > 1) {                       // activation arrays, counters and barrier inits visible to all, of every CTA of the cluster
-        __syncwarp();
+    __syncthreads();                    // (activation arrays,) counters and barrier inits visible to all
+    if (CL > 1 && !__all_sync(0xffffffffu, mbar_wait_hot(tables, 0))) {         // (nobody's bytes may find this CTA gone)
         cluster_arrive();
         cluster_wait();
-    } else {
-        __syncthreads();
+        return;
     }
 
     if (wid < compute_warps) {

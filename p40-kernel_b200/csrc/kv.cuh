@@ -193,18 +193,6 @@ __device__ __forceinline__ float ld_cluster_f32(const float *p, uint32_t rank) {
     return v;
 }
 
-// Into CTA `rank`'s shared memory, at the place that p is in this one's (8- and 16-byte aligned), counted on its barrier at `bar`.
-__device__ __forceinline__ void st_async_f32x2(const float *p, uint64_t *bar, uint32_t rank, float a, float b) {
-    asm volatile("{\n\t.reg .u32 x, y;\n\tmapa.shared::cluster.u32 x, %0, %2;\n\tmapa.shared::cluster.u32 y, %1, %2;\n\t"
-                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [x], {%3, %4}, [y];\n\t}"
-                 ::"r"(smem_u32(p)), "r"(smem_u32(bar)), "r"(rank), "f"(a), "f"(b) : "memory");
-}
-__device__ __forceinline__ void st_async_f32x4(const float *p, uint64_t *bar, uint32_t rank, float a, float b, float c, float d) {
-    asm volatile("{\n\t.reg .u32 x, y;\n\tmapa.shared::cluster.u32 x, %0, %2;\n\tmapa.shared::cluster.u32 y, %1, %2;\n\t"
-                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [x], {%3, %4, %5, %6}, [y];\n\t}"
-                 ::"r"(smem_u32(p)), "r"(smem_u32(bar)), "r"(rank), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 // grid (n_split, n_kv_head), cluster (CL, 1, 1), n_split a multiple of CL (PUSH: CL, else CL is KV_CLUSTER); split s covers positions
 // s * chunk .. min((s + 1) * chunk, pos + 1) - 1 (a split may be empty).  counters: one per (kv head, slice), zero before
 // and after every launch.

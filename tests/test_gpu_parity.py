@@ -334,21 +334,22 @@ def test_linear_one_call(gpu, port, n_out, n_in, signed):
     y = torch.zeros(n_out, dtype=torch.float32, device="cuda")
     xd = dev(x)
     Wd, sd = dev(W), None if sg is None else dev(sg)
-    assert gpu.linear(Wd, xd, sd, y, scratch, n_out, n_in) == 0          # default: two launches
+    assert gpu.linear(Wd, xd, sd, y, scratch, n_out, n_in) == 0          # default: by shape
     want_xq = port.quantize_q8_1(port.fwht_blocks(x, sg), True)
     assert np.array_equal(host(scratch), want_xq)
     assert np.array_equal(bits(host(xd)), bits(x))
     assert_close(host(y), port.gemv(W, want_xq, n_out, n_in, threads=4))
     fused = host(y).copy()
-    try:
-        gpu.set_option("fuse_linear", 1)                                  # one kernel, rotation in its prologue: same bits
-        y.zero_()
-        scratch.zero_()
-        assert gpu.linear(Wd, xd, sd, y, scratch, n_out, n_in) == 0
-    finally:
-        gpu.set_option("fuse_linear", 0)
-    assert np.array_equal(host(scratch), want_xq)
-    assert np.array_equal(bits(host(y)), bits(fused))
+    for fuse in (0, 1):                                                   # two launches; one kernel, rotation in its prologue: same bits
+        try:
+            gpu.set_option("fuse_linear", fuse)
+            y.zero_()
+            scratch.zero_()
+            assert gpu.linear(Wd, xd, sd, y, scratch, n_out, n_in) == 0
+        finally:
+            gpu.set_option("fuse_linear", -1)
+        assert np.array_equal(host(scratch), want_xq)
+        assert np.array_equal(bits(host(y)), bits(fused))
     assert gpu.linear(Wd, xd, None, y, scratch, n_out, 1000) == 1
 
 
