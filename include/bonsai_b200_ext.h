@@ -142,7 +142,7 @@ int bonsai_b200_stream_probe(const void *buf, int64_t bytes, int mode, void *sin
  * else the integer form), 2 = the small-batch kernel where it takes the shape, 3 = the integer tensor-core kernel
  * (csrc/gemm_tc.cuh: forms the host's int32 chunk sums, needs no scratch).  1, 2 and 3 hold fp32 Y to 1e-5 of
  * max |Y|.  How the fp16 form divides a call, and with it the order of a row's sum, follows from n_out, n_in and n_tok: the same call gives the same
- * bits every time, a row or a token of it in a call of another shape those of another order, within the bound.  The fp16 form keeps one scratch buffer per (device, stream), 4 bytes per token and input value, and 16 MB for
+ * bits every time, a row or a token of it in a call of another shape those of another order, within the bound.  The fp16 form keeps one scratch buffer per (device, stream), 4 bytes per token and input value, and 20 MB for
  * the parts of tiles, allocated with cudaMalloc on first use or growth -- never while the stream is being captured (then the
  * integer form runs).
  * key "fuse_linear": bonsai_b200_linear and _linear_static are -1 (default) = one launch where that is faster, else

@@ -1072,9 +1072,9 @@ static bool encode_w_map(CUtensorMap *map, const void *W, int64_t n_out, int64_t
                          68u, (uint32_t)TC_M, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
-// Scratch of the fp16 tensor-core mat-mul: a flag and a slot per CTA for its part of a tile, the activations as two fp16 planes, a
+// Scratch of the fp16 tensor-core mat-mul: counts and two slots per CTA for its parts of tiles, the activations as two fp16 planes, a
 // scale per token.  A call that gets none takes the integer kernel, which needs no scratch.
-static constexpr size_t T16_FLAGS_BYTES = (size_t)TC_MAX_CTAS * T16_PART_FLAGS * sizeof(unsigned int);
+static constexpr size_t T16_COUNTS_BYTES = (size_t)T16_MAX_CTAS * T16_PART_COUNTS * sizeof(unsigned int);
 static StreamScratch g_gemm_scratch(false);
 
 // Scratch of the prompt attention: k and v as tile images, 2 KB per position and kv head, what k and v take themselves.  Prompts of one
@@ -1092,9 +1092,9 @@ static void fill_tc_params(TcParams &P, int64_t n_out, int64_t n_in, int64_t n_t
     P.total_it = (long long)P.n_tiles * P.nblocks;
 }
 
-static constexpr size_t T16_PARTS_BYTES = (size_t)TC_MAX_CTAS * T16C<128, 2>::PART_FLOATS * sizeof(float);
+static constexpr size_t T16_PARTS_BYTES = (size_t)T16_MAX_CTAS * 2 * T16C<128, 2>::PART_FLOATS * sizeof(float);
 static size_t tc16_scratch_bytes(int64_t n_in, int64_t n_tok) {
-    return T16_FLAGS_BYTES + T16_PARTS_BYTES + 2 * (size_t)n_tok * (size_t)n_in * sizeof(__half) + (size_t)n_tok * sizeof(float);
+    return T16_COUNTS_BYTES + T16_PARTS_BYTES + 2 * (size_t)n_tok * (size_t)n_in * sizeof(__half) + (size_t)n_tok * sizeof(float);
 }
 
 // The fp16 tensor-core mat-mul (gemm_tc16.cuh).  -1: not taken (shape, alignment, no scratch, no tensor-map encoder).
@@ -1133,9 +1133,9 @@ static Tc16Plan plan_tc16(int64_t n_out, int64_t nblocks, int64_t n_tok, int wor
 }
 static int tc16_workers(int ctas) {
     int dev = 0, sms = 0;
-    if (ctas != 1) return std::min(g_tc16_pairs.ask(gemm_tc16_kernel<128, 2>, g_tc16_pairs_smem, 2, T16C<128, 2>::THREADS), (TC_MAX_CTAS - 1) / ctas);
+    if (ctas != 1) return std::min(g_tc16_pairs.ask(gemm_tc16_kernel<128, 2>, g_tc16_pairs_smem, 2, T16C<128, 2>::THREADS), T16_MAX_CTAS / ctas);
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    return std::min(sms, TC_MAX_CTAS - 1);
+    return std::min(sms, T16_MAX_CTAS);
 }
 
 // One launch over activations that lie in `planes`.
@@ -1144,7 +1144,7 @@ struct Tc16Args {
     int64_t n_out, nblocks, n_tok;
     const float *scale;
     float *parts;
-    unsigned int *flags;
+    unsigned int *counts;
     Tc16Maps maps;
 };
 template <int TN, int CTAS>
@@ -1168,15 +1168,15 @@ static cudaError_t launch_gemm_tc16_n(const Tc16Args &a, const Tc16Plan &plan, S
     cfg.dynamicSmemBytes = T16C<TN, CTAS>::SMEM_BYTES;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeCooperative;        // a CTA may wait for another's part of a tile: all must be resident
-    attr[0].val.cooperative = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = CTAS;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = CTAS == 1 ? 1 : 2;
-    if (CTAS != 1) return launch_clusters(cfg, gemm_tc16_kernel<TN, CTAS>, a.Y, P, a.scale, a.parts, a.flags, a.maps);
-    return cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN, CTAS>, a.Y, P, a.scale, a.parts, a.flags, a.maps);
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CTAS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;        // behind the split, which does not write weights
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = CTAS == 1 ? attr + 1 : attr;
+    cfg.numAttrs = (CTAS != 1) + (g_opt_overlap.load() != 0);
+    if (CTAS != 1) return launch_clusters(cfg, gemm_tc16_kernel<TN, CTAS>, a.Y, P, a.scale, a.parts, a.counts, a.maps);
+    return cudaLaunchKernelEx(&cfg, gemm_tc16_kernel<TN, CTAS>, a.Y, P, a.scale, a.parts, a.counts, a.maps);
 }
 }  // extern "C++"
 // Tiles of up to 64 tokens by a CTA, or of up to 128 by a pair of CTAs (the code expansion is paid once per tile, and each CTA fetches half
@@ -1196,9 +1196,9 @@ static int launch_gemm_tc16(const void *W, const void *Xq, float *Y, int64_t n_o
     const StreamScratch::Lease lease = g_gemm_scratch.get(tc16_scratch_bytes(n_in, n_tok), st);      // held until the launches are enqueued
     uint8_t *ws = static_cast<uint8_t *>(lease.ptr);
     if (!ws) return -1;
-    __half *planes = reinterpret_cast<__half *>(ws + T16_FLAGS_BYTES + T16_PARTS_BYTES);
-    float *scale = reinterpret_cast<float *>(ws + T16_FLAGS_BYTES + T16_PARTS_BYTES + 2 * plane_bytes);
-    alignas(64) Tc16Args a{Y, n_out, nblocks, n_tok, scale, reinterpret_cast<float *>(ws + T16_FLAGS_BYTES), reinterpret_cast<unsigned int *>(ws), {}};
+    __half *planes = reinterpret_cast<__half *>(ws + T16_COUNTS_BYTES + T16_PARTS_BYTES);
+    float *scale = reinterpret_cast<float *>(ws + T16_COUNTS_BYTES + T16_PARTS_BYTES + 2 * plane_bytes);
+    alignas(64) Tc16Args a{Y, n_out, nblocks, n_tok, scale, reinterpret_cast<float *>(ws + T16_COUNTS_BYTES), reinterpret_cast<unsigned int *>(ws), {}};
     auto map_activations = [&](int tokens) { return tensor_map_planes(&a.maps.x, planes, (uint64_t)n_in, (uint64_t)n_tok, (uint32_t)tokens); };
     if (!encode_w_map(&a.maps.w, W, n_out, nblocks * W_BLOCK_BYTES) || !map_activations(paired ? two.tile_n / 2 : one.tile_n)) return -1;
     const int n_chunks = (int)(n_in / 32);
@@ -1208,10 +1208,10 @@ static int launch_gemm_tc16(const void *W, const void *Xq, float *Y, int64_t n_o
     int passes = (n_chunks + T16_SPLIT_PASS - 1) / T16_SPLIT_PASS;
     passes = (int)((passes * groups + 2 * sms - 1) / (2 * sms));
     const int slice = passes * T16_SPLIT_PASS;
-    const int flagged = std::max(one.stream_k ? one.grid : 0, paired && two.stream_k ? 2 * two.grid : 0);      // CTAs that may raise flags
+    const int counted = std::max(one.stream_k ? one.grid : 0, paired && two.stream_k ? 2 * two.grid : 0);      // CTAs that may count parts
     cudaError_t e = launch(groups <= 2 * sms ? tc16_split_kernel<true> : tc16_split_kernel<false>,
                            dim3((unsigned)groups, (unsigned)((n_chunks + slice - 1) / slice)), dim3(T16_SPLIT_THREADS), 0, st, true, x32, n_chunks, (int)n_tok, slice,
-                           scale, planes, reinterpret_cast<uint4 *>(ws), flagged * T16_PART_FLAGS / 4);
+                           scale, planes, reinterpret_cast<uint4 *>(ws), counted * T16_PART_COUNTS / 4);
     if (e != cudaSuccess) return (int)e;
     if (paired) {
         e = launch_gemm_tc16_n<128, 2>(a, two, g_tc16_pairs_smem, st);

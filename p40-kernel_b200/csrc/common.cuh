@@ -87,6 +87,13 @@ __device__ __forceinline__ int chunk_sumi_scaled(uint32_t w0, uint32_t w1, const
 // ---- shared-memory barriers and bulk copies (sm_90+ PTX, every copy is local to its CTA) -------
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// Adds 1 to a counter in global memory; what the CTA wrote before the barrier in front of this call is visible to whoever
+// reads the sum, and what they wrote to this CTA after the barrier behind it.
+__device__ __forceinline__ unsigned int count_arrival(unsigned int *counter) {
+    unsigned int old;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
+    return old;
+}
 // ---- clusters of CTAs ----
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;

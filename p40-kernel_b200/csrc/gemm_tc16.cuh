@@ -47,7 +47,8 @@ constexpr int T16_WBUFS = 2;
 constexpr int T16_DWRING = 8;                              // weight scales of the last 8 blocks (the epilogue lags the producers)
 constexpr int T16_ISSUERS = 2;                             // issuing warps: warp k takes the blocks n with n % 2 == k
 constexpr int T16_TURN_STRIDE = 36, T16_TURN_FLOATS = 8 * T16_TURN_STRIDE;      // an epilogue warp turns 8 rows x 32 tokens round at once
-constexpr int T16_PART_FLAGS = 16;                         // flags of a CTA: one per epilogue warp
+constexpr int T16_PART_COUNTS = 16;                        // counts of a CTA whose share a tile begins in: one per epilogue warp
+constexpr int T16_MAX_CTAS = 160;
 // TN: the most tokens of a tile; CTAS: CTAs that multiply one tile together.
 template <int TN, int CTAS>
 struct T16C {
@@ -271,12 +272,12 @@ __device__ __forceinline__ int tc16_shift(unsigned int maxd_bits) {
 // between the maximum and the split -- then thread = (chunk, token): 32 values -> 32 + 32 fp16, in the order the quantiser
 // stored them (the order in which the code producers emit the codes).  planes: H at [tok][n_in], L at [n_tok + tok][n_in];
 // scale[tok] = 2^-S for the epilogue.  A warp takes 4 tokens x 8 consecutive chunks: its stores are four runs of 512 bytes
-// per plane.  Bound by launch and memory latency.  The first threads also lower the flags that the mat-mul's CTAs raise where they share
-// tiles, four at a time: a launch whose wait ran out leaves those raised that came later, and the next must not take them for its own.
+// per plane.  Bound by launch and memory latency.  The first threads also clear the counts of the mat-mul's CTAs that share
+// tiles, four at a time.
 constexpr int T16_SPLIT_THREADS = 256, T16_SPLIT_PASS = T16_SPLIT_THREADS / 4;      // chunks of four tokens a block takes at once
 template <bool FEW>
 __global__ void __launch_bounds__(T16_SPLIT_THREADS) tc16_split_kernel(const uint32_t *Xq, int n_chunks, int n_tok, int slice, float *scale,
-                                                                       __half *planes, uint4 *flags, int n_flags4) {
+                                                                       __half *planes, uint4 *counts, int n_counts4) {
     __shared__ unsigned int top[T16_SPLIT_THREADS / 32][4];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tok = 4 * (int)blockIdx.x + (lane >> 3), c_first = (int)blockIdx.y * slice + 8 * warp + (lane & 7);
@@ -292,9 +293,9 @@ __global__ void __launch_bounds__(T16_SPLIT_THREADS) tc16_split_kernel(const uin
         for (int k = 0; k < 9; ++k) w[k] = src[k];
     };
     if (FEW) fetch(c_first);
-    for (int i = ((int)blockIdx.y * (int)gridDim.x + (int)blockIdx.x) * T16_SPLIT_THREADS + (int)threadIdx.x; i < n_flags4;
+    for (int i = ((int)blockIdx.y * (int)gridDim.x + (int)blockIdx.x) * T16_SPLIT_THREADS + (int)threadIdx.x; i < n_counts4;
          i += (int)(gridDim.x * gridDim.y) * T16_SPLIT_THREADS)
-        flags[i] = make_uint4(0u, 0u, 0u, 0u);
+        counts[i] = make_uint4(0u, 0u, 0u, 0u);
     {   // four tokens are neighbours in memory: four lanes read one chunk's headers
         const int t = min(4 * (int)blockIdx.x + (lane & 3), n_tok - 1);
         unsigned int m = 0;
@@ -420,8 +421,8 @@ struct Tc16Maps {
 };
 
 template <int TN, int CTAS>
-__global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(float *Y, const T16Params P, const float *__restrict__ tokscale,
-                                                                               float *parts, unsigned int *flags, const __grid_constant__ Tc16Maps maps) {
+__global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(float *Y, const T16Params P, const float *tokscale,
+                                                                               float *parts, unsigned int *counts, const __grid_constant__ Tc16Maps maps) {
     using C = T16C<TN, CTAS>;
     constexpr int EPI_WARPS = C::EPI_WARPS, PROD_WARPS = C::PROD_WARPS, SETS = C::PROD_SETS, ACC = C::ACC, COLS = 32;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -480,6 +481,7 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
 
     if (wid < EPI_WARPS) {
         // ---------------- epilogue: one weight row per thread, 32 tokens ----------------
+        pdl_wait_prior_grid();                                           // token scales, counts and Y: the split's and its predecessors'
         const int q = wid & 3, cg = wid >> 2;
         const int row_l = 32 * q + lane;
         const bool second = COLS * cg + 16 < P.tile_n;
@@ -556,12 +558,20 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
             if (!ok) break;
             // ---- the tile (or this CTA's part of it) is done
             const int toks = min(min(COLS, P.tile_n - col0), n_tok - tokb);         // may be none
-            const float scale = lane < toks ? __ldg(tokscale + tokb + lane) : 0.0f;
-            if (kb0 > 0) {
-                // A later part of a tile: left in this CTA's slot, four tokens of a row per lane and store.  The CTA that has the tile's
-                // first blocks adds the parts, each of its warps those of its counterparts as soon as they are there.  (They were handed from CTA
-                // to CTA, each waiting for the one behind it: 37 tokens of 17408 -> 5120, four parts per tile, 69 us against 43 us.)
-                float *slot = parts + (size_t)blockIdx.x * C::PART_FLOATS + (size_t)col0 * T16_M + row_l;
+            const float scale = lane < toks ? tokscale[tokb + lane] : 0.0f;
+            if (kb0 > 0 || kb1 < nblocks) {
+                // A part of a tile that several workers share: left in this CTA's slot (one for the part at its start, one for the part at its end), four
+                // tokens of a row per lane and store.  Whoever of a warp and its counterparts comes last adds the parts in the order of their blocks: nobody
+                // waits for anybody, so the CTAs need not be resident at once and the launch need not be a cooperative one, which begins when everything
+                // in front of it has ended.  (us, norm or SwiGLU and quantiser in front, cooperative with the first part's CTA waiting for the others / now: 37 tokens of 17408 ->
+                // 5120 41.0 / 39.7, of 5120 -> 17408 32.3 / 28.6, 128 52.5 / 47.7, 64 of 1024 -> 5120 16.5 / 13.3, 20 of 5120 -> 5120 24.6 / 22.0, 512 of 5120 ->
+                // 1024 41.4 / 41.1.  Letting the next launch start as soon as this one's wait is over costs 8 - 40 us where tiles are shared.)
+                int head = worker, last = worker;
+                const long long begin = (long long)tile * nblocks, end = begin + nblocks;
+                while (t16_first(P, head, workers) > begin) --head;
+                while (last + 1 < workers && t16_first(P, last + 1, workers) < end) ++last;
+                auto slot_of = [&](int w) { return parts + ((size_t)(CTAS * w + rank) * 2 + (w == head ? 1 : 0)) * C::PART_FLOATS + (size_t)col0 * T16_M + row_l; };
+                float *slot = slot_of(worker);
 #pragma unroll
                 for (int j0 = 0; j0 < COLS; j0 += 8) {
                     if (j0 >= toks) break;
@@ -569,38 +579,21 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
                     for (int j = j0; j < j0 + 8; ++j) slot[j * T16_M] = acc[j];
                 }
                 __syncwarp();
-                if (lane == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + blockIdx.x * T16_PART_FLAGS + wid), "r"(1u) : "memory");
-                continue;
-            }
-            if (kb1 < nblocks) {
-                // the workers behind this one have the tile's other parts: added in their order
-                const long long tile_end = (long long)(tile + 1) * nblocks;
-                int last = worker + 1;
-                while (last + 1 < workers && t16_first(P, last + 1, workers) < tile_end) ++last;
-                for (int c = worker + 1 + lane; c <= last; c += 32) {
-                    const unsigned int *f = flags + (CTAS * c + rank) * T16_PART_FLAGS + wid;
-                    bool there = false;
-                    for (uint32_t k = 0; k < (1u << 23); ++k) {
-                        unsigned int fv;
-                        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(fv) : "l"(f) : "memory");
-                        if (fv != 0u) { there = true; break; }
-                        __nanosleep(32);
-                    }
-                    if (!there) atomicExch(&g_device_status, STATUS_GRID_TIMEOUT);
-                }
-                __syncwarp();
-                const float *slots = parts + (size_t)rank * C::PART_FLOATS + (size_t)col0 * T16_M + row_l;
-                for (int c = worker + 1; c <= last; ++c) {
-                    const float *slot = slots + (size_t)(CTAS * c) * C::PART_FLOATS;
+                unsigned int before = 0;
+                if (lane == 0) before = count_arrival(counts + (CTAS * head + rank) * T16_PART_COUNTS + wid);
+                before = __shfl_sync(0xffffffffu, before, 0);
+                if (before != (unsigned int)(last - head)) continue;
+                const float *from = slot_of(head);
 #pragma unroll
-                    for (int j0 = 0; j0 < COLS; j0 += 32) {
-                        if (j0 >= toks) break;
-                        float t[32];
+                for (int j = 0; j < COLS; ++j) acc[j] = __ldcg(from + j * T16_M);
+#pragma unroll 1
+                for (int c = head + 1; c <= last; ++c) {
+                    from = slot_of(c);
+                    float t[COLS];
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) t[j] = __ldcg(slot + (j0 + j) * T16_M);
+                    for (int j = 0; j < COLS; ++j) t[j] = __ldcg(from + j * T16_M);
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) acc[j0 + j] = __fadd_rn(acc[j0 + j], t[j]);
-                    }
+                    for (int j = 0; j < COLS; ++j) acc[j] = __fadd_rn(acc[j], t[j]);
                 }
             }
             // A row's tokens lie side by side in Y: turned round through shared memory eight rows at a time, a store writes 128 bytes of one
@@ -706,6 +699,7 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
         }
     } else if (wid == LOADER + 1) {
         // ---------------- activation loader: a block's two boxes as soon as its slot is free ----------------
+        pdl_wait_prior_grid();                                           // the planes
         const int bn = P.tile_n / CTAS;
         const uint32_t full0 = CTAS == 1 ? 0u : cluster_first(smem_u32(full));
         int n = 0;

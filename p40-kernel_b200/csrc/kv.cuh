@@ -178,13 +178,6 @@ __device__ __forceinline__ void split_rest_f16x2(float a, float b, uint32_t &hi,
 }
 __device__ __forceinline__ float half_bits_lo(uint32_t w) { return f16_bits_to_f32(w & 0xFFFFu); }
 __device__ __forceinline__ float half_bits_hi(uint32_t w) { return f16_bits_to_f32(w >> 16); }
-// Adds 1 to a counter in global memory; what the CTA wrote before the barrier in front of this call is visible to whoever
-// reads the sum, and what they wrote to this CTA after the barrier behind it.
-__device__ __forceinline__ unsigned int count_arrival(unsigned int *counter) {
-    unsigned int old;
-    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
-    return old;
-}
 __device__ __forceinline__ float ld_cluster_f32(const float *p, uint32_t rank) {
     uint32_t a;
     float v;
