@@ -1827,11 +1827,11 @@ int bonsai_kv_append_batch(bonsai_kv_cache *kv, int layer, int pos0, int n_tok, 
     const int nrow = n_tok * KVM_KV_HEADS;
     // any float pointer is taken; 16-byte aligned ones get 16-byte loads
     const bool vec = aligned16(k) && aligned16(v);
-    const int blocks = (nrow + 7) / 8;
+    const int blocks = (nrow + KV_APPEND_WARPS - 1) / KV_APPEND_WARPS;
     const bool early = blocks <= 8 * SM_COUNT;              // 2368 tokens: one wave of eight blocks of 256 threads per SM
     auto kernel = early ? (vec ? kv_append_kernel<true, true> : kv_append_kernel<false, true>)
                         : (vec ? kv_append_kernel<true, false> : kv_append_kernel<false, false>);
-    return (int)launch(kernel, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, kv->d_k, kv->d_v, k, v, pos0, n_tok,
+    return (int)launch(kernel, dim3((unsigned)blocks), dim3(32 * KV_APPEND_WARPS), 0, as_stream(stream), true, kv->d_k, kv->d_v, k, v, pos0, n_tok,
                        KVM_KV_HEADS, kv->capacity, layer);
 }
 

@@ -42,28 +42,24 @@ __device__ __forceinline__ void kv_words_8(const float (&x)[8], float id, uint32
         word[i >> 2] |= ((uint32_t)v & 0xFFu) << (8 * (i & 3));
     }
 }
-__device__ __forceinline__ void kv_quantise_8(const float (&x)[8], float &d_out, uint32_t (&word)[2]) {
-    const float d = __fdiv_rn(kv_amax_8(x), 127.0f);
-    kv_words_8(x, d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f, word);
-    d_out = d;
-}
-
 // One warp per (token, kv head) row of K and of V: lane = (block lane / 4, eight dims).
 // EARLY: the rows are asked into L2 while the launch before this one still runs (L2 hands out what it finds at the load, whoever writes
 // in between), an aligned row by one bulk request.  That pays while the grid is resident at once: blocks that start later have no wait to
-// hide it in.  16 layers in us, without / by lines / as here; inputs not in L2: 512 tokens 61.4 / 55.3 / 53.3, 1024 88.0 / 79.9 / 77.8, 4096
+// hide it in.  16 layers in us (rows stored by halfwords, as then), without / by lines / as here; inputs not in L2: 512 tokens 61.4 / 55.3 / 53.3, 1024 88.0 / 79.9 / 77.8, 4096
 // 178.2 / 182.3 / without; inputs in L2: 64 tokens 33.2 / 33.0 / 33.0, 512 44.5 / 49.4 / 46.9, 1024 80.2 / 74.7 / 74.0, 4096 172.5 / 176.4 /
-// without.  (The first tiles of the attention below, asked for likewise: no gain.)
+// without.  Stored as now, by calls, without / as here: 1 token 23.6 / 22.3, 200 37.4 / 33.3, 512 50.2 / 43.2, 1024 80.0 / 70.5, 2048 104.4 / 99.2.  (The first tiles of the attention below, asked for likewise: no gain.)
+constexpr int KV_APPEND_WARPS = 8;
 template <bool VEC, bool EARLY>
-__global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *K, uint8_t *V,
+__global__ void __launch_bounds__(32 * KV_APPEND_WARPS) kv_append_kernel(uint8_t *K, uint8_t *V,
                                                         const float *ksrc, const float *vsrc,
                                                         int pos0, int n_tok, int n_kv_head, int capacity, int layer) {
-    const int lane = threadIdx.x & 31;
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);        // token * n_kv_head + head
+    __shared__ __align__(16) uint8_t rows[KV_APPEND_WARPS][2][KV_ROW];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row = blockIdx.x * KV_APPEND_WARPS + warp;                        // token * n_kv_head + head
     if (row >= n_tok * n_kv_head) return;
     const int tok = row / n_kv_head, h = row - tok * n_kv_head;
     const int blk = lane >> 2, sub = lane & 3;
-    const size_t base = ((((size_t)layer * n_kv_head + h) * capacity + (size_t)(pos0 + tok)) * KV_NBLK + blk) * 34;
+    const size_t base = (((size_t)layer * n_kv_head + h) * capacity + (size_t)(pos0 + tok)) * KV_ROW;
     const float *kr = ksrc + (size_t)row * KV_D + blk * 32 + sub * 8;
     const float *vr = vsrc + (size_t)row * KV_D + blk * 32 + sub * 8;
     float kx[8], vx[8];
@@ -87,20 +83,28 @@ __global__ void __launch_bounds__(256) kv_append_kernel(uint8_t *K, uint8_t *V,
 #pragma unroll
         for (int i = 0; i < 8; ++i) { kx[i] = kr[i]; vx[i] = vr[i]; }
     }
-    float kd, vd;
+    // the divisions of K by the even lanes of the four, of V by the odd ones
+    const float kmax = kv_amax_8(kx), vmax = kv_amax_8(vx), d = __fdiv_rn(sub & 1 ? vmax : kmax, 127.0f), id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+    const uint32_t d16 = f32_to_f16_bits_ties_away(d);
     uint32_t kw[2], vw[2];
-    kv_quantise_8(kx, kd, kw);
-    kv_quantise_8(vx, vd, vw);
-    // blocks start on 2-byte boundaries: halfword stores (scale, then this lane's 8 bytes)
-    unsigned short *kp = reinterpret_cast<unsigned short *>(K + base), *vp = reinterpret_cast<unsigned short *>(V + base);
-    if (sub == 0) {
-        kp[0] = (unsigned short)f32_to_f16_bits_ties_away(kd);
-        vp[0] = (unsigned short)f32_to_f16_bits_ties_away(vd);
-    }
+    kv_words_8(kx, __shfl_sync(0xffffffffu, id, lane & ~3), kw);
+    kv_words_8(vx, __shfl_sync(0xffffffffu, id, lane | 1), vw);
+    // Blocks start on 2-byte boundaries, rows on 16-byte ones: a row is put together in shared memory by halfwords (scale, then this lane's 8 bytes) and
+    // stored by 17 lanes.  (By halfwords to memory, five stores a row, each to all of its sectors, and with a division per lane and row: 16 layers, us, by
+    // calls / as here: 1 token 25.0 / 22.3, 64 34.5 / 28.8, 512 51.5 / 43.2, 1024 89.7 / 70.5, 2048 103.8 / 99.0, 4096 176 / 170.5.)
+    uint8_t *kb = rows[warp][0], *vb = rows[warp][1];
+    unsigned short *kp = reinterpret_cast<unsigned short *>(kb + 34 * blk), *vp = reinterpret_cast<unsigned short *>(vb + 34 * blk);
+    if (sub < 2) (sub ? vp : kp)[0] = (unsigned short)d16;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
         kp[1 + 4 * sub + 2 * j] = (unsigned short)(kw[j] & 0xFFFFu); kp[2 + 4 * sub + 2 * j] = (unsigned short)(kw[j] >> 16);
         vp[1 + 4 * sub + 2 * j] = (unsigned short)(vw[j] & 0xFFFFu); vp[2 + 4 * sub + 2 * j] = (unsigned short)(vw[j] >> 16);
+    }
+    __syncwarp();
+    if (lane < KV_ROW / 16) {
+        const uint4 a = reinterpret_cast<const uint4 *>(kb)[lane], c = reinterpret_cast<const uint4 *>(vb)[lane];
+        reinterpret_cast<uint4 *>(K + base)[lane] = a;
+        reinterpret_cast<uint4 *>(V + base)[lane] = c;
     }
 }
 
