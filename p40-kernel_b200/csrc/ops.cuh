@@ -16,11 +16,14 @@ namespace b200 {
 // A vector is cut into slices of 128 floats; inside a slice lane l adds x[4l]^2 .. x[4l+3]^2 in that order and a
 // 5-step butterfly joins the lanes; slices are added in ascending order.  The fused producer of the list kernel
 // (gemv_chain.cuh) uses the same order, so a fused RMSNorm gives the bits of this kernel.
-__device__ __forceinline__ float slice_sumsq(float4 f) {
+__device__ __forceinline__ float lane_sumsq(float4 f) {
     float s = __fmul_rn(f.x, f.x);
     s = __fadd_rn(s, __fmul_rn(f.y, f.y));
     s = __fadd_rn(s, __fmul_rn(f.z, f.z));
-    s = __fadd_rn(s, __fmul_rn(f.w, f.w));
+    return __fadd_rn(s, __fmul_rn(f.w, f.w));
+}
+__device__ __forceinline__ float slice_sumsq(float4 f) {
+    float s = lane_sumsq(f);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
     return s;
@@ -84,9 +87,9 @@ __device__ __forceinline__ void rms_store(float *p, int i, int n, float4 f, floa
     }
 }
 template <bool VEC, int HOLD>
-__global__ void __launch_bounds__(RMS_THREADS, HOLD < 0 ? 8 : (HOLD == 8 && !VEC ? 3 : 0)) rmsnorm_kernel(const float *x, const float *w, float *y, int n, float eps) {
+__global__ void __launch_bounds__(RMS_THREADS, HOLD < 0 || HOLD == 1 ? 8 : (HOLD == 8 && !VEC ? 3 : 0)) rmsnorm_kernel(const float *x, const float *w, float *y, int n, float eps) {
     constexpr int NW = RMS_WARPS;
-    __shared__ float part[512];
+    __shared__ __align__(16) float part[512];
     __shared__ float scale;
     const float *xr = x + (size_t)blockIdx.x * n;
     float *yr = y + (size_t)blockIdx.x * n;
@@ -100,21 +103,36 @@ __global__ void __launch_bounds__(RMS_THREADS, HOLD < 0 ? 8 : (HOLD == 8 && !VEC
         for (int r = 0; r < HOLD; ++r) f[r] = rms_load<VEC>(xr, (wid + NW * r) * 128 + 4 * lane, n);
 #pragma unroll
         for (int r = 0; r < HOLD; ++r) g[r] = rms_load<VEC>(w, (wid + NW * r) * 128 + 4 * lane, n);
+        // the slices' sums side by side (as slice_sumsq; past the end they are zeros), added by every warp for itself: one barrier (one after the other, and added
+        // by one thread between two barriers: 8 rows of 5120 2.57 us, 2.18 now, 6144 2.84 and 2.47, 2048 rows of 5120 15.7 and 14.4).  Of one slice a warp one
+        // thread still adds: many CTAs have no issue slots to spare (2048 rows of 1024 3.58, by every warp 4.08)
+        float s[HOLD];
 #pragma unroll
-        for (int r = 0; r < HOLD; ++r) {
-            if (wid + NW * r >= nslice) break;              // warp-uniform
-            const float s = slice_sumsq(f[r]);
-            if (lane == 0) part[wid + NW * r] = s;
-        }
+        for (int r = 0; r < HOLD; ++r) s[r] = lane_sumsq(f[r]);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+            for (int r = 0; r < HOLD; ++r) s[r] = __fadd_rn(s[r], __shfl_xor_sync(0xffffffffu, s[r], o));
+#pragma unroll
+        for (int r = 0; r < HOLD; ++r)
+            if (lane == 0) part[wid + NW * r] = s[r];
         __syncthreads();
-        if (threadIdx.x == 0) {
+        float sc;
+        if (HOLD > 1 || threadIdx.x == 0) {
             float acc = 0.0f;
-#pragma unroll 8
-            for (int k = 0; k < nslice; ++k) acc = __fadd_rn(acc, part[k]);
-            scale = rms_scale(acc, n, eps);
+#pragma unroll 2
+            for (int k = 0; k + 4 <= nslice; k += 4) {
+                const float4 p = *reinterpret_cast<const float4 *>(part + k);
+                acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, p.x), p.y), p.z), p.w);
+            }
+            for (int k = nslice & ~3; k < nslice; ++k) acc = __fadd_rn(acc, part[k]);
+            sc = rms_scale(acc, n, eps);
+            if (HOLD == 1) scale = sc;
         }
-        __syncthreads();
-        const float sc = scale;
+        if (HOLD == 1) {
+            __syncthreads();
+            sc = scale;
+        }
 #pragma unroll
         for (int r = 0; r < HOLD; ++r) rms_store<VEC>(yr, (wid + NW * r) * 128 + 4 * lane, n, f[r], sc, g[r]);
     } else {
