@@ -22,7 +22,7 @@
 // columns: 256 output (before that, sums of the scores), 128 scores (then weights), 128 q low.
 // What bounds it (counted while a score was four sums): per tile 5900 of 10200 cycles were the tensor core's, most of them the score
 // products (N = 64: it waits for the q rows from shared memory), the rest softmax and the exchanges in front of it.  2048 tokens, 24 heads over 4: 2570 ->
-// 279 us; 1000 tokens 727 -> 90 us, 600 tokens 59 us.
+// 279 us; 1000 tokens 727 -> 90 us, 600 tokens 59 us, 511 tokens 186 -> 56 us, 300 tokens 90 -> 39 us.
 //
 // A plane pair holds 2^-39 of the largest value under its power of two, so what is far smaller loses bits to values that a row may not
 // even see.  A CTA whose queries and keys range too widely (atc_too_wide) does its queries again on the CUDA cores (attn_simt), with
@@ -35,11 +35,11 @@
 
 namespace b200 {
 
-// From this token count on.  It is faster from 100 tokens on (301: 40 us; the CUDA cores take 102 us for 340), but there the CUDA cores' longest sums
-// are short enough to be the more exact ones: relative error against 64 bits (normal values, 24 heads over 4) at 301 tokens
-// 1.8e-7 here and 1.8e-7 there, at 200 1.8e-7 and 1.6e-7; at 517 1.9e-7 and 2.1e-7, at 1000 2.0e-7 and 2.6e-7, at 2048
-// 2.1e-7 and 3.4e-7.
-constexpr int ATC_MIN_TOKENS = 512;
+// From this token count on.  It is faster from 64 tokens on (us, CUDA cores / here, 24 heads over 4: 64 18.6 / 17.2, 192 49 / 30, 301 90 / 39, 511 186 / 56; of one
+// head 192 47 / 27, 500 114 / 50), but for short rows the CUDA cores' sums are short enough to be the more exact ones.  Relative error against 64 bits, CUDA cores /
+// here (24 heads over 4): normal values 128 tokens 1.39e-7 / 1.50e-7, 192 1.55e-7 / 1.54e-7, 250 1.67e-7 / 1.57e-7, 511 2.06e-7 / 1.61e-7, 2047 3.4e-7 / 1.73e-7; of positive
+// v 192 1.57e-7 / 1.08e-7; of queries four times as large 192 2.75e-7 / 2.76e-7, 250 2.97e-7 / 2.88e-7; a twentieth as large 192 1.17e-7 / 1.19e-7, 250 1.29e-7 / 1.19e-7.
+constexpr int ATC_MIN_TOKENS = 192;
 constexpr int ATC_M = 128, ATC_KEYS = 64, ATC_WARPS = 16, ATC_THREADS = ATC_WARPS * 32;
 constexpr int ATC_CHUNK = 128 * 128;                         // bytes of 128 rows x 64 fp16
 constexpr int ATC_PLANES = 4 * ATC_CHUNK;                    // q high; k high + low; v high + low: 64 KB each
@@ -52,6 +52,11 @@ constexpr uint32_t ATC_COL_O = 0, ATC_COL_S = 256, ATC_COL_QL = 384;
 constexpr uint32_t ATC_HUGE = (127u + 60u) << 23;            // bits of 2^60
 constexpr uint32_t ATC_TINY = (127u - 100u) << 23;           // bits of 2^-100: a dim of v all below it is past the shift's cap
 constexpr uint32_t ATC_NONE = 0x7FFFFFFFu;
+// The tensor core cuts the last bits of a tile's sum of weights x v off, in four steps of about the sum's own size: 1.1e-7 of it is missing in the mean (700 - 2048
+// tokens of normal values, least squares against 64 bits; 0.7e-7 of one tile's).  The factor of a dim, a power of two, is one unit in the last place larger
+// for that: relative error 2.01e-7 -> 1.68e-7 at 1024 tokens, of positive v 2.2e-7 -> 1.1e-7.  (The scores' sums, short as they are, need none: with 4e-8 to 1e-7 more of
+// them 1.70e-7 - 1.73e-7.)
+constexpr float ATC_V_LIFT = 1.0f + 0x1p-23f;
 constexpr int ATC_V_RANGE = 12;                              // log2
 constexpr float ATC_QK_RANGE = 4096.0f;
 constexpr int ATC_REDO_QUERIES = ATC_WARPS * ATT_QPW;
@@ -163,7 +168,7 @@ __global__ void __launch_bounds__(ATC_PREP_THREADS) attn_planes_kernel(const flo
 #pragma unroll
         for (int e = 0; e < ATC_KEYS; ++e) seen = max(seen, atc_abs_bits(x[e]));
         const int s = atc_shift(seen, 112);
-        reinterpret_cast<float *>(img + ATC_IMG_VF)[d] = atc_pow2(-s - 14);          // and the weights' 2^-14
+        reinterpret_cast<float *>(img + ATC_IMG_VF)[d] = __fmul_rn(atc_pow2(-s - 14), ATC_V_LIFT);          // (and the weights' 2^-14)
 #pragma unroll
         for (int g = 0; g < ATC_KEYS / 8; ++g) {
             uint4 hi, lo;

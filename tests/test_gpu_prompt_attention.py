@@ -57,6 +57,13 @@ def test_against_float64(gpu, n, heads, kv_heads, spread):
     assert gpu.device_status() == 0
 
 
+@pytest.mark.parametrize("n,heads,kv_heads,spread", [
+    (191, 24, 4, 0.0), (192, 24, 4, 0.0), (193, 1, 1, 0.0), (255, 6, 2, 0.0), (256, 6, 2, 1.0), (257, 3, 1, 0.0), (319, 4, 4, 0.0), (321, 24, 4, 1.0), (448, 2, 2, 0.0)])
+def test_short_prompts(gpu, n, heads, kv_heads, spread):
+    """The lengths next to where the tensor cores begin to serve, and between there and 512 (the same oracle and bound)."""
+    test_against_float64(gpu, n, heads, kv_heads, spread)
+
+
 def test_values_that_do_not_survive_the_split(gpu):
     """Infinities, NaN and huge values give what the CUDA-core kernel gives: rows in front of them are untouched, rows behind
     see them where their weight is not zero."""
