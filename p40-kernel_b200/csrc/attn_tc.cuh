@@ -22,7 +22,7 @@
 // columns: 256 output (before that, sums of the scores), 128 scores (then weights), 128 q low.
 // What bounds it (counted while a score was four sums): per tile 5900 of 10200 cycles were the tensor core's, most of them the score
 // products (N = 64: it waits for the q rows from shared memory), the rest softmax and the exchanges in front of it.  2048 tokens, 24 heads over 4: 2570 ->
-// 279 us; 1000 tokens 727 -> 90 us, 600 tokens 59 us, 511 tokens 186 -> 56 us, 300 tokens 90 -> 39 us.
+// 279 us; 1000 tokens 727 -> 90 us, 600 tokens 59 us, 511 tokens 146 -> 56 us, 300 tokens 85 -> 39 us.
 //
 // A plane pair holds 2^-39 of the largest value under its power of two, so what is far smaller loses bits to values that a row may not
 // even see.  A CTA whose queries and keys range too widely (atc_too_wide) does its queries again on the CUDA cores (attn_simt), with
@@ -35,8 +35,8 @@
 
 namespace b200 {
 
-// From this token count on.  It is faster from 64 tokens on (us, CUDA cores / here, 24 heads over 4: 64 18.6 / 17.2, 192 49 / 30, 301 90 / 39, 511 186 / 56; of one
-// head 192 47 / 27, 500 114 / 50), but for short rows the CUDA cores' sums are short enough to be the more exact ones.  Relative error against 64 bits, CUDA cores /
+// From this token count on.  It is faster from 160 tokens on (us, CUDA cores / here, 24 heads over 4: 100 19.7 / 26, 128 28 / 30, 192 40 / 30, 300 85 / 39, 511 146 /
+// 56), and of short rows the CUDA cores' sums are short enough to be the more exact ones.  Relative error against 64 bits, CUDA cores /
 // here (24 heads over 4): normal values 128 tokens 1.39e-7 / 1.50e-7, 192 1.55e-7 / 1.54e-7, 250 1.67e-7 / 1.57e-7, 511 2.06e-7 / 1.61e-7, 2047 3.4e-7 / 1.73e-7; of positive
 // v 192 1.57e-7 / 1.08e-7; of queries four times as large 192 2.75e-7 / 2.76e-7, 250 2.97e-7 / 2.88e-7; a twentieth as large 192 1.17e-7 / 1.19e-7, 250 1.29e-7 / 1.19e-7.
 constexpr int ATC_MIN_TOKENS = 192;
@@ -60,7 +60,7 @@ constexpr float ATC_V_LIFT = 1.0f + 0x1p-23f;
 constexpr int ATC_V_RANGE = 12;                              // log2
 constexpr float ATC_QK_RANGE = 4096.0f;
 constexpr int ATC_REDO_QUERIES = ATC_WARPS * ATT_QPW;
-static_assert(ATT_SMEM_BYTES <= 3 * ATC_PLANES, "attn_simt reuses the planes");
+static_assert(att_smem_bytes(ATC_WARPS) <= 3 * ATC_PLANES, "attn_simt reuses the planes");
 
 __host__ __device__ constexpr uint32_t atc_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(ATC_M >> 4) << 24); }
 

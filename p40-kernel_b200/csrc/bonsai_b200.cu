@@ -1665,19 +1665,24 @@ int bonsai_p40_attn(const float *q, const float *k, const float *v, float *out, 
     if (head_dim != ATT_D || n_head_kv == 0 || (n_head % n_head_kv) != 0) return 1;
     if (n_tok <= 0 || n_head <= 0 || n_head_kv <= 0) return (n_tok <= 0) ? 0 : 1;
     if (!aligned16(k) || !aligned16(v) || !aligned4(q) || !aligned4(out)) return 1;    // rows of 256 floats: 16-byte loads
-    const long long blocks = (long long)n_head * ((n_tok + ATT_QPC - 1) / ATT_QPC);
-    if (blocks > INT32_MAX) return 1;
+    if ((long long)n_head * ((n_tok + 31) / 32) > INT32_MAX) return 1;
     if (n_tok >= ATC_MIN_TOKENS) {
         const int rc = launch_attn_tc(q, k, v, out, n_tok, n_head, n_head_kv, scale, as_stream(stream));
         if (rc >= 0) return rc;
     }
-    static SmemOptIn opt1, opt2;
-    const bool two = blocks > SM_COUNT;
-    auto kernel = two ? attn_kernel<true> : attn_kernel<false>;
-    cudaError_t err = (two ? opt2 : opt1).ensure(kernel);
+    // CTAs of 16 queries, or of 8 where those of 16 fill only half of the SMs or leave the last of two or three rounds half empty.  us by 32, 16, 8 queries: 24 heads,
+    // 16 tokens 6.4 / 6.6 / 5.1, 30 11.6 / 8.5 / 7.3, 70 18.1 / 13.3 / 15.4, 100 25.3 / 19.7 / 23.0, 130 31.5 / 27.7 / 30.4, 191 45.3 / 51.5 / 40.1; 64 heads,
+    // 50 14.1 / 16.3 / 12.9, 100 39 / 32 / 29, 191 76 / 63 / 82.
+    static SmemOptIn opt[2];
+    const long long of16 = (long long)n_head * ((n_tok + 15) / 16);
+    const bool few = 2 * of16 <= SM_COUNT || (2 * of16 > 3 * SM_COUNT && of16 <= 3 * SM_COUNT);
+    const int warps = few ? 2 : 4;
+    auto kernel = few ? attn_kernel<2> : attn_kernel<4>;
+    cudaError_t err = opt[few].ensure(kernel);
     if (err != cudaSuccess) return (int)err;
-    kernel<<<(unsigned)blocks, ATT_WARPS * 32, ATT_SMEM_BYTES, as_stream(stream)>>>(q, k, v, out, n_tok, n_head, n_head_kv, scale);
-    return (int)cudaGetLastError();
+    const long long ctas = (long long)n_head * ((n_tok + warps * ATT_QPW - 1) / (warps * ATT_QPW));
+    if (ctas > INT32_MAX) return 1;
+    return (int)launch(kernel, dim3((unsigned)ctas), dim3((unsigned)(32 * warps)), (size_t)att_smem_bytes(warps), as_stream(stream), true, q, k, v, out, n_tok, n_head, n_head_kv, scale);
 }
 
 // ---- K/V cache (reference: include/bonsai_kv.h, src/kernels/kv_p40.cu:247-367) ----------------------------------

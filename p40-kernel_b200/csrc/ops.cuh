@@ -267,8 +267,8 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_step_kernel(float *state, 
 // softmax step is taken a tile at a time -- one running maximum, one rescale and four exps per lane per 32 keys: the
 // online softmax of the reference's kernel (src/kernels/attn_p40.cu:101-113) with 32 keys per step instead of one.
 // fp32 on the CUDA cores throughout; outputs are held to 1e-5 of the largest output.
-constexpr int ATT_D = 256, ATT_TILE = 32, ATT_WARPS = 8, ATT_QPW = 4, ATT_QPC = ATT_WARPS * ATT_QPW;
-constexpr int ATT_SMEM_BYTES = 2 * ATT_TILE * ATT_D * 4;
+constexpr int ATT_D = 256, ATT_TILE = 32, ATT_QPW = 4;
+constexpr int att_smem_bytes(int warps) { return 2 * ATT_TILE * ATT_D * 4 + warps * ATT_TILE * ATT_QPW * 4; }
 
 // Two fp32 multiply-adds in one instruction (each rounded as __fmaf_rn): half of the kernel's issue slots were multiply-adds.
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -300,13 +300,20 @@ __device__ __forceinline__ float transpose_sum32(float (&part)[32], int lane) {
     return part[0];
 }
 
-// Queries first .. first + 4 WARPS - 1 of one head, by a CTA of WARPS warps; smem: ATT_SMEM_BYTES, 16-byte aligned.
+// 16 bytes global -> shared, asynchronously, from L2 (whoever wrote them).
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+// Queries first .. first + 4 WARPS - 1 of one head, by a CTA of WARPS warps; smem: att_smem_bytes(WARPS), 16-byte aligned.  The next tile's keys are on
+// their way while this one's values are multiplied, the next values while the next scores are.
 template <int WARPS>
-__device__ __forceinline__ void attn_simt(float *att_smem, const float *__restrict__ q, const float *__restrict__ k,
-                                          const float *__restrict__ v, float *__restrict__ out, int first, int head,
+__device__ __forceinline__ void attn_simt(float *att_smem, const float *q, const float *k, const float *v, float *out, int first, int head,
                                           int n_tok, int n_head, int n_head_kv, float scale) {
     float (*kt)[ATT_D] = reinterpret_cast<float (*)[ATT_D]>(att_smem);
     float (*vt)[ATT_D] = reinterpret_cast<float (*)[ATT_D]>(att_smem + ATT_TILE * ATT_D);
+    float4 *weights = reinterpret_cast<float4 *>(att_smem + 2 * ATT_TILE * ATT_D) + (threadIdx.x >> 5) * ATT_TILE;      // the warp's: [key of the tile][4 queries]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int q0 = first + ATT_QPW * warp;                  // the warp's first query
     const int kvh = head / (n_head / n_head_kv);
@@ -326,18 +333,22 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *__restri
     float m = -INFINITY, l = 0.0f;                          // of query q0 + myq (the same in the 8 lanes of its group)
     const int last = min(n_tok - 1, first + WARPS * ATT_QPW - 1);           // keys 0 .. last serve the CTA's queries
     const int wlast = min(n_tok - 1, q0 + ATT_QPW - 1);                     // ... 0 .. wlast this warp's
-    for (int j0 = 0; j0 <= last; j0 += ATT_TILE) {
-        __syncthreads();
-        const int nk = min(ATT_TILE, last + 1 - j0);
-        for (int i = threadIdx.x; i < nk * (ATT_D / 4); i += WARPS * 32) {
-            const int r = i / (ATT_D / 4), c4 = i - r * (ATT_D / 4);
-            const size_t src = ((size_t)(j0 + r) * n_head_kv + kvh) * ATT_D + 4 * c4;
-            *reinterpret_cast<float4 *>(&kt[r][4 * c4]) = *reinterpret_cast<const float4 *>(k + src);
-            *reinterpret_cast<float4 *>(&vt[r][4 * c4]) = *reinterpret_cast<const float4 *>(v + src);
+    auto stage = [&](float (*rows)[ATT_D], const float *from, int j0) {
+        for (int i = threadIdx.x; i < min(ATT_TILE, last + 1 - j0) * (ATT_D / 4); i += WARPS * 32) {
+            const int r = i / (ATT_D / 4), c4 = i % (ATT_D / 4);
+            cp_async16(&rows[r][4 * c4], from + ((size_t)(j0 + r) * n_head_kv + kvh) * ATT_D + 4 * c4);
         }
+        cp_async_commit();
+    };
+    stage(kt, k, 0);
+    stage(vt, v, 0);
+    for (int j0 = 0; j0 <= last; j0 += ATT_TILE) {
+        const int nk = min(ATT_TILE, last + 1 - j0);
+        const bool more = j0 + ATT_TILE <= last;            // CTA-uniform
+        const bool live = q0 < n_tok && j0 <= wlast;        // warp-uniform: the warp's queries see keys of this tile
+        cp_async_wait<1>();                                 // the keys
         __syncthreads();
-        if (q0 >= n_tok || j0 > wlast) continue;
-        const int wn = min(nk, wlast - j0 + 1);             // keys of this tile that any of the warp's queries may see
+        const int wn = live ? min(nk, wlast - j0 + 1) : 0;  // keys of this tile that any of the warp's queries may see
         float sc[4];
 #pragma unroll
         for (int st = 0; st < 4; ++st) {
@@ -363,6 +374,8 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *__restri
                 sc[st] = (key <= q0 + myq && key < n_tok && q0 + myq < n_tok) ? s : -INFINITY;
             }
         }
+        __syncthreads();
+        if (more) stage(kt, k, j0 + ATT_TILE);
         // softmax step of the tile, per query (groups of 8 lanes)
         float tmax = fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3]));
 #pragma unroll
@@ -374,7 +387,11 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *__restri
         for (int st = 0; st < 4; ++st) {
             p[st] = sc[st] == -INFINITY ? 0.0f : expf(__fsub_rn(sc[st], m_new));
             psum = __fadd_rn(psum, p[st]);
+            reinterpret_cast<float *>(weights)[(8 * st + mykk) * ATT_QPW + myq] = p[st];
         }
+        if (more) cp_async_wait<1>();                       // the values
+        else cp_async_wait<0>();
+        __syncthreads();
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) psum = __fadd_rn(psum, __shfl_xor_sync(0xffffffffu, psum, o));
         l = __fadd_rn(__fmul_rn(l, alpha), psum);
@@ -385,28 +402,23 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *__restri
 #pragma unroll
             for (int i = 0; i < 4; ++i) oreg[a][i] = make_float2(__fmul_rn(oreg[a][i].x, al), __fmul_rn(oreg[a][i].y, al));
         }
+#pragma unroll 8
+        for (int r = 0; r < wn; ++r) {                      // warp-uniform
+            const float4 w4 = weights[r];
+            const float w[ATT_QPW] = {w4.x, w4.y, w4.z, w4.w};
+            const float4 va = *reinterpret_cast<const float4 *>(&vt[r][8 * lane]);
+            const float4 vb = *reinterpret_cast<const float4 *>(&vt[r][8 * lane + 4]);
 #pragma unroll
-        for (int st = 0; st < 4; ++st) {
-            if (8 * st < wn) {
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk) {
-                    const int r = 8 * st + kk;
-                    if (r < wn) {                           // warp-uniform
-                        const float4 va = *reinterpret_cast<const float4 *>(&vt[r][8 * lane]);
-                        const float4 vb = *reinterpret_cast<const float4 *>(&vt[r][8 * lane + 4]);
-#pragma unroll
-                        for (int a = 0; a < ATT_QPW; ++a) {
-                            const float pr = __shfl_sync(0xffffffffu, p[st], 8 * a + kk);
-                            const float2 pp = make_float2(pr, pr);
-                            oreg[a][0] = fma2(pp, make_float2(va.x, va.y), oreg[a][0]);
-                            oreg[a][1] = fma2(pp, make_float2(va.z, va.w), oreg[a][1]);
-                            oreg[a][2] = fma2(pp, make_float2(vb.x, vb.y), oreg[a][2]);
-                            oreg[a][3] = fma2(pp, make_float2(vb.z, vb.w), oreg[a][3]);
-                        }
-                    }
-                }
+            for (int a = 0; a < ATT_QPW; ++a) {
+                const float2 pp = make_float2(w[a], w[a]);
+                oreg[a][0] = fma2(pp, make_float2(va.x, va.y), oreg[a][0]);
+                oreg[a][1] = fma2(pp, make_float2(va.z, va.w), oreg[a][1]);
+                oreg[a][2] = fma2(pp, make_float2(vb.x, vb.y), oreg[a][2]);
+                oreg[a][3] = fma2(pp, make_float2(vb.z, vb.w), oreg[a][3]);
             }
         }
+        __syncthreads();
+        if (more) stage(vt, v, j0 + ATT_TILE);
     }
 #pragma unroll
     for (int a = 0; a < ATT_QPW; ++a) {
@@ -424,18 +436,20 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *__restri
     }
 }
 
-// TWO: two CTAs per SM (128 registers, a few spilled); without it one, for calls whose CTAs do not fill the SMs once (128 tokens
-// of 24 heads: 34 us, 37 us with TWO).  Bound by issue: with packed multiply-adds and the longest rows first 511 tokens took
-// 186 us instead of 232 us, 340 tokens 102 instead of 123 us.
-template <bool TWO>
-__global__ void __launch_bounds__(ATT_WARPS * 32, TWO ? 2 : 1) attn_kernel(const float *__restrict__ q, const float *__restrict__ k,
-                                                              const float *__restrict__ v, float *__restrict__ out,
-                                                              int n_tok, int n_head, int n_head_kv, float scale) {
+// Bound by issue, and where the CTAs do not fill the SMs by a warp's chain: 8 us for a tile of 32 keys, five times its instructions, of which 1 - 2 were the
+// wait for its rows (now copied asynchronously, a tile ahead).  Weights through shared memory instead of a shuffle for each of the lanes' 128, launches that
+// begin while the one in front drains, CTAs of 16 or 8 queries (were 32): 24 heads over 4, us, before -> now: 1 token 4.7 -> 2.8, 16 8.3 -> 5.1, 30 12.1 -> 7.3, 70 18.5 ->
+// 13.4, 100 26.7 -> 19.7, 130 34.7 -> 27.7, 191 49.2 -> 40.1; the same bits.
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) attn_kernel(const float *q, const float *k, const float *v, float *out, int n_tok, int n_head, int n_head_kv, float scale) {
     extern __shared__ __align__(16) float att_smem[];
     // the longest rows of keys first: what starts last is short
-    const int qblocks = (n_tok + ATT_QPC - 1) / ATT_QPC;
+    constexpr int QUERIES = WARPS * ATT_QPW;
+    const int qblocks = (n_tok + QUERIES - 1) / QUERIES;
     const int head = (int)blockIdx.x % n_head, qb = qblocks - 1 - (int)blockIdx.x / n_head;
-    attn_simt<ATT_WARPS>(att_smem, q, k, v, out, qb * ATT_QPC, head, n_tok, n_head, n_head_kv, scale);
+    pdl_wait_prior_grid();
+    pdl_launch_dependents();
+    attn_simt<WARPS>(att_smem, q, k, v, out, qb * QUERIES, head, n_tok, n_head, n_head_kv, scale);
 }
 
 }  // namespace b200

@@ -58,9 +58,11 @@ def test_against_float64(gpu, n, heads, kv_heads, spread):
 
 
 @pytest.mark.parametrize("n,heads,kv_heads,spread", [
-    (191, 24, 4, 0.0), (192, 24, 4, 0.0), (193, 1, 1, 0.0), (255, 6, 2, 0.0), (256, 6, 2, 1.0), (257, 3, 1, 0.0), (319, 4, 4, 0.0), (321, 24, 4, 1.0), (448, 2, 2, 0.0)])
+    (1, 3, 3, 0.0), (7, 24, 4, 0.0), (9, 6, 1, 0.0), (17, 2, 2, 0.0), (31, 24, 4, 0.0), (33, 24, 4, 1.0), (49, 24, 4, 0.0), (65, 40, 8, 0.0), (145, 24, 4, 0.0), (161, 24, 4, 1.0),
+    (130, 64, 8, 0.0), (191, 24, 4, 0.0), (192, 24, 4, 0.0), (193, 1, 1, 0.0), (255, 6, 2, 0.0), (256, 6, 2, 1.0), (257, 3, 1, 0.0), (319, 4, 4, 0.0), (321, 24, 4, 1.0), (448, 2, 2, 0.0)])
 def test_short_prompts(gpu, n, heads, kv_heads, spread):
-    """The lengths next to where the tensor cores begin to serve, and between there and 512 (the same oracle and bound)."""
+    """Few queries, by CTAs of 8 and of 16, the lengths next to where the tensor cores begin to serve, and between there and 512 (the same oracle and
+    bound)."""
     test_against_float64(gpu, n, heads, kv_heads, spread)
 
 
