@@ -261,26 +261,34 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
 
     // ---- q: row of the thread, 64 dims; high plane to shared memory, low plane to tensor memory.  (The launch this one may
     // run beside is attn_planes_kernel, which does not write q.)
+    // Queries and outputs pass through shared memory (the planes' of k and v, a warp's 32 rows of 64 values each, 16-byte pieces swizzled), where a row's
+    // values become a thread's: 512 bytes of two rows per access.  (A row per thread, 16 bytes of 32 rows per access: 12 us of a CTA's time in front of its
+    // tiles and 7 behind them, where a tile takes 4.)
+    float4 *box = reinterpret_cast<float4 *>(kpl) + warp * 512;
+    const int row0 = first + 32 * (warp & 3);
     float qf;
     uint32_t seen;                                                       // magnitude bits of the row's largest q
     {
         float x[64];
         uint32_t m = 0;
-        const float *src = q + ((size_t)query * n_head + head) * ATT_D + 64 * cg;
-        if (query < n_tok) {
-            if ((reinterpret_cast<uintptr_t>(q) & 15u) == 0) {
+        if ((reinterpret_cast<uintptr_t>(q) & 15u) == 0) {
 #pragma unroll
-                for (int e = 0; e < 64; e += 4) {
-                    const float4 a = *reinterpret_cast<const float4 *>(src + e);
-                    x[e] = a.x; x[e + 1] = a.y; x[e + 2] = a.z; x[e + 3] = a.w;
-                }
-            } else {
+            for (int i = 0; i < 16; ++i) {
+                const int r = 2 * i + (lane >> 4), c = lane & 15;
+                if (row0 + r < n_tok) cp_async16(box + r * 16 + (c ^ (r & 15)), q + ((size_t)(row0 + r) * n_head + head) * ATT_D + 64 * cg + 4 * c);
+            }
+            cp_async_commit();
+            cp_async_wait<0>();
+            __syncwarp();
 #pragma unroll
-                for (int e = 0; e < 64; ++e) x[e] = src[e];
+            for (int c = 0; c < 16; ++c) {
+                const float4 a = query < n_tok ? box[lane * 16 + (c ^ (lane & 15))] : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[4 * c] = a.x; x[4 * c + 1] = a.y; x[4 * c + 2] = a.z; x[4 * c + 3] = a.w;
             }
         } else {
+            const float *src = q + ((size_t)query * n_head + head) * ATT_D + 64 * cg;
 #pragma unroll
-            for (int e = 0; e < 64; ++e) x[e] = 0.0f;
+            for (int e = 0; e < 64; ++e) x[e] = query < n_tok ? src[e] : 0.0f;
         }
 #pragma unroll
         for (int e = 0; e < 64; ++e) {
@@ -514,18 +522,22 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
         attn_redo(reinterpret_cast<float *>(qhi), q, k, v, out, first, head, n_tok, n_head, n_head_kv, scale);
         return;
     }
-    if (query < n_tok) {
-        const float l = __fadd_rn(__fadd_rn(red[row], red[ATC_M + row]), __fadd_rn(red[2 * ATC_M + row], red[3 * ATC_M + row]));
-        const float inv = __fdiv_rn(1.0f, l);
-        float *dst = out + ((size_t)query * n_head + head) * ATT_D + 64 * cg;
-        if ((reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+    const float l = __fadd_rn(__fadd_rn(red[row], red[ATC_M + row]), __fadd_rn(red[2 * ATC_M + row], red[3 * ATC_M + row]));
+    const float inv = __fdiv_rn(1.0f, l);
+    if ((reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
 #pragma unroll
-            for (int e = 0; e < 64; e += 4)
-                *reinterpret_cast<float4 *>(dst + e) = make_float4(__fmul_rn(acc[e], inv), __fmul_rn(acc[e + 1], inv), __fmul_rn(acc[e + 2], inv), __fmul_rn(acc[e + 3], inv));
-        } else {
+        for (int c = 0; c < 16; ++c)
+            box[lane * 16 + (c ^ (lane & 15))] = make_float4(__fmul_rn(acc[4 * c], inv), __fmul_rn(acc[4 * c + 1], inv), __fmul_rn(acc[4 * c + 2], inv), __fmul_rn(acc[4 * c + 3], inv));
+        __syncwarp();
 #pragma unroll
-            for (int e = 0; e < 64; ++e) dst[e] = __fmul_rn(acc[e], inv);
+        for (int i = 0; i < 16; ++i) {
+            const int r = 2 * i + (lane >> 4), c = lane & 15;
+            if (row0 + r < n_tok) *reinterpret_cast<float4 *>(out + ((size_t)(row0 + r) * n_head + head) * ATT_D + 64 * cg + 4 * c) = box[r * 16 + (c ^ (r & 15))];
         }
+    } else if (query < n_tok) {
+        float *dst = out + ((size_t)query * n_head + head) * ATT_D + 64 * cg;
+#pragma unroll
+        for (int e = 0; e < 64; ++e) dst[e] = __fmul_rn(acc[e], inv);
     }
 }
 
