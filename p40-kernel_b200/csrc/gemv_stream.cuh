@@ -229,8 +229,11 @@ __device__ __forceinline__ void put_activation(uint32_t *act_q, float *act_s, in
 // REPACK = true (with FUSED) is bonsai_p40_gemv_repack: W is in the repacked layout and x is quantised WITHOUT a
 // rotation (src/kernels/gemv_repack_p40.cu:91-162 fuses exactly that).
 // CL > 1 (with REPACK): the CTAs of a cluster quantise a share of x each and store it into the tables of all of them.
+// Registers: behind a quantiser of its own the mat-vec's CTAs fill the SMs that the next call's quantiser, eight warps of 32 registers, starts on while they run:
+// with 118 per thread there was no room beside them, and calls of 148 CTAs took 1 - 2 us more (5120 -> 2368 6.57 -> 5.44 us, -> 40000 17.7 -> 16.4, 17408 -> 1776
+// 9.2 -> 7.0; with SMs left over the same).  576 threads would have 112.
 template <bool FUSED, bool REPACK = false, int CL = 1>
-__global__ void __launch_bounds__(512, 1) gemv_stream_kernel(const uint8_t *__restrict__ W, const uint32_t *xq,
+__global__ void __launch_bounds__(FUSED ? 512 : 576, 1) gemv_stream_kernel(const uint8_t *__restrict__ W, const uint32_t *xq,
                                                              float *y, const StreamParams P,
                                                              const float *x, const float *signs,
                                                              uint32_t *xq_out) {
