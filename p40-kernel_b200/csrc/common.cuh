@@ -57,6 +57,35 @@ __device__ __forceinline__ int round_ties_away(float t) {
     return q;
 }
 
+// ---- two fp32 operations in one instruction, each rounded as __fmaf_rn and __fadd_rn ----
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t"
+        ".reg .b64 a, b, c, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 b, {%4, %5};\n\t"
+        "mov.b64 c, {%6, %7};\n\t"
+        "fma.rn.f32x2 d, a, b, c;\n\t"
+        "mov.b64 {%0, %1}, d;\n\t"
+        "}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t"
+        ".reg .b64 a, b, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 b, {%4, %5};\n\t"
+        "add.rn.f32x2 d, a, b;\n\t"
+        "mov.b64 {%0, %1}, d;\n\t"
+        "}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+
 // ---- integer dot ------------------------------------------------------------------------------
 // Four unsigned bytes of `w` times four signed bytes of `a`, plus c (reference: the host dp4a
 // emulation, src/p40_common.h:131-140, applied to codes 0..3 which are non-negative either way).

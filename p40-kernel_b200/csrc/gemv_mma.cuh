@@ -327,8 +327,10 @@ __global__ void __launch_bounds__(MMA_THREADS, 1) gemv_mma_kernel(const uint8_t 
 // 4 + t are the matching B rows); with C = -s (the activation sum) D would be the host's int32 sumi
 // (src/pq2_0.h:149-169) bit for bit, and it is that plus a constant: C starts at 0x4B400000 - s, so
 // D = 0x4B400000 + sumi, which read as a float is 12582912 + sumi exactly (|sumi| <= 8192), and one subtraction gives
-// (float)sumi without a conversion instruction.  Terms (dw * da) * (float)sumi as on the host, added in ascending
-// chunk order inside an item, items and segments in ascending order.
+// (float)sumi without a conversion instruction.  A block's chunks are added with their activation scales, the block with its weight scale, one rounding
+// each and two tokens to an instruction, in ascending order, items and segments too.  (Term by term as on the host, (dw * da) * (float)sumi and an addition,
+// sixteen instructions per MMA where four are now: 8 tokens of 5120 -> 17408 16.2 -> 14.6 us, of 5120 -> 60000 45.5 -> 40.0, 16 27.4 -> 25.6; relative error against
+// 64 bits 9.6e-8 -> 6.6e-8 at 5120, 1.07e-7 -> 8.0e-8 at 17408.)
 //
 // The kernel is bound by the shared-memory data pipe (loads of code words, of activation words and of the decoded
 // headers: ~12 wavefronts per MMA with one MMA per chunk), so a chunk's operand loads serve as many MMAs as fit:
@@ -359,7 +361,7 @@ struct MmabGeom {
     int nslot, slot_bytes;   // a slot holds nrg groups of 16 rows
     int pairs_max;           // block pairs in the longest segment
     int items, ppi;          // items per tile, block pairs per item
-    int act_bufs, act_buf_bytes;   // a buffer = the segment's Q8_1 blocks, then {da, 0x4B400000 - s} of every (chunk, token)
+    int act_bufs, act_buf_bytes;   // a buffer = the segment's Q8_1 blocks, then da of every (chunk, token), then 0x4B400000 - s
     int act_tab_off;               // bytes from a buffer's start to that table
     int early;                     // 1: two weight tiles may be copied while the previous launch still runs
     int ntg, nrg;                  // token groups of 8, row groups of 16 that share a chunk's operand loads
@@ -524,7 +526,7 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
         const size_t nch = (size_t)P.nb * 4;
         const int cstride = 9 * n_tok;                                  // words from a chunk's blocks to the next chunk's
         const int off_b = 9 * g + 1 + t;                                // the lane's token: int8 words t and 4 + t
-        const int off_h = 4 * t;                                        // {da, c} of tokens 2t and 2t + 1 in a chunk's table row (8 NTG tokens)
+        const int off_h = 2 * t;                                        // tokens 2t and 2t + 1 in a chunk's table row (8 NTG tokens)
         const int sh0 = 16 + 2 * t, sh1 = 2 * t;
         int q_seen = -1;
         const int nitems = P.items * ntiles;
@@ -544,15 +546,16 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
             if (!wait_count(&issued[0], T + 1)) break;
             if (!mbar_wait_bounded(&full[slot], (uint32_t)(lap & 1))) break;
             const int p_lo = k * P.ppi, p_hi = min(p_lo + P.ppi, sl >> 1);      // empty in a short segment
-            float acc[NRG][NTG][4];
+            float2 acc[NRG][NTG][2];                        // rows g and g + 8, tokens 2 t and 2 t + 1
 #pragma unroll
             for (int h = 0; h < NRG; ++h)
 #pragma unroll
-                for (int u = 0; u < NTG; ++u) acc[h][u][0] = acc[h][u][1] = acc[h][u][2] = acc[h][u][3] = 0.0f;
+                for (int u = 0; u < NTG; ++u) acc[h][u][0] = acc[h][u][1] = make_float2(0.0f, 0.0f);
             if (p_lo < p_hi) {
                 const uint8_t *r0 = ring + (size_t)slot * P.slot_bytes + (size_t)68 * p_lo + (size_t)g * P.stride;
                 const uint32_t *pb = act + (size_t)8 * p_lo * cstride + off_b;
-                const uint32_t *ph = act + P.act_tab_off / 4 + (size_t)8 * p_lo * 16 * NTG + off_h;
+                const uint32_t *ph = act + P.act_tab_off / 4 + (size_t)8 * p_lo * 8 * NTG + off_h;
+                const int tab_c = P.pairs_max * 64 * NTG;       // words from a chunk's da to its c
                 for (int p = p_lo; p < p_hi; ++p, r0 += 68) {
 #pragma unroll
                     for (int bl = 0; bl < 2; ++bl) {
@@ -572,15 +575,22 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
                             dw[h][0] = f16_bits_to_f32(bl ? (e[h][0][0] >> 16) : (e[h][0][0] & 0xFFFFu));
                             dw[h][1] = f16_bits_to_f32(bl ? (e[h][1][0] >> 16) : (e[h][1][0] & 0xFFFFu));
                         }
+                        float2 blk[NRG][NTG][2];            // of the block, without its weight scale
 #pragma unroll
-                        for (int c = 0; c < 4; ++c, pb += cstride, ph += 16 * NTG) {
+                        for (int h = 0; h < NRG; ++h)
+#pragma unroll
+                            for (int u = 0; u < NTG; ++u) blk[h][u][0] = blk[h][u][1] = make_float2(0.0f, 0.0f);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c, pb += cstride, ph += 8 * NTG) {
                             uint32_t bw[NTG][2];
-                            uint4 hv[NTG];
+                            float2 da[NTG];
+                            int2 ci[NTG];
 #pragma unroll
                             for (int u = 0; u < NTG; ++u) {
                                 bw[u][0] = pb[72 * u];
                                 bw[u][1] = pb[72 * u + 4];
-                                hv[u] = *reinterpret_cast<const uint4 *>(ph + 16 * u);
+                                da[u] = *reinterpret_cast<const float2 *>(ph + 8 * u);
+                                ci[u] = *reinterpret_cast<const int2 *>(ph + tab_c + 8 * u);
                             }
 #pragma unroll
                             for (int h = 0; h < NRG; ++h) {
@@ -598,27 +608,30 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
                                 for (int i = 0; i < 4; ++i) a[i] &= 0x03030303u;
 #pragma unroll
                                 for (int u = 0; u < NTG; ++u) {
-                                    const int cin[4] = {(int)hv[u].y, (int)hv[u].w, (int)hv[u].y, (int)hv[u].w};
+                                    const int cin[4] = {ci[u].x, ci[u].y, ci[u].x, ci[u].y};
                                     int d[4];
                                     mma_u8s8(d, a, bw[u][0], bw[u][1], cin);
-                                    const float da0 = __uint_as_float(hv[u].x), da1 = __uint_as_float(hv[u].z);
-                                    const float f0 = __fsub_rn(__int_as_float(d[0]), 12582912.0f), f1 = __fsub_rn(__int_as_float(d[1]), 12582912.0f);
-                                    const float f2 = __fsub_rn(__int_as_float(d[2]), 12582912.0f), f3 = __fsub_rn(__int_as_float(d[3]), 12582912.0f);
-                                    acc[h][u][0] = __fadd_rn(acc[h][u][0], __fmul_rn(__fmul_rn(dw[h][0], da0), f0));
-                                    acc[h][u][1] = __fadd_rn(acc[h][u][1], __fmul_rn(__fmul_rn(dw[h][0], da1), f1));
-                                    acc[h][u][2] = __fadd_rn(acc[h][u][2], __fmul_rn(__fmul_rn(dw[h][1], da0), f2));
-                                    acc[h][u][3] = __fadd_rn(acc[h][u][3], __fmul_rn(__fmul_rn(dw[h][1], da1), f3));
+                                    const float2 magic = make_float2(-12582912.0f, -12582912.0f);
+                                    blk[h][u][0] = fma2(add2(make_float2(__int_as_float(d[0]), __int_as_float(d[1])), magic), da[u], blk[h][u][0]);
+                                    blk[h][u][1] = fma2(add2(make_float2(__int_as_float(d[2]), __int_as_float(d[3])), magic), da[u], blk[h][u][1]);
                                     if (DUMP && u == 0 && NRG * pl + h < gb) {
-                                        const int ci = 4 * (sb + 2 * p + bl) + c;
+                                        const int at = 4 * (sb + 2 * p + bl) + c;
                                         const int ra = 16 * group_index(b, NRG * pl + h) + g, rb = ra + 8, ta = 2 * t, tb = ta + 1;
-                                        if (ra < P.n_out && ta < n_tok) dump[((size_t)ra * n_tok + ta) * nch + ci] = d[0] - MMAB_MAGIC;
-                                        if (ra < P.n_out && tb < n_tok) dump[((size_t)ra * n_tok + tb) * nch + ci] = d[1] - MMAB_MAGIC;
-                                        if (rb < P.n_out && ta < n_tok) dump[((size_t)rb * n_tok + ta) * nch + ci] = d[2] - MMAB_MAGIC;
-                                        if (rb < P.n_out && tb < n_tok) dump[((size_t)rb * n_tok + tb) * nch + ci] = d[3] - MMAB_MAGIC;
+                                        if (ra < P.n_out && ta < n_tok) dump[((size_t)ra * n_tok + ta) * nch + at] = d[0] - MMAB_MAGIC;
+                                        if (ra < P.n_out && tb < n_tok) dump[((size_t)ra * n_tok + tb) * nch + at] = d[1] - MMAB_MAGIC;
+                                        if (rb < P.n_out && ta < n_tok) dump[((size_t)rb * n_tok + ta) * nch + at] = d[2] - MMAB_MAGIC;
+                                        if (rb < P.n_out && tb < n_tok) dump[((size_t)rb * n_tok + tb) * nch + at] = d[3] - MMAB_MAGIC;
                                     }
                                 }
                             }
                         }
+#pragma unroll
+                        for (int h = 0; h < NRG; ++h)
+#pragma unroll
+                            for (int u = 0; u < NTG; ++u) {
+                                acc[h][u][0] = fma2(blk[h][u][0], make_float2(dw[h][0], dw[h][0]), acc[h][u][0]);
+                                acc[h][u][1] = fma2(blk[h][u][1], make_float2(dw[h][1], dw[h][1]), acc[h][u][1]);
+                            }
                     }
                 }
             }
@@ -632,7 +645,7 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
                     for (int u = 0; u < NTG; ++u) {
                         float *ts = tsum + (((size_t)slot * NRG + h) * NTG + u) * 128;
                         float2 *lo = reinterpret_cast<float2 *>(ts + g * 8 + 2 * t), *hi = reinterpret_cast<float2 *>(ts + (g + 8) * 8 + 2 * t);
-                        float2 vlo = make_float2(acc[h][u][0], acc[h][u][1]), vhi = make_float2(acc[h][u][2], acc[h][u][3]);
+                        float2 vlo = acc[h][u][0], vhi = acc[h][u][1];
                         if (k > 0) {
                             const float2 olo = *lo, ohi = *hi;
                             vlo.x = __fadd_rn(olo.x, vlo.x); vlo.y = __fadd_rn(olo.y, vlo.y);
@@ -712,7 +725,7 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
     } else {
         // activation warp: a step's Q8_1 blocks are asked for up to two steps ahead (three buffers; a buffer is free when
         // every tile of the step three before is taken), and when they have landed their headers are decoded once for
-        // all compute warps: {da as fp32, 0x4B400000 - s} per (chunk, token)
+        // all compute warps: da as fp32, and 0x4B400000 - s, per (chunk, token)
         const bool bulk_ok = (reinterpret_cast<uintptr_t>(Xq) & 15u) == 0;
         const uint64_t keep = policy_evict_normal();            // every CTA reads the same blocks: they stay in L2
         const int nsteps = P.nseg > 1 ? nbatch * P.nseg : (mg > 0 ? 1 : 0);
@@ -761,7 +774,8 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
             if (!mbar_wait_bounded(&actfull[ab], P.nseg > 1 ? (uint32_t)(q3 & 1) : 0u)) break;
             const int j = P.nseg > 1 ? qc % P.nseg : 0;
             const uint32_t *blk = reinterpret_cast<const uint32_t *>(actbuf + (size_t)ab * P.act_buf_bytes);
-            uint2 *tab = reinterpret_cast<uint2 *>(actbuf + (size_t)ab * P.act_buf_bytes + P.act_tab_off);
+            float *tab_d = reinterpret_cast<float *>(actbuf + (size_t)ab * P.act_buf_bytes + P.act_tab_off);
+            int *tab_c = reinterpret_cast<int *>(tab_d + P.pairs_max * 64 * NTG);
             // record i = chunk * TPC + tok (TPC = 8 NTG table entries per chunk): the lane's token is lane % TPC, its
             // chunks lane / TPC, + 32 / TPC, ...; all loads of a round first
             constexpr int TPC = 8 * NTG, CPW = 32 / TPC;
@@ -776,8 +790,10 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
                     h[u] = (i0 + 32 * u < n && tok < n_tok) ? src_h[(size_t)CPW * u * n_tok * 9] : 0u;
 #pragma unroll
                 for (int u = 0; u < CONV_UNROLL; ++u)
-                    if (i0 + 32 * u < n)
-                        tab[i0 + 32 * u] = make_uint2(__float_as_uint(f16_bits_to_f32(h[u] & 0xFFFFu)), (uint32_t)(MMAB_MAGIC - ((int)h[u] >> 16)));
+                    if (i0 + 32 * u < n) {
+                        tab_d[i0 + 32 * u] = f16_bits_to_f32(h[u] & 0xFFFFu);
+                        tab_c[i0 + 32 * u] = MMAB_MAGIC - ((int)h[u] >> 16);
+                    }
             }
             __syncwarp();
             if (lane == 0) {

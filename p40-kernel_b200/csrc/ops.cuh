@@ -270,21 +270,6 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_step_kernel(float *state, 
 constexpr int ATT_D = 256, ATT_TILE = 32, ATT_QPW = 4;
 constexpr int att_smem_bytes(int warps) { return 2 * ATT_TILE * ATT_D * 4 + warps * ATT_TILE * ATT_QPW * 4; }
 
-// Two fp32 multiply-adds in one instruction (each rounded as __fmaf_rn): half of the kernel's issue slots were multiply-adds.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{\n\t"
-        ".reg .b64 a, b, c, d;\n\t"
-        "mov.b64 a, {%2, %3};\n\t"
-        "mov.b64 b, {%4, %5};\n\t"
-        "mov.b64 c, {%6, %7};\n\t"
-        "fma.rn.f32x2 d, a, b, c;\n\t"
-        "mov.b64 {%0, %1}, d;\n\t"
-        "}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
 // part[r] of every lane -> returned value of lane r = sum over the lanes of part[r] (r = 0 .. 31).
 __device__ __forceinline__ float transpose_sum32(float (&part)[32], int lane) {
 #pragma unroll
