@@ -602,7 +602,7 @@ static int linear_one_launch(const void *W, const float *x, const float *signs, 
     // 2.45), -> 4096 4.36 / 3.03; 3072 -> 1500 4.80 / 3.45; 5120 -> 64 4.54 / 3.24 (3.78 / 3.04), -> 1024 4.92 / 3.91 (3.88 / 3.68), -> 1850 5.38 / 4.10;
     // 6144 -> 1000 5.15 / 4.22; 8192 -> 600 5.48 / 4.44.  With more pieces per warp, two blocks per CTA or CTAs two to an SM a graph's replay of two launches
     // is ahead: 5120 -> 3000 5.70 / 5.61 (4.84 / 5.28), 9216 -> 600 5.54 / 5.00 (4.40 / 4.80), 4096 -> 1500 in 32 clusters 5.07 / 4.41 (3.90 / 4.18).
-    if (nfb <= FEW_MAX_CLUSTER && plan_stream(n_out, nb, -1, sp, threads, smem_bytes)) {
+    if (nfb <= FEW_MAX_CLUSTER && plan_stream(n_out, nb, g_opt_gemv_variant.load(), sp, threads, smem_bytes)) {
         static const int FEW_ALONE[FEW_MAX_CLUSTER + 1] = {0, SM_COUNT, 74, 44, 24, 24, 15, 15, 15};
         const int room = nfb == 1 ? SM_COUNT : g_few_clusters[nfb].ask(gemv_few_kernel<FEW_HELD>, g_few_opt[FEW_HELD - 1], (unsigned)nfb, 32 * FEW_WARPS);
         const long long most = std::min(room, FEW_ALONE[nfb]), quads_in_all = (n_out + 3) / 4;
@@ -613,7 +613,7 @@ static int linear_one_launch(const void *W, const float *x, const float *signs, 
             attr[0].val.clusterDim.x = (unsigned)nfb;
             cfg.gridDim = dim3(clusters * (unsigned)nfb);
             cfg.blockDim = dim3(32 * FEW_WARPS);
-            cfg.dynamicSmemBytes = (size_t)few_smem_bytes(nb, quads);
+            cfg.dynamicSmemBytes = (size_t)few_smem_bytes(nb, quads, sp.nseg);
             cfg.attrs = nfb == 1 ? attr + 1 : attr;
             cfg.numAttrs = (nfb > 1) + (g_opt_overlap.load() != 0);
             auto go = [&](auto kernel, SmemOptIn &o) -> cudaError_t {

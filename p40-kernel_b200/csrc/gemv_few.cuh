@@ -22,8 +22,8 @@
 namespace b200 {
 
 constexpr int FEW_WARPS = 10, FEW_HELD = 2, FEW_MAX_CLUSTER = 8;
-inline int few_smem_bytes(int nb, int quads) {
-    return 16 + nb * (STREAM_ACT_WORDS + 4 + 4) * 4 + FWHT_N * 4 + quads * (nb / 8) * 32 * 16 + 4 * quads * ((nb + 39) / 40) * 4;
+inline int few_smem_bytes(int nb, int quads, int nseg) {
+    return 16 + nb * (STREAM_ACT_WORDS + 4 + 4) * 4 + FWHT_N * 4 + quads * (nb / 8) * 32 * 16 + 4 * quads * nseg * 4;
 }
 
 // A cluster of nb / 8 CTAs (at most 8), each rotates the 1024-block of its rank; a CTA takes 4 * quads rows: quads * nb / 8 pieces, at most HELD per warp.
