@@ -20,6 +20,8 @@ namespace b200 {
 // ---- quantiser core: 8 consecutive lanes own one 32-chunk, lane g (0..7) holds x[4g..4g+3] ----
 // Returns through `word` the Q8_1 data word this lane stores (word index g of qs) and through
 // `header` the d|s word (valid on every lane of the group).
+// LONG: rounding in the longer form, the same values (list launch: round_ties_away_long).
+template <bool LONG = false>
 __device__ __forceinline__ void quantise_chunk_8lanes(const float (&v)[4], int lane, uint32_t &word, uint32_t &header) {
     float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
 #pragma unroll
@@ -30,7 +32,7 @@ __device__ __forceinline__ void quantise_chunk_8lanes(const float (&v)[4], int l
     uint32_t packed = 0;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        int q = round_ties_away(__fmul_rn(v[e], id));
+        int q = LONG ? round_ties_away_long(__fmul_rn(v[e], id)) : round_ties_away(__fmul_rn(v[e], id));
         q = max(-127, min(127, q));
         sum += q;
         packed |= ((uint32_t)q & 0xFFu) << (8 * e);
@@ -53,59 +55,58 @@ __device__ __forceinline__ void quantise_chunk_8lanes(const float (&v)[4], int l
 
 // The same for N (up to eight) chunks of each eight lanes at once, the N chains side by side; lane g of the eight divides for chunk
 // g alone.
-template <int N>
+template <int N, bool LONG = false>
 __device__ __forceinline__ void quantise_chunks_8lanes(const float (&v)[N][4], int lane, uint32_t (&word)[N], uint32_t (&header)[N]) {
-    static_assert(N > 1 && N <= 8, "a lane of the eight per chunk; nothing to share in one");
-    float amax[N], mine;
+    static_assert(N >= 1 && N <= 8, "a lane of the eight per chunk");
+    if constexpr (N == 1) {                 // nothing to share
+        quantise_chunk_8lanes<LONG>(v[0], lane, word[0], header[0]);
+    } else {
+        float amax[N], mine;
 #pragma unroll
-    for (int k = 0; k < N; ++k) amax[k] = fmaxf(fmaxf(fabsf(v[k][0]), fabsf(v[k][1])), fmaxf(fabsf(v[k][2]), fabsf(v[k][3])));
+        for (int k = 0; k < N; ++k) amax[k] = fmaxf(fmaxf(fabsf(v[k][0]), fabsf(v[k][1])), fmaxf(fabsf(v[k][2]), fabsf(v[k][3])));
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1)
+        for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
-        for (int k = 0; k < N; ++k) amax[k] = fmaxf(amax[k], __shfl_xor_sync(0xffffffffu, amax[k], o));
-    mine = amax[0];
+            for (int k = 0; k < N; ++k) amax[k] = fmaxf(amax[k], __shfl_xor_sync(0xffffffffu, amax[k], o));
+        mine = amax[0];
 #pragma unroll
-    for (int k = 1; k < N; ++k) mine = (lane & 7) == k ? amax[k] : mine;
-    const float d = __fdiv_rn(mine, 127.0f);
-    const float my_id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-    const uint32_t my_d16 = f32_to_f16_bits_ties_away(d);
-    int sum[N];
-    uint32_t packed[N], d16[N];
+        for (int k = 1; k < N; ++k) mine = (lane & 7) == k ? amax[k] : mine;
+        const float d = __fdiv_rn(mine, 127.0f);
+        const float my_id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+        const uint32_t my_d16 = f32_to_f16_bits_ties_away(d);
+        int sum[N];
+        uint32_t packed[N], d16[N];
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-        const float id = __shfl_sync(0xffffffffu, my_id, (lane & ~7) + k);
-        d16[k] = __shfl_sync(0xffffffffu, my_d16, (lane & ~7) + k);
-        sum[k] = 0;
-        packed[k] = 0;
+        for (int k = 0; k < N; ++k) {
+            const float id = __shfl_sync(0xffffffffu, my_id, (lane & ~7) + k);
+            d16[k] = __shfl_sync(0xffffffffu, my_d16, (lane & ~7) + k);
+            sum[k] = 0;
+            packed[k] = 0;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            int q = round_ties_away(__fmul_rn(v[k][e], id));
-            q = max(-127, min(127, q));
-            sum[k] += q;
-            packed[k] |= ((uint32_t)q & 0xFFu) << (8 * e);
+            for (int e = 0; e < 4; ++e) {
+                int q = LONG ? round_ties_away_long(__fmul_rn(v[k][e], id)) : round_ties_away(__fmul_rn(v[k][e], id));
+                q = max(-127, min(127, q));
+                sum[k] += q;
+                packed[k] |= ((uint32_t)q & 0xFFu) << (8 * e);
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+            for (int k = 0; k < N; ++k) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+        // the 4x4 byte transpose of quantise_chunk_8lanes
+        const int m = lane & 3, base = lane & ~3;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            word[k] = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t other = __shfl_sync(0xffffffffu, packed[k], base + j);
+                word[k] |= ((other >> (8 * m)) & 0xFFu) << (8 * j);
+            }
+            header[k] = d16[k] | (((uint32_t)sum[k] & 0xFFFFu) << 16);
         }
     }
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1)
-#pragma unroll
-        for (int k = 0; k < N; ++k) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
-    // the 4x4 byte transpose of quantise_chunk_8lanes
-    const int m = lane & 3, base = lane & ~3;
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-        word[k] = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t other = __shfl_sync(0xffffffffu, packed[k], base + j);
-            word[k] |= ((other >> (8 * m)) & 0xFFu) << (8 * j);
-        }
-        header[k] = d16[k] | (((uint32_t)sum[k] & 0xFFFFu) << 16);
-    }
-}
-
-template <>
-__device__ __forceinline__ void quantise_chunks_8lanes<1>(const float (&v)[1][4], int lane, uint32_t (&word)[1], uint32_t (&header)[1]) {
-    quantise_chunk_8lanes(v[0], lane, word[0], header[0]);
 }
 
 // Four consecutive floats: one 16-byte access when the caller's pointer allows it (VEC), else four 4-byte

@@ -48,8 +48,13 @@ __device__ __forceinline__ uint32_t f32_to_f16_bits_ties_away(float f) {
     return sign | ((uint32_t)e << 10) | q;
 }
 
-// lroundf semantics for |t| < 2^23 (a NaN gives 0, as the host's conversion does on x86-64).
-__device__ __forceinline__ int round_ties_away(float t) {
+// lroundf semantics for |t| < 2^23 (a NaN gives 0, as the host's conversion does on x86-64): towards zero behind the largest float below a half, which takes
+// every t whose fraction is a half or more across the next integer and no other (all 2 x 2^30 floats of that range were compared).
+__device__ __forceinline__ int round_ties_away(float t) { return __float2int_rz(__fadd_rn(t, copysignf(0x1.fffffep-2f, t))); }
+
+// The same, five instructions longer.  For the list launch, whose multiply comes out of the compiler differently with every change around it: with the short
+// form in its quantiser the layer sweep, which quantises nothing, takes 118.9 us instead of 115.3 (the decode step 3152 instead of 3163).
+__device__ __forceinline__ int round_ties_away_long(float t) {
     const float r = truncf(t);
     const float frac = __fsub_rn(t, r);          // exact
     int q = (t == t) ? (int)r : 0;

@@ -222,7 +222,7 @@ __device__ __forceinline__ void chain_back_units(const float4 *scratch, int u0, 
         const int u = u0 + k * step;
         fwht_slice_back(scratch + (u >> 3) * 256, u & 7, lane, v[k]);
     }
-    quantise_chunks_8lanes<N>(v, lane, word, header);
+    quantise_chunks_8lanes<N, true>(v, lane, word, header);
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         const int chunk = chunk0 + (u0 + k * step) * 4 + (lane >> 3);

@@ -75,6 +75,25 @@ def test_quantiser_golden_and_ties(gpu, golden):
         assert np.array_equal(host(out), want)
 
 
+def test_quantiser_next_to_ties(gpu, port):
+    """The floats in front of, on and behind every half in a chunk whose scale is 1: the host's rounding, by a warp's and by a batch's quantiser."""
+    import torch
+    half = np.arange(-127, 127, dtype=np.float32) + np.float32(0.5)
+    edge = np.concatenate([np.nextafter(half, np.float32(s * 200)) for s in (-1, 1)] + [half, np.float32([0, -0.0])])
+    x = np.full((32, 32), 127, dtype=np.float32)
+    flat = np.zeros(31 * 32, dtype=np.float32)
+    flat[: len(edge)] = edge
+    x[:, 1:] = flat.reshape(32, 31)
+    want = port.quantize_q8_1(x.reshape(-1), True)
+    xq = torch.empty(len(want), dtype=torch.uint8, device="cuda")
+    assert gpu.quant_activations(torch.from_numpy(x.reshape(-1)).cuda(), xq, 1024) == 0
+    assert np.array_equal(xq.cpu().numpy(), want)
+    batch = torch.empty(3 * len(want), dtype=torch.uint8, device="cuda")
+    assert gpu.quant_batch(torch.from_numpy(np.tile(x.reshape(-1), (3, 1))).cuda(), None, batch, 1024, 3, False) == 0
+    got = batch.cpu().numpy().reshape(32, 3, 36)             # chunk-major
+    assert all(np.array_equal(got[:, k].reshape(-1), want) for k in range(3))
+
+
 def test_quantiser_fp16_scale_ties(gpu, port):
     # chunks whose scale amax/127 falls exactly between two fp16 values: the host rounds away
     import torch
