@@ -441,12 +441,6 @@ GemvPlan plan_rows(long long n_out, size_t row_bytes, size_t fixed, int granule,
     return p;
 }
 
-// Whether a grid of small CTAs gains from being launched while its predecessor drains.  One that leaves much of the chip free does; one that
-// fills more than half of it, but not all of it, is spread unevenly when its first CTAs take what the predecessor leaves free (eight CTAs
-// per SM are resident: 2500 blocks through the rotation and the quantiser, 625 CTAs, 9.2 us and 11.9 with overlap; 629 CTAs of the
-// quantiser alone 2.9 and 3.3); a larger one does not care.
-bool worth_overlap(long long ctas, int upto_per_sm) { return ctas <= 4 * SM_COUNT || ctas > (long long)upto_per_sm * SM_COUNT; }
-
 // Any float pointers are taken, as by the reference; 16-byte aligned ones get 16-byte accesses.
 int launch_fwht(bool vec, const float *x, const float *signs, float *x_rot, void *xq, int64_t n_in, int64_t n_tok, bonsai_stream stream) {
     const long long blocks = (n_in / FWHT_N) * n_tok;
@@ -457,11 +451,10 @@ int launch_fwht(bool vec, const float *x, const float *signs, float *x_rot, void
     // the rotation alone (256: 2.3 and 2.2, 148: 2.0 and 2.4).
     const bool warps = blocks > (long long)SM_COUNT * (!xq ? 2 : (x_rot || !vec ? 18 : 10));
     const long long ctas = warps ? (blocks + FWHT_WARP_BLOCKS - 1) / FWHT_WARP_BLOCKS : blocks;
-    const bool overlap = worth_overlap(ctas, warps ? 8 : 6);
     if (warps)
         return (int)launch(vec ? fwht_quant_warp_kernel<true> : fwht_quant_warp_kernel<false>, dim3((unsigned)ctas), dim3(32 * FWHT_WARP_BLOCKS), 0,
-                           as_stream(stream), overlap, x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
-    return (int)launch(vec ? fwht_quant_kernel<true> : fwht_quant_kernel<false>, dim3((unsigned)ctas), dim3(FWHT_THREADS), 0, as_stream(stream), overlap,
+                           as_stream(stream), true, x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
+    return (int)launch(vec ? fwht_quant_kernel<true> : fwht_quant_kernel<false>, dim3((unsigned)ctas), dim3(FWHT_THREADS), 0, as_stream(stream), true,
                        x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
 }
 
@@ -475,7 +468,7 @@ int bonsai_p40_quant_activations(const float *x, void *out, int64_t n, bonsai_st
     const long long threads = n / 4;
     const int blocks = (int)((threads + 255) / 256);
     // any float pointer is taken, as by the reference; 16-byte aligned ones get 16-byte loads
-    return (int)launch(aligned16(x) ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), worth_overlap(blocks, 6), x,
+    return (int)launch(aligned16(x) ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, x,
                        static_cast<uint32_t *>(out), (int)n, 1);
 }
 
@@ -505,7 +498,7 @@ int bonsai_b200_quant_batch(const float *X, const float *signs, void *Xq, int64_
     const long long threads = n_in / 4 * n_tok;
     long long blocks = (threads + 255) / 256;
     if (blocks > 8 * SM_COUNT * 4) blocks = 8 * SM_COUNT * 4;
-    return (int)launch(vec ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), worth_overlap(blocks, 6), X,
+    return (int)launch(vec ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, X,
                        static_cast<uint32_t *>(Xq), (int)n_in, (int)n_tok);
 }
 
@@ -1595,12 +1588,12 @@ int bonsai_p40_rmsnorm(const float *x, const float *w, float *y, int64_t n_rows,
     if (n > INT32_MAX || n_rows > INT32_MAX || !aligned4(x) || !aligned4(w) || !aligned4(y)) return 1;
     const bool vec = n % 4 == 0 && aligned16(x) && aligned16(w) && aligned16(y);
     const dim3 threads(32 * (unsigned)std::min<int64_t>(RMS_WARPS, (n + 127) / 128));
-    auto run = [&](auto kernel, bool overlap) {
-        return (int)launch(kernel, dim3((unsigned)n_rows), threads, 0, as_stream(stream), overlap, x, w, y, (int)n, eps);
+    auto run = [&](auto kernel) {
+        return (int)launch(kernel, dim3((unsigned)n_rows), threads, 0, as_stream(stream), true, x, w, y, (int)n, eps);
     };
     auto go = [&](auto hold) {
         constexpr int HOLD = decltype(hold)::value;
-        return vec ? run(rmsnorm_kernel<true, HOLD>, true) : run(rmsnorm_kernel<false, HOLD>, true);
+        return vec ? run(rmsnorm_kernel<true, HOLD>) : run(rmsnorm_kernel<false, HOLD>);
     };
     // Rows that fit stay in registers, which costs CTAs per SM: with 16-byte accesses and up to five slices per warp that is ahead at any
     // count of rows (5120 values, 8192 rows: 54 us, 70 us read twice), with eight up to four rows per SM (6144 values, 512 rows: 5.8 and 7.0 us,
@@ -1609,10 +1602,10 @@ int bonsai_p40_rmsnorm(const float *x, const float *w, float *y, int64_t n_rows,
         if (n <= 1024) return go(std::integral_constant<int, 1>{});
         if (n <= 2 * 1024) return go(std::integral_constant<int, 2>{});
         if (n <= 3 * 1024) return go(std::integral_constant<int, 3>{});
-        if (n <= 5 * 1024 && vec) return run(rmsnorm_kernel<true, 5>, true);
+        if (n <= 5 * 1024 && vec) return run(rmsnorm_kernel<true, 5>);
         if (n <= 8 * 1024) return go(std::integral_constant<int, 8>{});
     }
-    if (!vec && n_rows > 2 * SM_COUNT) return run(rmsnorm_kernel<false, -1>, worth_overlap(n_rows, 8));
+    if (!vec && n_rows > 2 * SM_COUNT) return run(rmsnorm_kernel<false, -1>);
     return go(std::integral_constant<int, 0>{});
 }
 
