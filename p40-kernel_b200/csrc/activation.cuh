@@ -128,7 +128,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(256) quant_q8_1_kernel(const float *X, uint32_t *__restrict__ out,
                                                          int n_in, int n_tok) {
     pdl_wait_prior_grid();
-    pdl_launch_dependents_of_few();
+    if (gridDim.x <= 148) pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
     const int per_tok = n_in >> 2;
     const long long total = (long long)per_tok * n_tok;
@@ -257,8 +257,7 @@ __global__ void __launch_bounds__(FWHT_THREADS) fwht_quant_kernel(const float *X
     const int tok = (int)blockIdx.x / blocks_per_tok, blk = (int)blockIdx.x - tok * blocks_per_tok;
     const size_t base = (size_t)tok * n_in + (size_t)blk * FWHT_N + r * 128 + 4 * lane;
     pdl_wait_prior_grid();
-    // (340 CTAs in front of their mat-mul, 20 tokens of 17408: 32.6 us, 33.5 with the limit at an SM each; 629 alone 4.84, 3.78 at the end)
-    pdl_launch_dependents_of_few(3 * PDL_FEW);
+    if (gridDim.x <= 3 * 148) pdl_launch_dependents();         // (340 CTAs in front of their mat-mul, 20 tokens of 17408: 32.6 us, by ending 33.5; 629 alone 4.84 and 3.78)
     const float4 f = load_f4<VEC>(X + base);
     float v[4] = {f.x, f.y, f.z, f.w};
     if (signs) {

@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
         if (lane == 0) issued[0] = early;
     }
     pdl_wait_prior_grid();
-    pdl_launch_dependents();
+    // (the next launch comes as this one ends: RMSNorm, quantiser and this, 8 tokens, 5120 -> 17408 20.6 us and 18.3, 17408 -> 5120 23.9 and 22.8, 16 41.1 and 40.5)
     auto wait_count = [&](volatile int *c, int need) -> bool {
         for (uint32_t n = 0; n < (1u << 22); ++n) {
             if (*c >= need) return true;

@@ -41,7 +41,6 @@ __device__ __forceinline__ float swiglu1(float g, float u) {
 template <bool VEC>
 __global__ void __launch_bounds__(256) swiglu_kernel(const float *gate, const float *up, float *y, int n) {
     pdl_wait_prior_grid();
-    pdl_launch_dependents_of_few();
     const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (VEC) {
         if (i < n / 4) {
@@ -96,7 +95,6 @@ __global__ void __launch_bounds__(RMS_THREADS, HOLD < 0 || HOLD == 1 ? 8 : (HOLD
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nslice = (n + 127) >> 7;
     pdl_wait_prior_grid();
-    pdl_launch_dependents_of_few();
     if constexpr (HOLD > 0) {
         float4 f[HOLD], g[HOLD];
 #pragma unroll
