@@ -153,54 +153,12 @@ __global__ void __launch_bounds__(256) quant_q8_1_kernel(const float *X, uint32_
     }
 }
 
-// ---- rotation of a 1024-block by one warp -------------------------------------------------------
-// Lane l holds v[r][e] = element r*128 + 4*l + e (r = 0..7, e = 0..3): index bits 0-1 are e,
-// bits 2-6 the lane, bits 7-9 r.
-__device__ __forceinline__ void fwht1024_warp(float (&v)[8][4], int lane) {
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {   // h = 1, 2: inside the lane
-        float a = v[r][0], b = v[r][1], c = v[r][2], d = v[r][3];
-        float s0 = __fadd_rn(a, b), s1 = __fsub_rn(a, b), s2 = __fadd_rn(c, d), s3 = __fsub_rn(c, d);
-        v[r][0] = __fadd_rn(s0, s2); v[r][2] = __fsub_rn(s0, s2);
-        v[r][1] = __fadd_rn(s1, s3); v[r][3] = __fsub_rn(s1, s3);
-    }
-#pragma unroll
-    for (int s = 0; s < 5; ++s) {   // h = 4 .. 64: across lanes
-        const bool upper = (lane >> s) & 1;
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float mine = v[r][e];
-                const float other = __shfl_xor_sync(0xffffffffu, mine, 1 << s);
-                v[r][e] = upper ? __fsub_rn(other, mine) : __fadd_rn(mine, other);
-            }
-    }
-#pragma unroll
-    for (int s = 0; s < 3; ++s) {   // h = 128, 256, 512: across r
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-            if (!((r >> s) & 1)) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float a = v[r][e], b = v[r | (1 << s)][e];
-                    v[r][e] = __fadd_rn(a, b);
-                    v[r | (1 << s)][e] = __fsub_rn(a, b);
-                }
-            }
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[r][e] = __fmul_rn(v[r][e], 0.03125f);
-}
-
 // ---- rotation split over warps: one warp per 128-element slice ----------------------------------
 // A 1024-block is eight slices r = 0..7 of 128 consecutive elements; lane l of the slice's warp holds
 // elements 4l .. 4l+3.  The butterflies with h = 1 .. 64 stay inside a slice (front); those with
 // h = 128, 256, 512 combine the eight slices element by element (back), through shared memory.  Every
-// output is still produced by the same a + b / a - b as in fwht1024_warp, stage by stage, so the bits
-// are the same: a - b is computed as (-b) + a ... with IEEE addition that is the same rounding.
+// output is still produced by the host's a + b / a - b, stage by stage, so the bits are the same: a - b is
+// computed as (-b) + a ... with IEEE addition that is the same rounding.
 __device__ __forceinline__ void fwht_slice_front(float (&v)[4], int lane) {
     {
         const float a = v[0], b = v[1], c = v[2], d = v[3];
@@ -257,7 +215,7 @@ __global__ void __launch_bounds__(FWHT_THREADS) fwht_quant_kernel(const float *X
     const int tok = (int)blockIdx.x / blocks_per_tok, blk = (int)blockIdx.x - tok * blocks_per_tok;
     const size_t base = (size_t)tok * n_in + (size_t)blk * FWHT_N + r * 128 + 4 * lane;
     pdl_wait_prior_grid();
-    if (gridDim.x <= 3 * 148) pdl_launch_dependents();         // (340 CTAs in front of their mat-mul, 20 tokens of 17408: 32.6 us, by ending 33.5; 629 alone 4.84 and 3.78)
+    pdl_launch_dependents();
     const float4 f = load_f4<VEC>(X + base);
     float v[4] = {f.x, f.y, f.z, f.w};
     if (signs) {
@@ -280,60 +238,117 @@ __global__ void __launch_bounds__(FWHT_THREADS) fwht_quant_kernel(const float *X
     }
 }
 
-// The same, one block per warp and no exchange through shared memory: fewer instructions a block, a longer chain.
-constexpr int FWHT_WARP_BLOCKS = 4;
+// The same, a warp per block: fewer instructions a block, a longer chain.  Bound by instruction issue and by the pipe that shuffles and shared memory
+// have in common.  Element 32 c + p of the block: the butterflies with h = 1 .. 16 run with four values of a lane's, by shuffles over eight lanes; then c is
+// the register and p the lane (through shared memory) for h = 32 .. 512; then a lane has a chunk to itself, whose maximum, sum and words need no other lane.
+// (32 values of a lane's all the way, every exchange a shuffle, 256 of them a block, four warps a CTA, us: 2000 blocks with quantiser 5.82 -> 4.65, 5000 10.55 ->
+// 8.50, 10000 17.8 -> 14.4, stored as well 19.4 -> 16.9; rotation alone 900 2.84 -> 2.46, 10000 11.7 both.)
+constexpr int FWHT_ROW = 36;           // words a row of 32: 16-byte accesses of eight rows, and 4-byte ones of any, meet no bank twice
 template <bool VEC>
-__global__ void __launch_bounds__(32 * FWHT_WARP_BLOCKS, 8) fwht_quant_warp_kernel(const float *X, const float *signs, float *x_rot, uint32_t *xq, int n_in, int n_tok) {
-    pdl_wait_prior_grid();
-    const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(32, 32) fwht_quant_warp_kernel(const float *X, const float *signs, float *x_rot, uint32_t *xq, int n_in, int n_tok) {
+    __shared__ __align__(16) float sm[32 * FWHT_ROW];
+    const int lane = threadIdx.x;
     const int blocks_per_tok = n_in / FWHT_N;
-    const long long nwarps = (long long)blocks_per_tok * n_tok;
-    const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (w >= nwarps) return;
-    const int tok = (int)(w / blocks_per_tok);
-    const int blk = (int)(w - (long long)tok * blocks_per_tok);
+    const int tok = (int)blockIdx.x / blocks_per_tok, blk = (int)blockIdx.x - tok * blocks_per_tok;
     const size_t base = (size_t)tok * n_in + (size_t)blk * FWHT_N;
-
-    float v[8][4];
+    pdl_wait_prior_grid();
+    float v[32];
+    {
+        float4 f[8];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const float4 f = load_f4<VEC>(X + base + r * 128 + 4 * lane);
-        v[r][0] = f.x; v[r][1] = f.y; v[r][2] = f.z; v[r][3] = f.w;
-    }
-    if (signs) {
+        for (int r = 0; r < 8; ++r) f[r] = load_f4<VEC>(X + base + r * 128 + 4 * lane);
+        if (signs) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const float4 s = load_f4<VEC>(signs + (size_t)blk * FWHT_N + r * 128 + 4 * lane);
-            v[r][0] = __fmul_rn(v[r][0], s.x); v[r][1] = __fmul_rn(v[r][1], s.y);
-            v[r][2] = __fmul_rn(v[r][2], s.z); v[r][3] = __fmul_rn(v[r][3], s.w);
-        }
-    }
-    fwht1024_warp(v, lane);
-    if (x_rot) {
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-            store_f4<VEC>(x_rot + base + r * 128 + 4 * lane, make_float4(v[r][0], v[r][1], v[r][2], v[r][3]));
-    }
-    if (xq) {
-#pragma unroll
-        // four slices side by side, their divisions shared: one after the other each was a chain of shuffles and two divisions (us per call:
-        // 5120 wide, 512 tokens 9.10 -> 8.03, 2048 tokens 24.7 -> 21.7; 17408 wide, 128 tokens 7.53 -> 6.61, 2048 tokens 78.0 -> 67.5; same bits)
-        for (int r0 = 0; r0 < 8; r0 += 4) {
-            float s[4][4];
-            uint32_t word[4], header[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s[r][e] = v[r0 + r][e];
-            quantise_chunks_8lanes<4>(s, lane, word, header);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int chunk = blk * 32 + (r0 + r) * 4 + (lane >> 3);
-                uint32_t *dst = xq + 9 * ((size_t)chunk * n_tok + tok);
-                dst[1 + (lane & 7)] = word[r];
-                if ((lane & 7) == 0) dst[0] = header[r];
+            for (int r = 0; r < 8; ++r) {
+                const float4 s = load_f4<VEC>(signs + (size_t)blk * FWHT_N + r * 128 + 4 * lane);
+                f[r].x = __fmul_rn(f[r].x, s.x); f[r].y = __fmul_rn(f[r].y, s.y);
+                f[r].z = __fmul_rn(f[r].z, s.z); f[r].w = __fmul_rn(f[r].w, s.w);
             }
         }
+        const float2 minus = make_float2(-1.0f, -1.0f);
+        float2 a[8], b[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {           // h = 1, 2
+            const float s0 = __fadd_rn(f[r].x, f[r].y), s1 = __fsub_rn(f[r].x, f[r].y), s2 = __fadd_rn(f[r].z, f[r].w), s3 = __fsub_rn(f[r].z, f[r].w);
+            a[r] = add2(make_float2(s0, s1), make_float2(s2, s3));
+            b[r] = fma2(make_float2(s2, s3), minus, make_float2(s0, s1));
+        }
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {           // h = 4, 8, 16: own + other, or other - own
+            const float sign = (lane >> s) & 1 ? -1.0f : 1.0f;
+            const float2 sign2 = make_float2(sign, sign);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const float2 oa = make_float2(__shfl_xor_sync(0xffffffffu, a[r].x, 1 << s), __shfl_xor_sync(0xffffffffu, a[r].y, 1 << s));
+                const float2 ob = make_float2(__shfl_xor_sync(0xffffffffu, b[r].x, 1 << s), __shfl_xor_sync(0xffffffffu, b[r].y, 1 << s));
+                a[r] = fma2(a[r], sign2, oa);
+                b[r] = fma2(b[r], sign2, ob);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+            *reinterpret_cast<float4 *>(sm + (4 * r + (lane >> 3)) * FWHT_ROW + 4 * (lane & 7)) = make_float4(a[r].x, a[r].y, b[r].x, b[r].y);
+        __syncwarp();
+        float2 z[16];                           // chunks 2 k and 2 k + 1
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const float lo = sm[2 * k * FWHT_ROW + lane], hi = sm[(2 * k + 1) * FWHT_ROW + lane];
+            z[k] = make_float2(__fadd_rn(lo, hi), __fsub_rn(lo, hi));          // h = 32
+        }
+#pragma unroll
+        for (int s = 0; s < 4; ++s)             // h = 64 .. 512
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+                if (!((k >> s) & 1)) {
+                    const float2 lo = z[k], hi = z[k | (1 << s)];
+                    z[k] = add2(lo, hi);
+                    z[k | (1 << s)] = fma2(hi, minus, lo);
+                }
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[2 * k] = __fmul_rn(z[k].x, 0.03125f), v[2 * k + 1] = __fmul_rn(z[k].y, 0.03125f);
+    }
+    if (x_rot) {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) x_rot[base + 32 * c + lane] = v[c];
+    }
+    if (!xq) return;
+#pragma unroll
+    for (int c = 0; c < 32; ++c) sm[c * FWHT_ROW + lane] = v[c];           // the words this lane has read
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float4 f = *reinterpret_cast<const float4 *>(sm + lane * FWHT_ROW + 4 * j);
+        v[4 * j] = f.x; v[4 * j + 1] = f.y; v[4 * j + 2] = f.z; v[4 * j + 3] = f.w;
+    }
+    float top[4] = {fabsf(v[0]), fabsf(v[1]), fabsf(v[2]), fabsf(v[3])};      // (not 0: of a chunk of NaN it is NaN)
+#pragma unroll
+    for (int i = 4; i < 32; ++i) top[i & 3] = fmaxf(top[i & 3], fabsf(v[i]));
+    const float d = __fdiv_rn(fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])), 127.0f);
+    const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+    uint32_t word[8];
+    int sum = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {               // word 4 a + m: values 16 a + m, + 4, + 8, + 12
+        word[i] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int q = max(-127, min(127, round_ties_away(__fmul_rn(v[16 * (i >> 2) + (i & 3) + 4 * j], id))));
+            word[i] |= ((uint32_t)q & 0xFFu) << (8 * j);
+        }
+        sum = __dp4a((int)word[i], 0x01010101, sum);
+    }
+    __syncwarp();                               // every row has been read
+    uint32_t *out = reinterpret_cast<uint32_t *>(sm);
+    out[9 * lane] = f32_to_f16_bits_ties_away(d) | (((uint32_t)sum & 0xFFFFu) << 16);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) out[9 * lane + 1 + i] = word[i];
+    __syncwarp();
+    const int part = lane / 9;                  // three chunks of nine words at a time
+    uint32_t *dst = xq + 9 * ((size_t)(blk * 32 + part) * n_tok + tok) + (lane - 9 * part);
+    if (lane < 27) {
+#pragma unroll
+        for (int k = 0; k < 11; ++k)
+            if (k < 10 || part < 2) dst[(size_t)k * 27 * n_tok] = out[27 * k + lane];
     }
 }
 

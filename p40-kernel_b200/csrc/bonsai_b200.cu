@@ -445,17 +445,12 @@ GemvPlan plan_rows(long long n_out, size_t row_bytes, size_t fixed, int granule,
 int launch_fwht(bool vec, const float *x, const float *signs, float *x_rot, void *xq, int64_t n_in, int64_t n_tok, bonsai_stream stream) {
     const long long blocks = (n_in / FWHT_N) * n_tok;
     if (blocks > INT32_MAX) return 1;
-    // A CTA per block for few blocks (a short chain, eight warps on it), a block per warp for many (a third of the instructions).  The line,
-    // in blocks per SM, with the times on both sides: 10 with the quantiser (1480 blocks: 6.5 us and 6.4, 1000: 5.0 and 5.5, 34816:
-    // 116 and 78); 18 where the rotated vector is stored as well or accesses are scalar (2500: 9.7 and 9.9, 3000: 11.3 and 11.0); 2 for
-    // the rotation alone (256: 2.3 and 2.2, 148: 2.0 and 2.4).
-    const bool warps = blocks > (long long)SM_COUNT * (!xq ? 2 : (x_rot || !vec ? 18 : 10));
-    const long long ctas = warps ? (blocks + FWHT_WARP_BLOCKS - 1) / FWHT_WARP_BLOCKS : blocks;
-    if (warps)
-        return (int)launch(vec ? fwht_quant_warp_kernel<true> : fwht_quant_warp_kernel<false>, dim3((unsigned)ctas), dim3(32 * FWHT_WARP_BLOCKS), 0,
-                           as_stream(stream), true, x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
-    return (int)launch(vec ? fwht_quant_kernel<true> : fwht_quant_kernel<false>, dim3((unsigned)ctas), dim3(FWHT_THREADS), 0, as_stream(stream), true,
-                       x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
+    // A CTA per block for few blocks (a short chain, eight warps on it), a warp per block for many (a third of the instructions).  The line, in blocks per SM,
+    // with the times on both sides: 2 with the quantiser (200 blocks: 2.29 us and 2.34, 340 2.78 and 2.68, 500 3.22 and 2.56; in front of their mat-mul 240 22.35
+    // and 22.65, 340 34.5 and 33.5), 1 for the rotation alone (120: 1.89 and 2.00, 200: 2.18 and 1.84).
+    const bool warps = blocks > (long long)SM_COUNT * (xq ? 2 : 1);
+    return (int)launch(warps ? (vec ? fwht_quant_warp_kernel<true> : fwht_quant_warp_kernel<false>) : (vec ? fwht_quant_kernel<true> : fwht_quant_kernel<false>),
+                       dim3((unsigned)blocks), dim3(warps ? 32 : FWHT_THREADS), 0, as_stream(stream), true, x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
 }
 
 }  // namespace

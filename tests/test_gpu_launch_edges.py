@@ -247,3 +247,25 @@ def test_rotation_and_quantiser_forms(gpu, blocks, odd):
         assert torch.equal(xb[:, b].reshape(-1), q1), b
         assert gpu.quant_activations(one, q1, N) == 0
         assert torch.equal(xn[:, b].reshape(-1), q1), b
+
+
+@pytest.mark.parametrize("n_in,n_tok", [(1024, 148), (1024, 149), (3072, 98), (3072, 99), (5120, 61)])
+def test_rotation_of_a_batch_on_both_sides_of_a_warp_per_block(gpu, port, n_in, n_tok):
+    """Blocks of several per token through both forms of the rotation: the host's bytes, and of a block with an infinity or a NaN (which the
+    rotation spreads over it) those of the block alone; rotated in place as one vector."""
+    import torch
+    X = synth.activations(n_in, seed=n_tok, batch=n_tok) * 1.7
+    sg = synth.signs(n_in, seed=n_in)
+    want = port.quantize_batch_chunk_major(np.stack([port.fwht_blocks(X[t], sg) for t in range(n_tok)]))
+    x, s, xq = torch.from_numpy(X).cuda(), torch.from_numpy(sg).cuda(), torch.zeros(want.size, dtype=torch.uint8, device="cuda")
+    assert gpu.quant_batch(x, s, xq, n_in, n_tok, True) == 0
+    assert np.array_equal(xq.cpu().numpy(), want)
+    flat, signs = x.reshape(-1).clone(), s.repeat(n_tok)
+    assert gpu.fwht(flat, signs, n_in * n_tok) == 0
+    assert np.array_equal(flat.cpu().numpy(), np.concatenate([port.fwht_blocks(X[t], sg) for t in range(n_tok)]))
+    x[5, 7], x[n_tok - 1, n_in - 1] = float("nan"), float("inf")
+    assert gpu.quant_batch(x, s, xq, n_in, n_tok, True) == 0
+    one = torch.zeros(n_in // 32 * 36, dtype=torch.uint8, device="cuda")
+    for t in (4, 5, n_tok - 1):
+        assert gpu.quant_batch(x[t:t + 1].clone(), s, one, n_in, 1, True) == 0
+        assert torch.equal(xq.view(n_in // 32, n_tok, 36)[:, t].reshape(-1), one), t
