@@ -503,7 +503,6 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
         if (lane == 0) issued[0] = early;
     }
     pdl_wait_prior_grid();
-    // (the next launch comes as this one ends: RMSNorm, quantiser and this, 8 tokens, 5120 -> 17408 20.6 us and 18.3, 17408 -> 5120 23.9 and 22.8, 16 41.1 and 40.5)
     auto wait_count = [&](volatile int *c, int need) -> bool {
         for (uint32_t n = 0; n < (1u << 22); ++n) {
             if (*c >= need) return true;
@@ -708,6 +707,10 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
                 mbar_arrive(&freeb[slot]);
             }
         }
+        // The next launch comes when the first warp runs out of items.  us, at the wait / here / at the end, of this kernel by itself and with RMSNorm and quantiser
+        // in front: 8 tokens 5120 -> 17408 14.6 / 14.5 / 15.0 and 20.7 / 18.9 / 18.7, 17408 -> 5120 19.3 / 19.2 / 20.1 and 23.9 / 23.3 / 23.1, 4 tokens 5120 -> 5120
+        // 8.70 / 8.76 / 9.69 and 13.9 / 12.8 / 12.7, 16 tokens 17408 -> 5120 36.3 / 36.7 / 37.2 and 41.3 / 40.8 / 40.8.
+        if (wid == 0) pdl_launch_dependents();
     } else if (wid == MMAB_C) {
         // weight warp: the rest of the first fill, then (one lane) every tile when its slot's previous tile is taken
         if (ntiles > 0 && !wait_count(&issued[2], 1)) return;
