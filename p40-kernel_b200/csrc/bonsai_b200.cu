@@ -453,6 +453,14 @@ int launch_fwht(bool vec, const float *x, const float *signs, float *x_rot, void
                        dim3((unsigned)blocks), dim3(warps ? 32 : FWHT_THREADS), 0, as_stream(stream), true, x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);
 }
 
+int launch_quant(bool vec, const float *X, void *Xq, int64_t n_in, int64_t n_tok, long long blocks, bonsai_stream stream) {
+    auto run = [&](auto kernel) {
+        return (int)launch(kernel, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, X, static_cast<uint32_t *>(Xq), (int)n_in, (int)n_tok);
+    };
+    if (blocks <= SM_COUNT) return vec ? run(quant_q8_1_kernel<true, true>) : run(quant_q8_1_kernel<false, true>);
+    return vec ? run(quant_q8_1_kernel<true, false>) : run(quant_q8_1_kernel<false, false>);
+}
+
 }  // namespace
 
 extern "C" {
@@ -463,8 +471,7 @@ int bonsai_p40_quant_activations(const float *x, void *out, int64_t n, bonsai_st
     const long long threads = n / 4;
     const int blocks = (int)((threads + 255) / 256);
     // any float pointer is taken, as by the reference; 16-byte aligned ones get 16-byte loads
-    return (int)launch(aligned16(x) ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, x,
-                       static_cast<uint32_t *>(out), (int)n, 1);
+    return launch_quant(aligned16(x), x, out, n, 1, blocks, stream);
 }
 
 int bonsai_p40_fwht(float *x, const float *signs, int64_t n, bonsai_stream stream) {
@@ -493,8 +500,7 @@ int bonsai_b200_quant_batch(const float *X, const float *signs, void *Xq, int64_
     const long long threads = n_in / 4 * n_tok;
     long long blocks = (threads + 255) / 256;
     if (blocks > 8 * SM_COUNT * 4) blocks = 8 * SM_COUNT * 4;
-    return (int)launch(vec ? quant_q8_1_kernel<true> : quant_q8_1_kernel<false>, dim3((unsigned)blocks), dim3(256), 0, as_stream(stream), true, X,
-                       static_cast<uint32_t *>(Xq), (int)n_in, (int)n_tok);
+    return launch_quant(vec, X, Xq, n_in, n_tok, blocks, stream);
 }
 
 // behind_quantiser: the launch before this one on the stream is this library's quantiser, so nothing that is still running
