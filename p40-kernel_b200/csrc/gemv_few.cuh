@@ -108,12 +108,9 @@ __global__ void __launch_bounds__(32 * FEW_WARPS, 2) gemv_few_kernel(const uint8
             if ((lane & 7) == 0) xq_out[9 * chunk] = header;
         }
     }
+    bool ok = true;
     if (nfb == 1) __syncthreads();
-    else if (!__all_sync(0xffffffffu, mbar_wait_hot(tables, 0))) {      // (nobody's bytes may find this CTA gone)
-        cluster_arrive();
-        cluster_wait();
-        return;
-    }
+    else ok = mbar_wait_hot(tables, 0);
 #pragma unroll
     for (int k = 0; k < HELD; ++k) {
         const int u = wid + FEW_WARPS * k;
@@ -136,7 +133,14 @@ __global__ void __launch_bounds__(32 * FEW_WARPS, 2) gemv_few_kernel(const uint8
         }
         terms[u * 32 + lane] = make_float4(t[0], t[1], t[2], t[3]);
     }
-    __syncthreads();
+    // (a warp whose wait ran out comes here too, with terms of whatever lies in the tables: the CTA leaves as a whole)
+    if (!__syncthreads_and(ok ? 1 : 0)) {
+        if (nfb > 1) {                                  // nobody's bytes may find this CTA gone
+            cluster_arrive();
+            cluster_wait();
+        }
+        return;
+    }
     for (int i = wid; i < (pieces ? quads * nseg : 0); i += FEW_WARPS) {
         const int quad = i / nseg, j = i - quad * nseg;
         float acc = 0.0f;
