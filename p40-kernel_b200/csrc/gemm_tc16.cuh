@@ -583,6 +583,7 @@ __global__ void __launch_bounds__(T16C<TN, CTAS>::THREADS, 1) gemm_tc16_kernel(f
                 if (lane == 0) before = count_arrival(counts + (CTAS * head + rank) * T16_PART_COUNTS + wid);
                 before = __shfl_sync(0xffffffffu, before, 0);
                 if (before != (unsigned int)(last - head)) continue;
+                __syncwarp();                               // what lane 0 acquired, every lane may read (a shuffle orders no memory)
                 const float *from = slot_of(head);
 #pragma unroll
                 for (int j = 0; j < COLS; ++j) acc[j] = __ldcg(from + j * T16_M);

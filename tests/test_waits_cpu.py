@@ -1,4 +1,5 @@
-"""Waits that run out, read from the sources (a run in which one runs out would take seconds and show one order of many)."""
+"""Waits that run out and arrivals that are counted, read from the sources (a run shows one order of many, and one in which a wait runs out
+takes seconds)."""
 import re
 
 from test_launch_order_cpu import functions
@@ -37,3 +38,16 @@ def test_no_barrier_behind_a_warp_that_leaves():
             seen.add(name)
             assert not re.search(BARRIER, behind(body, m.end())), (name, m[0])
     assert {"gemv_stream_kernel", "kv_attn_kernel"} <= seen
+
+
+def test_all_who_read_behind_a_count_have_met_who_counted():
+    """One thread counts an arrival and acquires what the others left.  The threads that read it meet that thread at a barrier of their own first:
+    a shuffle or a vote orders no memory."""
+    seen = set()
+    for name, (kernel, _, body) in functions().items():
+        for m in re.finditer(r"count_arrival\(", body) if kernel else ():
+            seen.add(name)
+            rest = body[m.end():]
+            read = re.search(r"__ldcg\(|ld\.global|\bws\b", rest)
+            assert read and re.search(r"__syncwarp\(|__syncthreads", rest[:read.start()]), name
+    assert seen == {"gemm_tc16_kernel", "kv_attn_kernel"}
