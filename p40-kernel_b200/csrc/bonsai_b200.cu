@@ -1589,12 +1589,18 @@ int bonsai_p40_rmsnorm(const float *x, const float *w, float *y, int64_t n_rows,
     if (n > INT32_MAX || n_rows > INT32_MAX || !aligned4(x) || !aligned4(w) || !aligned4(y)) return 1;
     const bool vec = n % 4 == 0 && aligned16(x) && aligned16(w) && aligned16(y);
     const dim3 threads(32 * (unsigned)std::min<int64_t>(RMS_WARPS, (n + 127) / 128));
+    // Behind one row comes its projection, which asks for its weights in front of its wait: it is let in at once.  Behind rows comes a batch's quantiser, which has nothing
+    // to ask for: let in by ending.  us by ending / at once: one row with bonsai_b200_linear 1024 -> 4096 (replayed by a graph) 4.35 / 3.95, 5120 -> 64 5.69 / 5.40, -> 1024 6.72 / 6.22,
+    // -> 1850 7.12 / 6.38, 8192 -> 600 7.76 / 7.22; rows with quantiser and mat-mul 12 x 1024 7.72 / 7.98, 8 x 5120 -> 17408 18.57 / 18.66, -> 5120 13.37 / 13.24, 37 x 5120 23.16 / 23.18,
+    // 100 x 6144 31.9 / 33.1, 148 x 3072 23.1 / 25.6, x 5120 30.8 / 35.0.
+    const bool early = n_rows == 1;
     auto run = [&](auto kernel) {
         return (int)launch(kernel, dim3((unsigned)n_rows), threads, 0, as_stream(stream), true, x, w, y, (int)n, eps);
     };
     auto go = [&](auto hold) {
         constexpr int HOLD = decltype(hold)::value;
-        return vec ? run(rmsnorm_kernel<true, HOLD>) : run(rmsnorm_kernel<false, HOLD>);
+        if (early) return vec ? run(rmsnorm_kernel<true, HOLD, true>) : run(rmsnorm_kernel<false, HOLD, true>);
+        return vec ? run(rmsnorm_kernel<true, HOLD, false>) : run(rmsnorm_kernel<false, HOLD, false>);
     };
     // Rows that fit stay in registers, which costs CTAs per SM: with 16-byte accesses and up to five slices per warp that is ahead at any
     // count of rows (5120 values, 8192 rows: 54 us, 70 us read twice), with eight up to four rows per SM (6144 values, 512 rows: 5.8 and 7.0 us,
@@ -1603,10 +1609,10 @@ int bonsai_p40_rmsnorm(const float *x, const float *w, float *y, int64_t n_rows,
         if (n <= 1024) return go(std::integral_constant<int, 1>{});
         if (n <= 2 * 1024) return go(std::integral_constant<int, 2>{});
         if (n <= 3 * 1024) return go(std::integral_constant<int, 3>{});
-        if (n <= 5 * 1024 && vec) return run(rmsnorm_kernel<true, 5>);
+        if (n <= 5 * 1024 && vec) return early ? run(rmsnorm_kernel<true, 5, true>) : run(rmsnorm_kernel<true, 5, false>);
         if (n <= 8 * 1024) return go(std::integral_constant<int, 8>{});
     }
-    if (!vec && n_rows > 2 * SM_COUNT) return run(rmsnorm_kernel<false, -1>);
+    if (!vec && n_rows > 2 * SM_COUNT) return run(rmsnorm_kernel<false, -1, false>);
     return go(std::integral_constant<int, 0>{});
 }
 
@@ -1614,8 +1620,12 @@ int bonsai_b200_swiglu(const float *gate, const float *up, float *y, int64_t n, 
     if (n <= 0 || n > INT32_MAX || !aligned4(gate) || !aligned4(up) || !aligned4(y)) return 1;
     const bool vec = n % 4 == 0 && aligned16(gate) && aligned16(up) && aligned16(y);
     const int64_t threads = vec ? n / 4 : n;
-    return (int)launch(vec ? swiglu_kernel<true> : swiglu_kernel<false>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, as_stream(stream), true,
-                       gate, up, y, (int)n);
+    const int64_t ctas = (threads + 255) / 256;
+    auto run = [&](auto kernel) { return (int)launch(kernel, dim3((unsigned)ctas), dim3(256), 0, as_stream(stream), true, gate, up, y, (int)n); };
+    // us, the next launch let in by ending / at once: 5120 values with bonsai_b200_linear -> 1024 6.17 / 5.64; with quantiser and mat-mul 8 x 5120 12.8 / 12.6, 16 x 5120 13.0 /
+    // 12.9, 8 x 17408 (136 CTAs) 23.2 / 23.1, 12 x 17408 39.2 / 39.5, 64 x 17408 41.1 / 44.8.
+    if (ctas <= SM_COUNT) return vec ? run(swiglu_kernel<true, true>) : run(swiglu_kernel<false, true>);
+    return vec ? run(swiglu_kernel<true, false>) : run(swiglu_kernel<false, false>);
 }
 
 int bonsai_p40_gdn_step(float *state, const float *q, const float *k, const float *v, const float *g, const float *beta,

@@ -312,11 +312,12 @@ __device__ __forceinline__ uint64_t policy_evict_last_or_default() {
 // option of the caller, who promises that nobody writes them, makes the kernel start early.)
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// A kernel that never lets the next launch in lets it in by ending, CTA by CTA.  That is better where the next one has nothing to do before its own wait: its CTAs
-// would go to what the running kernel leaves free, many on one SM and none on another, and stay there, or take issue slots and memory from it.  us, let in at the
-// first instruction (or launched plainly) / at the end: 512 rows of 5120 RMSNorm + rotation with quantiser 14.4 / 11.5, of 3072 13.1 / 8.2, 148 of 5120 10.1 / 5.5,
-// 700 of 1024 8.27 / 5.72; 37 x 17408 SwiGLU + the same 8.28 / 5.58; with their mat-mul 64 x 17408 47.6 / 43.3, 2 x 5120 9.54 / 9.20.  Where the next kernel asks
-// for its weights or its state first, early it is: mat-vec behind its quantiser, list of delta-net steps, K/V calls (append 37.8 / 44.4, 5120 -> 64 3.16 / 3.56).
+// A kernel that never lets the next launch in lets it in by ending, CTA by CTA.  That is better where the kernel fills much of the chip and the next one has nothing to do
+// before its own wait: its CTAs would go to what the running kernel leaves free, many on one SM and none on another, and stay there, or take issue slots and memory from
+// it.  us, let in at the first instruction (or launched plainly) / at the end: 512 rows of 5120 RMSNorm + rotation with quantiser 14.4 / 11.5, of 3072 13.1 / 8.2, 148 of
+// 5120 10.1 / 5.5, 700 of 1024 8.27 / 5.72; 37 x 17408 SwiGLU + the same 8.28 / 5.58, with the mat-mul 64 x 17408 44.8 / 41.1.  Few CTAs leave it room, and where the next kernel asks
+// for its weights or its state first, early it is: one row's RMSNorm and SwiGLU in front of its projection (bonsai_p40_rmsnorm, bonsai_b200_swiglu), mat-vec behind its
+// quantiser, list of delta-net steps, K/V calls (append 37.8 / 44.4, 5120 -> 64 3.16 / 3.56).
 
 // A coherent load that stays behind the wait (both are volatile), and that the compiler may take in front of stores to shared memory.
 __device__ __forceinline__ uint32_t ldg_u32(const void *p) {

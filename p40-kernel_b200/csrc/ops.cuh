@@ -37,10 +37,11 @@ __device__ __forceinline__ float swiglu1(float g, float u) {
     return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), u);
 }
 
-// VEC: four values per thread (n % 4 == 0, 16-byte aligned pointers).
-template <bool VEC>
+// VEC: four values per thread (n % 4 == 0, 16-byte aligned pointers).  EARLY: the next launch is let in at once, else by ending.
+template <bool VEC, bool EARLY>
 __global__ void __launch_bounds__(256) swiglu_kernel(const float *gate, const float *up, float *y, int n) {
     pdl_wait_prior_grid();
+    if (EARLY) pdl_launch_dependents();
     const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (VEC) {
         if (i < n / 4) {
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const float *gate, const fl
 // One CTA per row.  VEC (n % 4 == 0, all pointers 16-byte aligned): 16-byte accesses; otherwise scalar ones, same order of
 // sums.  HOLD > 0: rows of up to HOLD slices per warp stay in registers between the sum and the product, one trip to memory
 // instead of two; HOLD <= 0 takes rows of any length; HOLD < 0 with few registers, for many CTAs per SM.  A row of less than
-// eight slices has a warp per slice.
+// eight slices has a warp per slice.  EARLY: as above.
 constexpr int RMS_THREADS = 256, RMS_WARPS = RMS_THREADS / 32;
 template <bool VEC>
 __device__ __forceinline__ float4 rms_load(const float *p, int i, int n) {
@@ -85,7 +86,7 @@ __device__ __forceinline__ void rms_store(float *p, int i, int n, float4 f, floa
         if (i + 3 < n) p[i + 3] = f.w;
     }
 }
-template <bool VEC, int HOLD>
+template <bool VEC, int HOLD, bool EARLY>
 __global__ void __launch_bounds__(RMS_THREADS, HOLD < 0 || HOLD == 1 ? 8 : (HOLD == 8 && !VEC ? 3 : 0)) rmsnorm_kernel(const float *x, const float *w, float *y, int n, float eps) {
     constexpr int NW = RMS_WARPS;
     __shared__ __align__(16) float part[512];
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(RMS_THREADS, HOLD < 0 || HOLD == 1 ? 8 : (HOLD
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nslice = (n + 127) >> 7;
     pdl_wait_prior_grid();
+    if (EARLY) pdl_launch_dependents();
     if constexpr (HOLD > 0) {
         float4 f[HOLD], g[HOLD];
 #pragma unroll

@@ -269,3 +269,36 @@ def test_rotation_of_a_batch_on_both_sides_of_a_warp_per_block(gpu, port, n_in, 
     for t in (4, 5, n_tok - 1):
         assert gpu.quant_batch(x[t:t + 1].clone(), s, one, n_in, 1, True) == 0
         assert torch.equal(xq.view(n_in // 32, n_tok, 36)[:, t].reshape(-1), one), t
+
+
+@pytest.mark.parametrize("n_rows,n", [(1, 1024), (1, 5120), (1, 8192), (1, 17408), (2, 1024), (2, 5120), (37, 1028), (148, 1000), (149, 1024), (8, 17408), (9, 17408), (148, 1024)])
+def test_small_operators_in_front_of_their_projection(gpu, n_rows, n):
+    """RMSNorm and SwiGLU on both sides of what lets the next launch in at once, over and over into the same buffers in front of a projection (of
+    rows: of a quantiser): the bits of plain launches."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n_rows * n)
+    xs = [torch.randn(n_rows * n, generator=g, device="cuda") for _ in range(3)]
+    w, n_out = torch.randn(n, generator=g, device="cuda"), 64
+    W = torch.empty(n_out * (n // 128) * 34, dtype=torch.uint8, device="cuda")
+    assert n_rows > 1 or gpu.synth_pq2_0(W, 0, n_out * (n // 128), n) == 0
+    h, y, xq = torch.empty(n_rows * n, device="cuda"), torch.empty(n_out, device="cuda"), torch.empty(n // 32 * 36 * n_rows, dtype=torch.uint8, device="cuda")
+
+    def steps():
+        out = []
+        for i in range(6):
+            call = (lambda: gpu.rmsnorm(xs[i % 3], w, h, n_rows, n, 1e-6)) if i < 3 else (lambda: gpu.swiglu(xs[i % 3], xs[(i + 1) % 3], h, n_rows * n))
+            assert call() == 0
+            if n_rows == 1:
+                assert gpu.linear(W, h, None, y, xq, n_out, n) == 0
+            elif n % 32 == 0:
+                assert gpu.quant_batch(h, None, xq, n, n_rows, False) == 0
+            out += [h.clone(), y.clone() if n_rows == 1 else xq.clone()]
+        return out
+    y.zero_(), xq.zero_()
+    got = steps()
+    try:
+        assert gpu.set_option("overlap", 0) == 0
+        want = steps()
+    finally:
+        gpu.set_option("overlap", 1)
+    assert all(torch.equal(a.view(torch.int32), b.view(torch.int32)) if a.dtype == torch.float32 else torch.equal(a, b) for a, b in zip(got, want))
