@@ -52,11 +52,14 @@ constexpr uint32_t ATC_COL_O = 0, ATC_COL_S = 256, ATC_COL_QL = 384;
 constexpr uint32_t ATC_HUGE = (127u + 60u) << 23;            // bits of 2^60
 constexpr uint32_t ATC_TINY = (127u - 100u) << 23;           // bits of 2^-100: a dim of v all below it is past the shift's cap
 constexpr uint32_t ATC_NONE = 0x7FFFFFFFu;
-// The tensor core cuts the last bits of a tile's sum of weights x v off, in four steps of about the sum's own size: 1.1e-7 of it is missing in the mean (700 - 2048
-// tokens of normal values, least squares against 64 bits; 0.7e-7 of one tile's).  The factor of a dim, a power of two, is one unit in the last place larger
-// for that: relative error 2.01e-7 -> 1.68e-7 at 1024 tokens, of positive v 2.2e-7 -> 1.1e-7.  (The scores' sums, short as they are, need none: with 4e-8 to 1e-7 more of
-// them 1.70e-7 - 1.73e-7.)
-constexpr float ATC_V_LIFT = 1.0f + 0x1p-23f;
+// The tensor core cuts the last bits of a sum of weights x v off, a step of 16 keys at a time.  What is missing in the mean (24 heads over 4, normal values, least squares
+// against 64 bits, 1e-7 of the output): rows of 1 key 0.0, 2 0.4, 3 - 16 0.6, 17 - 32 1.0, 33 - 64 1.35, 1024 - 2048 1.55 (of positive v 0.0, 0.4, 0.5, 0.8, 1.65, 2.1; of queries a
+// twentieth as large 0.0, 0.35, 0.4, 0.6, 0.85, 0.9); long rows whose softmax sits on one key, to 2^-6 of it, 0 - 0.5.  So a row's output is one unit in the last place larger where it sees
+// more than 16 keys and its weights add up to more than that.  Relative error of a prompt, without / for every row / as here: normal 256 tokens 1.82e-7 / 1.57e-7 / 1.51e-7, 2047
+// 2.09e-7 / 1.74e-7 / 1.72e-7; positive v 2.23e-7 / 1.21e-7 / 1.26e-7; of a row of one key 4.3e-8 / 1.24e-7 / 4.3e-8.  (The scores' sums, short as they are, need none: with 4e-8 to 1e-7
+// more of them 1.70e-7 - 1.73e-7.)
+constexpr float ATC_LIFT = 1.0f + 0x1p-23f, ATC_LIFT_WEIGHTS = 1.0f + 0x1p-6f;
+constexpr int ATC_LIFT_KEYS = 17;
 constexpr int ATC_V_RANGE = 12;                              // log2
 constexpr float ATC_QK_RANGE = 4096.0f;
 constexpr int ATC_REDO_QUERIES = ATC_WARPS * ATT_QPW;
@@ -168,7 +171,7 @@ __global__ void __launch_bounds__(ATC_PREP_THREADS) attn_planes_kernel(const flo
 #pragma unroll
         for (int e = 0; e < ATC_KEYS; ++e) seen = max(seen, atc_abs_bits(x[e]));
         const int s = atc_shift(seen, 112);
-        reinterpret_cast<float *>(img + ATC_IMG_VF)[d] = __fmul_rn(atc_pow2(-s - 14), ATC_V_LIFT);          // (and the weights' 2^-14)
+        reinterpret_cast<float *>(img + ATC_IMG_VF)[d] = atc_pow2(-s - 14);          // (and the weights' 2^-14)
 #pragma unroll
         for (int g = 0; g < ATC_KEYS / 8; ++g) {
             uint4 hi, lo;
@@ -523,7 +526,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
         return;
     }
     const float l = __fadd_rn(__fadd_rn(red[row], red[ATC_M + row]), __fadd_rn(red[2 * ATC_M + row], red[3 * ATC_M + row]));
-    const float inv = __fdiv_rn(1.0f, l);
+    const float inv = __fdiv_rn(query + 1 >= ATC_LIFT_KEYS && l >= ATC_LIFT_WEIGHTS ? ATC_LIFT : 1.0f, l);
     if ((reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
 #pragma unroll
         for (int c = 0; c < 16; ++c)

@@ -66,6 +66,37 @@ def test_short_prompts(gpu, n, heads, kv_heads, spread):
     test_against_float64(gpu, n, heads, kv_heads, spread)
 
 
+def signed_error(got, want):
+    """Mean error in the direction of the result, relative to it."""
+    want = want.double()
+    return float(((got.double() - want) * want).sum() / (want * want).sum())
+
+
+@pytest.mark.parametrize("n", [256, 2048])
+def test_what_the_sums_lose(gpu, n):
+    """The tensor core cuts sums off, which is put back in the mean and only where something was cut: rows of one key and rows whose softmax sits
+    on one key are v to what a plane pair keeps of it (22 bits at least, 2^-23 at most lost, in the mean nothing: a tenth of 2^-22 is allowed), ones
+    stay ones in the first row, and the rows of a prompt are right in the mean to 0.6e-7 (1.0e-7 - 1.6e-7 was cut off)."""
+    import torch
+    heads, kv_heads = 24, 4
+    q, k, v = inputs(n, heads, kv_heads, 3)
+    own = v.repeat_interleave(heads // kv_heads, 1)
+
+    def run(q, k, v):
+        out = torch.full((n, heads, D), float("nan"), device="cuda")
+        assert gpu.attn(q, k, v, out, n, heads, kv_heads, D, SCALE) == 0
+        return out
+    out = run(q, k, v)
+    assert float((out[0] - own[0]).abs().max()) <= 2 ** -23 * float(v.abs().max()) and abs(signed_error(out[0], own[0])) < 0.25e-7
+    want = exact(q, k, v)
+    for rows in (slice(16, 64), slice(64, n)):
+        assert abs(signed_error(out[rows], want[rows])) < 0.6e-7, rows
+    assert bool((run(q, k, torch.ones_like(v))[0] == 1).all())
+    # a query that is ten times its own key: 160 against at most some 50 for any other
+    one = run(10 * k.repeat_interleave(heads // kv_heads, 1), k, v)
+    assert float((one - own).abs().max()) <= 2 ** -23 * float(v.abs().max()) and abs(signed_error(one, own)) < 0.25e-7
+
+
 def test_values_that_do_not_survive_the_split(gpu):
     """Infinities, NaN and huge values give what the CUDA-core kernel gives: rows in front of them are untouched, rows behind
     see them where their weight is not zero."""
