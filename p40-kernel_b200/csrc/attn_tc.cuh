@@ -21,8 +21,8 @@
 // Shared memory: q high, k and v images of one tile, 64 KB each (K-major, 128-byte swizzle).  Tensor memory, all 512
 // columns: 256 output (before that, sums of the scores), 128 scores (then weights), 128 q low.
 // What bounds it (counted while a score was four sums): per tile 5900 of 10200 cycles were the tensor core's, most of them the score
-// products (N = 64: it waits for the q rows from shared memory), the rest softmax and the exchanges in front of it.  2048 tokens, 24 heads over 4: 2570 ->
-// 279 us; 1000 tokens 727 -> 90 us, 600 tokens 59 us, 511 tokens 146 -> 56 us, 300 tokens 85 -> 39 us.
+// products (N = 64: it waits for the q rows from shared memory), the rest softmax and the exchanges in front of it.  us, CUDA cores / here, 24 heads over 4:
+// 2048 tokens 2054 / 236, 1000 511 / 78, 600 196 / 52, 300 86 / 31.
 //
 // A plane pair holds 2^-39 of the largest value under its power of two, so what is far smaller loses bits to values that a row may not
 // even see.  A CTA whose queries and keys range too widely (atc_too_wide) does its queries again on the CUDA cores (attn_simt), with
@@ -35,11 +35,12 @@
 
 namespace b200 {
 
-// From this token count on.  It is faster from 160 tokens on (us, CUDA cores / here, 24 heads over 4: 100 19.7 / 26, 128 28 / 30, 192 40 / 30, 300 85 / 39, 511 146 /
-// 56), and of short rows the CUDA cores' sums are short enough to be the more exact ones.  Relative error against 64 bits, CUDA cores /
-// here (24 heads over 4): normal values 128 tokens 1.39e-7 / 1.50e-7, 192 1.55e-7 / 1.54e-7, 250 1.67e-7 / 1.57e-7, 511 2.06e-7 / 1.61e-7, 2047 3.4e-7 / 1.73e-7; of positive
-// v 192 1.57e-7 / 1.08e-7; of queries four times as large 192 2.75e-7 / 2.76e-7, 250 2.97e-7 / 2.88e-7; a twentieth as large 192 1.17e-7 / 1.19e-7, 250 1.29e-7 / 1.19e-7.
-constexpr int ATC_MIN_TOKENS = 192;
+// From this token count on.  It is faster from 100 tokens on (us, CUDA cores / here, 24 heads over 4: 100 19.6 / 18.5, 128 27.4 / 19.3, 192 40.2 / 22.6, 223 46.4 / 27.0, 300 85.6 / 31.0, 511
+// 146 / 44.6), but of short rows the CUDA cores' sums are short enough to be the more exact ones.  Relative error against 64 bits, 1e-7, CUDA cores / here (24 heads over 4): normal
+// values 192 tokens 1.54 / 1.49, 224 1.62 / 1.49, 511 2.07 / 1.58, 2047 3.41 / 1.72; positive v 192 1.56 / 1.05, 224 1.67 / 1.07; queries a twentieth as large 192 1.17 / 0.97, 224
+// 1.25 / 0.98; four times as large 192 2.75 / 2.76, 208 2.83 / 2.79, 224 2.87 / 2.81, 256 3.00 / 2.87, 511 3.64 / 3.13.  (Scores of some tens, where the softmax of most rows sits on one or
+// two keys, are less exact here at every length: queries sixteen times as large 224 4.22 / 4.94, 511 4.85 / 5.43, 2047 5.61 / 6.27.)
+constexpr int ATC_MIN_TOKENS = 224;
 constexpr int ATC_M = 128, ATC_KEYS = 64, ATC_WARPS = 16, ATC_THREADS = ATC_WARPS * 32;
 constexpr int ATC_CHUNK = 128 * 128;                         // bytes of 128 rows x 64 fp16
 constexpr int ATC_PLANES = 4 * ATC_CHUNK;                    // q high; k high + low; v high + low: 64 KB each

@@ -6,6 +6,8 @@ additions per score and 12 per tile of outputs); the largest error seen on the C
 import numpy as np
 import pytest
 
+from captured import launches
+
 pytestmark = pytest.mark.gpu
 
 D = 256
@@ -64,6 +66,16 @@ def test_short_prompts(gpu, n, heads, kv_heads, spread):
     """Few queries, by CTAs of 8 and of 16, the lengths next to where the tensor cores begin to serve, and between there and 512 (the same oracle and
     bound)."""
     test_against_float64(gpu, n, heads, kv_heads, spread)
+
+
+@pytest.mark.parametrize("n,kernels", [(191, 1), (192, 1), (223, 1), (224, 2), (225, 2)])
+def test_where_the_tensor_cores_begin(gpu, n, kernels):
+    """One launch on the CUDA cores, which up to here are the more exact ones for some inputs; then two, and scratch."""
+    import torch
+    q, k, v = inputs(n, 24, 4, n)
+    out = torch.empty(n, 24, D, device="cuda")
+    assert len(launches(lambda: gpu.attn(q, k, v, out, n, 24, 4, D, SCALE))) == kernels
+    close(out, exact(q, k, v))
 
 
 def signed_error(got, want):
