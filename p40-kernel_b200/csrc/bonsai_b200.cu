@@ -1674,9 +1674,9 @@ int bonsai_p40_attn(const float *q, const float *k, const float *v, float *out, 
         const int rc = launch_attn_tc(q, k, v, out, n_tok, n_head, n_head_kv, scale, as_stream(stream));
         if (rc >= 0) return rc;
     }
-    // CTAs of 16 queries, or of 8 where those of 16 fill only half of the SMs or leave the last of two or three rounds half empty.  us by 32, 16, 8 queries: 24 heads,
-    // 16 tokens 6.4 / 6.6 / 5.1, 30 11.6 / 8.5 / 7.3, 70 18.1 / 13.3 / 15.4, 100 25.3 / 19.7 / 23.0, 130 31.5 / 27.7 / 30.4, 191 45.3 / 51.5 / 40.1; 64 heads,
-    // 50 14.1 / 16.3 / 12.9, 100 39 / 32 / 29, 191 76 / 63 / 82.
+    // CTAs of 16 queries, or of 8 where those of 16 fill only half of the SMs or leave the last of two or three rounds half empty.  us by 16, 8 queries: 24 heads,
+    // 16 tokens 6.5 / 4.9, 30 7.9 / 7.0, 70 12.6 / 13.2, 100 18.4 / 20.1, 130 26.3 / 26.8, 150 33.9 / 31.1, 191 49.2 / 37.4; 64 heads, 50 15.8 / 12.4, 100 31.5 / 25.6 (a fourth round
+    // of four CTAs: not looked for), 160 47.9 / 52.5, 191 60.8 / 72.6.  (Of 32 queries, with eight warps: 16 tokens 6.4, 191 45.3; 64 heads 191 76.)
     static SmemOptIn opt[2];
     const long long of16 = (long long)n_head * ((n_tok + 15) / 16);
     const bool few = 2 * of16 <= SM_COUNT || (2 * of16 > 3 * SM_COUNT && of16 <= 3 * SM_COUNT);

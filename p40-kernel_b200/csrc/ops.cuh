@@ -258,8 +258,8 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_step_kernel(float *state, 
 }
 
 // ---- causal attention, head_dim 256 ------------------------------------------------------------------------------
-// A warp owns FOUR consecutive queries of a head; lane l owns dimensions 8l .. 8l+7 of q and of the outputs.  The eight
-// warps of a CTA take 32 consecutive queries of ONE head, so they walk the same keys and values: a tile of 32 keys (K
+// A warp owns FOUR consecutive queries of a head; lane l owns dimensions 8l .. 8l+7 of q and of the outputs.  The two or four
+// warps of a CTA take 8 or 16 consecutive queries of ONE head (attn_redo: sixteen, 64), so they walk the same keys and values: a tile of 32 keys (K
 // and V rows, 64 KB) is staged in shared memory once per CTA, and every row a warp reads from it serves four queries
 // (with one query per warp the kernel was bound by shared-memory bandwidth: 2 KB read per (query, key)).  Scores: for
 // eight keys at a time the lanes' partial dot products of the 4 x 8 (query, key) pairs go through one transposing
@@ -423,10 +423,11 @@ __device__ __forceinline__ void attn_simt(float *att_smem, const float *q, const
 
 // Bound by issue, and where the CTAs do not fill the SMs by a warp's chain: 8 us for a tile of 32 keys, five times its instructions, of which 1 - 2 were the
 // wait for its rows (now copied asynchronously, a tile ahead).  Weights through shared memory instead of a shuffle for each of the lanes' 128, launches that
-// begin while the one in front drains, CTAs of 16 or 8 queries (were 32): 24 heads over 4, us, before -> now: 1 token 4.7 -> 2.8, 16 8.3 -> 5.1, 30 12.1 -> 7.3, 70 18.5 ->
-// 13.4, 100 26.7 -> 19.7, 130 34.7 -> 27.7, 191 49.2 -> 40.1; the same bits.
+// begin while the one in front drains, CTAs of 16 or 8 queries (were 32): 24 heads over 4, us, before -> now: 1 token 4.7 -> 2.7, 16 8.3 -> 4.9, 30 12.1 -> 7.0, 70 18.5 ->
+// 12.6, 100 26.7 -> 18.4, 130 34.7 -> 26.3, 191 49.2 -> 37.4; the same bits.  Shared memory holds three CTAs per SM of either size, and with the registers that three leave nothing is
+// spilled (bound to four or eight, 128 registers a thread: 36 bytes; 100 tokens 19.6, 191 39.7; 64 heads 100 tokens 30.7, now 31.5, 191 62.1 and 60.8).
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) attn_kernel(const float *q, const float *k, const float *v, float *out, int n_tok, int n_head, int n_head_kv, float scale) {
+__global__ void __launch_bounds__(WARPS * 32, 3) attn_kernel(const float *q, const float *k, const float *v, float *out, int n_tok, int n_head, int n_head_kv, float scale) {
     extern __shared__ __align__(16) float att_smem[];
     // the longest rows of keys first: what starts last is short
     constexpr int QUERIES = WARPS * ATT_QPW;

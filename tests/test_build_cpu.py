@@ -100,3 +100,20 @@ def test_mat_mul_kernel_keeps_its_registers(tmp_path):
     spilt = {f"{n}, {ctas}": int(stores) for n, ctas, stores in
              re.findall(r"properties for \S*gemm_tc16_kernelILi(\d+)ELi(\d)E\S*\n.*?(\d+) bytes spill stores", run.stderr)}
     assert set(spilt) == set(forms) and all(spilt[f] <= most for f, most in forms.items()), spilt or run.stderr[-2000:]
+
+
+def test_attention_kernel_spills_nothing(tmp_path):
+    """The CUDA-core attention: shared memory lets three CTAs of either size on an SM, and with the registers that three leave nothing is spilled."""
+    spec = importlib.util.spec_from_file_location("bonsai_b200_build_spills_attn", os.path.join(ROOT, "p40-kernel_b200", "build.py"))
+    b = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(b)
+    if not shutil.which(b.NVCC):
+        pytest.skip("no nvcc")
+    src = tmp_path / "forms_attn.cu"
+    src.write_text('#include "ops.cuh"\nusing namespace b200;\n' + "".join(
+        f"template __global__ void b200::attn_kernel<{w}>(const float *, const float *, const float *, float *, int, int, int, float);\n" for w in (2, 4)))
+    run = subprocess.run([b.NVCC, *[f for f in b.FLAGS if f != "-shared"], "-Xptxas", "-v", f"-I{b.CSRC}", "-c", str(src), "-o", str(tmp_path / "forms_attn.o")],
+                         capture_output=True, text=True)
+    assert run.returncode == 0, run.stderr[-2000:]
+    spilt = re.findall(r"properties for \S*11attn_kernelILi(\d)E\S*\n.*?(\d+) bytes spill stores", run.stderr)
+    assert sorted(spilt) == [("2", "0"), ("4", "0")], spilt or run.stderr[-2000:]
