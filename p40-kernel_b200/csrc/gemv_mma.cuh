@@ -385,6 +385,31 @@ __device__ __forceinline__ void mmab_tile_copy(void *dst, const CUtensorMap *map
                  : "memory");
 }
 
+// Outputs that came out infinite, once more term by term, when the compute warps have run out of items: of an infinite weight scale every term is infinite or
+// NaN, with a sign of its own, which a block's sum does not show (the host's 0 x infinity and infinity - infinity are NaN).  By the activation warp, whose
+// code is apart from the multiply's: what is added to that, or a call there, costs more (us without / here / by the compute warps behind their loop / a call where
+// the output is stored: 8 tokens 5120 -> 17408 18.44 / 18.53 / 18.76 / 18.92, 2 tokens 10.93 / 11.04 / 11.10 / 11.26, 9 tokens 27.0 / 27.8 / 27.8 / 27.75, of
+// 17408 -> 5120 8 tokens 21.52 / 21.54 / 22.1 / 21.8, 16 38.1 / 38.2 / 39.0 / 39.8).
+__device__ __forceinline__ void mmab_infinite_again(const uint8_t *W, const uint32_t *Xq, float *Y, int groups, int n_out, int nb, int n_tok) {
+#pragma unroll 1
+    for (int i = (int)threadIdx.x & 31; i < groups * 16 * n_tok; i += 32) {
+        const int at = i / n_tok, tok = i - at * n_tok, row = 16 * ((int)blockIdx.x + (at >> 4) * (int)gridDim.x) + (at & 15);
+        if (row >= n_out || !isinf(Y[(size_t)row * n_tok + tok])) continue;
+        float acc = 0.0f;
+#pragma unroll 1
+        for (int c = 0; c < 4 * nb; ++c) {
+            const unsigned short *blk = reinterpret_cast<const unsigned short *>(W + ((size_t)row * nb + (c >> 2)) * W_BLOCK_BYTES), *code = blk + 1 + 4 * (c & 3);
+            const uint32_t *act = Xq + 9 * ((size_t)c * n_tok + tok);
+            int a[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) a[k] = (int)act[1 + k];
+            const int sumi = chunk_sumi_scaled(code[0] | ((uint32_t)code[1] << 16), code[2] | ((uint32_t)code[3] << 16), a, -64 * (int)(short)(act[0] >> 16));
+            acc = __fadd_rn(acc, __fmul_rn(__fmul_rn(f16_bits_to_f32(blk[0]), f16_bits_to_f32(act[0] & 0xFFFFu)), (float)sumi));
+        }
+        Y[(size_t)row * n_tok + tok] = acc;
+    }
+}
+
 template <bool DUMP, int NTG, int NRG>
 __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t *__restrict__ W, const uint32_t *Xq,
                                                                   float *Y, const MmabGeom P, const int n_tok,
@@ -403,6 +428,7 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
     volatile int *turn = reinterpret_cast<volatile int *>(smem + 272);         // [12] the item whose turn it is to add into the slot's sums
     volatile int *gstage = reinterpret_cast<volatile int *>(smem + 320);       // [16] next segment of the batch's group l
     int *stepdone = reinterpret_cast<int *>(smem + 384);                       // [4] tiles of step q taken, at q % 4
+    volatile int *infinite = reinterpret_cast<volatile int *>(smem + 400);     // whether an output is
     uint8_t *actbuf = smem + 512;
     float *tsum = reinterpret_cast<float *>(actbuf + (size_t)P.act_bufs * P.act_buf_bytes);   // [slot][row group][token group][row 16][tok 8]
     float *gacc = tsum + (size_t)P.nslot * NRG * NTG * 128;                    // [group of the batch][token group][row 16][tok 8]
@@ -489,6 +515,7 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
         issued[0] = 0;
         issued[1] = 0;
         issued[2] = 0;
+        *infinite = 0;
         mbar_fence_init();
         if (P.tiled) asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
     }
@@ -692,6 +719,7 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
 #pragma unroll
                             for (int e2 = 0; e2 < 4; ++e2)
                                 if (tok0 + e2 < n_tok) Y[(size_t)row * n_tok + tok0 + e2] = out[e2];
+                            if (isinf(s.x) || isinf(s.y) || isinf(s.z) || isinf(s.w)) *infinite = 1;
                         }
                     }
                 }
@@ -711,6 +739,7 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
         // in front: 8 tokens 5120 -> 17408 14.6 / 14.5 / 15.0 and 20.7 / 18.9 / 18.7, 17408 -> 5120 19.3 / 19.2 / 20.1 and 23.9 / 23.3 / 23.1, 4 tokens 5120 -> 5120
         // 8.70 / 8.76 / 9.69 and 13.9 / 12.8 / 12.7, 16 tokens 17408 -> 5120 36.3 / 36.7 / 37.2 and 41.3 / 40.8 / 40.8.
         if (wid == 0) pdl_launch_dependents();
+        asm volatile("bar.arrive 1, %0;" ::"n"((MMAB_C + 1) * 32) : "memory");      // (whoever gave up a wait comes here too)
     } else if (wid == MMAB_C) {
         // weight warp: the rest of the first fill, then (one lane) every tile when its slot's previous tile is taken
         if (ntiles > 0 && !wait_count(&issued[2], 1)) return;
@@ -804,6 +833,9 @@ __global__ void __launch_bounds__(MMAB_THREADS, 1) gemm_mma_kernel(const uint8_t
                 issued[1] = qc + 1;
             }
         }
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"((MMAB_C + 1) * 32) : "memory");
+        if (__builtin_expect(*infinite, 0)) mmab_infinite_again(W, Xq, Y, mg, P.n_out, P.nb, n_tok);
     }
 }
 

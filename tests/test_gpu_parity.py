@@ -566,6 +566,33 @@ def test_gemm_tensor_core_ints_and_bound(gpu, port, n_out, n_in, n_tok):
     assert gpu.device_status() == 0
 
 
+@pytest.mark.parametrize("n_out,n_in,n_tok", [(37, 1024, 2), (203, 5120, 8), (100, 17408, 3), (33, 1024, 9), (100, 17408, 16), (70, 384, 5)])
+def test_gemm_small_batch_infinite_scales(gpu, port, n_out, n_in, n_tok):
+    """Rows with an infinite weight scale: what the host's terms add up to, an infinity of either sign where all of the block's agree and NaN where they do
+    not or one is 0 x infinity (a token of zeros among them); the other rows as ever."""
+    import torch
+    nb = n_in // 128
+    W = synth.pq2_0_weights(n_out, n_in, seed=n_tok).reshape(n_out, nb, 34).copy()
+    for r, (b, scale) in enumerate([(0, 0x7C00), (nb - 1, 0xFC00), (nb // 2, 0x7C00), (nb // 3, 0x7C00), (1 % nb, 0xFC00)]):
+        W[r, b, :2] = np.frombuffer(np.uint16(scale).tobytes(), dtype=np.uint8)
+        if r < 3:
+            W[r, b, 2:] = 0xFF              # codes that are all the same: a chunk's sum has the sign of the activations' sum
+    W[5, 0, :2] = W[5, nb - 1, :2] = W[0, 0, :2]
+    W[6, 0, :2], W[6, nb - 1, :2] = W[0, 0, :2], W[1, nb - 1, :2]
+    W = W.reshape(-1)
+    X = synth.activations(n_in, seed=n_out, batch=n_tok)
+    X[0], X[n_tok - 1, :n_in // 2] = np.abs(X[0]), 0
+    Xq = port.quantize_batch_chunk_major(X)
+    want = port.gemm(W, Xq, n_out, n_in, n_tok, threads=4)
+    assert np.isposinf(want[0, 0]) and np.isneginf(want[1, 0]) and np.isposinf(want[2, 0]) and np.isnan(want[:7]).any()
+    Y = torch.full((n_out, n_tok), 777.0, dtype=torch.float32, device="cuda")
+    assert gpu.gemm(dev(W), dev(Xq), Y, n_out, n_in, n_tok) == 0
+    got = host(Y)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[np.isinf(want)], want[np.isinf(want)])
+    assert_close(got[7:], want[7:])
+    assert gpu.device_status() == 0
+
+
 @pytest.mark.parametrize("n_out,n_in,n_tok", [(203, 5120, 9), (100, 17408, 16), (1500, 6144, 12), (40000, 4096, 13),
                                               (33, 1024, 10)])
 def test_gemm_small_batch_up_to_16_tokens(gpu, port, n_out, n_in, n_tok):
