@@ -152,7 +152,7 @@ int bonsai_b200_stream_probe(const void *buf, int64_t bytes, int mode, void *sin
  * A library compiled with -DBONSAI_B200_TUNING (the test build) also takes geometry keys ("gemv_variant",
  * "chain_threads", "chain_seg", "chain_tile_kb", "chain_spread_nb", "gemm_tile") that force a tiling; they change no result bits
  * beyond what the documented options say ("gemm_tile": as another shape of the call would, the bound holds) and are not part of the interface; nor are "kv_wide" (0 = decode attention over the cache keeps
- * clusters of eight CTAs at every length: the same bound, another order of sums) and "refuse_clusters" (the next n launches in clusters
+ * clusters of eight CTAs at every length), "kv_push" (0 = and where one of them serves a kv head, the form for several: both the same bound, another order of sums) and "refuse_clusters" (the next n launches in clusters
  * of CTAs that have a form without them are refused; 0 forgets that any was).
  * Returns 0, or 1 for an unknown key. */
 int bonsai_b200_set_option(const char *key, int64_t value);

@@ -53,6 +53,7 @@ std::atomic<int> g_opt_chain_threads{512};       // threads per CTA of the chain
 std::atomic<int> g_opt_chain_spread_nb{16};
 std::atomic<int> g_opt_chain_tile_kb{16};
 std::atomic<int> g_opt_kv_wide{1};                // decode attention: 0 = clusters of eight CTAs at every length
+std::atomic<int> g_opt_kv_push{1};                // ... 0 = of the eight the form for several clusters at every length
 std::atomic<int> g_opt_gemm_tile{0};              // fp16 tensor-core mat-mul: 0 by estimated time, else tiles of up to 64 tokens (a CTA) or 128 (a pair)
 std::atomic<int> g_opt_chain_seg{40};            // longest row segment of one task, in blocks: 8, 16, 24, 32 or 40        // target bytes of one ring slot
 std::atomic<int> g_opt_gemm_path{-1};          // -1: by token count, 0: integer SIMT kernel, 1: tensor cores, 2: small-batch kernel, 3: integer tensor-core kernel          // 0: streaming kernel (fixed tree order), 1: the host's sequential order
@@ -1553,6 +1554,7 @@ int bonsai_b200_set_option(const char *key, int64_t value) {
         return 0;
     }
     if (!std::strcmp(key, "kv_wide")) { g_opt_kv_wide.store(value != 0); return 0; }
+    if (!std::strcmp(key, "kv_push")) { g_opt_kv_push.store(value != 0); return 0; }
     if (!std::strcmp(key, "chain_tile_kb")) {
         if (value < 4 || value > 48) return 1;
         g_opt_chain_tile_kb.store((int)value);
@@ -1854,7 +1856,7 @@ int bonsai_kv_attn_decode(bonsai_kv_cache *kv, int layer, int pos, const float *
     if (pos < 0 || pos >= kv->capacity) return 1;
     const KvSplits s = kv_splits(pos + 1, kv->max_clusters, kv_wide_runs(kv->resident_wide));
     const bool wide = s.cluster == KV_WIDE_CLUSTER;
-    const int push = s.clusters == 1 && (wide || kv->push_runs) ? (s.chunk <= KV_TILE ? 1 : 2) : 0;
+    const int push = s.clusters == 1 && (wide || (kv->push_runs && g_opt_kv_push.load())) ? (s.chunk <= KV_TILE ? 1 : 2) : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(s.cluster * s.clusters), KVM_KV_HEADS);
     cfg.blockDim = dim3(kv_threads(push));

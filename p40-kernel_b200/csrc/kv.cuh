@@ -5,7 +5,7 @@
 //
 // Layout (unchanged, it is the format, src/kv_cache.h:35-46): head-major, K and V separate,
 // block[((layer * n_kv_head + kv_head) * capacity + pos) * 8 + blk], 34-byte blocks -- the 8 blocks of a position are
-// 272 contiguous bytes, consecutive positions follow each other, so a run of positions of one (layer, kv head) is PUSH
+// 272 contiguous bytes, consecutive positions follow each other, so a run of positions of one (layer, kv head) is ONE
 // contiguous, 16-byte aligned span.
 //
 // Decode on B200: one CTA per (kv head, split of the positions) serves the SIX query heads that share the kv head
