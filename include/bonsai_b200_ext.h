@@ -90,7 +90,7 @@ int bonsai_b200_gemm_dump(const void *W, const void *Xq, float *Y, int32_t *sums
  * 0, 1 for bad arguments, cudaErrorMemoryAllocation (2) when the buffer cannot be had.  No reference counterpart. */
 int bonsai_b200_gemm_reserve(int64_t n_in, int64_t n_tok, bonsai_stream stream);
 
-/* The same for bonsai_p40_attn, which keeps 2 KB per position and kv head per (device, stream) for prompts of 224 tokens and more: a
+/* The same for bonsai_p40_attn, which keeps 2 KB per position and kv head per (device, stream) for prompts of 512 tokens and more: a
  * captured call whose buffer is large enough gives the bits of a plain one, otherwise it runs the CUDA-core kernel, several times
  * slower.  Returns 0 (also where no buffer is needed), 1 for bad arguments, 2 when the buffer cannot be had.  No reference counterpart. */
 int bonsai_b200_attn_reserve(int n_tok, int n_head_kv, bonsai_stream stream);

@@ -22,7 +22,7 @@
 // columns: 256 output (before that, sums of the scores), 128 scores (then weights), 128 q low.
 // What bounds it (counted while a score was four sums): per tile 5900 of 10200 cycles were the tensor core's, most of them the score
 // products (N = 64: it waits for the q rows from shared memory), the rest softmax and the exchanges in front of it.  us, CUDA cores / here, 24 heads over 4:
-// 2048 tokens 2054 / 236, 1000 511 / 78, 600 196 / 52, 300 86 / 31.
+// 2048 tokens 2054 / 236, 1000 511 / 78, 600 196 / 52.
 //
 // A plane pair holds 2^-39 of the largest value under its power of two, so what is far smaller loses bits to values that a row may not
 // even see.  A CTA whose queries and keys range too widely (atc_too_wide) does its queries again on the CUDA cores (attn_simt), with
@@ -35,12 +35,19 @@
 
 namespace b200 {
 
-// From this token count on.  It is faster from 100 tokens on (us, CUDA cores / here, 24 heads over 4: 100 19.6 / 18.5, 128 27.4 / 19.3, 192 40.2 / 22.6, 223 46.4 / 27.0, 300 85.6 / 31.0, 511
-// 146 / 44.6), but of short rows the CUDA cores' sums are short enough to be the more exact ones.  Relative error against 64 bits, 1e-7, CUDA cores / here (24 heads over 4): normal
-// values 192 tokens 1.54 / 1.49, 224 1.62 / 1.49, 511 2.07 / 1.58, 2047 3.41 / 1.72; positive v 192 1.56 / 1.05, 224 1.67 / 1.07; queries a twentieth as large 192 1.17 / 0.97, 224
-// 1.25 / 0.98; four times as large 192 2.75 / 2.76, 208 2.83 / 2.79, 224 2.87 / 2.81, 256 3.00 / 2.87, 511 3.64 / 3.13.  (Scores of some tens, where the softmax of most rows sits on one or
-// two keys, are less exact here at every length: queries sixteen times as large 224 4.22 / 4.94, 511 4.85 / 5.43, 2047 5.61 / 6.27.)
-constexpr int ATC_MIN_TOKENS = 224;
+// From this token count on.  It is faster from 100 tokens on (us, CUDA cores / here, 24 heads over 4: 192 37.5 / 22.6, 224 47.9 / 27.0, 300 85.6 / 31.0, 511 146 / 44.4), but of short rows
+// the CUDA cores' sums are the more exact ones for some inputs: here products of small weights are cut off against the large ones, and scores are a few sums more.  Relative error against 64
+// bits, 1e-7, CUDA cores / here (24 heads over 4):
+//   tokens                                  224            320            511            1000           2047
+//   normal values                           1.62 / 1.50    1.80 / 1.53    2.08 / 1.58    2.62 / 1.65    3.42 / 1.72
+//   q 4 times as large                      2.88 / 2.82    3.19 / 2.96    3.64 / 3.13    4.47 / 3.37    5.70 / 3.65
+//   v of one sign                           1.67 / 1.07    1.96 / 1.09    2.43 / 1.11    3.36 / 1.17    4.78 / 1.26
+//   v of one sign, q 2 times as large       1.77 / 2.02    2.05 / 2.07    2.51 / 2.11    3.42 / 2.16    4.82 / 2.18
+//   v of one sign, q 4 times as large       2.21 / 3.29    2.65 / 3.40    3.57 / 3.50    6.34 / 3.61    13.2 / 3.65
+//   q 16 times as large                     4.22 / 4.86    4.54 / 5.17    4.86 / 5.48    5.21 / 5.86    5.63 / 6.30
+// From 500 tokens on all but the last are better here; those scores (some tens, where the softmax of most rows sits on one or two keys) do not turn.  (What the score's last additions round off,
+// kept and added in front of the exponential: q 16 times as large 224 3.93, 511 4.33, at a tenth of the time; v of one sign 3.22 and 3.42 all the same.)
+constexpr int ATC_MIN_TOKENS = 512;
 constexpr int ATC_M = 128, ATC_KEYS = 64, ATC_WARPS = 16, ATC_THREADS = ATC_WARPS * 32;
 constexpr int ATC_CHUNK = 128 * 128;                         // bytes of 128 rows x 64 fp16
 constexpr int ATC_PLANES = 4 * ATC_CHUNK;                    // q high; k high + low; v high + low: 64 KB each
