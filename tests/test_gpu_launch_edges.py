@@ -302,3 +302,30 @@ def test_small_operators_in_front_of_their_projection(gpu, n_rows, n):
     finally:
         gpu.set_option("overlap", 1)
     assert all(torch.equal(a.view(torch.int32), b.view(torch.int32)) if a.dtype == torch.float32 else torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("n_out,n_in,n_tok", [(1000, 1024, 17), (5120, 5120, 37), (5120, 17408, 37), (17408, 5120, 130)])
+def test_mat_mul_reads_the_weights_written_in_front_of_it(gpu, n_out, n_in, n_tok):
+    """The many-token mat-mul fetches its weights while its activations are split: they are written again in front of each call, as are the activations,
+    and results have the bits of calls made alone."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n_out + n_tok)
+    xs = [torch.randn(n_tok * n_in, generator=g, device="cuda") for _ in range(2)]
+    n = n_out * (n_in // 128)
+    W = torch.empty(n * 34, dtype=torch.uint8, device="cuda")
+    xq = torch.empty(n_in // 32 * 36 * n_tok, dtype=torch.uint8, device="cuda")
+    y = torch.empty(n_tok * n_out, device="cuda")
+
+    def steps(wait):
+        out = []
+        for i in range(6):
+            for call in (lambda: gpu.quant_batch(xs[i % 2], None, xq, n_in, n_tok, True), lambda: gpu.synth_pq2_0(W, 0, n, i), lambda: gpu.gemm(W, xq, y, n_out, n_in, n_tok)):
+                assert call() == 0
+                wait()
+            out.append(y.clone())
+            wait()
+        return out
+    want = steps(torch.cuda.synchronize)
+    got = steps(lambda: None)
+    assert all(torch.equal(a, b) for a, b in zip(want, got)) and not torch.equal(want[0], want[2])
+    assert gpu.device_status() == 0

@@ -38,3 +38,12 @@ def test_early_kernels_read_coherently():
             if not fns[called][0] and called != "attn_redo":      # (the CUDA-core attention reads what the launch in front of the planes wrote)
                 assert "__ldg(" not in fns[called][2] and "ld.global.nc" not in fns[called][2].replace("ld.global.nc.u16", ""), (name, called)
                 assert not re.findall(r"const \w+ \*\s*__restrict__", fns[called][1]), (name, called)
+
+
+def test_kernels_wait_before_they_let_the_next_launch_in():
+    """A launch that starts early waits for one predecessor, which has therefore to be behind its own wait before it lets anybody in.  The many-token mat-mul
+    relies on it without a wait of its own for the weights: the split in front of it has waited for whoever wrote them."""
+    inviting = {n: f[2] for n, f in functions().items() if "pdl_launch_dependents(" in f[2]}
+    assert {"tc16_split_kernel", "quant_q8_1_kernel", "fwht_quant_kernel", "attn_planes_kernel", "gemv_few_kernel", "gemv_stream_kernel", "kv_append_kernel"} <= set(inviting)
+    for name, body in inviting.items():
+        assert 0 <= body.find("pdl_wait_prior_grid(") < body.find("pdl_launch_dependents("), name
