@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) attn_tc_kernel(const float *q,
     };
     // Two warps issue the scores' products, half of the sums each: from one warp 16 dims take 39 (q low) or 55 cycles, and its chain of waits and
     // issues is not overlapped.  (One warp, a barrier for each half of the dims, waits polled back to back: 2048 tokens 287 us, 600 tokens 60.6;
-    // now 279 and 58.9.)
+    // with two 279 and 58.9, when queries and outputs still went by a row per thread.)
     auto issue_qk_a = [&] {                                              // dims 0 .. 63, two sums, into the score columns
         tc_fence_after();
         if (warp == 0) {

@@ -448,7 +448,9 @@ int launch_fwht(bool vec, const float *x, const float *signs, float *x_rot, void
     if (blocks > INT32_MAX) return 1;
     // A CTA per block for few blocks (a short chain, eight warps on it), a warp per block for many (a third of the instructions).  The line, in blocks per SM,
     // with the times on both sides: 2 with the quantiser (200 blocks: 2.29 us and 2.34, 340 2.78 and 2.68, 500 3.22 and 2.56; in front of their mat-mul 240 22.35
-    // and 22.65, 340 34.5 and 33.5), 1 for the rotation alone (120: 1.89 and 2.00, 200: 2.18 and 1.84).
+    // and 22.65, 340 34.5 and 33.5), 1 for the rotation alone (120: 1.89 and 2.00, 200: 2.18 and 1.84).  The same lines serve vectors that are stored as well and 4-byte accesses (replayed by a
+    // graph: with quantiser and stored 250 blocks 2.18 and 2.49, 300 2.59 and 2.63, 400 2.63 and 2.73, 600 4.44 and 3.21, 1800 6.93 and 5.09; by 4 bytes 250 2.39 and 2.63, 300 2.83 and 2.80, 400 2.90
+    // and 2.83, 600 4.57 and 3.41, 1800 7.85 and 5.80; both 400 3.04 and 2.93, 1800 8.47 and 6.18, 10000 40.9 and 26.9; rotation by 4 bytes 160 2.29 and 2.32, 300 2.53 and 2.46, 1800 7.31 and 4.98).
     const bool warps = blocks > (long long)SM_COUNT * (xq ? 2 : 1);
     return (int)launch(warps ? (vec ? fwht_quant_warp_kernel<true> : fwht_quant_warp_kernel<false>) : (vec ? fwht_quant_kernel<true> : fwht_quant_kernel<false>),
                        dim3((unsigned)blocks), dim3(warps ? 32 : FWHT_THREADS), 0, as_stream(stream), true, x, signs, x_rot, static_cast<uint32_t *>(xq), (int)n_in, (int)n_tok);

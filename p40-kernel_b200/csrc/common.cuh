@@ -49,7 +49,7 @@ __device__ __forceinline__ uint32_t f32_to_f16_bits_ties_away(float f) {
 }
 
 // lroundf semantics for |t| < 2^23 (a NaN gives 0, as the host's conversion does on x86-64): towards zero behind the largest float below a half, which takes
-// every t whose fraction is a half or more across the next integer and no other (all 2 x 2^30 floats of that range were compared).
+// every t whose fraction is a half or more across the next integer and no other (all 2.5 x 10^9 floats of that range, of either sign, were compared).
 __device__ __forceinline__ int round_ties_away(float t) { return __float2int_rz(__fadd_rn(t, copysignf(0x1.fffffep-2f, t))); }
 
 // The same, five instructions longer.  For the list launch, whose multiply comes out of the compiler differently with every change around it: with the short

@@ -12,7 +12,7 @@
 //     warp's piece is (four rows) x (one step of 8 blocks), lane = (row, block), as in gemv_stream.cuh, but the steps of a
 //     row are given to different warps, whose terms meet in shared memory to be added in order.  (One warp per four rows: 560
 //     instructions in a chain behind the tables.)
-//   * 10 warps of at most 102 registers: two CTAs per SM, so that the next launch's prologue runs beside this one.
+//   * 10 warps of 70 registers (54 with one piece a warp): two CTAs per SM, so that the next launch's prologue runs beside this one.
 // us per call, two launches -> this (in brackets: replayed by a graph): 5120 -> 64 4.54 -> 3.24 (3.78 -> 3.04), -> 1024 4.92 -> 3.91 (3.88 -> 3.68); 1024 ->
 // 1024 4.16 -> 2.85 (3.33 -> 2.60); which calls take it and why: linear_one_launch.
 #pragma once

@@ -231,7 +231,7 @@ __device__ __forceinline__ void put_activation(uint32_t *act_q, float *act_s, in
 // CL > 1 (with REPACK): the CTAs of a cluster quantise a share of x each and store it into the tables of all of them.
 // Registers: behind a quantiser of its own the mat-vec's CTAs fill the SMs that the next call's quantiser, eight warps of 32 registers, starts on while they run:
 // with 118 per thread there was no room beside them, and calls of 148 CTAs took 1 - 2 us more (5120 -> 2368 6.57 -> 5.44 us, -> 40000 17.7 -> 16.4, 17408 -> 1776
-// 9.2 -> 7.0; with SMs left over the same).  576 threads would have 112.
+// 9.2 -> 7.0; with SMs left over the same).  No CTA has 576 threads: bounded so the compiler takes 96 registers, at 512 it takes 118.
 template <bool FUSED, bool REPACK = false, int CL = 1>
 __global__ void __launch_bounds__(FUSED ? 512 : 576, 1) gemv_stream_kernel(const uint8_t *__restrict__ W, const uint32_t *xq,
                                                              float *y, const StreamParams P,
